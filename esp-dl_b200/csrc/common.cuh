@@ -75,6 +75,9 @@ int read_and_clear_device_error_dwpw();
 int image_preprocess(const espdl_image_desc &d, cudaStream_t s);
 int detect_candidates(const espdl_detect_desc &d, cudaStream_t s);
 int reduce_op(const espdl_reduce_desc &d, cudaStream_t s);
+// average over whole images, as a reduction (reduce.cu)
+bool average_pool_whole_supported(const espdl_pool_desc &d);
+int average_pool_whole(const espdl_pool_desc &d, float scale, cudaStream_t s);
 int pad_op(const espdl_pad_desc &d, cudaStream_t s);
 bool fused_block_supported(const espdl_block_desc &d);
 int fused_block_tc(const espdl_block_desc &d, cudaStream_t s);
@@ -128,6 +131,25 @@ __device__ __forceinline__ long long shift_round64(long long v, int shift, int h
         return q;
     }
     return (long long)((unsigned long long)v << (-shift));
+}
+
+// Constants of the one-add-one-shift int8 epilogue, q = (acc + bias_half) >> shift with bias_half = bias + 2^(s-1) (one less
+// for half to even, see shift_fast in tc_common.cuh).  It equals the wrapping 32-bit bias add and 64-bit rounding shift of
+// the reference as long as nothing leaves 32 bits, i.e. |bias| + |acc| + 2^(s-1) < 2^31; `acc_bound` bounds |acc| (2^14 per
+// term of the sum).  A shift beyond 31 - channels whose weights were all but zero when the model was quantised; model files
+// have shifts up to 39 and saturated biases there - gives 0 for every 32-bit sum: a positive constant below 2^31 shifted
+// out completely.  Returns false for channels that need the general form (shift < 1, a bias close to the type's ends).
+__device__ __forceinline__ bool fast_constants(int bias, int s, int acc_bound, int half_even, int &bias_half, int &shift)
+{
+    if (s > 31) {
+        bias_half = 1 << 29, shift = 31;
+        return acc_bound <= (1 << 29);
+    }
+    const int sh = max(1, s);
+    const unsigned half = 1u << (sh - 1);
+    bias_half = (int)((unsigned)bias + half - (half_even ? 1u : 0u));
+    shift = sh;
+    return s >= 1 && (long long)abs((long long)bias) + acc_bound + (long long)half <= 2147483647ll;
 }
 
 __device__ __forceinline__ int32_t sat8(int32_t v) { return max(-128, min(127, v)); }

@@ -11,6 +11,9 @@
 #include "common.cuh"
 
 #include <climits>
+#include <cooperative_groups.h>
+#include <cstring>
+#include <type_traits>
 
 namespace espdl {
 
@@ -25,7 +28,10 @@ struct ReduceParams {
     long long kstride[6], rstride[6];
     long long outputs, count;
     const float *exp_table;
+    float scale; // AVERAGE_POOL: 2^e_in / area * 2^-e_out as the reference forms it
 };
+
+constexpr int AVERAGE_POOL = 100; // an average pool over the whole image, beside the espdl_reduce_op_t values
 
 // tool::round of a float that may be no int32 (NaN, infinity): such a value converts to the minimum on x86
 __device__ __forceinline__ long long fround_x86(float v, int half_even)
@@ -33,6 +39,87 @@ __device__ __forceinline__ long long fround_x86(float v, int half_even)
     if (!(fabsf(v) < 2147483520.f))
         return (long long)INT_MIN;
     return fround(v, half_even);
+}
+
+// The output code of one integer accumulation (every operator but the product and the sum of exponentials).
+template <typename ACC>
+__device__ __forceinline__ long long finish_integer(const ReduceParams &p, ACC acc)
+{
+    if (p.op == ESPDL_REDUCE_MEAN) {
+        // tool::round(tmp * input_scale / count * output_scale), all in fp32
+        float f = __fmul_rn((float)acc, dl_scale(p.e_in));
+        f = __fdiv_rn(f, (float)(unsigned long long)p.count);
+        f = __fmul_rn(f, dl_rescale(p.e_out));
+        return fround(f, p.half_even);
+    }
+    if (p.op == AVERAGE_POOL) // int8: the reference sums in int32, int16: in int64; both convert the sum to fp32
+        return fround_half_up(__fmul_rn(sizeof(ACC) == 4 ? __int2float_rn((int)acc) : __ll2float_rn((long long)acc), p.scale));
+    if (p.op == ESPDL_REDUCE_L2) {
+        // math::sqrt_newton (dl_math.hpp:83-97): r = (r + x / r) * 0.5 until |r - last| <= 1e-5, every step rounded to fp32
+        const float x = __fmul_rn(sizeof(ACC) == 4 ? __int2float_rn((int)acc) : __ll2float_rn((long long)acc), dl_scale(2 * p.e_in));
+        float r = x;
+        if (x != 0.f) {
+            for (int it = 0; it < 100; it++) {
+                const float last = r;
+                r = __fmul_rn(__fadd_rn(last, __fdiv_rn(x, last)), 0.5f);
+                if (!(fabsf(__fsub_rn(r, last)) > 0.00001f))
+                    break;
+            }
+        }
+        return fround(__fmul_rn(r, dl_rescale(p.e_out)), p.half_even);
+    }
+    if (p.op == ESPDL_REDUCE_LOG_SUM) {
+        // static_cast<float>(sum * input_scale): the integer sum becomes a float before the multiplication
+        const float sumf = sizeof(ACC) == 4 ? __int2float_rn((int)acc) : __ll2float_rn((long long)acc);
+        return fround_x86(__fmul_rn(logf(__fmul_rn(sumf, dl_scale(p.e_in))), dl_rescale(p.e_out)), p.half_even);
+    }
+    if (p.op == ESPDL_REDUCE_SUM || p.op == ESPDL_REDUCE_L1 || p.op == ESPDL_REDUCE_SUM_SQUARE) {
+        const int shift = max(-62, min(62, p.e_out - (p.op == ESPDL_REDUCE_SUM_SQUARE ? 2 * p.e_in : p.e_in)));
+        return sizeof(ACC) == 4 ? (long long)shift_round32((int32_t)acc, max(-31, min(31, shift)), p.half_even)
+                                : shift_round64((long long)acc, shift, p.half_even);
+    }
+    return (long long)acc;
+}
+
+// How an element enters an integer accumulation.
+enum Fold { FOLD_SUM, FOLD_MAX, FOLD_MIN, FOLD_ABS, FOLD_SQUARE };
+
+__host__ __device__ __forceinline__ Fold fold_of(int op)
+{
+    switch (op) {
+    case ESPDL_REDUCE_MAX: return FOLD_MAX;
+    case ESPDL_REDUCE_MIN: return FOLD_MIN;
+    case ESPDL_REDUCE_L1: return FOLD_ABS;
+    case ESPDL_REDUCE_SUM_SQUARE:
+    case ESPDL_REDUCE_L2: return FOLD_SQUARE;
+    default: return FOLD_SUM;
+    }
+}
+
+template <typename ACC>
+__device__ __forceinline__ ACC fold_element(Fold f, ACC acc, ACC v)
+{
+    if (f == FOLD_MAX)
+        return acc > v ? acc : v;
+    if (f == FOLD_MIN)
+        return acc < v ? acc : v;
+    if (f == FOLD_ABS)
+        return acc + (v < 0 ? -v : v);
+    if (f == FOLD_SQUARE)
+        return acc + (ACC)((int)v * (int)v);
+    return acc + v;
+}
+
+template <typename ACC>
+__device__ __forceinline__ ACC fold_partial(Fold f, ACC a, ACC b)
+{
+    return f == FOLD_MAX ? (a > b ? a : b) : (f == FOLD_MIN ? (a < b ? a : b) : a + b);
+}
+
+template <typename T, typename ACC>
+__device__ __forceinline__ ACC fold_start(Fold f)
+{
+    return f == FOLD_MAX ? (ACC)(sizeof(T) == 1 ? -128 : -32768) : (f == FOLD_MIN ? (ACC)(sizeof(T) == 1 ? 127 : 32767) : (ACC)0);
 }
 
 template <typename T, typename ACC>
@@ -49,7 +136,8 @@ __global__ void __launch_bounds__(256) reduce_kernel(ReduceParams p)
         }
         int idx[6] = {0, 0, 0, 0, 0, 0};
         long long off = base;
-        ACC acc = p.op == ESPDL_REDUCE_MAX ? (ACC)lo : (p.op == ESPDL_REDUCE_MIN ? (ACC)hi : (ACC)0);
+        const Fold f = fold_of(p.op);
+        ACC acc = fold_start<T, ACC>(f);
         float facc = p.op == ESPDL_REDUCE_PROD ? 1.f : 0.f; // int8 product, both sums of exponentials
         double dacc = 1.0;                                   // int16 product
         const float in_scale = dl_scale(p.e_in);
@@ -63,16 +151,9 @@ __global__ void __launch_bounds__(256) reduce_kernel(ReduceParams p)
                     dacc = __dmul_rn(dacc, (double)t);
             } else if (p.op == ESPDL_REDUCE_LOG_SUM_EXP) {
                 facc = __fadd_rn(facc, sizeof(T) == 1 ? p.exp_table[(int)v + 128] : expf(__fmul_rn((float)(int)v, in_scale)));
-            } else if (p.op == ESPDL_REDUCE_MAX)
-                acc = acc > v ? acc : v;
-            else if (p.op == ESPDL_REDUCE_MIN)
-                acc = acc < v ? acc : v;
-            else if (p.op == ESPDL_REDUCE_L1)
-                acc += v < 0 ? -v : v;
-            else if (p.op == ESPDL_REDUCE_SUM_SQUARE || p.op == ESPDL_REDUCE_L2)
-                acc += (ACC)((int)v * (int)v);
-            else
-                acc += v;
+            } else {
+                acc = fold_element<ACC>(f, acc, v);
+            }
             for (int r = p.nr - 1; r >= 0; r--) { // odometer over the reduced axes
                 off += p.rstride[r];
                 if (++idx[r] < p.rsize[r])
@@ -82,26 +163,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(ReduceParams p)
             }
         }
         long long q;
-        if (p.op == ESPDL_REDUCE_MEAN) {
-            // tool::round(tmp * input_scale / count * output_scale), all in fp32
-            float f = __fmul_rn((float)acc, dl_scale(p.e_in));
-            f = __fdiv_rn(f, (float)(unsigned long long)p.count);
-            f = __fmul_rn(f, dl_rescale(p.e_out));
-            q = fround(f, p.half_even);
-        } else if (p.op == ESPDL_REDUCE_L2) {
-            // math::sqrt_newton (dl_math.hpp:83-97): r = (r + x / r) * 0.5 until |r - last| <= 1e-5, every step rounded to fp32
-            const float x = __fmul_rn(sizeof(ACC) == 4 ? __int2float_rn((int)acc) : __ll2float_rn((long long)acc), dl_scale(2 * p.e_in));
-            float r = x;
-            if (x != 0.f) {
-                for (int it = 0; it < 100; it++) {
-                    const float last = r;
-                    r = __fmul_rn(__fadd_rn(last, __fdiv_rn(x, last)), 0.5f);
-                    if (!(fabsf(__fsub_rn(r, last)) > 0.00001f))
-                        break;
-                }
-            }
-            q = fround(__fmul_rn(r, dl_rescale(p.e_out)), p.half_even);
-        } else if (p.op == ESPDL_REDUCE_PROD) {
+        if (p.op == ESPDL_REDUCE_PROD) {
             if (sizeof(T) == 1) {
                 q = fround_x86(__fmul_rn(facc, dl_rescale(p.e_out)), p.half_even);
             } else {
@@ -109,24 +171,166 @@ __global__ void __launch_bounds__(256) reduce_kernel(ReduceParams p)
                 const double v = __dmul_rn(dacc, (double)dl_rescale(p.e_out));
                 q = !(fabs(v) < 2147483647.0) ? (long long)INT_MIN : (p.half_even ? (long long)__double2ll_rn(v) : (long long)floor(__dadd_rn(v, 0.5)));
             }
-        } else if (p.op == ESPDL_REDUCE_LOG_SUM) {
-            // static_cast<float>(sum * input_scale): the integer sum becomes a float before the multiplication
-            const float sumf = sizeof(ACC) == 4 ? __int2float_rn((int)acc) : __ll2float_rn((long long)acc);
-            q = fround_x86(__fmul_rn(logf(__fmul_rn(sumf, in_scale)), dl_rescale(p.e_out)), p.half_even);
         } else if (p.op == ESPDL_REDUCE_LOG_SUM_EXP) {
             q = fround_x86(__fmul_rn(logf(facc), dl_rescale(p.e_out)), p.half_even);
-        } else if (p.op == ESPDL_REDUCE_SUM || p.op == ESPDL_REDUCE_L1 || p.op == ESPDL_REDUCE_SUM_SQUARE) {
-            const int shift = max(-62, min(62, p.e_out - (p.op == ESPDL_REDUCE_SUM_SQUARE ? 2 * p.e_in : p.e_in)));
-            q = sizeof(ACC) == 4 ? (long long)shift_round32((int32_t)acc, max(-31, min(31, shift)), p.half_even)
-                                 : shift_round64((long long)acc, shift, p.half_even);
         } else {
-            q = (long long)acc;
+            q = finish_integer<ACC>(p, acc);
         }
         out[o] = (T)max((long long)lo, min((long long)hi, q));
     }
 }
 
+// Reduction over the middle axis of [outer][count][C] (the spatial mean / pool of NHWC maps), integer operators.
+// Bound by memory: every input byte once.  A thread per output walked `count` elements one after another, a byte each, with
+// C threads at work per image (a 184x184x32 map took 2.2 ms, 5 GB/s); here a thread owns V = 16 bytes of channels and every
+// rows-th pixel, eight loads in flight, the partial results meet in shared memory, and with few images up to eight
+// thread blocks of a cluster share one (their partials are read through distributed shared memory by the first).
+// Integer sums and extrema do not depend on the order.
+template <typename T, int V, typename ACC, Fold F>
+__device__ __forceinline__ void fold_vector(ACC (&acc)[V], const T *v)
+{
+    if constexpr (sizeof(T) == 1 && V % 4 == 0 && F == FOLD_SUM) { // byte sums: dp4a against one-hot selectors
+#pragma unroll
+        for (int j = 0; j < V; j++) acc[j] = __dp4a(((const int *)v)[j / 4], 1 << (8 * (j % 4)), acc[j]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < V; j++) acc[j] = fold_element<ACC>(F, acc[j], (ACC)v[j]);
+    }
+}
+
+template <typename T, int V, typename ACC, Fold F>
+__global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int C, int slice_lanes, int slices, int rows)
+{
+    namespace cg = cooperative_groups;
+    __shared__ ACC part[V * 256]; // [channel of the lane][thread]: consecutive threads in consecutive words
+    cg::cluster_group cluster = cg::this_cluster();
+    const int cl = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const long long item = blockIdx.x / cl;
+    const long long image = item / slices;
+    const int slice = (int)(item - image * slices);
+    const int tx = threadIdx.x % slice_lanes, ty = threadIdx.x / slice_lanes;
+    const int c0 = (slice * slice_lanes + tx) * V;
+    const bool active = ty < rows && c0 < C;
+    const ACC start = fold_start<T, ACC>(F);
+    ACC acc[V];
+#pragma unroll
+    for (int j = 0; j < V; j++) acc[j] = start;
+    grid_dep_launch();
+    grid_dep_wait();
+    if (active) {
+        struct alignas(V * sizeof(T)) Vec {
+            T v[V];
+        };
+        const T *src = (const T *)p.in + image * p.count * C + c0;
+        const long long step = (long long)rows * cl;
+        long long r = (long long)rank * rows + ty;
+        auto take = [&](auto depth) { // `depth` loads in flight: a lone image is bound by their latency
+            constexpr int D = decltype(depth)::value;
+            for (; r + (D - 1) * step < p.count; r += D * step) {
+                Vec w[D];
+#pragma unroll
+                for (int u = 0; u < D; u++) w[u] = *(const Vec *)(src + (r + u * step) * C);
+#pragma unroll
+                for (int u = 0; u < D; u++) fold_vector<T, V, ACC, F>(acc, w[u].v);
+            }
+        };
+        take(std::integral_constant<int, 8>{});
+        take(std::integral_constant<int, 2>{});
+        take(std::integral_constant<int, 1>{});
+    }
+#pragma unroll
+    for (int j = 0; j < V; j++) part[j * 256 + threadIdx.x] = acc[j];
+    __syncthreads();
+    int half = 1;
+    while (half < rows) half <<= 1;
+    for (half >>= 1; half; half >>= 1) {
+        if (ty < half && ty + half < rows) {
+            const int other = threadIdx.x + half * slice_lanes;
+#pragma unroll
+            for (int j = 0; j < V; j++) part[j * 256 + threadIdx.x] = fold_partial<ACC>(F, part[j * 256 + threadIdx.x], part[j * 256 + other]);
+        }
+        __syncthreads();
+    }
+    if (cl > 1)
+        cluster.sync();
+    if (rank == 0) {
+        const int lo = sizeof(T) == 1 ? -128 : -32768, hi = sizeof(T) == 1 ? 127 : 32767;
+        const int cols = min(slice_lanes * V, C - slice * slice_lanes * V);
+        for (int col = threadIdx.x; col < cols; col += 256) {
+            const int at = (col % V) * 256 + col / V;
+            ACC sum = part[at];
+            for (int k = 1; k < cl; k++) sum = fold_partial<ACC>(F, sum, cluster.map_shared_rank(part, k)[at]);
+            const long long q = finish_integer<ACC>(p, sum);
+            ((T *)p.out)[image * C + slice * slice_lanes * V + col] = (T)max((long long)lo, min((long long)hi, q));
+        }
+    }
+    if (cl > 1)
+        cluster.sync(); // no block leaves while its partials may still be read
+}
+
+template <typename T, int V, typename ACC>
+int launch_channel_reduce(const ReduceParams &p, long long outer, int C, cudaStream_t s)
+{
+    const int lanes = (C + V - 1) / V;
+    // about sixteen pixels a thread, so that the meeting in shared memory stays small beside the loads (7x7x1280 over 1024 images:
+    // 54 us with five), and at least 128 contiguous bytes a block where the tensor has them
+    const int want = (int)max(1ll, min(256ll, p.count / 16));
+    const int widest = max(8, 256 / want);
+    const int slices = (lanes + widest - 1) / widest, slice_lanes = (lanes + slices - 1) / slices, rows = 256 / slice_lanes;
+    const long long items = outer * slices;
+    // blocks that share an image: only while they do not outnumber what the SMs hold at once, and each thread keeps a full round of loads
+    int cl = 1;
+    while (cl < 8 && items * cl * 2 <= 4ll * num_sms() && p.count >= 8ll * rows * cl) cl *= 2;
+    if (items * cl > 0x7fffffffll)
+        return ESPDL_ERR_TOO_LARGE;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(items * cl)), cfg.blockDim = dim3(256), cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cl, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr, cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    switch (fold_of(p.op)) {
+    case FOLD_SUM: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SUM>, p, C, slice_lanes, slices, rows); break;
+    case FOLD_MAX: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MAX>, p, C, slice_lanes, slices, rows); break;
+    case FOLD_MIN: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MIN>, p, C, slice_lanes, slices, rows); break;
+    case FOLD_ABS: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_ABS>, p, C, slice_lanes, slices, rows); break;
+    case FOLD_SQUARE: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SQUARE>, p, C, slice_lanes, slices, rows); break;
+    }
+    count_launch();
+    return check_launch("channel reduce");
+}
+
+// Below 2 KB an image keeps too few of a block's threads busy: a thread per output then (reduce_kernel, pool_kernel).
+bool channel_reduce_pays(long long count, int C, int elem_size) { return count * C * elem_size >= 2048; }
+
+template <typename T, typename ACC>
+int channel_reduce(const ReduceParams &p, long long outer, int C, cudaStream_t s)
+{
+    const uintptr_t a = (uintptr_t)p.in | (uintptr_t)(C * sizeof(T));
+    if (a % 16 == 0)
+        return launch_channel_reduce<T, 16 / sizeof(T), ACC>(p, outer, C, s);
+    if (a % 4 == 0)
+        return launch_channel_reduce<T, 4 / sizeof(T), ACC>(p, outer, C, s);
+    return launch_channel_reduce<T, 1, ACC>(p, outer, C, s);
+}
+
 } // namespace
+
+bool average_pool_whole_supported(const espdl_pool_desc &d)
+{
+    const long long pixels = (long long)d.in_h * d.in_w;
+    return d.op != ESPDL_POOL_MAX && channel_reduce_pays(pixels, d.c, d.dtype == ESPDL_DTYPE_INT8 ? 1 : 2);
+}
+
+int average_pool_whole(const espdl_pool_desc &d, float scale, cudaStream_t s)
+{
+    ReduceParams p;
+    memset(&p, 0, sizeof(p));
+    p.in = d.input, p.out = d.output, p.op = AVERAGE_POOL, p.scale = scale, p.count = (long long)d.in_h * d.in_w;
+    return d.dtype == ESPDL_DTYPE_INT8 ? channel_reduce<int8_t, int32_t>(p, d.n, d.c, s) : channel_reduce<int16_t, long long>(p, d.n, d.c, s);
+}
 
 int reduce_op(const espdl_reduce_desc &d, cudaStream_t s)
 {
@@ -139,7 +343,7 @@ int reduce_op(const espdl_reduce_desc &d, cudaStream_t s)
     ReduceParams p;
     p.in = d.input, p.out = d.output, p.op = d.op, p.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
     p.e_in = d.in_exponent, p.e_out = d.out_exponent;
-    p.exp_table = d.exp_table;
+    p.exp_table = d.exp_table, p.scale = 0.f;
     p.nk = p.nr = 0, p.outputs = 1, p.count = 1;
     long long stride = 1;
     long long strides[6];
@@ -160,6 +364,23 @@ int reduce_op(const espdl_reduce_desc &d, cudaStream_t s)
     }
     if (abs(p.e_in) > 30 || abs(p.e_out) > 30)
         return ESPDL_ERR_UNSUPPORTED;
+    // [outer][count][C]: one run of reduced axes between kept ones (unit axes may stand anywhere)
+    const bool ordered = d.op == ESPDL_REDUCE_PROD || d.op == ESPDL_REDUCE_LOG_SUM_EXP; // sums in floating point keep the reference's order
+    long long outer = 1, inner = 1;
+    int state = 0; // 0: leading kept axes, 1: reduced, 2: trailing kept
+    for (int i = 0; i < d.ndim && state < 3; i++) {
+        if (d.shape[i] == 1)
+            continue;
+        if (d.reduce[i])
+            state = state <= 1 ? 1 : 3;
+        else if (state == 0)
+            outer *= d.shape[i];
+        else
+            state = 2, inner *= d.shape[i];
+    }
+    if (!ordered && state < 3 && inner <= 65536 && channel_reduce_pays(p.count, (int)inner, d.dtype == ESPDL_DTYPE_INT8 ? 1 : 2))
+        return d.dtype == ESPDL_DTYPE_INT8 ? channel_reduce<int8_t, int32_t>(p, outer, (int)inner, s)
+                                           : channel_reduce<int16_t, long long>(p, outer, (int)inner, s);
     const long long blocks = (p.outputs + 255) / 256;
     const int grid = (int)(blocks < (long long)num_sms() * 8 ? blocks : (long long)num_sms() * 8);
     if (d.dtype == ESPDL_DTYPE_INT8)
