@@ -840,11 +840,11 @@ int fused_block_tc(const espdl_block_desc &d, cudaStream_t s)
     const int half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
     const int e_hidden = p.has_expand ? d.expand_exponent : d.in_exponent;
     p.e1 = EpiConfig{d.expand_bias, d.expand_filter_exponents, nullptr, d.expand_exponent - d.in_exponent, d.expand_filter_exponent, d.per_channel & 1,
-                     d.expand_activation == ESPDL_ACT_RELU, half_even};
+                     d.expand_activation == ESPDL_ACT_RELU, half_even, min(d.in_c, 65536) << 14};
     p.edw = EpiConfig{d.dw_bias, d.dw_filter_exponents, nullptr, d.dw_exponent - e_hidden, d.dw_filter_exponent, (d.per_channel >> 1) & 1,
                       d.dw_activation == ESPDL_ACT_RELU, half_even};
     p.e2 = EpiConfig{d.project_bias, d.project_filter_exponents, nullptr, d.out_exponent - d.dw_exponent, d.project_filter_exponent,
-                     (d.per_channel >> 2) & 1, d.project_activation == ESPDL_ACT_RELU, half_even};
+                     (d.per_channel >> 2) & 1, d.project_activation == ESPDL_ACT_RELU, half_even, min(d.hidden_c, 65536) << 14};
     p.clip1 = d.expand_clip_max > 127 ? 127 : d.expand_clip_max;
     p.clipdw = d.dw_clip_max > 127 ? 127 : d.dw_clip_max;
     if ((p.e1.per_channel && p.has_expand && !p.e1.ew) || (p.edw.per_channel && !p.edw.ew) || (p.e2.per_channel && !p.e2.ew))

@@ -64,6 +64,7 @@ struct BandParams {
     EpiConfig epi;
 };
 
+template <bool EVEN>
 __global__ void __launch_bounds__(BD_THREADS, 1)
 band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, const __grid_constant__ CUtensorMap map2,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ BandParams p)
@@ -219,18 +220,18 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                     if (p.epi.bias)
                         b = ((const int32_t *)p.epi.bias)[c];
                     sh = p.epi.e_shift_base - (p.epi.per_channel ? p.epi.ew[c] : p.epi.ew_scalar);
-                    if (sh < 1 || sh > 24 || b >= (1 << 30) || b <= -(1 << 30))
-                        bad = 1;
-                    sh = max(1, min(24, sh));
                 }
-                fast_s[col].bias_half = b + (1 << (sh - 1));
-                fast_s[col].shift = sh;
+                int bh, fs;
+                if (!fast_constants(b, sh, p.epi.acc_bound, EVEN, bh, fs))
+                    bad = 1;
+                fast_s[col].bias_half = bh;
+                fast_s[col].shift = fs;
             }
             if (bad)
                 atomicOr(slow_flag, 1);
         }
         asm volatile("bar.sync 1, %0;" ::"n"(16 * 32) : "memory");
-        const bool fast = !*slow_flag && !p.epi.half_even && !p.epi.lut_stride; // one fused table rides on the staged form, per-channel tables take the general path
+        const bool fast = !*slow_flag && !p.epi.lut_stride; // one fused table rides on the staged form, per-channel tables take the general path
         const uint32_t fp = epi_param_base(fast_s);
         uint32_t acc_phase = 0;
         bool ok = true;
@@ -264,13 +265,13 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 const int col0 = part * out_pw;
                 const int floor_q = p.epi.relu ? 0 : INT_MIN;
                 if (p.epi.lut)
-                    epilogue_stage_lut(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
+                    epilogue_stage_lut<EVEN>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
                 else if (out_pw == 128)
-                    epilogue_stage<128>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 128, floor_q);
+                    epilogue_stage<128, EVEN>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 128, floor_q);
                 else if (out_pw == 64)
-                    epilogue_stage<64>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 64, floor_q);
+                    epilogue_stage<64, EVEN>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 64, floor_q);
                 else
-                    epilogue_stage<0>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, out_pw, floor_q);
+                    epilogue_stage<0, EVEN>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, out_pw, floor_q);
                 fence_before();
                 fence_async_smem();
                 named_bar(2 + group, 128);
@@ -428,6 +429,7 @@ int conv2d_band_tc(const espdl_conv_desc &d, cudaStream_t s)
     p.epi.e_shift_base = d.out_exponent - d.in_exponent;
     p.epi.ew_scalar = d.filter_exponent, p.epi.per_channel = d.per_channel;
     p.epi.relu = d.activation == ESPDL_ACT_RELU, p.epi.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
+    p.epi.acc_bound = (9 * d.in_c) << 14;
 
     // shared memory: three filter planes, the staging tiles, and as many stages of three input planes as fit
     const size_t fixed = band_fixed_smem(p.ncol);
@@ -468,12 +470,17 @@ int conv2d_band_tc(const espdl_conv_desc &d, cudaStream_t s)
     const size_t smem = fixed + (size_t)p.stages * 3 * BD_A_BYTES;
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] { attr_err = cudaFuncSetAttribute(band_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024); });
+    std::call_once(attr_once, [] {
+        attr_err = cudaFuncSetAttribute(band_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(band_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+    });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(band_tc_kernel)");
     const int total = p.ngroups * p.yblocks * p.segs;
     const int grid = min(total, num_sms());
-    band_tc_kernel<<<grid, BD_THREADS, max(smem, (size_t)120 * 1024), s>>>(maps[0], maps[1], maps[2], mo, p);
+    const auto kernel = p.epi.half_even ? band_tc_kernel<true> : band_tc_kernel<false>;
+    kernel<<<grid, BD_THREADS, max(smem, (size_t)120 * 1024), s>>>(maps[0], maps[1], maps[2], mo, p);
     count_launch();
     return check_launch("band_tc");
 }

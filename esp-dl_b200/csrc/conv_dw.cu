@@ -121,7 +121,7 @@ __device__ __forceinline__ void dw_transpose_col(DwCol<S> &col, const uint32_t (
     col.extra = S == 2 ? raw[S == 2 ? 4 : 0] : 0u;
 }
 
-// Band of a thread whose channels do not qualify for the one-add-one-shift epilogue (a shift outside 1..24, a
+// Band of a thread whose channels do not qualify for the one-add-one-shift epilogue (a shift below 1, a
 // huge bias, half-even rounding or a fused table): plain loops with the general requantisation.  Kept out of line
 // so that the walk below carries none of its registers.
 __device__ __noinline__ void dw3x3_band_general(const DwParams &p, int S, int n, int c0, int oy0, int rows, int x_begin, int x_end)
@@ -148,7 +148,7 @@ __device__ __noinline__ void dw3x3_band_general(const DwParams &p, int S, int n,
             }
 }
 
-template <int S>
+template <int S, bool EVEN>
 __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xsegs, int ytiles, int cols_per_thread)
 {
     constexpr int ROWS_IN = S == 1 ? 6 : 5;
@@ -185,14 +185,14 @@ __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xseg
         }
     }
     int bias[4], shift[4];
-    bool fast = !p.half_even && !p.lut;
+    bool fast = !p.lut;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         bias[i] = p.bias ? __ldg((const int32_t *)p.bias + c0 + i) : 0;
         const int e = p.per_channel ? __ldg(p.ew + c0 + i) : p.ew_scalar;
-        shift[i] = max(-31, min(31, p.e_shift_base - e));
-        // (acc + bias + 2^(s-1)) >> s is exact while nothing can overflow: |acc| <= 9 * 2^14, |bias| < 2^30, 1 <= s <= 24
-        fast = fast && shift[i] >= 1 && shift[i] <= 24 && bias[i] < (1 << 30) && bias[i] > -(1 << 30);
+        int bh, fs;
+        fast = fast_constants(bias[i], p.e_shift_base - e, 9 << 14, EVEN, bh, fs) && fast;
+        bias[i] = bh, shift[i] = fs;
     }
     const int oy0 = yt * ROWS_OUT;
     const int x_begin = xs * cols_per_thread, x_end = min(p.ow, x_begin + cols_per_thread);
@@ -200,9 +200,7 @@ __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xseg
         dw3x3_band_general(p, S, n, c0, oy0, ROWS_OUT, x_begin, x_end);
         return;
     }
-    int init[4]; // accumulators start from bias plus the rounding half
-#pragma unroll
-    for (int i = 0; i < 4; i++) init[i] = bias[i] + (1 << (shift[i] - 1));
+    const int(&init)[4] = bias; // accumulators start from bias plus the rounding half
     const int floor_q = p.relu ? 0 : INT_MIN;
     const int iy0 = oy0 * S - p.pt;
     int ix = x_begin * S - p.pl; // column the row pointers stand on
@@ -257,6 +255,9 @@ __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xseg
         }
 #pragma unroll
         for (int ro = 0; ro < ROWS_OUT; ro++) {
+            if (EVEN)
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[ro][i] += (acc[ro][i] >> shift[i]) & 1;
             const int q0 = max(acc[ro][0] >> shift[0], floor_q), q1 = max(acc[ro][1] >> shift[1], floor_q);
             const int q2 = max(acc[ro][2] >> shift[2], floor_q), q3 = max(acc[ro][3] >> shift[3], floor_q);
             uint32_t hi, wd;
@@ -397,9 +398,9 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
         if (blocks > 0x7fffffffll)
             return ESPDL_ERR_TOO_LARGE;
         if (d.stride_h == 1)
-            dw3x3_dp4a_kernel<1><<<(unsigned)blocks, 128, 0, s>>>(p, xsegs, ytiles, cols);
+            (p.half_even ? dw3x3_dp4a_kernel<1, true> : dw3x3_dp4a_kernel<1, false>)<<<(unsigned)blocks, 128, 0, s>>>(p, xsegs, ytiles, cols);
         else
-            dw3x3_dp4a_kernel<2><<<(unsigned)blocks, 128, 0, s>>>(p, xsegs, ytiles, cols);
+            (p.half_even ? dw3x3_dp4a_kernel<2, true> : dw3x3_dp4a_kernel<2, false>)<<<(unsigned)blocks, 128, 0, s>>>(p, xsegs, ytiles, cols);
     } else if (vec) {
         p.chunks = d.in_c / 16;
         p.total = pixels * p.chunks;

@@ -73,8 +73,8 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, uint32_t sr
                  : "memory");
 }
 
-// The same run for channels outside the one-add-one-shift form (a shift outside 1..24, a huge bias, half-even rounding
-// or a fused table): plain loops over the patch with the general requantisation.
+// The same run for channels outside the one-add-one-shift form (a shift below 1, a huge bias or a fused
+// table): plain loops over the patch with the general requantisation.
 __device__ __noinline__ void dwt_walk_general(const DwtParams &pp, int S, const int8_t *ip, int8_t *op, int in_row_bytes, int out_row_bytes, int c0, int L)
 {
     const DwtSource &p = pp.src;
@@ -95,7 +95,7 @@ __device__ __noinline__ void dwt_walk_general(const DwtParams &pp, int S, const 
             }
 }
 
-template <int S, int CBT>
+template <int S, int CBT, bool EVEN>
 __global__ void __launch_bounds__(DWT_THREADS, 1)
 dw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_out, const __grid_constant__ DwtParams p)
 {
@@ -227,7 +227,7 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             break;
         const int cb = t / p.tiles_per_cb, t_in_cb = t - cb * p.tiles_per_cb;
         if (cb != have_cb && active) {
-            dwt_load_consts<S>(k, p.src, cb * CB + cw * 4);
+            dwt_load_consts<S, EVEN>(k, p.src, cb * CB + cw * 4);
             have_cb = cb;
         }
         const uint32_t *patch = (const uint32_t *)(patch0 + (size_t)stage * p.stage_bytes);
@@ -237,7 +237,7 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 uint32_t *op = obuf + out_off;
                 const int cb4 = CBT ? CBT / 4 : W4;
                 auto store = [=](int ro, int x, uint32_t word) { op[ro * out_row_words + x * cb4] = word; };
-                dwt_walk<S, CBT / 4>(k, patch + in_off, store, in_row_words, W4, p.L, floor_q);
+                dwt_walk<S, CBT / 4, EVEN>(k, patch + in_off, store, in_row_words, W4, p.L, floor_q);
             }
             else
                 dwt_walk_general(p, S, (const int8_t *)(patch + in_off), (int8_t *)(obuf + out_off), in_row_words * 4, out_row_words * 4,
@@ -365,10 +365,14 @@ int dwt_launch(const CUtensorMap &mi, const CUtensorMap &mo, const DwtParams &p,
 {
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] { attr_err = cudaFuncSetAttribute(dw3x3_tma_kernel<S, CBT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DWT_SMEM_BUDGET + 2048)); });
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(dw3x3_tma_kernel<S, CBT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DWT_SMEM_BUDGET + 2048));
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(dw3x3_tma_kernel<S, CBT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DWT_SMEM_BUDGET + 2048));
+    });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(dw3x3_tma_kernel)");
-    launch_overlapped(dw3x3_tma_kernel<S, CBT>, dim3(grid), dim3(DWT_THREADS), smem, s, mi, mo, p);
+    launch_overlapped(p.src.half_even ? dw3x3_tma_kernel<S, CBT, true> : dw3x3_tma_kernel<S, CBT, false>, dim3(grid), dim3(DWT_THREADS), smem, s, mi, mo, p);
     count_launch();
     return check_launch("dw3x3_tma");
 }

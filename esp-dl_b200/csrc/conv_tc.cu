@@ -64,6 +64,7 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, uint32_t sr
                  : "memory");
 }
 
+template <bool EVEN>
 __global__ void __launch_bounds__(CV_THREADS, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
                const ConvTcParams p)
@@ -205,7 +206,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             stage_lut(p.epi.lut, lut_s, et, 16 * 32);
         asm volatile("bar.sync 1, %0;" ::"n"(16 * 32) : "memory");
         // a fused table rides on the staged form; the direct-store form applies it in its general path
-        const bool fast = !*slow_flag && !p.epi.half_even && !p.epi.lut_stride && (long long)p.cin * p.kh * p.kw <= 32768;
+        const bool fast = !*slow_flag && !p.epi.lut_stride && (long long)p.cin * p.kh * p.kw <= 32768;
         const uint32_t fp_base = epi_param_base(fast_s);
         const int floor_q = p.epi.relu ? 0 : INT_MIN;
         const int ry = row_in_tile / p.P, rx = row_in_tile % p.P;
@@ -236,13 +237,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int col0 = part * p.out_pw;
                 const uint32_t fpp = fp_base + (uint32_t)(n0 + col0) * 8u;
                 if (p.epi.lut) {
-                    epilogue_stage_lut(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
+                    epilogue_stage_lut<EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
                 } else if (p.out_pw == 128)
-                    epilogue_stage<128>(t0 + col0, fpp, buf, row_in_tile, 128, floor_q);
+                    epilogue_stage<128, EVEN>(t0 + col0, fpp, buf, row_in_tile, 128, floor_q);
                 else if (p.out_pw == 64)
-                    epilogue_stage<64>(t0 + col0, fpp, buf, row_in_tile, 64, floor_q);
+                    epilogue_stage<64, EVEN>(t0 + col0, fpp, buf, row_in_tile, 64, floor_q);
                 else
-                    epilogue_stage<0>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, floor_q);
+                    epilogue_stage<0, EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, floor_q);
                 // the accumulator is free once this warp's TMEM loads are done: hand it back before the tile is stored
                 fence_before();
                 __syncwarp();
@@ -272,9 +273,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     uint32_t pk[8] = {0, 0, 0, 0, 0, 0, 0, 0};
                     if (fast) {
                         if (p.epi.relu)
-                            requant16_fast<true>(v, fast_s + n0 + c0, pk);
+                            requant16_fast<true, EVEN>(v, fast_s + n0 + c0, pk);
                         else
-                            requant16_fast<false>(v, fast_s + n0 + c0, pk);
+                            requant16_fast<false, EVEN>(v, fast_s + n0 + c0, pk);
                         if (p.epi.lut) { // a fused table on rows that leave unstaged: same lookups on the packed words
 #pragma unroll
                             for (int q = 0; q < 4; q++) pk[q] = lut4(pk[q], smem_u32(lut_s));
@@ -349,6 +350,7 @@ __device__ __forceinline__ void ld16_sum(uint32_t t, int kw, int stride, int32_t
     }
 }
 
+template <bool EVEN>
 static __device__ __noinline__ void epilogue_stage_stacked(uint32_t t0, int kw, int stride, uint32_t fp, uint32_t buf, int row, int pw, uint32_t mask,
                                                            int floor_q, uint32_t tbl)
 {
@@ -377,7 +379,7 @@ static __device__ __noinline__ void epilogue_stage_stacked(uint32_t t0, int kw, 
             }
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                pk[q] = requant4_floor(v + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q);
+                pk[q] = requant4_floor<EVEN>(v + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q);
                 if (tbl)
                     pk[q] = lut4(pk[q], tbl);
             }
@@ -393,7 +395,7 @@ static __device__ __noinline__ void epilogue_stage_stacked(uint32_t t0, int kw, 
         ld16_sum(t0 + c, kw, stride, v);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            pk[q] = requant4_floor(v + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q);
+            pk[q] = requant4_floor<EVEN>(v + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q);
             if (tbl)
                 pk[q] = lut4(pk[q], tbl);
         }
@@ -402,6 +404,7 @@ static __device__ __noinline__ void epilogue_stage_stacked(uint32_t t0, int kw, 
     }
 }
 
+template <bool EVEN>
 __global__ void __launch_bounds__(CV_THREADS, 1)
 conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
                   const __grid_constant__ PatchParams p)
@@ -532,7 +535,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (p.epi.lut)
             stage_lut(p.epi.lut, lut_s, et, 16 * 32);
         asm volatile("bar.sync 1, %0;" ::"n"(16 * 32) : "memory");
-        const bool fast = !*slow_flag && !p.epi.half_even && !p.epi.lut_stride && (long long)p.cin * p.kh * p.kw <= 32768;
+        const bool fast = !*slow_flag && !p.epi.lut_stride && (long long)p.cin * p.kh * p.kw <= 32768;
         const uint32_t fp_base = epi_param_base(fast_s);
         const int floor_q = p.epi.relu ? 0 : INT_MIN;
         uint32_t acc_phase = 0;
@@ -589,7 +592,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     ld16_sum(t0 + col0 + c, p.stack ? p.stack : 1, p.block_n, v);
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        pk[q] = requant4_floor(v + 4 * q, fpp + (uint32_t)(c + 4 * q) * 8u, floor_q);
+                        pk[q] = requant4_floor<EVEN>(v + 4 * q, fpp + (uint32_t)(c + 4 * q) * 8u, floor_q);
                         if (tbl)
                             pk[q] = lut4(pk[q], tbl);
                     }
@@ -608,16 +611,16 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 bulk_wait_read_all();
             named_bar(2 + group, 128);
             if (p.stack)
-                epilogue_stage_stacked(t0 + col0, p.stack, p.block_n, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q,
+                epilogue_stage_stacked<EVEN>(t0 + col0, p.stack, p.block_n, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q,
                                        p.epi.lut ? smem_u32(lut_s) : 0u);
             else if (p.epi.lut)
-                epilogue_stage_lut(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
+                epilogue_stage_lut<EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
             else if (p.out_pw == 128)
-                epilogue_stage<128>(t0 + col0, fpp, buf, row_in_tile, 128, floor_q);
+                epilogue_stage<128, EVEN>(t0 + col0, fpp, buf, row_in_tile, 128, floor_q);
             else if (p.out_pw == 64)
-                epilogue_stage<64>(t0 + col0, fpp, buf, row_in_tile, 64, floor_q);
+                epilogue_stage<64, EVEN>(t0 + col0, fpp, buf, row_in_tile, 64, floor_q);
             else
-                epilogue_stage<0>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, floor_q);
+                epilogue_stage<0, EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, floor_q);
             fence_before();
             __syncwarp();
             if (lane == 0)
@@ -810,6 +813,7 @@ int launch_patch(const espdl_conv_desc &d, PatchParams &p, cudaStream_t s)
     p.epi.e_shift_base = d.out_exponent - d.in_exponent;
     p.epi.ew_scalar = d.filter_exponent, p.epi.per_channel = d.per_channel;
     p.epi.relu = d.activation == ESPDL_ACT_RELU, p.epi.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
+    p.epi.acc_bound = min(d.in_c * d.kh * d.kw, 65536) << 14;
     CUtensorMap ma, mb, mo;
     {
         cuuint64_t dims[4] = {(cuuint64_t)d.in_c, (cuuint64_t)d.in_w, (cuuint64_t)d.in_h, (cuuint64_t)d.n};
@@ -846,13 +850,18 @@ int launch_patch(const espdl_conv_desc &d, PatchParams &p, cudaStream_t s)
         smem = 120 * 1024;
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] { attr_err = cudaFuncSetAttribute(conv_patch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PATCH_SMEM_BUDGET + 1024)); });
+    std::call_once(attr_once, [] {
+        attr_err = cudaFuncSetAttribute(conv_patch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PATCH_SMEM_BUDGET + 1024));
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(conv_patch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PATCH_SMEM_BUDGET + 1024));
+    });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(conv_patch_kernel)");
     const long long total = (long long)p.n * p.ytiles * p.xtiles;
     if (total > 0x7fffffffll)
         return ESPDL_ERR_TOO_LARGE;
-    conv_patch_kernel<<<(int)min(total, (long long)num_sms()), CV_THREADS, smem, s>>>(ma, mb, mo, p);
+    const auto kernel = p.epi.half_even ? conv_patch_kernel<true> : conv_patch_kernel<false>;
+    kernel<<<(int)min(total, (long long)num_sms()), CV_THREADS, smem, s>>>(ma, mb, mo, p);
     count_launch();
     return check_launch("conv_patch");
 }
@@ -897,6 +906,7 @@ int conv2d_conv_tc(const espdl_conv_desc &d, cudaStream_t s)
     p.epi.e_shift_base = d.out_exponent - d.in_exponent;
     p.epi.ew_scalar = d.filter_exponent, p.epi.per_channel = d.per_channel;
     p.epi.relu = d.activation == ESPDL_ACT_RELU, p.epi.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
+    p.epi.acc_bound = min(d.in_c * d.kh * d.kw, 65536) << 14;
 
     CUtensorMap ma, mb, mo;
     {
@@ -935,14 +945,19 @@ int conv2d_conv_tc(const espdl_conv_desc &d, cudaStream_t s)
         smem = 120 * 1024; // one CTA per SM, so that TMEM allocation never waits on a neighbour
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] { attr_err = cudaFuncSetAttribute(conv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(CV_SMEM_BUDGET + 2048)); });
+    std::call_once(attr_once, [] {
+        attr_err = cudaFuncSetAttribute(conv_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(CV_SMEM_BUDGET + 2048));
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(conv_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(CV_SMEM_BUDGET + 2048));
+    });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(conv_tc_kernel)");
     const long long total = (long long)p.n * p.ytiles * p.xtiles * p.n_tiles;
     if (total > 0x7fffffffll)
         return ESPDL_ERR_TOO_LARGE;
     const int grid = (int)min(total, (long long)num_sms());
-    conv_tc_kernel<<<grid, CV_THREADS, smem, s>>>(ma, mb, mo, p);
+    const auto kernel = p.epi.half_even ? conv_tc_kernel<true> : conv_tc_kernel<false>;
+    kernel<<<grid, CV_THREADS, smem, s>>>(ma, mb, mo, p);
     count_launch();
     return check_launch("conv_tc");
 }

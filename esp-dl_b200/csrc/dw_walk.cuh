@@ -27,7 +27,7 @@ struct DwtSource {
     int C, e_shift_base, ew_scalar, per_channel, relu, half_even;
 };
 
-template <int S>
+template <int S, bool EVEN = false>
 __device__ __forceinline__ void dwt_load_consts(DwtConsts<S> &k, const DwtSource &p, int c0)
 {
 #pragma unroll
@@ -47,16 +47,14 @@ __device__ __forceinline__ void dwt_load_consts(DwtConsts<S> &k, const DwtSource
             k.wsel[kx][i] = S == 2 ? (f[2] & (0xffu << (8 * i))) : 0u;
         }
     }
-    k.fast = !p.half_even && !p.lut;
+    k.fast = EVEN == (bool)p.half_even && !p.lut;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int b = p.bias ? __ldg(p.bias + c0 + i) : 0;
         const int e = p.per_channel ? __ldg(p.ew + c0 + i) : p.ew_scalar;
-        const int s = max(-31, min(31, p.e_shift_base - e));
-        // (acc + bias + 2^(s-1)) >> s is exact while nothing can overflow: |acc| <= 9 * 2^14, |bias| < 2^30, 1 <= s <= 24
-        k.fast = k.fast && s >= 1 && s <= 24 && b < (1 << 30) && b > -(1 << 30);
-        k.shift[i] = s - (p.relu ? 1 : 0); // what the walk shifts by (see dwt_emit); the general form recomputes its own
-        k.init[i] = b + (s >= 1 ? (1 << (s - 1)) : 0);
+        int s;
+        k.fast = fast_constants(b, p.e_shift_base - e, 9 << 14, EVEN, k.init[i], s) && k.fast;
+        k.shift[i] = s - (p.relu && !EVEN ? 1 : 0); // what the walk shifts by (see dwt_emit); the general form recomputes its own
     }
 }
 
@@ -89,7 +87,7 @@ __device__ __forceinline__ void dwt_transpose(DwtCol<S> &col, const uint32_t (&r
 
 // One output column of a band (ROWS_OUT pixels x four channels) from three transposed input columns.
 // `st(ro, x, word)` stores the four channels of output row `ro` of the band at column `x` of the run.
-template <int S, typename Store>
+template <int S, bool EVEN, typename Store>
 __device__ __forceinline__ void dwt_emit(const DwtConsts<S> &k, const DwtCol<S> &k0, const DwtCol<S> &k1, const DwtCol<S> &k2, const Store &st, int x, int floor_q)
 {
     constexpr int ROWS_OUT = S == 1 ? 4 : 2;
@@ -112,7 +110,22 @@ __device__ __forceinline__ void dwt_emit(const DwtConsts<S> &k, const DwtCol<S> 
             }
         }
     }
-    if (floor_q == 0) {
+    if constexpr (EVEN) {
+        // half to even: w = acc + bias + 2^(s-1) - 1, quotient (w + bit s of w) >> s (derived beside shift_fast in the tile kernels)
+#pragma unroll
+        for (int ro = 0; ro < ROWS_OUT; ro++) {
+            int q[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int w = max(acc[ro][i], floor_q);
+                q[i] = (w + ((w >> k.shift[i]) & 1)) >> k.shift[i];
+            }
+            uint32_t hi, wd;
+            asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(q[3]), "r"(q[2]));
+            asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(wd) : "r"(q[1]), "r"(q[0]), "r"(hi));
+            st(ro, x, wd);
+        }
+    } else if (floor_q == 0) {
         // ReLU: the staged shifts are one less than the real ones; packing with saturation to [0, 255] clamps below at
         // zero, halving every byte completes the shift and turns the upper clamp into 127 - a shift and a mask per
         // word instead of a max per output
@@ -139,7 +152,7 @@ __device__ __forceinline__ void dwt_emit(const DwtConsts<S> &k, const DwtCol<S> 
 // The run of one thread: L output columns of its band, four channels.  `ip` points at the thread's word in the
 // patch's first row and column of the run; results go through `st` (see dwt_emit).  CB4 = channel-block width in words:
 // a template argument where the launch has one (column steps become immediate offsets), else `cb4`.
-template <int S, int CB4T, typename Store>
+template <int S, int CB4T, bool EVEN = false, typename Store>
 __device__ __forceinline__ void dwt_walk(const DwtConsts<S> &k, const uint32_t *ip, const Store &st, int in_row_words, int cb4, int L, int floor_q)
 {
     constexpr int ROWS_IN = S == 1 ? 6 : 5;
@@ -167,17 +180,17 @@ __device__ __forceinline__ void dwt_walk(const DwtConsts<S> &k, const uint32_t *
         for (int x = 0; x < L; x += 3) {
             dwt_transpose<S>(cc, raw);
             load_col(3);
-            dwt_emit<S>(k, ca, cb, cc, st, x, floor_q);
+            dwt_emit<S, EVEN>(k, ca, cb, cc, st, x, floor_q);
             if (x + 1 >= L)
                 break;
             dwt_transpose<S>(ca, raw);
             load_col(4);
-            dwt_emit<S>(k, cb, cc, ca, st, x + 1, floor_q);
+            dwt_emit<S, EVEN>(k, cb, cc, ca, st, x + 1, floor_q);
             if (x + 2 >= L)
                 break;
             dwt_transpose<S>(cb, raw);
             load_col(5);
-            dwt_emit<S>(k, cc, ca, cb, st, x + 2, floor_q);
+            dwt_emit<S, EVEN>(k, cc, ca, cb, st, x + 2, floor_q);
             advance(3);
         }
     } else {
@@ -189,14 +202,14 @@ __device__ __forceinline__ void dwt_walk(const DwtConsts<S> &k, const uint32_t *
             dwt_transpose<S>(cb, raw);
             load_col(2);
             dwt_transpose<S>(cc, raw);
-            dwt_emit<S>(k, ca, cb, cc, st, x, floor_q);
+            dwt_emit<S, EVEN>(k, ca, cb, cc, st, x, floor_q);
             if (x + 1 >= L)
                 break;
             load_col(3);
             dwt_transpose<S>(cb, raw);
             load_col(4);
             dwt_transpose<S>(ca, raw);
-            dwt_emit<S>(k, cc, cb, ca, st, x + 1, floor_q);
+            dwt_emit<S, EVEN>(k, cc, cb, ca, st, x + 1, floor_q);
             advance(4);
         }
     }

@@ -533,7 +533,7 @@ int fused_dwpw(const espdl_block_desc &d, cudaStream_t s)
     p.dw.e_shift_base = d.dw_exponent - d.in_exponent, p.dw.ew_scalar = d.dw_filter_exponent, p.dw.per_channel = (d.per_channel >> 1) & 1;
     p.dw.relu = d.dw_activation == ESPDL_ACT_RELU, p.dw.half_even = 0;
     p.e2 = EpiConfig{d.project_bias, d.project_filter_exponents, nullptr, d.out_exponent - d.dw_exponent, d.project_filter_exponent, (d.per_channel >> 2) & 1,
-                     d.project_activation == ESPDL_ACT_RELU, 0};
+                     d.project_activation == ESPDL_ACT_RELU, 0, min(d.hidden_c, 65536) << 14};
     p.res = (const int8_t *)d.residual, p.out = (int8_t *)d.output;
     p.ops = d.out_c, p.rps = d.out_c;
     CUtensorMap mi, mw;

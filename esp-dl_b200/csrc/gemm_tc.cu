@@ -104,6 +104,7 @@ constexpr int TILE_RING = 32; // tile numbers on their way from the producer to 
 // Epilogue of one int8 tile for outputs that cannot go through the staged path (piece widths that are not whole
 // 16-byte groups, unaligned rows, channels outside the fast form): rows are stored directly from registers.  Out of
 // line on purpose: the staged path in the kernel then carries none of this code's registers.
+template <bool EVEN>
 __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastParam *fast_s, uint32_t fp_base, uint32_t t0, long long m, int n0,
                                                   bool row_ok, bool fast, int parts, int part, bool allow_wide = true, uint32_t tbl = 0u)
 {
@@ -118,9 +119,9 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
         const uint32_t fp = fp_base + (uint32_t)n0 * 8u;
         const int ncols = min(p.block_n, p.N - n0);
         if (p.epi.relu)
-            epilogue_lean<true>(t0, fp, orow, ncols, parts, part, row_ok, wide);
+            epilogue_lean<true, EVEN>(t0, fp, orow, ncols, parts, part, row_ok, wide);
         else
-            epilogue_lean<false>(t0, fp, orow, ncols, parts, part, row_ok, wide);
+            epilogue_lean<false, EVEN>(t0, fp, orow, ncols, parts, part, row_ok, wide);
         return;
     }
     int chunk = 0;
@@ -137,13 +138,13 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
         uint32_t pk[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (fast) {
             if (p.epi.relu) {
-                requant16_fast<true>(v, fast_s + n0 + c0, pk);
+                requant16_fast<true, EVEN>(v, fast_s + n0 + c0, pk);
                 if (two)
-                    requant16_fast<true>(v + 16, fast_s + n0 + c0 + 16, pk + 4);
+                    requant16_fast<true, EVEN>(v + 16, fast_s + n0 + c0 + 16, pk + 4);
             } else {
-                requant16_fast<false>(v, fast_s + n0 + c0, pk);
+                requant16_fast<false, EVEN>(v, fast_s + n0 + c0, pk);
                 if (two)
-                    requant16_fast<false>(v + 16, fast_s + n0 + c0 + 16, pk + 4);
+                    requant16_fast<false, EVEN>(v + 16, fast_s + n0 + c0 + 16, pk + 4);
             }
             if (tbl) { // a fused table on rows that leave unstaged (`tbl`: its shared-memory copy): same lookups on the packed words
 #pragma unroll
@@ -183,7 +184,7 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
     }
 }
 
-template <bool I16>
+template <bool I16, bool EVEN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_a_lo, const __grid_constant__ CUtensorMap map_b_lo,
@@ -257,7 +258,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (p.epi.lut)
             stage_lut(p.epi.lut, lut_s, (int)threadIdx.x, NUM_THREADS);
         __syncthreads();
-        fast = !*slow_flag && !p.epi.half_even && !p.epi.lut_stride && p.K <= 32768; // one table rides on the staged form and on the packed words of unstaged rows; per-channel tables take the general path
+        fast = !*slow_flag && !p.epi.lut_stride && p.K <= 32768; // one table rides on the staged form and on the packed words of unstaged rows; per-channel tables take the general path
     }
     // This CTA is set up (everything above reads launch parameters and model constants only): the next kernel's CTAs may
     // take SMs as they become free.  The producer below waits for the previous kernel before its first load, and every
@@ -500,18 +501,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const uint32_t fpp = fp_base + (uint32_t)(n0 + col0) * 8u;
                     const int floor_q = p.epi.relu ? 0 : INT_MIN;
                     if (p.epi.lut) {
-                        epilogue_stage_lut(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
+                        epilogue_stage_lut<EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
                     } else if (p.res)
-                        epilogue_stage_residual(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q,
+                        epilogue_stage_residual<EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q,
                                                 p.res + m * p.rps + n0 + col0, row_ok, p.N - (n0 + col0));
                     else if (p.out_pw == 128)
-                        epilogue_stage<128>(t0 + col0, fpp, buf, row_in_tile, 128, floor_q);
+                        epilogue_stage<128, EVEN>(t0 + col0, fpp, buf, row_in_tile, 128, floor_q);
                     else if (p.out_pw == 96)
-                        epilogue_stage<96>(t0 + col0, fpp, buf, row_in_tile, 96, floor_q);
+                        epilogue_stage<96, EVEN>(t0 + col0, fpp, buf, row_in_tile, 96, floor_q);
                     else if (p.out_pw == 64)
-                        epilogue_stage<64>(t0 + col0, fpp, buf, row_in_tile, 64, floor_q);
+                        epilogue_stage<64, EVEN>(t0 + col0, fpp, buf, row_in_tile, 64, floor_q);
                     else
-                        epilogue_stage<0>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, floor_q);
+                        epilogue_stage<0, EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, floor_q);
                     // the accumulator is free as soon as this warp's TMEM loads are done: hand it back before the
                     // shared-memory tile is completed and stored, so that the MMAs of the tile after next start earlier
                     fence_before();
@@ -526,7 +527,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                     continue;
                 }
-                epilogue_direct_tile(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, true, p.epi.lut ? smem_u32(lut_s) : 0u);
+                epilogue_direct_tile<EVEN>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, true, p.epi.lut ? smem_u32(lut_s) : 0u);
             } else {
                 int chunk = 0;
                 for (int c0 = 0; c0 < p.block_n; c0 += 16, chunk++) {
@@ -801,7 +802,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const long long m = (long long)m0 + row_in_tile;
             const uint32_t t0 = tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)(acc * p.block_n);
             // 128-bit stores: in this kernel the 256-bit form stored only the first word of each 32 bytes
-            epilogue_direct_tile(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, false);
+            epilogue_direct_tile<false>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, false);
             fence_before();
             __syncwarp();
             if (lane == 0)
@@ -1067,6 +1068,7 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
     p.epi.e_shift_base = d.out_exponent - d.in_exponent;
     p.epi.ew_scalar = d.filter_exponent, p.epi.per_channel = d.per_channel;
     p.epi.relu = d.activation == ESPDL_ACT_RELU, p.epi.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
+    p.epi.acc_bound = min(p.K, 65536) << 14;
     {
         TcParams pp = p;
         if (!i16 && n_peer == 0 && ips % 16 == 0 && pair_plan(d, pp))
@@ -1125,16 +1127,18 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
+        attr_err = cudaFuncSetAttribute(gemm_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
         if (attr_err == cudaSuccess)
-            attr_err = cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
+            attr_err = cudaFuncSetAttribute(gemm_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(gemm_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
     });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(gemm_tc_kernel)");
     if (i16)
-        gemm_tc_kernel<true><<<grid, NUM_THREADS, smem, s>>>(ma, mb, ma_lo, mb_lo, mo, p);
+        gemm_tc_kernel<true, false><<<grid, NUM_THREADS, smem, s>>>(ma, mb, ma_lo, mb_lo, mo, p);
     else
-        launch_overlapped(gemm_tc_kernel<false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
+        launch_overlapped(p.epi.half_even ? gemm_tc_kernel<false, true> : gemm_tc_kernel<false, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
     count_launch();
     return check_launch("gemm_tc");
 }

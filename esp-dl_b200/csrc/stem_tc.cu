@@ -62,6 +62,7 @@ struct StemParams {
     EpiConfig epi;
 };
 
+template <bool EVEN>
 __global__ void __launch_bounds__(ST_THREADS, 1)
 stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, const __grid_constant__ CUtensorMap map2,
                const __grid_constant__ CUtensorMap map_out, const StemParams p)
@@ -215,18 +216,18 @@ stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                     if (p.epi.bias)
                         b = ((const int32_t *)p.epi.bias)[c];
                     sh = p.epi.e_shift_base - (p.epi.per_channel ? p.epi.ew[c] : p.epi.ew_scalar);
-                    if (sh < 1 || sh > 24 || b >= (1 << 30) || b <= -(1 << 30))
-                        bad = 1;
-                    sh = max(1, min(24, sh));
                 }
-                fast_s[col].bias_half = b + (1 << (sh - 1));
-                fast_s[col].shift = sh;
+                int bh, fs;
+                if (!fast_constants(b, sh, p.epi.acc_bound, EVEN, bh, fs))
+                    bad = 1;
+                fast_s[col].bias_half = bh;
+                fast_s[col].shift = fs;
             }
             if (bad)
                 atomicOr(slow_flag, 1);
         }
         asm volatile("bar.sync 1, %0;" ::"n"(16 * 32) : "memory");
-        const bool fast = !*slow_flag && !p.epi.half_even && !p.epi.lut_stride; // one fused table rides on the staged form, per-channel tables take the general path
+        const bool fast = !*slow_flag && !p.epi.lut_stride; // one fused table rides on the staged form, per-channel tables take the general path
         const uint32_t fp = epi_param_base(fast_s);
         uint32_t acc_phase = 0;
         bool ok = true;
@@ -260,11 +261,11 @@ stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 const int col0 = part * out_pw;
                 const int floor_q = p.epi.relu ? 0 : INT_MIN;
                 if (p.epi.lut)
-                    epilogue_stage_lut(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, out_pw, out_pw == 128 ? 7u : 3u, floor_q, smem_u32(lut_s));
+                    epilogue_stage_lut<EVEN>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, out_pw, out_pw == 128 ? 7u : 3u, floor_q, smem_u32(lut_s));
                 else if (out_pw == 128)
-                    epilogue_stage<128>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 128, floor_q);
+                    epilogue_stage<128, EVEN>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 128, floor_q);
                 else
-                    epilogue_stage<64>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 64, floor_q);
+                    epilogue_stage<64, EVEN>(t0 + col0, fp + (uint32_t)col0 * 8u, buf, row_in_tile, 64, floor_q);
                 fence_before();
                 fence_async_smem();
                 named_bar(2 + group, 128);
@@ -373,6 +374,7 @@ int conv2d_stem_tc(const espdl_conv_desc &d, cudaStream_t s)
     p.epi.e_shift_base = d.out_exponent - d.in_exponent;
     p.epi.ew_scalar = d.filter_exponent, p.epi.per_channel = d.per_channel;
     p.epi.relu = d.activation == ESPDL_ACT_RELU, p.epi.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
+    p.epi.acc_bound = 27 << 14;
 
     // One map per filter row ky: input rows 2*y + ky - pad_top = 2*(y + q) + r, so the map starts at row r, steps
     // two rows per index and is addressed with y + q; indices outside [0, rows of that parity) read zeros.
@@ -409,12 +411,17 @@ int conv2d_stem_tc(const espdl_conv_desc &d, cudaStream_t s)
         (2 * ST_STAGES + 2 * ST_ACC) * 8 + 32 + 256 + 16;
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] { attr_err = cudaFuncSetAttribute(stem_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024); });
+    std::call_once(attr_once, [] {
+        attr_err = cudaFuncSetAttribute(stem_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(stem_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+    });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(stem_tc_kernel)");
     const int total = p.ngroups * p.yblocks * p.segs;
     const int grid = min(total, num_sms());
-    stem_tc_kernel<<<grid, ST_THREADS, max(smem, (size_t)120 * 1024), s>>>(maps[0], maps[1], maps[2], mo, p);
+    const auto kernel = p.epi.half_even ? stem_tc_kernel<true> : stem_tc_kernel<false>;
+    kernel<<<grid, ST_THREADS, max(smem, (size_t)120 * 1024), s>>>(maps[0], maps[1], maps[2], mo, p);
     count_launch();
     return check_launch("stem_tc");
 }

@@ -230,19 +230,30 @@ __device__ __forceinline__ uint32_t idesc_i8(int a_signed, int b_signed, int m, 
 }
 
 // ------------------------------------------------------------------------------------------ epilogue
-// Per-output-channel constants of the fast form, staged in shared memory: q = (acc + bias_half) >> shift with
-// bias_half = bias + 2^(shift-1).  Equal to the reference's wrapping 32-bit bias add followed by a 64-bit
-// round-half-up shift whenever nothing can overflow 32 bits: |acc| < 2^29, |bias| < 2^30, 1 <= shift <= 24.
+// Per-output-channel constants of the fast form, staged in shared memory: q = (acc + bias_half) >> shift (fast_constants
+// in common.cuh says when this equals the reference's arithmetic).
 struct FastParam {
     int bias_half;
     int shift;
 };
+
+// Round half to even in the same form, two more integer instructions and an add: with bias_half one smaller,
+// w = acc + bias + 2^(s-1) - 1, the quotient is (w + bit s of w) >> s.  Write acc + bias = q * 2^s + r: for r <= 2^(s-1) bit s of w is
+// the parity of q and only r = 2^(s-1) with q odd carries into bit s; for r > 2^(s-1) w >> s is already q + 1 and the
+// remainder left in w is too small for a carry.  EVEN is a template parameter of the kernels, so that half-up models
+// pay nothing for it.
+template <bool EVEN>
+__device__ __forceinline__ int shift_fast(int w, int s)
+{
+    return EVEN ? (w + ((w >> s) & 1)) >> s : w >> s;
+}
 
 struct EpiConfig {
     const void *bias;   // int32[N] (int8 op) / int64[N] (int16 op) or null
     const int32_t *ew;  // per-channel filter exponents or null
     const int8_t *lut;  // optional fused 256-entry table
     int e_shift_base, ew_scalar, per_channel, relu, half_even;
+    int acc_bound;      // bound of |acc|: 2^14 per term of an int8 sum
     int lut_stride;     // 0: one table; else entries between the tables of consecutive channels (general epilogue only)
 };
 
@@ -258,19 +269,19 @@ __device__ __forceinline__ void stage_fast_params(const EpiConfig &c, FastParam 
                 b = ((const int32_t *)c.bias)[n];
             const int e = c.per_channel ? c.ew[n] : c.ew_scalar;
             sh = c.e_shift_base - e;
-            if (sh < 1 || sh > 24 || b >= (1 << 30) || b <= -(1 << 30))
-                bad = 1;
-            sh = max(1, min(24, sh));
         }
-        fast[n].bias_half = b + (1 << (sh - 1));
-        fast[n].shift = sh;
+        int bh, fs;
+        if (!fast_constants(b, sh, c.acc_bound, c.half_even, bh, fs))
+            bad = 1;
+        fast[n].bias_half = bh;
+        fast[n].shift = fs;
     }
     if (bad)
         atomicOr(slow, 1);
 }
 
 // Requantises 16 accumulator columns with the fast form and packs them to 16 int8 (4 words).
-template <bool RELU>
+template <bool RELU, bool EVEN = false>
 __device__ __forceinline__ void requant16_fast(const int32_t *v, const FastParam *fp, uint32_t *pk)
 {
 #pragma unroll
@@ -278,10 +289,10 @@ __device__ __forceinline__ void requant16_fast(const int32_t *v, const FastParam
         // two channels per 128-bit shared-memory load
         const int4 p01 = *(const int4 *)(fp + q * 4);
         const int4 p23 = *(const int4 *)(fp + q * 4 + 2);
-        const int r0 = (v[q * 4 + 0] + p01.x) >> p01.y;
-        const int r1 = (v[q * 4 + 1] + p01.z) >> p01.w;
-        const int r2 = (v[q * 4 + 2] + p23.x) >> p23.y;
-        const int r3 = (v[q * 4 + 3] + p23.z) >> p23.w;
+        const int r0 = shift_fast<EVEN>(v[q * 4 + 0] + p01.x, p01.y);
+        const int r1 = shift_fast<EVEN>(v[q * 4 + 1] + p01.z, p01.w);
+        const int r2 = shift_fast<EVEN>(v[q * 4 + 2] + p23.x, p23.y);
+        const int r3 = shift_fast<EVEN>(v[q * 4 + 3] + p23.z, p23.w);
         uint32_t hi, w;
         if (RELU) {
             // ReLU + saturation: clamp to [0, 255] while packing, then a per-byte minimum with 127
@@ -300,7 +311,7 @@ __device__ __forceinline__ void requant16_fast(const int32_t *v, const FastParam
 // (address `fp`, 8 bytes per column) with two 128-bit loads.  With ReLU the add and the lower clamp are one
 // instruction (max(acc + bias_half, 0)), which commutes with the arithmetic shift; the pack saturates the top.
 // (Volatile loads: letting the compiler hoist them ahead of the TMEM wait cost registers and measured slower.)
-template <bool RELU>
+template <bool RELU, bool EVEN>
 __device__ __forceinline__ uint32_t requant4_lean(const int32_t *v, uint32_t fp)
 {
     int b0, s0, b1, s1, b2, s2, b3, s3;
@@ -308,15 +319,15 @@ __device__ __forceinline__ uint32_t requant4_lean(const int32_t *v, uint32_t fp)
     asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(b2), "=r"(s2), "=r"(b3), "=r"(s3) : "r"(fp + 16));
     int r0, r1, r2, r3;
     if (RELU) {
-        r0 = __viaddmax_s32(v[0], b0, 0) >> s0;
-        r1 = __viaddmax_s32(v[1], b1, 0) >> s1;
-        r2 = __viaddmax_s32(v[2], b2, 0) >> s2;
-        r3 = __viaddmax_s32(v[3], b3, 0) >> s3;
+        r0 = shift_fast<EVEN>(__viaddmax_s32(v[0], b0, 0), s0);
+        r1 = shift_fast<EVEN>(__viaddmax_s32(v[1], b1, 0), s1);
+        r2 = shift_fast<EVEN>(__viaddmax_s32(v[2], b2, 0), s2);
+        r3 = shift_fast<EVEN>(__viaddmax_s32(v[3], b3, 0), s3);
     } else {
-        r0 = (v[0] + b0) >> s0;
-        r1 = (v[1] + b1) >> s1;
-        r2 = (v[2] + b2) >> s2;
-        r3 = (v[3] + b3) >> s3;
+        r0 = shift_fast<EVEN>(v[0] + b0, s0);
+        r1 = shift_fast<EVEN>(v[1] + b1, s1);
+        r2 = shift_fast<EVEN>(v[2] + b2, s2);
+        r3 = shift_fast<EVEN>(v[3] + b3, s3);
     }
     uint32_t hi, w;
     asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(r3), "r"(r2));
@@ -333,18 +344,18 @@ __device__ __forceinline__ uint32_t epi_param_base(const FastParam *fast)
     return a;
 }
 
-template <bool RELU>
+template <bool RELU, bool EVEN>
 __device__ __forceinline__ void requant16_lean(const int32_t *v, uint32_t fp, uint32_t *pk)
 {
 #pragma unroll
-    for (int q = 0; q < 4; q++) pk[q] = requant4_lean<RELU>(v + 4 * q, fp + (uint32_t)(4 * q) * 8u);
+    for (int q = 0; q < 4; q++) pk[q] = requant4_lean<RELU, EVEN>(v + 4 * q, fp + (uint32_t)(4 * q) * 8u);
 }
 
 // One accumulator row (this thread's TMEM lane), columns [0, ncols) of a tile, ncols % 16 == 0, every `parts`-th
 // 32-column chunk starting with chunk `part`: requantise with the fast form and store.  `orow` is 16-byte
 // aligned; `wide` says it is 32-byte aligned as well (256-bit stores).  TMEM is read 16 columns at a time into
 // two register sets in turn: while one half chunk is requantised the load of the next is in flight.
-template <bool RELU>
+template <bool RELU, bool EVEN>
 __device__ __forceinline__ void epilogue_lean(uint32_t t0, uint32_t fp, int8_t *orow, int ncols, int parts, int part, bool row_ok, bool wide)
 {
     const int step = parts * 32;
@@ -357,13 +368,13 @@ __device__ __forceinline__ void epilogue_lean(uint32_t t0, uint32_t fp, int8_t *
         uint32_t pk[8];
         ld_wait16(va);
         ld16(t0 + c0 + 16, vb);
-        requant16_lean<RELU>(va, fp + (uint32_t)c0 * 8u, pk);
+        requant16_lean<RELU, EVEN>(va, fp + (uint32_t)c0 * 8u, pk);
         ld_wait16(vb);
         const int c1 = c0 + step;
         have = c1 + 32 <= ncols;
         if (have)
             ld16(t0 + c1, va);
-        requant16_lean<RELU>(vb, fp + (uint32_t)(c0 + 16) * 8u, pk + 4);
+        requant16_lean<RELU, EVEN>(vb, fp + (uint32_t)(c0 + 16) * 8u, pk + 4);
         if (row_ok) {
             if (wide) {
                 asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(orow + c0), "r"(pk[0]), "r"(pk[1]),
@@ -383,7 +394,7 @@ __device__ __forceinline__ void epilogue_lean(uint32_t t0, uint32_t fp, int8_t *
         ld_wait16(v);
         uint32_t pk[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) pk[q] = requant4_lean<RELU>(v + 4 * q, fp + (uint32_t)(ch + 4 * q) * 8u);
+        for (int q = 0; q < 4; q++) pk[q] = requant4_lean<RELU, EVEN>(v + 4 * q, fp + (uint32_t)(ch + 4 * q) * 8u);
         if (row_ok)
             *(uint4 *)(orow + ch) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
@@ -391,15 +402,16 @@ __device__ __forceinline__ void epilogue_lean(uint32_t t0, uint32_t fp, int8_t *
 
 // Four accumulator columns -> one word of four saturated int8; `floor_q` is 0 with ReLU and INT_MIN without, so
 // the add and the lower clamp are one instruction either way (max commutes with the arithmetic shift).
+template <bool EVEN = false>
 __device__ __forceinline__ uint32_t requant4_floor(const int32_t *v, uint32_t fp, int floor_q)
 {
     int b0, s0, b1, s1, b2, s2, b3, s3;
     asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(b0), "=r"(s0), "=r"(b1), "=r"(s1) : "r"(fp));
     asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(b2), "=r"(s2), "=r"(b3), "=r"(s3) : "r"(fp + 16));
-    const int r0 = __viaddmax_s32(v[0], b0, floor_q) >> s0;
-    const int r1 = __viaddmax_s32(v[1], b1, floor_q) >> s1;
-    const int r2 = __viaddmax_s32(v[2], b2, floor_q) >> s2;
-    const int r3 = __viaddmax_s32(v[3], b3, floor_q) >> s3;
+    const int r0 = shift_fast<EVEN>(__viaddmax_s32(v[0], b0, floor_q), s0);
+    const int r1 = shift_fast<EVEN>(__viaddmax_s32(v[1], b1, floor_q), s1);
+    const int r2 = shift_fast<EVEN>(__viaddmax_s32(v[2], b2, floor_q), s2);
+    const int r3 = shift_fast<EVEN>(__viaddmax_s32(v[3], b3, floor_q), s3);
     uint32_t hi, w;
     asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(r3), "r"(r2));
     asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(r1), "r"(r0), "r"(hi));
@@ -434,7 +446,7 @@ __device__ __forceinline__ uint32_t lut4(uint32_t w, uint32_t tbl)
 // other widths): 16-byte chunk index XOR bits 7.. of the byte offset, which for these widths is a function of the
 // row alone.  PW is a template parameter so that the walk over the columns is straight-line code; PW = 0 is the
 // generic form for any width (`pw`).  TMEM is read 16 columns at a time into two register sets in turn.
-template <int PW>
+template <int PW, bool EVEN>
 __device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_t buf, int row, int pw, int floor_q)
 {
     const int width = PW ? PW : pw;
@@ -458,7 +470,7 @@ __device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_
         if (second)
             ld16(t0 + c + 16, vb);
 #pragma unroll
-        for (int q = 0; q < 4; q++) pk[q] = requant4_floor(va + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q);
+        for (int q = 0; q < 4; q++) pk[q] = requant4_floor<EVEN>(va + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)c ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
                      : "memory");
         if (!second)
@@ -468,7 +480,7 @@ __device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_
         if (more)
             ld16(t0 + c + 32, va);
 #pragma unroll
-        for (int q = 0; q < 4; q++) pk[q] = requant4_floor(vb + 4 * q, fp + (uint32_t)(c + 16 + 4 * q) * 8u, floor_q);
+        for (int q = 0; q < 4; q++) pk[q] = requant4_floor<EVEN>(vb + 4 * q, fp + (uint32_t)(c + 16 + 4 * q) * 8u, floor_q);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)(c + 16) ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]),
                      "r"(pk[3])
                      : "memory");
@@ -478,6 +490,7 @@ __device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_
 // Staged epilogue with a fused table: as epilogue_stage, any piece width (a multiple of 16, at most 128; `mask` = 7 / 3 / 0
 // is the swizzle of 128- / 64-byte / other rows), every packed word goes through lut4 before it is stored.  A compact
 // loop kept out of line: the kernels that call it carry none of its registers in their other epilogues.
+template <bool EVEN>
 static __device__ __noinline__ void epilogue_stage_lut(uint32_t t0, uint32_t fp, uint32_t buf, int row, int pw, uint32_t mask, int floor_q, uint32_t tbl)
 {
     const uint32_t rx = ((((uint32_t)(row * pw)) >> 7) & mask) << 4;
@@ -489,7 +502,7 @@ static __device__ __noinline__ void epilogue_stage_lut(uint32_t t0, uint32_t fp,
         ld16(t0 + c, v);
         ld_wait16(v);
 #pragma unroll
-        for (int q = 0; q < 4; q++) pk[q] = lut4(requant4_floor(v + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q), tbl);
+        for (int q = 0; q < 4; q++) pk[q] = lut4(requant4_floor<EVEN>(v + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q), tbl);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)c ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
                      : "memory");
     }
@@ -498,6 +511,7 @@ static __device__ __noinline__ void epilogue_stage_lut(uint32_t t0, uint32_t fp,
 // Staged epilogue with a folded Add: as epilogue_stage<0>, and every requantised value is first clamped to int8, then
 // summed with the residual byte of the same row and column and saturated again (out = sat(sat(q) + r)).  `res` is
 // this thread's residual row at the piece's first column (16-byte aligned); `valid` = columns of the piece inside N.
+template <bool EVEN>
 __device__ __forceinline__ void epilogue_stage_residual(uint32_t t0, uint32_t fp, uint32_t buf, int row, int pw, uint32_t mask, int floor_q,
                                                         const int8_t *res, bool row_ok, int valid)
 {
@@ -523,7 +537,7 @@ __device__ __forceinline__ void epilogue_stage_residual(uint32_t t0, uint32_t fp
             int t[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int qv = min(max(__viaddmax_s32(v[4 * q + i], b[i], floor_q) >> s[i], -128), 127);
+                const int qv = min(max(shift_fast<EVEN>(__viaddmax_s32(v[4 * q + i], b[i], floor_q), s[i]), -128), 127);
                 t[i] = qv + (int)(int8_t)(rw[q] >> (8 * i));
             }
             uint32_t hi;
