@@ -14,6 +14,7 @@ static thread_local char g_last_error[512] = "";
 static std::atomic<uint64_t> g_launches{0};
 static int g_device = -1;
 static int g_num_sms = 0;
+static int *g_error_word = nullptr; // pinned, mapped: written by device-side waits that ran out
 static std::mutex g_ws_mutex;
 static void *g_ws = nullptr; // cached scratch of espdl_b200_conv2d (int16 limb planes)
 static size_t g_ws_bytes = 0;
@@ -105,12 +106,26 @@ int espdl_b200_init(int device)
         return set_error_text(ESPDL_ERR_INVALID_ARG, "espdl_b200_init(%d): this process is bound to device %d; call espdl_b200_shutdown first",
                               device, g_device);
     ESPDL_CUDA_TRY(cudaSetDevice(device));
+    if (g_device == device)
+        return ESPDL_OK; // done before: the properties of a device take milliseconds to ask for
     cudaDeviceProp prop;
     ESPDL_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
     if (prop.major != 10) {
         snprintf(g_last_error, sizeof(g_last_error), "device %d is sm_%d%d; this library holds sm_100a code only", device,
                  prop.major, prop.minor);
         return ESPDL_ERR_NO_DEVICE;
+    }
+    if (!g_error_word) {
+        ESPDL_CUDA_TRY(cudaHostAlloc((void **)&g_error_word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        *g_error_word = 0;
+    }
+    int *word = nullptr; // the word as the device addresses it
+    ESPDL_CUDA_TRY(cudaHostGetDevicePointer((void **)&word, g_error_word, 0));
+    for (int (*bind)(int *) : {bind_device_error, bind_device_error_stem, bind_device_error_band, bind_device_error_dw, bind_device_error_conv,
+                               bind_device_error_block, bind_device_error_dwpw}) {
+        const int st = bind(word);
+        if (st)
+            return st;
     }
     g_device = device;
     g_num_sms = prop.multiProcessorCount;
@@ -214,16 +229,8 @@ int espdl_b200_memset(void *dst_dev, int value, size_t bytes, void *stream)
 int espdl_b200_stream_sync(void *stream)
 {
     ESPDL_CUDA_TRY(cudaStreamSynchronize((cudaStream_t)stream));
-    // a tile kernel whose bounded wait expired leaves its status in a device word
-    int dev = read_and_clear_device_error();
-    const int dev_stem = read_and_clear_device_error_stem();
-    const int dev_dw = read_and_clear_device_error_dw();
-    const int dev_conv = read_and_clear_device_error_conv();
-    const int dev_block = read_and_clear_device_error_block();
-    const int dev_dwpw = read_and_clear_device_error_dwpw();
-    const int dev_band = read_and_clear_device_error_band();
-    if (!dev)
-        dev = dev_stem ? dev_stem : (dev_conv ? dev_conv : (dev_block ? dev_block : (dev_dw ? dev_dw : (dev_dwpw ? dev_dwpw : dev_band))));
+    // a tile kernel whose bounded wait expired left its status in the mapped word
+    const int dev = g_error_word && *(volatile int *)g_error_word ? __atomic_exchange_n(g_error_word, 0, __ATOMIC_SEQ_CST) : 0;
     if (dev) {
         snprintf(g_last_error, sizeof(g_last_error), "a device-side bounded wait expired in the tensor-core tile kernel");
         return dev;

@@ -26,18 +26,12 @@
 
 namespace espdl {
 
-__device__ int g_block_tc_error = 0;
+__device__ int *g_block_tc_error = nullptr; // the status word of bounded waits (common.cuh)
 
-int read_and_clear_device_error_block()
+int bind_device_error_block(int *word)
 {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_block_tc_error, sizeof(int)) != cudaSuccess)
-        return 0;
-    if (v) {
-        int zero = 0;
-        cudaMemcpyToSymbol(g_block_tc_error, &zero, sizeof(int));
-    }
-    return v;
+    ESPDL_CUDA_TRY(cudaMemcpyToSymbol(g_block_tc_error, &word, sizeof(word)));
+    return ESPDL_OK;
 }
 
 namespace {
@@ -423,7 +417,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
             }
             if (!ok)
-                atomicExch(&g_block_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_block_tc_error);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -461,7 +455,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
             }
             if (!ok)
-                atomicExch(&g_block_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_block_tc_error);
         }
         __syncwarp();
     } else if (warp == 2) {
@@ -494,7 +488,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
             }
             if (!ok)
-                atomicExch(&g_block_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_block_tc_error);
         }
         __syncwarp();
     } else if (warp < BK_CTRL_WARPS + BK_E_WARPS) {
@@ -676,7 +670,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         if (ok && pending_tile >= 0)
             ok = epilogue2(pending_tile, lt - 1);
         if (!ok && lane == 0)
-            atomicExch(&g_block_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_block_tc_error);
     } else {
         // ------------------------------------------------------------------ depthwise warps
         const int d = warp - BK_CTRL_WARPS - BK_E_WARPS;
@@ -722,7 +716,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             }
         }
         if (!ok && lane == 0)
-            atomicExch(&g_block_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_block_tc_error);
     }
 #undef BAR
 

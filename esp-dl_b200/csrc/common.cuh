@@ -46,6 +46,12 @@ cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // This CTA no longer minds the next kernel's CTAs becoming resident.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A bounded wait ran out: `word` is host memory.
+__device__ __forceinline__ void report_timeout(int *word)
+{
+    if (word)
+        atomicExch_system(word, ESPDL_ERR_TIMEOUT);
+}
 #endif
 
 #define ESPDL_CUDA_TRY(call)                                \
@@ -65,13 +71,16 @@ bool conv2d_tc_supported(const espdl_conv_desc &d);
 size_t conv2d_tc_workspace_bytes(const espdl_conv_desc &d);
 int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s, const long long *peer_delta = nullptr,
               int n_peer = 0); // peer_delta: byte distances to copies of the output on other GPUs that receive every row as well
-int read_and_clear_device_error(); // status word written by device-side bounded waits (0 = none)
-int read_and_clear_device_error_stem();
-int read_and_clear_device_error_band();
-int read_and_clear_device_error_dw();
-int read_and_clear_device_error_conv();
-int read_and_clear_device_error_block();
-int read_and_clear_device_error_dwpw();
+// Each translation unit with bounded device-side waits keeps the address of ONE status word in pinned, device-mapped host
+// memory: a wait that runs out stores ESPDL_ERR_TIMEOUT there, and espdl_b200_stream_sync reads it as ordinary memory.
+// (A device word per unit, copied back at every synchronisation, cost seven blocking copies: 60 us of a 160 us pass.)
+int bind_device_error(int *word);
+int bind_device_error_stem(int *word);
+int bind_device_error_band(int *word);
+int bind_device_error_dw(int *word);
+int bind_device_error_conv(int *word);
+int bind_device_error_block(int *word);
+int bind_device_error_dwpw(int *word);
 int image_preprocess(const espdl_image_desc &d, cudaStream_t s);
 int detect_candidates(const espdl_detect_desc &d, cudaStream_t s);
 int reduce_op(const espdl_reduce_desc &d, cudaStream_t s);

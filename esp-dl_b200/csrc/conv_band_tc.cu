@@ -26,18 +26,12 @@
 
 namespace espdl {
 
-__device__ int g_band_tc_error = 0;
+__device__ int *g_band_tc_error = nullptr; // the status word of bounded waits (common.cuh)
 
-int read_and_clear_device_error_band()
+int bind_device_error_band(int *word)
 {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_band_tc_error, sizeof(int)) != cudaSuccess)
-        return 0;
-    if (v) {
-        int zero = 0;
-        cudaMemcpyToSymbol(g_band_tc_error, &zero, sizeof(int));
-    }
-    return v;
+    ESPDL_CUDA_TRY(cudaMemcpyToSymbol(g_band_tc_error, &word, sizeof(word)));
+    return ESPDL_OK;
 }
 
 namespace {
@@ -158,7 +152,7 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 }
             }
             if (!ok)
-                atomicExch(&g_band_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_band_tc_error);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -198,7 +192,7 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 }
             }
             if (!ok)
-                atomicExch(&g_band_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_band_tc_error);
         }
         __syncwarp();
     } else {
@@ -314,7 +308,7 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 mbar_arrive(smem_u32(&tempty_bar[acc]));
         }
         if (!ok && lane == 0)
-            atomicExch(&g_band_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_band_tc_error);
         if ((ew & 3) == 0 && lane == 0)
             bulk_wait_all(); // shared memory stays allocated until the last store has left it
     }

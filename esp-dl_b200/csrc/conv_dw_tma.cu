@@ -28,18 +28,12 @@
 
 namespace espdl {
 
-__device__ int g_dwt_error = 0;
+__device__ int *g_dwt_error = nullptr; // the status word of bounded waits (common.cuh)
 
-int read_and_clear_device_error_dw()
+int bind_device_error_dw(int *word)
 {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_dwt_error, sizeof(int)) != cudaSuccess)
-        return 0;
-    if (v) {
-        int zero = 0;
-        cudaMemcpyToSymbol(g_dwt_error, &zero, sizeof(int));
-    }
-    return v;
+    ESPDL_CUDA_TRY(cudaMemcpyToSymbol(g_dwt_error, &word, sizeof(word)));
+    return ESPDL_OK;
 }
 
 namespace {
@@ -157,7 +151,7 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, p.wait_limit)) {
                 *abort_flag = 1;
                 if (lane == 0)
-                    atomicExch(&g_dwt_error, ESPDL_ERR_TIMEOUT);
+                    report_timeout(g_dwt_error);
                 ok = false;
                 break;
             }
@@ -220,7 +214,7 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             // the patch never came: note it and leave at the barrier below, where all threads see the flag together
             *abort_flag = 1;
             if (lane == 0)
-                atomicExch(&g_dwt_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_dwt_error);
         }
         const int t = *abort_flag ? 0 : tile_ring[local & (DWT_RING - 1)];
         if (t < 0)

@@ -21,18 +21,12 @@
 
 namespace espdl {
 
-__device__ int g_conv_tc_error = 0;
+__device__ int *g_conv_tc_error = nullptr; // the status word of bounded waits (common.cuh)
 
-int read_and_clear_device_error_conv()
+int bind_device_error_conv(int *word)
 {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_conv_tc_error, sizeof(int)) != cudaSuccess)
-        return 0;
-    if (v) {
-        int zero = 0;
-        cudaMemcpyToSymbol(g_conv_tc_error, &zero, sizeof(int));
-    }
-    return v;
+    ESPDL_CUDA_TRY(cudaMemcpyToSymbol(g_conv_tc_error, &word, sizeof(word)));
+    return ESPDL_OK;
 }
 
 namespace {
@@ -145,7 +139,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
             }
             if (!ok)
-                atomicExch(&g_conv_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_conv_tc_error);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -189,7 +183,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
             }
             if (!ok)
-                atomicExch(&g_conv_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_conv_tc_error);
         }
         __syncwarp();
     } else {
@@ -294,7 +288,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 mbar_arrive(smem_u32(&tempty_bar[acc]));
         }
         if (!ok && lane == 0)
-            atomicExch(&g_conv_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_conv_tc_error);
         if (p.out_pw && (ew & 3) == 0 && lane == 0)
             bulk_wait_all();
     }
@@ -477,7 +471,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
             }
             if (!ok)
-                atomicExch(&g_conv_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_conv_tc_error);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -519,7 +513,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
             }
             if (!ok)
-                atomicExch(&g_conv_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_conv_tc_error);
         }
         __syncwarp();
     } else {
@@ -634,7 +628,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
         if (!ok && lane == 0)
-            atomicExch(&g_conv_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_conv_tc_error);
         if ((ew & 3) == 0 && lane == 0)
             bulk_wait_all();
     }

@@ -33,18 +33,12 @@
 
 namespace espdl {
 
-__device__ int g_dwpw_error = 0;
+__device__ int *g_dwpw_error = nullptr; // the status word of bounded waits (common.cuh)
 
-int read_and_clear_device_error_dwpw()
+int bind_device_error_dwpw(int *word)
 {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_dwpw_error, sizeof(int)) != cudaSuccess)
-        return 0;
-    if (v) {
-        int zero = 0;
-        cudaMemcpyToSymbol(g_dwpw_error, &zero, sizeof(int));
-    }
-    return v;
+    ESPDL_CUDA_TRY(cudaMemcpyToSymbol(g_dwpw_error, &word, sizeof(word)));
+    return ESPDL_OK;
 }
 
 namespace {
@@ -157,7 +151,7 @@ dwpw_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ 
             }
             if (!ok) {
                 *abort_flag = 1;
-                atomicExch(&g_dwpw_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_dwpw_error);
             }
         }
         __syncwarp();
@@ -200,7 +194,7 @@ dwpw_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ 
             }
             if (!ok) {
                 *abort_flag = 1;
-                atomicExch(&g_dwpw_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_dwpw_error);
             }
         }
         __syncwarp();
@@ -265,7 +259,7 @@ dwpw_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ 
         }
         if (!ok && lane == 0) {
             *abort_flag = 1;
-            atomicExch(&g_dwpw_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_dwpw_error);
         }
     } else {
         // ------------------------------------------------------------ depthwise warps
@@ -297,7 +291,7 @@ dwpw_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ 
                     dead = true;
                     *abort_flag = 1;
                     if (lane == 0)
-                        atomicExch(&g_dwpw_error, ESPDL_ERR_TIMEOUT);
+                        report_timeout(g_dwpw_error);
                 }
                 if (!dead && *abort_flag)
                     dead = true;

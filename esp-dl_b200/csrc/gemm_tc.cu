@@ -35,18 +35,12 @@
 
 namespace espdl {
 
-__device__ int g_tc_error = 0;
+__device__ int *g_tc_error = nullptr; // the status word of bounded waits (common.cuh)
 
-int read_and_clear_device_error()
+int bind_device_error(int *word)
 {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_tc_error, sizeof(int)) != cudaSuccess)
-        return 0;
-    if (v) {
-        int zero = 0;
-        cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
-    }
-    return v;
+    ESPDL_CUDA_TRY(cudaMemcpyToSymbol(g_tc_error, &word, sizeof(word)));
+    return ESPDL_OK;
 }
 
 // Role cycle counters of the tile kernel, compiled in only with -DESPDL_TC_TIMING (a measurement build; the product
@@ -336,7 +330,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 ok = false;
         }
         if (!ok)
-            atomicExch(&g_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_tc_error);
         TC_REC(0, w_empty);
         TC_REC(1, w_load);
         }
@@ -448,7 +442,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
         if (!ok)
-            atomicExch(&g_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_tc_error);
         TC_REC(2, w_tempty);
         TC_REC(3, w_full);
         TC_REC(4, w_issue);
@@ -562,7 +556,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 mbar_arrive(smem_u32(&tempty_bar[acc]));
         }
         if (!ok && lane == 0)
-            atomicExch(&g_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_tc_error);
         if (ew == 0 && lane == 0) {
             TC_LAP(w_work);
             TC_REC(5, w_tfull);
@@ -722,7 +716,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
             if (!ok)
-                atomicExch(&g_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_tc_error);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -767,7 +761,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
             if (!ok)
-                atomicExch(&g_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_tc_error);
         }
         __syncwarp();
     } else {
@@ -809,7 +803,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 mbar_arrive_cluster(tempty_leader);
         }
         if (!ok && lane == 0)
-            atomicExch(&g_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_tc_error);
     }
 
     fence_before();

@@ -25,18 +25,12 @@
 
 namespace espdl {
 
-__device__ int g_stem_tc_error = 0;
+__device__ int *g_stem_tc_error = nullptr; // the status word of bounded waits (common.cuh)
 
-int read_and_clear_device_error_stem()
+int bind_device_error_stem(int *word)
 {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_stem_tc_error, sizeof(int)) != cudaSuccess)
-        return 0;
-    if (v) {
-        int zero = 0;
-        cudaMemcpyToSymbol(g_stem_tc_error, &zero, sizeof(int));
-    }
-    return v;
+    ESPDL_CUDA_TRY(cudaMemcpyToSymbol(g_stem_tc_error, &word, sizeof(word)));
+    return ESPDL_OK;
 }
 
 namespace {
@@ -156,7 +150,7 @@ stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 }
             }
             if (!ok)
-                atomicExch(&g_stem_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_stem_tc_error);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -194,7 +188,7 @@ stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 }
             }
             if (!ok)
-                atomicExch(&g_stem_tc_error, ESPDL_ERR_TIMEOUT);
+                report_timeout(g_stem_tc_error);
         }
         __syncwarp();
     } else {
@@ -302,7 +296,7 @@ stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                 mbar_arrive(smem_u32(&tempty_bar[acc]));
         }
         if (!ok && lane == 0)
-            atomicExch(&g_stem_tc_error, ESPDL_ERR_TIMEOUT);
+            report_timeout(g_stem_tc_error);
         if ((ew & 3) == 0 && lane == 0)
             bulk_wait_all(); // shared memory stays allocated until the last store has left it
     }
