@@ -31,8 +31,12 @@ public:
     /// (call invalidate() after each run).
     std::vector<result_t> &postprocess(int image);
     void invalidate() { m_valid = false; }
+    /// One image on its own: its row of codes is fetched and scored here, nothing is kept for another call.  The same exp table,
+    /// sequential sum, division and sort as the batch form, so the same bits and the same order.
+    std::vector<result_t> &postprocess_one(int image);
 
 protected:
+    bool create_scores();
     Model *m_model;
     TensorBase *m_model_output;
     TensorBase *m_output = nullptr; ///< float scores, device buffer + host copy
@@ -42,6 +46,8 @@ protected:
     bool m_need_softmax, m_valid = false;
     const char *const *m_cat_names = nullptr;
     std::vector<result_t> m_cls_result;
+    int8_t *m_row = nullptr; ///< pinned, one row of codes
+    std::vector<float> m_exp_table;
 };
 
 } // namespace cls

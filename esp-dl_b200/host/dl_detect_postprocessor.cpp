@@ -51,15 +51,15 @@ yolo11PostProcessor::yolo11PostProcessor(Model *model, dl::image::ImagePreproces
 
 yolo11PostProcessor::~yolo11PostProcessor()
 {
-    if (m_dev_records)
-        espdl_b200_arena_free(m_dev_records);
-    if (m_dev_count)
-        espdl_b200_arena_free(m_dev_count);
+    if (m_dev)
+        espdl_b200_arena_free(m_dev);
+    if (m_host)
+        espdl_b200_host_free(m_host);
 }
 
 void yolo11PostProcessor::clear_result() { m_box_lists.clear(); }
 
-esp_err_t yolo11PostProcessor::postprocess()
+esp_err_t yolo11PostProcessor::postprocess(int image)
 {
     clear_result();
     void *stream = m_model->stream();
@@ -72,24 +72,33 @@ esp_err_t yolo11PostProcessor::postprocess()
             return ESP_FAIL;
     }
     const int batch = scores[0]->shape[0];
+    if (image >= batch)
+        return ESP_FAIL;
+    const int first = image < 0 ? 0 : image, scanned = image < 0 ? batch : 1;
     m_box_lists.resize(batch);
-    if (!m_dev_count && espdl_b200_arena_alloc(16, &m_dev_count) != ESPDL_OK)
+    // One read-back brings the counter and the first records: more than that are rare (a detector's candidates of one image
+    // number in the dozens) and cost a second one.
+    constexpr size_t COUNTER = 16, HEAD_RECORDS = 64;
+    const size_t head_bytes = COUNTER + HEAD_RECORDS * sizeof(espdl_detect_record);
+    if (!m_host && espdl_b200_host_alloc(head_bytes, (void **)&m_host) != ESPDL_OK)
         return ESP_FAIL;
     std::vector<espdl_detect_record> records;
     for (int attempt = 0; attempt < 2; attempt++) {
-        if (!m_dev_records) {
+        if (!m_dev) {
             if (m_capacity == 0)
                 m_capacity = 4096 * batch;
-            if (espdl_b200_arena_alloc((size_t)m_capacity * sizeof(espdl_detect_record), &m_dev_records) != ESPDL_OK)
+            if (espdl_b200_arena_alloc(COUNTER + (size_t)m_capacity * sizeof(espdl_detect_record), &m_dev) != ESPDL_OK)
                 return ESP_FAIL;
         }
-        espdl_b200_memset(m_dev_count, 0, 16, stream);
+        espdl_detect_record *dev_records = (espdl_detect_record *)((char *)m_dev + COUNTER);
+        espdl_b200_memset(m_dev, 0, COUNTER, stream);
         for (size_t i = 0; i < m_stages.size(); i++) {
             espdl_detect_desc d;
             memset(&d, 0, sizeof(d));
-            d.score = (const int8_t *)scores[i]->device, d.box = (const int8_t *)boxes[i]->device;
-            d.records = (espdl_detect_record *)m_dev_records, d.count = (uint32_t *)m_dev_count;
-            d.n = batch, d.h = scores[i]->shape[1], d.w = scores[i]->shape[2], d.classes = scores[i]->shape[3], d.box_channels = 64;
+            d.n = scanned, d.h = scores[i]->shape[1], d.w = scores[i]->shape[2], d.classes = scores[i]->shape[3], d.box_channels = 64;
+            const size_t pixels = (size_t)d.h * d.w * first;
+            d.score = (const int8_t *)scores[i]->device + pixels * d.classes, d.box = (const int8_t *)boxes[i]->device + pixels * 64;
+            d.records = dev_records, d.count = (uint32_t *)m_dev;
             // T score_thr_quant = quantize<T>(inverse_sigmoid(score_thr), 1 / score_exp)  (dl_detect_yolo11_postprocessor.cpp:24)
             const float inv = 1.f / scale_of(scores[i]->exponent);
             int q = (int)floorf((float)((double)(inverse_sigmoid(m_score_thr) * inv) + 0.5));
@@ -100,18 +109,21 @@ esp_err_t yolo11PostProcessor::postprocess()
             if (espdl_b200_detect_candidates(&d, stream) != ESPDL_OK)
                 return ESP_FAIL;
         }
-        uint32_t count = 0;
-        if (espdl_b200_download(&count, m_dev_count, 4, stream) != ESPDL_OK || espdl_b200_stream_sync(stream) != ESPDL_OK)
+        if (espdl_b200_download(m_host, m_dev, head_bytes, stream) != ESPDL_OK || espdl_b200_stream_sync(stream) != ESPDL_OK)
             return ESP_FAIL;
+        const uint32_t count = *(const uint32_t *)m_host;
         if ((int)count > m_capacity) { // more candidates than room: grow once and scan again
-            espdl_b200_arena_free(m_dev_records);
-            m_dev_records = nullptr;
+            espdl_b200_arena_free(m_dev);
+            m_dev = nullptr;
             m_capacity = (int)count + 1024;
             continue;
         }
         records.resize(count);
-        if (count && (espdl_b200_download(records.data(), m_dev_records, (size_t)count * sizeof(espdl_detect_record), stream) != ESPDL_OK ||
-                      espdl_b200_stream_sync(stream) != ESPDL_OK))
+        const size_t head = std::min((size_t)count, HEAD_RECORDS);
+        if (head)
+            memcpy(records.data(), m_host + COUNTER, head * sizeof(espdl_detect_record));
+        if (count > head && (espdl_b200_download(records.data() + head, dev_records + head, (count - head) * sizeof(espdl_detect_record), stream) != ESPDL_OK ||
+                             espdl_b200_stream_sync(stream) != ESPDL_OK))
             return ESP_FAIL;
         break;
     }
@@ -143,7 +155,7 @@ esp_err_t yolo11PostProcessor::postprocess()
                   (int)(((center_y - dfl_integral(box_data + reg_max, reg_max - 1) * st.stride_y) - border_top) * inv_resize_scale_y),
                   (int)(((center_x + dfl_integral(box_data + 2 * reg_max, reg_max - 1) * st.stride_x) - border_left) * inv_resize_scale_x),
                   (int)(((center_y + dfl_integral(box_data + 3 * reg_max, reg_max - 1) * st.stride_y) - border_top) * inv_resize_scale_y)};
-        per_image[r.image].push_back(nb);
+        per_image[first + r.image].push_back(nb);
     }
     for (int b = 0; b < batch; b++) {
         std::stable_sort(per_image[b].begin(), per_image[b].end(), [](const result_t &x, const result_t &y) { return x.score > y.score; });

@@ -36,8 +36,10 @@ public:
     void set_output_names(const std::vector<std::pair<std::string, std::string>> &names) { m_names = names; }
     void set_score_thr(float v) { m_score_thr = v; }
     void set_nms_thr(float v) { m_nms_thr = v; }
+    void set_top_k(int v) { m_top_k = v; }
     void clear_result();
-    esp_err_t postprocess();
+    /// All images of the batch, or (image >= 0) only that one.
+    esp_err_t postprocess(int image = -1);
     std::list<result_t> &get_result(int width, int height, int image = 0);
 
 private:
@@ -49,7 +51,8 @@ private:
     std::vector<anchor_point_stage_t> m_stages;
     std::vector<std::pair<std::string, std::string>> m_names;
     std::vector<std::list<result_t>> m_box_lists; ///< per image
-    void *m_dev_records = nullptr, *m_dev_count = nullptr;
+    void *m_dev = nullptr;  ///< the candidate counter (16 bytes) and, behind it, m_capacity records
+    char *m_host = nullptr; ///< pinned: the counter and the first HEAD_RECORDS records of a scan, fetched together
     int m_capacity = 0;
 };
 

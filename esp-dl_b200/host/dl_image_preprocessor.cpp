@@ -1,5 +1,6 @@
 #include "dl_image_preprocessor.hpp"
 
+#include <algorithm>
 #include <math.h>
 #include <string.h>
 
@@ -113,34 +114,49 @@ esp_err_t ImagePreprocessor::preprocess(const std::vector<img_t> &imgs, const st
         m_inv_scale_x = (float)src_w / inner_w, m_inv_scale_y = (float)src_h / inner_h;
         m_scale_x = 1.f / m_inv_scale_x, m_scale_y = 1.f / m_inv_scale_y;
     }
-    // stage the images: pinned host buffer -> device
-    const size_t one = (size_t)w * h * m_channels, bytes = one * imgs.size();
+    const int x0 = crop_area.empty() ? 0 : crop_area[0], y0 = crop_area.empty() ? 0 : crop_area[1];
+    if (x0 < 0 || y0 < 0 || src_w <= 0 || src_h <= 0 || x0 + src_w > w || y0 + src_h > h || inner_w <= 0 || inner_h <= 0)
+        return ESP_FAIL;
+    // Stage the images: the crop's columns of the source rows that the resize reads, through a pinned host buffer.  A nearest
+    // resize to fewer rows reads one source row per destination row (the index map of the reference, evaluated here), so
+    // the rest of the frame is neither copied nor uploaded (480 -> 224 rows: 0.43 of 0.92 MB).
+    const bool pick_rows = inner_h < src_h;
+    const int rows = pick_rows ? inner_h : src_h;
+    const size_t row_bytes = (size_t)src_w * m_channels, one = row_bytes * rows, bytes = one * imgs.size();
+    void *stream = m_model->stream();
     if (bytes > m_images_bytes) {
-        espdl_b200_stream_sync(m_model->stream());
+        espdl_b200_stream_sync(stream);
         if (m_dev_images)
             espdl_b200_arena_free(m_dev_images);
         if (m_host_images)
             espdl_b200_host_free(m_host_images);
-        m_dev_images = m_host_images = nullptr;
+        m_dev_images = m_host_images = nullptr, m_images_bytes = 0;
         if (espdl_b200_arena_alloc(bytes, &m_dev_images) != ESPDL_OK || espdl_b200_host_alloc(bytes, &m_host_images) != ESPDL_OK)
             return ESP_FAIL;
         m_images_bytes = bytes;
     }
-    for (size_t i = 0; i < imgs.size(); i++) memcpy((uint8_t *)m_host_images + i * one, imgs[i].data, one);
-    void *stream = m_model->stream();
-    if (espdl_b200_upload(m_dev_images, m_host_images, bytes, stream) != ESPDL_OK)
-        return ESP_FAIL;
+    constexpr size_t PIECE = 128 << 10; // uploaded while the next piece is still being copied
+    size_t done = 0, sent = 0;
+    for (const img_t &im : imgs)
+        for (int r = 0; r < rows; r++) {
+            const int sy = pick_rows ? std::min((int)((float)r * m_inv_scale_y) + y0, y0 + src_h - 1) : y0 + r;
+            memcpy((uint8_t *)m_host_images + done, (const uint8_t *)im.data + ((size_t)sy * w + x0) * m_channels, row_bytes);
+            done += row_bytes;
+            if (done - sent >= PIECE || done == bytes) {
+                if (espdl_b200_upload((uint8_t *)m_dev_images + sent, (uint8_t *)m_host_images + sent, done - sent, stream) != ESPDL_OK)
+                    return ESP_FAIL;
+                sent = done;
+            }
+        }
     espdl_image_desc d;
     memset(&d, 0, sizeof(d));
     d.input = (const uint8_t *)m_dev_images, d.output = m_model_input->device, d.lut = m_dev_table;
-    d.n = (int)imgs.size(), d.src_h = h, d.src_w = w, d.channels = m_channels, d.dst_h = dst_h, d.dst_w = dst_w;
+    d.n = (int)imgs.size(), d.src_h = rows, d.src_w = src_w, d.channels = m_channels, d.dst_h = dst_h, d.dst_w = dst_w;
     d.out_dtype = m_model_input->dtype == DATA_TYPE_INT8 ? ESPDL_DTYPE_INT8 : ESPDL_DTYPE_INT16;
-    if (!crop_area.empty())
-        d.crop_x0 = crop_area[0], d.crop_y0 = crop_area[1], d.crop_x1 = crop_area[2], d.crop_y1 = crop_area[3];
     d.border_top = m_border[0], d.border_bottom = m_border[1], d.border_left = m_border[2], d.border_right = m_border[3];
     d.swap_rb = m_swap;
     memcpy(d.bg, m_bg, 4);
-    d.inv_scale_x = m_inv_scale_x, d.inv_scale_y = m_inv_scale_y;
+    d.inv_scale_x = m_inv_scale_x, d.inv_scale_y = pick_rows ? 1.f : m_inv_scale_y;
     if (espdl_b200_image_preprocess(&d, stream) != ESPDL_OK)
         return ESP_FAIL;
     return espdl_b200_stream_sync(stream) == ESPDL_OK ? ESP_OK : ESP_FAIL; // the pinned buffer may be refilled after this

@@ -7,6 +7,8 @@
 #include "espdl_b200.h"
 
 #include <cstring>
+#include <list>
+#include <memory>
 #include <string>
 
 using namespace dl;
@@ -16,6 +18,18 @@ struct Handle {
     Model *model = nullptr;
     std::vector<std::string> input_names, output_names;
     std::string text;
+    // What the calls below keep between calls: tables, staging buffers and counters on the device.  A program calls them with
+    // the same settings for every frame; the least recently used settings beyond four make room.
+    struct Pre {
+        std::vector<float> key;
+        std::unique_ptr<image::ImagePreprocessor> object;
+    };
+    std::list<Pre> pre; // most recently used first
+    std::unique_ptr<cls::ClsPostprocessor> classifier;
+    bool classifier_softmax = false;
+    std::unique_ptr<detect::yolo11PostProcessor> detector;
+    std::vector<std::string> detector_names;
+    std::vector<int> detector_strides;
 };
 
 TensorBase *io_tensor(Handle *h, int is_output, int index)
@@ -108,6 +122,9 @@ void espdl_model_destroy(void *handle)
 {
     Handle *h = (Handle *)handle;
     if (h) {
+        h->pre.clear(); // they hold on to the model
+        h->classifier.reset();
+        h->detector.reset();
         delete h->model;
         delete h;
     }
@@ -217,16 +234,25 @@ long long espdl_model_read_tensor(void *handle, const char *name, void *dst, siz
 int espdl_model_detect(void *handle, int image, int stages, const char *const *names, const int *strides, float score_thr, float nms_thr,
                        int top_k, int width, int height, int max_results, int *boxes, float *scores)
 {
-    Model *model = ((Handle *)handle)->model;
-    std::vector<detect::anchor_point_stage_t> st;
-    std::vector<std::pair<std::string, std::string>> nm;
-    for (int i = 0; i < stages; i++) {
-        st.push_back({strides[i], strides[i], strides[i] / 2, strides[i] / 2});
-        nm.push_back({names[2 * i], names[2 * i + 1]});
+    Handle *h = (Handle *)handle;
+    const std::vector<std::string> key(names, names + 2 * stages);
+    const std::vector<int> stride_key(strides, strides + stages);
+    if (!h->detector || h->detector_names != key || h->detector_strides != stride_key) {
+        std::vector<detect::anchor_point_stage_t> st;
+        std::vector<std::pair<std::string, std::string>> nm;
+        for (int i = 0; i < stages; i++) {
+            st.push_back({strides[i], strides[i], strides[i] / 2, strides[i] / 2});
+            nm.push_back({names[2 * i], names[2 * i + 1]});
+        }
+        h->detector.reset(new detect::yolo11PostProcessor(h->model, nullptr, score_thr, nms_thr, top_k, st));
+        h->detector->set_output_names(nm);
+        h->detector_names = key, h->detector_strides = stride_key;
     }
-    detect::yolo11PostProcessor post(model, nullptr, score_thr, nms_thr, top_k, st);
-    post.set_output_names(nm);
-    if (post.postprocess() != ESP_OK)
+    detect::yolo11PostProcessor &post = *h->detector;
+    post.set_score_thr(score_thr);
+    post.set_nms_thr(nms_thr);
+    post.set_top_k(top_k);
+    if (post.postprocess(image < 0 ? -1 : image) != ESP_OK)
         return -1;
     int k = 0;
     for (const detect::result_t &r : post.get_result(width, height, image)) {
@@ -243,9 +269,14 @@ int espdl_model_detect(void *handle, int image, int stages, const char *const *n
 /// best first.  Returns the number of results, -1 on error.
 int espdl_model_classify(void *handle, int image, int top_k, float score_thr, int need_softmax, int *categories, float *scores)
 {
-    Model *model = ((Handle *)handle)->model;
-    cls::ClsPostprocessor post(model, top_k, score_thr, need_softmax != 0);
-    std::vector<cls::result_t> &r = post.postprocess(image);
+    Handle *h = (Handle *)handle;
+    if (!h->classifier || h->classifier_softmax != (need_softmax != 0)) {
+        h->classifier.reset(new cls::ClsPostprocessor(h->model, top_k, score_thr, need_softmax != 0));
+        h->classifier_softmax = need_softmax != 0;
+    }
+    h->classifier->set_topk(top_k);
+    h->classifier->set_score_thr(score_thr);
+    std::vector<cls::result_t> &r = h->classifier->postprocess_one(image);
     for (size_t i = 0; i < r.size(); i++) categories[i] = r[i].category, scores[i] = r[i].score;
     return (int)r.size();
 }
@@ -255,16 +286,29 @@ int espdl_model_classify(void *handle, int image, int top_k, float score_thr, in
 int espdl_model_preprocess(void *handle, const unsigned char *images, int n, int h, int w, int channels, const float *mean, const float *stdv,
                            int rgb_swap, int letterbox_bg, const int *crop)
 {
-    Model *model = ((Handle *)handle)->model;
-    image::ImagePreprocessor *pre = channels == 3
-        ? new image::ImagePreprocessor(model, std::array<float, 3>{mean[0], mean[1], mean[2]}, std::array<float, 3>{stdv[0], stdv[1], stdv[2]}, rgb_swap != 0)
-        : new image::ImagePreprocessor(model, mean[0], stdv[0]);
-    if (letterbox_bg >= 0) {
-        if (channels == 3)
-            pre->enable_letterbox(std::array<uint8_t, 3>{(uint8_t)letterbox_bg, (uint8_t)letterbox_bg, (uint8_t)letterbox_bg});
-        else
-            pre->enable_letterbox((uint8_t)letterbox_bg);
+    Handle *handle_ = (Handle *)handle;
+    Model *model = handle_->model;
+    std::vector<float> key = {(float)channels, (float)(rgb_swap != 0), (float)letterbox_bg};
+    for (int c = 0; c < (channels == 3 ? 3 : 1); c++) key.push_back(mean[c]), key.push_back(stdv[c]);
+    std::list<Handle::Pre> &kept = handle_->pre;
+    auto it = kept.begin();
+    while (it != kept.end() && it->key != key) ++it;
+    if (it == kept.end()) {
+        std::unique_ptr<image::ImagePreprocessor> made(
+            channels == 3 ? new image::ImagePreprocessor(model, std::array<float, 3>{mean[0], mean[1], mean[2]}, std::array<float, 3>{stdv[0], stdv[1], stdv[2]}, rgb_swap != 0)
+                          : new image::ImagePreprocessor(model, mean[0], stdv[0]));
+        if (letterbox_bg >= 0) {
+            if (channels == 3)
+                made->enable_letterbox(std::array<uint8_t, 3>{(uint8_t)letterbox_bg, (uint8_t)letterbox_bg, (uint8_t)letterbox_bg});
+            else
+                made->enable_letterbox((uint8_t)letterbox_bg);
+        }
+        while (kept.size() >= 4) kept.pop_back();
+        kept.push_front({key, std::move(made)});
+    } else {
+        kept.splice(kept.begin(), kept, it);
     }
+    image::ImagePreprocessor *pre = kept.front().object.get();
     std::vector<image::img_t> imgs;
     for (int i = 0; i < n; i++)
         imgs.push_back({(void *)(images + (size_t)i * h * w * channels), (uint16_t)w, (uint16_t)h,
@@ -273,7 +317,6 @@ int espdl_model_preprocess(void *handle, const unsigned char *images, int n, int
     if (crop)
         crop_area.assign(crop, crop + 4);
     const esp_err_t e = pre->preprocess(imgs, crop_area);
-    delete pre;
     return e == ESP_OK ? 0 : -1;
 }
 
