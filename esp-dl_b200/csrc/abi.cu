@@ -200,6 +200,9 @@ int espdl_b200_download(void *dst_host, const void *src_dev, size_t bytes, void 
 
 } // extern "C"
 namespace espdl {
+static thread_local int g_model_scope = 0;
+bool in_model_scope() { return g_model_scope > 0; }
+
 bool pdl_enabled()
 {
     static const bool on = !getenv("ESPDL_B200_NO_PDL");
@@ -207,6 +210,8 @@ bool pdl_enabled()
 }
 } // namespace espdl
 extern "C" {
+
+void espdl_b200_model_scope(int enter) { g_model_scope += enter ? 1 : -1; }
 
 int espdl_b200_download_rows(void *dst_host, const void *src_dev, size_t row_bytes, size_t src_stride_bytes, size_t rows, void *stream)
 {

@@ -41,6 +41,18 @@ cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The kernels that move or rewrite tensors (elementwise operators, pools, copies, reductions ...) start with grid_dep_wait() and
+// take a last argument `early`: whether they let the next kernel's blocks become resident at once.  The conv kernels read
+// their parameters (filter, bias, exponents) before they wait, and a caller of the C ABI may have written those with
+// espdl_b200_copy or the like just before - so `early` only inside a model's plan, whose parameters no launch writes.
+bool in_model_scope();
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_mover(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args)
+{
+    return launch_overlapped(kernel, grid, block, smem, s, args..., (int)in_model_scope());
+}
+
 #ifdef __CUDACC__
 // Blocks until every kernel this one depends on has finished and its writes are visible to this grid.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

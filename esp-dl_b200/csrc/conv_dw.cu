@@ -26,6 +26,8 @@ __device__ __forceinline__ int sbyte(uint32_t x, int i) { return (int)(int8_t)(x
 
 __global__ void __launch_bounds__(256) dw_s8_vec16_kernel(DwParams p)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const int8_t *__restrict__ in = (const int8_t *)p.in;
     const int8_t *__restrict__ w = (const int8_t *)p.w;
     const int32_t *__restrict__ bias = (const int32_t *)p.bias;
@@ -151,6 +153,8 @@ __device__ __noinline__ void dw3x3_band_general(const DwParams &p, int S, int n,
 template <int S, bool EVEN>
 __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xsegs, int ytiles, int cols_per_thread)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     constexpr int ROWS_IN = S == 1 ? 6 : 5;
     constexpr int ROWS_OUT = S == 1 ? 4 : 2;
     const int quads = p.c >> 2;
@@ -325,6 +329,8 @@ __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xseg
 template <typename T, typename ACC, typename BIAS>
 __global__ void __launch_bounds__(256) dw_generic_kernel(DwParams p)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const T *__restrict__ in = (const T *)p.in;
     const T *__restrict__ w = (const T *)p.w;
     const BIAS *__restrict__ bias = (const BIAS *)p.bias;
@@ -398,22 +404,22 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
         if (blocks > 0x7fffffffll)
             return ESPDL_ERR_TOO_LARGE;
         if (d.stride_h == 1)
-            (p.half_even ? dw3x3_dp4a_kernel<1, true> : dw3x3_dp4a_kernel<1, false>)<<<(unsigned)blocks, 128, 0, s>>>(p, xsegs, ytiles, cols);
+            launch_overlapped(p.half_even ? dw3x3_dp4a_kernel<1, true> : dw3x3_dp4a_kernel<1, false>, dim3((unsigned)blocks), dim3(128), 0, s, p, xsegs, ytiles, cols);
         else
-            (p.half_even ? dw3x3_dp4a_kernel<2, true> : dw3x3_dp4a_kernel<2, false>)<<<(unsigned)blocks, 128, 0, s>>>(p, xsegs, ytiles, cols);
+            launch_overlapped(p.half_even ? dw3x3_dp4a_kernel<2, true> : dw3x3_dp4a_kernel<2, false>, dim3((unsigned)blocks), dim3(128), 0, s, p, xsegs, ytiles, cols);
     } else if (vec) {
         p.chunks = d.in_c / 16;
         p.total = pixels * p.chunks;
         long long blocks = min((p.total + threads - 1) / threads, max_blocks);
-        dw_s8_vec16_kernel<<<(unsigned)blocks, threads, 0, s>>>(p);
+        launch_overlapped(dw_s8_vec16_kernel, dim3((unsigned)blocks), dim3(threads), 0, s, p);
     } else {
         p.chunks = 0;
         p.total = pixels * d.in_c;
         long long blocks = min((p.total + threads - 1) / threads, max_blocks);
         if (d.dtype == ESPDL_DTYPE_INT8)
-            dw_generic_kernel<int8_t, int32_t, int32_t><<<(unsigned)blocks, threads, 0, s>>>(p);
+            launch_overlapped(dw_generic_kernel<int8_t, int32_t, int32_t>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
         else
-            dw_generic_kernel<int16_t, long long, long long><<<(unsigned)blocks, threads, 0, s>>>(p);
+            launch_overlapped(dw_generic_kernel<int16_t, long long, long long>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
     }
     count_launch();
     return check_launch("conv2d_depthwise");

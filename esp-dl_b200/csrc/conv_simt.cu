@@ -29,6 +29,8 @@ struct ConvParams {
 template <int OCT, bool DP4A>
 __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const int8_t *__restrict__ in = (const int8_t *)p.in;
     const int8_t *__restrict__ w = (const int8_t *)p.w;
     const int32_t *__restrict__ bias = (const int32_t *)p.bias;
@@ -98,6 +100,8 @@ __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
 template <int OCT>
 __global__ void __launch_bounds__(256) conv_s16_kernel(ConvParams p)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const int16_t *__restrict__ in = (const int16_t *)p.in;
     const int16_t *__restrict__ w = (const int16_t *)p.w;
     const long long *__restrict__ bias = (const long long *)p.bias;
@@ -157,6 +161,8 @@ constexpr int SMALL_MAX_OC = 64;
 template <int KH, int KW, int IC>
 __global__ void __launch_bounds__(256) conv_s8_small_k_kernel(ConvParams p)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     __shared__ int w_s[SMALL_MAX_OC * SMALL_MAX_WORDS];
     __shared__ int bias_s[SMALL_MAX_OC];
     __shared__ int shift_s[SMALL_MAX_OC];
@@ -260,19 +266,19 @@ int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
         const long long pixels = (long long)d.n * d.out_h * d.out_w;
         const unsigned grid = (unsigned)min((pixels + threads - 1) / threads, max_blocks);
         if (d.in_c == 3)
-            conv_s8_small_k_kernel<3, 3, 3><<<grid, threads, 0, s>>>(p);
+            launch_overlapped(conv_s8_small_k_kernel<3, 3, 3>, dim3(grid), dim3(threads), 0, s, p);
         else if (d.in_c == 1)
-            conv_s8_small_k_kernel<3, 3, 1><<<grid, threads, 0, s>>>(p);
+            launch_overlapped(conv_s8_small_k_kernel<3, 3, 1>, dim3(grid), dim3(threads), 0, s, p);
         else
-            conv_s8_small_k_kernel<3, 3, 4><<<grid, threads, 0, s>>>(p);
+            launch_overlapped(conv_s8_small_k_kernel<3, 3, 4>, dim3(grid), dim3(threads), 0, s, p);
     } else if (d.dtype == ESPDL_DTYPE_INT8) {
         const bool dp4a = d.in_c % 4 == 0 && p.ips % 4 == 0 && ((uintptr_t)d.input % 4) == 0 && ((uintptr_t)d.filter % 4) == 0;
         if (dp4a)
-            conv_s8_kernel<OCT, true><<<(unsigned)blocks, threads, 0, s>>>(p);
+            launch_overlapped(conv_s8_kernel<OCT, true>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
         else
-            conv_s8_kernel<OCT, false><<<(unsigned)blocks, threads, 0, s>>>(p);
+            launch_overlapped(conv_s8_kernel<OCT, false>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
     } else {
-        conv_s16_kernel<OCT><<<(unsigned)blocks, threads, 0, s>>>(p);
+        launch_overlapped(conv_s16_kernel<OCT>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
     }
     count_launch();
     return check_launch("conv2d_simt");

@@ -104,10 +104,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (threadIdx.x == 0)
+        grid_dep_launch(); // set up: the next kernel's CTAs may take SMs as they become free
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
+            grid_dep_wait(); // the previous kernel's output, before the first load; the other roles act on what the producer brought in
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -444,6 +447,8 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     __syncthreads();
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (threadIdx.x == 0)
+        grid_dep_launch(); // set up: the next kernel's CTAs may take SMs as they become free
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -451,6 +456,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             // the filter, once: one box per tap
             mbar_arrive_expect_tx(smem_u32(filt_bar), (uint32_t)(taps * b_tap));
             for (int tap = 0; tap < taps; tap++) tma_load_2d(smem_u32(filt_s + (size_t)tap * b_tap), &map_b, tap * p.cin, 0, smem_u32(filt_bar));
+            grid_dep_wait(); // the previous kernel's output, before the first patch; the other roles act on what the producer brought in
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -855,7 +861,7 @@ int launch_patch(const espdl_conv_desc &d, PatchParams &p, cudaStream_t s)
     if (total > 0x7fffffffll)
         return ESPDL_ERR_TOO_LARGE;
     const auto kernel = p.epi.half_even ? conv_patch_kernel<true> : conv_patch_kernel<false>;
-    kernel<<<(int)min(total, (long long)num_sms()), CV_THREADS, smem, s>>>(ma, mb, mo, p);
+    launch_overlapped(kernel, dim3((int)min(total, (long long)num_sms())), dim3(CV_THREADS), smem, s, ma, mb, mo, p);
     count_launch();
     return check_launch("conv_patch");
 }
@@ -951,7 +957,7 @@ int conv2d_conv_tc(const espdl_conv_desc &d, cudaStream_t s)
         return ESPDL_ERR_TOO_LARGE;
     const int grid = (int)min(total, (long long)num_sms());
     const auto kernel = p.epi.half_even ? conv_tc_kernel<true> : conv_tc_kernel<false>;
-    kernel<<<grid, CV_THREADS, smem, s>>>(ma, mb, mo, p);
+    launch_overlapped(kernel, dim3(grid), dim3(CV_THREADS), smem, s, ma, mb, mo, p);
     count_launch();
     return check_launch("conv_tc");
 }

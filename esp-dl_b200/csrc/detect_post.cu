@@ -9,8 +9,11 @@ namespace espdl {
 
 namespace {
 
-__global__ void __launch_bounds__(256) detect_candidates_kernel(espdl_detect_desc d, long long pixels)
+__global__ void __launch_bounds__(256) detect_candidates_kernel(espdl_detect_desc d, long long pixels, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long pix = blockIdx.x * (long long)blockDim.x + threadIdx.x; pix < pixels; pix += (long long)gridDim.x * blockDim.x) {
         const int8_t *sp = d.score + pix * d.classes;
         const bool vec = (d.classes % 16 == 0) && (((uintptr_t)d.score) % 16 == 0);
@@ -50,7 +53,7 @@ int detect_candidates(const espdl_detect_desc &d, cudaStream_t s)
     const long long pixels = (long long)d.n * d.h * d.w;
     const long long blocks = (pixels + 255) / 256;
     const int grid = (int)(blocks < (long long)num_sms() * 16 ? blocks : (long long)num_sms() * 16);
-    detect_candidates_kernel<<<grid, 256, 0, s>>>(d, pixels);
+    launch_mover(detect_candidates_kernel, dim3(grid), dim3(256), 0, s, d, pixels);
     count_launch();
     return check_launch("detect_candidates");
 }

@@ -145,8 +145,11 @@ __device__ __forceinline__ long long elt_int(const EltParams &p, long long a, lo
     }
 }
 
-__global__ void __launch_bounds__(256) elt_generic_kernel(EltParams p)
+__global__ void __launch_bounds__(256) elt_generic_kernel(EltParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
         long long r = i;
         const int i0 = (int)(r % p.os[3]);
@@ -189,8 +192,11 @@ __global__ void __launch_bounds__(256) elt_generic_kernel(EltParams p)
 
 // int8 -> int8, operands of identical shape, 16 elements per thread.
 template <int OP>
-__global__ void __launch_bounds__(256) elt_s8_vec16_kernel(EltParams p, long long nvec)
+__global__ void __launch_bounds__(256) elt_s8_vec16_kernel(EltParams p, long long nvec, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     __shared__ int8_t table[256];
     // One-operand int8 -> int8 operators are functions of the input byte: every block tabulates the operator once with
     // the scalar code (so the rounding is the reference's) and then runs as a table lookup like LUT itself.
@@ -247,8 +253,11 @@ __global__ void __launch_bounds__(256) elt_s8_vec16_kernel(EltParams p, long lon
 // int8 (op) one-element int8 -> int8 (Mul by a scalar factor, Add of a constant, ...): with the second operand fixed the
 // operator is a function of the input byte, so every block tabulates it once with the scalar code (the reference's
 // rounding, whatever the operator) and then runs as a table lookup at the speed of LUT.
-__global__ void __launch_bounds__(256) elt_s8_scalar_b_kernel(EltParams p, long long nvec)
+__global__ void __launch_bounds__(256) elt_s8_scalar_b_kernel(EltParams p, long long nvec, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     __shared__ int8_t table[256];
     const int b = (int)((const int8_t *)p.b)[0];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
@@ -278,7 +287,7 @@ static void launch_vec(const EltParams &p, long long nvec, cudaStream_t s)
 {
     const int threads = 256;
     long long blocks = min((nvec + threads - 1) / threads, (long long)num_sms() * 16);
-    elt_s8_vec16_kernel<OP><<<(unsigned)max(blocks, 1ll), threads, 0, s>>>(p, nvec);
+    launch_mover(elt_s8_vec16_kernel<OP>, dim3((unsigned)max(blocks, 1ll)), dim3(threads), 0, s, p, nvec);
 }
 
 } // namespace espdl
@@ -390,7 +399,7 @@ extern "C" int espdl_b200_eltwise(const espdl_eltwise_desc *d, void *stream)
     if (scalar_b) {
         const long long nvec = total / 16;
         const long long blocks = min((nvec + 255) / 256, (long long)num_sms() * 16);
-        elt_s8_scalar_b_kernel<<<(unsigned)max(blocks, 1ll), 256, 0, s>>>(p, nvec);
+        launch_mover(elt_s8_scalar_b_kernel, dim3((unsigned)max(blocks, 1ll)), dim3(256), 0, s, p, nvec);
     } else if (vec) {
         const long long nvec = total / 16;
         switch (d->op) {
@@ -415,7 +424,7 @@ extern "C" int espdl_b200_eltwise(const espdl_eltwise_desc *d, void *stream)
     } else {
         const int threads = 256;
         long long blocks = min((total + threads - 1) / threads, (long long)num_sms() * 32);
-        elt_generic_kernel<<<(unsigned)blocks, threads, 0, s>>>(p);
+        launch_mover(elt_generic_kernel, dim3((unsigned)blocks), dim3(threads), 0, s, p);
     }
     count_launch();
     return check_launch("eltwise");

@@ -819,6 +819,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 __global__ void __launch_bounds__(256) split_limbs_kernel(const int16_t *__restrict__ src, long long stride, int K, long long total,
                                                           int8_t *__restrict__ hi, uint8_t *__restrict__ lo)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long r = i / K;
         const int k = (int)(i % K);
@@ -1089,8 +1091,8 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
         uint8_t *b_lo = (uint8_t *)workspace + 2 * a + b;
         const long long ta = (long long)p.M * p.K, tb = (long long)p.N * p.K;
         const long long cap = (long long)num_sms() * 32;
-        split_limbs_kernel<<<(unsigned)min((ta + 255) / 256, cap), 256, 0, s>>>((const int16_t *)d.input, ips, p.K, ta, a_hi, a_lo);
-        split_limbs_kernel<<<(unsigned)min((tb + 255) / 256, cap), 256, 0, s>>>((const int16_t *)d.filter, p.K, p.K, tb, b_hi, b_lo);
+        launch_overlapped(split_limbs_kernel, dim3((unsigned)min((ta + 255) / 256, cap)), dim3(256), 0, s, (const int16_t *)d.input, ips, p.K, ta, a_hi, a_lo);
+        launch_overlapped(split_limbs_kernel, dim3((unsigned)min((tb + 255) / 256, cap)), dim3(256), 0, s, (const int16_t *)d.filter, p.K, p.K, tb, b_hi, b_lo);
         count_launch(2);
         if ((st = check_launch("split_limbs")))
             return st;
@@ -1130,7 +1132,7 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(gemm_tc_kernel)");
     if (i16)
-        gemm_tc_kernel<true, false><<<grid, NUM_THREADS, smem, s>>>(ma, mb, ma_lo, mb_lo, mo, p);
+        launch_overlapped(gemm_tc_kernel<true, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
     else
         launch_overlapped(p.epi.half_even ? gemm_tc_kernel<false, true> : gemm_tc_kernel<false, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
     count_launch();

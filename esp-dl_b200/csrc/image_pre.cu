@@ -24,8 +24,11 @@ struct ImgParams {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256) image_pre_kernel(ImgParams p)
+__global__ void __launch_bounds__(256) image_pre_kernel(ImgParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     __shared__ T lut_s[3 * 256];
     for (int i = threadIdx.x; i < p.ch * 256; i += blockDim.x) lut_s[i] = ((const T *)p.lut)[i];
     __syncthreads();
@@ -83,9 +86,9 @@ int image_preprocess(const espdl_image_desc &d, cudaStream_t s)
     const long long blocks = (p.total + 255) / 256;
     const int grid = (int)(blocks < (long long)num_sms() * 16 ? blocks : (long long)num_sms() * 16);
     if (d.out_dtype == ESPDL_DTYPE_INT8)
-        image_pre_kernel<int8_t><<<grid, 256, 0, s>>>(p);
+        launch_mover(image_pre_kernel<int8_t>, dim3(grid), dim3(256), 0, s, p);
     else
-        image_pre_kernel<int16_t><<<grid, 256, 0, s>>>(p);
+        launch_mover(image_pre_kernel<int16_t>, dim3(grid), dim3(256), 0, s, p);
     count_launch();
     return check_launch("image_pre");
 }

@@ -167,8 +167,11 @@ __device__ __forceinline__ void norm_row_words(const NormParams &p, const T *x, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) norm_kernel(NormParams p)
+__global__ void __launch_bounds__(256) norm_kernel(NormParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     __shared__ __align__(16) float stage_all[8][128];
     const bool words_ok = p.len % Word<T>::V == 0 && ((uintptr_t)p.in % 4) == 0 && ((uintptr_t)p.out % 4) == 0;
     const int lane = threadIdx.x & 31;
@@ -262,9 +265,9 @@ extern "C" int espdl_b200_norm(const espdl_norm_desc *d, void *stream)
     const long long blocks = (d->rows + 7) / 8; // eight rows (warps) per block
     const unsigned grid = (unsigned)min(blocks, (long long)num_sms() * 8);
     if (d->dtype == ESPDL_DTYPE_INT8)
-        norm_kernel<int8_t><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
+        launch_mover(norm_kernel<int8_t>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, p);
     else
-        norm_kernel<int16_t><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
+        launch_mover(norm_kernel<int16_t>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, p);
     count_launch();
     return check_launch("norm");
 }

@@ -16,8 +16,11 @@ struct PoolParams {
     long long total;
 };
 
-__global__ void __launch_bounds__(256) pool_kernel(PoolParams p)
+__global__ void __launch_bounds__(256) pool_kernel(PoolParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(i % p.c);
         const long long pix = i / p.c;
@@ -57,8 +60,11 @@ __global__ void __launch_bounds__(256) pool_kernel(PoolParams p)
 
 // Max pool, int8, C % 16 == 0: 16 channels per thread, 128-bit loads and stores, per-byte signed maximum over the
 // in-bounds taps (padding is excluded, as in pool_kernel).
-__global__ void __launch_bounds__(256) maxpool_s8_vec16_kernel(PoolParams p)
+__global__ void __launch_bounds__(256) maxpool_s8_vec16_kernel(PoolParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     const int chunks = p.c >> 4;
     const long long total = (long long)p.n * p.oh * p.ow * chunks;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -116,8 +122,11 @@ __device__ __forceinline__ void max_lanes(Lanes16 &a, const Lanes16 &b)
 }
 
 template <int K>
-__global__ void __launch_bounds__(256) maxpool_s8_walk_kernel(PoolParams p, int segments)
+__global__ void __launch_bounds__(256) maxpool_s8_walk_kernel(PoolParams p, int segments, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     const int chunks = p.c >> 4;
     const int seg_rows = (p.oh + segments - 1) / segments; // a column is cut into `segments` runs of output rows when there are few columns
     const long long total = (long long)p.n * segments * p.ow * chunks;
@@ -181,8 +190,11 @@ struct ResizeParams {
     long long total;
 };
 
-__global__ void __launch_bounds__(256) resize_nearest_kernel(ResizeParams p)
+__global__ void __launch_bounds__(256) resize_nearest_kernel(ResizeParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(i % p.c);
         const long long pix = i / p.c;
@@ -202,8 +214,11 @@ __global__ void __launch_bounds__(256) resize_nearest_kernel(ResizeParams p)
 
 // Nearest resize with equal input and output exponents is a pure gather ((float)q * 1 / 1 rounds back to q): 16
 // channels per thread, 128-bit loads and stores, a warp moves contiguous runs of both tensors.
-__global__ void __launch_bounds__(256) resize_nearest_vec16_kernel(ResizeParams p)
+__global__ void __launch_bounds__(256) resize_nearest_vec16_kernel(ResizeParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     const int chunks = p.c >> 4;
     const long long total = (long long)p.n * p.oh * p.ow * chunks;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -231,8 +246,11 @@ struct CopyParams {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256) copy_kernel(CopyParams p)
+__global__ void __launch_bounds__(256) copy_kernel(CopyParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
         long long r = i, si = 0, di = 0;
 #pragma unroll
@@ -251,8 +269,11 @@ __global__ void __launch_bounds__(256) copy_kernel(CopyParams p)
 // writes (along the innermost axis) touch consecutive addresses.  The row pitch of 64 * sizeof(T) + 4 bytes keeps the
 // column reads of the store phase on distinct banks.
 template <typename T>
-__global__ void __launch_bounds__(256) copy_transpose_kernel(CopyParams p, int ya, long long tiles)
+__global__ void __launch_bounds__(256) copy_transpose_kernel(CopyParams p, int ya, long long tiles, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     constexpr int TILE = 64, PITCH = TILE * (int)sizeof(T) + 4;
     __shared__ __align__(16) unsigned char tile[TILE * PITCH];
     const int nx = p.shape[5], ny = p.shape[ya];
@@ -299,8 +320,11 @@ __global__ void __launch_bounds__(256) copy_transpose_kernel(CopyParams p, int y
 // The same tile with 32-bit global accesses: V = 4 / sizeof(T) elements per access on both sides.  The caller has checked
 // that both extents, every stride that is not 1, and both pointers are multiples of V elements.
 template <typename T>
-__global__ void __launch_bounds__(256) copy_transpose_words_kernel(CopyParams p, int ya, long long tiles)
+__global__ void __launch_bounds__(256) copy_transpose_words_kernel(CopyParams p, int ya, long long tiles, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     constexpr int TILE = 64, PITCH = TILE * (int)sizeof(T) + 4, V = 4 / (int)sizeof(T), WPR = TILE / V; // words per tile row
     __shared__ __align__(16) unsigned char tile[TILE * PITCH];
     const int nx = p.shape[5], ny = p.shape[ya];
@@ -354,8 +378,11 @@ __global__ void __launch_bounds__(256) copy_transpose_words_kernel(CopyParams p,
 // destination order; the tile then leaves as whole words (16 bytes per thread where rows allow), 64 contiguous bytes per
 // destination row.  No byte-granular shared-memory traffic on either side.  Same preconditions as the word kernel above
 // (extents, strides and pointers multiples of 4).
-__global__ void __launch_bounds__(256) copy_transpose_bytes4_kernel(CopyParams p, int ya, long long tiles, int vec16)
+__global__ void __launch_bounds__(256) copy_transpose_bytes4_kernel(CopyParams p, int ya, long long tiles, int vec16, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     constexpr int TILE = 64, PITCH = TILE + 4; // 17 words per destination row: the block stores meet two-way conflicts at most
     __shared__ __align__(16) unsigned char tile[TILE * PITCH];
     const int nx = p.shape[5], ny = p.shape[ya];
@@ -460,20 +487,20 @@ extern "C" int espdl_b200_pool(const espdl_pool_desc *d, void *stream)
         const long long items = columns * segments;
         const unsigned grid = (unsigned)min((items + 255) / 256, (long long)num_sms() * 32);
         if (p.kh == 3)
-            maxpool_s8_walk_kernel<3><<<grid, 256, 0, (cudaStream_t)stream>>>(p, segments);
+            launch_mover(maxpool_s8_walk_kernel<3>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, p, segments);
         else
-            maxpool_s8_walk_kernel<5><<<grid, 256, 0, (cudaStream_t)stream>>>(p, segments);
+            launch_mover(maxpool_s8_walk_kernel<5>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, p, segments);
         count_launch();
         return check_launch("max pool walk");
     }
     if (d->op == ESPDL_POOL_MAX && !p.is16 && p.c % 16 == 0 && ((uintptr_t)d->input % 16) == 0 && ((uintptr_t)d->output % 16) == 0) {
         const long long items = p.total / 16;
-        maxpool_s8_vec16_kernel<<<(unsigned)min((items + 255) / 256, (long long)num_sms() * 32), 256, 0, (cudaStream_t)stream>>>(p);
+        launch_mover(maxpool_s8_vec16_kernel, dim3((unsigned)min((items + 255) / 256, (long long)num_sms() * 32)), dim3(256), 0, (cudaStream_t)stream, p);
         count_launch();
         return check_launch("max pool");
     }
     long long blocks = min((p.total + 255) / 256, (long long)num_sms() * 32);
-    pool_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(p);
+    launch_mover(pool_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, p);
     count_launch();
     return check_launch("pool");
 }
@@ -506,8 +533,11 @@ __device__ __forceinline__ void linear_coeffs_dev(int o, int &i, float &r0, floa
     r1 = fx;
 }
 
-__global__ void __launch_bounds__(256) resize_linear_kernel(ResizeLinearParams p)
+__global__ void __launch_bounds__(256) resize_linear_kernel(ResizeLinearParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(i % p.c);
         const long long pix = i / p.c;
@@ -560,7 +590,7 @@ extern "C" int espdl_b200_resize(const espdl_resize_desc *d, void *stream)
         q.total = (long long)q.n * q.oh * q.ow * q.c;
         if (q.total == 0)
             return ESPDL_OK;
-        resize_linear_kernel<<<(unsigned)min((q.total + 255) / 256, (long long)num_sms() * 32), 256, 0, (cudaStream_t)stream>>>(q);
+        launch_mover(resize_linear_kernel, dim3((unsigned)min((q.total + 255) / 256, (long long)num_sms() * 32)), dim3(256), 0, (cudaStream_t)stream, q);
         count_launch();
         return check_launch("resize_linear");
     }
@@ -583,12 +613,12 @@ extern "C" int espdl_b200_resize(const espdl_resize_desc *d, void *stream)
         return ESPDL_OK;
     if (oscale == 1 && shift == 0 && p.c % 16 == 0 && p.ops % 16 == 0 && ((uintptr_t)d->input % 16) == 0 && ((uintptr_t)d->output % 16) == 0) {
         const long long items = p.total / 16;
-        resize_nearest_vec16_kernel<<<(unsigned)min((items + 255) / 256, (long long)num_sms() * 32), 256, 0, (cudaStream_t)stream>>>(p);
+        launch_mover(resize_nearest_vec16_kernel, dim3((unsigned)min((items + 255) / 256, (long long)num_sms() * 32)), dim3(256), 0, (cudaStream_t)stream, p);
         count_launch();
         return check_launch("resize");
     }
     long long blocks = min((p.total + 255) / 256, (long long)num_sms() * 32);
-    resize_nearest_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(p);
+    launch_mover(resize_nearest_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, p);
     count_launch();
     return check_launch("resize");
 }
@@ -596,8 +626,11 @@ extern "C" int espdl_b200_resize(const espdl_resize_desc *d, void *stream)
 // Gather along one axis (dl_module_gather.hpp:66-96): rows of `inner` elements picked by index.  A thread moves one
 // unit of the row: 16 bytes when rows and pointers allow it, else one element.
 template <typename U>
-__global__ void __launch_bounds__(256) gather_kernel(const U *in, U *out, const int *indices, int num, long long outer, long long axis, long long inner)
+__global__ void __launch_bounds__(256) gather_kernel(const U *in, U *out, const int *indices, int num, long long outer, long long axis, long long inner, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     const long long total = outer * num * inner;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
         const long long col = t % inner, row = t / inner;
@@ -622,11 +655,11 @@ extern "C" int espdl_b200_gather(const espdl_gather_desc *d, void *stream)
     const unsigned blocks = (unsigned)min((total + 255) / 256, (long long)num_sms() * 32);
     cudaStream_t s = (cudaStream_t)stream;
     switch (es) {
-    case 1: gather_kernel<uint8_t><<<blocks, 256, 0, s>>>((const uint8_t *)d->input, (uint8_t *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
-    case 2: gather_kernel<uint16_t><<<blocks, 256, 0, s>>>((const uint16_t *)d->input, (uint16_t *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
-    case 4: gather_kernel<uint32_t><<<blocks, 256, 0, s>>>((const uint32_t *)d->input, (uint32_t *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
-    case 8: gather_kernel<uint2><<<blocks, 256, 0, s>>>((const uint2 *)d->input, (uint2 *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
-    default: gather_kernel<uint4><<<blocks, 256, 0, s>>>((const uint4 *)d->input, (uint4 *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
+    case 1: launch_mover(gather_kernel<uint8_t>, dim3(blocks), dim3(256), 0, s, (const uint8_t *)d->input, (uint8_t *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
+    case 2: launch_mover(gather_kernel<uint16_t>, dim3(blocks), dim3(256), 0, s, (const uint16_t *)d->input, (uint16_t *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
+    case 4: launch_mover(gather_kernel<uint32_t>, dim3(blocks), dim3(256), 0, s, (const uint32_t *)d->input, (uint32_t *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
+    case 8: launch_mover(gather_kernel<uint2>, dim3(blocks), dim3(256), 0, s, (const uint2 *)d->input, (uint2 *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
+    default: launch_mover(gather_kernel<uint4>, dim3(blocks), dim3(256), 0, s, (const uint4 *)d->input, (uint4 *)d->output, d->indices, d->num_indices, d->outer, d->axis_size, inner); break;
     }
     count_launch();
     return check_launch("gather");
@@ -645,8 +678,11 @@ struct PartsParams {
     long long total; // rows x units per row
 };
 
-__global__ void __launch_bounds__(256) concat_split_kernel(PartsParams p)
+__global__ void __launch_bounds__(256) concat_split_kernel(PartsParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     const int upr = p.start[p.n_parts];
     for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < p.total; u += (long long)gridDim.x * blockDim.x) {
         const long long row = u / upr;
@@ -698,7 +734,7 @@ extern "C" int espdl_b200_concat_split(const espdl_parts_desc *d, void *stream)
     if (p.total == 0)
         return ESPDL_OK;
     const long long blocks = (p.total + 255) / 256;
-    concat_split_kernel<<<(unsigned)min(blocks, (long long)num_sms() * 32), 256, 0, (cudaStream_t)stream>>>(p);
+    launch_mover(concat_split_kernel, dim3((unsigned)min(blocks, (long long)num_sms() * 32)), dim3(256), 0, (cudaStream_t)stream, p);
     count_launch();
     return check_launch("concat_split");
 }
@@ -762,26 +798,26 @@ extern "C" int espdl_b200_copy(const espdl_copy_desc *d, void *stream)
                 for (int k = 0; k < 5 && vec16; k++)
                     if (p.shape[k] > 1 && p.ds[k] % 16 != 0)
                         vec16 = false;
-                copy_transpose_bytes4_kernel<<<grid, 256, 0, s>>>(p, ya, tiles, vec16 ? 1 : 0);
+                launch_mover(copy_transpose_bytes4_kernel, dim3(grid), dim3(256), 0, s, p, ya, tiles, vec16 ? 1 : 0);
             } else if (words && es == 1)
-                copy_transpose_words_kernel<uint8_t><<<grid, 256, 0, s>>>(p, ya, tiles);
+                launch_mover(copy_transpose_words_kernel<uint8_t>, dim3(grid), dim3(256), 0, s, p, ya, tiles);
             else if (words)
-                copy_transpose_words_kernel<uint16_t><<<grid, 256, 0, s>>>(p, ya, tiles);
+                launch_mover(copy_transpose_words_kernel<uint16_t>, dim3(grid), dim3(256), 0, s, p, ya, tiles);
             else if (es == 1)
-                copy_transpose_kernel<uint8_t><<<grid, 256, 0, s>>>(p, ya, tiles);
+                launch_mover(copy_transpose_kernel<uint8_t>, dim3(grid), dim3(256), 0, s, p, ya, tiles);
             else
-                copy_transpose_kernel<uint16_t><<<grid, 256, 0, s>>>(p, ya, tiles);
+                launch_mover(copy_transpose_kernel<uint16_t>, dim3(grid), dim3(256), 0, s, p, ya, tiles);
             count_launch();
             return check_launch("copy");
         }
     }
     long long blocks = min((p.total + 255) / 256, (long long)num_sms() * 32);
     switch (es) {
-    case 1: copy_kernel<uint8_t><<<(unsigned)blocks, 256, 0, s>>>(p); break;
-    case 2: copy_kernel<uint16_t><<<(unsigned)blocks, 256, 0, s>>>(p); break;
-    case 4: copy_kernel<uint32_t><<<(unsigned)blocks, 256, 0, s>>>(p); break;
-    case 8: copy_kernel<uint2><<<(unsigned)blocks, 256, 0, s>>>(p); break;
-    default: copy_kernel<uint4><<<(unsigned)blocks, 256, 0, s>>>(p); break;
+    case 1: launch_mover(copy_kernel<uint8_t>, dim3((unsigned)blocks), dim3(256), 0, s, p); break;
+    case 2: launch_mover(copy_kernel<uint16_t>, dim3((unsigned)blocks), dim3(256), 0, s, p); break;
+    case 4: launch_mover(copy_kernel<uint32_t>, dim3((unsigned)blocks), dim3(256), 0, s, p); break;
+    case 8: launch_mover(copy_kernel<uint2>, dim3((unsigned)blocks), dim3(256), 0, s, p); break;
+    default: launch_mover(copy_kernel<uint4>, dim3((unsigned)blocks), dim3(256), 0, s, p); break;
     }
     count_launch();
     return check_launch("copy");

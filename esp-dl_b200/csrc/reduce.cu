@@ -123,8 +123,11 @@ __device__ __forceinline__ ACC fold_start(Fold f)
 }
 
 template <typename T, typename ACC>
-__global__ void __launch_bounds__(256) reduce_kernel(ReduceParams p)
+__global__ void __launch_bounds__(256) reduce_kernel(ReduceParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     const T *in = (const T *)p.in;
     T *out = (T *)p.out;
     const int lo = sizeof(T) == 1 ? -128 : -32768, hi = sizeof(T) == 1 ? 127 : 32767;
@@ -199,7 +202,7 @@ __device__ __forceinline__ void fold_vector(ACC (&acc)[V], const T *v)
 }
 
 template <typename T, int V, typename ACC, Fold F>
-__global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int C, int slice_lanes, int slices, int rows)
+__global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int C, int slice_lanes, int slices, int rows, int early)
 {
     namespace cg = cooperative_groups;
     __shared__ ACC part[V * 256]; // [channel of the lane][thread]: consecutive threads in consecutive words
@@ -215,7 +218,8 @@ __global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int
     ACC acc[V];
 #pragma unroll
     for (int j = 0; j < V; j++) acc[j] = start;
-    grid_dep_launch();
+    if (early)
+        grid_dep_launch();
     grid_dep_wait();
     if (active) {
         struct alignas(V * sizeof(T)) Vec {
@@ -292,11 +296,11 @@ int launch_channel_reduce(const ReduceParams &p, long long outer, int C, cudaStr
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = pdl_enabled() ? 2 : 1;
     switch (fold_of(p.op)) {
-    case FOLD_SUM: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SUM>, p, C, slice_lanes, slices, rows); break;
-    case FOLD_MAX: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MAX>, p, C, slice_lanes, slices, rows); break;
-    case FOLD_MIN: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MIN>, p, C, slice_lanes, slices, rows); break;
-    case FOLD_ABS: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_ABS>, p, C, slice_lanes, slices, rows); break;
-    case FOLD_SQUARE: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SQUARE>, p, C, slice_lanes, slices, rows); break;
+    case FOLD_SUM: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SUM>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
+    case FOLD_MAX: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MAX>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
+    case FOLD_MIN: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MIN>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
+    case FOLD_ABS: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_ABS>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
+    case FOLD_SQUARE: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SQUARE>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
     }
     count_launch();
     return check_launch("channel reduce");
@@ -384,9 +388,9 @@ int reduce_op(const espdl_reduce_desc &d, cudaStream_t s)
     const long long blocks = (p.outputs + 255) / 256;
     const int grid = (int)(blocks < (long long)num_sms() * 8 ? blocks : (long long)num_sms() * 8);
     if (d.dtype == ESPDL_DTYPE_INT8)
-        reduce_kernel<int8_t, int32_t><<<grid, 256, 0, s>>>(p);
+        launch_mover(reduce_kernel<int8_t, int32_t>, dim3(grid), dim3(256), 0, s, p);
     else
-        reduce_kernel<int16_t, long long><<<grid, 256, 0, s>>>(p);
+        launch_mover(reduce_kernel<int16_t, long long>, dim3(grid), dim3(256), 0, s, p);
     count_launch();
     return check_launch("reduce");
 }
@@ -407,8 +411,11 @@ struct PadParams {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256) pad_kernel(PadParams p)
+__global__ void __launch_bounds__(256) pad_kernel(PadParams p, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     const T *in = (const T *)p.in;
     T *out = (T *)p.out;
     for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < p.total; o += (long long)gridDim.x * blockDim.x) {
@@ -457,11 +464,11 @@ int pad_op(const espdl_pad_desc &d, cudaStream_t s)
     const long long blocks = (p.total + 255) / 256;
     const int grid = (int)(blocks < (long long)num_sms() * 16 ? blocks : (long long)num_sms() * 16);
     if (d.elem_size == 1)
-        pad_kernel<int8_t><<<grid, 256, 0, s>>>(p);
+        launch_mover(pad_kernel<int8_t>, dim3(grid), dim3(256), 0, s, p);
     else if (d.elem_size == 2)
-        pad_kernel<int16_t><<<grid, 256, 0, s>>>(p);
+        launch_mover(pad_kernel<int16_t>, dim3(grid), dim3(256), 0, s, p);
     else
-        pad_kernel<int32_t><<<grid, 256, 0, s>>>(p);
+        launch_mover(pad_kernel<int32_t>, dim3(grid), dim3(256), 0, s, p);
     count_launch();
     return check_launch("pad");
 }

@@ -15,8 +15,11 @@ namespace {
 // different orders: along the last axis y = round(x * (inv_norm * 2^-e_out)), along any other axis
 // y = round((x * inv_norm) * 2^-e_out).
 template <typename T>
-__global__ void __launch_bounds__(128) lp_norm_kernel(const T *in, T *out, long long rows, int len, long long inner, int p, float out_rescale, int half_even)
+__global__ void __launch_bounds__(128) lp_norm_kernel(const T *in, T *out, long long rows, int len, long long inner, int p, float out_rescale, int half_even, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows; r += (long long)gridDim.x * blockDim.x) {
         const long long base = (r / inner) * (long long)len * inner + (r % inner);
         float inv_norm;
@@ -51,8 +54,11 @@ __global__ void __launch_bounds__(128) lp_norm_kernel(const T *in, T *out, long 
 // ------------------------------------------------------------------------------------------ ReverseSequence
 template <typename T>
 __global__ void __launch_bounds__(256) reverse_sequence_kernel(const T *in, T *out, const long long *seq_lens, int batch_axis, int dim0, int dim1,
-                                                               long long feature, long long total)
+                                                               long long feature, long long total, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long f = i % feature;
         const long long r = i / feature;
@@ -91,8 +97,11 @@ __device__ __forceinline__ T scatter_apply(T cur, T upd, int reduction)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) scatter_nd_kernel(espdl_scatter_nd_desc d)
+__global__ void __launch_bounds__(256) scatter_nd_kernel(espdl_scatter_nd_desc d, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     T *out = (T *)d.output;
     const T *upd = (const T *)d.updates;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < d.slice_size; e += (long long)gridDim.x * blockDim.x) {
@@ -116,9 +125,9 @@ int lp_norm_op(const espdl_norm_desc &d, cudaStream_t s)
     const unsigned grid = (unsigned)min(blocks, (long long)num_sms() * 16);
     const int he = d.round_mode == ESPDL_ROUND_HALF_EVEN;
     if (d.dtype == ESPDL_DTYPE_INT8)
-        lp_norm_kernel<int8_t><<<grid, 128, 0, s>>>((const int8_t *)d.input, (int8_t *)d.output, d.rows, d.len, d.inner, d.p, dl_rescale(d.out_exponent), he);
+        launch_mover(lp_norm_kernel<int8_t>, dim3(grid), dim3(128), 0, s, (const int8_t *)d.input, (int8_t *)d.output, d.rows, d.len, d.inner, d.p, dl_rescale(d.out_exponent), he);
     else
-        lp_norm_kernel<int16_t><<<grid, 128, 0, s>>>((const int16_t *)d.input, (int16_t *)d.output, d.rows, d.len, d.inner, d.p, dl_rescale(d.out_exponent), he);
+        launch_mover(lp_norm_kernel<int16_t>, dim3(grid), dim3(128), 0, s, (const int16_t *)d.input, (int16_t *)d.output, d.rows, d.len, d.inner, d.p, dl_rescale(d.out_exponent), he);
     count_launch();
     return check_launch("lp_norm");
 }
@@ -139,11 +148,11 @@ extern "C" int espdl_b200_reverse_sequence(const espdl_reverse_sequence_desc *d,
     cudaStream_t s = (cudaStream_t)stream;
     const long long *lens = (const long long *)d->seq_lens;
     if (d->elem_size == 1)
-        reverse_sequence_kernel<int8_t><<<grid, 256, 0, s>>>((const int8_t *)d->input, (int8_t *)d->output, lens, d->batch_axis, d->dim0, d->dim1, d->feature, total);
+        launch_mover(reverse_sequence_kernel<int8_t>, dim3(grid), dim3(256), 0, s, (const int8_t *)d->input, (int8_t *)d->output, lens, d->batch_axis, d->dim0, d->dim1, d->feature, total);
     else if (d->elem_size == 2)
-        reverse_sequence_kernel<int16_t><<<grid, 256, 0, s>>>((const int16_t *)d->input, (int16_t *)d->output, lens, d->batch_axis, d->dim0, d->dim1, d->feature, total);
+        launch_mover(reverse_sequence_kernel<int16_t>, dim3(grid), dim3(256), 0, s, (const int16_t *)d->input, (int16_t *)d->output, lens, d->batch_axis, d->dim0, d->dim1, d->feature, total);
     else
-        reverse_sequence_kernel<int32_t><<<grid, 256, 0, s>>>((const int32_t *)d->input, (int32_t *)d->output, lens, d->batch_axis, d->dim0, d->dim1, d->feature, total);
+        launch_mover(reverse_sequence_kernel<int32_t>, dim3(grid), dim3(256), 0, s, (const int32_t *)d->input, (int32_t *)d->output, lens, d->batch_axis, d->dim0, d->dim1, d->feature, total);
     count_launch();
     return check_launch("reverse_sequence");
 }
@@ -165,11 +174,11 @@ extern "C" int espdl_b200_scatter_nd(const espdl_scatter_nd_desc *d, void *strea
         return ESPDL_OK;
     const unsigned grid = (unsigned)min((long long)((d->slice_size + 255) / 256), (long long)num_sms() * 8);
     if (d->dtype == ESPDL_DTYPE_INT8)
-        scatter_nd_kernel<int8_t><<<grid, 256, 0, s>>>(*d);
+        launch_mover(scatter_nd_kernel<int8_t>, dim3(grid), dim3(256), 0, s, *d);
     else if (d->dtype == ESPDL_DTYPE_INT16)
-        scatter_nd_kernel<int16_t><<<grid, 256, 0, s>>>(*d);
+        launch_mover(scatter_nd_kernel<int16_t>, dim3(grid), dim3(256), 0, s, *d);
     else
-        scatter_nd_kernel<float><<<grid, 256, 0, s>>>(*d);
+        launch_mover(scatter_nd_kernel<float>, dim3(grid), dim3(256), 0, s, *d);
     count_launch();
     return check_launch("scatter_nd");
 }

@@ -11,8 +11,11 @@
 
 namespace espdl {
 
-__global__ void __launch_bounds__(128) softmax_kernel(espdl_softmax_desc d, float out_rescale)
+__global__ void __launch_bounds__(128) softmax_kernel(espdl_softmax_desc d, float out_rescale, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     __shared__ float table[256];
     __shared__ float sum_s;
     extern __shared__ int8_t row[];
@@ -50,8 +53,11 @@ __global__ void __launch_bounds__(128) softmax_kernel(espdl_softmax_desc d, floa
 // words, so that thread r reading byte i of row r meets no bank conflict), thread r adds row r's exponentials in index
 // order - R ordered sums run at once instead of one -, then all threads write the R x len results.  Used whenever at
 // least 32 rows fit into shared memory; the kernel above keeps the long rows.
-__global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d, float out_rescale, int R, int pitch)
+__global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d, float out_rescale, int R, int pitch, int early)
 {
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
     __shared__ float table[256];
     extern __shared__ __align__(16) unsigned char sm[];
     float *sums = (float *)sm;               // R
@@ -169,12 +175,12 @@ extern "C" int espdl_b200_softmax(const espdl_softmax_desc *d, void *stream)
     if (fit >= 32 && d->rows >= 64) {
         const int R = min(256, fit);
         const int groups = (d->rows + R - 1) / R;
-        softmax_rows_kernel<<<min(groups, num_sms() * 8), 256, (size_t)R * (pitch + 4) + 16, (cudaStream_t)stream>>>(*d, dl_rescale(d->out_exponent), R, pitch);
+        launch_mover(softmax_rows_kernel, dim3(min(groups, num_sms() * 8)), dim3(256), (size_t)R * (pitch + 4) + 16, (cudaStream_t)stream, *d, dl_rescale(d->out_exponent), R, pitch);
         count_launch();
         return check_launch("softmax_rows");
     }
     const int blocks = min(d->rows, num_sms() * 16);
-    softmax_kernel<<<blocks, 128, (size_t)((d->len + 15) & ~15), (cudaStream_t)stream>>>(*d, dl_rescale(d->out_exponent));
+    launch_mover(softmax_kernel, dim3(blocks), dim3(128), (size_t)((d->len + 15) & ~15), (cudaStream_t)stream, *d, dl_rescale(d->out_exponent));
     count_launch();
     return check_launch("softmax");
 }

@@ -123,9 +123,13 @@ stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
     const uint32_t tmem_base = *tmem_slot;
     (void)b_bytes;
 
+    if (threadIdx.x == 0)
+        grid_dep_launch(); // set up: the next kernel's CTAs may take SMs as they become free
+
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
+            grid_dep_wait(); // the previous kernel's output, before the first load; the other roles act on what the producer brought in
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -415,7 +419,7 @@ int conv2d_stem_tc(const espdl_conv_desc &d, cudaStream_t s)
     const int total = p.ngroups * p.yblocks * p.segs;
     const int grid = min(total, num_sms());
     const auto kernel = p.epi.half_even ? stem_tc_kernel<true> : stem_tc_kernel<false>;
-    kernel<<<grid, ST_THREADS, max(smem, (size_t)120 * 1024), s>>>(maps[0], maps[1], maps[2], mo, p);
+    launch_overlapped(kernel, dim3(grid), dim3(ST_THREADS), max(smem, (size_t)120 * 1024), s, maps[0], maps[1], maps[2], mo, p);
     count_launch();
     return check_launch("stem_tc");
 }

@@ -905,14 +905,13 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
 esp_err_t Model::execute(int first, int last)
 {
     ModelContext *ctx = m_model_context;
-    for (int i = first; i < last; i++) {
-        m_execution_plan[i]->forward(ctx, RUNTIME_MODE_SINGLE_CORE);
-        if (ctx->status) {
-            m_status = ctx->status;
-            return ESP_FAIL;
-        }
-    }
-    return ESP_OK;
+    espdl_b200_model_scope(1); // the plan's parameters are constants
+    for (int i = first; i < last && !ctx->status; i++) m_execution_plan[i]->forward(ctx, RUNTIME_MODE_SINGLE_CORE);
+    espdl_b200_model_scope(0);
+    if (!ctx->status)
+        return ESP_OK;
+    m_status = ctx->status;
+    return ESP_FAIL;
 }
 
 esp_err_t Model::run_device(bool sync)

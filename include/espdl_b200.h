@@ -108,6 +108,10 @@ int espdl_b200_graph_begin(void *stream);                 /* start capturing wor
 int espdl_b200_graph_end(void *stream, void **graph);     /* stop capturing, instantiate                 */
 int espdl_b200_graph_launch(void *graph, void *stream);
 int espdl_b200_graph_destroy(void *graph);
+/* Between espdl_b200_model_scope(1) and espdl_b200_model_scope(0) the calling thread promises that no launch writes what a
+ * later launch takes as filter, bias or exponents (the plan of a model: parameters are constants).  Kernels then overlap their
+ * start with the end of the kernel before them more widely.  Nests. */
+void espdl_b200_model_scope(int enter);
 
 /* ------------------------------------------------------------ convolution */
 /*
