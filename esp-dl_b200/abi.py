@@ -212,6 +212,7 @@ SYMBOLS = {
     "espdl_b200_graph_launch": (C.c_int, [C.c_void_p, C.c_void_p]),
     "espdl_b200_graph_destroy": (C.c_int, [C.c_void_p]),
     "espdl_b200_model_scope": (None, [C.c_int]),
+    "espdl_b200_overlap": (None, [C.c_int]),
     "espdl_b200_conv2d": (C.c_int, [C.POINTER(ConvDesc), C.c_void_p]),
     "espdl_b200_conv2d_workspace_bytes": (C.c_int, [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]),
     "espdl_b200_conv2d_ws": (C.c_int, [C.POINTER(ConvDesc), C.c_void_p, C.c_size_t, C.c_void_p]),

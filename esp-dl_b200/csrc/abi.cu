@@ -6,7 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <unordered_map>
+#include <map>
 
 namespace espdl {
 
@@ -46,7 +46,7 @@ __device__ unsigned g_sched_words[2 * SCHED_PAIRS]; // zero at load; every kerne
 unsigned *sched_counters(cudaStream_t s)
 {
     static std::mutex mu;
-    static std::unordered_map<unsigned long long, int> pair_of; // stream handle / capture id -> pair
+    static std::map<std::pair<unsigned long long, cudaStream_t>, int> pair_of; // (capture id or 0, stream) -> pair
     static unsigned *base = nullptr;
     static const bool off = getenv("ESPDL_B200_STATIC_TILES") != nullptr;
     if (off)
@@ -57,8 +57,8 @@ unsigned *sched_counters(cudaStream_t s)
         cudaGetLastError();
         return nullptr;
     }
-    // keys: capture ids count up from 1 and stay far below 2^48; stream handles are pointers (or the small legacy values)
-    const unsigned long long key = cs == cudaStreamCaptureStatusActive ? (id | (1ull << 63)) : (unsigned long long)(uintptr_t)s;
+    // branches of one graph are captured on streams of their own and may run side by side
+    const std::pair<unsigned long long, cudaStream_t> key(cs == cudaStreamCaptureStatusActive ? id : 0ull, s);
     std::lock_guard<std::mutex> lock(mu);
     if (!base) {
         void *p = nullptr;
@@ -201,17 +201,19 @@ int espdl_b200_download(void *dst_host, const void *src_dev, size_t bytes, void 
 } // extern "C"
 namespace espdl {
 static thread_local int g_model_scope = 0;
+static thread_local bool g_overlap = true;
 bool in_model_scope() { return g_model_scope > 0; }
 
 bool pdl_enabled()
 {
     static const bool on = !getenv("ESPDL_B200_NO_PDL");
-    return on;
+    return on && g_overlap;
 }
 } // namespace espdl
 extern "C" {
 
 void espdl_b200_model_scope(int enter) { g_model_scope += enter ? 1 : -1; }
+void espdl_b200_overlap(int on) { g_overlap = on != 0; }
 
 int espdl_b200_download_rows(void *dst_host, const void *src_dev, size_t row_bytes, size_t src_stride_bytes, size_t rows, void *stream)
 {

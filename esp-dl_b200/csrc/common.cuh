@@ -15,9 +15,9 @@ int set_error_text(int status, const char *fmt, ...); // records text for espdl_
 void count_launch(int n = 1);
 int num_sms();
 // Work counters of a persistent kernel that hands out its tiles dynamically: two zero-initialised words {next tile,
-// CTAs done} in device memory that no other launch in flight uses - one pair per stream, or per capture sequence while
-// `s` is being captured into a graph (launches of one stream, and the nodes of one graph, run one after the other; two
-// graphs may run side by side).  The kernel's last CTA writes both words back to zero.  Null when no pair is left: the
+// CTAs done} in device memory that no other launch in flight uses - one pair per stream, or per stream and capture sequence
+// while `s` is being captured into a graph (launches of one stream, and the nodes captured on one stream, run one after
+// the other; two graphs, and the branches of one, may run side by side).  The kernel's last CTA writes both words back to zero.  Null when no pair is left: the
 // kernel then walks its tiles in the fixed order.
 unsigned *sched_counters(cudaStream_t s);
 int lp_norm_op(const espdl_norm_desc &d, cudaStream_t s); // sequence_ops.cu

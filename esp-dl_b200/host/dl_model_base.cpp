@@ -117,6 +117,8 @@ static void download_dense(void *host, TensorBase *t, void *stream)
 }
 
 // ----------------------------------------------------------------------------- model
+static constexpr size_t BRANCH_LIMIT = (size_t)1 << 30; // bytes of all tensors of a pass up to which its branches run side by side
+
 static bool env_flag(const char *name, bool def)
 {
     const char *v = getenv(name);
@@ -185,7 +187,11 @@ void Model::release()
         espdl_b200_graph_destroy(m_graph_head);
     if (m_graph_tail)
         espdl_b200_graph_destroy(m_graph_tail);
-    m_graph = m_graph_head = m_graph_tail = nullptr;
+    if (m_graph_io)
+        espdl_b200_graph_destroy(m_graph_io);
+    m_graph = m_graph_head = m_graph_tail = m_graph_io = nullptr;
+    for (void *stream : m_branch_streams) espdl_b200_stream_destroy(stream);
+    m_branch_streams.clear();
     for (auto *m : m_execution_plan) delete m;
     m_execution_plan.clear();
     if (m_model_context) {
@@ -838,7 +844,34 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
             }
         }
     }
-    m_arena_bytes = MemoryManagerGreedy::plan(infos, m_reuse_memory);
+    // Branches side by side (dl_model_capture.cpp) where the plan is wider than a chain: every tensor then has a buffer of its
+    // own, since a shared one would order the branches again.  Measured per pass, chain -> branches: re-identification of 1 / 27 /
+    // 128 crops 800 -> 418, 972 -> 627, 1673 -> 1353 us; 320x320 detector, 1 / 64 images 704 -> 547, 4449 -> 3708 us; 640x640,
+    // 32 images 1399 -> 1359 us.  The gain fades as launches fill the GPU while the buffers grow six-fold, hence the limit.
+    if (m_reuse_memory && m_use_graph && !m_plan_only && env_flag("ESPDL_B200_BRANCHES", true)) {
+        std::map<std::string, int> depth;
+        int longest = 0;
+        for (size_t step = 0; step < m_execution_plan.size(); step++) {
+            int d = 0;
+            for (const std::string &in : m_module_inputs[step]) {
+                auto it = depth.find(in);
+                d = std::max(d, it == depth.end() ? 0 : it->second);
+            }
+            for (const std::string &out : m_module_outputs[step]) depth[out] = d + 1;
+            longest = std::max(longest, d + 1);
+        }
+        const char *mb = getenv("ESPDL_B200_BRANCH_MB");
+        const size_t limit = mb ? (size_t)atoi(mb) << 20 : BRANCH_LIMIT;
+        std::vector<TensorInfo> apart = infos;
+        const size_t bytes = MemoryManagerGreedy::plan(apart, false);
+        if (longest * 10 < (int)m_execution_plan.size() * 9 && bytes <= limit) {
+            infos = apart;
+            m_arena_bytes = bytes;
+            m_branches = true;
+        }
+    }
+    if (!m_branches)
+        m_arena_bytes = MemoryManagerGreedy::plan(infos, m_reuse_memory);
     // the last step that reads a graph input's buffer (directly, or through a view / slice that lives in it)
     m_input_steps = 0;
     for (size_t i = 0; i < infos.size(); i++) {
@@ -914,6 +947,25 @@ esp_err_t Model::execute(int first, int last)
     return ESP_FAIL;
 }
 
+// One plain pass before the first capture settles lazily created state (tables, cached attributes).
+esp_err_t Model::settle()
+{
+    if (m_settled)
+        return ESP_OK;
+    if (execute(0, (int)m_execution_plan.size()) != ESP_OK || espdl_b200_stream_sync(m_model_context->stream) != ESPDL_OK)
+        return ESP_FAIL;
+    m_settled = true;
+    return ESP_OK;
+}
+
+std::vector<const void *> Model::io_buffers()
+{
+    std::vector<const void *> v;
+    for (auto &kv : m_inputs) v.push_back(kv.second->data);
+    for (auto &kv : m_outputs) v.push_back(kv.second->data);
+    return v;
+}
+
 esp_err_t Model::run_device(bool sync)
 {
     if (!m_built)
@@ -921,22 +973,8 @@ esp_err_t Model::run_device(bool sync)
     ModelContext *ctx = m_model_context;
     int st = ESPDL_OK;
     if (m_use_graph) {
-        if (!m_graph) {
-            // one plain pass first (it also settles lazily created state), then capture the same launches
-            if (execute(0, (int)m_execution_plan.size()) != ESP_OK || espdl_b200_stream_sync(ctx->stream) != ESPDL_OK)
-                return ESP_FAIL;
-            st = espdl_b200_graph_begin(ctx->stream);
-            if (!st) {
-                esp_err_t e = execute(0, (int)m_execution_plan.size());
-                st = espdl_b200_graph_end(ctx->stream, &m_graph);
-                if (e != ESP_OK)
-                    st = m_status;
-            }
-            if (st) {
-                m_status = st;
-                return ESP_FAIL;
-            }
-        }
+        if (!m_graph && (settle() != ESP_OK || capture_plan(0, (int)m_execution_plan.size(), false, &m_graph) != ESP_OK))
+            return ESP_FAIL;
         st = espdl_b200_graph_launch(m_graph, ctx->stream);
     } else if (execute(0, (int)m_execution_plan.size()) != ESP_OK) {
         return ESP_FAIL;
@@ -960,15 +998,8 @@ esp_err_t Model::run_part(bool head)
         return execute(first, last);
     void *&graph = head ? m_graph_head : m_graph_tail;
     int st = ESPDL_OK;
-    if (!graph) {
-        st = espdl_b200_graph_begin(ctx->stream);
-        if (!st) {
-            esp_err_t e = execute(first, last);
-            st = espdl_b200_graph_end(ctx->stream, &graph);
-            if (e != ESP_OK)
-                st = m_status ? m_status : ESPDL_ERR_CUDA;
-        }
-    }
+    if (!graph && capture_plan(first, last, false, &graph) != ESP_OK)
+        return ESP_FAIL;
     if (!st)
         st = espdl_b200_graph_launch(graph, ctx->stream);
     if (st)
@@ -982,9 +1013,28 @@ void Model::run(runtime_mode_t mode)
     if (!m_built)
         return;
     ModelContext *ctx = m_model_context;
-    for (auto &kv : m_inputs)
-        if (kv.second->data)
-            espdl_b200_upload(kv.second->device, kv.second->data, kv.second->get_bytes(), ctx->stream);
+    auto upload = [&] {
+        for (auto &kv : m_inputs)
+            if (kv.second->data)
+                espdl_b200_upload(kv.second->device, kv.second->data, kv.second->get_bytes(), ctx->stream);
+    };
+    // The copies are nodes of the graph: one launch for the whole pass, and with branches each output leaves when it is ready.  (A
+    // graph keeps the addresses it was captured with; a caller that moved a tensor's host buffer gets the plain form.)
+    if (m_use_graph && (!m_graph_io || m_graph_io_buffers == io_buffers())) {
+        if (!m_graph_io) {
+            upload();
+            m_graph_io_buffers = io_buffers();
+            if (settle() != ESP_OK || capture_plan(0, (int)m_execution_plan.size(), true, &m_graph_io) != ESP_OK)
+                return;
+        }
+        int st = espdl_b200_graph_launch(m_graph_io, ctx->stream);
+        if (!st)
+            st = espdl_b200_stream_sync(ctx->stream);
+        if (st)
+            m_status = st;
+        return;
+    }
+    upload();
     if (run_device(false) != ESP_OK)
         return;
     for (auto &kv : m_outputs)

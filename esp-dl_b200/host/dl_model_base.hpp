@@ -138,6 +138,16 @@ protected:
     void *m_arena = nullptr;
     size_t m_arena_bytes = 0;
     void *m_graph = nullptr;
+    void *m_graph_io = nullptr;                    ///< the plan with the copies of inputs and outputs: run()
+    std::vector<const void *> m_graph_io_buffers;  ///< the host buffers it was captured with
+    bool m_settled = false;                        ///< one plain pass has run: lazily created state exists
+    // Branches of the plan side by side in its graphs (dl_model_capture.cpp)
+    static constexpr int MAX_BRANCHES = 6;
+    bool m_branches = false;
+    std::vector<void *> m_branch_streams;
+    esp_err_t settle();
+    esp_err_t capture_plan(int first, int last, bool io, void **graph);
+    std::vector<const void *> io_buffers();
     // Pipelined passes (submit / wait) run the plan in two parts: the steps that read a graph input, then the rest.  Once the
     // first part of a pass is done its input buffers are free again, so the next pass's upload goes straight into them while
     // the second part runs - no staging copy.  m_input_steps = number of leading steps that belong to the first part.

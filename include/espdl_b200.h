@@ -112,6 +112,9 @@ int espdl_b200_graph_destroy(void *graph);
  * later launch takes as filter, bias or exponents (the plan of a model: parameters are constants).  Kernels then overlap their
  * start with the end of the kernel before them more widely.  Nests. */
 void espdl_b200_model_scope(int enter);
+/* 0: the calling thread's following launches start only when everything before them is done (no overlap of a kernel's start with
+ * the end of the one before it), 1: the default again.  For launches that join several streams of a capture. */
+void espdl_b200_overlap(int on);
 
 /* ------------------------------------------------------------ convolution */
 /*
