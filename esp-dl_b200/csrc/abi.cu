@@ -436,6 +436,13 @@ int espdl::conv_validate(const espdl_conv_desc *d)
     return ESPDL_OK;
 }
 
+// Shapes no kernel reads in place, large enough for packed operands to pay (a caller without the scratch gets the CUDA-core kernel).
+static bool runs_packed(const espdl_conv_desc &d)
+{
+    return d.kernel == ESPDL_KERNEL_AUTO && d.n > 0 && !conv2d_stem_tc_supported(d) && !conv2d_band_tc_supported(d) && !conv2d_conv_tc_supported(d) &&
+        !conv2d_tc_supported(d) && conv2d_packed_supported(d);
+}
+
 extern "C" {
 
 int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes)
@@ -446,8 +453,12 @@ int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes
     int st = conv_validate(desc);
     if (st)
         return st;
-    if (desc->kernel != ESPDL_KERNEL_SIMT && desc->group == 1 && conv2d_tc_supported(*desc))
+    if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1)
+        return ESPDL_OK;
+    if (conv2d_tc_supported(*desc))
         *bytes = conv2d_tc_workspace_bytes(*desc);
+    else if (runs_packed(*desc))
+        *bytes = conv2d_packed_workspace_bytes(*desc);
     return ESPDL_OK;
 }
 
@@ -483,25 +494,7 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
             return conv2d_tc(*desc, workspace, workspace_bytes, s);
         if (desc->kernel == ESPDL_KERNEL_TCGEN05)
             return ESPDL_ERR_UNSUPPORTED;
-        // 3x3 int8 with 16-byte channel runs: the TMA-fed kernel; ESPDL_KERNEL_SIMT asks for the kernels that read global
-        // memory directly
-        if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_dw_tma_supported(*desc))
-            return conv2d_dw_tma(*desc, s);
-        // shapes the tile kernel does not take: one call per image
-        const size_t es = desc->dtype == ESPDL_DTYPE_INT16 ? 2 : 1;
-        const long long ips = desc->in_pixel_stride ? desc->in_pixel_stride : desc->in_c;
-        const long long ops = desc->out_pixel_stride ? desc->out_pixel_stride : desc->out_c;
-        for (int i = 0; i < desc->n; i++) {
-            espdl_conv_desc one = *desc;
-            one.n = 1, one.filter_image_stride = 0;
-            one.input = (const char *)desc->input + (size_t)i * desc->in_h * desc->in_w * ips * es;
-            one.filter = (const char *)desc->filter + (size_t)i * desc->filter_image_stride * es;
-            one.output = (char *)desc->output + (size_t)i * desc->out_h * desc->out_w * ops * es;
-            const int st1 = espdl_b200_conv2d_ws(&one, workspace, workspace_bytes, stream);
-            if (st1)
-                return st1;
-        }
-        return ESPDL_OK;
+        return conv2d_simt(*desc, s); // all products in one launch (one per image: 128 launches, 1.5 ms, for the attention of 64 images)
     }
     if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_band_tc_supported(*desc))
         return conv2d_band_tc(*desc, s); // 3x3 with 8 or 16 input channels: banded filter over 128-byte row windows
@@ -517,6 +510,8 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
             return ESPDL_ERR_INVALID_ARG;
         return conv2d_tc(*desc, workspace, workspace_bytes, s);
     }
+    if (runs_packed(*desc) && workspace && workspace_bytes >= conv2d_packed_workspace_bytes(*desc))
+        return conv2d_packed(*desc, workspace, workspace_bytes, s);
     return conv2d_simt(*desc, s);
 }
 

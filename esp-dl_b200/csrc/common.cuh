@@ -82,7 +82,20 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s);
 bool conv2d_tc_supported(const espdl_conv_desc &d);
 size_t conv2d_tc_workspace_bytes(const espdl_conv_desc &d);
 int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s, const long long *peer_delta = nullptr,
-              int n_peer = 0); // peer_delta: byte distances to copies of the output on other GPUs that receive every row as well
+              int n_peer = 0, int *row_sums = nullptr); // peer_delta: byte distances to copies of the output on other GPUs that receive every row as well
+// Packed operands of the tile kernel (pack.cu): rows of Kp bytes, Kp a multiple of 16; int16 operands as two planes.
+struct PackedOperands {
+    void *a_hi, *a_lo, *b_hi, *b_lo;
+    int *row_sum; // int16: sum of every row of A
+    int Kp;
+};
+// Packs output pixels [row0, row0 + rows) and, with `filter`, the filter.
+int pack_operands(const espdl_conv_desc &d, long long row0, int rows, bool filter, const PackedOperands &o, cudaStream_t s);
+// Convs and products that run on the tile kernel once their operands are packed: reductions that are no multiple of 16, int16
+// windows, channel counts that are no multiple of 16.
+bool conv2d_packed_supported(const espdl_conv_desc &d);
+size_t conv2d_packed_workspace_bytes(const espdl_conv_desc &d);
+int conv2d_packed(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s);
 // Each translation unit with bounded device-side waits keeps the address of ONE status word in pinned, device-mapped host
 // memory: a wait that runs out stores ESPDL_ERR_TIMEOUT there, and espdl_b200_stream_sync reads it as ordinary memory.
 // (A device word per unit, copied back at every synchronisation, cost seven blocking copies: 60 us of a 160 us pass.)

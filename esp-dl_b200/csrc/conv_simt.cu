@@ -24,6 +24,7 @@ struct ConvParams {
     int ew_scalar, per_channel, relu, half_even;
     long long total; // number of (pixel, oc-group) work items
     int groups;      // oc groups per pixel
+    long long w_image; // elements between the filters of consecutive images (a batch of products), 0 = one filter
 };
 
 template <int OCT, bool DP4A>
@@ -56,7 +57,7 @@ __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
                 if (ix < 0 || ix >= p.iw)
                     continue;
                 const int8_t *ip = in + (((long long)n * p.ih + iy) * p.iw + ix) * p.ips;
-                const int8_t *wp = w + (long long)oc0 * wstride + ((long long)ky * p.kw + kx) * p.ic;
+                const int8_t *wp = w + n * p.w_image + (long long)oc0 * wstride + ((long long)ky * p.kw + kx) * p.ic;
                 if (DP4A) {
                     const int *ip4 = (const int *)ip;
                     for (int c = 0; c < p.ic / 4; c++) {
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(256) conv_s16_kernel(ConvParams p)
                 if (ix < 0 || ix >= p.iw)
                     continue;
                 const int16_t *ip = in + (((long long)n * p.ih + iy) * p.iw + ix) * p.ips;
-                const int16_t *wp = w + (long long)oc0 * wstride + ((long long)ky * p.kw + kx) * p.ic;
+                const int16_t *wp = w + n * p.w_image + (long long)oc0 * wstride + ((long long)ky * p.kw + kx) * p.ic;
                 for (int c = 0; c < p.ic; c++) {
                     const int a = ip[c];
 #pragma unroll
@@ -249,6 +250,7 @@ int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
     p.n = d.n, p.ih = d.in_h, p.iw = d.in_w, p.ic = d.in_c, p.oh = d.out_h, p.ow = d.out_w, p.oc = d.out_c;
     p.kh = d.kh, p.kw = d.kw, p.sh = d.stride_h, p.sw = d.stride_w, p.dh = d.dilation_h, p.dw = d.dilation_w;
     p.pt = d.pad_top, p.pl = d.pad_left;
+    p.w_image = d.filter_image_stride;
     p.ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
     p.ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     p.e_shift_base = d.out_exponent - d.in_exponent;
@@ -262,7 +264,7 @@ int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
     const long long max_blocks = (long long)num_sms() * 32;
     if (blocks > max_blocks)
         blocks = max_blocks;
-    if (d.dtype == ESPDL_DTYPE_INT8 && d.out_c <= SMALL_MAX_OC && d.kh == 3 && d.kw == 3 && (d.in_c == 3 || d.in_c == 1 || d.in_c == 4)) {
+    if (d.dtype == ESPDL_DTYPE_INT8 && !d.filter_image_stride && d.out_c <= SMALL_MAX_OC && d.kh == 3 && d.kw == 3 && (d.in_c == 3 || d.in_c == 1 || d.in_c == 4)) {
         const long long pixels = (long long)d.n * d.out_h * d.out_w;
         const unsigned grid = (unsigned)min((pixels + threads - 1) / threads, max_blocks);
         if (d.in_c == 3)
@@ -272,7 +274,7 @@ int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
         else
             launch_overlapped(conv_s8_small_k_kernel<3, 3, 4>, dim3(grid), dim3(threads), 0, s, p);
     } else if (d.dtype == ESPDL_DTYPE_INT8) {
-        const bool dp4a = d.in_c % 4 == 0 && p.ips % 4 == 0 && ((uintptr_t)d.input % 4) == 0 && ((uintptr_t)d.filter % 4) == 0;
+        const bool dp4a = d.in_c % 4 == 0 && p.ips % 4 == 0 && ((uintptr_t)d.input % 4) == 0 && ((uintptr_t)d.filter % 4) == 0 && d.filter_image_stride % 4 == 0;
         if (dp4a)
             launch_overlapped(conv_s8_kernel<OCT, true>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
         else

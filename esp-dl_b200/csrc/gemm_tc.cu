@@ -22,10 +22,13 @@
 //             are staged once in shared memory in a form that needs one add and one shift per output (see
 //             tc_common.cuh), and saturation happens inside the pack instruction.
 //
-// int16 operands: Blackwell tensor cores have no 16-bit integer MMA.  Each operand is split into a signed high byte
-// and an unsigned low byte (x = 256*hi + lo); a pre-pass writes the byte planes to scratch, and the tile kernel
-// accumulates hi*hi, hi*lo + lo*hi and lo*lo in three TMEM accumulators (kind::i8 takes signedness per operand),
-// recombined in 64 bits by the epilogue.  Exact as long as K <= 16384 (the partial sums stay below 2^31).
+// int16 operands: Blackwell tensor cores have no 16-bit integer MMA.  A pre-pass (pack.cu) writes each operand as two byte
+// planes, the input's x = 256*hi + lo (hi signed) and the shifted filter's w + 32768 = 256*uh + ul (both unsigned), and the
+// tile kernel accumulates hi*uh, hi*ul + lo*uh and lo*ul in three neighbouring TMEM accumulators: the filter's planes lie one
+// behind the other in shared memory, so ONE instruction of twice the width multiplies hi by both (into accumulators 0, 1)
+// and one multiplies lo by both (into 1, 2) - an M = 128 instruction costs the same for every width up to 256.  The
+// epilogue recombines in 64 bits and takes off 32768 * (sum of the input row).  Exact as long as K <= 16384 (a partial
+// sum stays below 97,665 * K < 2^31).  4096x1024x1024: see the figures at the launch.
 //
 // Every mbarrier wait is bounded (about two seconds); on expiry the kernel records ESPDL_ERR_TIMEOUT in a device word
 // that espdl_b200_stream_sync reports, and all roles leave.
@@ -84,6 +87,7 @@ struct TcParams {
     int out_mask;   // swizzle mask of the staging tiles (7, 3, 1, 0)
     void *out;
     long long ops;  // output row stride in elements
+    const int *row_sum; // int16: sum of every row of A
     const int8_t *res; // optional residual added to the result (same rows as the output), or null
     long long rps;     // residual row stride in elements
     long long peer_delta[7]; // byte distance from `out` to the same buffer on other GPUs: every result row is stored there too
@@ -351,9 +355,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         (void)w_tempty, (void)w_full, (void)w_issue;
         TC_LAP_INIT;
         const uint32_t idesc_ss = idesc_i8(1, 1, BLOCK_M, p.block_n);
-        const uint32_t idesc_su = idesc_i8(1, 0, BLOCK_M, p.block_n);
-        const uint32_t idesc_us = idesc_i8(0, 1, BLOCK_M, p.block_n);
-        const uint32_t idesc_uu = idesc_i8(0, 0, BLOCK_M, p.block_n);
+        const uint32_t idesc_su = idesc_i8(1, 0, BLOCK_M, 2 * p.block_n), idesc_uu = idesc_i8(0, 0, BLOCK_M, 2 * p.block_n); // int16: both planes
+        const uint32_t idesc_uu1 = idesc_i8(0, 0, BLOCK_M, p.block_n);
         const int ksteps = p.swz / 32;
         const int last_ksteps = (p.K - (p.k_blocks - 1) * p.swz + 31) / 32; // 32-byte K steps of the last block that hold data
         const uint32_t smem_base = smem_u32(smem);
@@ -415,15 +418,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         mma_i8(d0, da + 6, db + 6, idesc_ss, 1u);
                     commit(smem_u32(&empty_bar[stage]));
                 } else {
-                    const uint64_t da_lo = smem_desc_swizzled(st + a_bytes, p.swz);
-                    const uint64_t db_lo = smem_desc_swizzled(st + 2 * a_bytes + b_bytes, p.swz);
+                    const uint64_t da_lo = smem_desc_swizzled(st + a_bytes, p.swz); // the filter's low plane follows its high plane
                     for (int k = 0; k < ks; k++) {
-                        const uint32_t accum = (kb | k) != 0;
                         const uint64_t koff = (uint64_t)(k * 2); // 32 bytes of K, in 16-byte units
-                        mma_i8(d0, da + koff, db + koff, idesc_ss, accum);                      // hi * hi
-                        mma_i8(d0 + p.block_n, da + koff, db_lo + koff, idesc_su, accum);       // hi * lo
-                        mma_i8(d0 + p.block_n, da_lo + koff, db + koff, idesc_us, 1u);          // lo * hi
-                        mma_i8(d0 + 2 * p.block_n, da_lo + koff, db_lo + koff, idesc_uu, accum); // lo * lo
+                        if (kb | k) {
+                            mma_i8(d0, da + koff, db + koff, idesc_su, 1u);                 // hi * (uh | ul)
+                            mma_i8(d0 + p.block_n, da_lo + koff, db + koff, idesc_uu, 1u);  // lo * (uh | ul)
+                        } else { // the first step starts each accumulator once
+                            const uint64_t db_lo = smem_desc_swizzled(st + 2 * a_bytes + b_bytes, p.swz);
+                            mma_i8(d0, da, db, idesc_su, 0u);
+                            mma_i8(d0 + 2 * p.block_n, da_lo, db_lo, idesc_uu1, 0u);
+                            mma_i8(d0 + p.block_n, da_lo, db, idesc_uu1, 1u);
+                        }
                     }
                     commit(smem_u32(&empty_bar[stage]));
                 }
@@ -536,16 +542,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     tie16(vl);
                     if (row_ok && n0 + c0 < p.N) {
                         int16_t *op = (int16_t *)p.out + m * p.ops + n0 + c0;
+                        const long long base = -(long long)p.row_sum[m] * 32768;
+                        uint32_t pk[8];
 #pragma unroll
                         for (int j = 0; j < 16; j++) {
-                            const int n = n0 + c0 + j;
-                            if (n < p.N) {
-                                const long long a = ((long long)vh[j] << 16) + ((long long)vm[j] << 8) + (long long)vl[j];
-                                const int e = p.epi.per_channel ? __ldg(p.epi.ew + n) : p.epi.ew_scalar;
-                                const int shift = max(-62, min(62, p.epi.e_shift_base - e));
-                                const long long b = p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll;
-                                op[j] = (int16_t)requant16(a, b, shift, p.epi.relu, p.epi.half_even);
-                            }
+                            const int n = min(n0 + c0 + j, p.N - 1);
+                            const long long a = base + ((long long)vh[j] << 16) + ((long long)vm[j] << 8) + (long long)vl[j];
+                            const int e = p.epi.per_channel ? __ldg(p.epi.ew + n) : p.epi.ew_scalar;
+                            const int shift = max(-62, min(62, p.epi.e_shift_base - e));
+                            const long long b = p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll;
+                            const uint32_t q = (uint32_t)requant16(a, b, shift, p.epi.relu, p.epi.half_even) & 0xffffu;
+                            pk[j >> 1] = j & 1 ? pk[j >> 1] | (q << 16) : q;
+                        }
+                        if (n0 + c0 + 16 <= p.N && ((uintptr_t)op & 15) == 0) {
+                            *(uint4 *)op = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                            *(uint4 *)(op + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                if (n0 + c0 + j < p.N)
+                                    op[j] = (int16_t)(pk[j >> 1] >> (16 * (j & 1)));
                         }
                     }
                 }
@@ -815,21 +831,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
 }
 
-// int16 [rows][K] (row stride `stride` elements) -> dense byte planes hi (signed) and lo (unsigned).
-__global__ void __launch_bounds__(256) split_limbs_kernel(const int16_t *__restrict__ src, long long stride, int K, long long total,
-                                                          int8_t *__restrict__ hi, uint8_t *__restrict__ lo)
-{
-    grid_dep_launch();
-    grid_dep_wait();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / K;
-        const int k = (int)(i % K);
-        const int v = src[r * stride + k];
-        hi[i] = (int8_t)(v >> 8);
-        lo[i] = (uint8_t)(v & 0xff);
-    }
-}
-
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -1041,10 +1042,17 @@ size_t conv2d_tc_workspace_bytes(const espdl_conv_desc &d)
         return 0;
     const size_t M = (size_t)d.n * d.out_h * d.out_w;
     const size_t a = (M * d.in_c + 255) / 256 * 256, b = ((size_t)d.out_c * d.in_c + 255) / 256 * 256;
-    return 2 * a + 2 * b;
+    return 2 * a + 2 * b + M * sizeof(int);
 }
 
-int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s, const long long *peer_delta, int n_peer)
+namespace {
+
+// Operands already packed: the tile kernel over rows of `o.Kp` bytes.
+int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cudaStream_t s);
+
+} // namespace
+
+int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s, const long long *peer_delta, int n_peer, int *row_sums)
 {
     TcParams p;
     if (n_peer < 0 || n_peer > 7 || (n_peer > 0 && (d.dtype != ESPDL_DTYPE_INT8 || !peer_delta)))
@@ -1054,10 +1062,27 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
     p.n_peer = n_peer;
     p.sched = nullptr, p.static_tiles = 0;
     for (int i = 0; i < 7; i++) p.peer_delta[i] = i < n_peer ? peer_delta[i] : 0;
+    if (d.dtype != ESPDL_DTYPE_INT16)
+        return launch_tc(d, p, nullptr, s);
+    const size_t a = ((size_t)p.M * p.K + 255) / 256 * 256, b = ((size_t)p.N * p.K + 255) / 256 * 256;
+    if (workspace_bytes < 2 * a + 2 * b + (row_sums ? 0 : p.M * sizeof(int)) || !workspace || ((uintptr_t)workspace % 16))
+        return ESPDL_ERR_INVALID_ARG;
+    uint8_t *w = (uint8_t *)workspace;
+    const PackedOperands o = {w, w + a, w + 2 * a, w + 2 * a + b, row_sums ? row_sums : (int *)(w + 2 * a + 2 * b), p.K};
+    const int st = pack_operands(d, 0, p.M, true, o, s);
+    return st ? st : launch_tc(d, p, &o, s);
+}
+
+namespace {
+
+int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cudaStream_t s)
+{
+    const int n_peer = p.n_peer;
     const bool i16 = d.dtype == ESPDL_DTYPE_INT16;
     const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
     p.out = d.output;
     p.ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
+    p.row_sum = o ? o->row_sum : nullptr;
     p.res = (const int8_t *)d.residual;
     p.rps = d.residual_pixel_stride ? d.residual_pixel_stride : d.out_c;
     p.epi.bias = d.bias, p.epi.ew = d.filter_exponents, p.epi.lut = d.lut, p.epi.lut_stride = d.lut_channel_stride;
@@ -1081,26 +1106,11 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
                            (uint64_t)d.filter_image_stride)))
             return st;
         ma_lo = ma, mb_lo = mb;
-    } else {
-        const size_t a = ((size_t)p.M * p.K + 255) / 256 * 256, b = ((size_t)p.N * p.K + 255) / 256 * 256;
-        if (workspace_bytes < 2 * a + 2 * b || !workspace || ((uintptr_t)workspace % 16))
-            return ESPDL_ERR_INVALID_ARG;
-        int8_t *a_hi = (int8_t *)workspace;
-        uint8_t *a_lo = (uint8_t *)workspace + a;
-        int8_t *b_hi = (int8_t *)workspace + 2 * a;
-        uint8_t *b_lo = (uint8_t *)workspace + 2 * a + b;
-        const long long ta = (long long)p.M * p.K, tb = (long long)p.N * p.K;
-        const long long cap = (long long)num_sms() * 32;
-        launch_overlapped(split_limbs_kernel, dim3((unsigned)min((ta + 255) / 256, cap)), dim3(256), 0, s, (const int16_t *)d.input, ips, p.K, ta, a_hi, a_lo);
-        launch_overlapped(split_limbs_kernel, dim3((unsigned)min((tb + 255) / 256, cap)), dim3(256), 0, s, (const int16_t *)d.filter, p.K, p.K, tb, b_hi, b_lo);
-        count_launch(2);
-        if ((st = check_launch("split_limbs")))
-            return st;
-        if ((st = make_map(&ma, a_hi, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, BLOCK_M, (uint32_t)p.swz, p.swz)) ||
-            (st = make_map(&ma_lo, a_lo, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, BLOCK_M, (uint32_t)p.swz, p.swz)) ||
-            (st = make_map(&mb, b_hi, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, (uint32_t)p.block_n, (uint32_t)p.swz, p.swz)) ||
-            (st = make_map(&mb_lo, b_lo, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, (uint32_t)p.block_n, (uint32_t)p.swz, p.swz)))
-            return st;
+    } else if ((st = make_map(&ma, o->a_hi, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, BLOCK_M, (uint32_t)p.swz, p.swz)) ||
+               (st = make_map(&ma_lo, o->a_lo, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, BLOCK_M, (uint32_t)p.swz, p.swz)) ||
+               (st = make_map(&mb, o->b_hi, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, (uint32_t)p.block_n, (uint32_t)p.swz, p.swz)) ||
+               (st = make_map(&mb_lo, o->b_lo, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, (uint32_t)p.block_n, (uint32_t)p.swz, p.swz))) {
+        return st;
     }
     const size_t stage_bytes = (size_t)(i16 ? 2 : 1) * (BLOCK_M + p.block_n) * p.swz;
     size_t smem = 1024 + (size_t)p.stages * stage_bytes + 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023) + aux_bytes(p);
@@ -1139,6 +1149,84 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
     return check_launch("gemm_tc");
 }
 
+// The product that a packed conv is: rows = its output pixels, K = its window rounded up to 16 elements.
+espdl_conv_desc packed_product(const espdl_conv_desc &d, int rows)
+{
+    espdl_conv_desc g = d;
+    g.n = 1, g.in_h = g.out_h = 1, g.in_w = g.out_w = rows, g.in_c = (d.kh * d.kw * d.in_c + 15) / 16 * 16;
+    g.kh = g.kw = g.stride_h = g.stride_w = g.dilation_h = g.dilation_w = 1;
+    g.pad_top = g.pad_bottom = g.pad_left = g.pad_right = 0;
+    g.in_pixel_stride = 0;
+    g.out_pixel_stride = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
+    g.residual_pixel_stride = d.residual_pixel_stride ? d.residual_pixel_stride : d.out_c;
+    return g;
+}
+
+constexpr size_t PACK_CHUNK = 64u << 20; // bytes of packed input per launch: it stays in L2 between the packing and the product
+
+int packed_rows(const espdl_conv_desc &d)
+{
+    const long long M = (long long)d.n * d.out_h * d.out_w;
+    const long long row = (long long)((d.kh * d.kw * d.in_c + 15) / 16 * 16) * (d.dtype == ESPDL_DTYPE_INT16 ? 2 : 1);
+    return (int)min(M, max(1ll, (long long)PACK_CHUNK / row / BLOCK_M) * BLOCK_M);
+}
+
+size_t round256(size_t v) { return (v + 255) / 256 * 256; }
+
+} // namespace
+
+bool conv2d_packed_supported(const espdl_conv_desc &d)
+{
+    const bool i16 = d.dtype == ESPDL_DTYPE_INT16;
+    if (d.group != 1 || d.filter_image_stride != 0 || (i16 && (d.lut || d.residual)))
+        return false;
+    const long long M = (long long)d.n * d.out_h * d.out_w, K = (long long)d.kh * d.kw * d.in_c, macs = M * K * d.out_c;
+    // Against the CUDA-core kernel: that one needs no packing (two launches of a few microseconds) but makes 2.2 T (int8) or 0.5 T
+    // (int16) multiply-adds a second, and a thread of it walks the whole reduction.
+    if (K > (i16 ? 16384 : 65536) || M > 0x7fffffffll || (macs < (i16 ? 3000000 : 12000000) && K < 1024))
+        return false;
+    TcParams p;
+    return plan(packed_product(d, packed_rows(d)), p);
+}
+
+size_t conv2d_packed_workspace_bytes(const espdl_conv_desc &d)
+{
+    const size_t planes = d.dtype == ESPDL_DTYPE_INT16 ? 2 : 1, Kp = (size_t)(d.kh * d.kw * d.in_c + 15) / 16 * 16, rows = packed_rows(d);
+    return planes * (round256(rows * Kp) + round256(d.out_c * Kp)) + (planes == 2 ? rows * sizeof(int) : 0);
+}
+
+int conv2d_packed(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s)
+{
+    if (workspace_bytes < conv2d_packed_workspace_bytes(d) || !workspace || ((uintptr_t)workspace % 16))
+        return ESPDL_ERR_INVALID_ARG;
+    const bool i16 = d.dtype == ESPDL_DTYPE_INT16;
+    const long long M = (long long)d.n * d.out_h * d.out_w;
+    const int chunk = packed_rows(d), Kp = (d.kh * d.kw * d.in_c + 15) / 16 * 16;
+    const size_t a = round256((size_t)chunk * Kp), b = round256((size_t)d.out_c * Kp), es = i16 ? 2 : 1;
+    uint8_t *w = (uint8_t *)workspace;
+    PackedOperands o = {w, w + a, w + es * a, w + es * a + b, (int *)(w + 2 * a + 2 * b), Kp};
+    for (long long row = 0; row < M; row += chunk) {
+        const int rows = (int)min((long long)chunk, M - row);
+        int st = pack_operands(d, row, rows, row == 0, o, s);
+        if (st)
+            return st;
+        espdl_conv_desc g = packed_product(d, rows);
+        g.input = o.a_hi, g.filter = o.b_hi;
+        g.output = (char *)d.output + (size_t)row * g.out_pixel_stride * es;
+        if (d.residual)
+            g.residual = (const char *)d.residual + (size_t)row * g.residual_pixel_stride;
+        TcParams p;
+        if (!plan(g, p))
+            return ESPDL_ERR_UNSUPPORTED;
+        p.n_peer = 0;
+        for (long long &delta : p.peer_delta) delta = 0;
+        st = launch_tc(g, p, &o, s);
+        if (st)
+            return st;
+    }
+    return ESPDL_OK;
+}
+
 } // namespace espdl
 
 // ------------------------------------------------------------------ allocation-free int16 Gemm / pointwise conv
@@ -1147,6 +1235,7 @@ int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes,
 // that loads the library carries it until the process exits.
 namespace espdl {
 static __device__ __align__(256) unsigned char g_static_limb_scratch[ESPDL_B200_STATIC_SCRATCH_BYTES];
+static __device__ int g_static_row_sums[ESPDL_B200_STATIC_SCRATCH_BYTES / 2 / 16]; // one per row; a row's planes take 32 bytes at least
 }
 
 extern "C" int espdl_b200_gemm_s16_static(const espdl_conv_desc *desc, void *stream)
@@ -1160,7 +1249,7 @@ extern "C" int espdl_b200_gemm_s16_static(const espdl_conv_desc *desc, void *str
         return ESPDL_ERR_UNSUPPORTED;
     if (desc->n == 0)
         return ESPDL_OK;
-    const size_t need = conv2d_tc_workspace_bytes(*desc);
+    const size_t need = conv2d_tc_workspace_bytes(*desc) - (size_t)desc->n * desc->out_h * desc->out_w * sizeof(int); // the planes
     if (need > (size_t)ESPDL_B200_STATIC_SCRATCH_BYTES)
         return set_error_text(ESPDL_ERR_TOO_LARGE,
                               "espdl_b200_gemm_s16_static: %zu bytes of scratch needed, the fixed array holds %u; use "
@@ -1168,13 +1257,13 @@ extern "C" int espdl_b200_gemm_s16_static(const espdl_conv_desc *desc, void *str
                               need, (unsigned)ESPDL_B200_STATIC_SCRATCH_BYTES);
     // In host code the array's name is only a handle; the device address comes from cudaGetSymbolAddress, asked
     // once per device with that device current.
-    static void *addr_of_device[64] = {nullptr};
+    static void *addr_of_device[64] = {nullptr}, *sums_of_device[64] = {nullptr};
     static std::mutex addr_mutex;
     int dev = -1;
     ESPDL_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64)
         return ESPDL_ERR_NO_DEVICE;
-    void *scratch = nullptr;
+    void *scratch = nullptr, *sums = nullptr;
     {
         std::lock_guard<std::mutex> lock(addr_mutex);
         if (!addr_of_device[dev]) {
@@ -1182,11 +1271,13 @@ extern "C" int espdl_b200_gemm_s16_static(const espdl_conv_desc *desc, void *str
             cudaError_t e = cudaGetSymbolAddress(&p, g_static_limb_scratch);
             if (e != cudaSuccess)
                 return set_cuda_error(e, "cudaGetSymbolAddress(g_static_limb_scratch)");
+            if ((e = cudaGetSymbolAddress(&sums_of_device[dev], g_static_row_sums)) != cudaSuccess)
+                return set_cuda_error(e, "cudaGetSymbolAddress(g_static_row_sums)");
             addr_of_device[dev] = p;
         }
-        scratch = addr_of_device[dev];
+        scratch = addr_of_device[dev], sums = sums_of_device[dev];
     }
-    return conv2d_tc(*desc, scratch, (size_t)ESPDL_B200_STATIC_SCRATCH_BYTES, (cudaStream_t)stream);
+    return conv2d_tc(*desc, scratch, (size_t)ESPDL_B200_STATIC_SCRATCH_BYTES, (cudaStream_t)stream, nullptr, 0, (int *)sums);
 }
 
 #ifdef ESPDL_TC_TIMING

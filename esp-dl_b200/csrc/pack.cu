@@ -1,0 +1,164 @@
+// Operand packing for the products that the tile kernel cannot read in place: rows of K elements become rows of Kp = K
+// rounded up to 16 bytes, with the window of a convolution unrolled (a row is one output pixel), for
+//   int16   two byte planes per operand.  The input splits into a signed high and an unsigned low byte (x = 256*hi + lo); the filter
+//           is shifted into the unsigned range first, w + 32768 = 256*uh + ul, so that its two planes have ONE signedness and
+//           the tile kernel multiplies a plane of the input by both in one instruction of twice the width; what the shift adds,
+//           32768 * (sum of the input row), is taken off again in the epilogue with the row sums written here.
+//   int8    the rows themselves (reductions that are no multiple of 16, windows over channel counts that are none).
+// Bound by memory traffic: every source element is read once per window position it appears in (from L1 / L2 mostly), every
+// plane written once, 16 bytes per thread and store.  A group of lanes owns a row - as many as it has 16-element chunks, up to
+// a warp - so a row's sum is a shuffle away.
+#include "common.cuh"
+
+namespace espdl {
+
+namespace {
+
+struct PackParams {
+    const void *in, *w;
+    int8_t *a_hi, *b_hi;
+    uint8_t *a_lo, *b_lo; // int16
+    int *row_sum;         // int16: one per row of A
+    int rows, N, K, Kp, lanes;
+    long long row0; // first output pixel
+    int ih, iw, ic, oh, ow, kw, sh, sw, dh, dw, pt, pl, ips;
+};
+
+__device__ __forceinline__ uint32_t pack4(const int *v) { return (uint32_t)(v[0] & 255) | ((uint32_t)(v[1] & 255) << 8) | ((uint32_t)(v[2] & 255) << 16) | ((uint32_t)v[3] << 24); }
+
+__device__ __forceinline__ uint4 pack16(const int (&v)[16]) { return make_uint4(pack4(v), pack4(v + 4), pack4(v + 8), pack4(v + 12)); }
+
+// 16 consecutive elements of a dense row; `vec`: 16-byte loads are in order.
+template <typename T>
+__device__ __forceinline__ void dense16(const T *src, int count, bool vec, int (&v)[16])
+{
+    if (vec && count >= 16) {
+        alignas(16) T t[16];
+        *(uint4 *)t = __ldg((const uint4 *)src);
+        if (sizeof(T) == 2)
+            *(uint4 *)(t + 8) = __ldg((const uint4 *)(src + 8));
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = t[j];
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = j < count ? (int)src[j] : 0;
+    }
+}
+
+template <typename T, bool WINDOW>
+__global__ void __launch_bounds__(256) pack_kernel(PackParams p)
+{
+    grid_dep_launch(); // what this writes is read by the tile kernel's loads only, which wait for it
+    grid_dep_wait();
+    const int lane = threadIdx.x & 31, sub = lane % p.lanes, per_warp = 32 / p.lanes;
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    const long long groups = ((long long)p.rows + p.N + per_warp - 1) / per_warp;
+    const bool vec_w = p.K % 16 == 0 && ((uintptr_t)p.w & 15) == 0;
+    const bool vec_in = p.ips % 16 == 0 && p.ic % 16 == 0 && ((uintptr_t)p.in & 15) == 0;
+    for (long long g = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); g < groups; g += warps) {
+        const long long row = g * per_warp + lane / p.lanes;
+        const bool is_b = row >= p.rows, live = row < (long long)p.rows + p.N;
+        int sum = 0;
+        if (live && is_b) {
+            const long long n = row - p.rows;
+            for (int k = sub * 16; k < p.Kp; k += p.lanes * 16) {
+                int v[16];
+                dense16((const T *)p.w + n * p.K + k, p.K - k, vec_w, v);
+                if (sizeof(T) == 2) {
+                    int hi[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) {
+                        const int u = k + j < p.K ? v[j] + 32768 : 0;
+                        hi[j] = u >> 8, v[j] = u;
+                    }
+                    *(uint4 *)(p.b_hi + n * p.Kp + k) = pack16(hi);
+                    *(uint4 *)(p.b_lo + n * p.Kp + k) = pack16(v);
+                } else {
+                    *(uint4 *)(p.b_hi + n * p.Kp + k) = pack16(v);
+                }
+            }
+        } else if (live) {
+            const long long pix = p.row0 + row;
+            const T *src = (const T *)p.in + pix * p.ips;
+            int iy0 = 0, ix0 = 0;
+            if (WINDOW) {
+                const int ox = (int)(pix % p.ow), oy = (int)(pix / p.ow % p.oh);
+                src = (const T *)p.in + pix / ((long long)p.ow * p.oh) * p.ih * p.iw * p.ips;
+                iy0 = oy * p.sh - p.pt, ix0 = ox * p.sw - p.pl;
+            }
+            for (int k = sub * 16; k < p.Kp; k += p.lanes * 16) {
+                int v[16];
+                if (!WINDOW) {
+                    dense16(src + k, p.K - k, vec_in, v);
+                } else {
+                    int tap = k / p.ic, c = k - tap * p.ic;
+                    int ky = tap / p.kw, kx = tap - ky * p.kw;
+                    int iy = iy0 + ky * p.dh, ix = ix0 + kx * p.dw;
+                    bool in = (unsigned)iy < (unsigned)p.ih && (unsigned)ix < (unsigned)p.iw;
+                    const T *at = src + ((long long)iy * p.iw + ix) * p.ips;
+                    if (vec_in) { // a chunk never leaves its tap
+                        if (in && k < p.K) {
+                            dense16(at + c, 16, true, v);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; j++) v[j] = 0;
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {
+                            v[j] = in && k + j < p.K ? (int)at[c] : 0;
+                            if (++c == p.ic) {
+                                c = 0;
+                                if (++kx == p.kw)
+                                    kx = 0, ky++;
+                                iy = iy0 + ky * p.dh, ix = ix0 + kx * p.dw;
+                                in = (unsigned)iy < (unsigned)p.ih && (unsigned)ix < (unsigned)p.iw;
+                                at = src + ((long long)iy * p.iw + ix) * p.ips;
+                            }
+                        }
+                    }
+                }
+                if (sizeof(T) == 2) {
+                    int hi[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) hi[j] = v[j] >> 8, sum += v[j];
+                    *(uint4 *)(p.a_hi + row * p.Kp + k) = pack16(hi);
+                    *(uint4 *)(p.a_lo + row * p.Kp + k) = pack16(v);
+                } else {
+                    *(uint4 *)(p.a_hi + row * p.Kp + k) = pack16(v);
+                }
+            }
+        }
+        if (sizeof(T) == 2) {
+            for (int d = p.lanes >> 1; d; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            if (live && !is_b && sub == 0)
+                p.row_sum[row] = sum;
+        }
+    }
+}
+
+} // namespace
+
+int pack_operands(const espdl_conv_desc &d, long long row0, int rows, bool filter, const PackedOperands &o, cudaStream_t s)
+{
+    PackParams p;
+    p.in = d.input, p.w = d.filter;
+    p.a_hi = (int8_t *)o.a_hi, p.a_lo = (uint8_t *)o.a_lo, p.b_hi = (int8_t *)o.b_hi, p.b_lo = (uint8_t *)o.b_lo, p.row_sum = o.row_sum;
+    p.rows = rows, p.N = filter ? d.out_c : 0, p.K = d.kh * d.kw * d.in_c, p.Kp = o.Kp, p.row0 = row0;
+    p.ih = d.in_h, p.iw = d.in_w, p.ic = d.in_c, p.oh = d.out_h, p.ow = d.out_w, p.kw = d.kw;
+    p.sh = d.stride_h, p.sw = d.stride_w, p.dh = d.dilation_h, p.dw = d.dilation_w, p.pt = d.pad_top, p.pl = d.pad_left;
+    p.ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
+    p.lanes = 1;
+    while (p.lanes < 32 && p.lanes * 16 < p.Kp) p.lanes *= 2;
+    const long long groups = ((long long)p.rows + p.N + 32 / p.lanes - 1) / (32 / p.lanes);
+    const unsigned blocks = (unsigned)min((groups + 7) / 8, (long long)num_sms() * 16);
+    const bool window = d.kh != 1 || d.kw != 1 || d.stride_h != 1 || d.stride_w != 1 || d.pad_top || d.pad_bottom || d.pad_left || d.pad_right;
+    if (d.dtype == ESPDL_DTYPE_INT16)
+        launch_overlapped(window ? pack_kernel<int16_t, true> : pack_kernel<int16_t, false>, dim3(blocks), dim3(256), 0, s, p);
+    else
+        launch_overlapped(window ? pack_kernel<int8_t, true> : pack_kernel<int8_t, false>, dim3(blocks), dim3(256), 0, s, p);
+    count_launch();
+    return check_launch("pack_operands");
+}
+
+} // namespace espdl

@@ -1,0 +1,64 @@
+"""Convs whose operands are packed for the tile kernel (int16 windows, reductions and channel counts that are no multiple of 16),
+the int16 product's combined planes, and batches of products on the CUDA cores: bit-exact against the plain-C oracle at the
+extremes of the types, around tile and chunk ends."""
+import numpy as np
+import pytest
+
+import cases
+import gpu_util
+from espdl_b200 import abi
+
+pytestmark = pytest.mark.gpu
+
+S16 = dict(dtype=abi.DTYPE_INT16, e_in=-14, e_w=(-15, -14), e_out=-11)
+SHAPES = [
+    dict(n=2, h=20, w=21, cin=32, cout=48),                        # 3x3
+    dict(n=1, h=30, w=30, cin=24, cout=64, stride=2),              # channels no multiple of 16, stride
+    dict(n=3, h=17, w=19, cin=20, cout=33, kh=5, kw=5, dil=2, pad=(4, 4, 4, 4)),
+    dict(n=1, h=40, w=40, cin=40, cout=56, kh=1, kw=1, pad=(0, 0, 0, 0), in_stride=48, out_stride=72),
+    dict(n=2, h=30, w=28, cin=3, cout=40, kh=7, kw=7, stride=2),
+    dict(n=1, h=1, w=9, cin=1100, cout=300, kh=1, kw=1, pad=(0, 0, 0, 0)),   # few rows, a long reduction
+    dict(n=1, h=1, w=700, cin=127, cout=257, kh=1, kw=1, pad=(0, 0, 0, 0)),
+]
+
+
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("i", range(len(SHAPES)))
+def test_packed_conv(i, dtype, round_mode):
+    kw = dict(SHAPES[i], seed=i, per_channel=True, round_mode=round_mode)
+    if dtype == abi.DTYPE_INT16:
+        kw.update(S16, wide=True)
+    case = cases.conv_case(**kw)
+    want = gpu_util.run_conv_oracle(case)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+    assert want.std() > 0
+
+
+@pytest.mark.parametrize("m,k,n", [(129, 16, 16), (300, 16384, 8), (128, 4096, 129), (1000, 272, 260)])
+@pytest.mark.parametrize("sign", [-1, 1, 0])
+def test_int16_products_at_the_ends_of_the_type(m, k, n, sign):
+    """All operands at an end of int16 (the largest partial sums there are), and mixed."""
+    case = cases.gemm_case(seed=m, m=m, k=k, n_out=n, wide=True, **dict(S16, e_out=-4))
+    if sign:
+        case["x"][...] = 32767 if sign > 0 else -32768
+        case["w"][...] = -32768 if sign > 0 else 32767
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+
+
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("k,n", [(100, 100), (99, 17), (16, 3)])
+def test_batch_of_products_on_the_cuda_cores(k, n, dtype):
+    t = np.int8 if dtype == abi.DTYPE_INT8 else np.int16
+    rng = np.random.default_rng(k)
+    images, rows = 5, 13
+    x = rng.integers(-100, 100, size=(images, 1, rows, k), dtype=t)
+    w = rng.integers(-100, 100, size=(images, n, 1, 1, k), dtype=t)
+    extra = dict(S16, e_out=-20) if dtype == abi.DTYPE_INT16 else {}
+    whole = cases.conv_case(seed=1, n=images, h=1, w=rows, cin=k, cout=n, kh=1, kw=1, pad=(0, 0, 0, 0), bias=False, **extra)
+    whole.update(x=x, w=w, filter_image_stride=n * k)
+    got = gpu_util.run_conv_gpu(whole, kernel=abi.KERNEL_SIMT)
+    for i in range(images):
+        one = cases.conv_case(seed=1, n=1, h=1, w=rows, cin=k, cout=n, kh=1, kw=1, pad=(0, 0, 0, 0), bias=False, **extra)
+        one.update(x=x[i:i + 1], w=w[i], filter_exponent=whole["filter_exponent"])
+        np.testing.assert_array_equal(got[i:i + 1], gpu_util.run_conv_oracle(one))
