@@ -24,10 +24,54 @@ struct ConvParams {
     int ew_scalar, per_channel, relu, half_even;
     long long total; // number of (pixel, oc-group) work items
     int groups;      // oc groups per pixel
+    int lanes;       // threads that share an item's reduction (a power of two up to 32)
     long long w_image; // elements between the filters of consecutive images (a batch of products), 0 = one filter
 };
 
-template <int OCT, bool DP4A>
+// The reduction of one work item (an output pixel, OCT output channels), whole or - SPLIT - this lane's share of it: words of VEC
+// elements `sub`, sub + lanes, ... of the flattened window.
+template <int OCT, int VEC, bool SPLIT, typename ACC, typename MulAdd>
+__device__ __forceinline__ void simt_reduce(const ConvParams &p, int iy0, int ix0, long long in_image, long long w_first, int oc_left, long long wstride, int sub,
+                                            ACC (&acc)[OCT], const MulAdd &mul_add)
+{
+    const int icw = p.ic / VEC;
+    if constexpr (SPLIT) {
+        const int words = p.kh * p.kw * icw;
+#pragma unroll 4
+        for (int q = sub; q < words; q += p.lanes) {
+            const int tap = q / icw, c = (q - tap * icw) * VEC, ky = tap / p.kw, kx = tap - ky * p.kw;
+            const int iy = iy0 + ky * p.dh, ix = ix0 + kx * p.dw;
+            if ((unsigned)iy >= (unsigned)p.ih || (unsigned)ix >= (unsigned)p.iw)
+                continue;
+            const long long at = in_image + ((long long)iy * p.iw + ix) * p.ips + c, wt = w_first + (long long)q * VEC;
+#pragma unroll
+            for (int j = 0; j < OCT; j++)
+                if (j < oc_left)
+                    mul_add(at, wt + j * wstride, acc[j]);
+        }
+    } else {
+        for (int ky = 0; ky < p.kh; ky++) {
+            const int iy = iy0 + ky * p.dh;
+            if (iy < 0 || iy >= p.ih)
+                continue;
+            for (int kx = 0; kx < p.kw; kx++) {
+                const int ix = ix0 + kx * p.dw;
+                if (ix < 0 || ix >= p.iw)
+                    continue;
+                const long long at = in_image + ((long long)iy * p.iw + ix) * p.ips, wt = w_first + ((long long)ky * p.kw + kx) * p.ic;
+                for (int c = 0; c < icw; c++)
+#pragma unroll
+                    for (int j = 0; j < OCT; j++)
+                        if (j < oc_left)
+                            mul_add(at + c * VEC, wt + j * wstride + c * VEC, acc[j]);
+            }
+        }
+    }
+}
+
+// Bound by the latency of the loads along a reduction: with few outputs a thread that walks its reduction alone takes 0.3 to 0.5 us
+// per four elements (1x1024 by 1024: 143 us), so then `lanes` neighbouring threads share an item and add up by shuffles.
+template <int OCT, bool DP4A, bool SPLIT>
 __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
 {
     grid_dep_launch();
@@ -37,8 +81,11 @@ __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
     const int32_t *__restrict__ bias = (const int32_t *)p.bias;
     int8_t *__restrict__ out = (int8_t *)p.out;
     const long long wstride = (long long)p.kh * p.kw * p.ic; // elements per output channel
-    for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < p.total;
-         item += (long long)gridDim.x * blockDim.x) {
+    const int lanes = SPLIT ? p.lanes : 1, sub = SPLIT ? (int)(threadIdx.x % lanes) : 0;
+    const long long step = (long long)gridDim.x * blockDim.x / lanes;
+    for (long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / lanes; __any_sync(0xffffffffu, first < p.total); first += step) {
+        const bool live = first < p.total;
+        const long long item = live ? first : p.total - 1;
         const int g = (int)(item % p.groups);
         const long long pix = item / p.groups;
         const int ox = (int)(pix % p.ow);
@@ -48,43 +95,22 @@ __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
         int32_t acc[OCT];
 #pragma unroll
         for (int j = 0; j < OCT; j++) acc[j] = 0;
-        for (int ky = 0; ky < p.kh; ky++) {
-            const int iy = oy * p.sh + ky * p.dh - p.pt;
-            if (iy < 0 || iy >= p.ih)
-                continue;
-            for (int kx = 0; kx < p.kw; kx++) {
-                const int ix = ox * p.sw + kx * p.dw - p.pl;
-                if (ix < 0 || ix >= p.iw)
-                    continue;
-                const int8_t *ip = in + (((long long)n * p.ih + iy) * p.iw + ix) * p.ips;
-                const int8_t *wp = w + n * p.w_image + (long long)oc0 * wstride + ((long long)ky * p.kw + kx) * p.ic;
-                if (DP4A) {
-                    const int *ip4 = (const int *)ip;
-                    for (int c = 0; c < p.ic / 4; c++) {
-                        const int a = __ldg(ip4 + c);
+        simt_reduce<OCT, DP4A ? 4 : 1, SPLIT>(p, oy * p.sh - p.pt, ox * p.sw - p.pl, (long long)n * p.ih * p.iw * p.ips, n * p.w_image + (long long)oc0 * wstride, p.oc - oc0,
+                                              wstride, sub, acc, [&](long long at, long long wt, int32_t &sum) {
+                                                  if (DP4A)
+                                                      sum = __dp4a(__ldg((const int *)(in + at)), __ldg((const int *)(w + wt)), sum);
+                                                  else
+                                                      sum += (int)__ldg(in + at) * (int)__ldg(w + wt);
+                                              });
+        if (SPLIT)
+            for (int d = lanes >> 1; d; d >>= 1)
 #pragma unroll
-                        for (int j = 0; j < OCT; j++) {
-                            if (oc0 + j < p.oc)
-                                acc[j] = __dp4a(a, __ldg((const int *)(wp + j * wstride) + c), acc[j]);
-                        }
-                    }
-                } else {
-                    for (int c = 0; c < p.ic; c++) {
-                        const int a = ip[c];
-#pragma unroll
-                        for (int j = 0; j < OCT; j++) {
-                            if (oc0 + j < p.oc)
-                                acc[j] += a * (int)wp[j * wstride + c];
-                        }
-                    }
-                }
-            }
-        }
+                for (int j = 0; j < OCT; j++) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], d);
         int8_t *op = out + pix * p.ops + oc0;
 #pragma unroll
         for (int j = 0; j < OCT; j++) {
             const int oc = oc0 + j;
-            if (oc < p.oc) {
+            if (live && oc < p.oc && (!SPLIT || sub == j % lanes)) {
                 const int e = p.per_channel ? p.ew[oc] : p.ew_scalar;
                 const int shift = max(-31, min(31, p.e_shift_base - e));
                 int32_t q = requant8(acc[j], bias ? bias[oc] : 0, shift, p.relu, p.half_even);
@@ -98,7 +124,7 @@ __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
     }
 }
 
-template <int OCT>
+template <int OCT, bool SPLIT>
 __global__ void __launch_bounds__(256) conv_s16_kernel(ConvParams p)
 {
     grid_dep_launch();
@@ -108,8 +134,11 @@ __global__ void __launch_bounds__(256) conv_s16_kernel(ConvParams p)
     const long long *__restrict__ bias = (const long long *)p.bias;
     int16_t *__restrict__ out = (int16_t *)p.out;
     const long long wstride = (long long)p.kh * p.kw * p.ic;
-    for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < p.total;
-         item += (long long)gridDim.x * blockDim.x) {
+    const int lanes = SPLIT ? p.lanes : 1, sub = SPLIT ? (int)(threadIdx.x % lanes) : 0;
+    const long long step = (long long)gridDim.x * blockDim.x / lanes;
+    for (long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / lanes; __any_sync(0xffffffffu, first < p.total); first += step) {
+        const bool live = first < p.total;
+        const long long item = live ? first : p.total - 1;
         const int g = (int)(item % p.groups);
         const long long pix = item / p.groups;
         const int ox = (int)(pix % p.ow);
@@ -119,31 +148,19 @@ __global__ void __launch_bounds__(256) conv_s16_kernel(ConvParams p)
         long long acc[OCT];
 #pragma unroll
         for (int j = 0; j < OCT; j++) acc[j] = 0;
-        for (int ky = 0; ky < p.kh; ky++) {
-            const int iy = oy * p.sh + ky * p.dh - p.pt;
-            if (iy < 0 || iy >= p.ih)
-                continue;
-            for (int kx = 0; kx < p.kw; kx++) {
-                const int ix = ox * p.sw + kx * p.dw - p.pl;
-                if (ix < 0 || ix >= p.iw)
-                    continue;
-                const int16_t *ip = in + (((long long)n * p.ih + iy) * p.iw + ix) * p.ips;
-                const int16_t *wp = w + n * p.w_image + (long long)oc0 * wstride + ((long long)ky * p.kw + kx) * p.ic;
-                for (int c = 0; c < p.ic; c++) {
-                    const int a = ip[c];
+        simt_reduce<OCT, 1, SPLIT>(p, oy * p.sh - p.pt, ox * p.sw - p.pl, (long long)n * p.ih * p.iw * p.ips, n * p.w_image + (long long)oc0 * wstride, p.oc - oc0, wstride, sub,
+                                   acc, [&](long long at, long long wt, long long &sum) {
+                                       sum += (long long)((int)__ldg(in + at) * (int)__ldg(w + wt)); // |a*w| <= 2^30: exact in int32
+                                   });
+        if (SPLIT)
+            for (int d = lanes >> 1; d; d >>= 1)
 #pragma unroll
-                    for (int j = 0; j < OCT; j++) {
-                        if (oc0 + j < p.oc)
-                            acc[j] += (long long)(a * (int)wp[j * wstride + c]); // |a*w| < 2^31: exact in int32
-                    }
-                }
-            }
-        }
+                for (int j = 0; j < OCT; j++) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], d);
         int16_t *op = out + pix * p.ops + oc0;
 #pragma unroll
         for (int j = 0; j < OCT; j++) {
             const int oc = oc0 + j;
-            if (oc < p.oc) {
+            if (live && oc < p.oc && (!SPLIT || sub == j % lanes)) {
                 const int e = p.per_channel ? p.ew[oc] : p.ew_scalar;
                 const int shift = max(-62, min(62, p.e_shift_base - e));
                 op[j] = (int16_t)requant16(acc[j], bias ? bias[oc] : 0ll, shift, p.relu, p.half_even);
@@ -242,6 +259,29 @@ __global__ void __launch_bounds__(256) conv_s8_small_k_kernel(ConvParams p)
     }
 }
 
+static bool simt_dp4a(const espdl_conv_desc &d)
+{
+    const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
+    return d.dtype == ESPDL_DTYPE_INT8 && d.in_c % 4 == 0 && ips % 4 == 0 && ((uintptr_t)d.input % 4) == 0 && ((uintptr_t)d.filter % 4) == 0 && d.filter_image_stride % 4 == 0;
+}
+
+// Threads per item: until the GPU has work for all its schedulers, or a thread's share is down to four words (from twelve words on:
+// six ran 6.2 us whole and 8.9 us split).
+static int simt_lanes(const espdl_conv_desc &d)
+{
+    const long long items = (long long)d.n * d.out_h * d.out_w * ((d.out_c + 3) / 4), words = (long long)d.kh * d.kw * d.in_c / (simt_dp4a(d) ? 4 : 1);
+    int lanes = 1;
+    while (words >= 12 && lanes < 32 && words > 4 * lanes && items * lanes < (long long)num_sms() * 1024) lanes *= 2;
+    return lanes;
+}
+
+float conv2d_simt_estimate_us(const espdl_conv_desc &d)
+{
+    const double macs = (double)d.n * d.out_h * d.out_w * d.out_c * d.kh * d.kw * d.in_c, words = (double)d.kh * d.kw * d.in_c / (simt_dp4a(d) ? 4 : 1) / simt_lanes(d);
+    const double rate = d.dtype == ESPDL_DTYPE_INT16 ? 0.5e6 : (simt_dp4a(d) ? 2.2e6 : 0.8e6); // multiply-adds per us, measured
+    return (float)(3.0 + words * 0.3 + macs / rate);
+}
+
 int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
 {
     ConvParams p;
@@ -260,7 +300,8 @@ int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
     p.groups = (d.out_c + OCT - 1) / OCT;
     p.total = (long long)d.n * d.out_h * d.out_w * p.groups;
     const int threads = 256;
-    long long blocks = (p.total + threads - 1) / threads;
+    p.lanes = simt_lanes(d);
+    long long blocks = (p.total * p.lanes + threads - 1) / threads;
     const long long max_blocks = (long long)num_sms() * 32;
     if (blocks > max_blocks)
         blocks = max_blocks;
@@ -274,13 +315,12 @@ int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
         else
             launch_overlapped(conv_s8_small_k_kernel<3, 3, 4>, dim3(grid), dim3(threads), 0, s, p);
     } else if (d.dtype == ESPDL_DTYPE_INT8) {
-        const bool dp4a = d.in_c % 4 == 0 && p.ips % 4 == 0 && ((uintptr_t)d.input % 4) == 0 && ((uintptr_t)d.filter % 4) == 0 && d.filter_image_stride % 4 == 0;
-        if (dp4a)
-            launch_overlapped(conv_s8_kernel<OCT, true>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
-        else
-            launch_overlapped(conv_s8_kernel<OCT, false>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
+        const bool dp4a = simt_dp4a(d), split = p.lanes > 1;
+        launch_overlapped(dp4a ? (split ? conv_s8_kernel<OCT, true, true> : conv_s8_kernel<OCT, true, false>)
+                               : (split ? conv_s8_kernel<OCT, false, true> : conv_s8_kernel<OCT, false, false>),
+                          dim3((unsigned)blocks), dim3(threads), 0, s, p);
     } else {
-        launch_overlapped(conv_s16_kernel<OCT>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
+        launch_overlapped(p.lanes > 1 ? conv_s16_kernel<OCT, true> : conv_s16_kernel<OCT, false>, dim3((unsigned)blocks), dim3(threads), 0, s, p);
     }
     count_launch();
     return check_launch("conv2d_simt");

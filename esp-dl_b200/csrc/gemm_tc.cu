@@ -83,7 +83,9 @@ struct TcParams {
     int stages;
     int acc_stages; // TMEM accumulator buffers: 4 or 2 (int8), 1 (int16)
     int tmem_cols;  // power of two >= 32
-    int out_pw;     // staged epilogue: bytes per row of a group's output piece (0 = rows are stored directly)
+    int out_pw;     // staged epilogue: bytes per row of a group's output piece (0 = rows are stored directly); int16: a quarter
+                    // of the bytes per row of the one tile that all groups share
+    int out_rows;   // the staging tiles leave row by row, a warp per row (rows that no TMA store can address), not as one TMA store
     int out_mask;   // swizzle mask of the staging tiles (7, 3, 1, 0)
     void *out;
     long long ops;  // output row stride in elements
@@ -182,6 +184,50 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
     }
 }
 
+// One row of a staging tile to global memory by a whole warp: `len` bytes at offset `at` of the tile at `buf` (16-byte chunks swizzled
+// as the stages wrote them) to `dst`, any alignment.  A thread that stores its own unaligned row issues byte stores that touch 32
+// rows each; here a store instruction covers 128 consecutive bytes (25385 rows of 409 bytes, K = 170: 128 us before).
+__device__ __forceinline__ uint32_t staged_word(uint32_t buf, uint32_t off, uint32_t mask)
+{
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(buf + (off ^ (((off >> 7) & mask) << 4))));
+    return v;
+}
+
+__device__ __forceinline__ void store_staged_row(int8_t *dst, uint32_t buf, uint32_t at, int len, uint32_t mask, int lane)
+{
+    if ((((uintptr_t)dst | (uintptr_t)len) & 15) == 0) {
+        for (int c = lane * 16; c < len; c += 512) {
+            const uint32_t off = at + (uint32_t)c;
+            uint4 v;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(buf + (off ^ (((off >> 7) & mask) << 4))));
+            *(uint4 *)(dst + c) = v;
+        }
+        return;
+    }
+    const int head = min((int)((0u - (uint32_t)(uintptr_t)dst) & 3u), len), words = (len - head) >> 2;
+    const uint32_t sh = (uint32_t)(head & 3) * 8u;
+    for (int w = lane; w < words; w += 32) {
+        const uint32_t off = at + (uint32_t)(4 * w); // the aligned word that holds the first byte (head < 4)
+        uint32_t v = staged_word(buf, off, mask);
+        if (sh)
+            v = __funnelshift_r(v, staged_word(buf, off + 4, mask), sh);
+        *(uint32_t *)(dst + head + 4 * w) = v;
+    }
+    const int edge = len - 4 * words; // head and tail bytes
+    if (lane < edge) {
+        const int b = lane < head ? lane : lane + 4 * words;
+        const uint32_t off = at + (uint32_t)b;
+        dst[b] = (int8_t)(staged_word(buf, off & ~3u, mask) >> (8 * (off & 3u)));
+    }
+}
+
+// Per-column constants of an int16 tile: q = (sum + bias_half) >> shift in 64 bits, as the int8 form (fast_constants).
+struct WideParam {
+    long long bias_half;
+    int shift, pad;
+};
+
 template <bool I16, bool EVEN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -200,7 +246,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int out_tile_bytes = (BLOCK_M * p.out_pw + 1023) & ~1023;
     uint8_t *aux = out_stage + 4 * (size_t)out_tile_bytes;
     FastParam *fast_s = (FastParam *)aux; // n_pad entries, 16-byte aligned (block_n % 16 == 0)
-    uint64_t *bars = (uint64_t *)(aux + sizeof(FastParam) * (size_t)n_pad);
+    WideParam *wide_s = (WideParam *)aux; // int16: the current tile's columns
+    uint64_t *bars = (uint64_t *)(aux + (I16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)n_pad));
     uint64_t *full_bar = bars, *empty_bar = bars + MAX_STAGES, *tfull_bar = bars + 2 * MAX_STAGES, *tempty_bar = tfull_bar + MAX_ACC;
     uint32_t *tmem_slot = (uint32_t *)(tempty_bar + MAX_ACC);
     int *slow_flag = (int *)(tmem_slot + 1);
@@ -238,7 +285,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (I16) {
             prefetch_tensormap(&map_a_lo);
             prefetch_tensormap(&map_b_lo);
-        } else if (p.out_pw) {
+        } else if (p.out_pw && !p.out_rows) {
             prefetch_tensormap(&map_out);
         }
     }
@@ -493,7 +540,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     // staged: requantise into this group's shared-memory tile, one TMA store per piece
                     const bool leader = (ew & 3) == 0 && lane == 0;
                     const uint32_t buf = smem_u32(out_stage + (size_t)group * out_tile_bytes);
-                    if (leader)
+                    if (leader && !p.out_rows)
                         bulk_wait_read_all(); // the previous store out of this tile has been read
                     named_bar(2 + group, 128);
                     TC_LAP(w_store);
@@ -519,6 +566,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     __syncwarp();
                     if (lane == 0)
                         mbar_arrive(smem_u32(&tempty_bar[acc]));
+                    if (p.out_rows) {
+                        named_bar(2 + group, 128);
+                        const int len = min(p.out_pw, p.N - (n0 + col0)), rows_left = min(32, p.M - m0 - lane_group * 32);
+                        int8_t *dst = (int8_t *)p.out + ((long long)bi * p.M + m0 + lane_group * 32) * p.ops + n0 + col0;
+                        if (len > 0)
+                            for (int i = 0; i < rows_left; i++, dst += p.ops)
+                                store_staged_row(dst, buf, (uint32_t)((lane_group * 32 + i) * p.out_pw), len, (uint32_t)p.out_mask, lane);
+                        continue;
+                    }
                     fence_async_smem();
                     named_bar(2 + group, 128);
                     if (leader) {
@@ -529,6 +585,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 epilogue_direct_tile<EVEN>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, true, p.epi.lut ? smem_u32(lut_s) : 0u);
             } else {
+                // all groups share the tile: constants of its columns, then 16 columns at a time into a staging tile of [128][2 * block_n]
+                // bytes, then whole rows
+                constexpr int EPI_BAR = 6;
+                const int et = (int)threadIdx.x - 64;
+                named_bar(EPI_BAR, EPI_WARPS * 32); // the previous tile's rows and constants have been read
+                if (et == 0)
+                    *slow_flag = 0;
+                named_bar(EPI_BAR, EPI_WARPS * 32);
+                for (int j = et; j < p.block_n; j += EPI_WARPS * 32) {
+                    const int n = min(n0 + j, p.N - 1);
+                    const int e = p.epi.per_channel ? __ldg(p.epi.ew + n) : p.epi.ew_scalar, sh = p.epi.e_shift_base - e;
+                    const long long b = p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll;
+                    if (sh < 1 || sh > 58 || b >= (1ll << 58) || b <= -(1ll << 58)) // |sum| < 2^46
+                        *slow_flag = 1;
+                    const int fs = max(1, min(58, sh));
+                    wide_s[j].bias_half = b + (1ll << (fs - 1)) - (EVEN ? 1 : 0);
+                    wide_s[j].shift = fs;
+                }
+                named_bar(EPI_BAR, EPI_WARPS * 32);
+                const bool slow = *(volatile int *)slow_flag;
+                const long long base = row_ok ? -(long long)p.row_sum[m] * 32768 : 0ll;
+                const uint32_t buf = smem_u32(out_stage), pitch = 2u * (uint32_t)p.block_n, mask = 7u;
                 int chunk = 0;
                 for (int c0 = 0; c0 < p.block_n; c0 += 16, chunk++) {
                     if (chunk % parts != part)
@@ -540,31 +618,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     ld_wait16(vh);
                     tie16(vm);
                     tie16(vl);
-                    if (row_ok && n0 + c0 < p.N) {
-                        int16_t *op = (int16_t *)p.out + m * p.ops + n0 + c0;
-                        const long long base = -(long long)p.row_sum[m] * 32768;
-                        uint32_t pk[8];
+                    uint32_t pk[8];
 #pragma unroll
-                        for (int j = 0; j < 16; j++) {
+                    for (int j = 0; j < 16; j++) {
+                        long long w = base + (long long)vh[j] * 65536 + (long long)vm[j] * 256 + (long long)vl[j];
+                        int q;
+                        if (!slow) {
+                            const WideParam c = wide_s[c0 + j];
+                            w += c.bias_half;
+                            if (EVEN)
+                                w += (w >> c.shift) & 1;
+                            w >>= c.shift;
+                            const int lo = (int)w, hi = (int)(w >> 32);
+                            q = hi == (lo >> 31) ? max(-32768, min(32767, lo)) : (hi < 0 ? -32768 : 32767);
+                            if (p.epi.relu)
+                                q = max(q, 0);
+                        } else {
                             const int n = min(n0 + c0 + j, p.N - 1);
-                            const long long a = base + ((long long)vh[j] << 16) + ((long long)vm[j] << 8) + (long long)vl[j];
                             const int e = p.epi.per_channel ? __ldg(p.epi.ew + n) : p.epi.ew_scalar;
                             const int shift = max(-62, min(62, p.epi.e_shift_base - e));
-                            const long long b = p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll;
-                            const uint32_t q = (uint32_t)requant16(a, b, shift, p.epi.relu, p.epi.half_even) & 0xffffu;
-                            pk[j >> 1] = j & 1 ? pk[j >> 1] | (q << 16) : q;
+                            q = requant16(w, p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll, shift, p.epi.relu, p.epi.half_even);
                         }
-                        if (n0 + c0 + 16 <= p.N && ((uintptr_t)op & 15) == 0) {
-                            *(uint4 *)op = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                            *(uint4 *)(op + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; j++)
-                                if (n0 + c0 + j < p.N)
-                                    op[j] = (int16_t)(pk[j >> 1] >> (16 * (j & 1)));
-                        }
+                        pk[j >> 1] = j & 1 ? pk[j >> 1] | ((uint32_t)q << 16) : (uint32_t)q & 0xffffu;
                     }
+                    const uint32_t off = (uint32_t)row_in_tile * pitch + 2u * (uint32_t)c0;
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (off ^ (((off >> 7) & mask) << 4))), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+                    const uint32_t off2 = off + 16u;
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (off2 ^ (((off2 >> 7) & mask) << 4))), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
                 }
+                fence_before(); // the accumulator is free before the rows leave
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(smem_u32(&tempty_bar[acc]));
+                named_bar(EPI_BAR, EPI_WARPS * 32);
+                const int len = 2 * min(p.block_n, p.N - n0);
+                for (int row = ew; row < BLOCK_M && m0 + row < p.M; row += EPI_WARPS)
+                    store_staged_row((int8_t *)p.out + 2 * (((long long)bi * p.M + m0 + row) * p.ops + n0), buf, (uint32_t)row * pitch, len, mask, lane);
+                continue;
             }
             fence_before();
             __syncwarp();
@@ -579,7 +669,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             TC_REC(6, w_work);
             TC_REC(7, w_store);
         }
-        if (!I16 && p.out_pw && (ew & 3) == 0 && lane == 0)
+        if (!I16 && p.out_pw && !p.out_rows && (ew & 3) == 0 && lane == 0)
             bulk_wait_all(); // shared memory stays allocated until the last store has left it
     }
 
@@ -890,9 +980,9 @@ constexpr size_t SMEM_BUDGET = 200 * 1024;      // stages + staging tiles of the
 constexpr size_t SMEM_BUDGET_DEEP = 225 * 1024; // long reductions with direct row stores: one more stage in flight (1.79 -> 1.97 POPS
                                                 // at 65536x1024x1024); for the staged layers the larger budget measured 5 % slower
 
-size_t aux_bytes(const TcParams &p)
+size_t aux_bytes(const TcParams &p, bool i16 = false)
 {
-    return sizeof(FastParam) * (size_t)p.n_tiles * p.block_n + (2 * MAX_STAGES + 2 * MAX_ACC) * 8 + 32 + 256 + (TILE_RING + MAX_ACC) * 4;
+    return (i16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)p.n_tiles * p.block_n) + (2 * MAX_STAGES + 2 * MAX_ACC) * 8 + 32 + 256 + (TILE_RING + MAX_ACC) * 4;
 }
 
 bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
@@ -910,13 +1000,18 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     int max_bn = i16 ? 128 : 256;
     if (const char *cap = getenv("ESPDL_B200_MAX_BLOCK_N")) // tile width cap (a multiple of 16), for experiments
         max_bn = max(16, min(max_bn, atoi(cap) / 16 * 16));
+    p.m_tiles = (p.M + BLOCK_M - 1) / BLOCK_M;
+    // Few rows: narrower tiles put more SMs to work while they still make one wave - a tile's time is the stream of its filter rows
+    // through one SM plus its columns' epilogue.
+    while (max_bn > 32 && 2ll * p.batch * p.m_tiles * ((p.N + max_bn - 1) / max_bn) <= num_sms()) max_bn /= 2;
     p.n_tiles = (p.N + max_bn - 1) / max_bn;
     p.block_n = (((p.N + p.n_tiles - 1) / p.n_tiles) + 15) / 16 * 16;
     if (!i16 && p.block_n > 128)
         p.block_n = (p.block_n + 31) / 32 * 32; // two epilogue groups split a wide tile into whole 16-byte pieces
     p.n_tiles = (p.N + p.block_n - 1) / p.block_n;
-    p.m_tiles = (p.M + BLOCK_M - 1) / BLOCK_M;
     p.swz = pick_swz(p.K);
+    if (i16 && p.swz == 128 && p.block_n > 80)
+        p.swz = 64; // a stage holds two planes of each operand: 64-byte rows leave room for five stages beside a wide output tile
     p.k_blocks = (p.K + p.swz - 1) / p.swz;
     p.acc_stages = i16 ? 1 : (4 * p.block_n <= 512 ? 4 : 2);
     int cols = p.acc_stages * (i16 ? 3 : 1) * p.block_n;
@@ -930,7 +1025,11 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     p.out_pw = 0, p.out_mask = 0;
     const long long rps = d.residual_pixel_stride ? d.residual_pixel_stride : d.out_c;
     const bool res_ok = !d.residual || (rps % 16 == 0 && ((uintptr_t)d.residual % 16) == 0);
-    if (!i16 && ops % 16 == 0 && ((uintptr_t)d.output % 16) == 0 && res_ok && !force_direct && !getenv("ESPDL_B200_DIRECT_STORES")) {
+    p.out_rows = 0;
+    if (i16) {
+        p.out_pw = p.block_n / 2; // four times [128][out_pw] = the tile
+    } else if (res_ok && !force_direct && !getenv("ESPDL_B200_DIRECT_STORES")) {
+        p.out_rows = ops % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
         const int parts = 4 / p.acc_stages;
         if (p.block_n % (16 * parts) == 0 && p.block_n / parts <= 128) {
             p.out_pw = p.block_n / parts;
@@ -939,7 +1038,7 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     }
     size_t out_bytes = 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023);
     size_t stage_bytes = (size_t)(i16 ? 2 : 1) * (BLOCK_M + p.block_n) * p.swz;
-    int stages = (int)((SMEM_BUDGET - aux_bytes(p) - out_bytes - 1024) / stage_bytes);
+    int stages = (int)((SMEM_BUDGET - aux_bytes(p, i16) - out_bytes - 1024) / stage_bytes);
     // A wide tile with a reduction of two 128-byte blocks and room for only two or three stages has barely one tile's loads
     // in flight, and every tile then waits a full load latency (192 -> 256 columns over 3.3 M rows: 0.39 ms).  Blocks of 64
     // bytes make stages half as large: more of them, more tiles in flight (0.28 ms), although the TMA unit moves 64-byte
@@ -952,7 +1051,9 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
             p.swz = 64, p.k_blocks = kb64, stage_bytes = stage64, stages = stages64;
         }
     }
-    if (p.out_pw && p.k_blocks > 2 && stages < 4) {
+    if (p.out_rows && p.out_pw && stages < 4)
+        stages = (int)((SMEM_BUDGET_DEEP - aux_bytes(p) - out_bytes - 1024) / stage_bytes);
+    if (!i16 && p.out_pw && !p.out_rows && p.k_blocks > 2 && stages < 4) {
         // a long reduction needs the deep load pipeline more than the output needs staging
         p.out_pw = 0, p.out_mask = 0, out_bytes = 0;
         stages = (int)((SMEM_BUDGET_DEEP - aux_bytes(p) - 1024) / stage_bytes);
@@ -1113,9 +1214,9 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
         return st;
     }
     const size_t stage_bytes = (size_t)(i16 ? 2 : 1) * (BLOCK_M + p.block_n) * p.swz;
-    size_t smem = 1024 + (size_t)p.stages * stage_bytes + 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023) + aux_bytes(p);
+    size_t smem = 1024 + (size_t)p.stages * stage_bytes + 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023) + aux_bytes(p, i16);
     CUtensorMap mo = ma;
-    if (p.out_pw) {
+    if (!i16 && p.out_pw && !p.out_rows) {
         const int osw = p.out_pw == 128 ? 128 : (p.out_pw == 64 ? 64 : 0);
         if ((st = make_map(&mo, d.output, (uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.ops, BLOCK_M, (uint32_t)p.out_pw, osw, (uint64_t)p.batch,
                            (uint64_t)p.M * (uint64_t)p.ops)))
@@ -1138,11 +1239,13 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
             attr_err = cudaFuncSetAttribute(gemm_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
         if (attr_err == cudaSuccess)
             attr_err = cudaFuncSetAttribute(gemm_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(gemm_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
     });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(gemm_tc_kernel)");
     if (i16)
-        launch_overlapped(gemm_tc_kernel<true, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
+        launch_overlapped(p.epi.half_even ? gemm_tc_kernel<true, true> : gemm_tc_kernel<true, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
     else
         launch_overlapped(p.epi.half_even ? gemm_tc_kernel<false, true> : gemm_tc_kernel<false, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
     count_launch();
@@ -1180,10 +1283,9 @@ bool conv2d_packed_supported(const espdl_conv_desc &d)
     const bool i16 = d.dtype == ESPDL_DTYPE_INT16;
     if (d.group != 1 || d.filter_image_stride != 0 || (i16 && (d.lut || d.residual)))
         return false;
-    const long long M = (long long)d.n * d.out_h * d.out_w, K = (long long)d.kh * d.kw * d.in_c, macs = M * K * d.out_c;
-    // Against the CUDA-core kernel: that one needs no packing (two launches of a few microseconds) but makes 2.2 T (int8) or 0.5 T
-    // (int16) multiply-adds a second, and a thread of it walks the whole reduction.
-    if (K > (i16 ? 16384 : 65536) || M > 0x7fffffffll || (macs < (i16 ? 3000000 : 12000000) && K < 1024))
+    const long long M = (long long)d.n * d.out_h * d.out_w, K = (long long)d.kh * d.kw * d.in_c;
+    // Packing and product are two launches of a few microseconds each; below that the CUDA-core kernel reads the operands in place.
+    if (K > (i16 ? 16384 : 65536) || M > 0x7fffffffll || conv2d_simt_estimate_us(d) < (i16 ? 13.f : 11.f))
         return false;
     TcParams p;
     return plan(packed_product(d, packed_rows(d)), p);

@@ -117,6 +117,7 @@ static void download_dense(void *host, TensorBase *t, void *stream)
 }
 
 // ----------------------------------------------------------------------------- model
+static constexpr size_t PLAIN_STEP = 96u << 20;         // mean bytes of tensors per step from which launches are plain
 static constexpr size_t BRANCH_LIMIT = (size_t)1 << 30; // bytes of all tensors of a pass up to which its branches run side by side
 
 static bool env_flag(const char *name, bool def)
@@ -869,6 +870,9 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
             m_arena_bytes = bytes;
             m_branches = true;
         }
+        // Early-resident blocks crowd the SMs that finish first: a loss once a launch is long enough to hide the boundary anyway
+        // (classifier, 256 images = 64 MB a step: 1262 us plain, 1229 overlapped; 512: 2068, 2085; 1024: 3677, 3841)
+        m_plain_launches = !m_branches && bytes / std::max<size_t>(1, m_execution_plan.size()) > PLAIN_STEP;
     }
     if (!m_branches)
         m_arena_bytes = MemoryManagerGreedy::plan(infos, m_reuse_memory);

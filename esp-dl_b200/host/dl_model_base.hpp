@@ -144,6 +144,7 @@ protected:
     // Branches of the plan side by side in its graphs (dl_model_capture.cpp)
     static constexpr int MAX_BRANCHES = 6;
     bool m_branches = false;
+    bool m_plain_launches = false; ///< large steps: no overlap of a launch's start with the end of the one before it
     std::vector<void *> m_branch_streams;
     esp_err_t settle();
     esp_err_t capture_plan(int first, int last, bool io, void **graph);

@@ -175,7 +175,7 @@ esp_err_t Model::capture_plan(int first, int last, bool io, void **graph)
         for (int d : it.after)
             if (!st && items[d].stream != it.stream)
                 st = espdl_b200_stream_wait_event(stream, events[d]);
-        if (!it.chained)
+        if (!it.chained || m_plain_launches)
             espdl_b200_overlap(0); // joins: plain edges
         if (!st && it.io) {
             st = it.upload ? espdl_b200_upload(it.io->device, it.io->data, it.io->get_bytes(), stream)
@@ -187,8 +187,7 @@ esp_err_t Model::capture_plan(int first, int last, bool io, void **graph)
                 st = m_status ? m_status : ESPDL_ERR_CUDA;
             ctx->stream = own;
         }
-        if (!it.chained)
-            espdl_b200_overlap(1);
+        espdl_b200_overlap(1);
         if (it.event)
             record(j, stream);
     }

@@ -62,3 +62,25 @@ def test_batch_of_products_on_the_cuda_cores(k, n, dtype):
         one = cases.conv_case(seed=1, n=1, h=1, w=rows, cin=k, cout=n, kh=1, kw=1, pad=(0, 0, 0, 0), bias=False, **extra)
         one.update(x=x[i:i + 1], w=w[i], filter_exponent=whole["filter_exponent"])
         np.testing.assert_array_equal(got[i:i + 1], gpu_util.run_conv_oracle(one))
+
+
+# staged rows of every alignment: widths around the word, the 16-byte chunk and the tile, rows that start anywhere
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("m,k,n,stride,lut", [(130, 64, 15, 0, False), (257, 96, 17, 0, True), (100, 32, 127, 0, False), (300, 160, 129, 131, False), (128, 48, 301, 0, True),
+                                              (64, 512, 333, 350, False), (1, 64, 1001, 0, False), (4096, 16, 9, 0, False), (20000, 64, 37, 0, False)])
+def test_rows_of_any_alignment(m, k, n, stride, lut, dtype):
+    kw = dict(S16, wide=True) if dtype == abi.DTYPE_INT16 else dict(lut=lut)
+    for round_mode in (abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN):
+        case = cases.gemm_case(seed=n, m=m, k=k, n_out=n, per_channel=True, round_mode=round_mode, out_stride=stride, **kw)
+        case["out"][...] = 0x55
+        want = gpu_util.run_conv_oracle(case)
+        np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+
+
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("kw", [dict(n=1, h=1, w=1, cin=40, cout=7, kh=1, kw=1, pad=(0, 0, 0, 0)), dict(n=3, h=5, w=4, cin=7, cout=5), dict(n=1, h=9, w=9, cin=8, cout=8, kh=5, kw=5),
+                                dict(n=1, h=1, w=1, cin=1000, cout=3, kh=1, kw=1, pad=(0, 0, 0, 0)), dict(n=2, h=13, w=11, cin=12, cout=9, stride=2, dil=2)])
+def test_reductions_shared_by_lanes(kw, dtype):
+    extra = dict(S16, wide=True) if dtype == abi.DTYPE_INT16 else {}
+    case = cases.conv_case(seed=4, per_channel=True, act=abi.ACT_LINEAR, **dict(extra, **kw))
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_SIMT), gpu_util.run_conv_oracle(case))
