@@ -11,6 +11,8 @@
 // rounded on its own (no fused multiply-add), as in the reference built without contraction.
 #include "common.cuh"
 
+#include <mutex>
+
 namespace espdl {
 
 namespace {
@@ -232,6 +234,178 @@ __global__ void __launch_bounds__(256) norm_kernel(NormParams p, int early)
     }
 }
 
+// LayerNormalization with the rows of a block side by side in shared memory.  The variance is an ordered fp32 sum, so a row
+// costs `len` dependent additions whoever does them; a warp per row made all 32 lanes do the same ones.  Here a thread walks one
+// row (row pitch an odd number of words: thread r reading word i of row r meets no bank conflict), 32 rows of a warp side by
+// side, and the normalising pass gives every thread fixed columns, whose scale and bias stay in registers while it goes
+// down the rows.  Bound by instruction issue: about 5 instructions an element for the variance, 8 for the normalisation.
+// WORDS: rows are whole aligned words in global memory; otherwise the block's rows, one contiguous run of bytes, are dealt out to
+// and collected from the padded rows byte by byte.
+template <typename T, bool WORDS>
+__global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, int pitch, int early)
+{
+    if (early)
+        grid_dep_launch();
+    grid_dep_wait();
+    constexpr int V = Word<T>::V;
+    extern __shared__ __align__(16) uint32_t rows_s[]; // R x pitch words, then per row {mean, 1 / std}
+    float2 *stats = (float2 *)(rows_s + (size_t)R * pitch + ((R * pitch) & 1));
+    const int words = (p.len + V - 1) / V, row_bytes = p.len * (int)sizeof(T);
+    const long long groups = (p.rows + R - 1) / R;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (long long g = blockIdx.x; g < groups; g += gridDim.x) {
+        const long long r0 = g * R;
+        const int nr = (int)min((long long)R, p.rows - r0);
+        const uint32_t *src = (const uint32_t *)((const T *)p.in + r0 * p.len); // R is a multiple of 4: word aligned
+        const int total = nr * row_bytes;
+        __syncthreads();
+        if (WORDS) {
+            for (int rr = warp; rr < nr; rr += 8)
+                for (int i = lane; i < words; i += 32) rows_s[rr * pitch + i] = src[(long long)rr * words + i];
+        } else {
+            for (int w = threadIdx.x; 4 * w < total; w += 256) {
+                uint32_t v = 0;
+                if (4 * w + 4 <= total)
+                    v = src[w];
+                else
+                    for (int k = 0; 4 * w + k < total; k++) v |= (uint32_t)((const uint8_t *)src)[4 * w + k] << (8 * k);
+                int rr = 4 * w / row_bytes, o = 4 * w - rr * row_bytes;
+#pragma unroll
+                for (int k = 0; k < 4; k += (int)sizeof(T)) {
+                    if (rr < nr)
+                        *(T *)((uint8_t *)(rows_s + rr * pitch) + o) = (T)(v >> (8 * k));
+                    o += (int)sizeof(T);
+                    if (o == row_bytes)
+                        o = 0, rr++;
+                }
+            }
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < nr) {
+            const uint32_t *row = rows_s + threadIdx.x * pitch;
+            const int full = p.len / V;
+            int sum = 0;
+            for (int i = 0; i < full; i++) {
+                Word<T> a{row[i]};
+                if (V == 4) {
+                    sum = __dp4a((int)a.w, 0x01010101, sum);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < V; k++) sum += a.get(k);
+                }
+            }
+            Word<T> last{full < words ? row[full] : 0u};
+#pragma unroll
+            for (int k = 0; k < V; k++)
+                if (full * V + k < p.len)
+                    sum += last.get(k);
+            float mean = (float)((double)sum * 1.0 / (double)p.len);
+            float var = 0.f;
+            auto add = [&](int x) {
+                const float d = __fsub_rn(__int2float_rn(x), mean);
+                var = __fadd_rn(var, __fmul_rn(d, d));
+            };
+#pragma unroll 4
+            for (int i = 0; i < full; i++) {
+                Word<T> a{row[i]};
+#pragma unroll
+                for (int k = 0; k < V; k++) add(a.get(k));
+            }
+#pragma unroll
+            for (int k = 0; k < V; k++)
+                if (full * V + k < p.len)
+                    add(last.get(k));
+            const long long out_row = r0 + threadIdx.x;
+            if (p.mean)
+                store_q((T *)p.mean, out_row, fround(__fmul_rn(__fmul_rn(mean, p.mean_rescale), p.in_scale), p.half_even));
+            mean = __fmul_rn(mean, p.in_scale);
+            var = __fmul_rn(var, __fmul_rn(p.in_scale, p.in_scale));
+            var = __fdiv_rn(var, __int2float_rn(p.len));
+            const float inv_std = __fdiv_rn(1.0f, sqrt_newton_dev(__fadd_rn(var, p.epsilon)));
+            if (p.inv_std)
+                store_q((T *)p.inv_std, out_row, fround(__fmul_rn(inv_std, p.inv_std_rescale), p.half_even));
+            stats[threadIdx.x] = make_float2(mean, inv_std);
+        }
+        __syncthreads();
+        const T *sc = (const T *)p.scale, *bi = (const T *)p.bias;
+        const int across = min(words, 256), down = 256 / across; // threads along a row, rows at a time
+        const int first_row = threadIdx.x / across;
+        uint32_t *dst = (uint32_t *)((T *)p.out + r0 * p.len);
+        for (int cw = threadIdx.x % across; cw < words && first_row < down; cw += across) {
+            float sv[V], bv[V];
+#pragma unroll
+            for (int k = 0; k < V; k++) {
+                const int e = min(cw * V + k, p.len - 1);
+                sv[k] = sc ? __fmul_rn(__int2float_rn((int)sc[e]), p.scale_scale) : 1.0f;
+                bv[k] = bi ? __fmul_rn(__int2float_rn((int)bi[e]), p.bias_scale) : 0.0f;
+            }
+            for (int rr = first_row; rr < nr; rr += down) {
+                const float2 st = stats[rr];
+                Word<T> a{rows_s[rr * pitch + cw]};
+                int q[V];
+#pragma unroll
+                for (int k = 0; k < V; k++) {
+                    // products with a power of two are exact, so a fused multiply-add there rounds as the separate operations do
+                    const float d = __fmaf_rn(__int2float_rn(a.get(k)), p.in_scale, -st.x);
+                    const float y = __fadd_rn(__fmul_rn(__fmul_rn(d, st.y), sv[k]), bv[k]);
+                    q[k] = p.half_even ? __float2int_rn(__fmul_rn(y, p.out_rescale)) : __float2int_rd(__fmaf_rn(y, p.out_rescale, 0.5f));
+                }
+                uint32_t w;
+                if (V == 4) {
+                    uint32_t hi;
+                    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(q[V - 1]), "r"(q[V - 2]));
+                    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q[1]), "r"(q[0]), "r"(hi));
+                } else {
+                    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(w) : "r"(q[1]), "r"(q[0]));
+                }
+                if (WORDS)
+                    dst[(long long)rr * words + cw] = w;
+                else
+                    rows_s[rr * pitch + cw] = w;
+            }
+        }
+        if (!WORDS) {
+            __syncthreads();
+            for (int w = threadIdx.x; 4 * w < total; w += 256) {
+                int rr = 4 * w / row_bytes, o = 4 * w - rr * row_bytes;
+                uint32_t v = 0;
+#pragma unroll
+                for (int k = 0; k < 4; k += (int)sizeof(T)) {
+                    if (rr < nr)
+                        v |= (sizeof(T) == 1 ? (uint32_t)*((const uint8_t *)(rows_s + rr * pitch) + o) : (uint32_t)*(const uint16_t *)((const uint8_t *)(rows_s + rr * pitch) + o)) << (8 * k);
+                    o += (int)sizeof(T);
+                    if (o == row_bytes)
+                        o = 0, rr++;
+                }
+                if (4 * w + 4 <= total)
+                    dst[w] = v;
+                else
+                    for (int k = 0; 4 * w + k < total; k++) ((uint8_t *)dst)[4 * w + k] = (uint8_t)(v >> (8 * k));
+            }
+        }
+    }
+}
+
+template <typename T>
+int launch_layer_rows(const NormParams &p, int R, int pitch, cudaStream_t s)
+{
+    const bool words = p.len % Word<T>::V == 0;
+    const size_t smem = ((size_t)R * pitch + 1) * 4 + (size_t)R * sizeof(float2);
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(layer_rows_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(layer_rows_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    });
+    if (attr_err != cudaSuccess)
+        return set_cuda_error(attr_err, "cudaFuncSetAttribute(layer_rows_kernel)");
+    const long long groups = (p.rows + R - 1) / R;
+    launch_mover(words ? layer_rows_kernel<T, true> : layer_rows_kernel<T, false>, dim3((unsigned)min(groups, (long long)num_sms() * 8)), dim3(256), smem, s, p, R, pitch);
+    count_launch();
+    return check_launch("layer norm");
+}
+
 } // namespace
 
 } // namespace espdl
@@ -262,6 +436,14 @@ extern "C" int espdl_b200_norm(const espdl_norm_desc *d, void *stream)
     p.scale_scale = dl_scale(d->scale_exponent), p.bias_scale = dl_scale(d->bias_exponent);
     p.mean_rescale = dl_rescale(d->mean_exponent), p.inv_std_rescale = dl_rescale(d->inv_std_dev_exponent);
     p.epsilon = d->epsilon;
+    if (d->op == ESPDL_NORM_LAYER && ((uintptr_t)d->input % 4) == 0 && ((uintptr_t)d->output % 4) == 0) {
+        // rows a block: 48 KB of them (four blocks an SM keep eight warps at their rows), fewer where that leaves SMs without a block
+        const int V = d->dtype == ESPDL_DTYPE_INT8 ? 4 : 2, pitch = ((d->len + V - 1) / V) | 1;
+        const long long fit = (50 * 1024) / ((long long)pitch * 4 + 8), share = (d->rows + num_sms() - 1) / num_sms();
+        const int R = (int)min(min(256ll, max(fit, (96 * 1024) / ((long long)pitch * 4 + 8) >= 32 ? 32ll : 0ll)), max(32ll, share)) / 32 * 32;
+        if (R >= 32 && d->rows >= 256)
+            return d->dtype == ESPDL_DTYPE_INT8 ? launch_layer_rows<int8_t>(p, R, pitch, (cudaStream_t)stream) : launch_layer_rows<int16_t>(p, R, pitch, (cudaStream_t)stream);
+    }
     const long long blocks = (d->rows + 7) / 8; // eight rows (warps) per block
     const unsigned grid = (unsigned)min(blocks, (long long)num_sms() * 8);
     if (d->dtype == ESPDL_DTYPE_INT8)

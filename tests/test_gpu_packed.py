@@ -84,3 +84,45 @@ def test_reductions_shared_by_lanes(kw, dtype):
     extra = dict(S16, wide=True) if dtype == abi.DTYPE_INT16 else {}
     case = cases.conv_case(seed=4, per_channel=True, act=abi.ACT_LINEAR, **dict(extra, **kw))
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_SIMT), gpu_util.run_conv_oracle(case))
+
+
+@pytest.mark.parametrize("sa,sb", [((3, 2, 5, 16), (1, 2, 16, 7)), ((4, 3, 9, 12), (4, 1, 12, 20)), ((2, 3, 6, 32), (1, 3, 32, 32))])
+def test_matmul_whose_second_operand_repeats_over_some_slices(sa, sb, tmp_path):
+    import checkers
+    import graph_oracle
+    from espdl_b200 import espdl_file, model
+    rng = np.random.default_rng(5)
+    w = rng.integers(-60, 60, size=sb, dtype=np.int8)
+    g = espdl_file.GraphBuilder("matmul_spread", metadata={"target": "c"})
+    g.add_input("a", np.int8, list(sa), -5)
+    g.add_initializer("w", w, [-6])
+    g.add_node("MatMul", "mm", ["a", "w"], ["y"], quant_type="S8", activation="Linear")
+    so = [max(x, y) for x, y in zip(sa[:2], sb[:2])] + [sa[2], sb[3]]
+    g.add_output("y", np.int8, so, -3)
+    path = str(tmp_path / "m.espdl")
+    g.save(path)
+    m = model.Model(path)
+    a = rng.integers(-60, 60, size=sa, dtype=np.int8)
+    m.inputs[0].array[...] = a
+    m.run()
+    want = graph_oracle.matmul(checkers.oracle(), a, w, -5, -6, -3, abi.DTYPE_INT8, abi.ACT_LINEAR, abi.ROUND_HALF_UP)
+    np.testing.assert_array_equal(np.asarray(m.outputs[0].array).reshape(so), want.reshape(so))
+    m.close()
+
+
+@pytest.mark.parametrize("dt", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("rows,n", [(300, 768), (259, 33), (1000, 1), (257, 1022), (600, 100), (5000, 17), (256, 2050)])
+def test_layer_norm_rows_side_by_side(rows, n, dt):
+    import ctypes as C
+    import checkers
+    import test_norm
+    for stats, round_mode in ((True, abi.ROUND_HALF_UP), (False, abi.ROUND_HALF_EVEN)):
+        a = test_norm.make(abi.NORM_LAYER, dt, rows, n, seed=n, stats=stats, round_mode=round_mode)
+        want = test_norm.fresh(a)
+        assert checkers.oracle().oracle_norm(C.byref(test_norm.desc(want))) == 0
+        with gpu_util.DeviceBuffers() as dev:
+            ptrs = {k: dev.upload(a[k]) for k in ("x", "y", "scale", "bias", "mean", "inv") if a[k] is not None}
+            abi.check(dev.lib.espdl_b200_norm(C.byref(test_norm.desc(a, ptrs)), None), "norm")
+            for k in ("y", "mean", "inv"):
+                if a[k] is not None:
+                    np.testing.assert_array_equal(dev.download(ptrs[k], want[k]), want[k], err_msg=k)
