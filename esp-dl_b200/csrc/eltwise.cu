@@ -1,8 +1,8 @@
 // Elementwise operators of the quantized path: Add / Sub / Mul with numpy broadcasting,
 // RequantizeLinear (TensorBase::assign), 8-bit LUT activations, Clip, ReLU, PReLU.
-// All are bandwidth bound.  The int8 same-shape case (what a network's residual Adds, LUT
-// activations and requantize nodes are) runs a 128-bit vectorised kernel; everything else
-// (broadcast operands, int16, float endpoints) runs a strided scalar kernel.
+// All are bandwidth bound.  Operands of one shape (a network's residual Adds, LUT activations and requantize nodes) and a
+// second operand that repeats over the rows of an image (a squeeze-and-excite gate) run 128-bit vectorised kernels, int8 and
+// int16; everything else (other broadcasts, mixed types, float endpoints) runs a strided scalar kernel.
 //
 // Arithmetic follows the reference exactly, including its fp32 sequences:
 //   Add/Sub  esp-dl/dl/base/dl_base_add.cpp:8-44      Mul   esp-dl/dl/base/dl_base_mul.cpp:9-46
@@ -33,6 +33,7 @@ struct EltParams {
     // rows of the innermost axis that do not follow one another in memory (channel slices of a wider tensor): element
     // strides between rows of the output / the operands; 0 = dense.  Vector kernels: the same in 16-byte units.
     long long ro, ra, rb;
+    long long rows_per_image, b_image; // broadcast second operand: rows that share one, units from one to the next
     int vpr; // 16-byte units per row (vector kernels, strided rows only; 0 = flat)
     int vpr_shift; // log2(vpr) when it is a power of two, else -1
 };
@@ -145,6 +146,20 @@ __device__ __forceinline__ long long elt_int(const EltParams &p, long long a, lo
     }
 }
 
+// int16 LUT: nearest table entry, index = ((uint16)x ^ 0x8000) >> shift, rounded (dl_base_lut.cpp:50-69)
+__device__ __forceinline__ uint32_t lut16_index(const EltParams &p, int x)
+{
+    const uint32_t value = (uint32_t)(uint16_t)x ^ 0x8000u;
+    uint32_t index = value;
+    if (p.lut_shift > 0) {
+        index = value >> p.lut_shift;
+        const uint32_t rem = value & ((1u << p.lut_shift) - 1u), half = 1u << (p.lut_shift - 1);
+        if (p.half_even ? (rem > half || (rem == half && (index & 1u))) : rem >= half)
+            index++;
+    }
+    return index;
+}
+
 __global__ void __launch_bounds__(256) elt_generic_kernel(EltParams p, int early)
 {
     if (early)
@@ -162,16 +177,7 @@ __global__ void __launch_bounds__(256) elt_generic_kernel(EltParams p, int early
         const long long bi = i3 * p.sb[0] + i2 * p.sb[1] + i1 * p.sb[2] + i0 * p.sb[3];
         const long long oi = p.ro ? (i / p.os[3]) * p.ro + i0 : i;
         if (p.op == ESPDL_ELT_LUT && p.idt == ESPDL_DTYPE_INT16) {
-            // nearest table entry: index = ((uint16)x ^ 0x8000) >> shift, rounded (dl_base_lut.cpp:50-69)
-            const uint32_t value = (uint32_t)(uint16_t)((const int16_t *)p.a)[ai] ^ 0x8000u;
-            uint32_t index = value;
-            if (p.lut_shift > 0) {
-                index = value >> p.lut_shift;
-                const uint32_t rem = value & ((1u << p.lut_shift) - 1u), half = 1u << (p.lut_shift - 1);
-                if (p.half_even ? (rem > half || (rem == half && (index & 1u))) : rem >= half)
-                    index++;
-            }
-            ((int16_t *)p.out)[oi] = ((const int16_t *)p.b)[index];
+            ((int16_t *)p.out)[oi] = ((const int16_t *)p.b)[lut16_index(p, ((const int16_t *)p.a)[ai])];
         } else if (p.op == ESPDL_ELT_LUT) {
             ((int8_t *)p.out)[oi] = ((const int8_t *)p.b)[(uint8_t)((const int8_t *)p.a)[ai] ^ 0x80u];
         } else if (p.op == ESPDL_ELT_REQUANTIZE && p.idt == ESPDL_DTYPE_FLOAT) {
@@ -190,32 +196,56 @@ __global__ void __launch_bounds__(256) elt_generic_kernel(EltParams p, int early
     }
 }
 
-// int8 -> int8, operands of identical shape, 16 elements per thread.
-template <int OP>
-__global__ void __launch_bounds__(256) elt_s8_vec16_kernel(EltParams p, long long nvec, int early)
+// 16 bytes per thread: int8 or int16 in and out, operands of one shape or (BCAST) the second one repeated over the rows of an image - a
+// gate [n][1][1][c] over a map [n][h][w][c].  Flat tensors of any length: what does not fill a unit is done by single threads.
+// (int16 and lengths that are no multiple of 16 ran a strided scalar kernel: 0.75 TB/s and 0.37 TB/s against 5.8 here.)
+template <int OP, typename T, bool BCAST>
+__global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nvec, int early)
 {
     if (early)
         grid_dep_launch();
     grid_dep_wait();
+    constexpr int V = 16 / (int)sizeof(T), PER_WORD = 4 / (int)sizeof(T), BITS = 8 * (int)sizeof(T);
     __shared__ int8_t table[256];
     // One-operand int8 -> int8 operators are functions of the input byte: every block tabulates the operator once with
     // the scalar code (so the rounding is the reference's) and then runs as a table lookup like LUT itself.
-    constexpr bool TABULATED = OP == ESPDL_ELT_REQUANTIZE || OP == ESPDL_ELT_CLIP || OP == ESPDL_ELT_RELU;
-    if (OP == ESPDL_ELT_LUT) {
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) table[i] = ((const int8_t *)p.b)[i];
-        __syncthreads();
-    } else if (TABULATED) {
+    constexpr bool TABULATED = sizeof(T) == 1 && (OP == ESPDL_ELT_REQUANTIZE || OP == ESPDL_ELT_CLIP || OP == ESPDL_ELT_RELU);
+    constexpr bool LOOKUP = sizeof(T) == 1 && (OP == ESPDL_ELT_LUT || TABULATED);
+    if (LOOKUP) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-            EltParams q2 = p;
-            q2.op = OP;
-            const int a = (int)(int8_t)(uint8_t)(i ^ 0x80);
-            table[i] = (int8_t)sat8((int)max(-1000000ll, min(1000000ll, elt_int(q2, a, 0))));
+            if (OP == ESPDL_ELT_LUT) {
+                table[i] = ((const int8_t *)p.b)[i];
+            } else {
+                EltParams q2 = p;
+                q2.op = OP;
+                table[i] = (int8_t)sat8((int)max(-1000000ll, min(1000000ll, elt_int(q2, (int)(int8_t)(uint8_t)(i ^ 0x80), 0))));
+            }
         }
         __syncthreads();
     }
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvec; v += (long long)gridDim.x * blockDim.x) {
+    auto one = [&](int a, int b) -> int {
+        if (LOOKUP)
+            return table[(uint8_t)a ^ 0x80u];
+        if (OP == ESPDL_ELT_LUT) // int16
+            return ((const int16_t *)p.b)[lut16_index(p, a)];
+        long long v = OP == ESPDL_ELT_ADD ? a + b : (OP == ESPDL_ELT_SUB ? a - b : 0);
+        if (OP != ESPDL_ELT_ADD && OP != ESPDL_ELT_SUB) {
+            EltParams q2 = p;
+            q2.op = OP;
+            v = elt_int(q2, a, b);
+        }
+        const int lo = -(1 << (BITS - 1));
+        return (int)max((long long)lo, min((long long)(-lo - 1), v));
+    };
+    const long long threads = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long v = first; v < nvec; v += threads) {
         long long io, ia, ib;
-        vec_offsets(p, v, io, ia, ib);
+        if (BCAST) {
+            const long long row = v < 0x7fffffffll ? (long long)((unsigned)v / (unsigned)p.vpr) : v / p.vpr, col = v - row * p.vpr;
+            io = row * p.ro + col, ia = row * p.ra + col, ib = row / p.rows_per_image * p.b_image + col;
+        } else {
+            vec_offsets(p, v, io, ia, ib);
+        }
         const uint4 a4 = ((const uint4 *)p.a)[ia];
         uint4 b4 = make_uint4(0, 0, 0, 0);
         if (elt_two_operands(OP))
@@ -227,27 +257,17 @@ __global__ void __launch_bounds__(256) elt_s8_vec16_kernel(EltParams p, long lon
         for (int q = 0; q < 4; q++) {
             uint32_t wd = 0;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int a = (int)(int8_t)(aw[q] >> (8 * j));
-                const int b = (int)(int8_t)(bw[q] >> (8 * j));
-                int r;
-                if (OP == ESPDL_ELT_LUT || TABULATED) {
-                    r = table[(uint8_t)a ^ 0x80u];
-                } else if (OP == ESPDL_ELT_ADD) {
-                    r = sat8(a + b);
-                } else if (OP == ESPDL_ELT_SUB) {
-                    r = sat8(a - b);
-                } else {
-                    EltParams q2 = p;
-                    q2.op = OP;
-                    r = sat8((int)max(-1000000ll, min(1000000ll, elt_int(q2, a, b))));
-                }
-                wd |= ((uint32_t)r & 0xffu) << (8 * j);
+            for (int j = 0; j < PER_WORD; j++) {
+                const int a = (int)(T)(aw[q] >> (BITS * j)), b = (int)(T)(bw[q] >> (BITS * j));
+                wd |= ((uint32_t)one(a, b) & ((1u << BITS) - 1u)) << (BITS * j);
             }
             ow[q] = wd;
         }
         ((uint4 *)p.out)[io] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
     }
+    if (!BCAST && !p.vpr)
+        for (long long i = nvec * V + first; i < p.total; i += threads)
+            ((T *)p.out)[i] = (T)one((int)((const T *)p.a)[i], elt_two_operands(OP) ? (int)((const T *)p.b)[i] : 0);
 }
 
 // int8 (op) one-element int8 -> int8 (Mul by a scalar factor, Add of a constant, ...): with the second operand fixed the
@@ -280,14 +300,27 @@ __global__ void __launch_bounds__(256) elt_s8_scalar_b_kernel(EltParams p, long 
         }
         ((uint4 *)p.out)[io] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
     }
+    if (!p.vpr)
+        for (long long i = nvec * 16 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x)
+            ((int8_t *)p.out)[i] = table[((const uint8_t *)p.a)[i] ^ 0x80u];
 }
 
 template <int OP>
-static void launch_vec(const EltParams &p, long long nvec, cudaStream_t s)
+static void launch_vec(const EltParams &p, long long nvec, bool bcast, cudaStream_t s)
 {
-    const int threads = 256;
-    long long blocks = min((nvec + threads - 1) / threads, (long long)num_sms() * 16);
-    launch_mover(elt_s8_vec16_kernel<OP>, dim3((unsigned)max(blocks, 1ll)), dim3(threads), 0, s, p, nvec);
+    const dim3 grid((unsigned)max(min((nvec + 255) / 256, (long long)num_sms() * 16), 1ll)), block(256);
+    constexpr bool two = OP == ESPDL_ELT_ADD || OP == ESPDL_ELT_SUB || OP == ESPDL_ELT_MUL || OP == ESPDL_ELT_MAX || OP == ESPDL_ELT_MIN;
+    constexpr bool compares = OP >= ESPDL_ELT_GREATER && OP <= ESPDL_ELT_LESS_EQUAL; // int16 in, a byte out: the scalar kernel
+    if constexpr (two) {
+        if (bcast)
+            launch_mover(p.idt == ESPDL_DTYPE_INT8 ? elt_vec_kernel<OP, int8_t, true> : elt_vec_kernel<OP, int16_t, true>, grid, block, 0, s, p, nvec);
+    }
+    if (bcast)
+        return;
+    if constexpr (compares)
+        launch_mover(elt_vec_kernel<OP, int8_t, false>, grid, block, 0, s, p, nvec);
+    else
+        launch_mover(p.idt == ESPDL_DTYPE_INT8 ? elt_vec_kernel<OP, int8_t, false> : elt_vec_kernel<OP, int16_t, false>, grid, block, 0, s, p, nvec);
 }
 
 } // namespace espdl
@@ -349,14 +382,19 @@ extern "C" int espdl_b200_eltwise(const espdl_eltwise_desc *d, void *stream)
     if (strided && d->op == ESPDL_ELT_DIV)
         return ESPDL_ERR_UNSUPPORTED; // Div reads the operands' element counts
     p.ro = rso;
-    const bool rows16 = !strided || (os[3] % 16 == 0 && rs0 % 16 == 0 && rs1 % 16 == 0 && rso % 16 == 0);
-    if (strided && rows16) {
-        p.vpr = os[3] / 16;
+    const int V = d->in_dtype == ESPDL_DTYPE_INT16 ? 8 : 16; // elements per 16-byte unit
+    const bool rows16 = !strided || (os[3] % V == 0 && rs0 % V == 0 && rs1 % V == 0 && rso % V == 0);
+    // the second operand repeats over the rows of an image: [n or 1][1][1][c] beside [n][h][w][c]
+    const bool bcast = binary && !same && s0[0] == os[0] && s0[1] == os[1] && s0[2] == os[2] && s0[3] == os[3] && s1[3] == os[3] && s1[1] == 1 && s1[2] == 1 &&
+        os[3] % V == 0 && rows16;
+    if ((strided && rows16) || bcast) {
+        p.vpr = os[3] / V;
         p.vpr_shift = -1;
         for (int sft = 0; sft < 16; sft++)
             if ((1 << sft) == p.vpr)
                 p.vpr_shift = sft;
-        p.ra = (rs0 ? rs0 : os[3]) / 16, p.rb = (rs1 ? rs1 : os[3]) / 16;
+        p.ra = (rs0 ? rs0 : os[3]) / V, p.rb = (rs1 ? rs1 : os[3]) / V;
+        p.rows_per_image = (long long)os[1] * os[2], p.b_image = p.sb[0] / V;
     }
     p.a = d->input0, p.b = d->input1, p.out = d->output;
     p.op = d->op, p.idt = d->in_dtype, p.odt = d->out_dtype;
@@ -386,39 +424,42 @@ extern "C" int espdl_b200_eltwise(const espdl_eltwise_desc *d, void *stream)
     p.prelu_shift = p.eo - p.e0 - p.e1;
     p.total = total;
     cudaStream_t s = (cudaStream_t)stream;
-    const bool vec = same && rows16 && d->in_dtype == ESPDL_DTYPE_INT8 && (d->out_dtype == ESPDL_DTYPE_INT8 || compare) && total % 16 == 0 &&
-        ((uintptr_t)d->input0 % 16) == 0 && ((uintptr_t)d->output % 16) == 0 && (!binary || ((uintptr_t)d->input1 % 16) == 0) &&
-        d->op != ESPDL_ELT_PRELU && d->op != ESPDL_ELT_POW;
+    const bool aligned = ((uintptr_t)d->input0 % 16) == 0 && ((uintptr_t)d->output % 16) == 0 && (!binary || ((uintptr_t)d->input1 % 16) == 0);
+    const bool int8_ok = d->in_dtype == ESPDL_DTYPE_INT8 && (d->out_dtype == ESPDL_DTYPE_INT8 || compare);
+    const bool int16_ok = d->in_dtype == ESPDL_DTYPE_INT16 && d->out_dtype == ESPDL_DTYPE_INT16;
+    const bool gate = bcast && aligned && (int8_ok || int16_ok) &&
+        (d->op == ESPDL_ELT_ADD || d->op == ESPDL_ELT_SUB || d->op == ESPDL_ELT_MUL || d->op == ESPDL_ELT_MAX || d->op == ESPDL_ELT_MIN);
+    const bool vec = gate || (same && rows16 && aligned && (int8_ok || int16_ok) && d->op != ESPDL_ELT_PRELU && d->op != ESPDL_ELT_POW);
     // second operand of one element, first operand of the output's shape
     bool a_full = true;
     for (int i = 0; i < 4; i++) a_full = a_full && s0[i] == os[i];
-    const bool scalar_b = binary && !compare && !same && a_full && b == 1 && rows16 && d->in_dtype == ESPDL_DTYPE_INT8 && d->out_dtype == ESPDL_DTYPE_INT8 &&
-        total % 16 == 0 && ((uintptr_t)d->input0 % 16) == 0 && ((uintptr_t)d->output % 16) == 0 && d->op != ESPDL_ELT_POW;
+    const bool scalar_b = !gate && binary && !compare && !same && a_full && b == 1 && rows16 && d->in_dtype == ESPDL_DTYPE_INT8 && d->out_dtype == ESPDL_DTYPE_INT8 &&
+        ((uintptr_t)d->input0 % 16) == 0 && ((uintptr_t)d->output % 16) == 0 && d->op != ESPDL_ELT_POW;
     if ((scalar_b || vec) && p.vpr)
-        p.ro = (rso ? rso : os[3]) / 16;
+        p.ro = (rso ? rso : os[3]) / V;
     if (scalar_b) {
         const long long nvec = total / 16;
         const long long blocks = min((nvec + 255) / 256, (long long)num_sms() * 16);
         launch_mover(elt_s8_scalar_b_kernel, dim3((unsigned)max(blocks, 1ll)), dim3(256), 0, s, p, nvec);
     } else if (vec) {
-        const long long nvec = total / 16;
+        const long long nvec = total / V;
         switch (d->op) {
-        case ESPDL_ELT_ADD: launch_vec<ESPDL_ELT_ADD>(p, nvec, s); break;
-        case ESPDL_ELT_SUB: launch_vec<ESPDL_ELT_SUB>(p, nvec, s); break;
-        case ESPDL_ELT_MUL: launch_vec<ESPDL_ELT_MUL>(p, nvec, s); break;
-        case ESPDL_ELT_REQUANTIZE: launch_vec<ESPDL_ELT_REQUANTIZE>(p, nvec, s); break;
-        case ESPDL_ELT_LUT: launch_vec<ESPDL_ELT_LUT>(p, nvec, s); break;
-        case ESPDL_ELT_CLIP: launch_vec<ESPDL_ELT_CLIP>(p, nvec, s); break;
-        case ESPDL_ELT_RELU: launch_vec<ESPDL_ELT_RELU>(p, nvec, s); break;
-        case ESPDL_ELT_MAX: launch_vec<ESPDL_ELT_MAX>(p, nvec, s); break;
-        case ESPDL_ELT_MIN: launch_vec<ESPDL_ELT_MIN>(p, nvec, s); break;
-        case ESPDL_ELT_DIV: launch_vec<ESPDL_ELT_DIV>(p, nvec, s); break;
-        case ESPDL_ELT_MOD: launch_vec<ESPDL_ELT_MOD>(p, nvec, s); break;
-        case ESPDL_ELT_GREATER: launch_vec<ESPDL_ELT_GREATER>(p, nvec, s); break;
-        case ESPDL_ELT_GREATER_EQUAL: launch_vec<ESPDL_ELT_GREATER_EQUAL>(p, nvec, s); break;
-        case ESPDL_ELT_EQUAL: launch_vec<ESPDL_ELT_EQUAL>(p, nvec, s); break;
-        case ESPDL_ELT_LESS: launch_vec<ESPDL_ELT_LESS>(p, nvec, s); break;
-        case ESPDL_ELT_LESS_EQUAL: launch_vec<ESPDL_ELT_LESS_EQUAL>(p, nvec, s); break;
+        case ESPDL_ELT_ADD: launch_vec<ESPDL_ELT_ADD>(p, nvec, gate, s); break;
+        case ESPDL_ELT_SUB: launch_vec<ESPDL_ELT_SUB>(p, nvec, gate, s); break;
+        case ESPDL_ELT_MUL: launch_vec<ESPDL_ELT_MUL>(p, nvec, gate, s); break;
+        case ESPDL_ELT_REQUANTIZE: launch_vec<ESPDL_ELT_REQUANTIZE>(p, nvec, gate, s); break;
+        case ESPDL_ELT_LUT: launch_vec<ESPDL_ELT_LUT>(p, nvec, gate, s); break;
+        case ESPDL_ELT_CLIP: launch_vec<ESPDL_ELT_CLIP>(p, nvec, gate, s); break;
+        case ESPDL_ELT_RELU: launch_vec<ESPDL_ELT_RELU>(p, nvec, gate, s); break;
+        case ESPDL_ELT_MAX: launch_vec<ESPDL_ELT_MAX>(p, nvec, gate, s); break;
+        case ESPDL_ELT_MIN: launch_vec<ESPDL_ELT_MIN>(p, nvec, gate, s); break;
+        case ESPDL_ELT_DIV: launch_vec<ESPDL_ELT_DIV>(p, nvec, gate, s); break;
+        case ESPDL_ELT_MOD: launch_vec<ESPDL_ELT_MOD>(p, nvec, gate, s); break;
+        case ESPDL_ELT_GREATER: launch_vec<ESPDL_ELT_GREATER>(p, nvec, gate, s); break;
+        case ESPDL_ELT_GREATER_EQUAL: launch_vec<ESPDL_ELT_GREATER_EQUAL>(p, nvec, gate, s); break;
+        case ESPDL_ELT_EQUAL: launch_vec<ESPDL_ELT_EQUAL>(p, nvec, gate, s); break;
+        case ESPDL_ELT_LESS: launch_vec<ESPDL_ELT_LESS>(p, nvec, gate, s); break;
+        case ESPDL_ELT_LESS_EQUAL: launch_vec<ESPDL_ELT_LESS_EQUAL>(p, nvec, gate, s); break;
         default: return ESPDL_ERR_UNSUPPORTED;
         }
     } else {

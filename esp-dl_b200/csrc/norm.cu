@@ -9,7 +9,7 @@
 // lanes compute the squared differences of 32 consecutive elements in parallel and then every lane adds the 32 values
 // in element order, so the sum is the reference's sequential sum bit for bit.  Every fp32 product, sum and quotient is
 // rounded on its own (no fused multiply-add), as in the reference built without contraction.
-#include "common.cuh"
+#include "rows.cuh"
 
 #include <mutex>
 
@@ -263,22 +263,7 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
             for (int rr = warp; rr < nr; rr += 8)
                 for (int i = lane; i < words; i += 32) rows_s[rr * pitch + i] = src[(long long)rr * words + i];
         } else {
-            for (int w = threadIdx.x; 4 * w < total; w += 256) {
-                uint32_t v = 0;
-                if (4 * w + 4 <= total)
-                    v = src[w];
-                else
-                    for (int k = 0; 4 * w + k < total; k++) v |= (uint32_t)((const uint8_t *)src)[4 * w + k] << (8 * k);
-                int rr = 4 * w / row_bytes, o = 4 * w - rr * row_bytes;
-#pragma unroll
-                for (int k = 0; k < 4; k += (int)sizeof(T)) {
-                    if (rr < nr)
-                        *(T *)((uint8_t *)(rows_s + rr * pitch) + o) = (T)(v >> (8 * k));
-                    o += (int)sizeof(T);
-                    if (o == row_bytes)
-                        o = 0, rr++;
-                }
-            }
+            deal_rows<T>(src, total, row_bytes, rows_s, pitch);
         }
         __syncthreads();
         if ((int)threadIdx.x < nr) {
@@ -366,22 +351,7 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
         }
         if (!WORDS) {
             __syncthreads();
-            for (int w = threadIdx.x; 4 * w < total; w += 256) {
-                int rr = 4 * w / row_bytes, o = 4 * w - rr * row_bytes;
-                uint32_t v = 0;
-#pragma unroll
-                for (int k = 0; k < 4; k += (int)sizeof(T)) {
-                    if (rr < nr)
-                        v |= (sizeof(T) == 1 ? (uint32_t)*((const uint8_t *)(rows_s + rr * pitch) + o) : (uint32_t)*(const uint16_t *)((const uint8_t *)(rows_s + rr * pitch) + o)) << (8 * k);
-                    o += (int)sizeof(T);
-                    if (o == row_bytes)
-                        o = 0, rr++;
-                }
-                if (4 * w + 4 <= total)
-                    dst[w] = v;
-                else
-                    for (int k = 0; 4 * w + k < total; k++) ((uint8_t *)dst)[4 * w + k] = (uint8_t)(v >> (8 * k));
-            }
+            collect_rows<T>(dst, total, row_bytes, rows_s, pitch);
         }
     }
 }

@@ -7,7 +7,7 @@
 // (esp-dl/dl/tensor/src/dl_tensor_base.cpp:251-264).  The softmax axis may be any axis: a "row" is the `len` elements
 // that lie `inner` apart.  LogSoftmax on int8 (dl_module_log_softmax.hpp:150-215) uses the same table and the same
 // sequential sum: y = 2^e_in * x - logf(sum), with logf evaluated on the device.
-#include "common.cuh"
+#include "rows.cuh"
 
 namespace espdl {
 
@@ -49,6 +49,17 @@ __global__ void __launch_bounds__(128) softmax_kernel(espdl_softmax_desc d, floa
     }
 }
 
+// round(t / sum * 2^-e) for an int8 output.  t * (1 / sum) * 2^-e lies within 1.9e-7 relative of the rounded quotient times the power
+// of two, 5e-5 absolute below 256 (from 128 on the code saturates): unless it is that close to a rounding boundary (one
+// element in some thousands) the division need not be made, and either rounding rule gives the nearest integer.
+__device__ __forceinline__ int quotient_code(float t, float sum, float recip, float out_rescale, int he)
+{
+    const float v = t * recip * out_rescale;
+    if (v < 256.f && fabsf(v - floorf(v) - 0.5f) > 1e-4f)
+        return __float2int_rn(v);
+    return fround(__fmul_rn(__fdiv_rn(t, sum), out_rescale), he);
+}
+
 // The same arithmetic with the rows side by side: a block stages R rows in shared memory (row pitch an odd number of
 // words, so that thread r reading byte i of row r meets no bank conflict), thread r adds row r's exponentials in index
 // order - R ordered sums run at once instead of one -, then all threads write the R x len results.  Used whenever at
@@ -61,7 +72,7 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
     __shared__ float table[256];
     extern __shared__ __align__(16) unsigned char sm[];
     float *sums = (float *)sm;               // R
-    int8_t *rows = (int8_t *)(sums + R);     // R x pitch
+    int8_t *rows = (int8_t *)(sums + R);     // R x pitch, word aligned
     for (int i = threadIdx.x; i < 256; i += blockDim.x) table[i] = d.exp_table[i];
     const int inner = d.inner > 1 ? d.inner : 1;
     const float in_scale = dl_scale(d.in_exponent);
@@ -71,6 +82,7 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
         const int r0 = g * R, nr = min(R, d.rows - r0);
         __syncthreads();
         const bool words = inner == 1 && d.len % 4 == 0 && (((uintptr_t)d.input) & 3) == 0; // whole 32-bit words per row
+        const bool spans = inner == 1 && (((uintptr_t)d.input) & 3) == 0; // R is a multiple of 4
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5, len4 = d.len >> 2;
         if (words) {
             // a warp per row, a word per lane: no index divisions, 128-byte global reads
@@ -79,8 +91,10 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
                 uint32_t *dst = (uint32_t *)(rows + rr * pitch);
                 for (int i = lane; i < len4; i += 32) dst[i] = src[i];
             }
-        } else if (inner == 1) {
+        } else if (spans) {
             // rows r0 .. r0 + nr - 1 are one contiguous span of nr * len bytes
+            deal_rows<int8_t>((const uint32_t *)(d.input + (long long)r0 * d.len), nr * d.len, d.len, (uint32_t *)rows, pitch / 4);
+        } else if (inner == 1) {
             const int8_t *src = d.input + (long long)r0 * d.len;
             for (int e = threadIdx.x; e < nr * d.len; e += blockDim.x) rows[(e / d.len) * pitch + e % d.len] = src[e];
         } else {
@@ -93,10 +107,39 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
         if ((int)threadIdx.x < nr) {
             const int8_t *row = rows + threadIdx.x * pitch;
             float sum = 0.f;
-            for (int i = 0; i < d.len; i++) sum = __fadd_rn(sum, table[row[i] + 128]);
+            const int full = d.len >> 2;
+#pragma unroll 2
+            for (int i = 0; i < full; i++) { // the row pitch is an odd number of words
+                const uint32_t w = ((const uint32_t *)row)[i];
+#pragma unroll
+                for (int j = 0; j < 4; j++) sum = __fadd_rn(sum, table[(int)(int8_t)(w >> (8 * j)) + 128]);
+            }
+            for (int i = 4 * full; i < d.len; i++) sum = __fadd_rn(sum, table[row[i] + 128]);
             sums[threadIdx.x] = d.log ? logf(sum) : sum;
         }
         __syncthreads();
+        if (spans && d.out_dtype == ESPDL_DTYPE_INT8 && !d.log && (((uintptr_t)d.output) & 3) == 0) {
+            // codes straight out where a row is whole words, else in place of the inputs and out as one span
+            const int row_words = (d.len + 3) >> 2;
+            for (int rr = warp; rr < nr; rr += nwarps) {
+                uint32_t *row = (uint32_t *)(rows + rr * pitch);
+                uint32_t *to = words ? (uint32_t *)((int8_t *)d.output + (long long)(r0 + rr) * d.len) : row;
+                const float sum = sums[rr], recip = __fdiv_rn(1.f, sum);
+                for (int i = lane; i < row_words; i += 32) {
+                    const uint32_t w = row[i];
+                    uint32_t q = 0;
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        q |= ((uint32_t)sat8(quotient_code(table[(int)(int8_t)(w >> (8 * j)) + 128], sum, recip, out_rescale, he)) & 0xffu) << (8 * j);
+                    to[i] = q;
+                }
+            }
+            if (!words) {
+                __syncthreads();
+                collect_rows<int8_t>((uint32_t *)((int8_t *)d.output + (long long)r0 * d.len), nr * d.len, d.len, (const uint32_t *)rows, pitch / 4);
+            }
+            continue;
+        }
         if (words && d.out_dtype != ESPDL_DTYPE_INT16) {
             for (int rr = warp; rr < nr; rr += nwarps) {
                 const uint32_t *src = (const uint32_t *)(rows + rr * pitch);
@@ -173,7 +216,7 @@ extern "C" int espdl_b200_softmax(const espdl_softmax_desc *d, void *stream)
     const int pitch = (((d->len + 3) / 4) | 1) * 4;
     const int fit = (40 * 1024) / (pitch + 4);
     if (fit >= 32 && d->rows >= 64) {
-        const int R = min(256, fit);
+        const int R = min(256, fit) / 4 * 4;
         const int groups = (d->rows + R - 1) / R;
         launch_mover(softmax_rows_kernel, dim3(min(groups, num_sms() * 8)), dim3(256), (size_t)R * (pitch + 4) + 16, (cudaStream_t)stream, *d, dl_rescale(d->out_exponent), R, pitch);
         count_launch();
