@@ -215,6 +215,7 @@ SYMBOLS = {
     "espdl_b200_overlap": (None, [C.c_int]),
     "espdl_b200_conv2d": (C.c_int, [C.POINTER(ConvDesc), C.c_void_p]),
     "espdl_b200_conv2d_workspace_bytes": (C.c_int, [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]),
+    "espdl_b200_conv2d_is_small": (C.c_int, [C.POINTER(ConvDesc)]),
     "espdl_b200_conv2d_ws": (C.c_int, [C.POINTER(ConvDesc), C.c_void_p, C.c_size_t, C.c_void_p]),
     "espdl_b200_gemm_s16_static": (C.c_int, [C.POINTER(ConvDesc), C.c_void_p]),
     "espdl_b200_eltwise": (C.c_int, [C.POINTER(EltwiseDesc), C.c_void_p]),

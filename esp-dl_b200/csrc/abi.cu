@@ -436,6 +436,30 @@ int espdl::conv_validate(const espdl_conv_desc *d)
     return ESPDL_OK;
 }
 
+// Small enough for the warp-level matrix instructions?
+static bool runs_mma(const espdl_conv_desc &d)
+{
+    const char *knob = getenv("ESPDL_B200_SMALL_MMA"); // 0: never, always: wherever it can run
+    if (d.kernel != ESPDL_KERNEL_AUTO || d.n <= 0 || !conv2d_mma_supported(d) || (knob && *knob == '0'))
+        return false;
+    if (knob && *knob == 'a')
+        return true;
+    // What the kernel that would run otherwise takes for a small layer, from the same chains of launches (us): a start-up of 2.5
+    // to 4, and 0.33 for every 128 bytes of the reduction that its matrix instructions walk one after the other.  Large layers
+    // are decided by this estimate's growth: tile kernels stay below 6 us up to 200 M multiply-adds.
+    const int cin_blocks = (d.in_c + 127) / 128;
+    float other;
+    if (conv2d_band_tc_supported(d) && d.filter_image_stride == 0)
+        other = 8.f;
+    else if (d.filter_image_stride == 0 && conv2d_conv_tc_supported(d))
+        other = d.stride_h == 1 && d.dilation_h == 1 && cin_blocks == 1 && d.in_c % 32 == 0 && d.in_c != 96 && d.out_c <= 256 ? 3.9f : 2.5f + 0.33f * d.kh * d.kw * cin_blocks;
+    else if (conv2d_tc_supported(d))
+        other = 3.4f + 0.33f * (cin_blocks - 1) + ((d.out_pixel_stride ? d.out_pixel_stride : d.out_c) % 16 ? 9e-6f * d.n * d.out_h * d.out_w * d.out_c : 0.f);
+    else
+        other = conv2d_packed_supported(d) ? min(10.f, conv2d_simt_estimate_us(d)) : conv2d_simt_estimate_us(d);
+    return conv2d_mma_estimate_us(d) < other;
+}
+
 // Shapes no kernel reads in place, large enough for packed operands to pay (a caller without the scratch gets the CUDA-core kernel).
 static bool runs_packed(const espdl_conv_desc &d)
 {
@@ -453,7 +477,7 @@ int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes
     int st = conv_validate(desc);
     if (st)
         return st;
-    if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1)
+    if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1 || runs_mma(*desc))
         return ESPDL_OK;
     if (conv2d_tc_supported(*desc))
         *bytes = conv2d_tc_workspace_bytes(*desc);
@@ -461,6 +485,8 @@ int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes
         *bytes = conv2d_packed_workspace_bytes(*desc);
     return ESPDL_OK;
 }
+
+int espdl_b200_conv2d_is_small(const espdl_conv_desc *desc) { return conv_validate(desc) == ESPDL_OK && runs_mma(*desc) ? 1 : 0; }
 
 int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t workspace_bytes, void *stream)
 {
@@ -483,6 +509,8 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
             return conv2d_dw_tma(*desc, s);
         return conv2d_depthwise(*desc, s);
     }
+    if (runs_mma(*desc))
+        return conv2d_mma(*desc, s);
     if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_stem_tc_supported(*desc))
         return conv2d_stem_tc(*desc, s); // 3x3 stride-2 RGB first layer: banded-filter tensor-core kernel
     if (desc->filter_image_stride != 0) {

@@ -97,6 +97,10 @@ int pack_operands(const espdl_conv_desc &d, long long row0, int rows, bool filte
 bool conv2d_packed_supported(const espdl_conv_desc &d);
 size_t conv2d_packed_workspace_bytes(const espdl_conv_desc &d);
 int conv2d_packed(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s);
+// Small int8 convs and products with warp-level matrix instructions (conv_mma.cu); the estimate decides against the tile kernels.
+bool conv2d_mma_supported(const espdl_conv_desc &d);
+float conv2d_mma_estimate_us(const espdl_conv_desc &d);
+int conv2d_mma(const espdl_conv_desc &d, cudaStream_t s);
 // Each translation unit with bounded device-side waits keeps the address of ONE status word in pinned, device-mapped host
 // memory: a wait that runs out stores ESPDL_ERR_TIMEOUT there, and espdl_b200_stream_sync reads it as ordinary memory.
 // (A device word per unit, copied back at every synchronisation, cost seven blocking copies: 60 us of a 160 us pass.)

@@ -45,6 +45,7 @@ constexpr int BD_A_BYTES = 128 * BD_K;   // one ky plane of a stage
 constexpr int BD_MAX_STAGES = 4;
 
 struct BandParams {
+    int early; // the filter is a constant of the model: read ahead of the previous kernel's end
     int n, ih, iw, oh, ow, cin, cout, S, J;
     int ncol, out_pw, out_mask; // accumulator columns J * Cout; a group's piece = half of them; swizzle mask of the staging tile
     int stages;
@@ -82,6 +83,8 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_tiles = p.ngroups * p.yblocks * p.segs;
+    if (!p.early)
+        grid_dep_wait();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; s++) {
@@ -422,6 +425,7 @@ int conv2d_band_tc(const espdl_conv_desc &d, cudaStream_t s)
     p.seg_bytes = p.J * p.S * d.in_c;
     p.x_shift = shift_px * d.in_c;
     p.k_base = (shift_px - d.pad_left) * d.in_c;
+    p.early = in_model_scope();
     p.w = (const int8_t *)d.filter, p.out = d.output;
     p.epi.bias = d.bias, p.epi.ew = d.filter_exponents, p.epi.lut = d.lut, p.epi.lut_stride = d.lut_channel_stride;
     p.epi.e_shift_base = d.out_exponent - d.in_exponent;

@@ -316,6 +316,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // windows run into the next row); they are computed and dropped.  The whole filter stays in shared memory for the life of
 // the CTA.  Borders are TMA zero fill.  Epilogue and roles as above; a tile leaves through one TMA store per image row.
 struct PatchParams {
+    int early; // the filter is a constant of the model
     int n, oh, ow, cin, cout;
     int kh, kw, pt, pl;
     int PW, RT, PV;               // positions per patch row (32, 64 or 128), image rows per tile, outputs per row = PW - (KW - 1)
@@ -453,7 +454,9 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
-            // the filter, once: one box per tap
+            // the filter, once: one box per tap (ahead of the previous kernel's end where it is a model's constant)
+            if (!p.early)
+                grid_dep_wait();
             mbar_arrive_expect_tx(smem_u32(filt_bar), (uint32_t)(taps * b_tap));
             for (int tap = 0; tap < taps; tap++) tma_load_2d(smem_u32(filt_s + (size_t)tap * b_tap), &map_b, tap * p.cin, 0, smem_u32(filt_bar));
             grid_dep_wait(); // the previous kernel's output, before the first patch; the other roles act on what the producer brought in
@@ -893,6 +896,7 @@ int conv2d_conv_tc(const espdl_conv_desc &d, cudaStream_t s)
     {
         PatchParams pp;
         memset(&pp, 0, sizeof(pp));
+        pp.early = in_model_scope();
         if (patch_plan(d, pp))
             return launch_patch(d, pp, s);
     }

@@ -45,6 +45,7 @@ constexpr int ST_ACC = 2;
 constexpr int ST_A_BYTES = 128 * ST_K;   // one ky plane of a stage
 
 struct StemParams {
+    int early; // the filter is a constant of the model: read ahead of the previous kernel's end
     int n, ih, iw, oh, ow, cout;
     int pt, pl;
     int rows_n, rows_y;      // tile rows = rows_n images x rows_y output rows = 128
@@ -80,6 +81,8 @@ stem_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_tiles = p.ngroups * p.yblocks * p.segs;
+    if (!p.early)
+        grid_dep_wait();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST_STAGES; s++) {
@@ -367,6 +370,7 @@ int conv2d_stem_tc(const espdl_conv_desc &d, cudaStream_t s)
     p.ngroups = (d.n + p.rows_n - 1) / p.rows_n;
     p.x_shift = d.pad_left ? 16 : 0;
     p.k_base = d.pad_left ? 16 - 3 * d.pad_left : 0;
+    p.early = in_model_scope();
     p.w = (const int8_t *)d.filter, p.out = d.output;
     p.epi.bias = d.bias, p.epi.ew = d.filter_exponents, p.epi.lut = d.lut, p.epi.lut_stride = d.lut_channel_stride;
     p.epi.e_shift_base = d.out_exponent - d.in_exponent;

@@ -183,6 +183,13 @@ esp_err_t Conv::prepare(ModelContext *context)
         const bool sliced = input->row_stride || (output && output->row_stride); // a slice has no runs of whole pixels
         m_group_px = sliced || m_lut_stride ? 1 : choose_pixel_group(cin, cout, pixels); // per-channel tables are indexed by the real channel
         if (m_group_px > 1) {
+            const int grouped = m_group_px;
+            espdl_conv_desc plain;
+            m_group_px = 1;
+            if (fill_desc(context, &plain) != ESPDL_OK || !espdl_b200_conv2d_is_small(&plain))
+                m_group_px = grouped;
+        }
+        if (m_group_px > 1) {
             const int g = m_group_px;
             std::vector<int8_t> wf((size_t)g * cout * g * cin, 0);
             const int8_t *w = (const int8_t *)filter->data; // [cout][cin]
@@ -669,6 +676,9 @@ void MatMul::forward(ModelContext *context, runtime_mode_t mode)
         full1 = full1 && b1[i] == ob[i];
         none1 = none1 && b1[i] == 1;
     }
+    const bool constant = in1->device_owned; // else the previous steps of the plan write it: nothing of it is read ahead of them
+    if (!constant)
+        espdl_b200_model_scope(0);
     const void *filter = in1->device;
     const size_t spread = spread_bytes(b0, b1, (size_t)K * N * es);
     if (spread && spread <= context->workspace_bytes && (long long)K * N <= 0x7fffffffll) {
@@ -721,6 +731,8 @@ void MatMul::forward(ModelContext *context, runtime_mode_t mode)
         d.round_mode = context->round_mode;
         st = espdl_b200_conv2d_ws(&d, context->workspace, context->workspace_bytes, context->stream);
     }
+    if (!constant)
+        espdl_b200_model_scope(1);
     if (st)
         ESP_LOGE("MatMul", "%s failed: %s %s", name ? name : "?", espdl_b200_strerror(st), espdl_b200_last_error());
     context->note(st);

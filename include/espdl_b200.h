@@ -183,6 +183,8 @@ int espdl_b200_conv2d(const espdl_conv_desc *desc, void *stream);
  * espdl_b200_conv2d_ws; espdl_b200_conv2d allocates and caches one internally.
  */
 int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes);
+/* 1 if the call runs the kernel for small layers, which reads narrow rows as they are (no gain from grouping pixels), else 0. */
+int espdl_b200_conv2d_is_small(const espdl_conv_desc *desc);
 int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t workspace_bytes, void *stream);
 
 /*

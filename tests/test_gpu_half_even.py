@@ -12,6 +12,11 @@ from espdl_b200 import abi
 
 pytestmark = pytest.mark.gpu
 
+
+@pytest.fixture(autouse=True)
+def no_small_layers(monkeypatch):
+    monkeypatch.setenv("ESPDL_B200_SMALL_MMA", "0")  # the kernels meant here, whatever the size
+
 # one shape per kernel: the tile kernel (staged, unaligned rows, residual), filter windows (one box per tap, one patch per
 # tile stacked / unstaged), banded 8 / 16 channels, first layer, depthwise through the TMA unit and from global memory
 SHAPES = {

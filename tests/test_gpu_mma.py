@@ -1,0 +1,64 @@
+"""Small convs, Gemms and products on the warp-level matrix instructions: bit-exact against the plain-C oracle at the edges of
+fragments, splits and chunks, for every alignment, epilogue and stride."""
+import numpy as np
+import pytest
+
+import cases
+import gpu_util
+from espdl_b200 import abi
+
+pytestmark = pytest.mark.gpu
+
+P0 = dict(kh=1, kw=1, pad=(0, 0, 0, 0))
+SHAPES = [
+    dict(n=1, h=7, w=7, cin=160, cout=96, **P0),
+    dict(n=1, h=1, w=1, cin=16, cout=8, **P0),
+    dict(n=1, h=1, w=17, cin=1040, cout=9, **P0),
+    dict(n=3, h=5, w=7, cin=28, cout=33, **P0),
+    dict(n=1, h=10, w=10, cin=64, cout=64),
+    dict(n=2, h=9, w=11, cin=16, cout=40, stride=2),
+    dict(n=1, h=13, w=8, cin=12, cout=20, kh=5, kw=3, dil=2, pad=(4, 4, 2, 2)),
+    dict(n=1, h=6, w=6, cin=128, cout=257, stride=2),
+    dict(n=27, h=6, w=5, cin=32, cout=24, **P0),
+    dict(n=1, h=40, w=40, cin=24, cout=24, **P0),
+]
+
+
+@pytest.fixture
+def forced(monkeypatch):
+    monkeypatch.setenv("ESPDL_B200_SMALL_MMA", "always")
+
+
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("lut", [False, True, "channels"])
+@pytest.mark.parametrize("i", range(len(SHAPES)))
+def test_conv(i, lut, round_mode, forced):
+    case = cases.conv_case(seed=i, per_channel=True, lut=lut, round_mode=round_mode, act=abi.ACT_LINEAR if lut else abi.ACT_RELU, **SHAPES[i])
+    want = gpu_util.run_conv_oracle(case)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+    assert want.std() > 0
+
+
+@pytest.mark.parametrize("in_stride,out_stride", [(0, 0), (64, 96), (52, 47)])
+@pytest.mark.parametrize("e_w", [(-9, -6), (-1, 3), (-40, -25)])
+def test_strides_residual_and_any_shift(in_stride, out_stride, e_w, forced):
+    case = cases.conv_case(seed=3, n=2, h=6, w=9, cin=48, cout=45, per_channel=True, e_in=0, e_out=0, e_w=e_w, in_stride=in_stride, out_stride=out_stride, **P0)
+    case["res"] = np.random.default_rng(3).integers(-128, 128, size=case["out"].shape, dtype=np.int8)
+    case["residual_pixel_stride"] = case["out"].shape[-1]
+    case["out"][...] = 0x55
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+
+
+@pytest.mark.parametrize("k,n", [(100, 100), (32, 17), (16, 3), (256, 64)])
+def test_batch_of_products(k, n, forced):
+    rng = np.random.default_rng(k)
+    images, rows = 5, 21
+    x = rng.integers(-100, 100, size=(images, 1, rows, k), dtype=np.int8)
+    w = rng.integers(-100, 100, size=(images, n, 1, 1, k), dtype=np.int8)
+    whole = cases.conv_case(seed=1, n=images, h=1, w=rows, cin=k, cout=n, bias=False, **P0)
+    whole.update(x=x, w=w, filter_image_stride=n * k)
+    got = gpu_util.run_conv_gpu(whole)
+    for i in range(images):
+        one = cases.conv_case(seed=1, n=1, h=1, w=rows, cin=k, cout=n, bias=False, **P0)
+        one.update(x=x[i:i + 1], w=w[i], filter_exponent=whole["filter_exponent"])
+        np.testing.assert_array_equal(got[i:i + 1], gpu_util.run_conv_oracle(one))

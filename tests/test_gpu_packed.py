@@ -10,6 +10,11 @@ from espdl_b200 import abi
 
 pytestmark = pytest.mark.gpu
 
+
+@pytest.fixture(autouse=True)
+def no_small_layers(monkeypatch):
+    monkeypatch.setenv("ESPDL_B200_SMALL_MMA", "0")  # the kernels meant here, whatever the size
+
 S16 = dict(dtype=abi.DTYPE_INT16, e_in=-14, e_w=(-15, -14), e_out=-11)
 SHAPES = [
     dict(n=2, h=20, w=21, cin=32, cout=48),                        # 3x3
