@@ -436,6 +436,8 @@ int espdl::conv_validate(const espdl_conv_desc *d)
     return ESPDL_OK;
 }
 
+constexpr long long DW_SMALL = 8ll << 20; // outputs of a stride-2 conv; twice that at stride 1
+
 // Small enough for the warp-level matrix instructions?
 static bool runs_mma(const espdl_conv_desc &d)
 {
@@ -449,15 +451,19 @@ static bool runs_mma(const espdl_conv_desc &d)
     // are decided by this estimate's growth: tile kernels stay below 6 us up to 200 M multiply-adds.
     const int cin_blocks = (d.in_c + 127) / 128;
     float other;
-    if (conv2d_band_tc_supported(d) && d.filter_image_stride == 0)
-        other = 8.f;
+    if (conv2d_stem_tc_supported(d))
+        other = 4.f;
+    else if (conv2d_band_tc_supported(d) && d.filter_image_stride == 0)
+        other = 6.f;
     else if (d.filter_image_stride == 0 && conv2d_conv_tc_supported(d))
         other = d.stride_h == 1 && d.dilation_h == 1 && cin_blocks == 1 && d.in_c % 32 == 0 && d.in_c != 96 && d.out_c <= 256 ? 3.9f : 2.5f + 0.33f * d.kh * d.kw * cin_blocks;
     else if (conv2d_tc_supported(d))
         other = 3.4f + 0.33f * (cin_blocks - 1) + ((d.out_pixel_stride ? d.out_pixel_stride : d.out_c) % 16 ? 9e-6f * d.n * d.out_h * d.out_w * d.out_c : 0.f);
     else
-        other = conv2d_packed_supported(d) ? min(10.f, conv2d_simt_estimate_us(d)) : conv2d_simt_estimate_us(d);
-    return conv2d_mma_estimate_us(d) < other;
+        // packed operands: two launches, one pass over the unrolled rows; no kernel's start-up is worth waiting for beyond that
+        return conv2d_mma_estimate_us(d) < (conv2d_packed_supported(d) ? min(9.f + (d.in_c % 16 == 0 ? 2.5e-7f : 3.5e-6f) * (float)d.n * d.out_h * d.out_w * d.kh * d.kw * d.in_c, conv2d_simt_estimate_us(d))
+                                                                       : conv2d_simt_estimate_us(d));
+    return conv2d_mma_estimate_us(d) < min(other, 8.f);
 }
 
 // Shapes no kernel reads in place, large enough for packed operands to pay (a caller without the scratch gets the CUDA-core kernel).
@@ -486,7 +492,11 @@ int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes
     return ESPDL_OK;
 }
 
-int espdl_b200_conv2d_is_small(const espdl_conv_desc *desc) { return conv_validate(desc) == ESPDL_OK && runs_mma(*desc) ? 1 : 0; }
+int espdl_b200_conv2d_is_small(const espdl_conv_desc *desc)
+{
+    // ungrouped it has to beat the tile kernel on grouped rows, 3.4 us and up
+    return conv_validate(desc) == ESPDL_OK && runs_mma(*desc) && conv2d_mma_estimate_us(*desc) < 3.6f ? 1 : 0;
+}
 
 int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t workspace_bytes, void *stream)
 {
@@ -504,8 +514,11 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
         if (desc->kernel == ESPDL_KERNEL_TCGEN05)
             return ESPDL_ERR_UNSUPPORTED;
         // 3x3 int8 with 16-byte channel runs: the TMA-fed kernel; ESPDL_KERNEL_SIMT asks for the kernels that read global
-        // memory directly
-        if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_dw_tma_supported(*desc))
+        // memory directly.  Those are also the faster ones for tensors that fit into L2: no TMA pipeline to start (1.7 against 4.1 us
+        // for 14x14x384, 5.9 against 7.9 for 16 images of 56x56x144)
+        const bool small = desc->kernel == ESPDL_KERNEL_AUTO && (long long)desc->n * desc->out_h * desc->out_w * desc->out_c < (desc->stride_h == 1 ? 2 : 1) * DW_SMALL && desc->kh == 3 &&
+            !getenv("ESPDL_B200_DEBUG_WAIT_EXPIRY") && !getenv("ESPDL_B200_DW_TMA_NARROW");
+        if (desc->kernel != ESPDL_KERNEL_SIMT && !small && conv2d_dw_tma_supported(*desc))
             return conv2d_dw_tma(*desc, s);
         return conv2d_depthwise(*desc, s);
     }

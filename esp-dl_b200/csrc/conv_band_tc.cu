@@ -103,16 +103,21 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
     {
         const int words_per_plane = ncol * (BD_K / 4);
         const int tap_bytes = 3 * p.cin, step = p.S * p.cin;
+        const bool aligned = ((uintptr_t)p.w & 3) == 0;
         for (int i = threadIdx.x; i < 3 * words_per_plane; i += BD_THREADS) {
             const int ky = i / words_per_plane, r = i - ky * words_per_plane;
             const int row = r >> 5, k0 = (r & 31) * 4;
             const int j = row / p.cout, co = row - j * p.cout;
             uint32_t word = 0;
+            const int t0 = k0 - p.k_base - step * j; // Cin*kx + c: a multiple of 4, as is the run of taps
+            if (aligned) { // (byte by byte the planes took 5 of the 10 us of a small layer)
+                if (t0 >= 0 && t0 < tap_bytes)
+                    word = __ldg((const uint32_t *)(p.w + (co * 3 + ky) * tap_bytes + t0));
+            } else {
 #pragma unroll
-            for (int b = 0; b < 4; b++) {
-                const int t = k0 + b - p.k_base - step * j; // Cin*kx + c
-                if (t >= 0 && t < tap_bytes)
-                    word |= (uint32_t)(uint8_t)p.w[(co * 3 + ky) * tap_bytes + t] << (8 * b);
+                for (int b = 0; b < 4; b++)
+                    if (t0 + b >= 0 && t0 + b < tap_bytes)
+                        word |= (uint32_t)(uint8_t)p.w[(co * 3 + ky) * tap_bytes + t0 + b] << (8 * b);
             }
             const uint32_t off = (uint32_t)(row * BD_K + k0);
             *(uint32_t *)(b_s + (size_t)ky * b_plane + (off ^ (((off >> 7) & 7u) << 4))) = word;

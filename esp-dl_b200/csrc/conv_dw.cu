@@ -11,6 +11,7 @@
 namespace espdl {
 
 struct DwParams {
+    int early; // filter, bias and exponents are constants of a model: read ahead of the previous kernel's end
     const void *in, *w, *bias;
     void *out;
     const int32_t *ew;
@@ -154,7 +155,8 @@ template <int S, bool EVEN>
 __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xsegs, int ytiles, int cols_per_thread)
 {
     grid_dep_launch();
-    grid_dep_wait();
+    if (!p.early)
+        grid_dep_wait();
     constexpr int ROWS_IN = S == 1 ? 6 : 5;
     constexpr int ROWS_OUT = S == 1 ? 4 : 2;
     const int quads = p.c >> 2;
@@ -200,6 +202,8 @@ __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xseg
     }
     const int oy0 = yt * ROWS_OUT;
     const int x_begin = xs * cols_per_thread, x_end = min(p.ow, x_begin + cols_per_thread);
+    if (p.early)
+        grid_dep_wait();
     if (!fast) {
         dw3x3_band_general(p, S, n, c0, oy0, ROWS_OUT, x_begin, x_end);
         return;
@@ -381,6 +385,7 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
     p.e_shift_base = d.out_exponent - d.in_exponent;
     p.ew_scalar = d.filter_exponent, p.per_channel = d.per_channel;
     p.relu = d.activation == ESPDL_ACT_RELU, p.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
+    p.early = in_model_scope();
     const long long pixels = (long long)d.n * d.out_h * d.out_w;
     const int threads = 256;
     const long long max_blocks = (long long)num_sms() * 32;
@@ -397,6 +402,8 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
         const long long want = (long long)num_sms() * 2048;
         int cols = d.out_w;
         while (cols > 8 && per_seg * ((d.out_w + cols - 1) / cols) < want) cols = (cols + 1) / 2;
+        // a small layer is bound by the latency of the walk: short runs, although each reads two columns of its neighbour again
+        while (cols > 2 && per_seg * ((d.out_w + cols - 1) / cols) < (long long)num_sms() * 128) cols = (cols + 1) / 2;
         const int xsegs = (d.out_w + cols - 1) / cols;
         const long long items = per_seg * xsegs;
         p.total = items, p.chunks = 0;

@@ -11,7 +11,9 @@
 // Fragments: the order of the reduction is free as long as both operands agree, so lane (g, t) of a warp takes 16 consecutive bytes at
 // 64 * step + 16 * t of row g (input pixel or filter row): one 128-bit load per row and step, words 0, 1 feed the first
 // instruction and words 2, 3 the second.  A window's taps are consecutive runs of the reduction; with Cin a multiple of 16 a chunk never
-// leaves its tap.  ALIGN = 4: word loads, a word never leaves its tap (Cin a multiple of 4).
+// leaves its tap.  ALIGN = 4: word loads, a word never leaves its tap (Cin a multiple of 4).  ALIGN = 1: any channel count (first
+// layers): a filter row's taps are one run of KW * Cin bytes in the input too, padded here to whole chunks; a chunk is read as the five
+// aligned words around it, shifted, and masked where it crosses the image's edge (27 images 192x96x3 -> 16, 7x7: 129 us before).
 #include "common.cuh"
 
 #include <climits>
@@ -27,7 +29,8 @@ struct MmaParams {
     const int32_t *bias, *ew;
     int8_t *out;
     int M, N, K;                  // output pixels (per image of a batch of products), channels, reduction
-    int steps;                    // ceil(K / 64)
+    int steps;                    // 64-byte steps of the reduction
+    int run, run_chunks;          // ALIGN 1: bytes of a filter row and its chunks
     int split;                    // warps that share a tile's reduction: 1, 2, 4 or 8
     int tiles_n, tiles;           // tiles of a matrix
     int ic, ih, iw, oh, ow, kw, sh, sw, dh, dw, pt, pl, ips, ops, rps, lut_stride;
@@ -67,6 +70,43 @@ __device__ __noinline__ uint32_t general_word(const MmaParams &p, const int (&v)
     return word;
 }
 
+// 16 bytes from any address; words without a byte in [lo, hi) are not read.
+__device__ __forceinline__ uint4 unaligned_chunk(const int8_t *at, const int8_t *lo, const int8_t *hi)
+{
+    const uint32_t *base = (const uint32_t *)((uintptr_t)at & ~(uintptr_t)3);
+    const uint32_t sh = 8u * ((uint32_t)(uintptr_t)at & 3u);
+    uint32_t w[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) w[i] = (const int8_t *)(base + i) < hi && (const int8_t *)(base + i + 1) > lo ? __ldg(base + i) : 0u;
+    return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
+}
+
+// The first `have` of 16 bytes from any address, all of them readable.
+__device__ __forceinline__ uint4 inside_chunk(const int8_t *at, int have)
+{
+    const uint32_t *base = (const uint32_t *)((uintptr_t)at & ~(uintptr_t)3);
+    const int m = (int)((uintptr_t)at & 3);
+    uint32_t w[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) w[i] = 4 * i < have + m ? __ldg(base + i) : 0u;
+    return make_uint4(__funnelshift_r(w[0], w[1], 8 * m), __funnelshift_r(w[1], w[2], 8 * m), __funnelshift_r(w[2], w[3], 8 * m), __funnelshift_r(w[3], w[4], 8 * m));
+}
+
+// Bytes [from, to) of a chunk stay, the others become zero.
+__device__ __forceinline__ uint4 keep_bytes(uint4 v, int from, int to)
+{
+    if (from <= 0 && to >= 16)
+        return v;
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int a = min(max(from - 4 * i, 0), 4), b = min(max(to - 4 * i, 0), 4);
+        const uint32_t below_b = b == 4 ? 0xffffffffu : (1u << (8 * b)) - 1u, below_a = a == 4 ? 0xffffffffu : (1u << (8 * a)) - 1u;
+        w[i] &= below_b & ~below_a;
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 template <int MT, int NT, bool WINDOW, int ALIGN>
 __global__ void __launch_bounds__(32 * MMA_WARPS) conv_mma_kernel(const __grid_constant__ MmaParams p)
 {
@@ -92,8 +132,16 @@ __global__ void __launch_bounds__(32 * MMA_WARPS) conv_mma_kernel(const __grid_c
             for (int j = 0; j < NT; j++) {
                 const int s = s0 + d * p.split, n = tn * COLS + 8 * j + g;
                 b[d][j] = make_uint4(0u, 0u, 0u, 0u);
-                if (active && s < p.steps && n < p.N)
-                    b[d][j] = dense_chunk<ALIGN>(w + (long long)n * p.K, 64 * s + 16 * t, p.K);
+                if (active && s < p.steps && n < p.N) {
+                    if constexpr (ALIGN == 1) {
+                        const int q = 4 * s + t, ky = q / p.run_chunks, off = 16 * (q - ky * p.run_chunks), have = min(16, p.run - off);
+                        const int8_t *at = w + (long long)n * p.K + ky * p.run + off;
+                        if (ky * p.run < p.K)
+                            b[d][j] = keep_bytes(unaligned_chunk(at, at, at + have), 0, have);
+                    } else {
+                        b[d][j] = dense_chunk<ALIGN>(w + (long long)n * p.K, 64 * s + 16 * t, p.K);
+                    }
+                }
             }
     };
     load_b(kpart);
@@ -145,7 +193,24 @@ __global__ void __launch_bounds__(32 * MMA_WARPS) conv_mma_kernel(const __grid_c
 #pragma unroll
         for (int d = 0; d < DEPTH; d++) {
             const int k = 64 * (s0 + d * p.split) + 16 * t;
-            if (!WINDOW) {
+            if constexpr (ALIGN == 1) {
+                // what lies behind the run meets zeros of the filter; only the image's edges have to read as zero
+                const int q = k / 16, ky = q / p.run_chunks, off = 16 * (q - ky * p.run_chunks), width = p.iw * p.ic;
+#pragma unroll
+                for (int i = 0; i < MT; i++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int iy = iy0[i][h] + ky * p.dh, x = ix0[i][h] * p.ic + off;
+                        a[d][i][h] = make_uint4(0u, 0u, 0u, 0u);
+                        if (row_ok[i][h] && ky * p.run < p.K && (unsigned)iy < (unsigned)p.ih && x + 16 > 0 && x < width) {
+                            const int8_t *line = row[i][h] + iy * width;
+                            if (x >= 0 && x + 16 <= width)
+                                a[d][i][h] = inside_chunk(line + x, min(16, p.run - off));
+                            else
+                                a[d][i][h] = keep_bytes(unaligned_chunk(line + x, line, line + width), -x, width - x);
+                        }
+                    }
+            } else if (!WINDOW) {
 #pragma unroll
                 for (int i = 0; i < MT; i++)
 #pragma unroll
@@ -271,7 +336,14 @@ int mma_align(const espdl_conv_desc &d)
 {
     const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
     const uintptr_t a = (uintptr_t)d.input | (uintptr_t)d.filter | (uintptr_t)ips | (uintptr_t)d.in_c | (uintptr_t)d.filter_image_stride;
-    return a % 16 == 0 ? 16 : (a % 4 == 0 ? 4 : 0);
+    if (a % 4 == 0)
+        return a % 16 == 0 ? 16 : 4;
+    return ips == d.in_c && d.dilation_w == 1 && d.filter_image_stride == 0 ? 1 : 0;
+}
+
+int mma_steps(const espdl_conv_desc &d)
+{
+    return mma_align(d) == 1 ? (d.kh * ((d.kw * d.in_c + 15) / 16) + 3) / 4 : (d.kh * d.kw * d.in_c + 63) / 64;
 }
 
 // Tile and split with the least estimated time.  The estimate is a fit (12 % rms) to 106 timings of chains of 21 layers over all
@@ -281,8 +353,8 @@ MmaPlan mma_plan(const espdl_conv_desc &d)
 {
     const bool batched = d.filter_image_stride != 0;
     const long long M = (batched ? 1ll : (long long)d.n) * d.out_h * d.out_w, images = batched ? d.n : 1;
-    const int steps = (d.kh * d.kw * d.in_c + 63) / 64;
-    const float loads = mma_align(d) == 16 ? 1.f : 4.f, window = is_window(d) ? 0.0168f : 0.f;
+    const int steps = mma_steps(d);
+    const float loads = mma_align(d) == 16 ? 1.f : (mma_align(d) == 4 ? 4.f : 8.f), window = is_window(d) ? 0.0168f : 0.f;
     static const int shapes[3][2] = {{1, 1}, {1, 2}, {2, 2}};
     MmaPlan best = {0, 0, 0, 1e30f};
     for (const auto &s : shapes) {
@@ -305,8 +377,9 @@ void launch_mma(const MmaParams &p, bool window, int align, int images, cudaStre
 {
     const int per_block = MMA_WARPS / p.split;
     const dim3 grid((unsigned)((p.tiles + per_block - 1) / per_block), (unsigned)images);
-    const auto kernel = window ? (align == 16 ? conv_mma_kernel<MT, NT, true, 16> : conv_mma_kernel<MT, NT, true, 4>)
-                               : (align == 16 ? conv_mma_kernel<MT, NT, false, 16> : conv_mma_kernel<MT, NT, false, 4>);
+    const auto kernel = align == 1 ? conv_mma_kernel<MT, NT, true, 1>
+        : window                   ? (align == 16 ? conv_mma_kernel<MT, NT, true, 16> : conv_mma_kernel<MT, NT, true, 4>)
+                                   : (align == 16 ? conv_mma_kernel<MT, NT, false, 16> : conv_mma_kernel<MT, NT, false, 4>);
     launch_overlapped(kernel, grid, dim3(32 * MMA_WARPS), 0, s, p);
 }
 
@@ -333,7 +406,8 @@ int conv2d_mma(const espdl_conv_desc &d, cudaStream_t s)
     p.in = (const int8_t *)d.input, p.w = (const int8_t *)d.filter, p.lut = d.lut, p.res = (const int8_t *)d.residual;
     p.bias = (const int32_t *)d.bias, p.ew = d.filter_exponents, p.out = (int8_t *)d.output;
     p.M = (batched ? 1 : d.n) * d.out_h * d.out_w, p.N = d.out_c, p.K = d.kh * d.kw * d.in_c;
-    p.steps = (p.K + 63) / 64, p.split = plan.split;
+    p.steps = mma_steps(d), p.split = plan.split;
+    p.run = d.kw * d.in_c, p.run_chunks = (p.run + 15) / 16;
     p.tiles_n = (p.N + 8 * plan.nt - 1) / (8 * plan.nt), p.tiles = p.tiles_n * ((p.M + 16 * plan.mt - 1) / (16 * plan.mt));
     p.ic = d.in_c, p.ih = d.in_h, p.iw = d.in_w, p.oh = d.out_h, p.ow = d.out_w, p.kw = d.kw;
     p.sh = d.stride_h, p.sw = d.stride_w, p.dh = d.dilation_h, p.dw = d.dilation_w, p.pt = d.pad_top, p.pl = d.pad_left;

@@ -14,8 +14,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.fixture(autouse=True)
-def no_small_layers(monkeypatch):
+def no_small_layers(monkeypatch, request):
     monkeypatch.setenv("ESPDL_B200_SMALL_MMA", "0")  # the kernels meant here, whatever the size
+    if "dw-tma" in request.node.name:
+        monkeypatch.setenv("ESPDL_B200_DW_TMA_NARROW", "1")
 
 # one shape per kernel: the tile kernel (staged, unaligned rows, residual), filter windows (one box per tap, one patch per
 # tile stacked / unstaged), banded 8 / 16 channels, first layer, depthwise through the TMA unit and from global memory

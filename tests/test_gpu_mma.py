@@ -21,6 +21,11 @@ SHAPES = [
     dict(n=1, h=6, w=6, cin=128, cout=257, stride=2),
     dict(n=27, h=6, w=5, cin=32, cout=24, **P0),
     dict(n=1, h=40, w=40, cin=24, cout=24, **P0),
+    dict(n=2, h=23, w=31, cin=3, cout=16, kh=7, kw=7, stride=2),       # ragged runs: 21 bytes a filter row
+    dict(n=1, h=9, w=3, cin=1, cout=12, kh=3, kw=5, pad=(1, 1, 2, 2)),  # a window wider than the image
+    dict(n=3, h=8, w=8, cin=5, cout=9, kh=5, kw=5, stride=(2, 1), dil=(2, 1), pad=(4, 4, 2, 2)),
+    dict(n=1, h=1, w=50, cin=101, cout=40, **P0),
+    dict(n=2, h=16, w=20, cin=3, cout=33, stride=2, pad=(0, 1, 0, 1)),
 ]
 
 
