@@ -201,11 +201,11 @@ __device__ __forceinline__ void fold_vector(ACC (&acc)[V], const T *v)
     }
 }
 
-template <typename T, int V, typename ACC, Fold F>
-__global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int C, int slice_lanes, int slices, int rows, int early)
+template <typename T, int V, typename ACC, Fold F, int THREADS>
+__global__ void __launch_bounds__(THREADS) channel_reduce_kernel(ReduceParams p, int C, int slice_lanes, int slices, int rows, int early)
 {
     namespace cg = cooperative_groups;
-    __shared__ ACC part[V * 256]; // [channel of the lane][thread]: consecutive threads in consecutive words
+    __shared__ ACC part[V * THREADS]; // [channel of the lane][thread]: consecutive threads in consecutive words
     cg::cluster_group cluster = cg::this_cluster();
     const int cl = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const long long item = blockIdx.x / cl;
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int
         take(std::integral_constant<int, 1>{});
     }
 #pragma unroll
-    for (int j = 0; j < V; j++) part[j * 256 + threadIdx.x] = acc[j];
+    for (int j = 0; j < V; j++) part[j * THREADS + threadIdx.x] = acc[j];
     __syncthreads();
     int half = 1;
     while (half < rows) half <<= 1;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int
         if (ty < half && ty + half < rows) {
             const int other = threadIdx.x + half * slice_lanes;
 #pragma unroll
-            for (int j = 0; j < V; j++) part[j * 256 + threadIdx.x] = fold_partial<ACC>(F, part[j * 256 + threadIdx.x], part[j * 256 + other]);
+            for (int j = 0; j < V; j++) part[j * THREADS + threadIdx.x] = fold_partial<ACC>(F, part[j * THREADS + threadIdx.x], part[j * THREADS + other]);
         }
         __syncthreads();
     }
@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int
     if (rank == 0) {
         const int lo = sizeof(T) == 1 ? -128 : -32768, hi = sizeof(T) == 1 ? 127 : 32767;
         const int cols = min(slice_lanes * V, C - slice * slice_lanes * V);
-        for (int col = threadIdx.x; col < cols; col += 256) {
-            const int at = (col % V) * 256 + col / V;
+        for (int col = threadIdx.x; col < cols; col += THREADS) {
+            const int at = (col % V) * THREADS + col / V;
             ACC sum = part[at];
             for (int k = 1; k < cl; k++) sum = fold_partial<ACC>(F, sum, cluster.map_shared_rank(part, k)[at]);
             const long long q = finish_integer<ACC>(p, sum);
@@ -272,35 +272,41 @@ __global__ void __launch_bounds__(256) channel_reduce_kernel(ReduceParams p, int
         cluster.sync(); // no block leaves while its partials may still be read
 }
 
-template <typename T, int V, typename ACC>
+template <typename T, int V, typename ACC, int THREADS>
 int launch_channel_reduce(const ReduceParams &p, long long outer, int C, cudaStream_t s)
 {
     const int lanes = (C + V - 1) / V;
     // about sixteen pixels a thread, so that the meeting in shared memory stays small beside the loads (7x7x1280 over 1024 images:
     // 54 us with five), and at least 128 contiguous bytes a block where the tensor has them
-    const int want = (int)max(1ll, min(256ll, p.count / 16));
-    const int widest = max(8, 256 / want);
-    const int slices = (lanes + widest - 1) / widest, slice_lanes = (lanes + slices - 1) / slices, rows = 256 / slice_lanes;
+    const int want = (int)max(1ll, min((long long)THREADS, p.count / 16));
+    const int widest = max(8, THREADS / want);
+    const int slices = (lanes + widest - 1) / widest, slice_lanes = (lanes + slices - 1) / slices, rows = THREADS / slice_lanes;
     const long long items = outer * slices;
     // blocks that share an image: only while they do not outnumber what the SMs hold at once, and each thread keeps a full round of loads
+    constexpr int WIDEST_CLUSTER = THREADS > 256 ? 16 : 8; // 16 needs the kernel's consent (below)
     int cl = 1;
-    while (cl < 8 && items * cl * 2 <= 4ll * num_sms() && p.count >= 8ll * rows * cl) cl *= 2;
+    while (cl < WIDEST_CLUSTER && items * cl * 2 <= 4ll * num_sms() && p.count >= 8ll * rows * cl) cl *= 2;
     if (items * cl > 0x7fffffffll)
         return ESPDL_ERR_TOO_LARGE;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(items * cl)), cfg.blockDim = dim3(256), cfg.stream = s;
+    cfg.gridDim = dim3((unsigned)(items * cl)), cfg.blockDim = dim3(THREADS), cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)cl, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    auto launch = [&](auto kernel) {
+        if (cl > 8)
+            cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaLaunchKernelEx(&cfg, kernel, p, C, slice_lanes, slices, rows, (int)in_model_scope());
+    };
     switch (fold_of(p.op)) {
-    case FOLD_SUM: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SUM>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
-    case FOLD_MAX: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MAX>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
-    case FOLD_MIN: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_MIN>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
-    case FOLD_ABS: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_ABS>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
-    case FOLD_SQUARE: cudaLaunchKernelEx(&cfg, channel_reduce_kernel<T, V, ACC, FOLD_SQUARE>, p, C, slice_lanes, slices, rows, (int)in_model_scope()); break;
+    case FOLD_SUM: launch(channel_reduce_kernel<T, V, ACC, FOLD_SUM, THREADS>); break;
+    case FOLD_MAX: launch(channel_reduce_kernel<T, V, ACC, FOLD_MAX, THREADS>); break;
+    case FOLD_MIN: launch(channel_reduce_kernel<T, V, ACC, FOLD_MIN, THREADS>); break;
+    case FOLD_ABS: launch(channel_reduce_kernel<T, V, ACC, FOLD_ABS, THREADS>); break;
+    case FOLD_SQUARE: launch(channel_reduce_kernel<T, V, ACC, FOLD_SQUARE, THREADS>); break;
     }
     count_launch();
     return check_launch("channel reduce");
@@ -313,11 +319,15 @@ template <typename T, typename ACC>
 int channel_reduce(const ReduceParams &p, long long outer, int C, cudaStream_t s)
 {
     const uintptr_t a = (uintptr_t)p.in | (uintptr_t)(C * sizeof(T));
+    // a few large images: more than 8 loads a thread with eight blocks of 256 each, and SMs left for sixteen of 512
+    // (184x184x64, one image: about 20 -> 9.5 us)
+    if (a % 16 == 0 && outer <= num_sms() / 16 && p.count * C * (long long)sizeof(T) >= 8ll * 8 * 256 * 16)
+        return launch_channel_reduce<T, 16 / sizeof(T), ACC, 512>(p, outer, C, s);
     if (a % 16 == 0)
-        return launch_channel_reduce<T, 16 / sizeof(T), ACC>(p, outer, C, s);
+        return launch_channel_reduce<T, 16 / sizeof(T), ACC, 256>(p, outer, C, s);
     if (a % 4 == 0)
-        return launch_channel_reduce<T, 4 / sizeof(T), ACC>(p, outer, C, s);
-    return launch_channel_reduce<T, 1, ACC>(p, outer, C, s);
+        return launch_channel_reduce<T, 4 / sizeof(T), ACC, 256>(p, outer, C, s);
+    return launch_channel_reduce<T, 1, ACC, 256>(p, outer, C, s);
 }
 
 } // namespace

@@ -63,7 +63,8 @@ __device__ __forceinline__ int quotient_code(float t, float sum, float recip, fl
 // The same arithmetic with the rows side by side: a block stages R rows in shared memory (row pitch an odd number of
 // words, so that thread r reading byte i of row r meets no bank conflict), thread r adds row r's exponentials in index
 // order - R ordered sums run at once instead of one -, then all threads write the R x len results.  Used whenever at
-// least 32 rows fit into shared memory; the kernel above keeps the long rows.
+// least 32 rows fit into shared memory; the kernel above keeps the long rows.  Few rows go to many blocks (200 rows of 100:
+// 19 us in one block, 2.9 in fifty), and rows shorter than a warp's reach share one: 2, 4 .. lanes each (300000 rows of 17: 56 -> 22 us).
 __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d, float out_rescale, int R, int pitch, int early)
 {
     if (early)
@@ -83,13 +84,17 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
         __syncthreads();
         const bool words = inner == 1 && d.len % 4 == 0 && (((uintptr_t)d.input) & 3) == 0; // whole 32-bit words per row
         const bool spans = inner == 1 && (((uintptr_t)d.input) & 3) == 0; // R is a multiple of 4
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5, len4 = d.len >> 2;
+        // the lanes that share a row of words: a power of two, a warp at most
+        const int len4 = d.len >> 2, row_words = (d.len + 3) >> 2;
+        const int lanes = row_words >= 32 ? 32 : (row_words > 1 ? 1 << (32 - __clz(row_words - 1)) : 1);
+        const int warp = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1), nwarps = blockDim.x / lanes;
         if (words) {
-            // a warp per row, a word per lane: no index divisions, 128-byte global reads
+            // lanes side by side, a word each: no index divisions, 128-byte global reads
+#pragma unroll 4
             for (int rr = warp; rr < nr; rr += nwarps) {
                 const uint32_t *src = (const uint32_t *)(d.input + (long long)(r0 + rr) * d.len);
                 uint32_t *dst = (uint32_t *)(rows + rr * pitch);
-                for (int i = lane; i < len4; i += 32) dst[i] = src[i];
+                for (int i = lane; i < len4; i += lanes) dst[i] = __ldg(src + i);
             }
         } else if (spans) {
             // rows r0 .. r0 + nr - 1 are one contiguous span of nr * len bytes
@@ -108,7 +113,7 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
             const int8_t *row = rows + threadIdx.x * pitch;
             float sum = 0.f;
             const int full = d.len >> 2;
-#pragma unroll 2
+#pragma unroll 4
             for (int i = 0; i < full; i++) { // the row pitch is an odd number of words
                 const uint32_t w = ((const uint32_t *)row)[i];
 #pragma unroll
@@ -120,12 +125,11 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
         __syncthreads();
         if (spans && d.out_dtype == ESPDL_DTYPE_INT8 && !d.log && (((uintptr_t)d.output) & 3) == 0) {
             // codes straight out where a row is whole words, else in place of the inputs and out as one span
-            const int row_words = (d.len + 3) >> 2;
             for (int rr = warp; rr < nr; rr += nwarps) {
                 uint32_t *row = (uint32_t *)(rows + rr * pitch);
                 uint32_t *to = words ? (uint32_t *)((int8_t *)d.output + (long long)(r0 + rr) * d.len) : row;
                 const float sum = sums[rr], recip = __fdiv_rn(1.f, sum);
-                for (int i = lane; i < row_words; i += 32) {
+                for (int i = lane; i < row_words; i += lanes) {
                     const uint32_t w = row[i];
                     uint32_t q = 0;
 #pragma unroll
@@ -145,7 +149,7 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(espdl_softmax_desc d,
                 const uint32_t *src = (const uint32_t *)(rows + rr * pitch);
                 const float sum = sums[rr];
                 const long long o0 = (long long)(r0 + rr) * d.len;
-                for (int i = lane; i < len4; i += 32) {
+                for (int i = lane; i < len4; i += lanes) {
                     const uint32_t w = src[i];
                     float y[4];
 #pragma unroll
@@ -215,8 +219,10 @@ extern "C" int espdl_b200_softmax(const espdl_softmax_desc *d, void *stream)
     // rows side by side when at least 32 of them fit into 40 KB of shared memory
     const int pitch = (((d->len + 3) / 4) | 1) * 4;
     const int fit = (40 * 1024) / (pitch + 4);
-    if (fit >= 32 && d->rows >= 64) {
-        const int R = min(256, fit) / 4 * 4;
+    if (fit >= 32) {
+        // four blocks an SM before they get more rows: one's staging, ordered sums and quotients run beside another's
+        const int spread = (d->rows + 4 * num_sms() - 1) / (4 * num_sms());
+        const int R = min(min(256, fit) / 4 * 4, (spread + 3) / 4 * 4);
         const int groups = (d->rows + R - 1) / R;
         launch_mover(softmax_rows_kernel, dim3(min(groups, num_sms() * 8)), dim3(256), (size_t)R * (pitch + 4) + 16, (cudaStream_t)stream, *d, dl_rescale(d->out_exponent), R, pitch);
         count_launch();

@@ -34,15 +34,16 @@ def test_lengths_that_fill_no_unit(shape, op, dtype):
 @pytest.mark.parametrize("dtype", BOTH)
 @pytest.mark.parametrize("op", [abi.ELT_ADD, abi.ELT_SUB, abi.ELT_MUL, abi.ELT_MAX, abi.ELT_MIN])
 @pytest.mark.parametrize("shape,gate", [((3, 5, 7, 16), (3, 1, 1, 16)), ((2, 9, 4, 48), (1, 1, 1, 48)), ((1, 6, 6, 8), (1, 1, 1, 8)), ((4, 3, 3, 80), (4, 1, 1, 80)),
-                                        ((3, 5, 7, 12), (3, 1, 1, 12)), ((2, 1, 9, 32), (1, 1, 1, 1))])
+                                        ((3, 5, 7, 12), (3, 1, 1, 12)), ((2, 1, 9, 32), (1, 1, 1, 1)), ((3, 35, 24), (3, 1, 24)), ((2, 3, 5, 16), (2, 3, 1, 16)),
+                                        ((5, 33, 20), (1, 1, 20)), ((2, 3, 5, 4), (1, 3, 1, 4))])
 def test_gates(shape, gate, op, dtype):
-    check(cases.eltwise_case(op, seed=shape[3], dtype=dtype, out_shape=shape, in1_shape=gate))
+    check(cases.eltwise_case(op, seed=shape[-1], dtype=dtype, out_shape=shape, in1_shape=gate))
 
 
 # exponent -1 is the largest whose table stays finite (exp(63.5) < 3.4e38 < exp(127)): beyond it a row is inf / inf, and what the
 # reference's float -> int conversion of that NaN gives is undefined
 @pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
-@pytest.mark.parametrize("e_in,rows,length", [(-4, 300, 17), (-3, 64, 1), (-6, 1000, 127), (-2, 257, 130), (-4, 77, 316), (-7, 4000, 64), (-1, 128, 33)])
+@pytest.mark.parametrize("e_in,rows,length", [(-4, 300, 17), (-3, 64, 1), (-6, 1000, 127), (-2, 257, 130), (-4, 77, 316), (-7, 4000, 64), (-1, 128, 33), (-3, 1, 5), (-4, 7, 100), (-4, 3, 1200)])
 def test_softmax_codes(e_in, rows, length, round_mode):
     rng = np.random.default_rng(length)
     x = rng.integers(-128, 128, size=(rows, length), dtype=np.int8)
@@ -65,10 +66,32 @@ def test_softmax_codes(e_in, rows, length, round_mode):
                                 dict(n=3, h=40, w=3, c=1, kh=3, kw=3, pad=(1, 1, 1, 1)), dict(n=1, h=64, w=64, c=17, kh=5, kw=5, pad=(2, 2, 2, 2)),
                                 dict(n=2, h=5, w=6, c=8, kh=5, kw=5, pad=(0, 0, 1, 3)), dict(n=1, h=3, w=2, c=3, kh=3, kw=3, pad=(1, 1, 1, 1))])
 def test_max_pool_walk(kw, dtype):
-    case = cases.pool_case(abi.POOL_MAX, seed=kw["c"], dtype=dtype, stride=1, **kw)
+    pool_matches(cases.pool_case(abi.POOL_MAX, seed=kw["c"], dtype=dtype, stride=1, **kw))
+
+
+def pool_matches(case):
     want = case["out"].copy()
     assert checkers.oracle().oracle_pool(cases.pool_desc(dict(case, out=want))) == 0
     with gpu_util.DeviceBuffers() as dev:
         ptrs = dict(input=dev.upload(case["x"]), output=dev.upload(case["out"]))
         abi.check(dev.lib.espdl_b200_pool(C.byref(cases.pool_desc(case, ptrs)), None), "pool")
         np.testing.assert_array_equal(dev.download(ptrs["output"], want), want)
+
+
+# maps that go through shared memory: one band and several, windows past every edge, strides, pads of one side
+@pytest.mark.parametrize("dtype", BOTH)
+@pytest.mark.parametrize("kw", [dict(n=1, h=10, w=10, c=32, kh=5, kw=5, pad=(2, 2, 2, 2), stride=1), dict(n=3, h=23, w=7, c=16, kh=3, kw=5, pad=(1, 1, 2, 2), stride=2),
+                                dict(n=1, h=64, w=33, c=16, kh=2, kw=2, pad=(0, 0, 0, 0), stride=2), dict(n=2, h=5, w=6, c=48, kh=4, kw=3, pad=(3, 0, 0, 2), stride=1),
+                                dict(n=1, h=1, w=300, c=16, kh=3, kw=9, pad=(1, 1, 4, 4), stride=3), dict(n=1, h=200, w=180, c=16, kh=9, kw=9, pad=(4, 4, 4, 4), stride=1)])
+def test_max_pool_map(kw, dtype):
+    pool_matches(cases.pool_case(abi.POOL_MAX, seed=kw["c"], dtype=dtype, **kw))
+
+
+# one image over the blocks of a wide cluster
+@pytest.mark.parametrize("dtype", BOTH)
+@pytest.mark.parametrize("shape", [(1, 131, 129, 32), (2, 97, 101, 64)])
+def test_large_image_means(shape, dtype):
+    n, h, w, c = shape
+    case = cases.pool_case(abi.POOL_GLOBAL_AVG, seed=c, dtype=dtype, n=n, h=h, w=w, c=c)
+    case["x"] = case["x"] // 4 + np.arange(c, dtype=case["x"].dtype) # channels with means apart
+    pool_matches(case)
