@@ -378,7 +378,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int g = 0, lt = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, lt++) {
@@ -422,7 +422,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ expand MMA issuer
-        if (lane == 0 && p.has_expand) {
+        if (p.has_expand && elect_one()) {
             int g = 0, lt = 0;
             bool ok = true;
             const uint32_t idesc1 = idesc_i8(1, 1, 128, BK_CH);
@@ -460,7 +460,7 @@ block_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         __syncwarp();
     } else if (warp == 2) {
         // ------------------------------------------------------------------ project MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             int g = 0, lt = 0;
             bool ok = true;
             const uint32_t idesc2 = idesc_i8(1, 1, 128, p.npiece);

@@ -138,7 +138,7 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             grid_dep_wait(); // the previous kernel's output, before the first load; the other roles act on what the producer brought in
             int stage = 0;
             uint32_t phase = 0;
@@ -169,7 +169,7 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;

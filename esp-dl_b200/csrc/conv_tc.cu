@@ -109,7 +109,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             grid_dep_wait(); // the previous kernel's output, before the first load; the other roles act on what the producer brought in
             int stage = 0;
             uint32_t phase = 0;
@@ -147,7 +147,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
@@ -453,7 +453,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             // the filter, once: one box per tap (ahead of the previous kernel's end where it is a model's constant)
             if (!p.early)
                 grid_dep_wait();
@@ -485,7 +485,7 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = mbar_wait(smem_u32(filt_bar), 0);

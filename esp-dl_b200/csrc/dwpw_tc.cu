@@ -128,7 +128,7 @@ dwpw_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ 
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t phase = 0;
             int stage = 0, cb = 0;
             bool ok = true;
@@ -157,7 +157,7 @@ dwpw_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ 
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t phase = 0, dphase = 0;
             int stage = 0;
             bool ok = true;

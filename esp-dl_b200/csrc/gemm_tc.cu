@@ -313,10 +313,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        // One lane runs the loop and issues the copies.  (Letting the whole warp walk the tiles and wait, with lane 0
-        // issuing, measured the same on the network's short reductions and 25-35 % slower on the long reductions of a
-        // large Gemm, where the issue rate of this loop and of the MMA loop below is what bounds the kernel.)
-        const bool issuer = lane == 0;
+        // One elected lane runs the loop and issues the copies.
+        const bool issuer = elect_one();
         if (issuer) {
         grid_dep_wait(); // the previous kernel's output, and its use of the tile counter, before the first load
         int stage = 0;
@@ -388,10 +386,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        // One lane runs the loop and issues (see the producer).  Each tcgen05.mma of M = 128 costs this thread about 250
-        // cycles whatever N is (measured with the role cycle counters: 4 MMAs per tile of K = 128 take ~1000 cycles), so
-        // tiles are made as wide as TMEM allows and carry as few K steps as the layer has.
-        const bool issuer = lane == 0;
+        // One elected lane runs the loop and issues.  A tcgen05.mma of M = 128 costs it about 50 cycles (250 when the lane was chosen by its
+        // number, see elect_one), so that N = 128 and wider keep the tensor cores busy.
+        const bool issuer = elect_one();
         if (issuer) {
         int stage = 0;
         uint32_t phase = 0;
@@ -797,7 +794,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -827,7 +824,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (even CTA only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;

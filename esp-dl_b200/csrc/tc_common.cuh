@@ -127,6 +127,15 @@ __device__ __forceinline__ void commit(uint32_t bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// True in one lane of a converged warp, and the compiler knows that it is one: in a branch taken on `lane == 0` every tcgen05.mma, commit and
+// TMA copy is issued from a loop over the lanes that may be active, at some 200-250 cycles of this thread each.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
