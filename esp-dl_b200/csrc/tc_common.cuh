@@ -99,6 +99,14 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4, uint32_t bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
+        : "memory");
+}
+
 // TMA stores (shared -> global), bulk-group completion
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int c0, int c1)
 {
@@ -126,6 +134,25 @@ __device__ __forceinline__ void commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+
+// The tiles first, first + step, first + 2 step .. of images cut into xtiles x ytiles: divisions at the start, additions from then on
+// (three divisions a tile took the producer of a short tile longer than the tile's loads).
+struct TileWalk {
+    int x, y, n, sx, sy, sn, xtiles, ytiles;
+    __device__ __forceinline__ TileWalk(int first, int step, int xt, int yt) : xtiles(xt), ytiles(yt)
+    {
+        x = first % xt, y = first / xt % yt, n = first / xt / yt;
+        sx = step % xt, sy = step / xt % yt, sn = step / xt / yt;
+    }
+    __device__ __forceinline__ void next()
+    {
+        x += sx, y += sy, n += sn;
+        if (x >= xtiles)
+            x -= xtiles, y++;
+        if (y >= ytiles)
+            y -= ytiles, n++;
+    }
+};
 
 // True in one lane of a converged warp, and the compiler knows that it is one: in a branch taken on `lane == 0` every tcgen05.mma, commit and
 // TMA copy is issued from a loop over the lanes that may be active, at some 200-250 cycles of this thread each.
@@ -233,7 +260,7 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t addr, uint32_t lbo,
 
 // Instruction descriptor of tcgen05.mma kind::i8: D = S32 (bits 4-5 = 2), A/B format at bits 7-9 / 10-12
 // (0 = unsigned 8 bit, 1 = signed 8 bit), both operands K-major, N>>3 at bit 17, M>>4 at bit 24.
-__device__ __forceinline__ uint32_t idesc_i8(int a_signed, int b_signed, int m, int n)
+__host__ __device__ __forceinline__ uint32_t idesc_i8(int a_signed, int b_signed, int m, int n)
 {
     return (2u << 4) | ((uint32_t)a_signed << 7) | ((uint32_t)b_signed << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
@@ -456,17 +483,8 @@ __device__ __forceinline__ uint32_t lut4(uint32_t w, uint32_t tbl)
 // row alone.  PW is a template parameter so that the walk over the columns is straight-line code; PW = 0 is the
 // generic form for any width (`pw`).  TMEM is read 16 columns at a time into two register sets in turn.
 template <int PW, bool EVEN>
-__device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_t buf, int row, int pw, int floor_q)
+__device__ __forceinline__ void epilogue_stage_at(uint32_t t0, uint32_t fp, uint32_t rb, uint32_t rx, int pw, int floor_q, bool write)
 {
-    const int width = PW ? PW : pw;
-    uint32_t rx = 0; // what the chunk offset of this row is XORed with
-    if (PW == 128)
-        rx = ((uint32_t)row & 7u) << 4;
-    else if (PW == 64)
-        rx = (((uint32_t)row >> 1) & 3u) << 4;
-    else if (PW == 32)
-        rx = (((uint32_t)row >> 2) & 1u) << 4;
-    const uint32_t rb = buf + (uint32_t)(row * width);
     int32_t va[16], vb[16];
     ld16(t0, va);
 #pragma unroll
@@ -480,7 +498,8 @@ __device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_
             ld16(t0 + c + 16, vb);
 #pragma unroll
         for (int q = 0; q < 4; q++) pk[q] = requant4_floor<EVEN>(va + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)c ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
+        if (write)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)c ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
                      : "memory");
         if (!second)
             break;
@@ -490,17 +509,32 @@ __device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_
             ld16(t0 + c + 32, va);
 #pragma unroll
         for (int q = 0; q < 4; q++) pk[q] = requant4_floor<EVEN>(vb + 4 * q, fp + (uint32_t)(c + 16 + 4 * q) * 8u, floor_q);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)(c + 16) ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]),
+        if (write)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)(c + 16) ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]),
                      "r"(pk[3])
                      : "memory");
     }
+}
+
+template <int PW, bool EVEN>
+__device__ __forceinline__ void epilogue_stage(uint32_t t0, uint32_t fp, uint32_t buf, int row, int pw, int floor_q)
+{
+    uint32_t rx = 0; // what the chunk offset of this row is XORed with
+    if (PW == 128)
+        rx = ((uint32_t)row & 7u) << 4;
+    else if (PW == 64)
+        rx = (((uint32_t)row >> 1) & 3u) << 4;
+    else if (PW == 32)
+        rx = (((uint32_t)row >> 2) & 1u) << 4;
+    epilogue_stage_at<PW, EVEN>(t0, fp, buf + (uint32_t)(row * (PW ? PW : pw)), rx, pw, floor_q, true);
 }
 
 // Staged epilogue with a fused table: as epilogue_stage, any piece width (a multiple of 16, at most 128; `mask` = 7 / 3 / 0
 // is the swizzle of 128- / 64-byte / other rows), every packed word goes through lut4 before it is stored.  A compact
 // loop kept out of line: the kernels that call it carry none of its registers in their other epilogues.
 template <bool EVEN>
-static __device__ __noinline__ void epilogue_stage_lut(uint32_t t0, uint32_t fp, uint32_t buf, int row, int pw, uint32_t mask, int floor_q, uint32_t tbl)
+static __device__ __noinline__ void epilogue_stage_lut(uint32_t t0, uint32_t fp, uint32_t buf, int row, int pw, uint32_t mask, int floor_q, uint32_t tbl,
+                                                       bool write = true)
 {
     const uint32_t rx = ((((uint32_t)(row * pw)) >> 7) & mask) << 4;
     const uint32_t rb = buf + (uint32_t)(row * pw);
@@ -512,7 +546,8 @@ static __device__ __noinline__ void epilogue_stage_lut(uint32_t t0, uint32_t fp,
         ld_wait16(v);
 #pragma unroll
         for (int q = 0; q < 4; q++) pk[q] = lut4(requant4_floor<EVEN>(v + 4 * q, fp + (uint32_t)(c + 4 * q) * 8u, floor_q), tbl);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)c ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
+        if (write)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rb + ((uint32_t)c ^ rx)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
                      : "memory");
     }
 }

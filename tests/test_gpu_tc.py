@@ -286,6 +286,13 @@ PATCH = [
     dict(n=2, h=17, w=33, cin=64, cout=96),                                   # two taps side by side (192 columns), 48-column epilogue parts
     dict(n=1, h=20, w=31, cin=64, cout=64, kh=5, kw=5, pad=(2, 2, 2, 2)),     # four of five taps side by side
     dict(n=2, h=9, w=61, cin=32, cout=128),                                   # 32-byte rows, two taps side by side
+    dict(n=2, h=18, w=28, cin=64, cout=64, in_stride=96, out_stride=160),     # channel slices: a plane per pixel of a position, boxes of single pixels out
+    dict(n=1, h=10, w=36, cin=32, cout=64, in_stride=64),                     # four planes, 256 columns
+    dict(n=1, h=10, w=36, cin=32, cout=48, out_stride=96),                    # four pixels a position, rows of 48 channels out
+    dict(n=2, h=12, w=26, cin=128, cout=48, kw=4, pad=(1, 1, 2, 1)),          # two planes of 128-byte rows
+    dict(n=1, h=7, w=4, cin=32, cout=16, kh=5, kw=7, pad=(2, 2, 3, 3)),       # one position a row, windows over three
+    dict(n=1, h=6, w=132, cin=32, cout=16, kh=2, kw=8, pad=(0, 1, 5, 2)),     # windows over four positions
+    dict(n=150, h=4, w=260, cin=64, cout=32, kh=1, kw=3, pad=(0, 0, 1, 1)),   # several tiles a row and a block
 ]
 
 
