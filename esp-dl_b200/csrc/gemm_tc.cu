@@ -85,6 +85,7 @@ struct TcParams {
     int tmem_cols;  // power of two >= 32
     int out_pw;     // staged epilogue: bytes per row of a group's output piece (0 = rows are stored directly); int16: a quarter
                     // of the bytes per row of the one tile that all groups share
+    int one_tile;   // a CTA has one tile: all four epilogue groups share it, and it is staged in the memory its loads came through
     int out_rows;   // the staging tiles leave row by row, a warp per row (rows that no TMA store can address), not as one TMA store
     int out_mask;   // swizzle mask of the staging tiles (7, 3, 1, 0)
     void *out;
@@ -223,10 +224,29 @@ __device__ __forceinline__ void store_staged_row(int8_t *dst, uint32_t buf, uint
 }
 
 // Per-column constants of an int16 tile: q = (sum + bias_half) >> shift in 64 bits, as the int8 form (fast_constants).
-struct WideParam {
-    long long bias_half;
-    int shift, pad;
+// w = H * 65536 + L as two 32-bit numbers, L in 16 bits: the constant bias + 2^(s-1), the bound that saturates H before the shift, the shift.
+struct alignas(16) WideParam {
+    int h, l;
+    int limit; // |H| beyond it is outside int16 after the shift
+    int shift;
 };
+
+// The whole of int16's epilogue after the sums, in 32-bit instructions (64-bit sums, shifts and comparisons took more than twice as many: 4100
+// cycles per 16 columns of a tile, and 31 us for 4096x1024x1024, now 26).  1 <= shift <= 31.
+template <bool EVEN>
+__device__ __forceinline__ int requant_wide(int vh, int vm, int vl, int row_h, int row_l, const WideParam c)
+{
+    int h = vh + (vm >> 8) + (c.h + row_h);
+    int l = (int)__byte_perm((uint32_t)vm, 0u, 0x4404) + vl + c.l + row_l; // the low byte of vm in the second
+    h += l >> 16;
+    if (EVEN) { // a tie is rounded up only where that gives an even number
+        const uint32_t q = __funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+        l = (l & 0xffff) + (int)(q & 1u);
+        h += l >> 16;
+    }
+    h = max(min(h, c.limit), ~c.limit);
+    return (int)__funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+}
 
 template <bool I16, bool EVEN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -242,9 +262,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int b_bytes = p.block_n * p.swz;
     const int stage_bytes = NPLANE * (a_bytes + b_bytes);
     const int n_pad = p.n_tiles * p.block_n;
-    uint8_t *out_stage = smem + (size_t)p.stages * stage_bytes; // 4 tiles of [128][out_pw] bytes, 1024-byte aligned each
+    uint8_t *out_stage = p.one_tile ? smem : smem + (size_t)p.stages * stage_bytes; // 4 tiles of [128][out_pw] bytes, 1024-byte aligned each
     const int out_tile_bytes = (BLOCK_M * p.out_pw + 1023) & ~1023;
-    uint8_t *aux = out_stage + 4 * (size_t)out_tile_bytes;
+    uint8_t *aux = smem + (size_t)p.stages * stage_bytes + (p.one_tile ? 0 : 4 * (size_t)out_tile_bytes);
     FastParam *fast_s = (FastParam *)aux; // n_pad entries, 16-byte aligned (block_n % 16 == 0)
     WideParam *wide_s = (WideParam *)aux; // int16: the current tile's columns
     uint64_t *bars = (uint64_t *)(aux + (I16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)n_pad));
@@ -285,9 +305,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (I16) {
             prefetch_tensormap(&map_a_lo);
             prefetch_tensormap(&map_b_lo);
-        } else if (p.out_pw && !p.out_rows) {
-            prefetch_tensormap(&map_out);
         }
+        if (p.out_pw && !p.out_rows)
+            prefetch_tensormap(&map_out);
     }
     if (warp == 1)
         tmem_alloc(smem_u32(tmem_slot), p.tmem_cols);
@@ -296,18 +316,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    // Per-channel constants for every output channel, once per kernel, by all threads: {bias_half, shift} pairs.
-    bool fast = false;
-    if (!I16) {
-        stage_fast_params(p.epi, fast_s, p.N, n_pad, (int)threadIdx.x, NUM_THREADS, slow_flag);
-        if (p.epi.lut)
-            stage_lut(p.epi.lut, lut_s, (int)threadIdx.x, NUM_THREADS);
-        __syncthreads();
-        fast = !*slow_flag && !p.epi.lut_stride && p.K <= 32768; // one table rides on the staged form and on the packed words of unstaged rows; per-channel tables take the general path
-    }
-    // This CTA is set up (everything above reads launch parameters and model constants only): the next kernel's CTAs may
-    // take SMs as they become free.  The producer below waits for the previous kernel before its first load, and every
-    // other role only ever acts on what the producer brought in.
+    // This CTA is set up: the next kernel's CTAs may take SMs as they become free.  The producer below waits for the previous kernel before
+    // its first load, the epilogue warps read model constants only before they have a tile, and every other role only ever
+    // acts on what the producer brought in.
     if (threadIdx.x == 0)
         grid_dep_launch();
 
@@ -507,6 +518,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int lane_group = warp & 3;         // TMEM lanes this warp may read: 32*lane_group .. +31
         const int row_in_tile = lane_group * 32 + lane;
 
+        // Per-channel constants {bias_half, shift}, once per kernel: of every output channel, or of the only tile's.  The first loads are on
+        // their way meanwhile (when all warps did this before them, a lone tile of 128x256x1024 took 1.1 us longer).
+        bool fast = false;
+        const int et0 = (int)threadIdx.x - 64;
+        if (!I16) {
+            EpiConfig epi = p.epi;
+            const int first = p.one_tile ? (int)blockIdx.x % p.n_tiles * p.block_n : 0;
+            if (epi.bias)
+                epi.bias = (const int32_t *)epi.bias + first;
+            if (epi.per_channel)
+                epi.ew += first;
+            stage_fast_params(epi, fast_s + first, p.N - first, p.one_tile ? p.block_n : n_pad, et0, EPI_WARPS * 32, slow_flag);
+            if (p.epi.lut)
+                stage_lut(p.epi.lut, lut_s, et0, EPI_WARPS * 32);
+            named_bar(1, EPI_WARPS * 32);
+            fast = !*slow_flag && !p.epi.lut_stride && p.K <= 32768; // one table rides on the staged form and on the packed words of unstaged rows; per-channel tables take the general path
+        }
         const uint32_t fp_base = epi_param_base(fast_s);
         uint32_t acc_phase = 0;
         bool ok = true;
@@ -586,6 +614,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 // bytes, then whole rows
                 constexpr int EPI_BAR = 6;
                 const int et = (int)threadIdx.x - 64;
+                const int sum = row_ok ? p.row_sum[m] : 0; // times -32768 is added to the row's results
+                if (!p.out_rows && et == 0)
+                    bulk_wait_read_all();
                 named_bar(EPI_BAR, EPI_WARPS * 32); // the previous tile's rows and constants have been read
                 if (et == 0)
                     *slow_flag = 0;
@@ -594,16 +625,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const int n = min(n0 + j, p.N - 1);
                     const int e = p.epi.per_channel ? __ldg(p.epi.ew + n) : p.epi.ew_scalar, sh = p.epi.e_shift_base - e;
                     const long long b = p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll;
-                    if (sh < 1 || sh > 58 || b >= (1ll << 58) || b <= -(1ll << 58)) // |sum| < 2^46
+                    if (sh < 1 || sh > 31 || b >= (1ll << 45) || b <= -(1ll << 45)) // H stays below 2^30: K <= 16384
                         *slow_flag = 1;
-                    const int fs = max(1, min(58, sh));
-                    wide_s[j].bias_half = b + (1ll << (fs - 1)) - (EVEN ? 1 : 0);
-                    wide_s[j].shift = fs;
+                    const int fs = max(1, min(31, sh));
+                    const long long c = b + (1ll << (fs - 1)) - (EVEN ? 1 : 0);
+                    wide_s[j] = {(int)(c >> 16), (int)(c & 0xffff), (int)((32768ll << max(0, fs - 16)) - 1), fs};
                 }
                 named_bar(EPI_BAR, EPI_WARPS * 32);
                 const bool slow = *(volatile int *)slow_flag;
-                const long long base = row_ok ? -(long long)p.row_sum[m] * 32768 : 0ll;
-                const uint32_t buf = smem_u32(out_stage), pitch = 2u * (uint32_t)p.block_n, mask = 7u;
+                const long long base = -(long long)sum * 32768;
+                const int row_h = (int)(base >> 16), row_l = (int)(base & 0xffff);
+                // staged rows: pieces of 64 columns for a TMA store each, or whole rows
+                const uint32_t buf = smem_u32(out_stage), pitch = p.out_rows ? 2u * (uint32_t)p.block_n : 128u, mask = 7u;
                 int chunk = 0;
                 for (int c0 = 0; c0 < p.block_n; c0 += 16, chunk++) {
                     if (chunk % parts != part)
@@ -616,29 +649,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     tie16(vm);
                     tie16(vl);
                     uint32_t pk[8];
+                    if (!slow) {
 #pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        long long w = base + (long long)vh[j] * 65536 + (long long)vm[j] * 256 + (long long)vl[j];
-                        int q;
-                        if (!slow) {
-                            const WideParam c = wide_s[c0 + j];
-                            w += c.bias_half;
-                            if (EVEN)
-                                w += (w >> c.shift) & 1;
-                            w >>= c.shift;
-                            const int lo = (int)w, hi = (int)(w >> 32);
-                            q = hi == (lo >> 31) ? max(-32768, min(32767, lo)) : (hi < 0 ? -32768 : 32767);
+                        for (int j = 0; j < 16; j += 2) {
+                            const int q0 = requant_wide<EVEN>(vh[j], vm[j], vl[j], row_h, row_l, wide_s[c0 + j]);
+                            const int q1 = requant_wide<EVEN>(vh[j + 1], vm[j + 1], vl[j + 1], row_h, row_l, wide_s[c0 + j + 1]);
+                            asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(pk[j >> 1]) : "r"(q1), "r"(q0));
                             if (p.epi.relu)
-                                q = max(q, 0);
-                        } else {
+                                asm("max.s16x2 %0, %0, %1;" : "+r"(pk[j >> 1]) : "r"(0));
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {
+                            const long long w = base + (long long)vh[j] * 65536 + (long long)vm[j] * 256 + (long long)vl[j];
                             const int n = min(n0 + c0 + j, p.N - 1);
                             const int e = p.epi.per_channel ? __ldg(p.epi.ew + n) : p.epi.ew_scalar;
                             const int shift = max(-62, min(62, p.epi.e_shift_base - e));
-                            q = requant16(w, p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll, shift, p.epi.relu, p.epi.half_even);
+                            const int q = requant16(w, p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll, shift, p.epi.relu, p.epi.half_even);
+                            pk[j >> 1] = j & 1 ? pk[j >> 1] | ((uint32_t)q << 16) : (uint32_t)q & 0xffffu;
                         }
-                        pk[j >> 1] = j & 1 ? pk[j >> 1] | ((uint32_t)q << 16) : (uint32_t)q & 0xffffu;
                     }
-                    const uint32_t off = (uint32_t)row_in_tile * pitch + 2u * (uint32_t)c0;
+                    const uint32_t off = (p.out_rows ? 2u * (uint32_t)c0 : (uint32_t)(c0 >> 6) * (BLOCK_M * 128u) + 2u * (uint32_t)(c0 & 63)) + (uint32_t)row_in_tile * pitch;
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (off ^ (((off >> 7) & mask) << 4))), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
                     const uint32_t off2 = off + 16u;
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (off2 ^ (((off2 >> 7) & mask) << 4))), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
@@ -647,7 +678,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 __syncwarp();
                 if (lane == 0)
                     mbar_arrive(smem_u32(&tempty_bar[acc]));
+                if (!p.out_rows)
+                    fence_async_smem();
                 named_bar(EPI_BAR, EPI_WARPS * 32);
+                if (!p.out_rows) {
+                    if (et == 0) { // rows >= M and columns >= N are clipped
+                        for (int c0 = 0; c0 < p.block_n; c0 += 64) tma_store_3d(&map_out, buf + (uint32_t)(c0 >> 6) * (BLOCK_M * 128u), 2 * (n0 + c0), m0, bi);
+                        bulk_commit();
+                    }
+                    continue;
+                }
                 const int len = 2 * min(p.block_n, p.N - n0);
                 for (int row = ew; row < BLOCK_M && m0 + row < p.M; row += EPI_WARPS)
                     store_staged_row((int8_t *)p.out + 2 * (((long long)bi * p.M + m0 + row) * p.ops + n0), buf, (uint32_t)row * pitch, len, mask, lane);
@@ -666,7 +706,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             TC_REC(6, w_work);
             TC_REC(7, w_store);
         }
-        if (!I16 && p.out_pw && !p.out_rows && (ew & 3) == 0 && lane == 0)
+        if (p.out_pw && !p.out_rows && (ew & 3) == 0 && lane == 0)
             bulk_wait_all(); // shared memory stays allocated until the last store has left it
     }
 
@@ -1011,6 +1051,14 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
         p.swz = 64; // a stage holds two planes of each operand: 64-byte rows leave room for five stages beside a wide output tile
     p.k_blocks = (p.K + p.swz - 1) / p.swz;
     p.acc_stages = i16 ? 1 : (4 * p.block_n <= 512 ? 4 : 2);
+    const long long rps = d.residual_pixel_stride ? d.residual_pixel_stride : d.out_c;
+    const bool res_ok = !d.residual || (rps % 16 == 0 && ((uintptr_t)d.residual % 16) == 0);
+    const bool stageable = res_ok && !force_direct && !getenv("ESPDL_B200_DIRECT_STORES");
+    // A CTA with one tile has nothing to overlap its epilogue with: four groups instead of two take it, and staging costs no memory (4096x1024x1024:
+    // 10.1 -> 8.0 us; direct row stores took 3.8 us of it).
+    p.one_tile = !i16 && stageable && p.block_n % 64 == 0 && (long long)p.batch * p.m_tiles * p.n_tiles <= num_sms();
+    if (p.one_tile)
+        p.acc_stages = 1;
     int cols = p.acc_stages * (i16 ? 3 : 1) * p.block_n;
     int pow2 = 32;
     while (pow2 < cols) pow2 *= 2;
@@ -1020,12 +1068,11 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     // staged epilogue (int8): each group of four epilogue warps owns a piece of block_n / parts columns
     const long long ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     p.out_pw = 0, p.out_mask = 0;
-    const long long rps = d.residual_pixel_stride ? d.residual_pixel_stride : d.out_c;
-    const bool res_ok = !d.residual || (rps % 16 == 0 && ((uintptr_t)d.residual % 16) == 0);
     p.out_rows = 0;
     if (i16) {
         p.out_pw = p.block_n / 2; // four times [128][out_pw] = the tile
-    } else if (res_ok && !force_direct && !getenv("ESPDL_B200_DIRECT_STORES")) {
+        p.out_rows = p.block_n % 64 != 0 || ops % 8 != 0 || ((uintptr_t)d.output % 16) != 0;
+    } else if (stageable) {
         p.out_rows = ops % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
         const int parts = 4 / p.acc_stages;
         if (p.block_n % (16 * parts) == 0 && p.block_n / parts <= 128) {
@@ -1033,7 +1080,7 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
             p.out_mask = p.out_pw == 128 ? 7 : (p.out_pw == 64 ? 3 : 0);
         }
     }
-    size_t out_bytes = 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023);
+    size_t out_bytes = p.one_tile ? 0 : 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023);
     size_t stage_bytes = (size_t)(i16 ? 2 : 1) * (BLOCK_M + p.block_n) * p.swz;
     int stages = (int)((SMEM_BUDGET - aux_bytes(p, i16) - out_bytes - 1024) / stage_bytes);
     // A wide tile with a reduction of two 128-byte blocks and room for only two or three stages has barely one tile's loads
@@ -1048,9 +1095,9 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
             p.swz = 64, p.k_blocks = kb64, stage_bytes = stage64, stages = stages64;
         }
     }
-    if (p.out_rows && p.out_pw && stages < 4)
+    if (!i16 && p.out_rows && p.out_pw && stages < 4)
         stages = (int)((SMEM_BUDGET_DEEP - aux_bytes(p) - out_bytes - 1024) / stage_bytes);
-    if (!i16 && p.out_pw && !p.out_rows && p.k_blocks > 2 && stages < 4) {
+    if (!i16 && !p.one_tile && p.out_pw && !p.out_rows && p.k_blocks > 2 && stages < 4) {
         // a long reduction needs the deep load pipeline more than the output needs staging
         p.out_pw = 0, p.out_mask = 0, out_bytes = 0;
         stages = (int)((SMEM_BUDGET_DEEP - aux_bytes(p) - 1024) / stage_bytes);
@@ -1211,7 +1258,7 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
         return st;
     }
     const size_t stage_bytes = (size_t)(i16 ? 2 : 1) * (BLOCK_M + p.block_n) * p.swz;
-    size_t smem = 1024 + (size_t)p.stages * stage_bytes + 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023) + aux_bytes(p, i16);
+    size_t smem = 1024 + (size_t)p.stages * stage_bytes + (p.one_tile ? 0 : 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023)) + aux_bytes(p, i16);
     CUtensorMap mo = ma;
     if (!i16 && p.out_pw && !p.out_rows) {
         const int osw = p.out_pw == 128 ? 128 : (p.out_pw == 64 ? 64 : 0);
@@ -1219,6 +1266,8 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
                            (uint64_t)p.M * (uint64_t)p.ops)))
             return st;
     }
+    if (i16 && !p.out_rows && (st = make_map(&mo, d.output, (uint64_t)p.M, 2 * (uint64_t)p.N, 2 * (uint64_t)p.ops, BLOCK_M, 128, 128)))
+        return st;
     if (smem < 120 * 1024) // more than half an SM's shared memory: one CTA per SM, so TMEM allocation never waits on a neighbour
         smem = 120 * 1024;
     const long long all_tiles = (long long)p.batch * p.m_tiles * p.n_tiles;

@@ -376,3 +376,30 @@ def test_wide_tiles_with_two_k_blocks_take_64_byte_stages(m, k, n, monkeypatch):
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), want)
     monkeypatch.setenv("ESPDL_B200_NO_NARROW_K", "1")
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), want)
+
+
+@pytest.mark.parametrize("act", [abi.ACT_LINEAR, abi.ACT_RELU])
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("m,k,n,e_w,e_out,out_stride", [
+    (300, 96, 64, (-8, -8), -13, 0),        # shift 9: results come from below the 16-bit seam
+    (129, 64, 192, (-18, -13), -12, 0),     # shifts 15 to 20 beside one another
+    (257, 512, 128, (-30, -15), -12, 0),    # and up to 32: the general form
+    (200, 128, 256, (-16, -14), -12, 264),  # two-column tiles of a wider tensor
+    (140, 80, 72, (-18, -13), -12, 0),      # no whole 64-column pieces: rows leave one by one
+    (131, 2048, 64, (-19, -19), -2, 0),     # large sums, shift 31
+])
+def test_int16_rounding_in_two_halves(m, k, n, e_w, e_out, out_stride, round_mode, act):
+    case = cases.gemm_case(seed=m + n, dtype=abi.DTYPE_INT16, m=m, k=k, n_out=n, e_in=-14, e_w=e_w, e_out=e_out, wide=True, per_channel=True, act=act,
+                           round_mode=round_mode, out_stride=out_stride)
+    want = gpu_util.run_conv_oracle(case)
+    assert len(np.unique(want)) > 2
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), want)
+
+
+@pytest.mark.parametrize("lut", [False, True])
+@pytest.mark.parametrize("m,k,n,out_stride", [(1, 64, 64, 0), (130, 96, 256, 0), (127, 1040, 200, 0), (500, 128, 1000, 0), (260, 256, 128, 144), (140, 64, 100, 0)])
+def test_one_tile_per_block(m, k, n, out_stride, lut):
+    case = cases.gemm_case(seed=m + n, m=m, k=k, n_out=n, per_channel=True, act=abi.ACT_LINEAR, lut=lut, e_in=-7, e_out=-5, e_w=(-9, -7), out_stride=out_stride)
+    want = gpu_util.run_conv_oracle(case)
+    assert want.std() > 5
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), want)
