@@ -4,7 +4,7 @@
 //
 // The op is bandwidth bound by design (9 MACs per byte read).  3x3 filters with stride 1 or 2 - the shapes of
 // MobileNet-style networks - run on dw3x3_dp4a_kernel (a thread walks along a band of rows, dp4a over byte-transposed
-// columns); other int8 shapes with C % 16 == 0 on dw_s8_vec16_kernel (16 channels per thread, 128-bit loads and
+// columns), other windows of 3x3, 5x5 and 7x7 on dwk_dp4a_kernel; other int8 shapes with C % 16 == 0 on dw_s8_vec16_kernel (16 channels per thread, 128-bit loads and
 // stores, a warp reads and writes contiguous runs of the NHWC tensor); everything else on dw_generic_kernel.
 #include "common.cuh"
 
@@ -78,6 +78,83 @@ __global__ void __launch_bounds__(256) dw_s8_vec16_kernel(DwParams p)
             packed[q] = wd;
         }
         *(uint4 *)(out + pix * p.ops + ch) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+}
+
+// K x K depthwise (5x5, 7x7), int8, any stride, dilation 1: a thread owns four consecutive channels of one output pixel.  All K*K words of its
+// window are loaded before the first is used - small maps are bound by that latency -, groups of four taps are byte-transposed
+// into one word per channel and meet the transposed filter, which the block keeps in shared memory, in one dp4a each: about three
+// instructions a tap for four channels where the kernel above takes ten.  5x5 over 64 channels: 184x184 19.0 -> 12.9 us, 23x23 11.4 -> 2.4.
+template <int K>
+__global__ void __launch_bounds__(256) dwk_dp4a_kernel(DwParams p)
+{
+    constexpr int TAPS = K * K, GROUPS = (TAPS + 3) / 4;
+    extern __shared__ uint32_t dwk_w[]; // [group][channel of the word][word]
+    grid_dep_launch();
+    if (!p.early)
+        grid_dep_wait();
+    const int words = p.c / 4;
+    for (int i = threadIdx.x; i < GROUPS * words; i += 256) {
+        const int g = i / words, c4 = i - g * words;
+        uint32_t t[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) t[j] = 4 * g + j < TAPS ? __ldg((const uint32_t *)((const int8_t *)p.w + (long long)(4 * g + j) * p.c) + c4) : 0u;
+        const uint32_t lo0 = __byte_perm(t[0], t[1], 0x5140), lo1 = __byte_perm(t[2], t[3], 0x5140), hi0 = __byte_perm(t[0], t[1], 0x7362), hi1 = __byte_perm(t[2], t[3], 0x7362);
+        dwk_w[(g * 4 + 0) * words + c4] = __byte_perm(lo0, lo1, 0x5410);
+        dwk_w[(g * 4 + 1) * words + c4] = __byte_perm(lo0, lo1, 0x7632);
+        dwk_w[(g * 4 + 2) * words + c4] = __byte_perm(hi0, hi1, 0x5410);
+        dwk_w[(g * 4 + 3) * words + c4] = __byte_perm(hi0, hi1, 0x7632);
+    }
+    if (p.early)
+        grid_dep_wait();
+    __syncthreads();
+    const unsigned total = (unsigned)(p.total); // words of the output, below 2^31
+    for (unsigned item = blockIdx.x * 256u + threadIdx.x; item < total; item += gridDim.x * 256u) {
+        const unsigned pix = item / (unsigned)words, c4 = item - pix * (unsigned)words, line = pix / (unsigned)p.ow, n = line / (unsigned)p.oh;
+        const int ox = (int)(pix - line * (unsigned)p.ow), oy = (int)(line - n * (unsigned)p.oh);
+        const int iy0 = oy * p.sh - p.pt, ix0 = ox * p.sw - p.pl;
+        const int8_t *at = (const int8_t *)p.in + (((long long)n * p.ih + iy0) * p.iw + ix0) * p.ips + 4 * c4;
+        uint32_t raw[GROUPS * 4];
+        if (iy0 >= 0 && ix0 >= 0 && iy0 + K <= p.ih && ix0 + K <= p.iw) {
+#pragma unroll
+            for (int ky = 0; ky < K; ky++)
+#pragma unroll
+                for (int kx = 0; kx < K; kx++) raw[ky * K + kx] = __ldg((const uint32_t *)(at + ((long long)ky * p.iw + kx) * p.ips));
+        } else {
+#pragma unroll
+            for (int ky = 0; ky < K; ky++)
+#pragma unroll
+                for (int kx = 0; kx < K; kx++) {
+                    raw[ky * K + kx] = 0u;
+                    if ((unsigned)(iy0 + ky) < (unsigned)p.ih && (unsigned)(ix0 + kx) < (unsigned)p.iw)
+                        raw[ky * K + kx] = __ldg((const uint32_t *)(at + ((long long)ky * p.iw + kx) * p.ips));
+                }
+        }
+#pragma unroll
+        for (int t = TAPS; t < GROUPS * 4; t++) raw[t] = 0u;
+        int acc[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int g = 0; g < GROUPS; g++) {
+            const uint32_t lo0 = __byte_perm(raw[4 * g], raw[4 * g + 1], 0x5140), lo1 = __byte_perm(raw[4 * g + 2], raw[4 * g + 3], 0x5140);
+            const uint32_t hi0 = __byte_perm(raw[4 * g], raw[4 * g + 1], 0x7362), hi1 = __byte_perm(raw[4 * g + 2], raw[4 * g + 3], 0x7362);
+            const uint32_t *f = dwk_w + g * 4 * words + c4;
+            acc[0] = __dp4a((int)__byte_perm(lo0, lo1, 0x5410), (int)f[0], acc[0]);
+            acc[1] = __dp4a((int)__byte_perm(lo0, lo1, 0x7632), (int)f[words], acc[1]);
+            acc[2] = __dp4a((int)__byte_perm(hi0, hi1, 0x5410), (int)f[2 * words], acc[2]);
+            acc[3] = __dp4a((int)__byte_perm(hi0, hi1, 0x7632), (int)f[3 * words], acc[3]);
+        }
+        uint32_t wd = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int c = (int)c4 * 4 + i;
+            const int e = p.per_channel ? __ldg(p.ew + c) : p.ew_scalar;
+            const int shift = max(-31, min(31, p.e_shift_base - e));
+            int32_t v = requant8(acc[i], p.bias ? __ldg((const int32_t *)p.bias + c) : 0, shift, p.relu, p.half_even);
+            if (p.lut)
+                v = p.lut[(long long)c * p.lut_stride + ((uint8_t)v ^ 0x80u)];
+            wd |= ((uint32_t)v & 0xffu) << (8 * i);
+        }
+        *(uint32_t *)((int8_t *)p.out + (long long)pix * p.ops + 4 * c4) = wd;
     }
 }
 
@@ -391,9 +468,11 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
     const long long max_blocks = (long long)num_sms() * 32;
     const bool vec = d.dtype == ESPDL_DTYPE_INT8 && d.in_c % 16 == 0 && p.ips % 16 == 0 && p.ops % 16 == 0 &&
         ((uintptr_t)d.input % 16) == 0 && ((uintptr_t)d.output % 16) == 0 && ((uintptr_t)d.filter % 16) == 0;
-    const bool k3 = d.dtype == ESPDL_DTYPE_INT8 && d.kh == 3 && d.kw == 3 && d.dilation_h == 1 && d.dilation_w == 1 &&
-        d.stride_h == d.stride_w && (d.stride_h == 1 || d.stride_h == 2) && d.in_c % 4 == 0 && p.ips % 4 == 0 && p.ops % 4 == 0 &&
-        ((uintptr_t)d.input % 4) == 0 && ((uintptr_t)d.output % 4) == 0 && ((uintptr_t)d.filter % 4) == 0;
+    const bool words4 = d.dtype == ESPDL_DTYPE_INT8 && d.in_c % 4 == 0 && p.ips % 4 == 0 && p.ops % 4 == 0 && ((uintptr_t)d.input % 4) == 0 &&
+        ((uintptr_t)d.output % 4) == 0 && ((uintptr_t)d.filter % 4) == 0;
+    const bool k3 = words4 && d.kh == 3 && d.kw == 3 && d.dilation_h == 1 && d.dilation_w == 1 && d.stride_h == d.stride_w &&
+        (d.stride_h == 1 || d.stride_h == 2);
+    const long long filter_bytes = (d.kh * d.kw + 3ll) / 4 * 4 * d.in_c; // of dwk_dp4a_kernel
     if (k3 && ((long long)d.in_w + 10) * p.ips <= DW_ZERO_ROW_BYTES) {
         // a thread walks along a whole band of rows when the batch gives enough threads without cutting the band
         const int rows_out = d.stride_h == 1 ? 4 : 2;
@@ -414,6 +493,12 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
             launch_overlapped(p.half_even ? dw3x3_dp4a_kernel<1, true> : dw3x3_dp4a_kernel<1, false>, dim3((unsigned)blocks), dim3(128), 0, s, p, xsegs, ytiles, cols);
         else
             launch_overlapped(p.half_even ? dw3x3_dp4a_kernel<2, true> : dw3x3_dp4a_kernel<2, false>, dim3((unsigned)blocks), dim3(128), 0, s, p, xsegs, ytiles, cols);
+    } else if (words4 && (d.kh == 3 || d.kh == 5 || d.kh == 7) && d.kh == d.kw && d.dilation_h == 1 && d.dilation_w == 1 && filter_bytes <= 48 * 1024 &&
+               pixels * (d.in_c / 4) < (d.kh == 7 ? 1024ll * num_sms() : 1ll << 31)) { // 49 words a thread leave too few threads for large maps (16x56x56x96: 85 us, 58 below)
+        p.chunks = 0;
+        p.total = pixels * (d.in_c / 4);
+        const long long blocks = min((p.total + 255) / 256, max_blocks);
+        launch_overlapped(d.kh == 3 ? dwk_dp4a_kernel<3> : (d.kh == 5 ? dwk_dp4a_kernel<5> : dwk_dp4a_kernel<7>), dim3((unsigned)blocks), dim3(256), (size_t)filter_bytes, s, p);
     } else if (vec) {
         p.chunks = d.in_c / 16;
         p.total = pixels * p.chunks;

@@ -95,3 +95,25 @@ def test_large_image_means(shape, dtype):
     case = cases.pool_case(abi.POOL_GLOBAL_AVG, seed=c, dtype=dtype, n=n, h=h, w=w, c=c)
     case["x"] = case["x"] // 4 + np.arange(c, dtype=case["x"].dtype) # channels with means apart
     pool_matches(case)
+
+
+# windows of K x K taps, four channels a thread: maps smaller than the window, uneven strides and pads, channel slices
+@pytest.mark.parametrize("act,lut,round_mode", [(abi.ACT_RELU, False, abi.ROUND_HALF_UP), (abi.ACT_LINEAR, True, abi.ROUND_HALF_EVEN)])
+@pytest.mark.parametrize("kw", [dict(n=2, h=23, w=19, cin=64, kh=5, kw=5), dict(n=1, h=3, w=4, cin=20, kh=7, kw=7), dict(n=3, h=12, w=13, cin=36, kh=5, kw=5, stride=2),
+                                dict(n=1, h=9, w=30, cin=8, kh=3, kw=3, stride=(2, 1)), dict(n=2, h=10, w=11, cin=16, kh=7, kw=7, stride=3, pad=(3, 0, 0, 2)),
+                                dict(n=1, h=8, w=8, cin=12, kh=5, kw=5, in_stride=20, out_stride=24), dict(n=1, h=6, w=6, cin=1600, kh=5, kw=5)])
+def test_depthwise_windows(kw, act, lut, round_mode):
+    case = cases.conv_case(seed=kw["cin"], depthwise=True, cout=kw["cin"], per_channel=True, act=act, lut=lut, round_mode=round_mode, e_in=-7, e_out=-5, e_w=(-9, -7), **kw)
+    want = gpu_util.run_conv_oracle(case)
+    assert want.std() > 0
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+
+
+# image means whose pixels take 1, 2, 3, 8, 32 and 40 lanes
+@pytest.mark.parametrize("dtype", BOTH)
+@pytest.mark.parametrize("shape", [(3, 19, 17, 16), (2, 24, 12, 32), (2, 15, 15, 48), (1, 23, 23, 128), (5, 9, 9, 512), (1, 20, 20, 640), (1, 60, 60, 4)])
+def test_image_means(shape, dtype):
+    n, h, w, c = shape
+    case = cases.pool_case(abi.POOL_GLOBAL_AVG, seed=c, dtype=dtype, n=n, h=h, w=w, c=c)
+    case["x"] = case["x"] // 4 + np.arange(c, dtype=case["x"].dtype) % 90
+    pool_matches(case)
