@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <cmath>
 #include <mutex>
 #include <map>
 
@@ -438,6 +439,26 @@ int espdl::conv_validate(const espdl_conv_desc *d)
 
 constexpr long long DW_SMALL = 8ll << 20; // outputs of a stride-2 conv; twice that at stride 1
 
+// Short windows with few output channels: the CUDA cores where every other kernel would take longer.  The tile kernel's time is that of its waves
+// of 128-pixel tiles, each its taps' loads one after the other and its rows' epilogue (from 2x2 and 3x3 windows of 33 to 540 thousand pixels); the
+// warp-level instructions take about twice their estimate where chunks are words.
+static bool runs_narrow(const espdl_conv_desc &d)
+{
+    const char *knob = getenv("ESPDL_B200_NARROW"); // 0: never, always: wherever it can run
+    if (d.kernel != ESPDL_KERNEL_AUTO || d.n <= 0 || !conv2d_narrow_supported(d) || (knob && *knob == '0'))
+        return false;
+    if (knob && *knob == 'a')
+        return true;
+    if (conv2d_stem_tc_supported(d) || conv2d_band_tc_supported(d) || (d.in_c % 8 && d.kh * d.kw * d.in_c > 64)) // longer windows of words: packed operands
+        return false;
+    const float us = conv2d_narrow_estimate_us(d);
+    const float mma = conv2d_mma_supported(d) ? conv2d_mma_estimate_us(d) : 8.f;
+    if (mma < 8.f && mma * (d.in_c % 16 ? 2.f : 1.f) < 1.1f * us)
+        return false;
+    const double waves = ceil((double)d.n * d.out_h * d.out_w / 128 / num_sms());
+    return us < (conv2d_conv_tc_supported(d) ? 2.5 + waves * (0.6 + 0.17 * d.kh * d.kw + 0.045 * d.out_c) : (double)conv2d_simt_estimate_us(d));
+}
+
 // Small enough for the warp-level matrix instructions?
 static bool runs_mma(const espdl_conv_desc &d)
 {
@@ -483,7 +504,7 @@ int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes
     int st = conv_validate(desc);
     if (st)
         return st;
-    if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1 || runs_mma(*desc))
+    if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1 || runs_narrow(*desc) || runs_mma(*desc))
         return ESPDL_OK;
     if (conv2d_tc_supported(*desc))
         *bytes = conv2d_tc_workspace_bytes(*desc);
@@ -522,6 +543,8 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
             return conv2d_dw_tma(*desc, s);
         return conv2d_depthwise(*desc, s);
     }
+    if (runs_narrow(*desc))
+        return conv2d_narrow(*desc, s);
     if (runs_mma(*desc))
         return conv2d_mma(*desc, s);
     if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_stem_tc_supported(*desc))

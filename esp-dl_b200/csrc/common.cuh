@@ -78,6 +78,9 @@ int conv_validate(const espdl_conv_desc *d);
 
 // kernels behind the C ABI (one translation unit each)
 int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s);
+int conv2d_narrow(const espdl_conv_desc &d, cudaStream_t s); // short windows, few output channels
+bool conv2d_narrow_supported(const espdl_conv_desc &d);
+float conv2d_narrow_estimate_us(const espdl_conv_desc &d);
 float conv2d_simt_estimate_us(const espdl_conv_desc &d); // about what it takes, for the choice against packed operands
 int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s);
 bool conv2d_tc_supported(const espdl_conv_desc &d);

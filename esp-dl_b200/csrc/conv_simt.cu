@@ -259,6 +259,116 @@ __global__ void __launch_bounds__(256) conv_s8_small_k_kernel(ConvParams p)
     }
 }
 
+// Short windows with few output channels over large maps (the 2x2 convs of a text detector's first and last layers), int8: a thread owns an
+// output pixel and four channels, the filter sits in shared memory as [chunk][channel of four][group], so that the lanes of a pixel
+// read neighbouring chunks at once, and the loads of four chunks of the window are in flight together.  A tile kernel spends 1.3
+// to 2.6 us per wave of 128-pixel tiles on these, nearly all of it on the tile's way through its pipeline, for 64 multiply-adds an
+// output: 735x735x16 -> 1, 2x2 40 -> 13.5 us, 367x367x16 -> 16 18.5 -> 13.5, 368x368x8 -> 16 24.3 -> 12.1.
+constexpr int NARROW_MAX_K = 144, NARROW_MAX_OC = 32;
+
+template <typename U>
+__global__ void __launch_bounds__(256) conv_s8_narrow_kernel(ConvParams p, int early)
+{
+    constexpr int CH = (int)sizeof(U), WORDS = CH / 4;
+    struct alignas(CH) Chunk {
+        int w[WORDS];
+    };
+    extern __shared__ __align__(16) uint8_t narrow_w[];
+    Chunk *w_s = (Chunk *)narrow_w;
+    grid_dep_launch();
+    if (!early)
+        grid_dep_wait();
+    const int per_tap = p.ic / CH, chunks = p.kh * p.kw * per_tap, groups = p.groups;
+    for (int i = threadIdx.x; i < chunks * 4 * groups; i += 256) {
+        const int g = i % groups, j = i / groups % 4, q = i / groups / 4, oc = 4 * g + j;
+        Chunk v = {};
+        if (oc < p.oc) {
+            const U t = __ldg((const U *)((const int8_t *)p.w + (long long)oc * chunks * CH) + q);
+            v = *(const Chunk *)&t;
+        }
+        w_s[i] = v;
+    }
+    if (early)
+        grid_dep_wait();
+    __syncthreads();
+    const unsigned total = (unsigned)p.total; // below 2^31
+    for (unsigned item = blockIdx.x * 256u + threadIdx.x; item < total; item += gridDim.x * 256u) {
+        const unsigned pix = item / (unsigned)groups, g = item - pix * (unsigned)groups, line = pix / (unsigned)p.ow, n = line / (unsigned)p.oh;
+        const int iy0 = (int)(line - n * (unsigned)p.oh) * p.sh - p.pt, ix0 = (int)(pix - line * (unsigned)p.ow) * p.sw - p.pl;
+        const int8_t *image = (const int8_t *)p.in + (long long)n * p.ih * p.iw * p.ips;
+        int acc[4] = {0, 0, 0, 0};
+        int ky = 0, kx = 0, c = 0; // of chunk q
+#pragma unroll 1
+        for (int q0 = 0; q0 < chunks; q0 += 4) {
+            Chunk a[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int iy = iy0 + ky * p.dh, ix = ix0 + kx * p.dw;
+                a[u] = {};
+                if (q0 + u < chunks && (unsigned)iy < (unsigned)p.ih && (unsigned)ix < (unsigned)p.iw) {
+                    const U t = __ldg((const U *)(image + ((long long)iy * p.iw + ix) * p.ips) + c);
+                    a[u] = *(const Chunk *)&t;
+                }
+                if (++c == per_tap) {
+                    c = 0;
+                    if (++kx == p.kw)
+                        kx = 0, ky++;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (q0 + u >= chunks)
+                    break;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const Chunk b = w_s[((q0 + u) * 4 + j) * groups + g];
+#pragma unroll
+                    for (int i = 0; i < WORDS; i++) acc[j] = __dp4a(a[u].w[i], b.w[i], acc[j]);
+                }
+            }
+        }
+        const int oc0 = (int)g * 4;
+        int8_t *op = (int8_t *)p.out + (long long)pix * p.ops + oc0;
+        uint32_t word = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int oc = min(oc0 + j, p.oc - 1);
+            const int shift = max(-31, min(31, p.e_shift_base - (p.per_channel ? __ldg(p.ew + oc) : p.ew_scalar)));
+            int q = requant8(acc[j], p.bias ? __ldg((const int32_t *)p.bias + oc) : 0, shift, p.relu, p.half_even);
+            if (p.lut)
+                q = p.lut[(long long)oc * p.lut_stride + ((uint8_t)q ^ 0x80u)];
+            if (p.res)
+                q = sat8(q + (int)p.res[(long long)pix * p.rps + oc]);
+            word |= ((uint32_t)q & 0xffu) << (8 * j);
+        }
+        if (oc0 + 4 <= p.oc && (p.ops & 3) == 0 && ((uintptr_t)p.out & 3) == 0) {
+            *(uint32_t *)op = word;
+        } else {
+            for (int j = 0; j < 4 && oc0 + j < p.oc; j++) op[j] = (int8_t)(word >> (8 * j));
+        }
+    }
+}
+
+static int narrow_chunk(const espdl_conv_desc &d)
+{
+    const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
+    const uintptr_t all = (uintptr_t)d.in_c | (uintptr_t)ips | (uintptr_t)d.input | (uintptr_t)d.filter;
+    return all % 16 == 0 ? 16 : (all % 8 == 0 ? 8 : (all % 4 == 0 ? 4 : 0));
+}
+
+bool conv2d_narrow_supported(const espdl_conv_desc &d)
+{
+    return d.dtype == ESPDL_DTYPE_INT8 && d.group == 1 && d.filter_image_stride == 0 && d.kh * d.kw > 1 && d.kh * d.kw * d.in_c <= NARROW_MAX_K && d.out_c <= NARROW_MAX_OC &&
+        narrow_chunk(d) && (long long)d.n * d.out_h * d.out_w * ((d.out_c + 3) / 4) < (1ll << 31);
+}
+
+// A thread's instructions - a dot product per word and channel, about fourteen per chunk, sixty for the ends - at the measured issue rate.
+float conv2d_narrow_estimate_us(const espdl_conv_desc &d)
+{
+    const double items = (double)d.n * d.out_h * d.out_w * ((d.out_c + 3) / 4), K = d.kh * d.kw * d.in_c;
+    return (float)(2.0 + items * (K + 14 * K / narrow_chunk(d) + 60) / (num_sms() * 4 * 32 * 430.0));
+}
+
 static bool simt_dp4a(const espdl_conv_desc &d)
 {
     const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
@@ -282,9 +392,8 @@ float conv2d_simt_estimate_us(const espdl_conv_desc &d)
     return (float)(3.0 + words * 0.3 + macs / rate);
 }
 
-int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
+static void fill_params(const espdl_conv_desc &d, ConvParams &p)
 {
-    ConvParams p;
     p.res = (const int8_t *)d.residual, p.rps = d.residual_pixel_stride ? d.residual_pixel_stride : d.out_c;
     p.in = d.input, p.w = d.filter, p.bias = d.bias, p.out = d.output, p.ew = d.filter_exponents, p.lut = d.lut, p.lut_stride = d.lut_channel_stride;
     p.n = d.n, p.ih = d.in_h, p.iw = d.in_w, p.ic = d.in_c, p.oh = d.out_h, p.ow = d.out_w, p.oc = d.out_c;
@@ -296,9 +405,29 @@ int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
     p.e_shift_base = d.out_exponent - d.in_exponent;
     p.ew_scalar = d.filter_exponent, p.per_channel = d.per_channel;
     p.relu = d.activation == ESPDL_ACT_RELU, p.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
-    constexpr int OCT = 4;
-    p.groups = (d.out_c + OCT - 1) / OCT;
+    p.groups = (d.out_c + 3) / 4;
     p.total = (long long)d.n * d.out_h * d.out_w * p.groups;
+}
+
+int conv2d_narrow(const espdl_conv_desc &d, cudaStream_t s)
+{
+    ConvParams p;
+    fill_params(d, p);
+    p.lanes = 1;
+    const unsigned grid = (unsigned)min((p.total + 255) / 256, (long long)num_sms() * 32);
+    const size_t smem = (size_t)p.groups * 4 * d.kh * d.kw * d.in_c;
+    const int chunk = narrow_chunk(d);
+    launch_overlapped(chunk == 16 ? conv_s8_narrow_kernel<uint4> : (chunk == 8 ? conv_s8_narrow_kernel<uint2> : conv_s8_narrow_kernel<uint32_t>), dim3(grid), dim3(256), smem, s, p,
+                      (int)in_model_scope());
+    count_launch();
+    return check_launch("conv2d_narrow");
+}
+
+int conv2d_simt(const espdl_conv_desc &d, cudaStream_t s)
+{
+    ConvParams p;
+    fill_params(d, p);
+    constexpr int OCT = 4;
     const int threads = 256;
     p.lanes = simt_lanes(d);
     long long blocks = (p.total * p.lanes + threads - 1) / threads;

@@ -67,3 +67,16 @@ def test_batch_of_products(k, n, forced):
         one = cases.conv_case(seed=1, n=1, h=1, w=rows, cin=k, cout=n, bias=False, **P0)
         one.update(x=x[i:i + 1], w=w[i], filter_exponent=whole["filter_exponent"])
         np.testing.assert_array_equal(got[i:i + 1], gpu_util.run_conv_oracle(one))
+
+
+# short windows with few output channels on the CUDA cores: chunks of 16, 8 and 4 bytes, ragged channels, slices, every border
+@pytest.mark.parametrize("act,lut,round_mode", [(abi.ACT_RELU, False, abi.ROUND_HALF_UP), (abi.ACT_LINEAR, True, abi.ROUND_HALF_EVEN)])
+@pytest.mark.parametrize("kw", [dict(n=2, h=31, w=29, cin=16, cout=1, kh=2, kw=2, pad=(1, 1, 1, 1)), dict(n=1, h=40, w=17, cin=8, cout=16, kh=2, kw=2, pad=(0, 1, 0, 1)),
+                                dict(n=1, h=9, w=9, cin=4, cout=30, kh=5, kw=5, stride=2), dict(n=3, h=7, w=20, cin=48, cout=6, kh=1, kw=3, in_stride=64, out_stride=12),
+                                dict(n=1, h=12, w=12, cin=12, cout=32, kh=3, kw=4, dil=2, pad=(2, 2, 3, 3)), dict(n=70, h=60, w=50, cin=16, cout=3, kh=2, kw=2, pad=(1, 0, 1, 0))])
+def test_narrow_windows(kw, act, lut, round_mode, monkeypatch):
+    monkeypatch.setenv("ESPDL_B200_NARROW", "always")
+    case = cases.conv_case(seed=kw["cin"] + kw["h"], per_channel=True, act=act, lut=lut, round_mode=round_mode, e_in=-7, e_out=-6, e_w=(-9, -7), **kw)
+    want = gpu_util.run_conv_oracle(case)
+    assert want.std() > 0
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
