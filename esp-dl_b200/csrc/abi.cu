@@ -437,7 +437,14 @@ int espdl::conv_validate(const espdl_conv_desc *d)
     return ESPDL_OK;
 }
 
-constexpr long long DW_SMALL = 8ll << 20; // outputs of a stride-2 conv; twice that at stride 1
+// 3x3 depthwise tensors, in outputs, below which the kernel without the TMA pipeline is the faster one.  In a model's stream of overlapping
+// launches up to 16 M at stride 1 and 2 M at stride 2 (14x14x384 1.7 against 4.1 us, 16 images of 56x56x144 5.8 / 7.9; 64 of 28x28x192 at stride
+// 2 5.6 / 5.2); launched one by one, where it has no previous kernel to hide its first loads behind, up to 1 M and 256 K (16 of
+// 28x28x192 6.3 / 5.3).
+static long long dw_small(int stride)
+{
+    return stride == 1 ? (espdl::in_model_scope() ? 16ll << 20 : 1ll << 20) : (espdl::in_model_scope() ? 2ll << 20 : 256ll << 10);
+}
 
 // Short windows with few output channels: the CUDA cores where every other kernel would take longer.  The tile kernel's time is that of its waves
 // of 128-pixel tiles, each its taps' loads one after the other and its rows' epilogue (from 2x2 and 3x3 windows of 33 to 540 thousand pixels); the
@@ -535,9 +542,8 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
         if (desc->kernel == ESPDL_KERNEL_TCGEN05)
             return ESPDL_ERR_UNSUPPORTED;
         // 3x3 int8 with 16-byte channel runs: the TMA-fed kernel; ESPDL_KERNEL_SIMT asks for the kernels that read global
-        // memory directly.  Those are also the faster ones for tensors that fit into L2: no TMA pipeline to start (1.7 against 4.1 us
-        // for 14x14x384, 5.9 against 7.9 for 16 images of 56x56x144)
-        const bool small = desc->kernel == ESPDL_KERNEL_AUTO && (long long)desc->n * desc->out_h * desc->out_w * desc->out_c < (desc->stride_h == 1 ? 2 : 1) * DW_SMALL && desc->kh == 3 &&
+        // memory directly, which also run small layers (dw_small)
+        const bool small = desc->kernel == ESPDL_KERNEL_AUTO && (long long)desc->n * desc->out_h * desc->out_w * desc->out_c < dw_small(desc->stride_h) && desc->kh == 3 &&
             !getenv("ESPDL_B200_DEBUG_WAIT_EXPIRY") && !getenv("ESPDL_B200_DW_TMA_NARROW");
         if (desc->kernel != ESPDL_KERNEL_SIMT && !small && conv2d_dw_tma_supported(*desc))
             return conv2d_dw_tma(*desc, s);

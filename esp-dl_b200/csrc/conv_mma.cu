@@ -354,7 +354,7 @@ MmaPlan mma_plan(const espdl_conv_desc &d)
     const bool batched = d.filter_image_stride != 0;
     const long long M = (batched ? 1ll : (long long)d.n) * d.out_h * d.out_w, images = batched ? d.n : 1;
     const int steps = mma_steps(d);
-    const float loads = mma_align(d) == 16 ? 1.f : (mma_align(d) == 4 ? 4.f : 8.f), window = is_window(d) ? 0.0168f : 0.f;
+    const float loads = mma_align(d) == 16 ? 1.f : (mma_align(d) == 4 ? 4.f : 8.f), window = is_window(d) ? (mma_align(d) == 4 ? 0.2f : 0.0168f) : 0.f; // words find their tap one by one
     static const int shapes[3][2] = {{1, 1}, {1, 2}, {2, 2}};
     MmaPlan best = {0, 0, 0, 1e30f};
     for (const auto &s : shapes) {

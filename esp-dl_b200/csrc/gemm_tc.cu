@@ -1075,7 +1075,15 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     } else if (stageable) {
         p.out_rows = ops % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
         const int parts = 4 / p.acc_stages;
-        if (p.block_n % (16 * parts) == 0 && p.block_n / parts <= 128) {
+        // Rows that no TMA store can address: a warp per staged row takes a tile 3.3 us whatever its width, a thread storing its own row about 1.2 and
+        // 0.12 for every store its alignment makes of it (131072 rows of 64: 14 columns 11.1 against 24.6 staged, 40 13.3 / 22.5, 100 28.7 / 24.9, 150
+        // 202 / 48); a lone tile waits for either.
+        const uintptr_t mixed = (uintptr_t)ops | (uintptr_t)d.output | (p.n_tiles > 1 ? (uintptr_t)p.block_n : 16u) | 16u;
+        const int stores = min(p.N, p.block_n) / (int)(mixed & (~mixed + 1));
+        const bool few_stores = p.out_rows && stores < ((long long)p.batch * p.m_tiles * p.n_tiles > 4ll * num_sms() ? 20 : 30);
+        if (few_stores)
+            p.out_rows = 0;
+        else if (p.block_n % (16 * parts) == 0 && p.block_n / parts <= 128) {
             p.out_pw = p.block_n / parts;
             p.out_mask = p.out_pw == 128 ? 7 : (p.out_pw == 64 ? 3 : 0);
         }

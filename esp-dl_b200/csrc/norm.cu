@@ -431,7 +431,9 @@ extern "C" int espdl_b200_norm(const espdl_norm_desc *d, void *stream)
         const int V = d->dtype == ESPDL_DTYPE_INT8 ? 4 : 2, pitch = ((d->len + V - 1) / V) | 1;
         const long long fit = (50 * 1024) / ((long long)pitch * 4 + 8), share = (d->rows + num_sms() - 1) / num_sms();
         const int R = (int)min(min(256ll, max(fit, (96 * 1024) / ((long long)pitch * 4 + 8) >= 32 ? 32ll : 0ll)), max(32ll, share)) / 32 * 32;
-        if (R >= 32 && d->rows >= 256)
+        // long rows: a block of 32 takes its time whatever else there is (11 us for 768 int8, 18 int16), a warp per row is faster below some waves of rows
+        const long long few = d->len <= 128 ? 256 : (long long)num_sms() * (V == 4 ? 24 : 32);
+        if (R >= 32 && d->rows >= few)
             return d->dtype == ESPDL_DTYPE_INT8 ? launch_layer_rows<int8_t>(p, R, pitch, (cudaStream_t)stream) : launch_layer_rows<int16_t>(p, R, pitch, (cudaStream_t)stream);
     }
     const long long blocks = (d->rows + 7) / 8; // eight rows (warps) per block
