@@ -537,8 +537,7 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
         return ESPDL_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if (desc->group != 1) {
-        // Depthwise convs run on the CUDA cores (dp4a): a tcgen05 MMA of M=128 takes ~143 cycles however small N is,
-        // which caps any diagonal-filter formulation on the tensor cores far below the dp4a walk.
+        // Depthwise convs run on the CUDA cores (dp4a)
         if (desc->kernel == ESPDL_KERNEL_TCGEN05)
             return ESPDL_ERR_UNSUPPORTED;
         // 3x3 int8 with 16-byte channel runs: the TMA-fed kernel; ESPDL_KERNEL_SIMT asks for the kernels that read global

@@ -1,7 +1,7 @@
 // Small int8 convs, Gemms and products with the warp-level matrix instruction (mma.sync m16n8k32).
 //
-// The tile kernels start a TMA pipeline, tensor memory and eighteen warps per CTA and issue M = 128 instructions that take the
-// tensor pipe 174 cycles each: right for large products, but a layer of one image (a few hundred pixels) is then all start-up - 3.1 us
+// The tile kernels start a TMA pipeline, tensor memory and eighteen warps per CTA and issue M = 128 instructions one after the other:
+// right for large products, but a layer of one image (a few hundred pixels) is then all start-up - 3.1 us
 // for next to nothing, 0.35 us more for every 128 bytes of the reduction (7x7x960 -> 160: 5.9 us, 10x10x128 -> 256 3x3 stride 2:
 // 8.9 us) against 1.2 us for an empty kernel.  Here a warp computes a tile of (16 MT) x (8 NT) outputs straight from global
 // memory (everything involved sits in L2), up to eight warps share a tile's reduction and add up through shared memory, and the first
