@@ -9,6 +9,7 @@
 // accumulations (the product, the sum of exponentials) are not associative: the walk visits the reduced elements in
 // the reference's order (row-major over the reduced axes), one thread per output.
 #include "common.cuh"
+#include "reduce_plan.cuh"
 
 #include <climits>
 #include <cooperative_groups.h>
@@ -329,21 +330,11 @@ __global__ void __launch_bounds__(THREADS) channel_reduce_kernel(ReduceParams p,
 template <typename T, int V, typename ACC, int THREADS>
 int launch_channel_reduce(const ReduceParams &p, long long outer, int C, cudaStream_t s)
 {
-    const int lanes = (C + V - 1) / V;
-    // about sixteen pixels a thread, so that the meeting in shared memory stays small beside the loads (7x7x1280 over 1024 images:
-    // 54 us with five), and at least 128 contiguous bytes a block where the tensor has them
-    const int want = (int)max(1ll, min((long long)THREADS, p.count / 16));
-    const int widest = max(8, THREADS / want);
-    int slices = (lanes + widest - 1) / widest, slice_lanes = (lanes + slices - 1) / slices;
-    // few images: slices whose lanes are a power of two (the short meeting), although neighbouring slices then share memory sectors
-    if ((slice_lanes & (slice_lanes - 1)) && outer * (lanes / (lanes & -lanes)) <= num_sms())
-        slice_lanes = lanes & -lanes, slices = lanes / slice_lanes;
-    const int rows = THREADS / slice_lanes;
+    const ReducePlan plan = reduce_plan(outer, p.count, C, V, THREADS, num_sms());
+    if (plan.rows < 1)
+        return ESPDL_ERR_UNSUPPORTED;
+    const int slice_lanes = plan.slice_lanes, slices = plan.slices, rows = plan.rows, cl = plan.cluster;
     const long long items = outer * slices;
-    // blocks that share an image: only while they do not outnumber what the SMs hold at once, and each thread keeps a full round of loads
-    constexpr int WIDEST_CLUSTER = THREADS > 256 ? 16 : 8; // 16 needs the kernel's consent (below)
-    int cl = 1;
-    while (cl < WIDEST_CLUSTER && items * cl * 2 <= 4ll * num_sms() && p.count >= 8ll * rows * cl) cl *= 2;
     if (items * cl > 0x7fffffffll)
         return ESPDL_ERR_TOO_LARGE;
     cudaLaunchConfig_t cfg = {};

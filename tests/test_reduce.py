@@ -137,3 +137,59 @@ def test_reduce_and_slice_nodes_in_a_model(tmp_path):
     for out in m.outputs:
         np.testing.assert_array_equal(out.array, want[out.name])
     m.close()
+
+
+PLAN_PROGRAM = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "reduce_plan.cuh"
+int main()
+{
+    long long checked = 0;
+    for (int threads : {256, 512})
+        for (int V : {1, 2, 4, 8, 16})
+            for (int C = 1; C <= 65536; C += C < 2048 ? 1 : (C % 256 ? 256 - C % 256 : 256))
+                for (long long count : {1ll, 2ll, 15ll, 16ll, 31ll, 48ll, 49ll, 80ll, 127ll, 256ll, 399ll, 1000ll, 4096ll, 33856ll, 1000000ll})
+                    for (long long outer : {1ll, 3ll, 27ll, 148ll, 1024ll}) {
+                        const espdl::ReducePlan q = espdl::reduce_plan(outer, count, C, V, threads, 148);
+                        const int lanes = (C + V - 1) / V;
+                        checked++;
+                        if (q.rows < 1 || q.slice_lanes < 1 || q.slice_lanes * q.rows > threads || (long long)q.slices * q.slice_lanes < lanes ||
+                            (long long)(q.slices - 1) * q.slice_lanes >= lanes || q.cluster < 1 || q.cluster > (threads > 256 ? 16 : 8)) {
+                            printf("threads %d V %d C %d count %lld outer %lld: lanes %d slices %d rows %d cluster %d\n", threads, V, C, count, outer, q.slice_lanes,
+                                   q.slices, q.rows, q.cluster);
+                            return 1;
+                        }
+                    }
+    printf("%lld plans\n", checked);
+    return 0;
+}
+"""
+
+
+def test_channel_reduction_plan_covers_every_channel_count(tmp_path):
+    """Every plan keeps at least one row of pixels in a block, covers all channels with no empty slice and stays inside the block
+    (512 lanes a slice in blocks of 256 threads read nothing: 8192 int8 channels in one image)."""
+    import os
+    import subprocess
+    src = tmp_path / "plan.cpp"
+    src.write_text(PLAN_PROGRAM)
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "esp-dl_b200", "csrc")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-I" + csrc, str(src), "-o", str(tmp_path / "plan")])
+    r = subprocess.run([str(tmp_path / "plan")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("c", [4096, 8192, 24576])
+@pytest.mark.parametrize("count", [49, 80])
+def test_many_channels_of_few_images(c, count, dtype):
+    import gpu_util
+    for op in (abi.REDUCE_MEAN, abi.REDUCE_SUM, abi.REDUCE_MAX, abi.REDUCE_L1):
+        d, x, y = make(op, dtype, (1, count, c), (1,), *exps(op, dtype), seed=c + count)
+        assert checkers.oracle().oracle_reduce(C.byref(d)) == 0
+        with gpu_util.DeviceBuffers() as dev:
+            d.input, d.output = dev.upload(x), dev.upload(np.zeros_like(y))
+            abi.check(dev.lib.espdl_b200_reduce(C.byref(d), None), "reduce")
+            np.testing.assert_array_equal(dev.download(d.output, y), y)
