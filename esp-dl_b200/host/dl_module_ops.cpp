@@ -609,34 +609,56 @@ static size_t spread_bytes(const std::vector<int> &b0, const std::vector<int> &b
     return full0 && !full1 && !none1 && count * slice <= (64u << 20) ? count * slice : 0;
 }
 
+// `n` products [M][K] x [N][K], `image_stride` elements from the filter of one to the next (0: all share one).
+void MatMul::fill_desc(ModelContext *context, void *desc, const void *input, const void *filter, void *output, int n, int M, int K, int N, int image_stride)
+{
+    espdl_conv_desc &d = *(espdl_conv_desc *)desc;
+    TensorBase *in0 = context->get_tensor(m_inputs_index[0]), *in1 = context->get_tensor(m_inputs_index[1]), *out = context->get_tensor(m_outputs_index[0]);
+    memset(&d, 0, sizeof(d));
+    d.input = input, d.filter = filter, d.output = output;
+    d.dtype = quant_dtype(quant_type);
+    d.n = n, d.in_h = d.out_h = 1, d.in_w = d.out_w = M, d.in_c = K, d.out_c = N, d.kh = d.kw = 1;
+    d.stride_h = d.stride_w = d.dilation_h = d.dilation_w = 1, d.group = 1;
+    d.filter_image_stride = image_stride;
+    d.in_exponent = in0->exponent, d.out_exponent = out->exponent, d.filter_exponent = in1->exponent, d.per_channel = 0;
+    d.activation = m_activation == ReLU ? ESPDL_ACT_RELU : ESPDL_ACT_LINEAR;
+    d.round_mode = context->round_mode;
+}
+
+// The scratch of the launches that forward() makes, from the same descriptors: a step that declares none is handed none, since the plan
+// orders branches by what their steps declare.
 size_t MatMul::workspace_bytes(ModelContext *context)
 {
     std::vector<int> b0, b1;
     int M, K, N;
-    if (!slices(context, b0, b1, M, K, N))
+    m_scratch = 0;
+    TensorBase *in0 = context->get_tensor(m_inputs_index[0]), *in1 = context->get_tensor(m_inputs_index[1]), *out = context->get_tensor(m_outputs_index[0]);
+    if (!in0 || !in1 || !out || !in0->device || !in1->device || !out->device || !slices(context, b0, b1, M, K, N))
         return 0;
-    const size_t spread = spread_bytes(b0, b1, (size_t)K * N * (quant_type == QUANT_TYPE_SYMM_16BIT ? 2 : 1));
-    if (spread || quant_type != QUANT_TYPE_SYMM_16BIT)
-        return spread;
-    espdl_conv_desc d;
-    memset(&d, 0, sizeof(d));
-    d.dtype = ESPDL_DTYPE_INT16, d.n = 1, d.in_h = d.out_h = 1, d.in_w = d.out_w = M, d.in_c = K, d.out_c = N, d.kh = d.kw = 1;
-    d.stride_h = d.stride_w = d.dilation_h = d.dilation_w = 1, d.group = 1;
-    // the query validates the descriptor like a launch does, so it needs the operands' addresses too
-    TensorBase *in0 = context->get_tensor(m_inputs_index[0]), *in1 = context->get_tensor(m_inputs_index[1]);
-    TensorBase *out = context->get_tensor(m_outputs_index[0]);
-    if (!in0 || !in1 || !out || !in0->device || !in1->device || !out->device)
-        return 0;
-    d.input = in0->device, d.filter = in1->device, d.output = out->device;
-    // the batched form (one launch over all slices) splits all rows at once
+    const size_t es = quant_type == QUANT_TYPE_SYMM_16BIT ? 2 : 1;
+    const size_t spread = spread_bytes(b0, b1, (size_t)K * N * es);
     long long count = 1;
-    for (size_t i = 0; i < b0.size(); i++) count *= std::max(b0[i], b1[i]);
-    bool shared = true;
-    for (int v : b1) shared = shared && v == 1;
-    if (shared && count > 1 && count <= 0x7fffffffll)
-        d.n = (int)count;
-    size_t bytes = 0;
-    return espdl_b200_conv2d_workspace_bytes(&d, &bytes) == ESPDL_OK ? bytes : 0;
+    bool full0 = true, full1 = true, none1 = true;
+    for (size_t i = 0; i < b0.size(); i++) {
+        const int o = std::max(b0[i], b1[i]);
+        full0 = full0 && b0[i] == o, full1 = full1 && b1[i] == o, none1 = none1 && b1[i] == 1;
+        count *= o;
+    }
+    auto need = [&](size_t at, int n, int image_stride) {
+        espdl_conv_desc d;
+        size_t bytes = 0;
+        fill_desc(context, &d, (const char *)in0->device + at * M * K * es, (const char *)in1->device + at * K * N * es, (char *)out->device + at * M * N * es, n, M, K, N, image_stride);
+        if (espdl_b200_conv2d_workspace_bytes(&d, &bytes) == ESPDL_OK)
+            m_scratch = std::max(m_scratch, bytes);
+    };
+    if (spread) {
+        m_scratch = spread;
+    } else if (count > 1 && full0 && (full1 || none1) && count <= 0x7fffffffll && (long long)K * N <= 0x7fffffffll) {
+        need(0, (int)count, none1 ? 0 : K * N);
+    } else { // slices may start at different alignments: as many as there are within 16 bytes
+        for (size_t i = 0; i < 16; i++) need(i, 1, 0);
+    }
+    return m_scratch;
 }
 
 esp_err_t MatMul::prepare(ModelContext *context)
@@ -693,19 +715,12 @@ void MatMul::forward(ModelContext *context, runtime_mode_t mode)
         st = enqueue_copy(context, in1->device, context->workspace, (int)es, shape, from, to);
         filter = context->workspace, full1 = true;
     }
+    void *scratch = m_scratch && !spread ? context->workspace : nullptr;
+    const size_t scratch_bytes = scratch ? context->workspace_bytes : 0;
     if (!st && count > 1 && full0 && (full1 || none1) && count <= 0x7fffffffll && (long long)K * N <= 0x7fffffffll) {
         espdl_conv_desc d;
-        memset(&d, 0, sizeof(d));
-        d.input = in0->device, d.filter = filter, d.output = out->device;
-        d.dtype = quant_dtype(quant_type);
-        d.n = (int)count, d.in_h = d.out_h = 1, d.in_w = d.out_w = M, d.in_c = K, d.out_c = N, d.kh = d.kw = 1;
-        d.stride_h = d.stride_w = d.dilation_h = d.dilation_w = 1, d.group = 1;
-        d.filter_image_stride = none1 ? 0 : K * N;
-        d.in_exponent = in0->exponent, d.out_exponent = out->exponent, d.filter_exponent = in1->exponent, d.per_channel = 0;
-        d.activation = m_activation == ReLU ? ESPDL_ACT_RELU : ESPDL_ACT_LINEAR;
-        d.round_mode = context->round_mode;
-        st = spread ? espdl_b200_conv2d_ws(&d, nullptr, 0, context->stream)
-                    : espdl_b200_conv2d_ws(&d, context->workspace, context->workspace_bytes, context->stream);
+        fill_desc(context, &d, in0->device, filter, out->device, (int)count, M, K, N, none1 ? 0 : K * N);
+        st = espdl_b200_conv2d_ws(&d, scratch, scratch_bytes, context->stream);
         count = 0; // nothing left for the per-slice loop
     }
     for (long long s = 0; s < count && !st; s++) {
@@ -718,18 +733,10 @@ void MatMul::forward(ModelContext *context, runtime_mode_t mode)
             m0 *= b0[i];
             m1 *= b1[i];
         }
-        espdl_conv_desc d;
-        memset(&d, 0, sizeof(d));
-        d.input = (const char *)in0->device + (size_t)i0 * M * K * es;
-        d.filter = (const char *)in1->device + (size_t)i1 * K * N * es; // read as [N][K], as the reference's conv kernel does
-        d.output = (char *)out->device + (size_t)s * M * N * es;
-        d.dtype = quant_dtype(quant_type);
-        d.n = 1, d.in_h = d.out_h = 1, d.in_w = d.out_w = M, d.in_c = K, d.out_c = N, d.kh = d.kw = 1;
-        d.stride_h = d.stride_w = d.dilation_h = d.dilation_w = 1, d.group = 1;
-        d.in_exponent = in0->exponent, d.out_exponent = out->exponent, d.filter_exponent = in1->exponent, d.per_channel = 0;
-        d.activation = m_activation == ReLU ? ESPDL_ACT_RELU : ESPDL_ACT_LINEAR;
-        d.round_mode = context->round_mode;
-        st = espdl_b200_conv2d_ws(&d, context->workspace, context->workspace_bytes, context->stream);
+        espdl_conv_desc d; // the filter is read as [N][K], as the reference's conv kernel does
+        fill_desc(context, &d, (const char *)in0->device + (size_t)i0 * M * K * es, (const char *)in1->device + (size_t)i1 * K * N * es,
+                  (char *)out->device + (size_t)s * M * N * es, 1, M, K, N, 0);
+        st = espdl_b200_conv2d_ws(&d, scratch, scratch_bytes, context->stream);
     }
     if (!constant)
         espdl_b200_model_scope(1);

@@ -136,7 +136,9 @@ public:
 
 protected:
     activation_type_t m_activation;
+    size_t m_scratch = 0; ///< what workspace_bytes() declared
     bool slices(ModelContext *context, std::vector<int> &b0, std::vector<int> &b1, int &M, int &K, int &N);
+    void fill_desc(ModelContext *context, void *desc, const void *input, const void *filter, void *output, int n, int M, int K, int N, int image_stride);
 };
 
 /// Add / Sub / Mul with numpy broadcasting, reference: dl_module_add.hpp:14-105, dl_module_mul.hpp, dl_module_sub.hpp.

@@ -131,3 +131,32 @@ def test_layer_norm_rows_side_by_side(rows, n, dt):
             for k in ("y", "mean", "inv"):
                 if a[k] is not None:
                     np.testing.assert_array_equal(dev.download(ptrs[k], want[k]), want[k], err_msg=k)
+
+
+def products_model(tmp_path, pairs, rng):
+    """A model of parallel MatMuls by constants (test_recorded_plans.matmul_graph) run twice on fresh inputs, against the oracle."""
+    import checkers
+    import graph_oracle
+    import test_recorded_plans
+    from espdl_b200 import model
+    g = test_recorded_plans.matmul_graph(pairs)
+    path = str(tmp_path / "m.espdl")
+    g.save(path)
+    m = model.Model(path)
+    weights = {name: arr for name, arr, _ in g.initializers}
+    ins, outs = {t.name: t for t in m.inputs}, {t.name: t for t in m.outputs}
+    for _ in range(2):
+        for t in ins.values():
+            t.array[...] = rng.integers(-60, 60, size=t.shape, dtype=t.array.dtype)
+        m.run()
+        for i, (sa, sb, qt) in enumerate(pairs):
+            want = graph_oracle.matmul(checkers.oracle(), ins[f"a{i}"].array, weights[f"b{i}"], -5, -6, -3, abi.DTYPE_INT8 if qt == "S8" else abi.DTYPE_INT16,
+                                       abi.ACT_LINEAR, abi.ROUND_HALF_UP)
+            np.testing.assert_array_equal(np.asarray(outs[f"y{i}"].array).reshape(want.shape), want, err_msg=f"product {i}")
+    m.close()
+
+
+def test_parallel_products_that_share_the_scratch(tmp_path):
+    """int8 products that pack their operands, in branches beside one another and an int16 one that splits its own."""
+    products_model(tmp_path, [((4096, 100), (100, 512), "S8"), ((512, 128), (128, 64), "S16"), ((3000, 60), (60, 512), "S8"), ((4096, 100), (100, 512), "S8")],
+                   np.random.default_rng(8))

@@ -1,0 +1,127 @@
+"""What a model's plan hands to the device: the launches, their scratch and the order the captured streams keep them in, recorded by a
+stand-in for the CUDA library (fake_device.c) in a process of its own.  No GPU."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from espdl_b200 import abi, espdl_file, model
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+CHILD = r"""
+import ctypes as C, sys
+host = C.CDLL(sys.argv[1])
+host.espdl_model_create.restype = C.c_void_p
+host.espdl_model_create.argtypes = [C.c_char_p, C.c_int, C.c_int]
+for f in ("run", "destroy"):
+    getattr(host, "espdl_model_" + f).argtypes = [C.c_void_p]
+host.espdl_model_run_device.argtypes = [C.c_void_p, C.c_int]
+host.espdl_model_arena_bytes.argtypes = [C.c_void_p]
+host.espdl_model_arena_bytes.restype = C.c_size_t
+h = host.espdl_model_create(sys.argv[2].encode(), int(sys.argv[3]), 0)
+if not h:
+    print("status none")
+    sys.exit()
+print("arena", host.espdl_model_arena_bytes(h))
+for what in sys.argv[4].split(","):
+    print(what, host.espdl_model_run(h) if what == "run" else host.espdl_model_run_device(h, 1))
+host.espdl_model_destroy(h)
+"""
+
+
+@pytest.fixture(scope="session")
+def fake(tmp_path_factory):
+    """The host library beside a fake device library (it finds its device library through $ORIGIN)."""
+    d = tmp_path_factory.mktemp("fake")
+    host = d / os.path.basename(model.HOST_LIB_PATH)
+    host.write_bytes(open(model.HOST_LIB_PATH, "rb").read())
+    src = open(os.path.join(HERE, "fake_device.c")).read()
+    names = subprocess.run(["nm", "-D", "--undefined-only", str(host)], capture_output=True, text=True, check=True).stdout.split()
+    stubs = [n for n in names if n.startswith("espdl_b200_") and n + "(" not in src]
+    (d / "fake.c").write_text(src + "".join(f'int {n}_stub(const void *d, void *s) __asm__("{n}");\n'
+                                            f'int {n}_stub(const void *d, void *s) {{ line("{n[11:]} stream=%p scope=%d", s, scope); return 0; }}\n' for n in stubs))
+    subprocess.check_call(["gcc", "-O1", "-shared", "-fPIC", "-Wno-unused-parameter", "-I" + os.path.join(ROOT, "include"), str(d / "fake.c"), "-o", str(d / "libespdl_b200.so"), "-ldl"])
+    return str(host)
+
+
+def record(fake, tmp_path, graph, calls="run", batch=0, **env):
+    """[(call, {argument: value})] and the child's printed lines."""
+    path, log = str(tmp_path / "g.espdl"), str(tmp_path / "log.txt")
+    if isinstance(graph, str):
+        path = graph
+    else:
+        graph.save(path)
+    r = subprocess.run([sys.executable, "-c", CHILD, fake, path, str(batch), calls], capture_output=True, text=True,
+                       env=dict(os.environ, FAKE_DEVICE_LOG=log, REAL_DEVICE_LIB=abi.LIB_PATH, **env))
+    assert r.returncode == 0, r.stderr
+    lines = []
+    for text in open(log).read().splitlines():
+        name, *args = text.split()
+        lines.append((name, dict(a.split("=") for a in args)))
+    return lines, dict(t.split() for t in r.stdout.splitlines())
+
+
+def captured(lines):
+    """The calls between the first graph_begin and its graph_end."""
+    names = [n for n, _ in lines]
+    return lines[names.index("graph_begin") + 1:names.index("graph_end")]
+
+
+def before(lines):
+    """happens[j] = the captured calls that are done when call j starts: earlier ones of its stream and what its stream waited for."""
+    done_of_stream, done_of_event, out = {}, {}, []
+    for j, (name, a) in enumerate(lines):
+        done = done_of_stream.setdefault(a.get("stream"), set())
+        if name == "record":
+            done_of_event[a["event"]] = set(done)
+        elif name == "wait":
+            done |= done_of_event[a["event"]]
+        out.append(set(done))
+        done.add(j)
+    return out
+
+
+def matmul_graph(pairs, second="constant"):
+    """Parallel MatMuls: pairs = [(shape a, shape b, type)]; `second` operands are parameters or graph inputs."""
+    rng = np.random.default_rng(5)
+    g = espdl_file.GraphBuilder("products", metadata={"target": "c"})
+    for i, (sa, sb, qt) in enumerate(pairs):
+        t = np.int8 if qt == "S8" else np.int16
+        g.add_input(f"a{i}", t, list(sa), -5)
+        if second == "constant":
+            g.add_initializer(f"b{i}", rng.integers(-60, 60, size=sb, dtype=t), [-6])
+        else:
+            g.add_input(f"b{i}", t, list(sb), -6)
+        g.add_node("MatMul", f"mm{i}", [f"a{i}", f"b{i}"], [f"y{i}"], quant_type=qt, activation="Linear")
+        lead = [max(x, y) for x, y in zip(sa[:-2], ([1] * (len(sa) - len(sb)) + list(sb))[:-2])]
+        g.add_output(f"y{i}", t, lead + [sa[-2], sb[-1]], -3)
+    return g
+
+
+PACKED, PLAIN, WIDE = ((4096, 100), (100, 512), "S8"), ((256, 64), (64, 64), "S8"), ((512, 128), (128, 64), "S16")
+
+
+def test_int8_products_that_pack_operands_are_ordered_by_their_scratch(fake, tmp_path):
+    """Products whose reduction is no multiple of 16 pack their operands into the scratch: a step that uses it declares it, so that
+    two of them in different branches never pack at the same time."""
+    lines, _ = record(fake, tmp_path, matmul_graph([PACKED, WIDE, PACKED, PLAIN, PACKED]))
+    caught = captured(lines)
+    ordered = before(caught)
+    users = [j for j, (n, a) in enumerate(caught) if n == "conv" and int(a["need"])]
+    assert len(users) == 4
+    for j in users:
+        assert int(caught[j][1]["ws_bytes"]) >= int(caught[j][1]["need"]), "the plan has scratch for it"
+    for i, a in enumerate(users):
+        for b in users[i + 1:]:
+            assert a in ordered[b], "two steps that write the scratch run side by side"
+
+
+def test_products_without_scratch_of_their_own_get_none(fake, tmp_path):
+    """Whether a product packs its operands does not depend on what other steps made the plan allocate."""
+    lines, _ = record(fake, tmp_path, matmul_graph([WIDE, PLAIN, ((64, 30), (30, 17), "S8")]))
+    small = [a for n, a in captured(lines) if n == "conv" and not int(a["need"])]
+    assert len(small) == 2 and all(int(a["ws_bytes"]) == 0 for a in small)
