@@ -467,8 +467,16 @@ void Conv::forward(ModelContext *context, runtime_mode_t mode)
     (void)mode;
     espdl_conv_desc d;
     int st = fill_desc(context, &d);
-    if (st == ESPDL_OK)
+    if (st == ESPDL_OK) {
+        // a filter or bias that is another step's output is not read ahead of it
+        bool constant = true;
+        for (size_t i = 1; i < m_inputs_index.size() - (m_residual ? 1 : 0); i++) constant = constant && context->get_tensor(m_inputs_index[i])->device_owned;
+        if (!constant)
+            espdl_b200_model_scope(0);
         st = espdl_b200_conv2d_ws(&d, context->workspace, context->workspace_bytes, context->stream);
+        if (!constant)
+            espdl_b200_model_scope(1);
+    }
     if (st)
         ESP_LOGE("Conv", "%s failed: %s %s", name ? name : "?", espdl_b200_strerror(st), espdl_b200_last_error());
     context->note(st);
@@ -698,11 +706,12 @@ void MatMul::forward(ModelContext *context, runtime_mode_t mode)
         full1 = full1 && b1[i] == ob[i];
         none1 = none1 && b1[i] == 1;
     }
-    const bool constant = in1->device_owned; // else the previous steps of the plan write it: nothing of it is read ahead of them
-    if (!constant)
-        espdl_b200_model_scope(0);
     const void *filter = in1->device;
     const size_t spread = spread_bytes(b0, b1, (size_t)K * N * es);
+    // written by the previous steps of the plan, or by the copy below, it is not read ahead of them
+    const bool constant = in1->device_owned && !spread;
+    if (!constant)
+        espdl_b200_model_scope(0);
     if (spread && spread <= context->workspace_bytes && (long long)K * N <= 0x7fffffffll) {
         std::vector<int> shape(ob);
         std::vector<long long> from(ob.size() + 1, 1), to(ob.size() + 1, 1);

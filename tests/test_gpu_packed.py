@@ -160,3 +160,9 @@ def test_parallel_products_that_share_the_scratch(tmp_path):
     """int8 products that pack their operands, in branches beside one another and an int16 one that splits its own."""
     products_model(tmp_path, [((4096, 100), (100, 512), "S8"), ((512, 128), (128, 64), "S16"), ((3000, 60), (60, 512), "S8"), ((4096, 100), (100, 512), "S8")],
                    np.random.default_rng(8))
+
+
+def test_constants_that_repeat_over_slices_one_behind_the_other(tmp_path):
+    """Each repeats its constant into the same scratch and multiplies by it from there."""
+    products_model(tmp_path, [((3, 2, 64, 32), (1, 2, 32, 48), "S8"), ((5, 2, 33, 32), (1, 2, 32, 48), "S8"), ((4, 3, 9, 12), (1, 3, 12, 20), "S8")],
+                   np.random.default_rng(9))

@@ -125,3 +125,29 @@ def test_products_without_scratch_of_their_own_get_none(fake, tmp_path):
     lines, _ = record(fake, tmp_path, matmul_graph([WIDE, PLAIN, ((64, 30), (30, 17), "S8")]))
     small = [a for n, a in captured(lines) if n == "conv" and not int(a["need"])]
     assert len(small) == 2 and all(int(a["ws_bytes"]) == 0 for a in small)
+
+
+def test_only_constants_are_read_ahead_of_the_previous_kernel(fake, tmp_path):
+    """Inside a plan's scope kernels read their filter before the launches in front of them are done.  A filter that one of these
+    writes - a constant repeated into the scratch, or another step's output - is launched outside of it; a constant inside."""
+    repeated = ((3, 2, 64, 32), (1, 2, 32, 48), "S8")
+    lines, _ = record(fake, tmp_path, matmul_graph([repeated, PLAIN]))
+    caught = captured(lines)
+    copies = {a["dst"] for n, a in caught if n == "copy"}
+    scope = {(a["filter"] in copies): int(a["scope"]) for n, a in caught if n == "conv"}
+    assert scope == {True: 0, False: 1}
+    lines, _ = record(fake, tmp_path, matmul_graph([PLAIN], second="input"))
+    assert [int(a["scope"]) for n, a in captured(lines) if n == "conv"] == [0]
+
+
+def test_a_conv_whose_filter_another_step_writes(fake, tmp_path):
+    g = espdl_file.GraphBuilder("dynamic", metadata={"target": "c"})
+    g.add_input("x", np.int8, [1, 12, 12, 16], -5)
+    g.add_input("f", np.int8, [1, 1, 16, 24], -6)
+    g.add_initializer("w", np.ones((1, 1, 24, 16), dtype=np.int8), [-6])
+    g.add_node("Conv", "c0", ["x", "f"], ["y"], quant_type="S8", activation="Linear", pads=[0, 0, 0, 0], strides=[1, 1], dilations=[1, 1], group=1)
+    g.add_value_info("y", np.int8, [1, 12, 12, 24], -5)
+    g.add_node("Conv", "c1", ["y", "w"], ["z"], quant_type="S8", activation="Linear", pads=[0, 0, 0, 0], strides=[1, 1], dilations=[1, 1], group=1)
+    g.add_output("z", np.int8, [1, 12, 12, 16], -5)
+    lines, _ = record(fake, tmp_path, g)
+    assert [int(a["scope"]) for n, a in captured(lines) if n == "conv"] == [0, 1]
