@@ -501,6 +501,34 @@ static bool runs_packed(const espdl_conv_desc &d)
         !conv2d_tc_supported(d) && conv2d_packed_supported(d);
 }
 
+// Image i of a batch of products.
+static espdl_conv_desc product_of_image(const espdl_conv_desc &d, int i)
+{
+    const size_t es = d.dtype == ESPDL_DTYPE_INT16 ? 2 : 1;
+    const long long ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c, ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
+    espdl_conv_desc one = d;
+    one.n = 1, one.filter_image_stride = 0;
+    one.input = (const char *)d.input + (size_t)i * d.in_h * d.in_w * ips * es;
+    one.filter = (const char *)d.filter + (size_t)i * d.filter_image_stride * es;
+    one.output = (char *)d.output + (size_t)i * d.out_h * d.out_w * ops * es;
+    return one;
+}
+
+// Scratch of a batch of int16 products that runs one after the other on the tile kernel, 0 where one launch of the CUDA cores over all
+// of them is as fast.  A slice takes the packing's and the tile kernel's start, 6.3 to 9.1 us, the CUDA cores 0.62 to 0.86 M
+// multiply-adds a us, 0.27 M where 32 threads read filter rows a multiple of 64 bytes apart.  One by one against together, us: 8 slices of
+// 512x512x512 72 / 3927, 2 of 256x64x256 15 / 17, 64 of 400x32x400 469 / 1199; 64 of 128x64x128 482 / 249, of 400x400x32 576 / 383.
+static size_t one_by_one_bytes(const espdl_conv_desc &d)
+{
+    if (d.kernel != ESPDL_KERNEL_AUTO || d.dtype != ESPDL_DTYPE_INT16 || d.filter_image_stride <= 0 || d.n < 1)
+        return 0;
+    const espdl_conv_desc one = product_of_image(d, 0);
+    const double macs = (double)d.out_h * d.out_w * d.in_c * d.out_c;
+    if (4 + d.n * macs / (d.in_c % 32 == 0 && d.out_c >= 128 ? 0.27e6 : 0.7e6) < d.n * (8.5 + macs / 2e8))
+        return 0;
+    return conv2d_tc_supported(one) ? conv2d_tc_workspace_bytes(one) : (conv2d_packed_supported(one) ? conv2d_packed_workspace_bytes(one) : 0);
+}
+
 extern "C" {
 
 int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes)
@@ -513,7 +541,9 @@ int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes
         return st;
     if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1 || runs_narrow(*desc) || runs_mma(*desc))
         return ESPDL_OK;
-    if (conv2d_tc_supported(*desc))
+    if (desc->filter_image_stride != 0 && !conv2d_tc_supported(*desc))
+        *bytes = one_by_one_bytes(*desc);
+    else if (conv2d_tc_supported(*desc))
         *bytes = conv2d_tc_workspace_bytes(*desc);
     else if (runs_packed(*desc))
         *bytes = conv2d_packed_workspace_bytes(*desc);
@@ -563,6 +593,14 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
             return conv2d_tc(*desc, workspace, workspace_bytes, s);
         if (desc->kernel == ESPDL_KERNEL_TCGEN05)
             return ESPDL_ERR_UNSUPPORTED;
+        const size_t one_by_one = one_by_one_bytes(*desc);
+        if (one_by_one && workspace && workspace_bytes >= one_by_one) {
+            for (int i = 0; i < desc->n && !st; i++) {
+                const espdl_conv_desc one = product_of_image(*desc, i);
+                st = conv2d_tc_supported(one) ? conv2d_tc(one, workspace, workspace_bytes, s) : conv2d_packed(one, workspace, workspace_bytes, s);
+            }
+            return st;
+        }
         return conv2d_simt(*desc, s); // all products in one launch (one per image: 128 launches, 1.5 ms, for the attention of 64 images)
     }
     if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_band_tc_supported(*desc))

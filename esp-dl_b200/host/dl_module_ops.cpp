@@ -659,8 +659,9 @@ size_t MatMul::workspace_bytes(ModelContext *context)
         if (espdl_b200_conv2d_workspace_bytes(&d, &bytes) == ESPDL_OK)
             m_scratch = std::max(m_scratch, bytes);
     };
-    if (spread) {
-        m_scratch = spread;
+    if (spread && (long long)K * N <= 0x7fffffffll) { // the repeated operand, behind it what its product takes
+        need(0, (int)count, K * N);
+        m_scratch += (spread + 255) / 256 * 256;
     } else if (count > 1 && full0 && (full1 || none1) && count <= 0x7fffffffll && (long long)K * N <= 0x7fffffffll) {
         need(0, (int)count, none1 ? 0 : K * N);
     } else { // slices may start at different alignments: as many as there are within 16 bytes
@@ -724,8 +725,9 @@ void MatMul::forward(ModelContext *context, runtime_mode_t mode)
         st = enqueue_copy(context, in1->device, context->workspace, (int)es, shape, from, to);
         filter = context->workspace, full1 = true;
     }
-    void *scratch = m_scratch && !spread ? context->workspace : nullptr;
-    const size_t scratch_bytes = scratch ? context->workspace_bytes : 0;
+    const size_t taken = filter == in1->device ? 0 : (spread + 255) / 256 * 256;
+    void *scratch = m_scratch > taken ? (char *)context->workspace + taken : nullptr;
+    const size_t scratch_bytes = scratch ? context->workspace_bytes - taken : 0;
     if (!st && count > 1 && full0 && (full1 || none1) && count <= 0x7fffffffll && (long long)K * N <= 0x7fffffffll) {
         espdl_conv_desc d;
         fill_desc(context, &d, in0->device, filter, out->device, (int)count, M, K, N, none1 ? 0 : K * N);

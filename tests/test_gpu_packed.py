@@ -166,3 +166,35 @@ def test_constants_that_repeat_over_slices_one_behind_the_other(tmp_path):
     """Each repeats its constant into the same scratch and multiplies by it from there."""
     products_model(tmp_path, [((3, 2, 64, 32), (1, 2, 32, 48), "S8"), ((5, 2, 33, 32), (1, 2, 32, 48), "S8"), ((4, 3, 9, 12), (1, 3, 12, 20), "S8")],
                    np.random.default_rng(9))
+
+
+@pytest.mark.parametrize("n,m,k,cout", [(2, 256, 64, 256), (8, 300, 512, 129), (3, 200, 100, 300), (64, 16, 48, 24)])
+def test_batch_of_int16_products_with_the_scratch_it_asks_for(n, m, k, cout):
+    """Large slices run one by one on the tile kernel out of the scratch that the query names, small ones together; without the scratch
+    every batch runs on the CUDA cores."""
+    import ctypes as C
+    rng = np.random.default_rng(k)
+    whole = cases.conv_case(seed=1, n=n, h=1, w=m, cin=k, cout=cout, kh=1, kw=1, pad=(0, 0, 0, 0), bias=False, **dict(S16, e_out=-14))
+    whole.update(x=rng.integers(-32768, 32768, size=(n, 1, m, k), dtype=np.int16), w=rng.integers(-32768, 32768, size=(n, cout, 1, 1, k), dtype=np.int16),
+                 filter_image_stride=cout * k)
+    want = np.zeros_like(whole["out"])
+    for i in range(n):
+        one = cases.conv_case(seed=1, n=1, h=1, w=m, cin=k, cout=cout, kh=1, kw=1, pad=(0, 0, 0, 0), bias=False, **dict(S16, e_out=-14))
+        one.update(x=whole["x"][i:i + 1], w=whole["w"][i], filter_exponent=whole["filter_exponent"])
+        want[i:i + 1] = gpu_util.run_conv_oracle(one)
+    with gpu_util.DeviceBuffers() as dev:
+        out = dev.upload(whole["out"])
+        d = cases.conv_desc(whole, dict(input=dev.upload(whole["x"]), filter=dev.upload(whole["w"]), output=out))
+        need = C.c_size_t(0)
+        abi.check(dev.lib.espdl_b200_conv2d_workspace_bytes(C.byref(d), C.byref(need)), "workspace")
+        assert (need.value > 0) == (n < 64)
+        for size in {need.value, 0}:
+            scratch = dev.upload(np.zeros(max(size, 1), dtype=np.uint8))
+            abi.check(dev.lib.espdl_b200_conv2d_ws(C.byref(d), scratch if size else None, size, None), "conv2d_ws")
+            np.testing.assert_array_equal(dev.download(out, want), want)
+
+
+@pytest.mark.parametrize("pairs", [[((4, 3, 260, 64), (4, 3, 64, 256), "S16")], [((4, 3, 260, 64), (1, 3, 64, 256), "S16"), ((3, 2, 9, 12), (1, 2, 12, 5), "S16")]])
+def test_matmul_of_int16_slices(pairs, tmp_path):
+    """Slices of one matrix each, and second operands that repeat over some of them, on the tile kernel and on the CUDA cores."""
+    products_model(tmp_path, pairs, np.random.default_rng(10))

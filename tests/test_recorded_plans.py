@@ -151,3 +151,16 @@ def test_a_conv_whose_filter_another_step_writes(fake, tmp_path):
     g.add_output("z", np.int8, [1, 12, 12, 16], -5)
     lines, _ = record(fake, tmp_path, g)
     assert [int(a["scope"]) for n, a in captured(lines) if n == "conv"] == [0, 1]
+
+
+def test_int16_slices_have_the_scratch_of_the_tile_kernel(fake, tmp_path):
+    """Batches of large int16 products run slice by slice on the tile kernel, which needs scratch for one: their own operand each, or one
+    that repeats over some slices (then behind the repeated operand)."""
+    lines, _ = record(fake, tmp_path, matmul_graph([((4, 3, 260, 64), (4, 3, 64, 256), "S16"), ((4, 3, 260, 64), (1, 3, 64, 256), "S16")]))
+    convs = [a for n, a in captured(lines) if n == "conv"]
+    spread = {int(a["dst"], 16) for n, a in captured(lines) if n == "copy"}
+    assert len(convs) == 2 and len(spread) == 1
+    for a in convs:
+        assert int(a["need"]) and int(a["ws_bytes"]) >= int(a["need"])
+        if int(a["filter"], 16) in spread:
+            assert int(a["ws"], 16) >= int(a["filter"], 16) + 12 * 64 * 256 * 2
