@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(32 * MMA_WARPS) conv_mma_kernel(const __grid_c
     constexpr int QUADS = COLS / 4;
     const int e_lane = kpart * 32 + lane, cq = e_lane % QUADS, oc0 = tn * COLS + 4 * cq;
     int bias_half[4], shift[4];
-    bool fast = true;
+    bool fast = p.K <= 65536; // 2^14 a term: beyond that the sum alone may reach 2^31 and the rounding's half leave 32 bits
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int n = min(oc0 + i, p.N - 1);

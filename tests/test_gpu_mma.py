@@ -80,3 +80,18 @@ def test_narrow_windows(kw, act, lut, round_mode, monkeypatch):
     want = gpu_util.run_conv_oracle(case)
     assert want.std() > 0
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+
+
+@pytest.mark.parametrize("act", [abi.ACT_RELU, abi.ACT_LINEAR])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_reductions_beyond_65536_terms(sign, act, forced):
+    """73500 terms at the ends of int8 reach 1.2e9; with this bias the sum is 101 below (above) the end of int32, and only the rounding's
+    half takes it across."""
+    case = cases.conv_case(seed=1, n=1, h=8, w=8, cin=1500, cout=9, kh=7, kw=7, pad=(0, 0, 0, 0), per_channel=True, act=act, e_in=0, e_out=0, e_w=(-15, -15))
+    case["x"][...], case["w"][...] = -128, -128 if sign > 0 else 127
+    acc = 7 * 7 * 1500 * 128 * (128 if sign > 0 else -127)
+    case["b"][...] = sign * (2 ** 31 - 101) - acc
+    case["b"][1::3] = 5  # others take the one-add form
+    want = gpu_util.run_conv_oracle(case)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+    assert want.max() == (127 if sign > 0 else 0 if act == abi.ACT_RELU else -128)
