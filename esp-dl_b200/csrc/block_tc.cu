@@ -135,7 +135,7 @@ __device__ __noinline__ void bk_band_general(const BlockParams &p, uint32_t hid,
                         acc += v * (int)p.dw_w[(ky * 3 + kx) * p.chid + c];
                     }
                 const int e = p.edw.per_channel ? p.edw.ew[c] : p.edw.ew_scalar;
-                const int shift = max(-31, min(31, p.edw.e_shift_base - e));
+                const int shift = max(-31, min(32, p.edw.e_shift_base - e));
                 const int q = min(requant8(acc, p.edw.bias ? ((const int32_t *)p.edw.bias)[c] : 0, shift, p.edw.relu, p.edw.half_even), p.clipdw);
                 wd |= ((uint32_t)q & 0xffu) << (8 * i);
             }

@@ -140,9 +140,11 @@ int conv2d_band_tc(const espdl_conv_desc &d, cudaStream_t s);
 //   shift > 0 : HALF_UP   floor((v + 2^(s-1)) / 2^s)  ==  (v >> s) + bit (s-1) of v
 //               HALF_EVEN floor, +1 if remainder > half or (== half and quotient odd)
 //   shift <= 0: (int64)v << -shift, saturated to int32
-// Callers guarantee |shift| <= 31.
+// Callers guarantee shift >= -31.
 __device__ __forceinline__ int32_t shift_round32(int32_t v, int shift, int half_even)
 {
+    if (shift > 31)
+        return 0; // |v| is at most 2^31, half a step of 2^32, and that tie goes to 0 either way
     if (shift > 0) {
         int32_t q = v >> shift;
         if (!half_even) {

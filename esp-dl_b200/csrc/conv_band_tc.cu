@@ -298,7 +298,7 @@ band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__
                     for (int i = 0; i < 16; i++) {
                         const int c = (c0 + i) % p.cout;
                         const int e = p.epi.per_channel ? __ldg(p.epi.ew + c) : p.epi.ew_scalar;
-                        const int shift = max(-31, min(31, p.epi.e_shift_base - e));
+                        const int shift = max(-31, min(32, p.epi.e_shift_base - e));
                         int32_t r = requant8(v[i], p.epi.bias ? __ldg((const int32_t *)p.epi.bias + c) : 0, shift, p.epi.relu, p.epi.half_even);
                         if (p.epi.lut)
                             r = p.epi.lut[(long long)c * p.epi.lut_stride + ((uint8_t)r ^ 0x80u)];

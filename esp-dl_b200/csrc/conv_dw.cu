@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(256) dw_s8_vec16_kernel(DwParams p)
             for (int i = 0; i < 4; i++) {
                 const int c = ch + q * 4 + i;
                 const int e = p.per_channel ? __ldg(p.ew + c) : p.ew_scalar;
-                const int shift = max(-31, min(31, p.e_shift_base - e));
+                const int shift = max(-31, min(32, p.e_shift_base - e));
                 int32_t v = requant8(acc[q * 4 + i], bias ? __ldg(bias + c) : 0, shift, p.relu, p.half_even);
                 if (p.lut)
                     v = p.lut[(long long)c * p.lut_stride + ((uint8_t)v ^ 0x80u)];
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256) dwk_dp4a_kernel(DwParams p)
         for (int i = 0; i < 4; i++) {
             const int c = (int)c4 * 4 + i;
             const int e = p.per_channel ? __ldg(p.ew + c) : p.ew_scalar;
-            const int shift = max(-31, min(31, p.e_shift_base - e));
+            const int shift = max(-31, min(32, p.e_shift_base - e));
             int32_t v = requant8(acc[i], p.bias ? __ldg((const int32_t *)p.bias + c) : 0, shift, p.relu, p.half_even);
             if (p.lut)
                 v = p.lut[(long long)c * p.lut_stride + ((uint8_t)v ^ 0x80u)];
@@ -220,7 +220,7 @@ __device__ __noinline__ void dw3x3_band_general(const DwParams &p, int S, int n,
                             acc += (int)in[((long long)iy * p.iw + ix) * p.ips + c] * (int)((const int8_t *)p.w)[(ky * 3 + kx) * p.c + c];
                     }
                 const int e = p.per_channel ? p.ew[c] : p.ew_scalar;
-                const int shift = max(-31, min(31, p.e_shift_base - e));
+                const int shift = max(-31, min(32, p.e_shift_base - e));
                 int32_t v = requant8(acc, p.bias ? ((const int32_t *)p.bias)[c] : 0, shift, p.relu, p.half_even);
                 if (p.lut)
                     v = p.lut[(long long)c * p.lut_stride + ((uint8_t)v ^ 0x80u)];
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(256) dw_generic_kernel(DwParams p)
         }
         const int e = p.per_channel ? p.ew[c] : p.ew_scalar;
         if (sizeof(T) == 1) {
-            const int shift = max(-31, min(31, p.e_shift_base - e));
+            const int shift = max(-31, min(32, p.e_shift_base - e));
             int32_t v = requant8((int32_t)acc, bias ? (int32_t)bias[c] : 0, shift, p.relu, p.half_even);
             if (p.lut)
                 v = p.lut[(long long)c * p.lut_stride + ((uint8_t)v ^ 0x80u)];

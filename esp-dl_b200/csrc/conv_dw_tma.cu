@@ -81,7 +81,7 @@ __device__ __noinline__ void dwt_walk_general(const DwtParams &pp, int S, const 
                     for (int kx = 0; kx < 3; kx++)
                         acc += (int)ip[(ro * S + ky) * in_row_bytes + (x * S + kx) * pp.CB + i] * (int)p.w[(ky * 3 + kx) * p.C + c0 + i];
                 const int e = p.per_channel ? p.ew[c0 + i] : p.ew_scalar;
-                const int shift = max(-31, min(31, p.e_shift_base - e));
+                const int shift = max(-31, min(32, p.e_shift_base - e));
                 int32_t v = requant8(acc, p.bias ? p.bias[c0 + i] : 0, shift, p.relu, p.half_even);
                 if (p.lut)
                     v = p.lut[(long long)(c0 + i) * p.lut_stride + ((uint8_t)v ^ 0x80u)];

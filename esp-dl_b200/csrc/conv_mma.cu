@@ -64,7 +64,7 @@ __device__ __noinline__ uint32_t general_word(const MmaParams &p, const int (&v)
     uint32_t word = 0;
     for (int i = 0; i < 4; i++) {
         const int n = min(oc0 + i, p.N - 1);
-        const int shift = max(-31, min(31, p.e_shift_base - (p.per_channel ? __ldg(p.ew + n) : p.ew_scalar)));
+        const int shift = max(-31, min(32, p.e_shift_base - (p.per_channel ? __ldg(p.ew + n) : p.ew_scalar)));
         word |= ((uint32_t)requant8(v[i], p.bias ? __ldg(p.bias + n) : 0, shift, p.relu, p.half_even) & 0xffu) << (8 * i);
     }
     return word;

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
             const int oc = oc0 + j;
             if (live && oc < p.oc && (!SPLIT || sub == j % lanes)) {
                 const int e = p.per_channel ? p.ew[oc] : p.ew_scalar;
-                const int shift = max(-31, min(31, p.e_shift_base - e));
+                const int shift = max(-31, min(32, p.e_shift_base - e));
                 int32_t q = requant8(acc[j], bias ? bias[oc] : 0, shift, p.relu, p.half_even);
                 if (p.lut)
                     q = p.lut[(long long)oc * p.lut_stride + ((uint8_t)q ^ 0x80u)];
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) conv_s8_small_k_kernel(ConvParams p)
     for (int oc = threadIdx.x; oc < p.oc; oc += blockDim.x) {
         bias_s[oc] = p.bias ? ((const int32_t *)p.bias)[oc] : 0;
         const int e = p.per_channel ? p.ew[oc] : p.ew_scalar;
-        shift_s[oc] = max(-31, min(31, p.e_shift_base - e));
+        shift_s[oc] = max(-31, min(32, p.e_shift_base - e));
     }
     __syncthreads();
     const long long pixels = (long long)p.n * p.oh * p.ow;
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(256) conv_s8_narrow_kernel(ConvParams p, int e
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int oc = min(oc0 + j, p.oc - 1);
-            const int shift = max(-31, min(31, p.e_shift_base - (p.per_channel ? __ldg(p.ew + oc) : p.ew_scalar)));
+            const int shift = max(-31, min(32, p.e_shift_base - (p.per_channel ? __ldg(p.ew + oc) : p.ew_scalar)));
             int q = requant8(acc[j], p.bias ? __ldg((const int32_t *)p.bias + oc) : 0, shift, p.relu, p.half_even);
             if (p.lut)
                 q = p.lut[(long long)oc * p.lut_stride + ((uint8_t)q ^ 0x80u)];

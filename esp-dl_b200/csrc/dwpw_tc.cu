@@ -317,7 +317,7 @@ dwpw_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ 
                                         for (int kx = 0; kx < 3; kx++)
                                             acc += (int)ip[((ro * S + ky) * p.IW + (x * S + kx)) * CB + i] * (int)p.dw.w[(ky * 3 + kx) * p.dw.C + c];
                                     const int e = p.dw.per_channel ? p.dw.ew[c] : p.dw.ew_scalar;
-                                    const int shift = max(-31, min(31, p.dw.e_shift_base - e));
+                                    const int shift = max(-31, min(32, p.dw.e_shift_base - e));
                                     const int32_t v = requant8(acc, p.dw.bias ? p.dw.bias[c] : 0, shift, p.dw.relu, p.dw.half_even);
                                     word |= ((uint32_t)v & 0xffu) << (8 * i);
                                 }

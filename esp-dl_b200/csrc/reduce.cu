@@ -76,7 +76,7 @@ __device__ __forceinline__ long long finish_integer(const ReduceParams &p, ACC a
     }
     if (p.op == ESPDL_REDUCE_SUM || p.op == ESPDL_REDUCE_L1 || p.op == ESPDL_REDUCE_SUM_SQUARE) {
         const int shift = max(-62, min(62, p.e_out - (p.op == ESPDL_REDUCE_SUM_SQUARE ? 2 * p.e_in : p.e_in)));
-        return sizeof(ACC) == 4 ? (long long)shift_round32((int32_t)acc, max(-31, min(31, shift)), p.half_even)
+        return sizeof(ACC) == 4 ? (long long)shift_round32((int32_t)acc, max(-31, min(32, shift)), p.half_even)
                                 : shift_round64((long long)acc, shift, p.half_even);
     }
     return (long long)acc;

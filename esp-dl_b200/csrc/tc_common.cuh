@@ -604,7 +604,7 @@ __device__ __forceinline__ void requant16_general(const int32_t *v, const EpiCon
         for (int i = 0; i < 4; i++) {
             const int n = min(n_first + q * 4 + i, N - 1);
             const int e = c.per_channel ? __ldg(c.ew + n) : c.ew_scalar;
-            const int shift = max(-31, min(31, c.e_shift_base - e));
+            const int shift = max(-31, min(32, c.e_shift_base - e));
             const int b = c.bias ? __ldg((const int32_t *)c.bias + n) : 0;
             int32_t r = requant8(v[q * 4 + i], b, shift, c.relu, c.half_even);
             if (c.lut)

@@ -71,6 +71,45 @@ def test_shifts_and_biases_of_dead_channels(name, round_mode):
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
 
 
+# kernel -> (layer, switches, kernel asked for): the kernels that requantise channel by channel, and those that do so for channels outside
+# the one-add form
+GENERAL = {
+    "mma": (dict(n=2, h=6, w=9, cin=48, cout=45, kh=1, kw=1, pad=(0, 0, 0, 0)), {"ESPDL_B200_SMALL_MMA": "always"}, abi.KERNEL_AUTO),
+    "narrow": (dict(n=2, h=15, w=14, cin=16, cout=13, kh=2, kw=2, pad=(0, 1, 0, 1)), {"ESPDL_B200_NARROW": "always"}, abi.KERNEL_AUTO),
+    "dw3": (dict(n=1, h=9, w=11, cin=20, depthwise=True), {}, abi.KERNEL_AUTO),
+    "dw3-tma": (dict(n=2, h=14, w=15, cin=96, depthwise=True), {"ESPDL_B200_DW_TMA_NARROW": "1"}, abi.KERNEL_AUTO),
+    "dw5": (dict(n=1, h=9, w=11, cin=20, kh=5, kw=5, pad=(2, 2, 2, 2), depthwise=True), {}, abi.KERNEL_AUTO),
+    "dw7": (dict(n=1, h=9, w=11, cin=24, kh=7, kw=7, pad=(3, 3, 3, 3), depthwise=True), {}, abi.KERNEL_AUTO),
+    "dw-vec": (dict(n=1, h=9, w=11, cin=32, kh=3, kw=5, pad=(1, 1, 2, 2), depthwise=True), {}, abi.KERNEL_AUTO),
+    "dw-any": (dict(n=1, h=9, w=11, cin=21, kh=3, kw=5, pad=(1, 1, 2, 2), depthwise=True), {}, abi.KERNEL_AUTO),
+    "cores": (dict(n=1, h=7, w=9, cin=20, cout=18), {}, abi.KERNEL_SIMT),
+    "cores-first": (dict(n=1, h=7, w=9, cin=3, cout=18), {}, abi.KERNEL_SIMT),
+    "tile": (dict(n=1, h=1, w=130, cin=64, cout=48, kh=1, kw=1, pad=(0, 0, 0, 0)), {}, abi.KERNEL_TCGEN05),
+    "patch": (dict(n=2, h=11, w=33, cin=64, cout=64), {}, abi.KERNEL_TCGEN05),
+    "band": (dict(n=2, h=12, w=24, cin=8, cout=16), {}, abi.KERNEL_AUTO),
+    "first": (dict(n=2, h=32, w=48, cin=3, cout=16, stride=2), {}, abi.KERNEL_AUTO),
+}
+
+
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("name", list(GENERAL))
+def test_dead_channels_beside_channels_outside_the_fast_form(name, round_mode, monkeypatch):
+    """A shift beyond 31 gives 0 for every 32-bit sum, also in the form that a neighbour with a left shift or a huge bias brings about."""
+    kw, switches, kernel = GENERAL[name]
+    for k, v in switches.items():
+        monkeypatch.setenv(k, v)
+    case = cases.conv_case(seed=len(name), per_channel=True, round_mode=round_mode, act=abi.ACT_LINEAR, e_in=0, e_out=0, e_w=(-12, -7), **kw)
+    rng = np.random.default_rng(7)
+    for c in range(0, case["out_c"], 4):
+        case["ew"][c], case["b"][c] = -int(rng.integers(31, 41)), [2 ** 31 - 1, -2 ** 31, 2 ** 30 + 3, -2 ** 30 - 3][c // 4 % 4]
+        if c + 2 < case["out_c"]:
+            case["ew"][c + 2] = int(rng.integers(0, 3))  # a left shift: outside the one-add form
+    for c in range(0, case["out_c"], 4):
+        if case["ew"][c] == -31:  # within the reach of the sum
+            case["b"][c] //= 2
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=kernel), gpu_util.run_conv_oracle(case))
+
+
 # pixels and channels around what a thread block covers at once, images shared by one, two and eight blocks
 @pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
 @pytest.mark.parametrize("n,h,w,c", [(1, 184, 184, 32), (3, 23, 23, 48), (2, 33, 31, 6), (1, 3, 700, 1), (300, 7, 7, 1280), (2, 16, 16, 520), (1, 2048, 1, 3)])
