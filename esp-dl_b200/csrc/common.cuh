@@ -42,9 +42,9 @@ cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 }
 
 // The kernels that move or rewrite tensors (elementwise operators, pools, copies, reductions ...) start with grid_dep_wait() and
-// take a last argument `early`: whether they let the next kernel's blocks become resident at once.  The conv kernels read
-// their parameters (filter, bias, exponents) before they wait, and a caller of the C ABI may have written those with
-// espdl_b200_copy or the like just before - so `early` only inside a model's plan, whose parameters no launch writes.
+// take a last argument `early`: whether they let the next kernel's blocks become resident at once.  Inside a model's plan, whose
+// parameters no launch writes, the conv kernels read theirs (filter, bias, exponents, table) before they wait; outside of it a caller of
+// the C ABI may have written them just before, with espdl_b200_copy or a kernel of its own: both sides are `early` only inside.
 bool in_model_scope();
 
 template <typename... KArgs, typename... Args>

@@ -39,6 +39,7 @@ constexpr int CV_MAX_ACC = 4;
 constexpr size_t CV_SMEM_BUDGET = 200 * 1024;
 
 struct ConvTcParams {
+    int early; // bias, exponents and table are constants of the model: read ahead of the previous kernel's end
     int n, oh, ow, cin, cout;
     int kh, kw, S, D, pt, pl;
     int P, R;                     // tile: R rows x P columns of output pixels
@@ -198,6 +199,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int lane_group = warp & 3;
         const int row_in_tile = lane_group * 32 + lane;
         const int et = threadIdx.x - 64;
+        if (!p.early)
+            grid_dep_wait(); // bias, exponents and table may be what the previous kernel wrote
         stage_fast_params(p.epi, fast_s, p.cout, n_pad, et, 16 * 32, slow_flag);
         if (p.epi.lut)
             stage_lut(p.epi.lut, lut_s, et, 16 * 32);
@@ -335,7 +338,7 @@ constexpr int PATCH_MAX_STEPS = 16;
 constexpr int PATCH_THREADS = CV_THREADS + 32; // a second MMA warp
 
 struct PatchParams {
-    int early; // the filter is a constant of the model
+    int early; // filter, bias, exponents and table are constants of the model: read ahead of the previous kernel's end
     int n, oh, ow, cin, cout;
     int kh, kw, pt, pl;
     int G, glo;                   // pixels per position; the first position a window reaches, relative to its own (0 or negative)
@@ -518,6 +521,8 @@ conv_patch_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const int lane_group = warp & 3;
         const int row_in_tile = lane_group * 32 + lane;
         const int et = threadIdx.x - 64;
+        if (!p.early)
+            grid_dep_wait(); // bias, exponents and table may be what the previous kernel wrote
         for (int j = 0; j < p.G; j++) stage_fast_params(p.epi, fast_s + j * p.cout, p.cout, p.cout, et, 16 * 32, slow_flag);
         if (p.epi.lut)
             stage_lut(p.epi.lut, lut_s, et, 16 * 32);
@@ -926,6 +931,7 @@ int conv2d_conv_tc(const espdl_conv_desc &d, cudaStream_t s)
     if (!enc)
         return set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled entry point not found");
     const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
+    p.early = in_model_scope();
     p.out = d.output;
     p.ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     p.epi.bias = d.bias, p.epi.ew = d.filter_exponents, p.epi.lut = d.lut, p.epi.lut_stride = d.lut_channel_stride;

@@ -2,6 +2,8 @@
 and replay of the reference's golden Gemm models through the C ABI."""
 import os
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -403,3 +405,45 @@ def test_one_tile_per_block(m, k, n, out_stride, lut):
     want = gpu_util.run_conv_oracle(case)
     assert want.std() > 5
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), want)
+
+
+PARAMETER_SHAPES = {
+    "tile": dict(n=1, h=1, w=300, cin=64, cout=96, kh=1, kw=1, pad=(0, 0, 0, 0)),
+    "one tile": dict(n=1, h=1, w=120, cin=256, cout=64, kh=1, kw=1, pad=(0, 0, 0, 0)),
+    "taps": dict(n=2, h=15, w=15, cin=48, cout=48, stride=2),
+    "patch": dict(n=2, h=11, w=33, cin=64, cout=64),
+    "band": dict(n=2, h=12, w=24, cin=8, cout=16),
+    "first": dict(n=2, h=32, w=48, cin=3, cout=16, stride=2),
+    "depthwise": dict(n=2, h=14, w=15, cin=96, depthwise=True),
+}
+
+
+@pytest.mark.parametrize("small", ["0", "always"])
+@pytest.mark.parametrize("name", list(PARAMETER_SHAPES))
+def test_parameters_written_by_the_launches_in_front(name, small, monkeypatch):
+    """A caller of the C ABI may write filter, bias, exponents and table with launches of the same stream: layer after layer with other
+    parameters each, nothing between them but the copies that bring these."""
+    monkeypatch.setenv("ESPDL_B200_SMALL_MMA", small)
+    lib = gpu_util.lib()
+    sets = [cases.conv_case(seed=s, per_channel=True, lut=name != "depthwise", act=abi.ACT_LINEAR, e_in=-6, e_out=-5, e_w=(-10, -7), **PARAMETER_SHAPES[name]) for s in (1, 2, 3)]
+    want = []
+    for c in sets:
+        c["x"] = sets[0]["x"]
+        want.append(gpu_util.run_conv_oracle(c))
+    keys = dict(filter="w", bias="b", filter_exponents="ew", lut="lut")
+    with gpu_util.DeviceBuffers() as dev:
+        sources = [{k: dev.upload(c[a]) for k, a in keys.items() if c[a] is not None} for c in sets]
+        ptrs = {k: dev.upload(sets[0][a]) for k, a in keys.items() if sets[0][a] is not None}
+        ptrs["input"] = dev.upload(sets[0]["x"])
+        outs = [dev.upload(sets[0]["out"]) for _ in range(12)]
+        for i, out in enumerate(outs):
+            for k, a in keys.items():
+                if sets[0][a] is not None:
+                    d = abi.CopyDesc()
+                    d.src, d.dst, d.elem_size, d.ndim = sources[i % 3][k], ptrs[k], 1, 1
+                    d.shape[0], d.src_stride[0], d.dst_stride[0] = sets[0][a].nbytes, 1, 1
+                    abi.check(lib.espdl_b200_copy(C.byref(d), None), "copy")
+            ptrs["output"] = out
+            abi.check(lib.espdl_b200_conv2d_ws(C.byref(cases.conv_desc(sets[0], ptrs)), None, 0, None), "conv2d_ws")
+        for i, out in enumerate(outs):
+            np.testing.assert_array_equal(dev.download(out, want[i % 3]), want[i % 3], err_msg=f"layer {i}")
