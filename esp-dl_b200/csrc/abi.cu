@@ -19,6 +19,14 @@ static int *g_error_word = nullptr; // pinned, mapped: written by device-side wa
 static std::mutex g_ws_mutex;
 static void *g_ws = nullptr; // cached scratch of espdl_b200_conv2d (int16 limb planes)
 static size_t g_ws_bytes = 0;
+// Scratch of espdl_b200_conv2d for calls that can do without: a few streams keep one each, the least recently used makes room.
+struct StreamScratch {
+    unsigned long long stream = 0, used = 0; // the stream's id (never given to another one), the call that used it last
+    void *p = nullptr;
+    size_t bytes = 0;
+};
+static StreamScratch g_stream_scratch[4];
+static unsigned long long g_scratch_calls = 0;
 
 int set_cuda_error(cudaError_t e, const char *what)
 {
@@ -140,6 +148,11 @@ void espdl_b200_shutdown(void)
         cudaFree(g_ws);
         g_ws = nullptr;
         g_ws_bytes = 0;
+    }
+    for (StreamScratch &slot : g_stream_scratch) {
+        if (slot.p)
+            cudaFree(slot.p);
+        slot = StreamScratch();
     }
     g_device = -1;
 }
@@ -529,6 +542,45 @@ static size_t one_by_one_bytes(const espdl_conv_desc &d)
     return conv2d_tc_supported(one) ? conv2d_tc_workspace_bytes(one) : (conv2d_packed_supported(one) ? conv2d_packed_workspace_bytes(one) : 0);
 }
 
+// The scratch that `s` keeps, at least `need` bytes; null (the call does without) while the stream is being captured, whose graph would
+// keep the address, and where there is no memory.  g_ws_mutex is held.
+static StreamScratch *stream_scratch(cudaStream_t s, size_t need)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone || cudaStreamGetId(s, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    StreamScratch *slot = g_stream_scratch;
+    for (StreamScratch &c : g_stream_scratch) {
+        if (c.p && c.stream == id) {
+            slot = &c;
+            break;
+        }
+        if (c.used < slot->used)
+            slot = &c;
+    }
+    if (!slot->p || slot->stream != id || slot->bytes < need) {
+        // what still runs on the old block ends first: its own stream's work, or that of a stream which may be gone
+        if (slot->p && (slot->stream == id ? cudaStreamSynchronize(s) : cudaDeviceSynchronize()) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (slot->p)
+            cudaFree(slot->p);
+        *slot = StreamScratch();
+        if (cudaMalloc(&slot->p, need) != cudaSuccess) {
+            cudaGetLastError();
+            slot->p = nullptr;
+            return nullptr;
+        }
+        slot->stream = id, slot->bytes = need;
+    }
+    slot->used = ++g_scratch_calls;
+    return slot;
+}
+
 extern "C" {
 
 int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes)
@@ -630,9 +682,13 @@ int espdl_b200_conv2d(const espdl_conv_desc *desc, void *stream)
         return st;
     if (need == 0)
         return espdl_b200_conv2d_ws(desc, nullptr, 0, stream);
-    // The cached scratch is shared by all calls of this entry point: calls that need it are
-    // serialised on the host here and must be ordered on the device by the caller's streams.
     std::lock_guard<std::mutex> lock(g_ws_mutex);
+    if (!conv2d_tc_supported(*desc)) { // the CUDA cores run it as it is, the scratch only makes it faster
+        StreamScratch *scratch = stream_scratch((cudaStream_t)stream, need);
+        return espdl_b200_conv2d_ws(desc, scratch ? scratch->p : nullptr, scratch ? scratch->bytes : 0, stream);
+    }
+    // int16 Gemms and pointwise convs: the cached scratch is shared by all of them, which are serialised on the host here and must be
+    // ordered on the device by the caller's streams.
     if (need > g_ws_bytes) {
         if (g_ws) {
             ESPDL_CUDA_TRY(cudaDeviceSynchronize());

@@ -178,9 +178,15 @@ typedef struct espdl_conv_desc {
 int espdl_b200_conv2d(const espdl_conv_desc *desc, void *stream);
 
 /*
- * Scratch the int16 tensor-core path needs (the 8-bit limb planes of both
- * operands).  Returns 0 bytes for shapes that need none.  Pass the buffer with
- * espdl_b200_conv2d_ws; espdl_b200_conv2d allocates and caches one internally.
+ * Scratch a call runs with: int16 Gemms and pointwise convs need it (the 8-bit
+ * limb planes of both operands); other int16 convs, batches of int16 products and
+ * int8 layers that no kernel reads in place (a reduction that is no multiple of
+ * 16) are faster with it and run without it as well.  Returns 0 bytes for shapes
+ * that use none.  Pass the buffer with espdl_b200_conv2d_ws, one that no other
+ * launch in flight uses.  espdl_b200_conv2d brings its own: one for all int16
+ * Gemms and pointwise convs, which the caller's streams must keep in order, and for
+ * the others one a stream (four at most, the least recently used is given back;
+ * none while the stream is being captured).
  */
 int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes);
 /* 1 if the call runs the kernel for small layers, which reads narrow rows as they are (no gain from grouping pixels), else 0. */
@@ -198,7 +204,7 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
  * espdl_b200_conv2d_ws.  The 8-bit limb planes of both operands go into an array that is part of the library
  * image, ESPDL_B200_STATIC_SCRATCH_BYTES large; every GPU that loads the library holds it until the process ends.
  *
- *  - scratch needed is what espdl_b200_conv2d_workspace_bytes reports, 2*(M*K + N*K) bytes rounded up; a larger
+ *  - scratch needed is 2*(M*K + N*K) bytes rounded up (what espdl_b200_conv2d_workspace_bytes reports, less 4 M); a larger
  *    problem is rejected with ESPDL_ERR_TOO_LARGE, shapes the tensor-core int16 path does not take (K % 16 != 0,
  *    filters other than 1x1, K > 16384) with ESPDL_ERR_UNSUPPORTED;
  *  - the first call on each device looks up the array's device address (cudaGetSymbolAddress) and keeps it; that

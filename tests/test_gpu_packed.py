@@ -198,3 +198,63 @@ def test_batch_of_int16_products_with_the_scratch_it_asks_for(n, m, k, cout):
 def test_matmul_of_int16_slices(pairs, tmp_path):
     """Slices of one matrix each, and second operands that repeat over some of them, on the tile kernel and on the CUDA cores."""
     products_model(tmp_path, pairs, np.random.default_rng(10))
+
+
+def conv_on(lib, case, stream, dev, ptrs):
+    """One espdl_b200_conv2d on `stream`; returns the output's address."""
+    import ctypes as C
+    out = dev.upload(np.full_like(case["out"], 0x55))
+    abi.check(lib.espdl_b200_conv2d(C.byref(cases.conv_desc(case, dict(ptrs, output=out))), stream), "conv2d")
+    return out
+
+
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+def test_packed_convs_under_capture(dtype):
+    """Packing is an option of espdl_b200_conv2d: a capture, also the first time this size is met, runs without the scratch."""
+    import ctypes as C
+    lib = gpu_util.lib()
+    extra = dict(S16, wide=True) if dtype == abi.DTYPE_INT16 else {}
+    case = cases.conv_case(seed=3, n=3, h=61, w=59, cin=20, cout=40, kh=5, kw=5, pad=(2, 2, 2, 2), per_channel=True, **extra)
+    want = gpu_util.run_conv_oracle(case)
+    stream, graph = C.c_void_p(), C.c_void_p()
+    abi.check(lib.espdl_b200_stream_create(C.byref(stream)), "stream")
+    with gpu_util.DeviceBuffers() as dev:
+        ptrs = dict(input=dev.upload(case["x"]), filter=dev.upload(case["w"]), bias=dev.upload(case["b"]), filter_exponents=dev.upload(case["ew"]))
+        out = dev.upload(np.full_like(case["out"], 0x55))
+        d = cases.conv_desc(case, dict(ptrs, output=out))
+        need = C.c_size_t(0)
+        abi.check(lib.espdl_b200_conv2d_workspace_bytes(C.byref(d), C.byref(need)), "workspace")
+        assert need.value > 0
+        abi.check(lib.espdl_b200_graph_begin(stream), "begin")
+        st = lib.espdl_b200_conv2d(C.byref(d), stream)
+        end = lib.espdl_b200_graph_end(stream, C.byref(graph))
+        assert (st, end) == (abi.OK, abi.OK)
+        abi.check(lib.espdl_b200_graph_launch(graph, stream), "launch")
+        abi.check(lib.espdl_b200_stream_sync(stream), "sync")
+        np.testing.assert_array_equal(dev.download(out, want), want)
+        lib.espdl_b200_graph_destroy(graph)
+    lib.espdl_b200_stream_destroy(stream)
+
+
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+def test_packed_convs_on_streams_of_their_own(dtype):
+    """Streams that nothing orders, more of them than keep a scratch, sizes that grow: each its own inputs and results."""
+    import ctypes as C
+    lib = gpu_util.lib()
+    extra = dict(S16, wide=True) if dtype == abi.DTYPE_INT16 else {}
+    layers = [cases.conv_case(seed=i, n=1 + i % 3, h=40, w=37, cin=20, cout=40, per_channel=True, **extra) for i in range(6)]
+    want = [gpu_util.run_conv_oracle(c) for c in layers]
+    streams = [C.c_void_p() for _ in range(6)]
+    for s in streams:
+        abi.check(lib.espdl_b200_stream_create(C.byref(s)), "stream")
+    with gpu_util.DeviceBuffers() as dev:
+        ptrs = [dict(input=dev.upload(c["x"]), filter=dev.upload(c["w"]), bias=dev.upload(c["b"]), filter_exponents=dev.upload(c["ew"])) for c in layers]
+        outs = []
+        for i in [0, 1] * 8 + list(range(6)) * 3:
+            outs.append((i, conv_on(lib, layers[i], streams[i], dev, ptrs[i])))
+        for s in streams:
+            abi.check(lib.espdl_b200_stream_sync(s), "sync")
+        for i, out in outs:
+            np.testing.assert_array_equal(dev.download(out, want[i]), want[i])
+    for s in streams:
+        lib.espdl_b200_stream_destroy(s)
