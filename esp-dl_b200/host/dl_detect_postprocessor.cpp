@@ -72,10 +72,10 @@ esp_err_t yolo11PostProcessor::postprocess(int image)
             return ESP_FAIL;
     }
     const int batch = scores[0]->shape[0];
-    if (image >= batch)
-        return ESP_FAIL;
-    const int first = image < 0 ? 0 : image, scanned = image < 0 ? batch : 1;
     m_box_lists.resize(batch);
+    if (image >= batch)
+        return ESP_OK; // no such image, no results
+    const int first = image < 0 ? 0 : image, scanned = image < 0 ? batch : 1;
     // One read-back brings the counter and the first records: more than that are rare (a detector's candidates of one image
     // number in the dozens) and cost a second one.
     constexpr size_t COUNTER = 16, HEAD_RECORDS = 64;

@@ -48,14 +48,14 @@ def fake(tmp_path_factory):
     return str(host)
 
 
-def record(fake, tmp_path, graph, calls="run", batch=0, **env):
+def record(fake, tmp_path, graph, calls="run", batch=0, child=CHILD, **env):
     """[(call, {argument: value})] and the child's printed lines."""
     path, log = str(tmp_path / "g.espdl"), str(tmp_path / "log.txt")
     if isinstance(graph, str):
         path = graph
     else:
         graph.save(path)
-    r = subprocess.run([sys.executable, "-c", CHILD, fake, path, str(batch), calls], capture_output=True, text=True,
+    r = subprocess.run([sys.executable, "-c", child, fake, path, str(batch), calls], capture_output=True, text=True,
                        env=dict(os.environ, FAKE_DEVICE_LOG=log, REAL_DEVICE_LIB=abi.LIB_PATH, **env))
     assert r.returncode == 0, r.stderr
     lines = []
@@ -164,3 +164,45 @@ def test_int16_slices_have_the_scratch_of_the_tile_kernel(fake, tmp_path):
         assert int(a["need"]) and int(a["ws_bytes"]) >= int(a["need"])
         if int(a["filter"], 16) in spread:
             assert int(a["ws"], 16) >= int(a["filter"], 16) + 12 * 64 * 256 * 2
+
+
+SCORING_CHILD = r"""
+import ctypes as C, sys, threading
+import numpy as np
+host = C.CDLL(sys.argv[1])
+host.espdl_model_create.restype = C.c_void_p
+host.espdl_model_create.argtypes = [C.c_char_p, C.c_int, C.c_int]
+host.espdl_model_run.argtypes = [C.c_void_p]
+host.espdl_model_io_info.argtypes = [C.c_void_p, C.c_int, C.c_int] + [C.c_void_p] * 7
+host.espdl_model_classify.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_float)]
+host.espdl_model_detect.argtypes = [C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_char_p), C.POINTER(C.c_int), C.c_float, C.c_float, C.c_int, C.c_int, C.c_int, C.c_int,
+                                    C.POINTER(C.c_int), C.POINTER(C.c_float)]
+host.espdl_model_preprocess.argtypes = [C.c_void_p, C.c_void_p] + [C.c_int] * 4 + [C.POINTER(C.c_float)] * 2 + [C.c_int] * 2 + [C.c_void_p]
+h = host.espdl_model_create(sys.argv[2].encode(), 0, 0)
+assert host.espdl_model_run(h) == 0
+name, ndim, shape, dtype, e, hp, dp = C.c_char_p(), C.c_int(), (C.c_int * 8)(), C.c_int(), C.c_int(), C.c_void_p(), C.c_void_p()
+host.espdl_model_io_info(h, 1, 0, C.byref(name), C.byref(ndim), shape, C.byref(dtype), C.byref(e), C.byref(hp), C.byref(dp))
+dims = list(shape[:ndim.value])
+n = int(np.prod(dims))
+logits = np.frombuffer((C.c_char * n).from_address(dp.value), dtype=np.int8).reshape(dims)  # the stand-in's device memory
+logits[...] = np.random.default_rng(1).integers(-128, 128, size=dims, dtype=np.int8)
+
+def classify(image, k=20):
+    cat, score = (C.c_int * k)(), (C.c_float * k)()
+    found = host.espdl_model_classify(h, image, k, 0.0, image % 2, cat, score)
+    return found, list(cat[:max(found, 0)]), list(score[:max(found, 0)])
+
+def detect(image, k=20):
+    names = (C.c_char_p * 2)(b"y0", b"y0")
+    box, score = (C.c_int * (5 * k))(), (C.c_float * k)()
+    return host.espdl_model_detect(h, image, 1, names, (C.c_int * 1)(8), 0.5, 0.5, k, 64, 64, k, box, score)
+"""
+
+
+def test_images_outside_the_batch_have_no_results(fake, tmp_path):
+    child = SCORING_CHILD + r"""
+print("detect", ",".join(str(detect(i)) for i in (0, 1, 2, 7, -1)))
+print("classify", ",".join(str(classify(i)[0]) for i in (2, 7, -1)))
+"""
+    _, said = record(fake, tmp_path, matmul_graph([((2, 4, 4, 16), (16, 64), "S8")]), child=child)
+    assert said == {"detect": "0,0,0,0,0", "classify": "0,0,0"}
