@@ -9,6 +9,7 @@
 #include <cstring>
 #include <list>
 #include <memory>
+#include <mutex>
 #include <string>
 
 using namespace dl;
@@ -19,7 +20,9 @@ struct Handle {
     std::vector<std::string> input_names, output_names;
     std::string text;
     // What the calls below keep between calls: tables, staging buffers and counters on the device.  A program calls them with
-    // the same settings for every frame; the least recently used settings beyond four make room.
+    // the same settings for every frame; the least recently used settings beyond four make room.  One call at a time uses them:
+    // several threads may preprocess for, or score the images of, one model.
+    std::mutex calls;
     struct Pre {
         std::vector<float> key;
         std::unique_ptr<image::ImagePreprocessor> object;
@@ -235,6 +238,7 @@ int espdl_model_detect(void *handle, int image, int stages, const char *const *n
                        int top_k, int width, int height, int max_results, int *boxes, float *scores)
 {
     Handle *h = (Handle *)handle;
+    std::lock_guard<std::mutex> lock(h->calls);
     const std::vector<std::string> key(names, names + 2 * stages);
     const std::vector<int> stride_key(strides, strides + stages);
     if (!h->detector || h->detector_names != key || h->detector_strides != stride_key) {
@@ -270,6 +274,7 @@ int espdl_model_detect(void *handle, int image, int stages, const char *const *n
 int espdl_model_classify(void *handle, int image, int top_k, float score_thr, int need_softmax, int *categories, float *scores)
 {
     Handle *h = (Handle *)handle;
+    std::lock_guard<std::mutex> lock(h->calls);
     if (!h->classifier || h->classifier_softmax != (need_softmax != 0)) {
         h->classifier.reset(new cls::ClsPostprocessor(h->model, top_k, score_thr, need_softmax != 0));
         h->classifier_softmax = need_softmax != 0;
@@ -287,6 +292,7 @@ int espdl_model_preprocess(void *handle, const unsigned char *images, int n, int
                            int rgb_swap, int letterbox_bg, const int *crop)
 {
     Handle *handle_ = (Handle *)handle;
+    std::lock_guard<std::mutex> lock(handle_->calls);
     Model *model = handle_->model;
     std::vector<float> key = {(float)channels, (float)(rgb_swap != 0), (float)letterbox_bg};
     for (int c = 0; c < (channels == 3 ? 3 : 1); c++) key.push_back(mean[c]), key.push_back(stdv[c]);

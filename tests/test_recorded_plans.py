@@ -206,3 +206,31 @@ print("classify", ",".join(str(classify(i)[0]) for i in (2, 7, -1)))
 """
     _, said = record(fake, tmp_path, matmul_graph([((2, 4, 4, 16), (16, 64), "S8")]), child=child)
     assert said == {"detect": "0,0,0,0,0", "classify": "0,0,0"}
+
+
+def test_several_threads_score_one_finished_batch(fake, tmp_path):
+    """The objects that a handle keeps between calls serve one call at a time: threads that score different images, with and without
+    softmax, detect and preprocess beside one another get what a single one gets."""
+    child = SCORING_CHILD + r"""
+want = [classify(i) for i in range(32)]
+wrong = []
+mean, std = (C.c_float * 3)(0, 0, 0), (C.c_float * 3)(1, 1, 1)
+def score(part):
+    for _ in range(40):
+        for i in range(part, 32, 8):
+            if classify(i) != want[i]:
+                wrong.append(i)
+def others(which):
+    frames = np.zeros((1, 9 + which, 11, 1), dtype=np.uint8)
+    for k in range(300):
+        if detect(k % 32) != 0:
+            wrong.append(-1)
+        one = (C.c_float * 3)(k % 7, 0, 0)
+        host.espdl_model_preprocess(h, frames.ctypes.data, 1, 9 + which, 11, 1, one, std, 0, -1, None)
+threads = [threading.Thread(target=score, args=(p,)) for p in range(8)] + [threading.Thread(target=others, args=(w,)) for w in range(2)]
+for t in threads: t.start()
+for t in threads: t.join()
+print("wrong", len(wrong))
+"""
+    _, said = record(fake, tmp_path, matmul_graph([((32, 1, 1, 16), (16, 64), "S8")]), child=child)
+    assert said == {"wrong": "0"}
