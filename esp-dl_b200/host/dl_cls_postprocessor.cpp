@@ -75,13 +75,15 @@ std::vector<result_t> &ClsPostprocessor::postprocess(int image)
 
 std::vector<result_t> &ClsPostprocessor::postprocess_one(int image)
 {
-    if (!m_model_output || m_model_output->dtype != DATA_TYPE_INT8 || m_model_output->shape.empty()) {
+    const bool shaped = m_model_output && !m_model_output->shape.empty();
+    const int batch = shaped ? m_model_output->shape[0] : 0;
+    const int classes = batch > 0 ? m_model_output->get_size() / batch : 0;
+    // Softmax runs along the last axis: the row of an image only where that axis is all it has
+    if (!shaped || m_model_output->dtype != DATA_TYPE_INT8 || m_model_output->shape.back() != classes) {
         invalidate();
         return postprocess(image);
     }
     m_cls_result.clear();
-    const int batch = m_model_output->shape[0];
-    const int classes = m_model_output->get_size() / (batch > 0 ? batch : 1);
     if (image < 0 || image >= batch || (!m_row && espdl_b200_host_alloc(classes, (void **)&m_row) != ESPDL_OK))
         return m_cls_result;
     void *stream = m_model->stream();

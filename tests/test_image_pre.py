@@ -182,3 +182,33 @@ def test_model_preprocessor_fills_the_input_tensor(tmp_path, letterbox, swap, cr
         for cat, score in top:
             assert probs[image][cat] == np.float32(score)
     m.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2, 3, 16), (2, 1, 16), (2, 2, 3, 16), (5, 16), (16,)])
+def test_classes_in_several_axes(shape, tmp_path):
+    """The classes of an image are all its elements; softmax runs along the last axis, as dl::module::Softmax with axis -1 does."""
+    import cases
+    from espdl_b200 import espdl_file, model
+    rng = np.random.default_rng(4)
+    g = espdl_file.GraphBuilder("classes", metadata={"target": "c"})
+    g.add_input("x", np.int8, list(shape), -5)
+    g.add_initializer("w", rng.integers(-60, 60, size=(16, 6), dtype=np.int8), [-6])
+    g.add_node("MatMul", "mm", ["x", "w"], ["y"], quant_type="S8", activation="Linear")
+    g.add_output("y", np.int8, list(shape[:-1]) + [6], -4)
+    path = str(tmp_path / "m.espdl")
+    g.save(path)
+    m = model.Model(path)
+    m.inputs[0].array[...] = rng.integers(-60, 60, size=m.inputs[0].shape, dtype=np.int8)
+    m.run()
+    logits = np.array(m.outputs[0].array)
+    table_f = np.zeros(256, dtype=np.float32)
+    checkers.oracle().oracle_softmax_table(table_f.ctypes.data, -4)
+    probs = np.zeros(logits.shape, dtype=np.float32)
+    assert checkers.oracle().oracle_softmax(cases.softmax_desc(logits.ctypes.data, probs.ctypes.data, table_f.ctypes.data, logits.size // 6, 6, abi.DTYPE_FLOAT, 0)) == 0
+    for image in range(logits.shape[0]):
+        for softmax, scores in ((True, probs), (False, logits * np.float32(2.0 ** -4))):
+            want = np.sort(np.asarray(scores, dtype=np.float32).reshape(logits.shape[0], -1)[image])[::-1]
+            got = m.classify(image=image, top_k=want.size, score_thr=-100.0, need_softmax=softmax)
+            np.testing.assert_array_equal(np.array([s for _, s in got], dtype=np.float32), want)
+    m.close()
