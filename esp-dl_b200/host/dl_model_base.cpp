@@ -849,6 +849,7 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
     // own, since a shared one would order the branches again.  Measured per pass, chain -> branches: re-identification of 1 / 27 /
     // 128 crops 800 -> 418, 972 -> 627, 1673 -> 1353 us; 320x320 detector, 1 / 64 images 704 -> 547, 4449 -> 3708 us; 640x640,
     // 32 images 1399 -> 1359 us.  The gain fades as launches fill the GPU while the buffers grow six-fold, hence the limit.
+    std::vector<TensorInfo> chain; // the plan to go back to where there is no memory for buffers of their own
     if (m_reuse_memory && m_use_graph && !m_plan_only && env_flag("ESPDL_B200_BRANCHES", true)) {
         std::map<std::string, int> depth;
         int longest = 0;
@@ -866,6 +867,7 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
         std::vector<TensorInfo> apart = infos;
         const size_t bytes = MemoryManagerGreedy::plan(apart, false);
         if (longest * 10 < (int)m_execution_plan.size() * 9 && bytes <= limit) {
+            chain = infos;
             infos = apart;
             m_arena_bytes = bytes;
             m_branches = true;
@@ -890,7 +892,14 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
     }
     if (m_plan_only)
         return;
-    if (espdl_b200_arena_alloc(m_arena_bytes + 256, &m_arena) != ESPDL_OK) {
+    int st = espdl_b200_arena_alloc(m_arena_bytes + 256, &m_arena);
+    if (st != ESPDL_OK && m_branches) {
+        infos = chain;
+        m_branches = false;
+        m_arena_bytes = MemoryManagerGreedy::plan(infos, m_reuse_memory);
+        st = espdl_b200_arena_alloc(m_arena_bytes + 256, &m_arena);
+    }
+    if (st != ESPDL_OK) {
         ESP_LOGE("dl::Model", "Failed to allocate a %.1f MB device arena", m_arena_bytes / 1048576.0);
         m_status = ESPDL_ERR_NO_MEM;
         return;

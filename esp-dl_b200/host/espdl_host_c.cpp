@@ -79,7 +79,8 @@ void *espdl_model_create(const char *path, int batch, int flags)
     return h;
 }
 
-/// Loads a model and plans its arena without touching a device.  Returns the number of planned tensors (negative on
+/// Loads a model and plans its arena without touching a device, for its steps as one chain (a loaded model whose branches run side by
+/// side takes more: espdl_model_arena_bytes).  Returns the number of planned tensors (negative on
 /// error); *arena_bytes and *slices receive the arena size and the number of channel slices, and `text` (capacity `cap`)
 /// one line per slice: "name<TAB>name of the tensor it lives in<TAB>byte offset inside it<TAB>row stride in elements".
 int espdl_model_plan(const char *path, int batch, int reuse, size_t *arena_bytes, int *slices, char *text, size_t cap)

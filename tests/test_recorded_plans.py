@@ -234,3 +234,18 @@ print("wrong", len(wrong))
 """
     _, said = record(fake, tmp_path, matmul_graph([((32, 1, 1, 16), (16, 64), "S8")]), child=child)
     assert said == {"wrong": "0"}
+
+
+def test_no_memory_for_buffers_of_their_own_is_a_chain(fake, tmp_path):
+    """Where the arena of a branched plan cannot be allocated the model takes the chain's, which loaded before there were branches."""
+    from espdl_b200 import zoo
+    g = zoo.yolo11n_style(seed=6, input_hw=96)
+    lines, said = record(fake, tmp_path, g)
+    branches = int(said["arena"])
+    assert any(n == "wait" for n, _ in captured(lines))
+    _, said = record(fake, tmp_path, g, ESPDL_B200_BRANCHES="0")
+    chain = int(said["arena"])
+    assert chain < branches
+    lines, said = record(fake, tmp_path, g, FAKE_ARENA_LIMIT=str(branches))
+    assert said == {"arena": str(chain), "run": "0"}
+    assert not any(n == "wait" for n, _ in captured(lines))
