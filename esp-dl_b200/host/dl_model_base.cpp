@@ -849,7 +849,8 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
     // own, since a shared one would order the branches again.  Measured per pass, chain -> branches: re-identification of 1 / 27 /
     // 128 crops 800 -> 418, 972 -> 627, 1673 -> 1353 us; 320x320 detector, 1 / 64 images 704 -> 547, 4449 -> 3708 us; 640x640,
     // 32 images 1399 -> 1359 us.  The gain fades as launches fill the GPU while the buffers grow six-fold, hence the limit.
-    std::vector<TensorInfo> chain; // the plan to go back to where there is no memory for buffers of their own
+    std::vector<TensorInfo> chain, apart = infos; // chain: the plan to go back to where there is no memory for buffers of their own
+    const size_t bytes = MemoryManagerGreedy::plan(apart, false);
     if (m_reuse_memory && m_use_graph && !m_plan_only && env_flag("ESPDL_B200_BRANCHES", true)) {
         std::map<std::string, int> depth;
         int longest = 0;
@@ -864,18 +865,16 @@ void Model::build(size_t max_internal_size, memory_manager_t mm_type, bool prelo
         }
         const char *mb = getenv("ESPDL_B200_BRANCH_MB");
         const size_t limit = mb ? (size_t)atoi(mb) << 20 : BRANCH_LIMIT;
-        std::vector<TensorInfo> apart = infos;
-        const size_t bytes = MemoryManagerGreedy::plan(apart, false);
         if (longest * 10 < (int)m_execution_plan.size() * 9 && bytes <= limit) {
             chain = infos;
             infos = apart;
             m_arena_bytes = bytes;
             m_branches = true;
         }
-        // Early-resident blocks crowd the SMs that finish first: a loss once a launch is long enough to hide the boundary anyway
-        // (classifier, 256 images = 64 MB a step: 1262 us plain, 1229 overlapped; 512: 2068, 2085; 1024: 3677, 3841)
-        m_plain_launches = !m_branches && bytes / std::max<size_t>(1, m_execution_plan.size()) > PLAIN_STEP;
     }
+    // Early-resident blocks crowd the SMs that finish first: a loss once a launch is long enough to hide the boundary anyway
+    // (classifier, 256 images = 64 MB a step: 1262 us plain, 1229 overlapped; 512: 2068, 2085; 1024: 3677, 3841)
+    m_plain_launches = !m_branches && bytes / std::max<size_t>(1, m_execution_plan.size()) > PLAIN_STEP;
     if (!m_branches)
         m_arena_bytes = MemoryManagerGreedy::plan(infos, m_reuse_memory);
     // the last step that reads a graph input's buffer (directly, or through a view / slice that lives in it)

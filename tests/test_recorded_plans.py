@@ -22,7 +22,7 @@ for f in ("run", "destroy"):
 host.espdl_model_run_device.argtypes = [C.c_void_p, C.c_int]
 host.espdl_model_arena_bytes.argtypes = [C.c_void_p]
 host.espdl_model_arena_bytes.restype = C.c_size_t
-h = host.espdl_model_create(sys.argv[2].encode(), int(sys.argv[3]), 0)
+h = host.espdl_model_create(sys.argv[2].encode(), int(sys.argv[3]), int(sys.argv[5]))
 if not h:
     print("status none")
     sys.exit()
@@ -48,14 +48,14 @@ def fake(tmp_path_factory):
     return str(host)
 
 
-def record(fake, tmp_path, graph, calls="run", batch=0, child=CHILD, **env):
+def record(fake, tmp_path, graph, calls="run", batch=0, child=CHILD, flags=0, **env):
     """[(call, {argument: value})] and the child's printed lines."""
     path, log = str(tmp_path / "g.espdl"), str(tmp_path / "log.txt")
     if isinstance(graph, str):
         path = graph
     else:
         graph.save(path)
-    r = subprocess.run([sys.executable, "-c", child, fake, path, str(batch), calls], capture_output=True, text=True,
+    r = subprocess.run([sys.executable, "-c", child, fake, path, str(batch), calls, str(flags)], capture_output=True, text=True,
                        env=dict(os.environ, FAKE_DEVICE_LOG=log, REAL_DEVICE_LIB=abi.LIB_PATH, **env))
     assert r.returncode == 0, r.stderr
     lines = []
@@ -249,3 +249,21 @@ def test_no_memory_for_buffers_of_their_own_is_a_chain(fake, tmp_path):
     lines, said = record(fake, tmp_path, g, FAKE_ARENA_LIMIT=str(branches))
     assert said == {"arena": str(chain), "run": "0"}
     assert not any(n == "wait" for n, _ in captured(lines))
+
+
+def large_layer():
+    """One 1x1 conv between tensors of 100 MB."""
+    g = espdl_file.GraphBuilder("large", metadata={"target": "c"})
+    g.add_input("x", np.int8, [1, 1024, 1024, 96], -5)
+    g.add_initializer("w", np.ones((1, 1, 96, 96), dtype=np.int8), [-6])
+    g.add_node("Conv", "c0", ["x", "w"], ["y"], quant_type="S8", activation="Linear", pads=[0, 0, 0, 0], strides=[1, 1], dilations=[1, 1], group=1)
+    g.add_output("y", np.int8, [1, 1024, 1024, 96], -5)
+    return g
+
+
+def test_large_steps_are_plain_launches_however_buffers_are_planned(fake, tmp_path):
+    for flags, env in ((0, {}), (0, {"ESPDL_B200_BRANCHES": "0"}), (2, {})):
+        lines, _ = record(fake, tmp_path, large_layer(), calls="run_device", flags=flags, **env)
+        assert [a["overlap"] for n, a in captured(lines) if n == "conv"] == ["0"], (flags, env)
+    lines, _ = record(fake, tmp_path, matmul_graph([PLAIN]), calls="run_device")
+    assert [a["overlap"] for n, a in captured(lines) if n == "conv"] == ["1"]
