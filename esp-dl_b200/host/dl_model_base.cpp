@@ -1031,8 +1031,9 @@ void Model::run(runtime_mode_t mode)
                 espdl_b200_upload(kv.second->device, kv.second->data, kv.second->get_bytes(), ctx->stream);
     };
     // The copies are nodes of the graph: one launch for the whole pass, and with branches each output leaves when it is ready.  (A
-    // graph keeps the addresses it was captured with; a caller that moved a tensor's host buffer gets the plain form.)
-    if (m_use_graph && (!m_graph_io || m_graph_io_buffers == io_buffers())) {
+    // graph keeps the addresses it was captured with; a caller that moved a tensor's host buffer gets the plain form.)  Large steps
+    // gain nothing from that: they share the graph of run_device(), which a program that uses both would capture besides.
+    if (m_use_graph && !m_plain_launches && (!m_graph_io || m_graph_io_buffers == io_buffers())) {
         if (!m_graph_io) {
             upload();
             m_graph_io_buffers = io_buffers();

@@ -267,3 +267,14 @@ def test_large_steps_are_plain_launches_however_buffers_are_planned(fake, tmp_pa
         assert [a["overlap"] for n, a in captured(lines) if n == "conv"] == ["0"], (flags, env)
     lines, _ = record(fake, tmp_path, matmul_graph([PLAIN]), calls="run_device")
     assert [a["overlap"] for n, a in captured(lines) if n == "conv"] == ["1"]
+
+
+def test_run_and_run_device_share_the_graph_of_large_steps(fake, tmp_path):
+    """The copies are part of the captured graph where a pass is short enough for launches to count."""
+    lines, said = record(fake, tmp_path, large_layer(), calls="run,run_device,run")
+    names = [n for n, _ in lines]
+    assert names.count("graph_begin") == 1 and names.count("graph_launch") == 3 and said["run"] == "0"
+    assert "upload" not in [n for n, _ in captured(lines)]
+    lines, _ = record(fake, tmp_path, matmul_graph([PLAIN]), calls="run,run_device,run")
+    names = [n for n, _ in lines]
+    assert names.count("graph_begin") == 2 and "upload" in [n for n, _ in captured(lines)]
