@@ -145,8 +145,11 @@ esp_err_t Model::capture_plan(int first, int last, bool io, void **graph)
     }
     while ((int)m_branch_streams.size() < limit - 1) {
         void *s = nullptr;
-        if (espdl_b200_stream_create(&s) != ESPDL_OK)
+        const int made = espdl_b200_stream_create(&s);
+        if (made) {
+            m_status = made;
             return ESP_FAIL;
+        }
         m_branch_streams.push_back(s);
     }
     std::vector<void *> streams = {ctx->stream};

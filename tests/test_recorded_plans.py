@@ -278,3 +278,9 @@ def test_run_and_run_device_share_the_graph_of_large_steps(fake, tmp_path):
     lines, _ = record(fake, tmp_path, matmul_graph([PLAIN]), calls="run,run_device,run")
     names = [n for n, _ in lines]
     assert names.count("graph_begin") == 2 and "upload" in [n for n, _ in captured(lines)]
+
+
+def test_a_capture_that_gets_no_stream_is_an_error(fake, tmp_path):
+    """run() has no result of its own: what went wrong is the model's status, not the last pass's outputs in silence."""
+    _, said = record(fake, tmp_path, matmul_graph([PLAIN, PLAIN, PLAIN]), calls="run,run_device", FAKE_STREAM_LIMIT="1")
+    assert int(said["run"]) == abi.ERR_CUDA and int(said["run_device"]) != 0
