@@ -211,6 +211,8 @@ SYMBOLS = {
     "espdl_b200_graph_end": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p)]),
     "espdl_b200_graph_launch": (C.c_int, [C.c_void_p, C.c_void_p]),
     "espdl_b200_graph_destroy": (C.c_int, [C.c_void_p]),
+    "espdl_b200_graph_destroy_idle": (C.c_int, [C.c_void_p]),
+    "espdl_b200_tile_counters": (C.c_int, []),
     "espdl_b200_model_scope": (None, [C.c_int]),
     "espdl_b200_overlap": (None, [C.c_int]),
     "espdl_b200_conv2d": (C.c_int, [C.POINTER(ConvDesc), C.c_void_p]),

@@ -1,5 +1,6 @@
 // C ABI: life cycle, memory and the conv2d dispatcher (include/espdl_b200.h).
 #include "common.cuh"
+#include "tile_counters.cuh"
 
 #include <atomic>
 #include <cstdarg>
@@ -50,25 +51,35 @@ int num_sms() { return g_num_sms > 0 ? g_num_sms : 148; }
 namespace {
 constexpr int SCHED_PAIRS = 2048;
 __device__ unsigned g_sched_words[2 * SCHED_PAIRS]; // zero at load; every kernel leaves its pair zero
+std::mutex g_sched_mutex;
+TileCounters g_sched_pairs(SCHED_PAIRS);
+std::map<cudaGraphExec_t, unsigned long long> g_graph_capture; // whose capture a graph came from, while it lives
+
+// The capture that `s` is in, 0 for none; false where that cannot be asked.
+bool capture_of(cudaStream_t s, unsigned long long &id)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    id = 0;
+    if (cudaStreamGetCaptureInfo(s, &cs, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (cs != cudaStreamCaptureStatusActive)
+        id = 0;
+    return true;
+}
 }
 
 unsigned *sched_counters(cudaStream_t s)
 {
-    static std::mutex mu;
-    static std::map<std::pair<unsigned long long, cudaStream_t>, int> pair_of; // (capture id or 0, stream) -> pair
     static unsigned *base = nullptr;
     static const bool off = getenv("ESPDL_B200_STATIC_TILES") != nullptr;
     if (off)
         return nullptr;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     unsigned long long id = 0;
-    if (cudaStreamGetCaptureInfo(s, &cs, &id) != cudaSuccess) {
-        cudaGetLastError();
+    if (!capture_of(s, id))
         return nullptr;
-    }
-    // branches of one graph are captured on streams of their own and may run side by side
-    const std::pair<unsigned long long, cudaStream_t> key(cs == cudaStreamCaptureStatusActive ? id : 0ull, s);
-    std::lock_guard<std::mutex> lock(mu);
+    std::lock_guard<std::mutex> lock(g_sched_mutex);
     if (!base) {
         void *p = nullptr;
         if (cudaGetSymbolAddress(&p, g_sched_words) != cudaSuccess) {
@@ -77,13 +88,9 @@ unsigned *sched_counters(cudaStream_t s)
         }
         base = (unsigned *)p;
     }
-    auto it = pair_of.find(key);
-    if (it == pair_of.end()) {
-        if ((int)pair_of.size() >= SCHED_PAIRS)
-            return nullptr;
-        it = pair_of.emplace(key, (int)pair_of.size()).first;
-    }
-    return base + 2 * it->second;
+    // branches of one graph are captured on streams of their own and may run side by side
+    const int pair = g_sched_pairs.get(id, s);
+    return pair < 0 ? nullptr : base + 2 * pair;
 }
 
 int check_launch(const char *what)
@@ -299,8 +306,15 @@ int espdl_b200_stream_create(void **stream)
 
 int espdl_b200_stream_destroy(void *stream)
 {
-    if (stream)
-        ESPDL_CUDA_TRY(cudaStreamDestroy((cudaStream_t)stream));
+    if (!stream)
+        return ESPDL_OK;
+    unsigned long long id = 0;
+    if (capture_of((cudaStream_t)stream, id) && !id && cudaStreamQuery((cudaStream_t)stream) == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(g_sched_mutex);
+        g_sched_pairs.give_back_stream(stream);
+    }
+    cudaGetLastError(); // work in flight: its pair stays taken
+    ESPDL_CUDA_TRY(cudaStreamDestroy((cudaStream_t)stream));
     return ESPDL_OK;
 }
 
@@ -374,13 +388,23 @@ int espdl_b200_graph_end(void *stream, void **graph)
 {
     if (!stream || !graph)
         return ESPDL_ERR_INVALID_ARG;
+    unsigned long long id = 0;
+    capture_of((cudaStream_t)stream, id);
     cudaGraph_t g = nullptr;
-    ESPDL_CUDA_TRY(cudaStreamEndCapture((cudaStream_t)stream, &g));
     cudaGraphExec_t exec = nullptr;
-    cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess)
-        return set_cuda_error(e, "cudaGraphInstantiate");
+    cudaError_t e = cudaStreamEndCapture((cudaStream_t)stream, &g);
+    const char *what = "cudaStreamEndCapture";
+    if (e == cudaSuccess) {
+        what = "cudaGraphInstantiate";
+        e = cudaGraphInstantiate(&exec, g, 0);
+        cudaGraphDestroy(g);
+    }
+    std::lock_guard<std::mutex> lock(g_sched_mutex);
+    if (e != cudaSuccess) {
+        g_sched_pairs.give_back_capture(id); // nothing of it was ever launched
+        return set_cuda_error(e, what);
+    }
+    g_graph_capture[exec] = id;
     *graph = (void *)exec;
     return ESPDL_OK;
 }
@@ -393,11 +417,30 @@ int espdl_b200_graph_launch(void *graph, void *stream)
     return ESPDL_OK;
 }
 
-int espdl_b200_graph_destroy(void *graph)
+static int graph_destroy(void *graph, bool idle)
 {
-    if (graph)
-        ESPDL_CUDA_TRY(cudaGraphExecDestroy((cudaGraphExec_t)graph));
+    if (!graph)
+        return ESPDL_OK;
+    {
+        std::lock_guard<std::mutex> lock(g_sched_mutex);
+        auto it = g_graph_capture.find((cudaGraphExec_t)graph);
+        if (it != g_graph_capture.end()) {
+            if (idle && it->second)
+                g_sched_pairs.give_back_capture(it->second);
+            g_graph_capture.erase(it);
+        }
+    }
+    ESPDL_CUDA_TRY(cudaGraphExecDestroy((cudaGraphExec_t)graph));
     return ESPDL_OK;
+}
+
+int espdl_b200_graph_destroy(void *graph) { return graph_destroy(graph, false); }
+int espdl_b200_graph_destroy_idle(void *graph) { return graph_destroy(graph, true); }
+
+int espdl_b200_tile_counters(void)
+{
+    std::lock_guard<std::mutex> lock(g_sched_mutex);
+    return g_sched_pairs.taken();
 }
 
 } // extern "C"

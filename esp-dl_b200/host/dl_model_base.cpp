@@ -179,17 +179,11 @@ void Model::release_pipeline()
 
 void Model::release()
 {
-    if (m_model_context && m_model_context->stream)
-        espdl_b200_stream_sync(m_model_context->stream);
+    const bool idle = m_model_context && m_model_context->stream && espdl_b200_stream_sync(m_model_context->stream) == ESPDL_OK;
     release_pipeline();
-    if (m_graph)
-        espdl_b200_graph_destroy(m_graph);
-    if (m_graph_head)
-        espdl_b200_graph_destroy(m_graph_head);
-    if (m_graph_tail)
-        espdl_b200_graph_destroy(m_graph_tail);
-    if (m_graph_io)
-        espdl_b200_graph_destroy(m_graph_io);
+    for (void *graph : {m_graph, m_graph_head, m_graph_tail, m_graph_io})
+        if (graph)
+            idle ? espdl_b200_graph_destroy_idle(graph) : espdl_b200_graph_destroy(graph);
     m_graph = m_graph_head = m_graph_tail = m_graph_io = nullptr;
     for (void *stream : m_branch_streams) espdl_b200_stream_destroy(stream);
     m_branch_streams.clear();

@@ -108,6 +108,10 @@ int espdl_b200_graph_begin(void *stream);                 /* start capturing wor
 int espdl_b200_graph_end(void *stream, void **graph);     /* stop capturing, instantiate                 */
 int espdl_b200_graph_launch(void *graph, void *stream);
 int espdl_b200_graph_destroy(void *graph);
+/* The same for a graph whose launches have all finished: the tile counters that its persistent kernels hold (2048 pairs there are, a
+ * pair a stream and a pair a stream of each capture; kernels that get none deal out their tiles in the fixed order) serve others again. */
+int espdl_b200_graph_destroy_idle(void *graph);
+int espdl_b200_tile_counters(void); /* pairs held at the moment */
 /* Between espdl_b200_model_scope(1) and espdl_b200_model_scope(0) the calling thread promises that no launch writes what a
  * later launch takes as filter, bias or exponents (the plan of a model: parameters are constants).  Kernels then overlap their
  * start with the end of the kernel before them more widely.  Nests. */

@@ -546,3 +546,22 @@ def test_prelu_folding_pass(monkeypatch):
         np.testing.assert_array_equal(got.reshape(want[name].shape), want[name])
         np.testing.assert_array_equal(got, outs["0"][0][name])
         assert want[name].astype(np.float32).std() > 0
+
+
+def test_models_that_come_and_go_keep_no_tile_counters(tmp_path):
+    """Persistent kernels take pairs of counters per stream and capture, of which there are 2048 in the process."""
+    path = str(tmp_path / "net.espdl")
+    zoo.mobilenet_v2(seed=5).save(path)
+    lib = abi.load()
+    held = []
+    for _ in range(4):
+        m = model.Model(path, batch=64)
+        m.run()
+        m.run_device()
+        m.submit()
+        m.wait()
+        during = lib.espdl_b200_tile_counters()
+        m.close()
+        held.append(lib.espdl_b200_tile_counters())
+        assert during > held[-1]
+    assert held[0] == held[-1]

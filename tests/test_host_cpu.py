@@ -3,6 +3,7 @@ golden files and on generated networks, and the lifetime-based arena planner."""
 import ctypes as C
 import glob
 import os
+import subprocess
 
 import numpy as np
 import pytest
@@ -367,3 +368,46 @@ def test_planner_leaves_ragged_concats_alone(host):
         pytest.skip("fixture not present")
     n, arena, slices, views = _plan(host, path)
     assert n > 40 and slices == 0 and arena > 0
+
+
+COUNTERS_PROGRAM = r"""
+#include <cstdio>
+#include <set>
+#include "tile_counters.cuh"
+int main()
+{
+    espdl::TileCounters t(64);
+    char streams[16];
+    std::set<int> seen;
+    for (int i = 0; i < 8; i++) seen.insert(t.get(0, streams + i)); // streams
+    for (int round = 1; round <= 1000; round++) // models that come and go: two captures of six streams each
+        for (int k = 0; k < 2; k++) {
+            const unsigned long long id = 2ull * round + k;
+            std::set<int> own;
+            for (int i = 0; i < 6; i++) {
+                const int p = t.get(id, streams + i);
+                if (p < 0 || p >= 64 || seen.count(p) || !own.insert(p).second || t.get(id, streams + i) != p)
+                    return printf("round %d capture %llu stream %d: pair %d\n", round, id, i, p), 1;
+            }
+            if (round % 3 || k) // one is kept a round longer
+                t.give_back_capture(id);
+            if (k == 0 && round % 3 == 1 && round > 1)
+                t.give_back_capture(2ull * (round - 1));
+        }
+    for (int i = 0; i < 8; i++) t.give_back_stream(streams + i), t.give_back_stream(streams + i);
+    while (t.get(5000, streams) >= 0 && t.taken() < 64) t.get(6000 + t.taken(), streams + t.taken() % 16);
+    if (t.taken() != 64 || t.get(9999, streams) != -1 || t.get(5000, streams) < 0)
+        return printf("taken %d\n", t.taken()), 1;
+    return 0;
+}
+"""
+
+
+def test_tile_counters_are_given_back(tmp_path):
+    """Pairs of captures and streams that are gone serve others; pairs in use are never handed out twice; none left is said."""
+    src = tmp_path / "counters.cpp"
+    src.write_text(COUNTERS_PROGRAM)
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "esp-dl_b200", "csrc")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-I" + csrc, str(src), "-o", str(tmp_path / "counters")])
+    r = subprocess.run([str(tmp_path / "counters")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout

@@ -284,3 +284,11 @@ def test_a_capture_that_gets_no_stream_is_an_error(fake, tmp_path):
     """run() has no result of its own: what went wrong is the model's status, not the last pass's outputs in silence."""
     _, said = record(fake, tmp_path, matmul_graph([PLAIN, PLAIN, PLAIN]), calls="run,run_device", FAKE_STREAM_LIMIT="1")
     assert int(said["run"]) == abi.ERR_CUDA and int(said["run_device"]) != 0
+
+
+def test_a_released_model_gives_its_tile_counters_back(fake, tmp_path):
+    """Its graphs are idle by then: synchronised, then destroyed as such."""
+    lines, _ = record(fake, tmp_path, matmul_graph([PLAIN]), calls="run,run_device")
+    names = [n for n, _ in lines]
+    assert names.count("graph_destroy_idle") == names.count("graph_begin") == 2 and "graph_destroy" not in names
+    assert "stream_sync" in names[len(names) - 1 - names[::-1].index("graph_launch"):names.index("graph_destroy_idle")]
