@@ -143,8 +143,8 @@ int conv2d_band_tc(const espdl_conv_desc &d, cudaStream_t s);
 // Callers guarantee shift >= -31.
 __device__ __forceinline__ int32_t shift_round32(int32_t v, int shift, int half_even)
 {
-    if (shift > 31)
-        return 0; // |v| is at most 2^31, half a step of 2^32, and that tie goes to 0 either way
+    if (shift > 31) // |v| is at most 2^31, half a step of 2^32, and that tie goes to 0 either way
+        v = 0, shift = 31;
     if (shift > 0) {
         int32_t q = v >> shift;
         if (!half_even) {

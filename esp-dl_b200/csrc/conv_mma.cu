@@ -36,6 +36,7 @@ struct MmaParams {
     int ic, ih, iw, oh, ow, kw, sh, sw, dh, dw, pt, pl, ips, ops, rps, lut_stride;
     long long w_image;            // batch of products: elements from one image's filter to the next (gridDim.y images)
     int e_shift_base, ew_scalar, per_channel, relu, half_even;
+    int acc_bound; // of |sum|, see fast_constants
     int early; // the filter is a constant of the model: loaded before the wait for the previous kernel
 };
 
@@ -62,6 +63,7 @@ __device__ __forceinline__ uint4 dense_chunk(const int8_t *row, int k, int K)
 __device__ __noinline__ uint32_t general_word(const MmaParams &p, const int (&v)[4], int oc0)
 {
     uint32_t word = 0;
+#pragma unroll 1 // rare: four copies of the form are half of a small kernel's code
     for (int i = 0; i < 4; i++) {
         const int n = min(oc0 + i, p.N - 1);
         const int shift = max(-31, min(32, p.e_shift_base - (p.per_channel ? __ldg(p.ew + n) : p.ew_scalar)));
@@ -149,11 +151,11 @@ __global__ void __launch_bounds__(32 * MMA_WARPS) conv_mma_kernel(const __grid_c
     constexpr int QUADS = COLS / 4;
     const int e_lane = kpart * 32 + lane, cq = e_lane % QUADS, oc0 = tn * COLS + 4 * cq;
     int bias_half[4], shift[4];
-    bool fast = p.K <= 65536; // 2^14 a term: beyond that the sum alone may reach 2^31 and the rounding's half leave 32 bits
+    bool fast = true;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int n = min(oc0 + i, p.N - 1);
-        fast = fast_constants(p.bias ? __ldg(p.bias + n) : 0, p.e_shift_base - (p.per_channel ? __ldg(p.ew + n) : p.ew_scalar), min(p.K, 65536) << 14, p.half_even,
+        fast = fast_constants(p.bias ? __ldg(p.bias + n) : 0, p.e_shift_base - (p.per_channel ? __ldg(p.ew + n) : p.ew_scalar), p.acc_bound, p.half_even,
                               bias_half[i], shift[i]) && fast;
     }
     // the input rows of this lane's fragments
@@ -416,6 +418,8 @@ int conv2d_mma(const espdl_conv_desc &d, cudaStream_t s)
     p.w_image = d.filter_image_stride;
     p.e_shift_base = d.out_exponent - d.in_exponent, p.ew_scalar = d.filter_exponent, p.per_channel = d.per_channel;
     p.relu = d.activation == ESPDL_ACT_RELU, p.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
+    // 2^14 a term: beyond 65536 the sum alone may reach 2^31 and the rounding's half leave 32 bits, which no channel may risk
+    p.acc_bound = p.K <= 65536 ? p.K << 14 : INT_MAX;
     p.early = in_model_scope();
     const bool window = is_window(d);
     const int align = mma_align(d), images = batched ? d.n : 1;
