@@ -27,3 +27,10 @@ load_package()
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: test needs a B200 (run with -m gpu)")
+
+
+def pytest_terminal_summary(terminalreporter):
+    """How many comparisons with the reference's own operators did not take place."""
+    missing = [r for r in terminalreporter.stats.get("skipped", []) if "libespdl_ref.so not built" in str(r.longrepr)]
+    if missing:
+        terminalreporter.write_line(f"{len(missing)} comparisons with the reference's own operators skipped: oracle/_ref/libespdl_ref.so not built")

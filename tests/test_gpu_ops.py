@@ -85,16 +85,14 @@ DW_SHAPES = [
 ]
 
 
-@pytest.mark.parametrize("narrow", [False, True], ids=["auto", "tma-narrow"])
+@pytest.mark.parametrize("tma", [False, True], ids=["auto", "tma"])
 @pytest.mark.parametrize("kw", DW_SHAPES, ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "pad"))
-def test_depthwise_3x3_shapes(kw, narrow, monkeypatch):
+def test_depthwise_3x3_shapes(kw, tma, monkeypatch):
     """The 3x3 depthwise kernels on the network's layer shapes, ragged extents and unusual paddings, against the oracle:
-    the TMA-fed kernel (the default from 64 channels on; with ESPDL_B200_DW_TMA_NARROW=1 also below) and the kernel that
-    reads global memory directly (ESPDL_KERNEL_SIMT).  A depthwise conv has no tensor-core form, so asking for one is
-    refused."""
-    if narrow:
-        if kw["cin"] >= 64:
-            pytest.skip("already on the TMA-fed kernel")
+    the TMA-fed kernel (the default for large layers from 64 channels on; ESPDL_B200_DW_TMA_NARROW=1: for any size and channel
+    count) and the kernel that reads global memory directly (the default below, and ESPDL_KERNEL_SIMT).  A depthwise conv has
+    no tensor-core form, so asking for one is refused."""
+    if tma:
         monkeypatch.setenv("ESPDL_B200_DW_TMA_NARROW", "1")
     case = cases.conv_case(seed=61, depthwise=True, kh=3, kw=3, per_channel=True, e_in=-5, e_out=-5, e_w=(-9, -5), **kw)
     want = gpu_util.run_conv_oracle(case)
@@ -106,7 +104,10 @@ def test_depthwise_3x3_shapes(kw, narrow, monkeypatch):
 
 @pytest.mark.parametrize("round_mode,act,bias,lut", [(abi.ROUND_HALF_EVEN, abi.ACT_RELU, True, False), (abi.ROUND_HALF_UP, abi.ACT_LINEAR, False, False),
                                                      (abi.ROUND_HALF_UP, abi.ACT_RELU, True, True)])
-def test_depthwise_3x3_epilogue_variants(round_mode, act, bias, lut):
+@pytest.mark.parametrize("tma", [False, True], ids=["auto", "tma"])
+def test_depthwise_3x3_epilogue_variants(round_mode, act, bias, lut, tma, monkeypatch):
+    if tma:
+        monkeypatch.setenv("ESPDL_B200_DW_TMA_NARROW", "1")
     case = cases.conv_case(seed=63, n=2, h=19, w=23, cin=80, depthwise=True, kh=3, kw=3, per_channel=True, round_mode=round_mode, act=act,
                            bias=bias, lut=lut, in_stride=96, out_stride=112)
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))

@@ -187,9 +187,9 @@ def test_conv_implicit_gemm_epilogue_variants(round_mode, act, bias, lut, direct
 
 @pytest.mark.parametrize("n,m,k,nout,kernel", [(6, 100, 32, 100, abi.KERNEL_TCGEN05), (3, 400, 400, 64, abi.KERNEL_TCGEN05), (5, 130, 64, 40, abi.KERNEL_AUTO),
                                                (4, 9, 24, 7, abi.KERNEL_AUTO)])
-def test_batched_matrix_products(n, m, k, nout, kernel):
+def test_batched_matrix_products(n, m, k, nout, kernel, monkeypatch):
     """filter_image_stride: image i multiplies by its own filter - all slices of a MatMul in one launch of the tile
-    kernel (the last case, K = 24, takes the one-call-per-image fallback)."""
+    kernel (the last case, K = 24, in one of the CUDA cores); small ones on the warp-level instructions."""
     rng = np.random.default_rng(5)
     case = cases.conv_case(seed=21, n=n, h=1, w=m, cin=k, cout=nout, kh=1, kw=1, pad=(0, 0, 0, 0), per_channel=False, bias=False,
                            act=abi.ACT_LINEAR, e_in=-6, e_w=(-7, -7), e_out=-4)
@@ -201,6 +201,8 @@ def test_batched_matrix_products(n, m, k, nout, kernel):
         one = cases.gemm_case(seed=0, m=m, k=k, n_out=nout, per_channel=False, bias=False, e_in=-6, e_w=(-7, -7), e_out=-4)
         one["x"], one["w"] = np.ascontiguousarray(case["x"][i:i + 1]), np.ascontiguousarray(case["w"][i])
         np.testing.assert_array_equal(gpu_util.run_conv_oracle(one)[0], want[i])
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=kernel), want)
+    monkeypatch.setenv("ESPDL_B200_SMALL_MMA", "0")
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=kernel), want)
 
 
@@ -256,16 +258,20 @@ def test_small_channel_conv_banded_kernel(cin, cout, stride, pad, n, h, w, act, 
     case = cases.conv_case(seed=cin + cout + h, n=n, h=h, w=w, cin=cin, cout=cout, kh=3, kw=3, stride=stride, pad=pad, act=act,
                            per_channel=per_channel, e_in=-6, e_out=-5, e_w=(-9, -7), lut=lut)
     want = gpu_util.run_conv_oracle(case)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), want)
+    # the choice for small layers and the CUDA-core kernels give the same bytes
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
-    # the CUDA-core kernels give the same bytes
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_SIMT), want)
 
 
 @pytest.mark.parametrize("round_mode,lut", [(abi.ROUND_HALF_EVEN, False), (abi.ROUND_HALF_UP, True), (abi.ROUND_HALF_EVEN, True)])
 def test_small_channel_conv_general_epilogue(round_mode, lut):
-    """Half-even rounding takes the banded kernel's general epilogue; a fused table is applied in the staged epilogue."""
-    case = cases.conv_case(seed=3, n=2, h=18, w=22, cin=16, cout=16, kh=3, kw=3, per_channel=True, round_mode=round_mode, lut=lut)
-    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+    """Half-even rounding and a fused table in the banded kernel's staged epilogue, and (a left shift) its general one."""
+    for left in (False, True):
+        case = cases.conv_case(seed=3, n=2, h=18, w=22, cin=16, cout=16, kh=3, kw=3, per_channel=True, round_mode=round_mode, lut=lut)
+        if left:
+            case["ew"][5] = 8
+        np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), gpu_util.run_conv_oracle(case))
 
 
 # Stride-1 windows over 32, 64 or 128 input channels: one input patch per tile, taps as shifted descriptor starts, the
@@ -344,8 +350,8 @@ def test_strided_conv_with_fused_table_and_256_columns(direct, monkeypatch):
 # in its general epilogue.
 CHANNEL_TABLES = [
     dict(n=1, h=1, w=300, cin=64, cout=48, kh=1, kw=1, pad=(0, 0, 0, 0)),            # tile kernel
-    dict(n=2, h=18, w=22, cin=32, cout=48),                                          # implicit GEMM, one MMA per tap
-    dict(n=2, h=20, w=20, cin=64, cout=64),                                          # one patch per tile, stacked taps
+    dict(n=2, h=18, w=22, cin=32, cout=48),                                          # one patch per tile, 48 columns a pixel
+    dict(n=2, h=20, w=20, cin=64, cout=64),                                          # one patch per tile, pixels grouped
     dict(n=2, h=18, w=22, cin=16, cout=16),                                          # banded filter
     dict(n=2, h=48, w=64, cin=3, cout=16, stride=2, pad=(0, 1, 0, 1)),               # first layer
     dict(n=2, h=19, w=23, cin=80, cout=80, depthwise=True),                          # depthwise, TMA patches
@@ -356,14 +362,21 @@ CHANNEL_TABLES = [
 
 @pytest.mark.parametrize("kw", CHANNEL_TABLES, ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "pad"))
 @pytest.mark.parametrize("act", [abi.ACT_LINEAR, abi.ACT_RELU])
-def test_conv_with_per_channel_tables(kw, act):
+@pytest.mark.parametrize("small", [True, False], ids=["auto", "large-layer kernel"])
+def test_conv_with_per_channel_tables(kw, act, small, monkeypatch):
+    """`small`: the choice for layers of this size, else the kernel named beside the shape."""
     kw = dict(kw)
+    kernel = abi.KERNEL_AUTO
+    if not small:
+        kernel = abi.KERNEL_AUTO if kw.get("depthwise") else abi.KERNEL_SIMT if kw["cin"] == 20 else abi.KERNEL_TCGEN05
+        if kw.get("depthwise") and kw["cin"] == 80:
+            monkeypatch.setenv("ESPDL_B200_DW_TMA_NARROW", "1")
     kw.setdefault("kh", 3)
     kw.setdefault("kw", 3)
     case = cases.conv_case(seed=17, per_channel=True, e_in=-7, e_out=-6, e_w=(-9, -7), act=act, lut="channels", **kw)
     want = gpu_util.run_conv_oracle(case)
     assert want.std() > 5
-    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=kernel), want)
     one = dict(case, lut=np.ascontiguousarray(case["lut"][:256]))        # the same conv with the first channel's table for all
     assert not np.array_equal(gpu_util.run_conv_oracle(one), want)
 
