@@ -26,12 +26,13 @@
 // planes, the input's x = 256*hi + lo (hi signed) and the shifted filter's w + 32768 = 256*uh + ul (both unsigned), and the
 // tile kernel accumulates hi*uh, hi*ul + lo*uh and lo*ul in three neighbouring TMEM accumulators: the filter's planes lie one
 // behind the other in shared memory, so ONE instruction of twice the width multiplies hi by both (into accumulators 0, 1)
-// and one multiplies lo by both (into 1, 2) - an M = 128 instruction costs the same for every width up to 256.  The
-// epilogue recombines in 64 bits and takes off 32768 * (sum of the input row).  Exact as long as K <= 16384 (a partial
-// sum stays below 97,665 * K < 2^31).  4096x1024x1024: see the figures at the launch.
+// and one multiplies lo by both (into 1, 2): half the instructions of four separate products, and each wide enough to be bound
+// by its math (max(N/2, 32 + N/4) cycles at M = 128).  The epilogue recombines in two 32-bit halves (requant_wide; 64 bits for
+// shifts outside 1 .. 31) and takes off 32768 * (sum of the input row).  Exact as long as K <= 16384 (a partial sum stays below
+// 97,665 * K < 2^31).  4096x1024x1024 with the packing: 85 us with four products and 64-bit sums, 25 now.
 //
-// Every mbarrier wait is bounded (about two seconds); on expiry the kernel records ESPDL_ERR_TIMEOUT in a device word
-// that espdl_b200_stream_sync reports, and all roles leave.
+// Every mbarrier wait is bounded (about two seconds); on expiry the kernel records ESPDL_ERR_TIMEOUT in the mapped host word
+// (common.cuh) that espdl_b200_stream_sync reports, and all roles leave.
 #include "tc_common.cuh"
 
 #include <mutex>
@@ -524,7 +525,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         bool fast = false;
         const int et0 = (int)threadIdx.x - 64;
         if (!I16) {
-            // only the threads that read (all sixteen warps woken at once cost a lone wave 0.06 us more: 4096x1024x1024 7.85 us read ahead, 7.91, 7.97)
+            // Only the threads that read wait, us a call read ahead / this way / all sixteen warps: 4096x1024x1024 7.85 / 7.91 / 7.97, 28038x1184x76
+            // 14.5 / 15.1.  One wait by the producer and a barrier behind it took 8.2 and 15.3, first loads ahead of the producer's 8.5 and 15.1.
             if (!p.early && (p.epi.lut || et0 < (p.one_tile ? p.block_n : n_pad)))
                 grid_dep_wait();
             EpiConfig epi = p.epi;

@@ -3,11 +3,12 @@
 // ReduceLogSum, ReduceLogSumExp (dl_module_reduce_prod.hpp, dl_module_reduce_log_sum.hpp, dl_module_reduce_log_sum_exp.hpp).
 // Replaces dl::module::ReduceBase::forward_template and the reduce functions of the modules built on it
 // (esp-dl/dl/module/include/dl_module_reduce_base.hpp:121-262, dl_module_reduce_mean.hpp:17-45, dl_module_reduce_sum.hpp:
-// 17-42).  A thread owns one output element and walks the reduced axes; with channels innermost and kept (the usual
-// spatial mean of an NHWC map) neighbouring threads read neighbouring bytes.  Integer sums are exact, so the order
-// of the walk does not matter; the mean's fp32 expression is evaluated in the reference's order.  The floating-point
-// accumulations (the product, the sum of exponentials) are not associative: the walk visits the reduced elements in
-// the reference's order (row-major over the reduced axes), one thread per output.
+// 17-42), and average pools over whole images.  Two kernels.  channel_reduce_kernel: one run of reduced axes between kept ones (the
+// usual spatial mean of an NHWC map) from 2 KB an image on, integer accumulations; pixels shared by the threads of a block and the
+// blocks of a cluster.  reduce_kernel: everything else, a thread owns one output element and walks the reduced axes.  Integer sums
+// are exact, so the order does not matter; the mean's fp32 expression is evaluated in the reference's order.  The floating-point
+// accumulations (the product, the sum of exponentials) are not associative: the walk visits the reduced elements in the reference's
+// order (row-major over the reduced axes), one thread per output.
 #include "common.cuh"
 #include "reduce_plan.cuh"
 
