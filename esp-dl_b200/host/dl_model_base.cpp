@@ -419,7 +419,7 @@ void Model::fuse_blocks()
 // and writes the LUT node's output; the node and the tensor between the two leave the plan.  Exactly the reference's
 // arithmetic: requantise and saturate to the intermediate exponent, then table[(uint8)q ^ 0x80]
 // (esp-dl/dl/base/dl_base_lut.cpp:10-15).  Only convs the tensor-core tile kernels take (input channels a multiple of
-// 16) are folded; ESPDL_B200_FOLD_LUT=0 keeps the nodes.
+// 16) and those of one pixel an image are folded; ESPDL_B200_FOLD_LUT=0 keeps the nodes.
 void Model::fold_luts()
 {
     if (!env_flag("ESPDL_B200_FOLD_LUT", true) || !m_reuse_memory)
@@ -455,7 +455,10 @@ void Model::fold_luts()
         if (!conv || !conv->can_fuse_lut() || !filter || filter->shape.size() != 4)
             continue;
         const bool banded = filter->shape[0] == 3 && filter->shape[1] == 3 && (filter->shape[2] == 3 || filter->shape[2] == 8);
-        if (filter->shape[2] % 16 != 0 && !banded)
+        // gates: one pixel an image, a launch of its own (1.6 us and up) against a few table reads in any conv kernel's epilogue
+        const std::vector<int> shape = m_fbs_model->get_value_info_shape(x);
+        const bool one_pixel = shape.size() == 4 && shape[1] == 1 && shape[2] == 1;
+        if (filter->shape[2] % 16 != 0 && !banded && !one_pixel)
             continue;
         conv->set_fused_lut(lut->release_table(), m_fbs_model->get_value_info_exponent(x));
         m_module_outputs[producer][0] = y;

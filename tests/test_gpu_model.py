@@ -495,6 +495,25 @@ def test_lut_folding_pass(tmp_path, monkeypatch):
     assert len(folded) == len(plain) - (plain.count("Swish") - folded.count("Swish"))
 
 
+def test_gate_tables_fold_whatever_the_channel_count(monkeypatch):
+    """The gates of the re-identification network (one pixel, 4 to 6 channels into the second conv): their Sigmoid tables leave the plan and the outputs
+    stay the same."""
+    path = os.path.join(GOLDEN, "esp32p4__zoo_person_reid.espdl")
+    kinds, outs = [], []
+    for fold in ("1", "0"):
+        monkeypatch.setenv("ESPDL_B200_FOLD_LUT", fold)
+        m = model.Model(path, batch=3)
+        m.inputs[0].array[...] = np.random.default_rng(4).integers(-128, 128, size=m.inputs[0].shape, dtype=np.int8)
+        m.run()
+        kinds.append([r[1] for r in m.profile()])
+        outs.append([np.array(o.array, copy=True) for o in m.outputs])
+        m.close()
+    assert kinds[0].count("Sigmoid") == 0 and kinds[1].count("Sigmoid") == 18
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
+        assert a.std() > 0
+
+
 def test_concat_and_split_as_channel_slices(tmp_path, monkeypatch):
     """The planner places Concat inputs inside the Concat's output and makes Split outputs windows into the Split's input
     wherever the producers / readers take a row stride: fewer bytes move, every tensor still equals the oracle's, and the
