@@ -23,6 +23,7 @@ struct NormParams {
     int op, half_even, len;
     long long rows;
     float in_scale, out_rescale, scale_scale, bias_scale, mean_rescale, inv_std_rescale, epsilon;
+    float one = 1.0f; // see add_product2
 };
 
 // math::sqrt_newton (esp-dl/dl/math/include/dl_math.hpp:83-97); the iteration ends by itself, the cap only bounds it
@@ -245,12 +246,56 @@ __device__ __forceinline__ float code_to_float(uint32_t flipped, int k)
     return __fsub_rn(__uint_as_float(__byte_perm(flipped, 0x4b000000u, k ? 0x7432u : 0x7410u)), 8421376.f);
 }
 
+// Two floats of one instruction: every operation rounds each as the scalar one does, at half the issue slots.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pair(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void split(F2 x, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// a + b where a is a product: with a factor of one that the compiler cannot see, because it contracts packed products and sums, whatever rounding they
+// name (20 of 77 M results differed).
+__device__ __forceinline__ F2 add_product2(F2 a, F2 b, F2 one) { return fma2(a, one, b); }
+
+// Codes k and k + 1 of a word (see code_to_float).
+template <typename T>
+__device__ __forceinline__ F2 codes_to_floats(uint32_t flipped, int k)
+{
+    if (sizeof(T) == 1)
+        return add2(pair(__uint_as_float(__byte_perm(flipped, 0x4b000000u, 0x7440u | (uint32_t)k)), __uint_as_float(__byte_perm(flipped, 0x4b000000u, 0x7441u + (uint32_t)k))),
+                    pair(-8388736.f, -8388736.f));
+    return add2(pair(__uint_as_float(__byte_perm(flipped, 0x4b000000u, 0x7410u)), __uint_as_float(__byte_perm(flipped, 0x4b000000u, 0x7432u))), pair(-8421376.f, -8421376.f));
+}
+
 // LayerNormalization with the rows of a block side by side in shared memory.  The variance is an ordered fp32 sum, so a row
 // costs `len` dependent additions whoever does them; a warp per row made all 32 lanes do the same ones.  Here a thread walks one
 // row (row pitch an odd number of words: thread r reading word i of row r meets no bank conflict), 32 rows of a warp side by
 // side, and the normalising pass gives every thread fixed columns, whose scale and bias stay in registers while it goes
-// down the rows.  Bound by instruction issue (79 % of the slots; 100352 rows of 768: 101 -> 80 us with asynchronous copies in, codes to
-// floats without conversions, all threads in the normalising pass and as many blocks as there are groups of rows).
+// down the rows.  Bound by instruction issue (100352 rows of 768: 101 -> 80 us with asynchronous copies in, codes to floats without conversions, all
+// threads in the normalising pass and as many blocks as there are groups of rows; 80 -> 69 with two elements an instruction).
 // WORDS: rows are whole aligned words in global memory; otherwise the block's rows, one contiguous run of bytes, are dealt out to
 // and collected from the padded rows byte by byte.
 template <typename T, bool WORDS, bool EVEN>
@@ -307,11 +352,17 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
                 const float d = __fsub_rn(x, mean);
                 var = __fadd_rn(var, __fmul_rn(d, d));
             };
+            const F2 minus_mean = pair(-mean, -mean);
 #pragma unroll 4
             for (int i = 0; i < full; i++) {
                 const uint32_t w = row[i] ^ FLIP;
 #pragma unroll
-                for (int k = 0; k < V; k++) add(code_to_float<T>(w, k));
+                for (int k = 0; k < V; k += 2) {
+                    const F2 d = add2(codes_to_floats<T>(w, k), minus_mean);
+                    float a, b;
+                    split(mul2(d, d), a, b);
+                    var = __fadd_rn(__fadd_rn(var, a), b);
+                }
             }
 #pragma unroll
             for (int k = 0; k < V; k++)
@@ -334,24 +385,33 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
         const int first_row = threadIdx.x / across;
         uint32_t *dst = (uint32_t *)((T *)p.out + r0 * p.len);
         for (int cw = threadIdx.x % across; cw < words && first_row < down; cw += across) {
-            float sv[V], bv[V];
+            F2 sv[V / 2], bv[V / 2];
 #pragma unroll
-            for (int k = 0; k < V; k++) {
-                const int e = min(cw * V + k, p.len - 1);
-                sv[k] = sc ? __fmul_rn(__int2float_rn((int)sc[e]), p.scale_scale) : 1.0f;
-                bv[k] = bi ? __fmul_rn(__int2float_rn((int)bi[e]), p.bias_scale) : 0.0f;
+            for (int k = 0; k < V; k += 2) {
+                float s2[2], b2[2];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int e = min(cw * V + k + h, p.len - 1);
+                    s2[h] = sc ? __fmul_rn(__int2float_rn((int)sc[e]), p.scale_scale) : 1.0f;
+                    b2[h] = bi ? __fmul_rn(__int2float_rn((int)bi[e]), p.bias_scale) : 0.0f;
+                }
+                sv[k / 2] = pair(s2[0], s2[1]), bv[k / 2] = pair(b2[0], b2[1]);
             }
+            const F2 in_scale = pair(p.in_scale, p.in_scale), rescale = pair(p.out_rescale, p.out_rescale), half = pair(0.5f, 0.5f), one = pair(p.one, p.one);
 #pragma unroll 2
             for (int rr = first_row; rr < nr; rr += down) {
                 const float2 st = stats[rr];
                 const uint32_t codes = rows_s[rr * pitch + cw] ^ FLIP;
+                const F2 minus_mean = pair(-st.x, -st.x), inv_std = pair(st.y, st.y);
                 int q[V];
 #pragma unroll
-                for (int k = 0; k < V; k++) {
+                for (int k = 0; k < V; k += 2) {
                     // products with a power of two are exact, so a fused multiply-add there rounds as the separate operations do
-                    const float d = __fmaf_rn(code_to_float<T>(codes, k), p.in_scale, -st.x);
-                    const float y = __fadd_rn(__fmul_rn(__fmul_rn(d, st.y), sv[k]), bv[k]);
-                    q[k] = EVEN ? __float2int_rn(__fmul_rn(y, p.out_rescale)) : __float2int_rd(__fmaf_rn(y, p.out_rescale, 0.5f));
+                    const F2 d = fma2(codes_to_floats<T>(codes, k), in_scale, minus_mean);
+                    const F2 y = add_product2(mul2(mul2(d, inv_std), sv[k / 2]), bv[k / 2], one);
+                    float a, b;
+                    split(EVEN ? mul2(y, rescale) : fma2(y, rescale, half), a, b);
+                    q[k] = EVEN ? __float2int_rn(a) : __float2int_rd(a), q[k + 1] = EVEN ? __float2int_rn(b) : __float2int_rd(b);
                 }
                 uint32_t w;
                 if (V == 4) {
