@@ -137,7 +137,7 @@ int espdl_b200_init(int device)
     }
     int *word = nullptr; // the word as the device addresses it
     ESPDL_CUDA_TRY(cudaHostGetDevicePointer((void **)&word, g_error_word, 0));
-    for (int (*bind)(int *) : {bind_device_error, bind_device_error_stem, bind_device_error_band, bind_device_error_dw, bind_device_error_conv,
+    for (int (*bind)(int *) : {bind_device_error, bind_device_error_stem, bind_device_error_band, bind_device_error_dw, bind_device_error_dw_mma, bind_device_error_conv,
                                bind_device_error_block, bind_device_error_dwpw}) {
         const int st = bind(word);
         if (st)
@@ -502,6 +502,17 @@ static long long dw_small(int stride)
     return stride == 1 ? (espdl::in_model_scope() ? 16ll << 20 : 1ll << 20) : (espdl::in_model_scope() ? 2ll << 20 : 256ll << 10);
 }
 
+// Depthwise on the matrix instruction?
+static bool runs_dw_mma(const espdl_conv_desc &d, bool small)
+{
+    const char *knob = getenv("ESPDL_B200_DW_MMA"); // 0: never, always: wherever it can run
+    if (d.kernel != ESPDL_KERNEL_AUTO || (knob && *knob == '0') || getenv("ESPDL_B200_NO_DW_TMA"))
+        return false;
+    if (knob && *knob == 'a')
+        return conv2d_dw_mma_supported(d);
+    return !small && !getenv("ESPDL_B200_DEBUG_WAIT_EXPIRY") && !getenv("ESPDL_B200_DW_TMA_NARROW") && conv2d_dw_mma_pays(d);
+}
+
 // Short windows with few output channels: the CUDA cores where every other kernel would take longer.  The tile kernel's time is that of its waves
 // of 128-pixel tiles, each its taps' loads one after the other and its rows' epilogue (from 2x2 and 3x3 windows of 33 to 540 thousand pixels); the
 // warp-level instructions take about twice their estimate where chunks are words.
@@ -662,13 +673,15 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
         return ESPDL_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if (desc->group != 1) {
-        // Depthwise convs run on the CUDA cores (dp4a)
+        // Depthwise convs have no tensor-core tile kernel
         if (desc->kernel == ESPDL_KERNEL_TCGEN05)
             return ESPDL_ERR_UNSUPPORTED;
-        // 3x3 int8 with 16-byte channel runs: the TMA-fed kernel; ESPDL_KERNEL_SIMT asks for the kernels that read global
+        // 3x3 int8 with 16-byte channel runs: the TMA-fed kernels; ESPDL_KERNEL_SIMT asks for the kernels that read global
         // memory directly, which also run small layers (dw_small)
         const bool small = desc->kernel == ESPDL_KERNEL_AUTO && (long long)desc->n * desc->out_h * desc->out_w * desc->out_c < dw_small(desc->stride_h) && desc->kh == 3 &&
             !getenv("ESPDL_B200_DEBUG_WAIT_EXPIRY") && !getenv("ESPDL_B200_DW_TMA_NARROW");
+        if (runs_dw_mma(*desc, small))
+            return conv2d_dw_mma(*desc, s);
         if (desc->kernel != ESPDL_KERNEL_SIMT && !small && conv2d_dw_tma_supported(*desc))
             return conv2d_dw_tma(*desc, s);
         return conv2d_depthwise(*desc, s);

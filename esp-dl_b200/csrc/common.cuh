@@ -111,6 +111,7 @@ int bind_device_error(int *word);
 int bind_device_error_stem(int *word);
 int bind_device_error_band(int *word);
 int bind_device_error_dw(int *word);
+int bind_device_error_dw_mma(int *word);
 int bind_device_error_conv(int *word);
 int bind_device_error_block(int *word);
 int bind_device_error_dwpw(int *word);
@@ -129,6 +130,9 @@ bool conv2d_conv_tc_supported(const espdl_conv_desc &d);
 int conv2d_conv_tc(const espdl_conv_desc &d, cudaStream_t s);
 bool conv2d_dw_tma_supported(const espdl_conv_desc &d);
 int conv2d_dw_tma(const espdl_conv_desc &d, cudaStream_t s);
+bool conv2d_dw_mma_supported(const espdl_conv_desc &d); // 3x3 at stride 1 on the warp-level matrix instruction (conv_dw_mma.cu)
+bool conv2d_dw_mma_pays(const espdl_conv_desc &d);
+int conv2d_dw_mma(const espdl_conv_desc &d, cudaStream_t s);
 bool conv2d_stem_tc_supported(const espdl_conv_desc &d);
 int conv2d_stem_tc(const espdl_conv_desc &d, cudaStream_t s);
 // 3x3 conv with 8 or 16 input channels: banded-filter tensor-core kernel over 128-byte row windows (conv_band_tc.cu)

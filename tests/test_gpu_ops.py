@@ -113,6 +113,20 @@ def test_depthwise_3x3_epilogue_variants(round_mode, act, bias, lut, tma, monkey
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
 
 
+# stride 1 on the matrix instruction: positions of two pixels in eights, bands of rows in threes, dense rows as runs and channel slices, several
+# images a tile, more tiles than are dealt out in the fixed order, channels that share lines of memory
+@pytest.mark.parametrize("act,round_mode", [(abi.ACT_RELU, abi.ROUND_HALF_UP), (abi.ACT_LINEAR, abi.ROUND_HALF_EVEN)])
+@pytest.mark.parametrize("kw", [
+    dict(n=1, h=1, w=1, cin=16), dict(n=3, h=2, w=3, cin=48), dict(n=1, h=5, w=17, cin=32), dict(n=2, h=31, w=33, cin=32, in_stride=64, out_stride=48),
+    dict(n=37, h=7, w=7, cin=240), dict(n=19, h=9, w=5, cin=128), dict(n=2, h=57, w=58, cin=64), dict(n=130, h=28, w=27, cin=96),
+    dict(n=1, h=3, w=300, cin=16, pad=(3, 0, 2, 5)), dict(n=700, h=14, w=14, cin=32),
+])
+def test_depthwise_matrix_instruction(kw, act, round_mode, monkeypatch):
+    monkeypatch.setenv("ESPDL_B200_DW_MMA", "always")
+    case = cases.conv_case(seed=67 + kw["w"], depthwise=True, kh=3, kw=3, per_channel=True, act=act, round_mode=round_mode, e_in=-5, e_out=-5, e_w=(-9, -5), **kw)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+
+
 def test_depthwise_block_shape():
     """The inverted-residual block's depthwise layer shape: 112x112x192, 3x3 stride 1 (two images)."""
     case = cases.conv_case(seed=43, n=2, h=112, w=112, cin=192, kh=3, kw=3, depthwise=True, per_channel=True, e_in=-5, e_out=-5, e_w=(-9, -5))
