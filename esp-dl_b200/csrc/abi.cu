@@ -561,6 +561,24 @@ static bool runs_mma(const espdl_conv_desc &d)
     return conv2d_mma_estimate_us(d) < min(other, 8.f);
 }
 
+// int16 on the warp-level instructions, where packing and the tile kernel take clearly longer: two launches, the reduction's length, the unrolled
+// rows (windows about twice), the results and the products, from the same 37 layers.  Their rate is a third of the tile kernel's: 4096x1024x1024 25 us
+// there, 66 here.  Results of fewer than 16 channels leave the tile kernel a row at a time (58800x96x8 22.4 / 11.0).
+static bool runs_mma16(const espdl_conv_desc &d)
+{
+    if (d.dtype != ESPDL_DTYPE_INT16 || d.kernel != ESPDL_KERNEL_AUTO || d.n <= 0 || !conv2d_mma16_supported(d))
+        return false;
+    const char *knob = getenv("ESPDL_B200_MMA16"); // 0: never, always: wherever it can run
+    if (knob && (*knob == '0' || *knob == 'a'))
+        return *knob == 'a';
+    if (!conv2d_tc_supported(d) && !conv2d_packed_supported(d))
+        return conv2d_mma16_estimate_us(d) < conv2d_simt_estimate_us(d);
+    const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c;
+    const float tile = 8.0f + 2.5e-3f * K + M * K * (conv2d_tc_supported(d) ? 0.6e-6f : 1.07e-6f) + M * d.out_c * 2.0e-6f + M * K * d.out_c * 1.6e-9f +
+        (d.out_c < 16 ? M * 1.6e-4f : 0.0f);
+    return conv2d_mma16_estimate_us(d) < 0.85f * tile;
+}
+
 // Shapes no kernel reads in place, large enough for packed operands to pay (a caller without the scratch gets the CUDA-core kernel).
 static bool runs_packed(const espdl_conv_desc &d)
 {
@@ -645,7 +663,7 @@ int espdl_b200_conv2d_workspace_bytes(const espdl_conv_desc *desc, size_t *bytes
     int st = conv_validate(desc);
     if (st)
         return st;
-    if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1 || runs_narrow(*desc) || runs_mma(*desc))
+    if (desc->kernel == ESPDL_KERNEL_SIMT || desc->group != 1 || runs_narrow(*desc) || runs_mma(*desc) || (runs_mma16(*desc) && !conv2d_tc_supported(*desc)))
         return ESPDL_OK;
     if (desc->filter_image_stride != 0 && !conv2d_tc_supported(*desc))
         *bytes = one_by_one_bytes(*desc);
@@ -690,6 +708,11 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
         return conv2d_narrow(*desc, s);
     if (runs_mma(*desc))
         return conv2d_mma(*desc, s);
+    if (runs_mma16(*desc)) {
+        // products declare the tile kernel's scratch whichever kernel runs them, and are refused without it
+        const size_t need = conv2d_tc_supported(*desc) ? conv2d_tc_workspace_bytes(*desc) : 0;
+        return need > workspace_bytes || (need && !workspace) ? ESPDL_ERR_INVALID_ARG : conv2d_mma16(*desc, s);
+    }
     if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_stem_tc_supported(*desc))
         return conv2d_stem_tc(*desc, s); // 3x3 stride-2 RGB first layer: banded-filter tensor-core kernel
     if (desc->filter_image_stride != 0) {
@@ -738,6 +761,8 @@ int espdl_b200_conv2d(const espdl_conv_desc *desc, void *stream)
         return st;
     if (need == 0)
         return espdl_b200_conv2d_ws(desc, nullptr, 0, stream);
+    if (g_device >= 0 && runs_mma16(*desc))
+        return conv2d_mma16(*desc, (cudaStream_t)stream);
     std::lock_guard<std::mutex> lock(g_ws_mutex);
     if (!conv2d_tc_supported(*desc)) { // the CUDA cores run it as it is, the scratch only makes it faster
         StreamScratch *scratch = stream_scratch((cudaStream_t)stream, need);

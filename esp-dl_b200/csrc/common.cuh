@@ -104,6 +104,10 @@ int conv2d_packed(const espdl_conv_desc &d, void *workspace, size_t workspace_by
 bool conv2d_mma_supported(const espdl_conv_desc &d);
 float conv2d_mma_estimate_us(const espdl_conv_desc &d);
 int conv2d_mma(const espdl_conv_desc &d, cudaStream_t s);
+// The same for int16, split into byte planes in registers (conv_mma16.cu).
+bool conv2d_mma16_supported(const espdl_conv_desc &d);
+float conv2d_mma16_estimate_us(const espdl_conv_desc &d);
+int conv2d_mma16(const espdl_conv_desc &d, cudaStream_t s);
 // Each translation unit with bounded device-side waits keeps the address of ONE status word in pinned, device-mapped host
 // memory: a wait that runs out stores ESPDL_ERR_TIMEOUT there, and espdl_b200_stream_sync reads it as ordinary memory.
 // (A device word per unit, copied back at every synchronisation, cost seven blocking copies: 60 us of a 160 us pass.)

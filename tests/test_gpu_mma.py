@@ -95,3 +95,37 @@ def test_reductions_beyond_65536_terms(sign, act, forced):
     want = gpu_util.run_conv_oracle(case)
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
     assert want.max() == (127 if sign > 0 else 0 if act == abi.ACT_RELU else -128)
+
+
+# int16 on byte planes: ragged reductions (runs of 64), pixels and channels around the tiles' edges, windows that leave the image on every side
+SHAPES16 = [
+    dict(n=4, h=40, w=40, cin=64, cout=64),
+    dict(n=1, h=1, w=1, cin=8, cout=1, **P0),
+    dict(n=1, h=1, w=65, cin=72, cout=33, **P0),
+    dict(n=3, h=9, w=7, cin=24, cout=31, stride=2),
+    dict(n=1, h=13, w=8, cin=16, cout=66, kh=5, kw=3, dil=2, pad=(4, 4, 2, 2)),
+    dict(n=2, h=6, w=9, cin=40, cout=45, in_stride=56, out_stride=47),
+    dict(n=1, h=1, w=33, cin=16384, cout=32, **P0),
+    dict(n=40, h=20, w=20, cin=64, cout=64, **P0),
+]
+
+
+@pytest.mark.parametrize("act,round_mode", [(abi.ACT_RELU, abi.ROUND_HALF_UP), (abi.ACT_LINEAR, abi.ROUND_HALF_EVEN)])
+@pytest.mark.parametrize("i", range(len(SHAPES16)))
+def test_conv_int16(i, act, round_mode, monkeypatch):
+    monkeypatch.setenv("ESPDL_B200_MMA16", "always")
+    case = cases.conv_case(seed=20 + i, dtype=abi.DTYPE_INT16, per_channel=True, act=act, round_mode=round_mode, e_in=-13, e_out=-5, e_w=(-14, -11), **SHAPES16[i])
+    want = gpu_util.run_conv_oracle(case)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+    assert want.size < 8 or want.std() > 0
+
+
+@pytest.mark.parametrize("e_w", [(-60, -30), (-1, 3), (20, 40)])
+def test_conv_int16_ends_of_the_range_and_any_shift(e_w, monkeypatch):
+    """Every element at an end of the type, so that each plane's sum is as large as it gets; shifts from far left to beyond the sum."""
+    monkeypatch.setenv("ESPDL_B200_MMA16", "always")
+    case = cases.conv_case(seed=5, dtype=abi.DTYPE_INT16, n=1, h=4, w=9, cin=16384, cout=34, per_channel=True, e_in=0, e_out=0, e_w=e_w, act=abi.ACT_LINEAR, **P0)
+    rng = np.random.default_rng(5)
+    case["x"][...] = np.where(rng.random((1, 4, 9, 1)) < 0.5, -32768, 32767)
+    case["w"][...] = np.where(rng.random((34, 1, 1, 1)) < 0.5, -32768, 32767)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
