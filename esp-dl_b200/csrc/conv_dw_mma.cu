@@ -25,8 +25,8 @@
 //   the others  consumers, in teams that take the tiles in turn: a warp owns 16 channels and walks groups of 8 positions down a band of rows, writing the
 //               requantised words into an output tile in shared memory.
 // Bound by the latency of a warp's walk, some 260 cycles a row with three or four warps a scheduler (matrix pipe 40 %, issue slots 45 % busy); loads and
-// stores alone run at the copy bandwidth.  1024 images, dp4a before and now, us: 112x112x32 207 -> 171, 28x28x192 83 -> 77, 14x14x384 54 -> 43,
-// 14x14x576 75 -> 63, 7x7x960 44 -> 34.  Where tiles' channel blocks share lines of memory they follow one another (fetched twice otherwise: 28x28x192
+// stores alone run at the copy bandwidth.  1024 images, dp4a before and now, us: 112x112x32 207 -> 165, 28x28x192 83 -> 75, 14x14x384 54 -> 41,
+// 14x14x576 75 -> 60, 7x7x960 44 -> 30.  Where tiles' channel blocks share lines of memory they follow one another (fetched twice otherwise: 28x28x192
 // could not be below 78), and with two stages a tile waited half its time for its load.
 // A fragment load is 16 bytes of 6 pixels to a quarter warp: without bank conflicts where CB / 16 is odd, two-way for 32 and 96,
 // and never a multiple of 128 (dwm_plan).
@@ -58,7 +58,7 @@ constexpr int DWM_MAX_CONSUMER_WARPS = 15; // with the producer's four warps a s
 constexpr int DWM_MAX_THREADS = (DWM_MAX_CONSUMER_WARPS + 1) * 32;
 constexpr int DWM_MAX_STAGES = 8, DWM_MAX_TEAMS = 7;
 constexpr int DWM_RING = 16; // tile numbers on their way from the producer to the consumers (more than stages and teams together)
-constexpr int DWM_BARRIER_BYTES = 8 * (DWM_MAX_STAGES + 4 * DWM_MAX_TEAMS) + 4 + 4 * DWM_RING + 12;
+constexpr int DWM_BARRIER_BYTES = 8 * (DWM_MAX_STAGES + 4 * DWM_MAX_TEAMS) + 4 + 8 * DWM_RING + 12;
 constexpr size_t DWM_SMEM_BUDGET = 220 * 1024;
 
 // Where the filter and the requantisation constants come from.
@@ -268,7 +268,8 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     // a patch is there; all of a team have computed their part of an output tile; it has left
     uint64_t *full_bar = bars, *done_bar = full_bar + DWM_MAX_STAGES, *free_bar = done_bar + 2 * DWM_MAX_TEAMS;
     volatile int *abort_flag = (volatile int *)(free_bar + 2 * DWM_MAX_TEAMS);
-    volatile int *tile_ring = abort_flag + 1; // DWM_RING tile numbers, producer -> consumers (published by the "full" arrive)
+    volatile int *block_ring = abort_flag + 1; // DWM_RING tiles' channel blocks, -1 behind the last, producer -> consumers (published by the "full" arrive)
+    volatile int *tile_ring = block_ring + DWM_RING; // and their numbers, for the producer's stores
     int2 *position = (int2 *)((uint8_t *)bars + DWM_BARRIER_BYTES); // of every position: bytes into the patch, and into the output tile (-1: padding, odd: one pixel)
     uint8_t *nowhere = out0 + (size_t)NO * p.out_bytes - 16; // results of padding
 
@@ -280,7 +281,7 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             mbar_init(smem_u32(&free_bar[s]), 1);
         }
         *abort_flag = 0;
-        for (int i = 0; i < DWM_RING; i++) tile_ring[i] = 0; // never negative before the producer says so
+        for (int i = 0; i < DWM_RING; i++) block_ring[i] = 0; // never negative before the producer says so
         fence_barrier_init();
     }
     if (threadIdx.x == 32) {
@@ -329,7 +330,7 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             const bool more = next < p.total_tiles;
             if (elect_one()) {
                 const uint32_t bar = smem_u32(&full_bar[s]), to = smem_u32(patch0 + (size_t)s * p.stage_bytes);
-                tile_ring[i & (DWM_RING - 1)] = more ? next : -1;
+                block_ring[i & (DWM_RING - 1)] = more ? next_at.cb : -1, tile_ring[i & (DWM_RING - 1)] = next;
                 if (more) {
                     mbar_arrive_expect_tx(bar, (uint32_t)p.tx_bytes);
                     if (p.flat)
@@ -416,10 +417,9 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             if (lane == 0)
                 report_timeout(g_dwm_error);
         }
-        const int t = tile_ring[i & (DWM_RING - 1)];
-        if (*abort_flag || t < 0)
+        const int cb = block_ring[i & (DWM_RING - 1)];
+        if (*abort_flag || cb < 0)
             break;
-        const int t_in_cb = t / p.cblocks, cb = t - t_in_cb * p.cblocks;
         const int c0 = cb * CB + 16 * cb16;
         if (cb != have_cb) {
             dwm_load_consts<EVEN>(k, p.src, c0, g, t4);
@@ -642,8 +642,9 @@ int conv2d_dw_mma(const espdl_conv_desc &d, cudaStream_t s)
     const size_t smem = dwm_smem_bytes(p);
     const int sms = num_sms() >= 2 * p.cblocks ? num_sms() / p.cblocks * p.cblocks : num_sms(); // a CTA keeps to one channel block and its constants
     const int grid = min(p.total_tiles, sms);
-    // three quarters of the tiles in the fixed order, the last quarter to whichever SM is free
-    p.sched = p.total_tiles >= 4 * grid ? sched_counters(s) : nullptr;
+    // three quarters of the tiles in the fixed order, the last quarter to whichever SM is free; with several channel blocks a tile handed out would mostly be
+    // another block's, whose constants take longer to load than the slow SMs lose (7x7x960 32.8 us, 29.9 in the fixed order)
+    p.sched = p.total_tiles >= 4 * grid && p.cblocks == 1 ? sched_counters(s) : nullptr;
     p.static_tiles = p.sched ? (int)((long long)p.total_tiles * 3 / 4 / grid) * grid : p.total_tiles;
     return dwm_launch(mi, mo, p, smem, grid, s);
 }
