@@ -410,7 +410,7 @@ def roofline_of(m, parsed, batch):
     peaks = measured_peaks()
     peak = float(peaks.get("hbm_gbs", 6650.0))
     achieved = dom["bytes"] / (dom["us"] * 1e-6) / 1e9
-    kernel_names = {"pointwise_tc": "gemm_tc_kernel", "depthwise": "dw3x3_tma_kernel", "conv_simt": "stem_tc_kernel",
+    kernel_names = {"pointwise_tc": "gemm_tc_kernel", "depthwise": "dw3x3_mma_kernel, dw3x3_tma_kernel", "conv_simt": "stem_tc_kernel",
                     "depthwise_pointwise_fused": "dwpw_kernel"}
     # DRAM bytes moved per algorithmic byte, from one profiler capture of each kernel on a layer larger than L2
     # (profiles/): the launches of a step differ in shape, so the per-launch traffic is that ratio applied to

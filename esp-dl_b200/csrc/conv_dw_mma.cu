@@ -607,7 +607,7 @@ bool conv2d_dw_mma_supported(const espdl_conv_desc &d)
 bool conv2d_dw_mma_pays(const espdl_conv_desc &d)
 {
     DwmParams p;
-    if (!conv2d_dw_mma_supported(d) || !dwm_plan(d, p) || p.CB % 64 == 0)
+    if (d.lut || !conv2d_dw_mma_supported(d) || !dwm_plan(d, p) || p.CB % 64 == 0) // a table is the general form's, whose loops have more threads on dp4a
         return false;
     return p.flat && d.in_c < 64 ? true : p.CB >= 80 && (long long)d.n * d.out_h * d.out_w * d.in_c >= 32ll << 20;
 }
