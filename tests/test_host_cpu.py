@@ -411,3 +411,91 @@ def test_tile_counters_are_given_back(tmp_path):
     subprocess.check_call(["g++", "-O2", "-std=c++17", "-I" + csrc, str(src), "-o", str(tmp_path / "counters")])
     r = subprocess.run([str(tmp_path / "counters")], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+DEPTHWISE_PLANS_PROGRAM = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "dw_mma_plan.cuh"
+int main()
+{
+    for (int C = 16; C <= 1024; C += C < 256 ? 16 : 96)
+        for (int hw : {1, 3, 7, 10, 14, 20, 28, 46, 56, 83, 112})
+            for (int n : {1, 3, 16, 64, 317, 1024}) {
+                const espdl::DwmParams p = espdl::dwm_search(C, hw, hw + (n & 1) * (hw / 8), n, C % 32 == 0 || C < 128, 148);
+                if (p.nw && ((size_t)p.stages * p.stage_bytes == 0 || espdl::dwm_smem_bytes(p) > espdl::DWM_SMEM_BUDGET || p.nw * p.teams > espdl::DWM_MAX_CONSUMER_WARPS))
+                    return fprintf(stderr, "%d images of %dx%d: teams %d stages %d\n", n, hw, C, p.teams, p.stages), 1;
+                if (p.nw)
+                    printf("%d %d\n", p.teams, p.stages);
+            }
+    for (auto &l : {std::initializer_list<int>{64, 112, 112, 16}, {117, 46, 45, 240}, {676, 62, 59, 16}, {317, 52, 51, 48}}) {
+        const int *d = l.begin();
+        const espdl::DwmParams p = espdl::dwm_search(d[3], d[1], d[2], d[0], true, 148);
+        printf("%d %d\n", p.teams, p.stages);
+    }
+    return 0;
+}
+"""
+
+
+def tile_read_before_it_landed(teams, stages, waits, tiles=40):
+    """The barriers of dw3x3_mma_kernel (conv_dw_mma.cu) with one load that takes as long as it can: everything else goes as far as it gets, then that
+    load lands and those issued behind it are on their way.  The first tile that a team computes from a patch that is not there, or None.
+    `waits`: a team's two waits, one after the other."""
+    out = 2 * teams  # output tiles
+
+    def passed(completed, phase):  # mbarrier.try_wait.parity
+        return completed & 1 != phase & 1
+
+    for slow in range(tiles):
+        full, free, done, landed = [0] * stages, [0] * out, [0] * out, set()
+        stored, at, step = 0, list(range(teams)), [0] * teams  # the producer's tile, each team's and the waits it has behind it there
+        for arrives in (lambda i: i != slow, lambda i: False):
+
+            def load(i):
+                if i < tiles and arrives(i):
+                    landed.add(i)
+                    full[i % stages] += 1
+
+            if stored == 0 and not landed:
+                for i in range(stages):
+                    load(i)
+            elif slow < stored + stages:
+                landed.add(slow)
+                full[slow % stages] += 1
+            moved = True
+            while moved:
+                moved = False
+                if stored < tiles and passed(done[stored % out], stored // out):
+                    load(stored + stages)
+                    free[stored % out] += 1
+                    stored, moved = stored + 1, True
+                for t in range(teams):
+                    i = at[t]
+                    if i >= tiles:
+                        continue
+                    if step[t] < 2 and (passed(full[i % stages], i // stages) if waits[step[t]] == "full" else passed(free[i % out], i // out + 1)):
+                        step[t], moved = step[t] + 1, True
+                    if step[t] == 2:
+                        if i not in landed:
+                            return i
+                        done[i % out] += 1
+                        at[t], step[t], moved = i + teams, 0, True
+    return None
+
+
+def test_depthwise_teams_never_compute_from_a_patch_on_its_way(tmp_path):
+    """Every (teams, stages) that the planner comes to, with any one load as slow as can be.  Waiting for the patch first was unsound wherever the
+    stages are no multiple of the teams."""
+    src = tmp_path / "plans.cpp"
+    src.write_text(DEPTHWISE_PLANS_PROGRAM)
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "esp-dl_b200", "csrc")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-I" + csrc, str(src), "-o", str(tmp_path / "plans")])
+    r = subprocess.run([str(tmp_path / "plans")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    plans = {tuple(map(int, line.split())) for line in r.stdout.splitlines()}
+    assert any(t > 1 and s % t for t, s in plans)
+    for teams, stages in sorted(plans):
+        assert tile_read_before_it_landed(teams, stages, ("free", "full")) is None, (teams, stages)
+    kernel = open(os.path.join(csrc, "conv_dw_mma.cu")).read()
+    assert kernel.index("mbar_wait(smem_u32(&free_bar[o])") < kernel.index("mbar_wait(smem_u32(&full_bar[s])")  # the order that is modelled
