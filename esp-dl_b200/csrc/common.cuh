@@ -134,6 +134,7 @@ bool conv2d_conv_tc_supported(const espdl_conv_desc &d);
 int conv2d_conv_tc(const espdl_conv_desc &d, cudaStream_t s);
 bool conv2d_dw_tma_supported(const espdl_conv_desc &d);
 int conv2d_dw_tma(const espdl_conv_desc &d, cudaStream_t s);
+bool conv2d_dw_tma_whole(const espdl_conv_desc &d); // its tiles have all channels of a pixel
 bool conv2d_dw_mma_supported(const espdl_conv_desc &d); // 3x3 at stride 1 on the warp-level matrix instruction (conv_dw_mma.cu)
 bool conv2d_dw_mma_pays(const espdl_conv_desc &d);
 int conv2d_dw_mma(const espdl_conv_desc &d, cudaStream_t s);

@@ -462,6 +462,8 @@ bool dwm_plan(const espdl_conv_desc &d, DwmParams &p)
     p = dwm_search(d.in_c, d.out_h, d.out_w, d.n, dense, num_sms());
     {
         std::lock_guard<std::mutex> lock(mu);
+        if (memo.size() >= 4096)
+            memo.clear();
         memo[key] = p;
     }
     return p.nw > 0;
@@ -500,16 +502,14 @@ bool conv2d_dw_mma_supported(const espdl_conv_desc &d)
     return dwm_plan(d, p);
 }
 
-// Large layers: in a tile of 64 channels the pixels' banks collide (300 of 20x20x256: 26.5 us, 21.0 on dp4a), narrower ones that are not dense rows are
-// the TMA unit's short runs, and below some 32 M outputs the ring's start costs what the walk saves (64 of 57x58x96 15.6 / 13.8, 256 of 7x7x960
-// 15.8 / 14.6; 1024 of them 33.8 / 44).  Dense rows of few channels, which dp4a reads straight from global memory: 1024 of 112x112x32 171 / 207,
-// 100 of 28x28x16 4.5 / 6.0.
 bool conv2d_dw_mma_pays(const espdl_conv_desc &d)
 {
-    DwmParams p;
-    if (d.lut || !conv2d_dw_mma_supported(d) || !dwm_plan(d, p) || p.CB % 64 == 0) // a table is the general form's, whose loops have more threads on dp4a
+    // the size before the search for a plan; a table is the general form's, whose loops have more threads on dp4a
+    if (d.lut || !dwm_large(d.in_c, (long long)d.n * d.out_h * d.out_w * d.in_c) || !conv2d_dw_mma_supported(d))
         return false;
-    return p.flat && d.in_c < 64 ? true : p.CB >= 80 && (long long)d.n * d.out_h * d.out_w * d.in_c >= 32ll << 20;
+    DwmParams p;
+    auto pays = [&](bool whole) { return dwm_pays(p, d.in_c, d.out_h, d.out_w, d.n, d.round_mode == ESPDL_ROUND_HALF_EVEN, whole, num_sms()); };
+    return dwm_plan(d, p) && (pays(true) || (pays(false) && !conv2d_dw_tma_whole(d))); // dp4a's plan only where it decides
 }
 
 int conv2d_dw_mma(const espdl_conv_desc &d, cudaStream_t s)
@@ -540,8 +540,7 @@ int conv2d_dw_mma(const espdl_conv_desc &d, cudaStream_t s)
     if (!encode(&mi, const_cast<void *>(d.input), d.in_w, d.in_h, ips, p.IW, p.IH) || !encode(&mo, d.output, d.out_w, d.out_h, ops, p.TW, p.TH))
         return set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled(depthwise)");
     const size_t smem = dwm_smem_bytes(p);
-    const int sms = num_sms() >= 2 * p.cblocks ? num_sms() / p.cblocks * p.cblocks : num_sms(); // a CTA keeps to one channel block and its constants
-    const int grid = min(p.total_tiles, sms);
+    const int grid = dwm_grid(p, num_sms());
     // three quarters of the tiles in the fixed order, the last quarter to whichever SM is free; with several channel blocks a tile handed out would mostly be
     // another block's, whose constants take longer to load than the slow SMs lose (7x7x960 32.8 us, 29.9 in the fixed order)
     p.sched = p.total_tiles >= 4 * grid && p.cblocks == 1 ? sched_counters(s) : nullptr;

@@ -406,6 +406,12 @@ bool conv2d_dw_tma_supported(const espdl_conv_desc &d)
     return dwt_plan(d, p);
 }
 
+bool conv2d_dw_tma_whole(const espdl_conv_desc &d)
+{
+    DwtParams p;
+    return d.in_c <= 256 && conv2d_dw_tma_supported(d) && dwt_plan(d, p) && p.CB == d.in_c;
+}
+
 int conv2d_dw_tma(const espdl_conv_desc &d, cudaStream_t s)
 {
     DwtParams p;

@@ -121,4 +121,53 @@ inline DwmParams dwm_search(int C, int out_h, int out_w, int n, bool dense, int 
     return best;
 }
 
+// CTAs of a launch: a CTA keeps to one channel block and its constants.
+inline int dwm_grid(const DwmParams &p, int sms)
+{
+    return std::min(p.total_tiles, sms >= 2 * p.cblocks ? sms / p.cblocks * p.cblocks : sms);
+}
+
+// What a launch takes, us.  Beside the terms of dwm_shape there are the producer's turn (1700 cycles a tile: the wait for a tile's end, its store, the next
+// load, one after the other), the hand-over, the constants where a CTA's next tile is another block's, and the SMs that whole channel blocks leave idle;
+// the norm stands for terms that meet.  Fitted to 2000 layers of 16 to 6000 channels, which it meets to within 5 % (standard deviation) from 32 M
+// outputs on; of smaller ones the previous kernel hides up to 4 us.
+inline double dwm_estimate_us(const DwmParams &p, int sms)
+{
+    const int rounds = (p.groups + p.wpc - 1) / p.wpc, run = (p.CB + 127) / 128, ctas = dwm_grid(p, sms);
+    const double walks = (double)p.groups * p.ncb, in = p.tx_bytes, out = (double)p.NB * p.TH * p.TW * p.CB;
+    const double runs = p.NB * (p.flat ? p.IH * ((p.IW * p.CB + 127) / 128) + p.TH * ((p.TW * p.CB + 127) / 128) : (p.IH * p.IW + p.TH * p.TW) * run);
+    double sum = 0;
+    for (double x : {walks * (p.RB * 57.0 + 50.0) / 2.4, rounds * (p.RB * 250.0 + 285.0) / p.teams, walks * p.RB * 12.0, 0.026 * in + 0.067 * out, 3.5 * runs,
+                     3400.0 / (p.stages - p.teams), 1700.0}) {
+        x *= x, x *= x, x *= x;
+        sum += x * x;
+    }
+    const double tile = sqrt(sqrt(sqrt(sqrt(sum)))) + 400.0 + (ctas % p.cblocks ? 900.0 : 0.0);
+    return 6.7 + ((double)p.total_tiles / ctas + 0.5) * tile / 1965.0;
+}
+
+// Large enough to be planned at all: below some 32 M outputs the ring's start costs what the walk saves (64 of 57x58x96 15.6 / 13.8, 256 of 7x7x960
+// 15.8 / 14.6; 1024 of them 33.8 / 44), except in narrow tensors, whose rows are few runs here and which dp4a reads straight from global memory.
+inline bool dwm_large(int C, long long outputs) { return C < 64 || outputs >= 32ll << 20; }
+
+// The planned launch against dp4a.  In a tile of 64 channels the pixels' banks collide (300 of 20x20x256: 26.5 us, 21.0 on dp4a), and narrower ones that are not
+// dense rows are the TMA unit's short runs.  For the others dp4a's time, from 2200 layers: 0.45 ps an output for 96 channels and 0.51 for other widths
+// that its tile takes whole (`dp4a_whole`), a quarter more for images below 200 pixels; 0.7 and more where it cuts pixels up; 0.49 for narrow tensors, more
+// for small images and for 16 channels (0.6 to 0.9, never less than here).  us here / there: 619 of 20x20x144 28.6 / 22.6, 928 of 20x20x96 29.8 / 22.1, 650 of
+// 28x28x144 45.3 / 41.1, 1024 of 80x80x48 201 / 170, 104 of 28x27x4000 231 / 219; 1024 of 112x112x32 171 / 207, 3715 of 14x14x144 60.8 / 67.0.  Half to
+// even is 29 % slower here and 16 % there (160 of 57x56x144 55.9 / 50.3, half up 43.4 both).  Narrow tensors
+// below 64 M outputs stay here, whichever way the estimate falls (mostly 0.7 to 1.0 of dp4a's time, in eight of 155 layers 1.05 to 1.24).
+inline bool dwm_pays(const DwmParams &p, int C, int out_h, int out_w, int n, bool half_even, bool dp4a_whole, int sms)
+{
+    const double outputs = (double)n * out_h * out_w * C, pixels = (double)out_h * out_w;
+    if (p.nw == 0 || p.CB % 64 == 0 || (C < 64 ? !p.flat : p.CB < 80))
+        return false;
+    const double us = dwm_estimate_us(p, sms) * (half_even ? 1.1 : 1.0);
+    if (C < 64)
+        return C == 16 || pixels <= 200 || outputs < (64 << 20) || us < 8.0 + 0.49e-6 * outputs;
+    if (dp4a_whole)
+        return us < 5.5 + (C == 96 ? 0.45e-6 : 0.51e-6) * (pixels <= 200 ? 1.25 : 1.0) * outputs;
+    return us < 8.0 + 0.7e-6 * (pixels <= 200 ? 1.12 : 1.0) * outputs;
+}
+
 } // namespace espdl

@@ -499,3 +499,39 @@ def test_depthwise_teams_never_compute_from_a_patch_on_its_way(tmp_path):
         assert tile_read_before_it_landed(teams, stages, ("free", "full")) is None, (teams, stages)
     kernel = open(os.path.join(csrc, "conv_dw_mma.cu")).read()
     assert kernel.index("mbar_wait(smem_u32(&free_bar[o])") < kernel.index("mbar_wait(smem_u32(&full_bar[s])")  # the order that is modelled
+
+
+DEPTHWISE_CHOICE_PROGRAM = r"""
+#include <cstdio>
+#include "dw_mma_plan.cuh"
+int main()
+{
+    int C, h, w, n, even, whole;
+    while (scanf("%d %d %d %d %d %d", &C, &h, &w, &n, &even, &whole) == 6)
+        printf("%d\n", espdl::dwm_large(C, (long long)n * h * w * C) && espdl::dwm_pays(espdl::dwm_search(C, h, w, n, true, 148), C, h, w, n, even, whole, 148));
+    return 0;
+}
+"""
+
+# images, height, width, channels, does the dp4a kernel's tile take whole pixels; us on the matrix instruction and on dp4a
+DEPTHWISE_TIMES = [
+    (1024, 112, 112, 32, 0, 171, 207), (1024, 56, 56, 144, 1, 209, 217), (1024, 28, 28, 192, 0, 75, 83), (1024, 14, 14, 384, 0, 41, 54), (1024, 14, 14, 576, 0, 60, 75),
+    (1024, 7, 7, 960, 0, 30, 44), (3715, 14, 14, 144, 1, 60.8, 67.0), (18725, 7, 7, 80, 1, 43.6, 54.7), (218453, 5, 9, 32, 0, 170, 282), (1274, 20, 20, 144, 0, 51, 147),
+    (619, 20, 20, 144, 1, 28.6, 22.6), (2731, 20, 20, 144, 1, 101.7, 82.3), (928, 20, 20, 96, 1, 29.8, 22.1), (1365, 20, 20, 96, 1, 41.9, 29.7),
+    (650, 28, 28, 144, 1, 45.3, 41.1), (1024, 80, 80, 48, 0, 201, 170), (3080, 57, 56, 32, 0, 178, 156), (104, 28, 27, 4000, 0, 231, 219), (64, 57, 58, 96, 1, 15.6, 13.8),
+]
+DEPTHWISE_TIMES_HALF_EVEN = [(160, 57, 56, 144, 1, 55.9, 50.3), (41, 112, 112, 144, 1, 52.5, 48.1)]
+
+
+def test_depthwise_layers_take_the_faster_kernel(tmp_path):
+    """Layers beside the line between the two kernels, as measured: wide images of 20 to 28 pixels, tiles of short walks and layers whose channel blocks leave
+    SMs idle were sent to the slower one."""
+    src = tmp_path / "choice.cpp"
+    src.write_text(DEPTHWISE_CHOICE_PROGRAM)
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "esp-dl_b200", "csrc")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-I" + csrc, str(src), "-o", str(tmp_path / "choice")])
+    layers = [(0, layer) for layer in DEPTHWISE_TIMES] + [(1, layer) for layer in DEPTHWISE_TIMES_HALF_EVEN]
+    lines = "\n".join(f"{c} {h} {w} {n} {even} {whole}" for even, (n, h, w, c, whole, _, _) in layers)
+    got = subprocess.run([str(tmp_path / "choice")], input=lines, capture_output=True, text=True).stdout.split()
+    for (_, layer), choice in zip(layers, got, strict=True):
+        assert (choice == "1") == (layer[5] < layer[6]), layer
