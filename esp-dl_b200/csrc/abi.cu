@@ -561,9 +561,11 @@ static bool runs_mma(const espdl_conv_desc &d)
     return conv2d_mma_estimate_us(d) < min(other, 8.f);
 }
 
-// int16 on the warp-level instructions, where packing and the tile kernel take clearly longer: two launches, the reduction's length, the unrolled
-// rows (windows about twice), the results and the products, from the same 37 layers.  Their rate is a third of the tile kernel's: 4096x1024x1024 25 us
-// there, 66 here.  Results of fewer than 16 channels leave the tile kernel a row at a time (58800x96x8 22.4 / 11.0).
+// int16 on the warp-level instructions, where the other kernels take longer.  Packing and the tile kernel: two launches, the reduction's length, the
+// unrolled rows (windows about twice), the results and the products, from 37 layers, 20 % (standard deviation) off 380 others.  The
+// products' rate is a third of theirs: 4096x1024x1024 25 us there, 66 here; 45 of 11x11x256 -> 80, 3x3 22 / 37.  Results of fewer than 16 channels leave the tile kernel a row at a time
+// (58800x96x8 22.4 / 11.0).  Eight-element reductions are padded to 64 here, and the CUDA cores read them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
+// 6.0; 1088x8x192 8.9 / 3.8).
 static bool runs_mma16(const espdl_conv_desc &d)
 {
     if (d.dtype != ESPDL_DTYPE_INT16 || d.kernel != ESPDL_KERNEL_AUTO || d.n <= 0 || !conv2d_mma16_supported(d))
@@ -571,12 +573,13 @@ static bool runs_mma16(const espdl_conv_desc &d)
     const char *knob = getenv("ESPDL_B200_MMA16"); // 0: never, always: wherever it can run
     if (knob && (*knob == '0' || *knob == 'a'))
         return *knob == 'a';
-    if (!conv2d_tc_supported(d) && !conv2d_packed_supported(d))
-        return conv2d_mma16_estimate_us(d) < conv2d_simt_estimate_us(d);
-    const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c;
-    const float tile = 8.0f + 2.5e-3f * K + M * K * (conv2d_tc_supported(d) ? 0.6e-6f : 1.07e-6f) + M * d.out_c * 2.0e-6f + M * K * d.out_c * 1.6e-9f +
+    const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c, us = conv2d_mma16_estimate_us(d);
+    const bool product = conv2d_tc_supported(d);
+    if (!product && !conv2d_packed_supported(d))
+        return us < (K <= 8 && d.out_c <= 64 ? 2.9f + M * K * d.out_c / 1.3e6f : conv2d_simt_estimate_us(d));
+    const float tile = 8.0f + 2.5e-3f * K + M * K * (product ? 0.6e-6f : 1.07e-6f) + M * d.out_c * 2.0e-6f + M * K * d.out_c * 1.6e-9f +
         (d.out_c < 16 ? M * 1.6e-4f : 0.0f);
-    return conv2d_mma16_estimate_us(d) < 0.85f * tile;
+    return us < 0.97f * tile;
 }
 
 // Shapes no kernel reads in place, large enough for packed operands to pay (a caller without the scratch gets the CUDA-core kernel).

@@ -210,22 +210,29 @@ struct Mma16Plan {
     float us;
 };
 
-// The tile with the least estimated time, from 37 layers of 16 to 200 thousand pixels: waves of as many blocks as an SM holds, each its start, its
-// results, and its runs, which take their share of the matrix instructions or the latency of copies and fragments (4 of 40x40x64 -> 64, 3x3:
-// 13.2 us with 64 x 64, 10.2 with 64 x 32, 12.0 with 32 x 32; 400x1152x128 14.5, 10.6, 7.9; 102400x576x64 70, 88, 112).
+// The tile by waves of as many blocks as an SM holds, each its start, its results, and its runs, which take their share of the matrix instructions or the
+// latency of copies and fragments (4 of 40x40x64 -> 64, 3x3: 13.2 us with 64 x 64, 10.2 with 64 x 32, 12.0 with 32 x 32; 400x1152x128 14.5, 10.6, 7.9;
+// 102400x576x64 70, 88, 112).  Its time for the choice against the other kernels by what 500 layers took in the tile that they get, inputs in L2 and not:
+// launch, a wave's start, what a block and a run cost beside others and alone; within 12 % (standard deviation).
 Mma16Plan mma16_plan(const espdl_conv_desc &d)
 {
     static const struct {
         int bm, bn, resident;
-        float start, block, run, latency; // us
-    } shapes[3] = {{64, 64, 2, 1.3f, 1.8f, 0.42f, 0.85f}, {64, 32, 3, 1.3f, 1.2f, 0.263f, 0.5f}, {32, 32, 4, 1.0f, 1.0f, 0.2f, 0.22f}};
+        float start, block, run, latency; // us, of the choice
+        float launch, wave, side, beside, alone, first;
+    } shapes[3] = {{64, 64, 2, 1.3f, 1.8f, 0.42f, 0.85f, 2.9f, 0.85f, 2.25f, 0.35f, 0.98f, -0.6f},
+                   {64, 32, 3, 1.3f, 1.2f, 0.263f, 0.5f, 1.2f, 1.3f, 1.1f, 0.285f, 0.96f, -1.45f},
+                   {32, 32, 4, 1.0f, 1.0f, 0.2f, 0.22f, 0.1f, 0.1f, 1.95f, 0.3f, 0.205f, -1.05f}};
     const float M = (float)d.n * d.out_h * d.out_w, runs = ceilf((float)d.kh * d.kw * d.in_c / M16_RUN);
     Mma16Plan best = {0, 0, 1e30f};
+    float least = 1e30f;
     for (const auto &s : shapes) {
         const float blocks = ceilf(M / s.bm) * ceilf((float)d.out_c / s.bn), side = fminf((float)s.resident, ceilf(blocks / num_sms()));
-        const float us = 2.0f + fmaxf(1.0f, blocks / (num_sms() * s.resident)) * (s.start + s.block * side + runs * fmaxf(s.latency, side * s.run));
-        if (us < best.us)
-            best = {s.bm, s.bn, us};
+        const float waves = fmaxf(1.0f, blocks / (num_sms() * s.resident)), us = 2.0f + waves * (s.start + s.block * side + runs * fmaxf(s.latency, side * s.run));
+        if (us < least) {
+            least = us;
+            best = {s.bm, s.bn, s.launch + waves * (s.wave + s.side * side + fmaxf(runs * s.alone + s.first, side * runs * s.beside))};
+        }
     }
     return best;
 }

@@ -54,3 +54,22 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(abi, "_lib", None)
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         abi.load()
+
+
+# windows of int16: pixels, filter, channels in and out; us on the warp-level instructions and on packed operands.  Only the latter asks for scratch.
+INT16_TIMES = [((4, 40, 40), 3, 64, 64, 9.7, 12.3), ((47, 13, 12), 3, 96, 24, 12.9, 17.3), ((44, 14, 13), 3, 24, 128, 11.6, 13.7),
+               ((45, 11, 11), 3, 256, 80, 37.3, 22.1), ((1, 72, 70), 5, 32, 96, 17.8, 15.6), ((27, 13, 14), 5, 32, 80, 17.5, 15.2)]
+
+
+@pytest.mark.parametrize("image,k,cin,cout,here,packed", INT16_TIMES)
+def test_int16_windows_take_the_faster_kernel(library, image, k, cin, cout, here, packed):
+    """Layers on both sides of the line, as measured; long reductions of few blocks were sent to the slower one."""
+    d = abi.ConvDesc()
+    d.input, d.filter, d.output = 1 << 20, 2 << 20, 3 << 20  # nothing is read
+    d.dtype, d.n, d.in_h, d.in_w, d.in_c, d.out_c = abi.DTYPE_INT16, *image, cin, cout
+    d.out_h, d.out_w, d.kh, d.kw, d.group = d.in_h, d.in_w, k, k, 1
+    d.stride_h = d.stride_w = d.dilation_h = d.dilation_w = 1
+    d.pad_top = d.pad_bottom = d.pad_left = d.pad_right = k // 2
+    need = C.c_size_t(0)
+    assert library.espdl_b200_conv2d_workspace_bytes(C.byref(d), C.byref(need)) == abi.OK
+    assert (need.value == 0) == (here < packed)
