@@ -561,20 +561,34 @@ static bool runs_mma(const espdl_conv_desc &d)
     return conv2d_mma_estimate_us(d) < min(other, 8.f);
 }
 
+// Do results lie where inputs do?  Channels side by side in the same rows don't.
+static bool overlaps(const espdl_conv_desc &d)
+{
+    const long long es = d.dtype == ESPDL_DTYPE_INT16 ? 2 : 1, ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c, ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
+    const long long in_bytes = (((long long)d.n * d.in_h * d.in_w - 1) * ips + d.in_c) * es, out_bytes = (((long long)d.n * d.out_h * d.out_w - 1) * ops + d.out_c) * es;
+    const long long ahead = (long long)((intptr_t)d.output - (intptr_t)d.input);
+    if (ahead >= in_bytes || -ahead >= out_bytes)
+        return false;
+    const long long row = ips * es, into = (ahead % row + row) % row; // of the output into the input's row
+    return !(ips == ops && into >= d.in_c * es && into + d.out_c * es <= row);
+}
+
 // int16 on the warp-level instructions, where the other kernels take longer.  Packing and the tile kernel: two launches, the reduction's length, the
 // unrolled rows (windows about twice), the results and the products, from 37 layers, 20 % (standard deviation) off 380 others.  The
 // products' rate is a third of theirs: 4096x1024x1024 25 us there, 66 here; 45 of 11x11x256 -> 80, 3x3 22 / 37.  Results of fewer than 16 channels leave the tile kernel a row at a time
 // (58800x96x8 22.4 / 11.0).  Eight-element reductions are padded to 64 here, and the CUDA cores read them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
-// 6.0; 1088x8x192 8.9 / 3.8).
+// 6.0; 1088x8x192 8.9 / 3.8).  A product whose results overwrite its inputs stays with the tile kernel, which has copied those before it writes.
 static bool runs_mma16(const espdl_conv_desc &d)
 {
     if (d.dtype != ESPDL_DTYPE_INT16 || d.kernel != ESPDL_KERNEL_AUTO || d.n <= 0 || !conv2d_mma16_supported(d))
         return false;
     const char *knob = getenv("ESPDL_B200_MMA16"); // 0: never, always: wherever it can run
-    if (knob && (*knob == '0' || *knob == 'a'))
-        return *knob == 'a';
-    const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c, us = conv2d_mma16_estimate_us(d);
     const bool product = conv2d_tc_supported(d);
+    if ((knob && *knob == '0') || (product && overlaps(d)))
+        return false;
+    if (knob && *knob == 'a')
+        return true;
+    const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c, us = conv2d_mma16_estimate_us(d);
     if (!product && !conv2d_packed_supported(d))
         return us < (K <= 8 && d.out_c <= 64 ? 2.9f + M * K * d.out_c / 1.3e6f : conv2d_simt_estimate_us(d));
     const float tile = 8.0f + 2.5e-3f * K + M * K * (product ? 0.6e-6f : 1.07e-6f) + M * d.out_c * 2.0e-6f + M * K * d.out_c * 1.6e-9f +
