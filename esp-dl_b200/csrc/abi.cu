@@ -726,9 +726,9 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
     if (runs_mma(*desc))
         return conv2d_mma(*desc, s);
     if (runs_mma16(*desc)) {
-        // products declare the tile kernel's scratch whichever kernel runs them, and are refused without it
+        // products declare the tile kernel's scratch whichever kernel runs them, and are refused without it or where it is not aligned
         const size_t need = conv2d_tc_supported(*desc) ? conv2d_tc_workspace_bytes(*desc) : 0;
-        return need > workspace_bytes || (need && !workspace) ? ESPDL_ERR_INVALID_ARG : conv2d_mma16(*desc, s);
+        return need > workspace_bytes || (need && (!workspace || (uintptr_t)workspace % 16)) ? ESPDL_ERR_INVALID_ARG : conv2d_mma16(*desc, s);
     }
     if (desc->kernel != ESPDL_KERNEL_SIMT && conv2d_stem_tc_supported(*desc))
         return conv2d_stem_tc(*desc, s); // 3x3 stride-2 RGB first layer: banded-filter tensor-core kernel

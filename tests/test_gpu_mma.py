@@ -147,3 +147,22 @@ def test_int16_product_in_place(monkeypatch):
             abi.check(dev.lib.espdl_b200_conv2d(C.byref(cases.conv_desc(case, ptrs)), None), "conv2d")
             rows = dev.download(x, case["x"])
         np.testing.assert_array_equal(rows[..., ahead:ahead + cout], want[..., :cout])
+
+
+@pytest.mark.parametrize("knob", ["always", "0"])
+def test_int16_product_refuses_scratch_it_cannot_use(knob, monkeypatch):
+    """Whichever kernel runs a product: scratch that is missing, short or not aligned to 16 bytes is an error."""
+    monkeypatch.setenv("ESPDL_B200_MMA16", knob)
+    case = cases.conv_case(seed=1, dtype=abi.DTYPE_INT16, n=1, h=1, w=100, cin=64, cout=48, per_channel=True, e_in=-13, e_out=-5, e_w=(-14, -11), **P0)
+    with gpu_util.DeviceBuffers() as dev:
+        out = dev.upload(case["out"])
+        ptrs = dict(input=dev.upload(case["x"]), output=out, filter=dev.upload(case["w"]), bias=dev.upload(case["b"]), filter_exponents=dev.upload(case["ew"]))
+        d, need = cases.conv_desc(case, ptrs), C.c_size_t(0)
+        abi.check(dev.lib.espdl_b200_conv2d_workspace_bytes(C.byref(d), C.byref(need)), "workspace")
+        scratch = dev.alloc(need.value + 16)
+        assert need.value > 0
+        for at, size in ((None, need.value), (scratch, need.value - 1), (scratch + 8, need.value)):
+            assert dev.lib.espdl_b200_conv2d_ws(C.byref(d), at, size, None) == abi.ERR_INVALID_ARG
+        abi.check(dev.lib.espdl_b200_conv2d_ws(C.byref(d), scratch, need.value, None), "conv2d_ws")
+        want = gpu_util.run_conv_oracle(case)
+        np.testing.assert_array_equal(dev.download(out, want), want)
