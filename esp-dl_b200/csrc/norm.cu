@@ -299,8 +299,9 @@ __device__ __forceinline__ F2 codes_to_floats(uint32_t flipped, int k)
 // Rows of whole aligned 16-byte units have a pitch of an odd number of those: copies and a row's reads are of 16 bytes then, a quarter warp's
 // without bank conflicts as well (69 -> 65 us).
 // WORDS: rows are whole aligned words in global memory; otherwise the block's rows, one contiguous run of bytes, are dealt out to
-// and collected from the padded rows byte by byte.
-template <typename T, bool WORDS, bool EVEN>
+// and collected from the padded rows byte by byte.  UNITS: rows of whole 16-byte units; forms of their own, because what a block fetches of a kernel's code
+// counts in the shortest launches (6250 rows of 16: 3.77 us, 3.99 with both forms in one kernel).
+template <typename T, bool WORDS, bool EVEN, bool UNITS>
 __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, int pitch, int early)
 {
     if (early)
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
         if (WORDS) {
             // asynchronous copies: all of the block's rows in flight at once (with loads through registers a block spent half its time here)
             const uint32_t to = (uint32_t)__cvta_generic_to_shared(rows_s);
-            if (pitch % 4 == 0)
+            if (UNITS)
                 for (int rr = warp; rr < nr; rr += 8)
                     for (int i = 4 * lane; i < words; i += 128)
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 4u * (uint32_t)(rr * pitch + i)), "l"(src + (long long)rr * words + i) : "memory");
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
                     for (int k = 0; k < V; k++) sum += a.get(k);
                 }
             };
-            if (pitch % 4 == 0)
+            if (UNITS)
                 for (int i = 0; i < full; i += 4) {
                     const uint4 w = *(const uint4 *)(row + i);
                     add_word(w.x), add_word(w.y), add_word(w.z), add_word(w.w);
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
                     var = __fadd_rn(__fadd_rn(var, a), b);
                 }
             };
-            if (pitch % 4 == 0)
+            if (UNITS)
                 for (int i = 0; i < full; i += 4) {
                     const uint4 w = *(const uint4 *)(row + i);
                     add_squares(w.x), add_squares(w.y), add_squares(w.z), add_squares(w.w);
@@ -463,15 +464,17 @@ int launch_layer_rows(const NormParams &p, int R, int pitch, cudaStream_t s)
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        for (auto k : {layer_rows_kernel<T, true, false>, layer_rows_kernel<T, true, true>, layer_rows_kernel<T, false, false>, layer_rows_kernel<T, false, true>})
+        for (auto k : {layer_rows_kernel<T, true, false, false>, layer_rows_kernel<T, true, true, false>, layer_rows_kernel<T, false, false, false>,
+                       layer_rows_kernel<T, false, true, false>, layer_rows_kernel<T, true, false, true>, layer_rows_kernel<T, true, true, true>})
             if (attr_err == cudaSuccess)
                 attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(layer_rows_kernel)");
     const long long groups = (p.rows + R - 1) / R;
-    const auto kernel = words ? (p.half_even ? layer_rows_kernel<T, true, true> : layer_rows_kernel<T, true, false>)
-                              : (p.half_even ? layer_rows_kernel<T, false, true> : layer_rows_kernel<T, false, false>);
+    const auto kernel = pitch % 4 == 0 ? (p.half_even ? layer_rows_kernel<T, true, true, true> : layer_rows_kernel<T, true, false, true>)
+        : words                        ? (p.half_even ? layer_rows_kernel<T, true, true, false> : layer_rows_kernel<T, true, false, false>)
+                                       : (p.half_even ? layer_rows_kernel<T, false, true, false> : layer_rows_kernel<T, false, false, false>);
     launch_mover(kernel, dim3((unsigned)min(groups, (long long)num_sms() * 64)), dim3(256), smem, s, p, R, pitch);
     count_launch();
     return check_launch("layer norm");

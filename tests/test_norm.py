@@ -112,6 +112,32 @@ def test_gpu_in_place(op):
         np.testing.assert_array_equal(dev.download(ptrs["y"], a["y"]), want["y"])
 
 
+# rows of whole 16-byte units, enough of them for the kernel that puts rows side by side (256 up to 128 elements, beyond that 32 an SM): one unit a row, an
+# even and an odd number of units, the last block's rows ragged; 24 elements are units in int16 only.  `skip`: elements the tensors start behind an aligned address
+@pytest.mark.gpu
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("dt", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("kw", [{}, dict(bias=False), dict(scale=False, bias=False, stats=False)])
+@pytest.mark.parametrize("rows,n,skip,in_place", [(259, 16, 0, False), (600, 64, 0, False), (300, 128, 0, True), (4801, 24, 0, False), (5003, 768, 0, False), (5003, 144, 0, True),
+                                                  (5003, 256, 4, False), (259, 16, 4, True)])
+def test_gpu_rows_of_whole_units(rows, n, skip, in_place, kw, dt, round_mode):
+    import gpu_util
+    a = make(abi.NORM_LAYER, dt, rows, n, seed=rows + n, round_mode=round_mode, **kw)
+    want = fresh(a)
+    assert checkers.oracle().oracle_norm(C.byref(desc(want))) == 0
+    with gpu_util.DeviceBuffers() as dev:
+        pad = np.zeros(skip, dtype=a["x"].dtype)
+        ptrs = {k: dev.upload(a[k]) for k in ("scale", "bias", "mean", "inv") if a[k] is not None}
+        whole = {k: dev.upload(np.concatenate([pad, a[k].reshape(-1)])) for k in (("x",) if in_place else ("x", "y"))}
+        ptrs["x"] = whole["x"] + pad.nbytes
+        ptrs["y"] = ptrs["x"] if in_place else whole["y"] + pad.nbytes
+        abi.check(dev.lib.espdl_b200_norm(C.byref(desc(a, ptrs)), None), "norm")
+        for k in ("y", "mean", "inv"):
+            if a[k] is not None:
+                np.testing.assert_array_equal(dev.download(ptrs[k], want[k]), want[k], err_msg=k)
+    assert want["y"].std() > 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("op", [abi.NORM_RMS, abi.NORM_LAYER])
 @pytest.mark.parametrize("shape,axis", [((2, 9, 64), -1), ((3, 4, 5, 16), 2)])
