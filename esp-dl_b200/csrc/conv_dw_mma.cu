@@ -334,7 +334,7 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 mbar_arrive(smem_u32(&free_bar[(i - 1) % NO]));
             }
             __syncwarp();
-            ok = !*abort_flag && mbar_wait(smem_u32(&done_bar[s]), (i / NO) & 1);
+            ok = !*abort_flag && mbar_wait(smem_u32(&done_bar[s]), (i / NO) & 1, p.wait_limit);
             if (!ok) {
                 *abort_flag = 1;
                 if (lane == 0)
@@ -355,7 +355,7 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             advance();
         }
         if (!ok) // the loads on their way land before shared memory is given back
-            for (; i < loaded; i++) mbar_wait(smem_u32(&full_bar[i % NS]), (i / NS) & 1);
+            for (; i < loaded; i++) mbar_wait(smem_u32(&full_bar[i % NS]), (i / NS) & 1, p.wait_limit);
         if (elect_one())
             bulk_wait_all(); // shared memory stays allocated until the last store has left it
         __syncwarp();
@@ -386,7 +386,7 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
         // The output tile first: tile i - NO has left it, so the producer has seen the end of every tile up to that one, tile i - NS among them
         // (NS >= NO), and the stage's barrier is at most one phase behind.  The other way round, a load of another team's tile i - NS still on its
         // way would leave the parity as it is after tile i.
-        if (!mbar_wait(smem_u32(&free_bar[o]), (i / NO & 1) ^ 1) || !mbar_wait(smem_u32(&full_bar[s]), (i / NS) & 1)) {
+        if (!mbar_wait(smem_u32(&free_bar[o]), (i / NO & 1) ^ 1, p.wait_limit) || !mbar_wait(smem_u32(&full_bar[s]), (i / NS) & 1, p.wait_limit)) {
             *abort_flag = 1; // the tile before never left, or the patch never came
             if (lane == 0)
                 report_timeout(g_dwm_error);
@@ -417,7 +417,7 @@ dw3x3_mma_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
         }
         fence_async_smem(); // the output words are visible to the TMA unit
         __syncwarp();
-        if (lane == 0)
+        if (lane == 0 && !(p.withhold_arrive && warp == 0))
             mbar_arrive(smem_u32(&done_bar[o]));
     }
 }
@@ -522,6 +522,11 @@ int conv2d_dw_mma(const espdl_conv_desc &d, cudaStream_t s)
         return set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled entry point not found");
     const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c, ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     p.pt = d.pad_top, p.pl = d.pad_left;
+    // ESPDL_B200_DEBUG_WAIT_EXPIRY=<milliseconds> (with ESPDL_B200_DW_MMA=always), the test of the bounded waits: one arrival is withheld and the limit that
+    // short, so the producer's wait runs out and every role leaves; espdl_b200_stream_sync then reports ESPDL_ERR_TIMEOUT.
+    const char *expiry = getenv("ESPDL_B200_DEBUG_WAIT_EXPIRY");
+    p.withhold_arrive = expiry && atoi(expiry) > 0 ? 1 : 0;
+    p.wait_limit = p.withhold_arrive ? (long long)atoi(expiry) * 2000000ll : WAIT_LIMIT_CYCLES;
     p.src.C = d.in_c;
     p.src.w = (const int8_t *)d.filter, p.src.bias = (const int32_t *)d.bias, p.src.ew = d.filter_exponents, p.src.lut = d.lut, p.src.lut_stride = d.lut_channel_stride;
     p.src.e_shift_base = d.out_exponent - d.in_exponent;

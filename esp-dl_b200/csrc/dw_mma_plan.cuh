@@ -36,6 +36,8 @@ struct DwmParams {
     int stage_bytes, out_bytes, tx_bytes; // patch stride in the ring, output tile size, bytes one patch load delivers
     unsigned *sched;                      // {next tile, CTAs done}: the tiles from static_tiles on are handed out by this counter; null = fixed walk
     int static_tiles;                     // tiles walked in the fixed order (a multiple of the grid size)
+    long long wait_limit;                 // cycles a wait may take (WAIT_LIMIT_CYCLES; shorter only in the expiry test)
+    int withhold_arrive;                  // expiry test: consumer warp 0 never reports its part of a tile, so the producer's wait runs out
     DwmSource src;
 };
 

@@ -393,13 +393,16 @@ def test_invalid_arguments_are_rejected():
     assert b"invalid" in L.espdl_b200_strerror(abi.ERR_INVALID_ARG)
 
 
-def test_a_bounded_wait_that_runs_out_is_reported_and_the_next_launch_works(monkeypatch):
+@pytest.mark.parametrize("cin,mma", [(64, None), (48, "always")], ids=["dp4a", "mma"])
+def test_a_bounded_wait_that_runs_out_is_reported_and_the_next_launch_works(cin, mma, monkeypatch):
     """Every mbarrier wait of the persistent kernels has a limit.  With ESPDL_B200_DEBUG_WAIT_EXPIRY the TMA-fed depthwise
-    kernel withholds one arrival and shortens the limit to a few milliseconds: the wait runs out, the CTA raises its flag,
+    kernels (the second one with several teams, and tiles handed out by counters) withhold one arrival and shortens the limit to a few milliseconds: the wait runs out, the CTA raises its flag,
     every role leaves (nothing traps, nothing spins on), espdl_b200_stream_sync reports ESPDL_ERR_TIMEOUT - and the same
     launch without the switch gives the oracle's result on the same context."""
     import ctypes as C
-    case = cases.conv_case(seed=71, n=96, h=56, w=56, cin=64, kh=3, kw=3, depthwise=True, per_channel=True, e_in=-5, e_out=-5, e_w=(-9, -5))
+    if mma:
+        monkeypatch.setenv("ESPDL_B200_DW_MMA", mma)
+    case = cases.conv_case(seed=71, n=96, h=56, w=56, cin=cin, kh=3, kw=3, depthwise=True, per_channel=True, e_in=-5, e_out=-5, e_w=(-9, -5))
     want = gpu_util.run_conv_oracle(case)
     with gpu_util.DeviceBuffers() as dev:
         ptrs = dict(input=dev.upload(case["x"]), filter=dev.upload(case["w"]), bias=dev.upload(case["b"]),
