@@ -99,7 +99,7 @@ __device__ __forceinline__ void dwm_load_consts(DwmConsts &k, const DwmSource &p
                 k.a[ky][j][h] = second ? 0u : v, k.a[ky][j][2 + h] = second ? v : 0u;
             }
         }
-    bool fast = !p.lut;
+    bool fast = true;
 #pragma unroll
     for (int q = 0; q < DwmConsts::QUADS; q++)
 #pragma unroll
@@ -113,8 +113,7 @@ __device__ __forceinline__ void dwm_load_consts(DwmConsts &k, const DwmSource &p
     k.form = !__all_sync(0xffffffffu, fast) ? DwmForm::General : (p.relu ? DwmForm::Relu : DwmForm::Linear);
 }
 
-// A lane's share of a group with channels outside the one-add-one-shift form (a shift below 1, a huge bias or a fused table): `pixels` output
-// pixels of its position, four channels from `c` on, `rows` rows, by plain loops and the general requantisation.
+// A lane's share of a group with channels outside the one-add-one-shift form (a shift below 1, a huge bias): `pixels` output pixels of its position, four channels from `c` on, `rows` rows, by plain loops and the general requantisation.
 __device__ __noinline__ void dwm_walk_general(const DwmSource &p, const int8_t *ip, int8_t *op, int in_row, int out_row, int CB, int rows, int pixels, int c)
 {
     for (int y = 0; y < rows; y++)
@@ -124,10 +123,7 @@ __device__ __noinline__ void dwm_walk_general(const DwmSource &p, const int8_t *
                 for (int ky = 0; ky < 3; ky++)
                     for (int kx = 0; kx < 3; kx++) acc += (int)ip[(y + ky) * in_row + (x + kx) * CB + i] * (int)p.w[(ky * 3 + kx) * p.C + c + i];
                 const int shift = max(-31, min(32, p.e_shift_base - (p.per_channel ? p.ew[c + i] : p.ew_scalar)));
-                int32_t v = requant8(acc, p.bias ? p.bias[c + i] : 0, shift, p.relu, p.half_even);
-                if (p.lut)
-                    v = p.lut[(long long)(c + i) * p.lut_stride + ((uint8_t)v ^ 0x80u)];
-                op[y * out_row + x * CB + i] = (int8_t)v;
+                op[y * out_row + x * CB + i] = (int8_t)requant8(acc, p.bias ? p.bias[c + i] : 0, shift, p.relu, p.half_even);
             }
 }
 
@@ -491,7 +487,7 @@ bool conv2d_dw_mma_supported(const espdl_conv_desc &d)
 {
     if (d.dtype != ESPDL_DTYPE_INT8 || d.group == 1 || d.kh != 3 || d.kw != 3 || d.dilation_h != 1 || d.dilation_w != 1)
         return false;
-    if (d.stride_h != 1 || d.stride_w != 1)
+    if (d.stride_h != 1 || d.stride_w != 1 || d.lut) // a table would be the general form's, whose loops have more threads on dp4a
         return false;
     const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c, ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     if (d.in_c % 16 || ips % 16 || ops % 16 || ((uintptr_t)d.input % 16) || ((uintptr_t)d.output % 16) || ((uintptr_t)d.filter % 4))
@@ -504,8 +500,8 @@ bool conv2d_dw_mma_supported(const espdl_conv_desc &d)
 
 bool conv2d_dw_mma_pays(const espdl_conv_desc &d)
 {
-    // the size before the search for a plan; a table is the general form's, whose loops have more threads on dp4a
-    if (d.lut || !dwm_large(d.in_c, (long long)d.n * d.out_h * d.out_w * d.in_c) || !conv2d_dw_mma_supported(d))
+    // the size before the search for a plan
+    if (!dwm_large(d.in_c, (long long)d.n * d.out_h * d.out_w * d.in_c) || !conv2d_dw_mma_supported(d))
         return false;
     DwmParams p;
     auto pays = [&](bool whole) { return dwm_pays(p, d.in_c, d.out_h, d.out_w, d.n, d.round_mode == ESPDL_ROUND_HALF_EVEN, whole, num_sms()); };
@@ -528,7 +524,7 @@ int conv2d_dw_mma(const espdl_conv_desc &d, cudaStream_t s)
     p.withhold_arrive = expiry && atoi(expiry) > 0 ? 1 : 0;
     p.wait_limit = p.withhold_arrive ? (long long)atoi(expiry) * 2000000ll : WAIT_LIMIT_CYCLES;
     p.src.C = d.in_c;
-    p.src.w = (const int8_t *)d.filter, p.src.bias = (const int32_t *)d.bias, p.src.ew = d.filter_exponents, p.src.lut = d.lut, p.src.lut_stride = d.lut_channel_stride;
+    p.src.w = (const int8_t *)d.filter, p.src.bias = (const int32_t *)d.bias, p.src.ew = d.filter_exponents;
     p.src.e_shift_base = d.out_exponent - d.in_exponent;
     p.src.ew_scalar = d.filter_exponent, p.src.per_channel = d.per_channel;
     p.src.relu = d.activation == ESPDL_ACT_RELU, p.src.half_even = d.round_mode == ESPDL_ROUND_HALF_EVEN;
