@@ -18,9 +18,11 @@ def no_small_layers(monkeypatch, request):
     monkeypatch.setenv("ESPDL_B200_SMALL_MMA", "0")  # the kernels meant here, whatever the size
     if "dw-tma" in request.node.name:
         monkeypatch.setenv("ESPDL_B200_DW_TMA_NARROW", "1")
+    if "dw-mma" in request.node.name:
+        monkeypatch.setenv("ESPDL_B200_DW_MMA", "always")
 
 # one shape per kernel: the tile kernel (staged, unaligned rows, residual), filter windows (one box per tap, one patch per
-# tile stacked / unstaged), banded 8 / 16 channels, first layer, depthwise through the TMA unit and from global memory
+# tile stacked / unstaged), banded 8 / 16 channels, first layer, depthwise through the TMA unit, on the matrix instruction and from global memory
 SHAPES = {
     "tile": dict(n=2, h=9, w=13, cin=64, cout=96, kh=1, kw=1, pad=(0, 0, 0, 0)),
     "tile-wide": dict(n=1, h=1, w=130, cin=512, cout=256, kh=1, kw=1, pad=(0, 0, 0, 0)),
@@ -34,6 +36,8 @@ SHAPES = {
     "first": dict(n=2, h=32, w=48, cin=3, cout=16, stride=2),
     "dw-tma": dict(n=2, h=14, w=15, cin=96, depthwise=True),
     "dw-tma-s2": dict(n=2, h=15, w=14, cin=64, stride=2, depthwise=True),
+    "dw-mma": dict(n=2, h=14, w=15, cin=96, depthwise=True),
+    "dw-mma-slices": dict(n=3, h=9, w=7, cin=32, depthwise=True, in_stride=48, out_stride=64),
     "dw-narrow": dict(n=2, h=9, w=17, cin=24, depthwise=True),
     "dw-narrow-s2": dict(n=2, h=10, w=17, cin=32, stride=2, depthwise=True),
 }
@@ -78,6 +82,8 @@ GENERAL = {
     "narrow": (dict(n=2, h=15, w=14, cin=16, cout=13, kh=2, kw=2, pad=(0, 1, 0, 1)), {"ESPDL_B200_NARROW": "always"}, abi.KERNEL_AUTO),
     "dw3": (dict(n=1, h=9, w=11, cin=20, depthwise=True), {}, abi.KERNEL_AUTO),
     "dw3-tma": (dict(n=2, h=14, w=15, cin=96, depthwise=True), {"ESPDL_B200_DW_TMA_NARROW": "1"}, abi.KERNEL_AUTO),
+    "dw3-mma": (dict(n=2, h=14, w=15, cin=96, depthwise=True), {"ESPDL_B200_DW_MMA": "always"}, abi.KERNEL_AUTO),
+    "dw3-mma-slices": (dict(n=3, h=9, w=7, cin=32, depthwise=True, in_stride=48, out_stride=64), {"ESPDL_B200_DW_MMA": "always"}, abi.KERNEL_AUTO),
     "dw5": (dict(n=1, h=9, w=11, cin=20, kh=5, kw=5, pad=(2, 2, 2, 2), depthwise=True), {}, abi.KERNEL_AUTO),
     "dw7": (dict(n=1, h=9, w=11, cin=24, kh=7, kw=7, pad=(3, 3, 3, 3), depthwise=True), {}, abi.KERNEL_AUTO),
     "dw-vec": (dict(n=1, h=9, w=11, cin=32, kh=3, kw=5, pad=(1, 1, 2, 2), depthwise=True), {}, abi.KERNEL_AUTO),

@@ -88,10 +88,9 @@ DW_SHAPES = [
 @pytest.mark.parametrize("tma", [False, True], ids=["auto", "tma"])
 @pytest.mark.parametrize("kw", DW_SHAPES, ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "pad"))
 def test_depthwise_3x3_shapes(kw, tma, monkeypatch):
-    """The 3x3 depthwise kernels on the network's layer shapes, ragged extents and unusual paddings, against the oracle:
-    the TMA-fed kernel (the default for large layers from 64 channels on; ESPDL_B200_DW_TMA_NARROW=1: for any size and channel
-    count) and the kernel that reads global memory directly (the default below, and ESPDL_KERNEL_SIMT).  A depthwise conv has
-    no tensor-core form, so asking for one is refused."""
+    """The 3x3 depthwise kernels on dp4a on the network's layer shapes, ragged extents and unusual paddings, against the oracle:
+    the TMA-fed kernel (ESPDL_B200_DW_TMA_NARROW=1: for any size and channel count) and the kernel that reads global memory directly (the default
+    for layers of this size, and ESPDL_KERNEL_SIMT).  A depthwise conv has no tensor-core tile kernel, so asking for one is refused."""
     if tma:
         monkeypatch.setenv("ESPDL_B200_DW_TMA_NARROW", "1")
     case = cases.conv_case(seed=61, depthwise=True, kh=3, kw=3, per_channel=True, e_in=-5, e_out=-5, e_w=(-9, -5), **kw)
@@ -104,27 +103,47 @@ def test_depthwise_3x3_shapes(kw, tma, monkeypatch):
 
 @pytest.mark.parametrize("round_mode,act,bias,lut", [(abi.ROUND_HALF_EVEN, abi.ACT_RELU, True, False), (abi.ROUND_HALF_UP, abi.ACT_LINEAR, False, False),
                                                      (abi.ROUND_HALF_UP, abi.ACT_RELU, True, True)])
-@pytest.mark.parametrize("tma", [False, True], ids=["auto", "tma"])
-def test_depthwise_3x3_epilogue_variants(round_mode, act, bias, lut, tma, monkeypatch):
-    if tma:
-        monkeypatch.setenv("ESPDL_B200_DW_TMA_NARROW", "1")
+@pytest.mark.parametrize("knob", [None, ("ESPDL_B200_DW_TMA_NARROW", "1"), ("ESPDL_B200_DW_MMA", "always")], ids=["auto", "tma", "mma"])
+def test_depthwise_3x3_epilogue_variants(round_mode, act, bias, lut, knob, monkeypatch):
+    if knob:
+        monkeypatch.setenv(*knob)
     case = cases.conv_case(seed=63, n=2, h=19, w=23, cin=80, depthwise=True, kh=3, kw=3, per_channel=True, round_mode=round_mode, act=act,
                            bias=bias, lut=lut, in_stride=96, out_stride=112)
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
 
 
 # stride 1 on the matrix instruction: positions of two pixels in eights, bands of rows in threes, dense rows as runs and channel slices, several
-# images a tile, more tiles than are dealt out in the fixed order, channels that share lines of memory
-@pytest.mark.parametrize("act,round_mode", [(abi.ACT_RELU, abi.ROUND_HALF_UP), (abi.ACT_LINEAR, abi.ROUND_HALF_EVEN)])
+# images a tile, more tiles than are dealt out in the fixed order, channels that share lines of memory; several teams whose number divides the stages or not
+@pytest.mark.parametrize("act", [abi.ACT_LINEAR, abi.ACT_RELU])
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
 @pytest.mark.parametrize("kw", [
     dict(n=1, h=1, w=1, cin=16), dict(n=3, h=2, w=3, cin=48), dict(n=1, h=5, w=17, cin=32), dict(n=2, h=31, w=33, cin=32, in_stride=64, out_stride=48),
     dict(n=37, h=7, w=7, cin=240), dict(n=19, h=9, w=5, cin=128), dict(n=2, h=57, w=58, cin=64), dict(n=130, h=28, w=27, cin=96),
-    dict(n=1, h=3, w=300, cin=16, pad=(3, 0, 2, 5)), dict(n=700, h=14, w=14, cin=32),
+    dict(n=1, h=3, w=300, cin=16, pad=(3, 0, 2, 5)), dict(n=700, h=14, w=14, cin=32), dict(n=64, h=112, w=112, cin=16), dict(n=24, h=46, w=45, cin=240),
 ])
 def test_depthwise_matrix_instruction(kw, act, round_mode, monkeypatch):
     monkeypatch.setenv("ESPDL_B200_DW_MMA", "always")
     case = cases.conv_case(seed=67 + kw["w"], depthwise=True, kh=3, kw=3, per_channel=True, act=act, round_mode=round_mode, e_in=-5, e_out=-5, e_w=(-9, -5), **kw)
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+
+
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("per_channel,bias", [(True, True), (True, False), (False, True)])
+def test_depthwise_matrix_instruction_constants(per_channel, bias, round_mode, monkeypatch):
+    """No bias, one exponent for all channels, and one block of 16 channels with left shifts and a huge bias beside blocks of the one-add form, their shifts
+    from the least."""
+    monkeypatch.setenv("ESPDL_B200_DW_MMA", "always")
+    for act in (abi.ACT_RELU, abi.ACT_LINEAR):
+        case = cases.conv_case(seed=91, n=5, h=11, w=10, cin=48, depthwise=True, kh=3, kw=3, per_channel=per_channel, bias=bias, act=act, round_mode=round_mode,
+                               e_in=0, e_out=0, e_w=(-9, -1))
+        if per_channel:
+            case["ew"][17], case["ew"][20], case["ew"][40] = 2, 0, -1
+            if bias:
+                case["b"][31] = 2 ** 31 - 1
+                case["ew"][31] = -24
+        want = gpu_util.run_conv_oracle(case)
+        np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), want)
+        assert want.std() > 0
 
 
 def test_depthwise_block_shape():

@@ -14,6 +14,7 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture(autouse=True)
 def no_small_layers(monkeypatch):
     monkeypatch.setenv("ESPDL_B200_SMALL_MMA", "0")  # the kernels meant here, whatever the size
+    monkeypatch.setenv("ESPDL_B200_MMA16", "0")
 
 S16 = dict(dtype=abi.DTYPE_INT16, e_in=-14, e_w=(-15, -14), e_out=-11)
 SHAPES = [
