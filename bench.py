@@ -54,7 +54,9 @@ def parse_args():
 
 
 TRAFFIC_RATIO_GEMM_TC = 0.87  # gemm_tc_kernel, 401408x128x768: 313.2 MB DRAM for 359.8 MB algorithmic (the output tail is still in L2)
-TRAFFIC_RATIO_DW = 1.034      # dw3x3_dp4a_kernel, 256x112x112x96: 637.4 MB DRAM for 616.6 MB algorithmic
+# dw3x3_mma_kernel, 1024x28x28x192: 262.1 MB DRAM for 308.3 MB algorithmic (0.85, the output tail is still in L2), and dw3x3_tma_kernel, 256x112x112x96 at stride 2:
+# 368.9 for 385.4 (0.957), weighted by the network's bytes in either (3.64 and 2.40 MB an image)
+TRAFFIC_RATIO_DW = 0.89
 
 
 # ------------------------------------------------------------------------------------------ clocks
@@ -412,7 +414,7 @@ def roofline_of(m, parsed, batch):
     achieved = dom["bytes"] / (dom["us"] * 1e-6) / 1e9
     kernel_names = {"pointwise_tc": "gemm_tc_kernel", "depthwise": "dw3x3_mma_kernel, dw3x3_tma_kernel", "conv_simt": "stem_tc_kernel",
                     "depthwise_pointwise_fused": "dwpw_kernel"}
-    # DRAM bytes moved per algorithmic byte, from one profiler capture of each kernel on a layer larger than L2
+    # DRAM bytes moved per algorithmic byte, from profiler captures of the kernels on layers larger than L2
     # (profiles/): the launches of a step differ in shape, so the per-launch traffic is that ratio applied to
     # the average algorithmic bytes of a launch.
     dram_per_algorithmic = {"pointwise_tc": TRAFFIC_RATIO_GEMM_TC, "depthwise": TRAFFIC_RATIO_DW}

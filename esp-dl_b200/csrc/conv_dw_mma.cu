@@ -1,4 +1,4 @@
-// 3x3 DepthwiseConv2D, int8, stride 1, on the warp-level matrix instruction, fed by TMA: large NHWC tensors whose channel count is a multiple of 16.
+// 3x3 DepthwiseConv2D, int8, stride 1, on the warp-level matrix instruction, fed by TMA: large NHWC tensors whose channel count is a multiple of 16 (which of them: dwm_pays).
 // Replaces dl::base::depthwise_conv2d<int8_t,...> (esp-dl/dl/base/dl_base_depthwise_conv2d.cpp:47-66, shell
 // esp-dl/dl/base/dl_base.hpp:1209-2107): out[y,x,c] = sat8(act(rnd((sum_{ky,kx} in[y+ky-pt, x+kx-pl, c] * w[ky,kx,c] + bias[c]) >> shift[c]))),
 // taps outside the image contribute nothing.
@@ -24,7 +24,7 @@
 //               (all channels in the block) move as runs of whole rows: the unit takes 3.5 cycles for a run, whatever its length;
 //   the others  consumers, in teams that take the tiles in turn: a warp owns 16 channels and walks groups of 8 positions down a band of rows, writing the
 //               requantised words into an output tile in shared memory.
-// Bound by the latency of a warp's walk, some 260 cycles a row with three or four warps a scheduler (matrix pipe 40 %, issue slots 45 % busy); loads and
+// Bound by the latency of a warp's walk, some 260 cycles a row with three or four warps a scheduler (1024 of 28x28x192: matrix pipe 43 %, issue slots 45 % busy); loads and
 // stores alone run at the copy bandwidth.  1024 images, dp4a before and now, us: 112x112x32 207 -> 165, 28x28x192 83 -> 75, 14x14x384 54 -> 41,
 // 14x14x576 75 -> 60, 7x7x960 44 -> 30.  Where tiles' channel blocks share lines of memory they follow one another (fetched twice otherwise: 28x28x192
 // could not be below 78), and with two stages a tile waited half its time for its load.

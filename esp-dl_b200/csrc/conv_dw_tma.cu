@@ -1,5 +1,5 @@
-// 3x3 DepthwiseConv2D, int8, stride 1 or 2, fed by TMA: the default depthwise kernel for NHWC tensors whose channel
-// count is a multiple of 16.
+// 3x3 DepthwiseConv2D, int8, stride 1 or 2, on dp4a, fed by TMA: NHWC tensors from 64 channels on whose channel count is a multiple of 16 - at stride 2, and at
+// stride 1 where the matrix instruction (conv_dw_mma.cu) takes longer, with a fused table always.
 // Replaces dl::base::depthwise_conv2d<int8_t,...> (esp-dl/dl/base/dl_base_depthwise_conv2d.cpp:47-66, shell
 // esp-dl/dl/base/dl_base.hpp:1209-2107): out[y,x,c] = sat8(act(rnd((sum_{ky,kx} in[y*s+ky-pt, x*s+kx-pl, c] * w[ky,kx,c] + bias[c]) >> shift[c]))),
 // taps outside the image contribute nothing.

@@ -1,7 +1,7 @@
 // int16 convs, Gemms and products of small and middling tensors with the warp-level matrix instruction (mma.sync m16n8k32) on byte planes.
 //
 // Replaces dl::base::conv2d<int16_t,...> (esp-dl/dl/base/dl_base_conv2d.cpp) where the tensor-core tile kernel's two launches - its operands
-// unrolled and split into byte planes in memory first - are most of the time: 4 x 40x40x64 -> 64, 3x3 took 12.8 us, 8 of them
+// unrolled and split into byte planes in memory first - are most of the time: 4 x 40x40x64 -> 64, 3x3 took 12.3 us, 8 of them
 // the packing and its launch.  Here the planes never reach memory: a block copies 64-element runs of its input
 // pixels' windows and filter rows to shared memory as they are (asynchronous copies, four stages, zero fill outside the image), a warp splits
 // the words of a fragment into high and low bytes by byte permutes, and multiplies: x = 256 xh + xl with xh signed and xl unsigned, so a
@@ -9,9 +9,10 @@
 // reductions up to 16384 terms, put together in 64 bits.
 // The order of the reduction is free as long as both operands agree: lane (g, t) takes the 16 consecutive elements 16t .. 16t + 15 of a run.  A run's 16-byte
 // units lie XORed with the row, so a quarter warp's 16-byte reads meet no bank conflict.
-// Bound by the latency of a run - its copies, fragments and 32 products a warp, one after the other - while there is a block an SM, by the
-// matrix instruction (46 % busy), permutes and addresses together beyond that.  us before and now: 4 of 40x40x64 -> 64 12.8 / 10.2, one of them 12.4 / 5.8,
-// 112x112x8 -> 16 at stride 2 12.3 / 4.1, 128x512x512 10.0 / 4.7, 51200x288x32 37 / 18.5, 200704x576x64 171 / 136.
+// Bound by the latency of a run - its copies, fragments and 32 products a warp, one after the other - while there is a block an SM (4 of 40x40: matrix pipe
+// 21 %, issue slots 44 % busy), by the matrix instruction (39 %), permutes and addresses (issue slots 53 %) together beyond that (256 of 28x28).  The 64 x 64
+// form spills 64 bytes at 128 registers, 64 x 32 8 bytes at 80.  us before and now: 4 of 40x40x64 -> 64 12.3 / 9.7, one of them 12.4 / 5.4,
+// 112x112x8 -> 16 at stride 2 12.3 / 3.7, 128x512x512 10.1 / 4.6, 51200x288x32 37 / 18, 200704x576x64 173 / 136.
 #include "common.cuh"
 
 #include <climits>

@@ -297,7 +297,7 @@ __device__ __forceinline__ F2 codes_to_floats(uint32_t flipped, int k)
 // down the rows.  Bound by instruction issue (100352 rows of 768: 101 -> 80 us with asynchronous copies in, codes to floats without conversions, all
 // threads in the normalising pass and as many blocks as there are groups of rows; 80 -> 69 with two elements an instruction).
 // Rows of whole aligned 16-byte units have a pitch of an odd number of those: copies and a row's reads are of 16 bytes then, a quarter warp's
-// without bank conflicts as well (69 -> 65 us).
+// without bank conflicts as well (69 -> 63 us, issue slots 68 % busy).
 // WORDS: rows are whole aligned words in global memory; otherwise the block's rows, one contiguous run of bytes, are dealt out to
 // and collected from the padded rows byte by byte.  UNITS: rows of whole 16-byte units; forms of their own, because what a block fetches of a kernel's code
 // counts in the shortest launches (6250 rows of 16: 3.77 us, 3.99 with both forms in one kernel).
