@@ -576,8 +576,8 @@ static bool overlaps(const espdl_conv_desc &d)
 // int16 on the warp-level instructions, where the other kernels take longer.  Packing and the tile kernel: two launches, the reduction's length, the
 // unrolled rows (windows about twice), the results and the products, from 37 layers, 20 % (standard deviation) off 380 others.  The
 // products' rate is a third of theirs: 4096x1024x1024 25 us there, 66 here; 45 of 11x11x256 -> 80, 3x3 22 / 37.  Results of fewer than 16 channels leave the tile kernel a row at a time
-// (58800x96x8 22.4 / 11.0).  Eight-element reductions are padded to 64 here, and the CUDA cores read them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
-// 6.0; 1088x8x192 8.9 / 3.8).  A product whose results overwrite its inputs stays with the tile kernel, which has copied those before it writes.
+// (58800x96x8 22.4 / 11.0).  Eight-element reductions are padded to 64 here, and the CUDA cores read many of them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
+// 6.0; 5977x8x5 3.6 / 3.3, 1088x8x192 8.9 / 3.8).  A product whose results overwrite its inputs stays with the tile kernel, which has copied those before it writes.
 static bool runs_mma16(const espdl_conv_desc &d)
 {
     if (d.dtype != ESPDL_DTYPE_INT16 || d.kernel != ESPDL_KERNEL_AUTO || d.n <= 0 || !conv2d_mma16_supported(d))
@@ -590,10 +590,10 @@ static bool runs_mma16(const espdl_conv_desc &d)
         return true;
     const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c, us = conv2d_mma16_estimate_us(d);
     if (!product && !conv2d_packed_supported(d))
-        return us < (K <= 8 && d.out_c <= 64 ? 2.9f + M * K * d.out_c / 1.3e6f : conv2d_simt_estimate_us(d));
+        return us < conv2d_simt_estimate_us(d) && !(K <= 8 && d.out_c <= 64 && M >= 7000);
     const float tile = 8.0f + 2.5e-3f * K + M * K * (product ? 0.6e-6f : 1.07e-6f) + M * d.out_c * 2.0e-6f + M * K * d.out_c * 1.6e-9f +
         (d.out_c < 16 ? M * 1.6e-4f : 0.0f);
-    return us < 0.97f * tile;
+    return us < 0.85f * tile;
 }
 
 // Shapes no kernel reads in place, large enough for packed operands to pay (a caller without the scratch gets the CUDA-core kernel).

@@ -213,8 +213,9 @@ struct Mma16Plan {
 
 // The tile by waves of as many blocks as an SM holds, each its start, its results, and its runs, which take their share of the matrix instructions or the
 // latency of copies and fragments (4 of 40x40x64 -> 64, 3x3: 13.2 us with 64 x 64, 10.2 with 64 x 32, 12.0 with 32 x 32; 400x1152x128 14.5, 10.6, 7.9;
-// 102400x576x64 70, 88, 112).  Its time for the choice against the other kernels by what 500 layers took in the tile that they get, inputs in L2 and not:
-// launch, a wave's start, what a block and a run cost beside others and alone; within 12 % (standard deviation).
+// 102400x576x64 70, 88, 112).  That estimate is low for long reductions in few blocks, so the choice against the other kernels also looks at what 500 layers
+// took in the tile that they get, inputs in L2 and not: launch, a wave's start, what a block and a run cost beside others and alone; within 12 % (standard
+// deviation).  It counts 0.88 of that, as runs_mma16 asks for 0.85 of the other kernels' time where the first estimate decides and 0.97 where this one does.
 Mma16Plan mma16_plan(const espdl_conv_desc &d)
 {
     static const struct {
@@ -232,7 +233,7 @@ Mma16Plan mma16_plan(const espdl_conv_desc &d)
         const float waves = fmaxf(1.0f, blocks / (num_sms() * s.resident)), us = 2.0f + waves * (s.start + s.block * side + runs * fmaxf(s.latency, side * s.run));
         if (us < least) {
             least = us;
-            best = {s.bm, s.bn, s.launch + waves * (s.wave + s.side * side + fmaxf(runs * s.alone + s.first, side * runs * s.beside))};
+            best = {s.bm, s.bn, fmaxf(us, 0.876f * (s.launch + waves * (s.wave + s.side * side + fmaxf(runs * s.alone + s.first, side * runs * s.beside))))};
         }
     }
     return best;
