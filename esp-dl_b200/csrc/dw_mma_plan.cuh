@@ -151,23 +151,26 @@ inline double dwm_estimate_us(const DwmParams &p, int sms)
 inline bool dwm_large(int C, long long outputs) { return C < 64 || outputs >= 32ll << 20; }
 
 // The planned launch against dp4a.  In a tile of 64 channels the pixels' banks collide (300 of 20x20x256: 26.5 us, 21.0 on dp4a), and narrower ones that are not
-// dense rows are the TMA unit's short runs.  For the others dp4a's time, from 2200 layers: 0.45 ps an output for 96 channels and 0.51 for other widths
-// that its tile takes whole (`dp4a_whole`), a quarter more for images below 200 pixels; 0.7 and more where it cuts pixels up; 0.49 for narrow tensors, more
-// for small images and for 16 channels (0.6 to 0.9, never less than here).  us here / there: 619 of 20x20x144 28.6 / 22.6, 928 of 20x20x96 29.8 / 22.1, 650 of
-// 28x28x144 45.3 / 41.1, 1024 of 80x80x48 201 / 170, 104 of 28x27x4000 231 / 219; 1024 of 112x112x32 171 / 207, 3715 of 14x14x144 60.8 / 67.0.  Half to
-// even is 29 % slower here and 16 % there (160 of 57x56x144 55.9 / 50.3, half up 43.4 both).  Narrow tensors
-// below 64 M outputs stay here, whichever way the estimate falls (mostly 0.7 to 1.0 of dp4a's time, in eight of 155 layers 1.05 to 1.24).
+// dense rows are the TMA unit's short runs.  For the others dp4a's time, from 2200 layers half up and 1400 half to even, which takes 1.22 of the estimate here:
+// 0.45 / 0.59 ps an output for 96 channels, 0.49 / 0.54 for 144 (widths that dp4a has forms of its own for) and 0.53 / 0.66 for others that its tile takes
+// whole (`dp4a_whole`), a quarter more for images below 200 pixels; 0.7 / 0.83 and more where it cuts pixels up; 0.49 / 0.57 for narrow tensors, more for small images and for 16 channels
+// (0.6 to 0.9, never less than here).  us here / there: 619 of 20x20x144 28.6 / 22.6, 928 of 20x20x96 29.8 / 22.1, 650 of 28x28x144 45.3 / 41.1, 1024 of
+// 80x80x48 201 / 170, 104 of 28x27x4000 231 / 219; 1024 of 112x112x32 171 / 207, 3715 of 14x14x144 60.8 / 67.0; half to even 160 of 57x56x144 55.9 / 50.3,
+// 836 of 28x28x112 45.7 / 56.2.  Narrow tensors below 64 M outputs stay here, whichever way the estimate falls (mostly 0.7 to 1.0 of dp4a's time, in
+// eight of 155 layers 1.05 to 1.24).
 inline bool dwm_pays(const DwmParams &p, int C, int out_h, int out_w, int n, bool half_even, bool dp4a_whole, int sms)
 {
     const double outputs = (double)n * out_h * out_w * C, pixels = (double)out_h * out_w;
     if (p.nw == 0 || p.CB % 64 == 0 || (C < 64 ? !p.flat : p.CB < 80))
         return false;
-    const double us = dwm_estimate_us(p, sms) * (half_even ? 1.1 : 1.0);
+    const double us = dwm_estimate_us(p, sms) * (half_even ? 1.22 : 1.0);
     if (C < 64)
-        return C == 16 || pixels <= 200 || outputs < (64 << 20) || us < 8.0 + 0.49e-6 * outputs;
-    if (dp4a_whole)
-        return us < 5.5 + (C == 96 ? 0.45e-6 : 0.51e-6) * (pixels <= 200 ? 1.25 : 1.0) * outputs;
-    return us < 8.0 + 0.7e-6 * (pixels <= 200 ? 1.12 : 1.0) * outputs;
+        return C == 16 || pixels <= 200 || outputs < (64 << 20) || us < 8.0 + (half_even ? 0.57e-6 : 0.49e-6) * outputs;
+    if (dp4a_whole) {
+        const double each = half_even ? (C == 96 ? 0.59e-6 : C == 144 ? 0.54e-6 : 0.66e-6) : (C == 96 ? 0.45e-6 : C == 144 ? 0.49e-6 : 0.53e-6);
+        return us < (half_even ? 7.5 : 6.5) + each * (pixels <= 200 ? 1.25 : 1.0) * outputs;
+    }
+    return us < 8.0 + (half_even ? 0.83e-6 : 0.7e-6) * (pixels <= 200 ? 1.12 : 1.0) * outputs;
 }
 
 } // namespace espdl

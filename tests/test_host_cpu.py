@@ -520,7 +520,8 @@ DEPTHWISE_TIMES = [
     (619, 20, 20, 144, 1, 28.6, 22.6), (2731, 20, 20, 144, 1, 101.7, 82.3), (928, 20, 20, 96, 1, 29.8, 22.1), (1365, 20, 20, 96, 1, 41.9, 29.7),
     (650, 28, 28, 144, 1, 45.3, 41.1), (1024, 80, 80, 48, 0, 201, 170), (3080, 57, 56, 32, 0, 178, 156), (104, 28, 27, 4000, 0, 231, 219), (64, 57, 58, 96, 1, 15.6, 13.8),
 ]
-DEPTHWISE_TIMES_HALF_EVEN = [(160, 57, 56, 144, 1, 55.9, 50.3), (41, 112, 112, 144, 1, 52.5, 48.1)]
+DEPTHWISE_TIMES_HALF_EVEN = [(650, 28, 28, 144, 1, 55.5, 48.9), (41, 112, 112, 144, 1, 52.5, 48.1), (836, 28, 28, 112, 1, 45.7, 56.2), (406, 28, 28, 112, 1, 24.1, 29.9),
+                             (61, 112, 112, 96, 1, 42.9, 47.9), (73, 112, 112, 80, 1, 47.4, 52.3), (2731, 20, 20, 144, 1, 121.5, 100.3)]
 
 
 def test_depthwise_layers_take_the_faster_kernel(tmp_path):
