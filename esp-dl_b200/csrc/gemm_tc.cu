@@ -15,12 +15,16 @@
 //             int32 in TMEM; tcgen05.commit releases the stage and, at the end of a tile, hands the accumulator over.
 //   warps 2-17 epilogue, four groups of four warps (a warp may read only its quarter of the 128 TMEM lanes).  With
 //             four accumulator buffers each group owns one buffer and every fourth tile; with two buffers two groups
-//             share a tile and split its columns.  Each thread owns one output row: tcgen05.ld, bias + ESP-DL's
-//             shift/round/saturate with per-channel shifts, ReLU, optional 8-bit LUT, 256-bit NHWC stores.
+//             share a tile and split its columns.  tcgen05.ld, bias + ESP-DL's shift/round/saturate with per-channel
+//             shifts, ReLU, optional 8-bit LUT, then a warp's 32 rows leave with a TMA store of their own.
 //             Most layers the network workloads bring are memory bound with a few hundred int8 outputs per input
 //             row, so the epilogue's instruction count per output decides the kernel's speed: per-channel constants
 //             are staged once in shared memory in a form that needs one add and one shift per output (see
-//             tc_common.cuh), and saturation happens inside the pack instruction.
+//             tc_common.cuh), and saturation happens inside the pack instruction.  A thread holds fragments of several rows
+//             (epilogue_frag), so that a constant read from shared memory serves four results; a thread holds a row
+//             where the columns are no multiple of 16, every image has its own filter, or a table is fused in.
+//
+// Short reductions over many rows keep the filter in shared memory (RES, plan_resident), a form of the kernel of its own.
 //
 // int16 operands: Blackwell tensor cores have no 16-bit integer MMA.  A pre-pass (pack.cu) writes each operand as two byte
 // planes, the input's x = 256*hi + lo (hi signed) and the shifted filter's w + 32768 = 256*uh + ul (both unsigned), and the
@@ -73,7 +77,7 @@ constexpr int BLOCK_M = 128;
 constexpr int EPI_WARPS = 16;
 constexpr int NUM_THREADS = 64 + EPI_WARPS * 32; // 1 TMA warp + 1 MMA warp + 16 epilogue warps
 constexpr int MAX_STAGES = 12;
-constexpr int MAX_ACC = 4;
+constexpr int MAX_ACC = 8;
 
 struct TcParams {
     int early; // bias, exponents and table are constants of the model: read ahead of the previous kernel's end
@@ -90,6 +94,7 @@ struct TcParams {
     int one_tile;   // a CTA has one tile: all four epilogue groups share it, and it is staged in the memory its loads came through
     int out_rows;   // the staging tiles leave row by row, a warp per row (rows that no TMA store can address), not as one TMA store
     int out_mask;   // swizzle mask of the staging tiles (7, 3, 1, 0)
+    int frag;       // staged epilogue on fragments: the columns of a tile are channels in the order frag_channel (map_b has five dimensions)
     void *out;
     long long ops;  // output row stride in elements
     const int *row_sum; // int16: sum of every row of A
@@ -98,18 +103,21 @@ struct TcParams {
     long long peer_delta[7]; // byte distance from `out` to the same buffer on other GPUs: every result row is stored there too
     int n_peer;
     unsigned *sched; // {next tile, CTAs done}: the tiles from static_tiles on are handed out by this counter; null = fixed walk
-    int static_tiles; // tiles walked in the fixed order (a multiple of the grid size; all of them without a counter)
+    int static_tiles; // tiles walked in the fixed order (a multiple of the grid size; all of them without a counter); resident: row tiles
+    int resident;     // the filter stays in shared memory, see plan_resident: column tiles of a CTA (0: tiles bring their part of it with them)
+    int in_turn;      // resident: epilogue groups take two accumulators in turn and stage pieces of 64 columns in two buffers, see plan_resident
+    int n_groups;     // resident: groups of CTAs, each with its own column tiles (resident_share)
     EpiConfig epi;
 };
 
 constexpr int TILE_RING = 32; // tile numbers on their way from the producer to the MMA issuer (more than stages + accumulators)
 
 // Epilogue of one int8 tile for outputs that cannot go through the staged path (piece widths that are not whole
-// 16-byte groups, unaligned rows, channels outside the fast form): rows are stored directly from registers.  Out of
-// line on purpose: the staged path in the kernel then carries none of this code's registers.
-template <bool EVEN>
-__device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastParam *fast_s, uint32_t fp_base, uint32_t t0, long long m, int n0,
-                                                  bool row_ok, bool fast, int parts, int part, bool allow_wide = true, uint32_t tbl = 0u)
+// 16-byte groups, unaligned rows, channels outside the fast form): rows are stored directly from registers.  WIDE: in 256-bit stores where they
+// are aligned, as part of the kernel only: in a function of its own such a store wrote its first word and no more (nvcc 12.9).
+template <bool EVEN, bool WIDE>
+__device__ __forceinline__ void epilogue_direct(const TcParams &p, const FastParam *fast_s, uint32_t fp_base, uint32_t t0, long long m, int n0,
+                                                bool row_ok, bool fast, int parts, int part, uint32_t tbl)
 {
     int8_t *orow = (int8_t *)p.out + m * p.ops + n0;
     const bool vec_ok = (p.ops % 16 == 0) && ((((uintptr_t)p.out) + n0) % 16 == 0);
@@ -118,7 +126,7 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
     const int out_align = (int)(amix & (~amix + 1));
     if (fast && !tbl && vec_ok && p.N % 16 == 0 && !p.res && p.n_peer == 0) {
         // whole 16-column groups, aligned rows, one-add-one-shift constants
-        const bool wide = allow_wide && (p.ops % 32 == 0) && ((((uintptr_t)p.out) + n0) % 32 == 0);
+        const bool wide = WIDE && (p.ops % 32 == 0) && ((((uintptr_t)p.out) + n0) % 32 == 0);
         const uint32_t fp = fp_base + (uint32_t)n0 * 8u;
         const int ncols = min(p.block_n, p.N - n0);
         if (p.epi.relu)
@@ -176,7 +184,7 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
                 if (count > 16)
                     store_bytes(prow + 16, pk + 4, count - 16, out_align);
             }
-            if (count > 0 && allow_wide) {
+            if (WIDE && count > 0) {
                 store_bytes(orow + c0, pk, count, out_align);
             } else if (count > 0) {
                 store_bytes(orow + c0, pk, min(count, 16), out_align);
@@ -184,6 +192,47 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
                     store_bytes(orow + c0 + 16, pk + 4, count - 16, out_align);
             }
         }
+    }
+}
+
+// Out of line: the other paths of a kernel then carry none of this code's registers.
+template <bool EVEN>
+__device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastParam *fast_s, uint32_t fp_base, uint32_t t0, long long m, int n0, bool row_ok, bool fast,
+                                                  int parts, int part, uint32_t tbl)
+{
+    epilogue_direct<EVEN, false>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, tbl);
+}
+
+// The general epilogue of a tile whose columns are channels in the order frag_channel (a channel outside the fast form, or tables of channels): 16 columns
+// at a time, put back into order.  Rows are 16-byte aligned, columns whole groups of 16.
+__device__ __noinline__ void epilogue_frag_general(const TcParams &p, uint32_t t0, long long m, int n0, bool row_ok, int parts, int part)
+{
+    const int ncols = min(p.block_n, p.N - n0);
+    int8_t *orow = (int8_t *)p.out + m * p.ops + n0;
+    const int8_t *rrow = p.res + m * p.rps + n0;
+#pragma unroll 1
+    for (int c0 = 16 * part; c0 < ncols; c0 += 16 * parts) {
+        int32_t u[16], v[16];
+        ld16(t0 + c0, u);
+        ld_wait16(u);
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[frag_channel(j)] = u[j];
+        uint32_t pk[4];
+        requant16_general(v, p.epi, n0 + c0, p.N, pk);
+        if (!row_ok)
+            continue;
+        if (p.res) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint32_t r = *(const uint32_t *)(rrow + c0 + 4 * q);
+                uint32_t w = 0;
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    w |= ((uint32_t)max(-128, min(127, (int)(int8_t)(pk[q] >> (8 * i)) + (int)(int8_t)(r >> (8 * i)))) & 0xffu) << (8 * i);
+                pk[q] = w;
+            }
+        }
+        *(uint4 *)(orow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
 }
 
@@ -250,7 +299,256 @@ __device__ __forceinline__ int requant_wide(int vh, int vm, int vl, int row_h, i
     return (int)__funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
 }
 
-template <bool I16, bool EVEN>
+// Whose column tiles a CTA has: group g has tiles g * resident .. + resident - 1 of the filter and a share of the CTAs in proportion to its columns.
+struct ResidentShare {
+    int first, across;   // column tiles
+    int member, members; // this CTA's place in its group
+};
+__device__ __forceinline__ ResidentShare resident_share(const TcParams &p)
+{
+    const int width = p.resident * p.block_n, grid = (int)gridDim.x;
+    int g = 0, begin = 0, end = grid;
+    for (; g < p.n_groups; g++, begin = end) {
+        end = g + 1 == p.n_groups ? grid : (int)((long long)grid * ((g + 1) * width) / p.N);
+        if ((int)blockIdx.x < end)
+            break;
+    }
+    return {g * p.resident, min(p.resident, p.n_tiles - g * p.resident), (int)blockIdx.x - begin, end - begin};
+}
+
+// The producer's walk with a resident filter (plan_resident): the CTA's column tiles of the filter once, then the rows of its tiles, each row tile
+// once for all neighbouring column tiles.  A ring entry is the first of `count` tiles.  With a counter the CTAs go through the first p.static_tiles row
+// tiles side by side and the tiles of the others are handed out one at a time, asked for one ahead; without, a CTA has an equal run of its
+// group's tiles.  False when a wait ran out.
+__device__ __forceinline__ bool produce_resident(const TcParams &p, const CUtensorMap &map_a, const CUtensorMap &map_b, uint32_t smem, uint64_t *full_bar,
+                                                 uint64_t *empty_bar, uint64_t *filter_bar, volatile int *ring_row, volatile int *ring_col)
+{
+    const int a_bytes = BLOCK_M * p.swz, b_bytes = p.block_n * p.swz;
+    const ResidentShare share = resident_share(p);
+    const int first = share.first, across = share.across, member = share.member, members = share.members;
+    if (!p.early)
+        grid_dep_wait(); // outside a model's plan a caller may just have written the filter
+    const uint32_t fbar = smem_u32(filter_bar), filter = smem + (uint32_t)(p.stages * a_bytes);
+    mbar_arrive_expect_tx(fbar, (uint32_t)(across * p.k_blocks * b_bytes));
+    for (int j = 0; j < across; j++)
+        for (int kb = 0; kb < p.k_blocks; kb++) {
+            const uint32_t to = filter + (uint32_t)((j * p.k_blocks + kb) * b_bytes);
+            if (p.frag)
+                tma_load_5d(to, &map_b, kb * p.swz, 0, 0, 0, (first + j) * p.block_n >> 4, fbar);
+            else
+                tma_load_3d(to, &map_b, kb * p.swz, (first + j) * p.block_n, 0, fbar);
+        }
+    grid_dep_wait();
+    int stage = 0, local = 0;
+    uint32_t phase = 0;
+    auto put = [&](int row, int j, int count) {
+        ring_row[local & (TILE_RING - 1)] = row;
+        ring_col[local & (TILE_RING - 1)] = first + j + (count << 16);
+        local++;
+        for (int kb = 0; kb < p.k_blocks; kb++) {
+            if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1))
+                return false;
+            const uint32_t bar = smem_u32(&full_bar[stage]);
+            mbar_arrive_expect_tx(bar, (uint32_t)a_bytes);
+            tma_load_3d(smem + (uint32_t)(stage * a_bytes), &map_a, kb * p.swz, row * BLOCK_M, 0, bar);
+            if (++stage == p.stages)
+                stage = 0, phase ^= 1;
+        }
+        return true;
+    };
+    const int total = p.m_tiles * across, fixed = p.static_tiles * across;
+    if (p.sched) {
+        int next = fixed + (int)atomicAdd(p.sched, 1u);
+        for (int row = member; row < p.static_tiles; row += members)
+            if (!put(row, 0, across))
+                return false;
+        while (next < total) {
+            const int row = next / across, j = next - row * across;
+            next = fixed + (int)atomicAdd(p.sched, 1u);
+            if (!put(row, j, 1))
+                return false;
+        }
+    } else {
+        const int end = (int)((long long)total * (member + 1) / members);
+        for (int u = (int)((long long)total * member / members); u < end;) {
+            const int row = u / across, j = u - row * across, count = min(across - j, end - u);
+            if (!put(row, j, count))
+                return false;
+            u += count;
+        }
+    }
+    ring_row[local & (TILE_RING - 1)] = -1; // the end: one stage without data
+    if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1))
+        return false;
+    mbar_arrive(smem_u32(&full_bar[stage]));
+    return true;
+}
+
+// The MMA issuer's side: the row tile's stages are waited for at the first of its tiles and given back at the last.  One thread does this beside warps
+// that keep its scheduler busy, so its instructions count: with the descriptors, barriers and divisions worked out for each tile it took 740 cycles for
+// a tile whose products take 256 (128 x 128, K = 128).
+__device__ __forceinline__ bool multiply_resident(const TcParams &p, uint32_t smem, uint32_t tmem_base, uint64_t *full_bar, uint64_t *empty_bar, uint64_t *filter_bar,
+                                                  uint64_t *tfull_bar, uint64_t *tempty_bar, volatile int *ring_row, volatile int *ring_col, volatile int *epi_row, volatile int *epi_col)
+{
+    const uint32_t idesc = idesc_i8(1, 1, BLOCK_M, p.block_n);
+    const int b_bytes = p.block_n * p.swz, ksteps = p.swz / 32;
+    const int last_ksteps = (p.K - (p.k_blocks - 1) * p.swz + 31) / 32; // see the other walk
+    const uint32_t a_units = (uint32_t)(BLOCK_M * p.swz) >> 4, b_units = (uint32_t)b_bytes >> 4; // 16-byte units, as descriptors count
+    const uint64_t a_desc = smem_desc_swizzled(smem, p.swz), b_desc = smem_desc_swizzled(smem + (uint32_t)(p.stages * BLOCK_M * p.swz), p.swz);
+    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), tfull0 = smem_u32(tfull_bar), tempty0 = smem_u32(tempty_bar);
+    const uint32_t filter_units = (uint32_t)p.k_blocks * b_units;
+    const int first = resident_share(p).first;
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 1, d0 = tmem_base;
+    if (!mbar_wait(smem_u32(filter_bar), 0))
+        return false;
+    long long w_tempty = 0, w_full = 0, w_issue = 0;
+    (void)w_tempty, (void)w_full, (void)w_issue;
+    TC_LAP_INIT;
+    for (int local = 0;; local++) {
+        TC_LAP(w_issue);
+        if (!mbar_wait(full0 + 8u * (uint32_t)stage, phase))
+            return false;
+        TC_LAP(w_full);
+        const int row = ring_row[local & (TILE_RING - 1)], cols = ring_col[local & (TILE_RING - 1)];
+        if (row < 0)
+            break;
+        const int col0 = cols & 0xffff, end = col0 + (cols >> 16);
+        uint64_t db = b_desc + (uint32_t)(col0 - first) * filter_units;
+        int s = stage;
+        uint32_t ph = phase;
+        for (int col = col0; col < end; col++) {
+            TC_LAP(w_issue);
+            if (!mbar_wait(tempty0 + 8u * (uint32_t)acc, acc_phase))
+                return false;
+            TC_LAP(w_tempty);
+            fence_after();
+            epi_row[acc] = row;
+            epi_col[acc] = col;
+            s = stage, ph = phase;
+            for (int kb = 0; kb < p.k_blocks; kb++) {
+                if (kb != 0 && col == col0) {
+                    if (!mbar_wait(full0 + 8u * (uint32_t)s, ph))
+                        return false;
+                    fence_after();
+                }
+                const uint64_t da = a_desc + (uint32_t)s * a_units;
+                const int ks = kb == p.k_blocks - 1 ? last_ksteps : ksteps;
+                mma_i8(d0, da, db, idesc, kb != 0 ? 1u : 0u);
+                if (ks > 1)
+                    mma_i8(d0, da + 2, db + 2, idesc, 1u);
+                if (ks > 2)
+                    mma_i8(d0, da + 4, db + 4, idesc, 1u);
+                if (ks > 3)
+                    mma_i8(d0, da + 6, db + 6, idesc, 1u);
+                if (col == end - 1)
+                    commit(empty0 + 8u * (uint32_t)s);
+                db += b_units;
+                if (++s == p.stages)
+                    s = 0, ph ^= 1;
+            }
+            commit(tfull0 + 8u * (uint32_t)acc);
+            mbar_arrive(tfull0 + 8u * (uint32_t)acc); // publishes epi_row / epi_col[acc]
+            d0 += (uint32_t)p.block_n;
+            if (++acc == p.acc_stages)
+                acc = 0, acc_phase ^= 1, d0 = tmem_base;
+        }
+        stage = s, phase = ph; // (a row tile may have more blocks than the ring has stages)
+    }
+    TC_REC(2, w_tempty);
+    TC_REC(3, w_full);
+    TC_REC(4, w_issue);
+    for (int a = 0; a < p.acc_stages; a++) { // every accumulator's epilogue groups are told, in the order they wait
+        if (!mbar_wait(tempty0 + 8u * (uint32_t)acc, acc_phase))
+            return false;
+        epi_row[acc] = -1;
+        mbar_arrive(tfull0 + 8u * (uint32_t)acc);
+        mbar_arrive(tfull0 + 8u * (uint32_t)acc);
+        if (++acc == p.acc_stages)
+            acc = 0, acc_phase ^= 1;
+    }
+    return true;
+}
+
+// The epilogue beside a resident filter: pieces of 64 columns.  A loop of its own, one for each KIND (0 plain, 1 fused table, 2 folded Add): what a warp does for
+// a piece besides requantising it stands between its tiles.  A warp stores its own 32 rows, so the warps of a group need no
+// barrier, and an accumulator is given back when its sums are in registers.  False when a wait ran out.
+template <bool EVEN, int KIND>
+__device__ __forceinline__ bool epilogue_resident(const TcParams &p, const CUtensorMap &map_out, uint32_t tmem_base, uint32_t fp_base, uint32_t stage, uint64_t *tfull_bar,
+                                                  uint64_t *tempty_bar, volatile int *epi_row, volatile int *epi_col, uint32_t tbl, int group, int lane_group, int lane)
+{
+    constexpr int PIECE = 64, PIECE_BYTES = BLOCK_M * PIECE;
+    const int sets = p.acc_stages / 2, last_part = 4 / sets - 1, set = group % sets, block_n = p.block_n, N = p.N, M = p.M - lane_group * 32;
+    const int floor_q = p.epi.relu ? 0 : INT_MIN;
+    const uint32_t tfull0 = smem_u32(tfull_bar), tempty0 = smem_u32(tempty_bar), tmem = tmem_base + ((uint32_t)(lane_group * 32) << 16);
+    int acc = set, part = group / sets;
+    uint32_t phase = 0, buf = stage + (uint32_t)(2 * group * PIECE_BYTES);
+    long long w_tfull = 0, w_work = 0, w_store = 0;
+    (void)w_tfull, (void)w_work, (void)w_store;
+    TC_LAP_INIT;
+    while (true) {
+        TC_LAP(w_work);
+        if (!mbar_wait(tfull0 + 8u * (uint32_t)acc, phase))
+            return false;
+        TC_LAP(w_tfull);
+        const int row = epi_row[acc];
+        if (row < 0)
+            break;
+        const int n = epi_col[acc] * block_n + part * PIECE, cols = min(PIECE, N - n);
+        fence_after();
+        if (elect_one())
+            bulk_wait_read_but_one(); // the store out of this buffer has read it, the other buffer's may be under way
+        __syncwarp();
+        TC_LAP(w_store);
+        const uint32_t t0 = tmem + (uint32_t)(acc * block_n + part * PIECE), fp = fp_base + (uint32_t)n * 8u;
+        auto loaded = [&] {
+            fence_before();
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(tempty0 + 8u * (uint32_t)acc);
+        };
+        if (KIND == 0 && cols == 64) {
+            epilogue_frag<PIECE, 64, EVEN>(t0, fp, buf, lane_group, lane, floor_q, loaded);
+        } else if (KIND == 0 && cols == 32) {
+            epilogue_frag<PIECE, 32, EVEN>(t0, fp, buf, lane_group, lane, floor_q, loaded);
+        } else {
+            if (KIND == 1)
+                epilogue_frag_lut<EVEN>(t0, fp, buf, lane_group, lane, cols, PIECE, 3u, floor_q, tbl);
+            else if (KIND == 2)
+                epilogue_frag_residual<EVEN>(t0, fp, buf, lane_group, lane, cols, PIECE, 3u, floor_q, p.res + (long long)row * BLOCK_M * p.rps + n, p.rps, p.M - row * BLOCK_M);
+            else
+                epilogue_frag_each(t0, fp, buf, lane_group, lane, cols, PIECE, 3u, [=](const int32_t *v, int i, const FragConst &k) { return frag_word<EVEN>(v, i, k, floor_q); });
+            loaded();
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (cols > 0 && row * BLOCK_M < M && elect_one()) { // rows >= M and columns >= N are clipped
+            tma_store_3d(&map_out, buf + (uint32_t)(lane_group * 32 * PIECE), n, row * BLOCK_M + lane_group * 32, 0);
+            bulk_commit();
+        }
+        __syncwarp();
+        // The other accumulator and buffer.  Pieces of a tile of 65 to 127 columns change hands, they are not two of 64.
+        part = last_part - part;
+        if (acc == set) {
+            acc = set + sets, buf += PIECE_BYTES;
+        } else {
+            acc = set, buf -= PIECE_BYTES;
+            phase ^= 1;
+        }
+    }
+    if (elect_one())
+        bulk_wait_all(); // shared memory stays allocated until the last store has left it
+    __syncwarp();
+    if (group == 0 && lane_group == 2 && lane == 0) {
+        TC_REC(5, w_tfull);
+        TC_REC(6, w_work);
+        TC_REC(7, w_store);
+    }
+    return true;
+}
+
+// RES: the filter is resident (plan_resident), a kernel of its own so that neither form carries the other's code.
+template <bool I16, bool EVEN, bool RES>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_a_lo, const __grid_constant__ CUtensorMap map_b_lo,
@@ -262,25 +560,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     constexpr int NACC = I16 ? 3 : 1;
     const int a_bytes = BLOCK_M * p.swz;
     const int b_bytes = p.block_n * p.swz;
-    const int stage_bytes = NPLANE * (a_bytes + b_bytes);
+    const int stage_bytes = RES ? a_bytes : NPLANE * (a_bytes + b_bytes);
+    const int load_bytes = p.stages * stage_bytes + (RES ? (p.resident * p.k_blocks * b_bytes + 1023) & ~1023 : 0); // the ring, then a resident filter
     const int n_pad = p.n_tiles * p.block_n;
-    uint8_t *out_stage = p.one_tile ? smem : smem + (size_t)p.stages * stage_bytes; // 4 tiles of [128][out_pw] bytes, 1024-byte aligned each
-    const int out_tile_bytes = (BLOCK_M * p.out_pw + 1023) & ~1023;
-    uint8_t *aux = smem + (size_t)p.stages * stage_bytes + (p.one_tile ? 0 : 4 * (size_t)out_tile_bytes);
+    uint8_t *out_stage = p.one_tile ? smem : smem + load_bytes; // 4 tiles of [128][out_pw] bytes, 1024-byte aligned each
+    const int out_tile_bytes = ((BLOCK_M * p.out_pw + 1023) & ~1023) << (RES ? p.in_turn : 0); // (in turn: of two buffers)
+    uint8_t *aux = smem + load_bytes + (p.one_tile ? 0 : 4 * (size_t)out_tile_bytes);
     FastParam *fast_s = (FastParam *)aux; // n_pad entries, 16-byte aligned (block_n % 16 == 0)
     WideParam *wide_s = (WideParam *)aux; // int16: the current tile's columns
     uint64_t *bars = (uint64_t *)(aux + (I16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)n_pad));
     uint64_t *full_bar = bars, *empty_bar = bars + MAX_STAGES, *tfull_bar = bars + 2 * MAX_STAGES, *tempty_bar = tfull_bar + MAX_ACC;
-    uint32_t *tmem_slot = (uint32_t *)(tempty_bar + MAX_ACC);
+    uint64_t *filter_bar = tempty_bar + MAX_ACC;
+    uint32_t *tmem_slot = (uint32_t *)(filter_bar + 2); // (16-byte aligned)
     int *slow_flag = (int *)(tmem_slot + 1);
     uint8_t *lut_s = (uint8_t *)(slow_flag + 3); // the fused 8-bit table, 256 bytes, 16-byte aligned
-    volatile int *tile_ring = (volatile int *)(lut_s + 256); // TILE_RING tile numbers, producer -> MMA issuer
-    volatile int *epi_tile = tile_ring + TILE_RING;          // MAX_ACC tile numbers, MMA issuer -> the accumulator's epilogue groups
+    volatile int *ring_row = (volatile int *)(lut_s + 256); // TILE_RING tiles, producer -> MMA issuer: row tile, column tile
+    volatile int *ring_col = ring_row + TILE_RING;          // (resident: the first of `col >> 16` neighbouring ones)
+    volatile int *epi_row = ring_col + TILE_RING;           // MAX_ACC tiles, MMA issuer -> the accumulator's epilogue groups
+    volatile int *epi_col = epi_row + MAX_ACC;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     TC_STAMP(0);
     const int total_tiles = p.batch * p.m_tiles * p.n_tiles;
-    const int parts = 4 / p.acc_stages; // epilogue groups that share one tile (they split its columns)
+    const int sets = RES && p.in_turn ? p.acc_stages / 2 : p.acc_stages;
+    const int parts = 4 / sets; // epilogue groups that share one tile (they split its columns)
     // Tiles are numbered n-fastest: tile = row_tile * n_tiles + n_tile with row_tile running over batch x m_tiles.  A CTA
     // starts with tile blockIdx.x; every further tile comes from a global counter (p.sched), so that an SM that runs
     // slower than the others (measured: one in ten takes 15-25 % longer per tile) gets fewer tiles instead of setting
@@ -298,6 +601,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             mbar_init(smem_u32(&tfull_bar[a]), 2);
             mbar_init(smem_u32(&tempty_bar[a]), 4 * parts);
         }
+        mbar_init(smem_u32(filter_bar), 1);
         *slow_flag = 0;
         fence_barrier_init();
     }
@@ -328,7 +632,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // ------------------------------------------------------------ TMA producer
         // One elected lane runs the loop and issues the copies.
         const bool issuer = elect_one();
-        if (issuer) {
+        if (RES && issuer) {
+            if (!produce_resident(p, map_a, map_b, smem_u32(smem), full_bar, empty_bar, filter_bar, ring_row, ring_col))
+                report_timeout(g_tc_error);
+        } else if (issuer) {
         grid_dep_wait(); // the previous kernel's output, and its use of the tile counter, before the first load
         int stage = 0;
         uint32_t phase = 0;
@@ -352,8 +659,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         int next = after(tile);
         int local = 0;
         for (; tile < total_tiles && ok; local++) {
-            tile_ring[local & (TILE_RING - 1)] = tile;
             const int rows = tile / p.n_tiles, nt = tile - rows * p.n_tiles;
+            ring_row[local & (TILE_RING - 1)] = rows;
+            ring_col[local & (TILE_RING - 1)] = nt;
             const int bi = p.batch == 1 ? 0 : rows / p.m_tiles;
             const int m0 = (p.batch == 1 ? rows : rows % p.m_tiles) * BLOCK_M;
             const int n0 = nt * p.block_n;
@@ -368,7 +676,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const uint32_t st = smem_u32(smem) + (uint32_t)(stage * stage_bytes);
                 mbar_arrive_expect_tx(bar, (uint32_t)stage_bytes);
                 tma_load_3d(st, &map_a, kb * p.swz, m0, bi, bar);
-                tma_load_3d(st + NPLANE * a_bytes, &map_b, kb * p.swz, n0, bi, bar);
+                if (!I16 && p.frag)
+                    tma_load_5d(st + a_bytes, &map_b, kb * p.swz, 0, 0, 0, n0 >> 4, bar);
+                else
+                    tma_load_3d(st + NPLANE * a_bytes, &map_b, kb * p.swz, n0, bi, bar);
                 if (I16) {
                     tma_load_3d(st + a_bytes, &map_a_lo, kb * p.swz, m0, bi, bar);
                     tma_load_3d(st + 2 * a_bytes + b_bytes, &map_b_lo, kb * p.swz, n0, bi, bar);
@@ -385,7 +696,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         if (ok) {
             // end of the walk: one stage without data whose ring entry is negative
-            tile_ring[local & (TILE_RING - 1)] = -1;
+            ring_row[local & (TILE_RING - 1)] = -1;
             if (mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1))
                 mbar_arrive(smem_u32(&full_bar[stage]));
             else
@@ -402,7 +713,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // One elected lane runs the loop and issues.  A tcgen05.mma of M = 128 costs it about 50 cycles (250 when the lane was chosen by its
         // number, see elect_one), so that N = 128 and wider keep the tensor cores busy.
         const bool issuer = elect_one();
-        if (issuer) {
+        if (RES && issuer) {
+            if (!multiply_resident(p, smem_u32(smem), tmem_base, full_bar, empty_bar, filter_bar, tfull_bar, tempty_bar, ring_row, ring_col, epi_row, epi_col))
+                report_timeout(g_tc_error);
+        } else if (issuer) {
         int stage = 0;
         uint32_t phase = 0;
         int acc = 0;
@@ -425,15 +739,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 break;
             }
             TC_LAP(w_full);
-            const int tile = tile_ring[local & (TILE_RING - 1)];
-            if (tile < 0) {
+            const int row = ring_row[local & (TILE_RING - 1)], col = ring_col[local & (TILE_RING - 1)];
+            if (row < 0) {
                 // end of the walk: every accumulator's epilogue groups are told, in the order they wait
                 for (int a = 0; a < p.acc_stages && ok; a++) {
                     if (!mbar_wait(smem_u32(&tempty_bar[acc]), acc_phase ^ 1)) {
                         ok = false;
                         break;
                     }
-                    epi_tile[acc] = -1;
+                    epi_row[acc] = -1;
                     mbar_arrive(smem_u32(&tfull_bar[acc]));
                     mbar_arrive(smem_u32(&tfull_bar[acc]));
                     if (++acc == p.acc_stages) {
@@ -449,7 +763,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             TC_LAP(w_tempty);
             fence_after();
-            epi_tile[acc] = tile;
+            epi_row[acc] = row;
+            epi_col[acc] = col;
             const uint32_t d0 = tmem_base + (uint32_t)(acc * NACC * p.block_n);
             for (int kb = 0; kb < p.k_blocks; kb++) {
                 TC_LAP(w_issue);
@@ -498,7 +813,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (!ok)
                 break;
             commit(smem_u32(&tfull_bar[acc]));
-            mbar_arrive(smem_u32(&tfull_bar[acc])); // publishes epi_tile[acc]
+            mbar_arrive(smem_u32(&tfull_bar[acc])); // publishes epi_row / epi_col[acc]
             if (++acc == p.acc_stages) {
                 acc = 0;
                 acc_phase ^= 1;
@@ -515,8 +830,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // ------------------------------------------------------------ epilogue (warps 2..17)
         const int ew = warp - 2;
         const int group = ew >> 2;               // 0..3
-        const int acc = group % p.acc_stages;    // accumulator buffer this group reads
-        const int part = group / p.acc_stages;   // which share of the tile's columns
+        const int own_acc = group % sets;        // accumulator buffer this group reads (in turn: with the one `sets` further)
+        const int part = group / sets;           // which share of the tile's columns
+        int turn = 0;
         const int lane_group = warp & 3;         // TMEM lanes this warp may read: 32*lane_group .. +31
         const int row_in_tile = lane_group * 32 + lane;
 
@@ -547,50 +863,78 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         long long w_tfull = 0, w_work = 0, w_store = 0;
         (void)w_tfull, (void)w_work, (void)w_store;
         TC_LAP_INIT;
-        while (ok) {
+        const bool own_loop = RES && fast && p.in_turn;
+        if (RES && own_loop) {
+            const uint32_t stage = smem_u32(out_stage), tbl = smem_u32(lut_s);
+            if (p.epi.lut)
+                ok = epilogue_resident<EVEN, 1>(p, map_out, tmem_base, fp_base, stage, tfull_bar, tempty_bar, epi_row, epi_col, tbl, group, lane_group, lane);
+            else if (p.res)
+                ok = epilogue_resident<EVEN, 2>(p, map_out, tmem_base, fp_base, stage, tfull_bar, tempty_bar, epi_row, epi_col, tbl, group, lane_group, lane);
+            else
+                ok = epilogue_resident<EVEN, 0>(p, map_out, tmem_base, fp_base, stage, tfull_bar, tempty_bar, epi_row, epi_col, tbl, group, lane_group, lane);
+        }
+        while (ok && !own_loop) {
+            const int acc = RES ? own_acc + turn : own_acc;
             TC_LAP(w_work);
             if (!mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase)) {
                 ok = false;
                 break;
             }
             TC_LAP(w_tfull);
-            const int tile = epi_tile[acc];
-            if (tile < 0)
+            const int rows = epi_row[acc];
+            if (rows < 0)
                 break;
-            const int rows = tile / p.n_tiles, nt = tile - rows * p.n_tiles;
+            const int nt = epi_col[acc];
             const int bi = p.batch == 1 ? 0 : rows / p.m_tiles;
             const int m0 = (p.batch == 1 ? rows : rows % p.m_tiles) * BLOCK_M;
             const int n0 = nt * p.block_n;
-            acc_phase ^= 1;
             fence_after();
             const bool row_ok = m0 + row_in_tile < p.M;
             const long long m = (long long)bi * p.M + m0 + row_in_tile; // row of the output tensor
             const uint32_t t0 = tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)(acc * NACC * p.block_n);
+            acc_phase ^= 1;
+            if (RES && p.in_turn) { // (general epilogue: a channel outside the fast form)
+                if (!turn)
+                    acc_phase ^= 1;
+                turn = sets - turn;
+            }
             if (!I16) {
                 if (fast && p.out_pw) {
-                    // staged: requantise into this group's shared-memory tile, one TMA store per piece
-                    const bool leader = (ew & 3) == 0 && lane == 0;
+                    // staged: every warp requantises its 32 rows into its part of the group's shared-memory tile and sends them off with a TMA store of
+                    // its own.  (One store for the four warps took two barriers a tile, at which a group stood for a seventh of its time.)
                     const uint32_t buf = smem_u32(out_stage + (size_t)group * out_tile_bytes);
-                    if (leader && !p.out_rows)
-                        bulk_wait_read_all(); // the previous store out of this tile has been read
-                    named_bar(2 + group, 128);
-                    TC_LAP(w_store);
                     const int col0 = part * p.out_pw;
-                    const uint32_t fpp = fp_base + (uint32_t)(n0 + col0) * 8u;
+                    if (!p.out_rows && elect_one())
+                        bulk_wait_read_all(); // the previous store out of these rows has read them
+                    __syncwarp();
+                    TC_LAP(w_store);
                     const int floor_q = p.epi.relu ? 0 : INT_MIN;
-                    if (p.epi.lut) {
-                        epilogue_stage_lut<EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
+                    if (p.frag) {
+                        const int cols = min(p.block_n / parts, p.N - (n0 + col0));
+                        const uint32_t tc = t0 + col0, fpp = fp_base + (uint32_t)(n0 + col0) * 8u;
+                        if (p.res)
+                            epilogue_frag_residual<EVEN>(tc, fpp, buf, lane_group, lane, cols, p.out_pw, (uint32_t)p.out_mask, floor_q, p.res + (long long)m0 * p.rps + n0 + col0,
+                                                         p.rps, p.M - m0);
+                        else if (p.out_pw == 128 && cols == 128)
+                            epilogue_frag<128, 128, EVEN>(tc, fpp, buf, lane_group, lane, floor_q, [] {});
+                        else if (p.out_pw == 64 && cols == 64)
+                            epilogue_frag<64, 64, EVEN>(tc, fpp, buf, lane_group, lane, floor_q, [] {});
+                        else
+                            epilogue_frag_each(tc, fpp, buf, lane_group, lane, cols, p.out_pw, (uint32_t)p.out_mask,
+                                               [=](const int32_t *v, int i, const FragConst &k) { return frag_word<EVEN>(v, i, k, floor_q); });
+                    } else if (p.epi.lut) {
+                        epilogue_stage_lut<EVEN>(t0 + col0, fp_base + (uint32_t)(n0 + col0) * 8u, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q, smem_u32(lut_s));
                     } else if (p.res)
-                        epilogue_stage_residual<EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q,
+                        epilogue_stage_residual<EVEN>(t0 + col0, fp_base + (uint32_t)(n0 + col0) * 8u, buf, row_in_tile, p.out_pw, (uint32_t)p.out_mask, floor_q,
                                                 p.res + m * p.rps + n0 + col0, row_ok, p.N - (n0 + col0));
                     else if (p.out_pw == 128)
-                        epilogue_stage<128, EVEN>(t0 + col0, fpp, buf, row_in_tile, 128, floor_q);
+                        epilogue_stage<128, EVEN>(t0 + col0, fp_base + (uint32_t)(n0 + col0) * 8u, buf, row_in_tile, 128, floor_q);
                     else if (p.out_pw == 96)
-                        epilogue_stage<96, EVEN>(t0 + col0, fpp, buf, row_in_tile, 96, floor_q);
+                        epilogue_stage<96, EVEN>(t0 + col0, fp_base + (uint32_t)(n0 + col0) * 8u, buf, row_in_tile, 96, floor_q);
                     else if (p.out_pw == 64)
-                        epilogue_stage<64, EVEN>(t0 + col0, fpp, buf, row_in_tile, 64, floor_q);
+                        epilogue_stage<64, EVEN>(t0 + col0, fp_base + (uint32_t)(n0 + col0) * 8u, buf, row_in_tile, 64, floor_q);
                     else
-                        epilogue_stage<0, EVEN>(t0 + col0, fpp, buf, row_in_tile, p.out_pw, floor_q);
+                        epilogue_stage<0, EVEN>(t0 + col0, fp_base + (uint32_t)(n0 + col0) * 8u, buf, row_in_tile, p.out_pw, floor_q);
                     // the accumulator is free as soon as this warp's TMEM loads are done: hand it back before the
                     // shared-memory tile is completed and stored, so that the MMAs of the tile after next start earlier
                     fence_before();
@@ -598,7 +942,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (lane == 0)
                         mbar_arrive(smem_u32(&tempty_bar[acc]));
                     if (p.out_rows) {
-                        named_bar(2 + group, 128);
                         const int len = min(p.out_pw, p.N - (n0 + col0)), rows_left = min(32, p.M - m0 - lane_group * 32);
                         int8_t *dst = (int8_t *)p.out + ((long long)bi * p.M + m0 + lane_group * 32) * p.ops + n0 + col0;
                         if (len > 0)
@@ -607,14 +950,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         continue;
                     }
                     fence_async_smem();
-                    named_bar(2 + group, 128);
-                    if (leader) {
-                        tma_store_3d(&map_out, buf, n0 + col0, m0, bi); // rows >= M and columns >= N are clipped
+                    __syncwarp();
+                    if (m0 + lane_group * 32 < p.M && n0 + col0 < p.N && elect_one()) { // rows >= M and columns >= N are clipped
+                        tma_store_3d(&map_out, buf + (uint32_t)(lane_group * 32 * p.out_pw), n0 + col0, m0 + lane_group * 32, bi);
                         bulk_commit();
                     }
+                    __syncwarp();
                     continue;
                 }
-                epilogue_direct_tile<EVEN>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, true, p.epi.lut ? smem_u32(lut_s) : 0u);
+                if (p.frag)
+                    epilogue_frag_general(p, t0, m, n0, row_ok, parts, part);
+                else if (RES)
+                    epilogue_direct_tile<EVEN>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, p.epi.lut ? smem_u32(lut_s) : 0u);
+                else
+                    epilogue_direct<EVEN, true>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, p.epi.lut ? smem_u32(lut_s) : 0u);
             } else {
                 // all groups share the tile: constants of its columns, then 16 columns at a time into a staging tile of [128][2 * block_n]
                 // bytes, then whole rows
@@ -706,14 +1055,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         if (!ok && lane == 0)
             report_timeout(g_tc_error);
-        if (ew == 0 && lane == 0) {
+        if (ew == 0 && lane == 0 && !own_loop) {
             TC_LAP(w_work);
             TC_REC(5, w_tfull);
             TC_REC(6, w_work);
             TC_REC(7, w_store);
         }
-        if (p.out_pw && !p.out_rows && (ew & 3) == 0 && lane == 0)
+        if (I16 ? !p.out_rows && et0 == 0 : p.out_pw && !p.out_rows && elect_one())
             bulk_wait_all(); // shared memory stays allocated until the last store has left it
+        __syncwarp();
     }
 
     fence_before();
@@ -945,7 +1295,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const long long m = (long long)m0 + row_in_tile;
             const uint32_t t0 = tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)(acc * p.block_n);
             // 128-bit stores: in this kernel the 256-bit form stored only the first word of each 32 bytes
-            epilogue_direct_tile<false>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, false);
+            epilogue_direct_tile<false>(p, fast_s, fp_base, t0, m, n0, row_ok, fast, parts, part, 0u);
             fence_before();
             __syncwarp();
             if (lane == 0)
@@ -1008,6 +1358,25 @@ int make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, u
     return ESPDL_OK;
 }
 
+// The filter's rows in the order of the fragments (frag_channel): [N / 16][2][4][2] rows of K bytes, a box of box_rows of them.
+int make_frag_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows, int swz)
+{
+    EncodeTiledFn enc = get_encode();
+    if (!enc)
+        return set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled entry point not found");
+    cuuint64_t dims[5] = {cols, 2, 4, 2, rows / 16};
+    cuuint64_t strides[4] = {cols, 4 * cols, 2 * cols, 16 * cols};
+    cuuint32_t box[5] = {(cuuint32_t)swz, 2, 4, 2, box_rows / 16};
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUtensorMapSwizzle sw = swz == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (swz == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+    if (enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
+        return ESPDL_ERR_CUDA;
+    }
+    return ESPDL_OK;
+}
+
 // Bytes of K per stage row (= TMA box width = swizzle width).  Wide rows move fastest through the TMA unit, so
 // 128 is used as soon as K fills three quarters of such a row; columns past K are zero-filled, not fetched.
 int pick_swz(int K)
@@ -1025,7 +1394,44 @@ constexpr size_t SMEM_BUDGET_DEEP = 225 * 1024; // long reductions with direct r
 
 size_t aux_bytes(const TcParams &p, bool i16 = false)
 {
-    return (i16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)p.n_tiles * p.block_n) + (2 * MAX_STAGES + 2 * MAX_ACC) * 8 + 32 + 256 + (TILE_RING + MAX_ACC) * 4;
+    return (i16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)p.n_tiles * p.block_n) + (2 * MAX_STAGES + 2 * MAX_ACC + 2) * 8 + 32 + 256 + 2 * (TILE_RING + MAX_ACC) * 4;
+}
+
+// A filter that stays in shared memory.  With tiles that bring their part of the filter along, a tile of a short reduction loads more of the filter than
+// of the rows, two or three stages hold it all, and the next tile's loads come too late (401408 rows of 128 -> 768: the MMA issuer
+// waited for loads half of the time).  Here a CTA loads as many column tiles as fit beside a ring of row tiles once - groups of CTAs share the column
+// tiles out where they do not all fit - and every row tile serves all of them.  Tiles are 128 columns wide: two accumulators for each of two sets of
+// epilogue warps, so that a warp finds the next tile's sums ready (64 columns and fewer: for each of four).  us before / after (floor: bytes): 401408 x 128 ->
+// 768 93 / 73 (55), 802816 x 96 -> 96 56 / 28 (24), 200704 x 64 -> 384 27.4 / 23.5 (14), 50176 x 320 -> 1280 46 / 30 (12), 65536 x 384 -> 384 24 / 15 (8).
+// From two row tiles a CTA on: below, the filter is not used often enough (8192 x 256 -> 1024: 7.1 us, 8.5 resident).
+void plan_resident(TcParams &p)
+{
+    p.resident = p.in_turn = 0, p.n_groups = 1;
+    if (p.one_tile || !p.out_pw || p.batch != 1)
+        return;
+    TcParams q = p;
+    if (q.N % 16 == 0 && !q.out_rows) {
+        q.block_n = min(128, q.N), q.n_tiles = (q.N + q.block_n - 1) / q.block_n;
+        q.in_turn = 1, q.acc_stages = q.block_n > 64 ? 4 : 8, q.tmem_cols = 512;
+        q.out_pw = 64, q.out_mask = 3;
+    }
+    const size_t a_stage = (size_t)BLOCK_M * q.swz, b_tile = (size_t)q.block_n * q.k_blocks * q.swz;
+    const size_t room = SMEM_BUDGET_DEEP - aux_bytes(q) - 4 * ((size_t)((BLOCK_M * q.out_pw + 1023) & ~1023) << q.in_turn) - 2048;
+    // one column tile: a row tile's stages are free as soon as they are multiplied; several: two row tiles
+    const size_t ring = a_stage * (q.n_tiles == 1 ? 4 : max(2 * q.k_blocks, 3));
+    if (room < ring + b_tile)
+        return;
+    const int fit = (int)min((long long)q.n_tiles, (long long)((room - ring) / b_tile));
+    q.n_groups = (q.n_tiles + fit - 1) / fit;
+    q.resident = (q.n_tiles + q.n_groups - 1) / q.n_groups;
+    q.n_groups = (q.n_tiles + q.resident - 1) / q.resident;
+    if (q.n_groups > num_sms() / 8 || (long long)q.m_tiles * q.n_groups < 2ll * num_sms())
+        return;
+    // more memory than the other plans take only for what has to fit: what it leaves of an SM's serves kernels of parallel branches
+    q.stages = (int)min((size_t)MAX_STAGES, max(ring, room - q.resident * b_tile - min(room - q.resident * b_tile, SMEM_BUDGET_DEEP - SMEM_BUDGET)) / a_stage);
+    if (q.resident > 1 && q.stages < 2 * q.k_blocks) // (more stages than there are barriers)
+        return;
+    p = q;
 }
 
 bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
@@ -1111,6 +1517,13 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     }
     if (!i16 && p.out_rows && p.out_pw && stages < 4)
         stages = (int)((SMEM_BUDGET_DEEP - aux_bytes(p) - out_bytes - 1024) / stage_bytes);
+    p.resident = p.in_turn = 0;
+    if (!i16)
+        plan_resident(p);
+    if (p.resident) {
+        p.frag = p.N % 16 == 0;
+        return true;
+    }
     if (!i16 && !p.one_tile && p.out_pw && !p.out_rows && p.k_blocks > 2 && stages < 4) {
         // a long reduction needs the deep load pipeline more than the output needs staging
         p.out_pw = 0, p.out_mask = 0, out_bytes = 0;
@@ -1119,6 +1532,8 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     if (stages < 2)
         return false;
     p.stages = stages > MAX_STAGES ? MAX_STAGES : stages;
+    // (a fused table's lookups outweigh the constants: a network of such layers at 16 images 817 us by rows, 822 on fragments)
+    p.frag = !i16 && p.out_pw && !batched && p.N % 16 == 0 && !d.lut;
     return true;
 }
 
@@ -1143,7 +1558,7 @@ bool pair_plan(const espdl_conv_desc &d, TcParams &p)
     if (p.acc_stages < 2)
         return false;
     p.tmem_cols = 512;
-    p.out_pw = 0, p.out_mask = 0;
+    p.out_pw = 0, p.out_mask = 0, p.frag = 0, p.resident = p.in_turn = 0;
     const size_t stage_bytes = (size_t)(BLOCK_M + p.block_n / 2) * p.swz;
     const int stages = (int)((SMEM_BUDGET_DEEP - aux_bytes(p) - 1024) / stage_bytes);
     if (stages < 3)
@@ -1262,8 +1677,10 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
         if ((st = make_map(&ma, d.input, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)ips, BLOCK_M, (uint32_t)p.swz, p.swz, (uint64_t)p.batch,
                            (uint64_t)p.M * ips)))
             return st;
-        if ((st = make_map(&mb, d.filter, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, (uint32_t)p.block_n, (uint32_t)p.swz, p.swz, (uint64_t)p.batch,
-                           (uint64_t)d.filter_image_stride)))
+        st = p.frag ? make_frag_map(&mb, d.filter, (uint64_t)p.N, (uint64_t)p.K, (uint32_t)p.block_n, p.swz)
+                    : make_map(&mb, d.filter, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, (uint32_t)p.block_n, (uint32_t)p.swz, p.swz, (uint64_t)p.batch,
+                               (uint64_t)d.filter_image_stride);
+        if (st)
             return st;
         ma_lo = ma, mb_lo = mb;
     } else if ((st = make_map(&ma, o->a_hi, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, BLOCK_M, (uint32_t)p.swz, p.swz)) ||
@@ -1273,11 +1690,12 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
         return st;
     }
     const size_t stage_bytes = (size_t)(i16 ? 2 : 1) * (BLOCK_M + p.block_n) * p.swz;
-    size_t smem = 1024 + (size_t)p.stages * stage_bytes + (p.one_tile ? 0 : 4 * (size_t)((BLOCK_M * p.out_pw + 1023) & ~1023)) + aux_bytes(p, i16);
+    const size_t filter_bytes = p.resident ? ((size_t)p.resident * p.k_blocks * p.block_n * p.swz + 1023) & ~(size_t)1023 : 0;
+    size_t smem = 1024 + (size_t)p.stages * (p.resident ? (size_t)BLOCK_M * p.swz : stage_bytes) + filter_bytes + (p.one_tile ? 0 : 4 * ((size_t)((BLOCK_M * p.out_pw + 1023) & ~1023) << p.in_turn)) + aux_bytes(p, i16);
     CUtensorMap mo = ma;
     if (!i16 && p.out_pw && !p.out_rows) {
         const int osw = p.out_pw == 128 ? 128 : (p.out_pw == 64 ? 64 : 0);
-        if ((st = make_map(&mo, d.output, (uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.ops, BLOCK_M, (uint32_t)p.out_pw, osw, (uint64_t)p.batch,
+        if ((st = make_map(&mo, d.output, (uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.ops, 32, (uint32_t)p.out_pw, osw, (uint64_t)p.batch,
                            (uint64_t)p.M * (uint64_t)p.ops)))
             return st;
     }
@@ -1292,23 +1710,26 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
     // three quarters of the tiles in the fixed order, the last quarter to whichever SM is free
     p.sched = all_tiles >= 4ll * grid && all_tiles < (1ll << 30) ? sched_counters(s) : nullptr;
     p.static_tiles = p.sched ? (int)(all_tiles * 3 / 4 / grid) * grid : (int)all_tiles;
+    if (p.resident) { // row tiles; a group of CTAs among several has no counter of its own (65536 x 256 -> 256 without / with one: 10.8 / 11.4 us)
+        if (p.n_groups > 1 || p.m_tiles < 4 * grid)
+            p.sched = nullptr;
+        p.static_tiles = p.sched ? p.m_tiles * 3ll / 4 / grid * grid : p.m_tiles;
+    }
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(gemm_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
-        if (attr_err == cudaSuccess)
-            attr_err = cudaFuncSetAttribute(gemm_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
-        if (attr_err == cudaSuccess)
-            attr_err = cudaFuncSetAttribute(gemm_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
-        if (attr_err == cudaSuccess)
-            attr_err = cudaFuncSetAttribute(gemm_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
+        for (auto k : {gemm_tc_kernel<false, false, false>, gemm_tc_kernel<false, true, false>, gemm_tc_kernel<true, false, false>, gemm_tc_kernel<true, true, false>,
+                       gemm_tc_kernel<false, false, true>, gemm_tc_kernel<false, true, true>})
+            if (attr_err == cudaSuccess)
+                attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_BUDGET_DEEP + 2048));
     });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(gemm_tc_kernel)");
-    if (i16)
-        launch_overlapped(p.epi.half_even ? gemm_tc_kernel<true, true> : gemm_tc_kernel<true, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
-    else
-        launch_overlapped(p.epi.half_even ? gemm_tc_kernel<false, true> : gemm_tc_kernel<false, false>, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
+    const bool even = p.epi.half_even;
+    const auto kernel = i16 ? (even ? gemm_tc_kernel<true, true, false> : gemm_tc_kernel<true, false, false>)
+        : p.resident        ? (even ? gemm_tc_kernel<false, true, true> : gemm_tc_kernel<false, false, true>)
+                            : (even ? gemm_tc_kernel<false, true, false> : gemm_tc_kernel<false, false, false>);
+    launch_overlapped(kernel, dim3(grid), dim3(NUM_THREADS), smem, s, ma, mb, ma_lo, mb_lo, mo, p);
     count_launch();
     return check_launch("gemm_tc");
 }

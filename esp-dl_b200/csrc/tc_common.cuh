@@ -123,6 +123,7 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t sr
 
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void named_bar(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
@@ -591,6 +592,191 @@ __device__ __forceinline__ void epilogue_stage_residual(uint32_t t0, uint32_t fp
         uint32_t off = rbase + (uint32_t)c;
         off ^= ((off >> 7) & mask) << 4;
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + off), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+    }
+}
+
+// Fragments: 16 TMEM lanes x 8-column blocks, of which thread t of the warp receives rows t / 4 and t / 4 + 8, columns 2 * (t % 4) and the next:
+// v[4 * block + 0 .. 1] of the first row, v[4 * block + 2 .. 3] of the second.  A thread then meets few channels and several rows of each, so the
+// per-channel constants are read from shared memory once for four rows: the row-per-thread form reads 8 bytes a result, two of the 2.5 data-pipe
+// cycles of a warp's results, and that pipe bounds it (89 % busy).  Two neighbouring columns would leave as 2-byte stores (slower than all that is saved);
+// the kernels therefore load the filter's rows in the order frag_channel, by which two blocks give a thread four consecutive channels.
+__device__ __forceinline__ void ld_frag4(uint32_t taddr, int32_t *v) // four blocks, 32 columns
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void ld_frag2(uint32_t taddr, int32_t *v) // two blocks, 16 columns
+{
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+// The channel of a group of 16 whose sums are in column j of its two blocks.  A 5-D view of the filter (row pitch p: strides p, 4p, 2p, 16p over 2, 4, 2
+// and N / 16 rows) lets one TMA copy bring the rows in this order.
+__host__ __device__ constexpr int frag_channel(int j) { return 4 * ((j & 7) >> 1) + 2 * (j >> 3) + (j & 1); }
+
+// {bias_half, shift} of a thread's four channels of a 16-column group.
+struct FragConst {
+    int b[4], s[4];
+    __device__ __forceinline__ void load(uint32_t fp)
+    {
+        asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(b[0]), "=r"(s[0]), "=r"(b[1]), "=r"(s[1]) : "r"(fp));
+        asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(b[2]), "=r"(s[2]), "=r"(b[3]), "=r"(s[3]) : "r"(fp + 16));
+    }
+};
+
+// The word of one row (0: t / 4, 1: t / 4 + 8) of a 16-column group whose two blocks are v[0 .. 3] and v[4 .. 7].
+template <bool EVEN>
+__device__ __forceinline__ uint32_t frag_word(const int32_t *v, int row, const FragConst &c, int floor_q)
+{
+    const int r0 = shift_fast<EVEN>(__viaddmax_s32(v[2 * row], c.b[0], floor_q), c.s[0]);
+    const int r1 = shift_fast<EVEN>(__viaddmax_s32(v[2 * row + 1], c.b[1], floor_q), c.s[1]);
+    const int r2 = shift_fast<EVEN>(__viaddmax_s32(v[2 * row + 4], c.b[2], floor_q), c.s[2]);
+    const int r3 = shift_fast<EVEN>(__viaddmax_s32(v[2 * row + 5], c.b[3], floor_q), c.s[3]);
+    uint32_t hi, w;
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(r3), "r"(r2));
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(r1), "r"(r0), "r"(hi));
+    return w;
+}
+
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
+// Staged epilogue on fragments: COLS columns (a multiple of 16) of the warp's 32 lanes from TMEM address t0, into its rows of the [128][PITCH] tile at
+// `buf` (see epilogue_stage; rows 8 apart have the same swizzle, and the eight rows of a store meet no bank conflict
+// with these two pitches; rows of 96 bytes do: a fifth slower).  `fp`: constants of the first channel.  `loaded` is called once the sums have left TMEM.
+template <int PITCH, int COLS, bool EVEN, typename F>
+__device__ __forceinline__ void epilogue_frag(uint32_t t0, uint32_t fp, uint32_t buf, int lane_group, int lane, int floor_q, F loaded)
+{
+    static_assert(PITCH == 128 || PITCH == 64, "");
+    const uint32_t r = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u;
+    const uint32_t rx = PITCH == 128 ? r << 4 : (r >> 1) << 4;
+    const uint32_t rb = buf + ((uint32_t)lane_group * 32u + r) * PITCH + 4u * t, hi = t0 + (16u << 16);
+    fp += 32u * t;
+    int32_t va[16], vb[16];
+    if (COLS >= 32)
+        ld_frag4(t0, va);
+#pragma unroll
+    for (int c = 0; c + 32 <= COLS; c += 32) {
+        FragConst k0, k1;
+        k0.load(fp + (uint32_t)c * 8u);
+        k1.load(fp + (uint32_t)c * 8u + 128u);
+        const uint32_t p0 = rb + ((uint32_t)c ^ rx), p1 = rb + ((uint32_t)(c + 16) ^ rx);
+        ld_wait16(va);
+        ld_frag4(hi + c, vb);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            sts32(p0 + 8 * PITCH * i, frag_word<EVEN>(va, i, k0, floor_q));
+            sts32(p1 + 8 * PITCH * i, frag_word<EVEN>(va + 8, i, k1, floor_q));
+        }
+        ld_wait16(vb);
+        if (c + 64 <= COLS) {
+            ld_frag4(t0 + c + 32, va);
+        } else if (COLS & 16) {
+            ld_frag2(t0 + c + 32, va);
+            ld_frag2(hi + c + 32, va + 8);
+        } else {
+            loaded();
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            sts32(p0 + 8 * PITCH * (i + 2), frag_word<EVEN>(vb, i, k0, floor_q));
+            sts32(p1 + 8 * PITCH * (i + 2), frag_word<EVEN>(vb + 8, i, k1, floor_q));
+        }
+    }
+    if (COLS & 16) {
+        constexpr uint32_t c = COLS & ~31;
+        if (COLS < 32) {
+            ld_frag2(t0, va);
+            ld_frag2(hi, va + 8);
+        }
+        FragConst k;
+        k.load(fp + c * 8u);
+        ld_wait16(va);
+        loaded();
+#pragma unroll
+        for (int i = 0; i < 4; i++) sts32(rb + ((uint32_t)c ^ rx) + 8 * PITCH * i, frag_word<EVEN>(va + 8 * (i >> 1), i & 1, k, floor_q));
+    }
+}
+
+// Any pitch (a multiple of 16; `mask`: swizzle of the tile), 16 columns at a time; f(v, i, k) makes the word of row i of a group.
+template <typename F>
+__device__ __forceinline__ void epilogue_frag_each(uint32_t t0, uint32_t fp, uint32_t buf, int lane_group, int lane, int cols, int pitch, uint32_t mask, F f)
+{
+    const uint32_t r = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, row0 = (uint32_t)lane_group * 32u + r;
+    const uint32_t rx = ((row0 * (uint32_t)pitch) >> 7 & mask) << 4, rb = buf + row0 * (uint32_t)pitch + 4u * t;
+    fp += 32u * t;
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 16) {
+        int32_t v[16];
+        ld_frag2(t0 + c, v);
+        ld_frag2(t0 + (16u << 16) + c, v + 8);
+        FragConst k;
+        k.load(fp + (uint32_t)c * 8u);
+        ld_wait16(v);
+        const uint32_t at = rb + ((uint32_t)c ^ rx);
+#pragma unroll
+        for (int i = 0; i < 4; i++) sts32(at + (uint32_t)(8 * i * pitch), f(v + 8 * (i >> 1), i & 1, k));
+    }
+}
+
+// With a fused table (see epilogue_stage_lut).
+template <bool EVEN>
+static __device__ __noinline__ void epilogue_frag_lut(uint32_t t0, uint32_t fp, uint32_t buf, int lane_group, int lane, int cols, int pitch, uint32_t mask,
+                                                      int floor_q, uint32_t tbl)
+{
+    epilogue_frag_each(t0, fp, buf, lane_group, lane, cols, pitch, mask,
+                       [=](const int32_t *v, int i, const FragConst &k) { return lut4(frag_word<EVEN>(v, i, k, floor_q), tbl); });
+}
+
+// With a folded Add (see epilogue_stage_residual): `res` = the residual of the tile's first row at the piece's first column, rows `rps` apart and 4-byte
+// aligned; rows from `rows` on have none.  The words of the next 16 columns are on their way while these are summed.
+template <bool EVEN>
+__device__ __forceinline__ void epilogue_frag_residual(uint32_t t0, uint32_t fp, uint32_t buf, int lane_group, int lane, int cols, int pitch, uint32_t mask,
+                                                       int floor_q, const int8_t *res, long long rps, int rows)
+{
+    const uint32_t r = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, row0 = (uint32_t)lane_group * 32u + r;
+    const uint32_t rx = ((row0 * (uint32_t)pitch) >> 7 & mask) << 4, rb = buf + row0 * (uint32_t)pitch + 4u * t;
+    fp += 32u * t;
+    res += (long long)row0 * rps + 4u * t;
+    uint32_t next[4];
+    auto fetch = [&](int c) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) next[i] = (int)row0 + 8 * i < rows ? __ldg((const uint32_t *)(res + 8 * i * rps + c)) : 0u;
+    };
+    if (cols > 0)
+        fetch(0);
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 16) {
+        int32_t v[16];
+        ld_frag2(t0 + c, v);
+        ld_frag2(t0 + (16u << 16) + c, v + 8);
+        FragConst k;
+        k.load(fp + (uint32_t)c * 8u);
+        uint32_t rr[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) rr[i] = next[i];
+        if (c + 16 < cols)
+            fetch(c + 16);
+        ld_wait16(v);
+        const uint32_t at = rb + ((uint32_t)c ^ rx);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int32_t *a = v + 8 * (i >> 1) + 2 * (i & 1);
+            int q[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                q[j] = min(max(shift_fast<EVEN>(__viaddmax_s32(a[(j & 1) + 4 * (j >> 1)], k.b[j], floor_q), k.s[j]), -128), 127) + (int)(int8_t)(rr[i] >> (8 * j));
+            uint32_t hi, w;
+            asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(q[3]), "r"(q[2]));
+            asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q[1]), "r"(q[0]), "r"(hi));
+            sts32(at + (uint32_t)(8 * i * pitch), w);
+        }
     }
 }
 

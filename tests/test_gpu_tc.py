@@ -20,6 +20,7 @@ TC_SHAPES = [
     (128, 128, 128), (256, 64, 64), (100, 32, 32), (1, 16, 16), (300, 16, 96), (777, 96, 24), (130, 144, 32),
     (257, 192, 32), (384, 32, 192), (50, 384, 64), (64, 576, 96), (33, 960, 160), (200, 320, 1280), (129, 1280, 1000),
     (512, 160, 960), (90, 48, 17), (128, 256, 256), (1000, 64, 40),
+    (19200, 512, 256), (30000, 800, 96),  # several tiles a CTA, rows stored from registers
 ]
 
 
@@ -30,6 +31,35 @@ def test_gemm_s8_tc(shape):
     want = gpu_util.run_conv_oracle(case)
     got = gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05)
     np.testing.assert_array_equal(got, want)
+    assert want.std() > 0
+
+
+# Filters that stay in shared memory (two row tiles of 128 an SM and more): (M, K, N, options).
+RESIDENT_SHAPES = [
+    (38000, 64, 128, {}), (38000, 64, 80, {}), (37900, 96, 48, {}), (37900, 32, 16, {}),  # whole pieces, ragged ones, eight accumulators, one piece a tile
+    (37900, 128, 272, {}), (38000, 48, 192, {}),                                          # several column tiles, the last of 16 / 64 columns
+    (37900, 1040, 32, {}),                                                               # more blocks of K than stages
+    (13000, 320, 272, {}),                                                               # groups of CTAs, a column tile each
+    (76000, 16, 32, {}), (80000, 32, 144, {}),                                           # tiles handed out by the counter
+    (38000, 32, 50, {}), (37900, 48, 100, {}), (40000, 16, 410, {}),                         # columns that are no multiple of 16
+    (37900, 64, 96, dict(e_out=-14)), (37900, 32, 176, dict(e_out=-14, res=True)),                                                    # shifts outside the fast form
+    (37900, 64, 96, dict(lut=True)), (37900, 32, 80, dict(lut="channels")), (37900, 64, 208, dict(lut=True, act=abi.ACT_LINEAR)),
+    (38000, 96, 96, dict(res=True)), (38000, 32, 176, dict(res=True, act=abi.ACT_LINEAR)), (37900, 64, 32, dict(res=True, out_stride=48)),
+]
+
+
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("shape", RESIDENT_SHAPES, ids=lambda s: "x".join(map(str, s[:3])) + "".join("_" + k for k in s[3]))
+def test_gemm_s8_resident_filter(shape, round_mode):
+    m, k, n, opts = shape
+    opts = dict(dict(per_channel=True, e_in=-7, e_out=-5 + (k > 256), e_w=(-9, -6), act=abi.ACT_RELU), **opts)
+    res = opts.pop("res", False)
+    case = cases.gemm_case(seed=m + k + n, m=m, k=k, n_out=n, round_mode=round_mode, **opts)
+    if res:
+        case["res"] = np.random.default_rng(n).integers(-128, 128, size=case["out"].shape, dtype=np.int8)
+        case["residual_pixel_stride"] = opts.get("out_stride", 0)
+    want = gpu_util.run_conv_oracle(case)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), want)
     assert want.std() > 0
 
 
