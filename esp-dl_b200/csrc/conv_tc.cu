@@ -681,7 +681,7 @@ bool conv_plan(const espdl_conv_desc &d, ConvTcParams &p)
     p.tmem_cols = pow2;
     const long long ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     p.out_pw = 0, p.out_mask = 0;
-    if (ops % 16 == 0 && ((uintptr_t)d.output % 16) == 0 && !getenv("ESPDL_B200_DIRECT_STORES")) {
+    if (ops % 16 == 0 && d.out_c % 16 == 0 && ((uintptr_t)d.output % 16) == 0 && !getenv("ESPDL_B200_DIRECT_STORES")) { // (a TMA store clips rows in units of 16 bytes)
         const int parts = 4 / p.acc_stages;
         if (p.block_n % (16 * parts) == 0 && p.block_n / parts <= 128) {
             p.out_pw = p.block_n / parts;

@@ -1483,9 +1483,10 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     p.out_rows = 0;
     if (i16) {
         p.out_pw = p.block_n / 2; // four times [128][out_pw] = the tile
-        p.out_rows = p.block_n % 64 != 0 || ops % 8 != 0 || ((uintptr_t)d.output % 16) != 0;
+        p.out_rows = p.block_n % 64 != 0 || ops % 8 != 0 || p.N % 8 != 0 || ((uintptr_t)d.output % 16) != 0; // (see below)
     } else if (stageable) {
-        p.out_rows = ops % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
+        // A TMA store clips rows in units of 16 bytes: behind a row that ends in the middle of one it would write the neighbour's columns.
+        p.out_rows = ops % 16 != 0 || p.N % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
         const int parts = 4 / p.acc_stages;
         // Rows that no TMA store can address: a warp per staged row takes a tile 3.3 us whatever its width, a thread storing its own row about 1.2 and
         // 0.12 for every store its alignment makes of it (131072 rows of 64: 14 columns 11.1 against 24.6 staged, 40 13.3 / 22.5, 100 28.7 / 24.9, 150

@@ -78,6 +78,18 @@ def test_pointwise_conv_tc_nhwc_and_strides():
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), gpu_util.run_conv_oracle(case))
 
 
+@pytest.mark.parametrize("kind", ["rows", "resident", "rows-int16", "window"])
+def test_rows_that_end_inside_a_16_byte_unit_leave_the_neighbours_columns(kind):
+    """100 channels into rows of 112 (int16: 60 of 64): the columns behind them belong to another tensor of a Concat."""
+    if kind == "window":
+        case = cases.conv_case(seed=3, n=2, h=20, w=30, cin=32, cout=100, kh=3, kw=3, per_channel=True, out_stride=112)
+    elif kind == "rows-int16":
+        case = cases.gemm_case(seed=4, dtype=abi.DTYPE_INT16, m=300, k=64, n_out=60, e_in=-14, e_w=(-15, -15), e_out=-12, out_stride=64)
+    else:
+        case = cases.gemm_case(seed=5, m=300 if kind == "rows" else 37900, k=48, n_out=100, per_channel=True, out_stride=112)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), gpu_util.run_conv_oracle(case))
+
+
 def test_tc_and_simt_agree_and_auto_picks_tc():
     case = cases.gemm_case(seed=9, m=500, k=96, n_out=144, per_channel=True)
     a = gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05)
