@@ -290,6 +290,77 @@ __device__ __forceinline__ F2 codes_to_floats(uint32_t flipped, int k)
     return add2(pair(__uint_as_float(__byte_perm(flipped, 0x4b000000u, 0x7410u)), __uint_as_float(__byte_perm(flipped, 0x4b000000u, 0x7432u))), pair(-8421376.f, -8421376.f));
 }
 
+// The squared differences of a 16-byte unit of codes from the row's mean.
+template <typename T>
+__device__ __forceinline__ void unit_squares(uint4 w, F2 minus_mean, float (&d2)[16 / sizeof(T)])
+{
+    constexpr int V = Word<T>::V;
+    constexpr uint32_t FLIP = sizeof(T) == 1 ? 0x80808080u : 0x80008000u;
+    const uint32_t x[4] = {w.x ^ FLIP, w.y ^ FLIP, w.z ^ FLIP, w.w ^ FLIP};
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int k = 0; k < V; k += 2) {
+            const F2 d = add2(codes_to_floats<T>(x[j], k), minus_mean);
+            split(mul2(d, d), d2[j * V + k], d2[j * V + k + 1]);
+        }
+}
+
+// The ordered sum of a row's squared differences, `units` 16-byte units: the next unit's squares are made beside the chain of this one's additions, which
+// alone is four cycles an element (100352 rows of 768: 57.3 us pair by pair, 54.9; 40000 of 1024, where its registers cost a block an SM, 31.1 / 33.8).
+template <typename T>
+__device__ __forceinline__ float ordered_squares(const uint4 *row, int units, float mean)
+{
+    const F2 minus_mean = pair(-mean, -mean);
+    float a[16 / sizeof(T)], b[16 / sizeof(T)], var = 0.f;
+    unit_squares<T>(row[0], minus_mean, a);
+    int i = 1;
+    for (; i + 1 < units; i += 2) {
+        const uint4 wb = row[i], wa = row[i + 1];
+        unit_squares<T>(wb, minus_mean, b);
+#pragma unroll
+        for (int k = 0; k < 16 / (int)sizeof(T); k++) var = __fadd_rn(var, a[k]);
+        unit_squares<T>(wa, minus_mean, a);
+#pragma unroll
+        for (int k = 0; k < 16 / (int)sizeof(T); k++) var = __fadd_rn(var, b[k]);
+    }
+    if (i < units)
+        unit_squares<T>(row[i], minus_mean, b);
+#pragma unroll
+    for (int k = 0; k < 16 / (int)sizeof(T); k++) var = __fadd_rn(var, a[k]);
+    if (i < units) {
+#pragma unroll
+        for (int k = 0; k < 16 / (int)sizeof(T); k++) var = __fadd_rn(var, b[k]);
+    }
+    return var;
+}
+
+// One word of results from one of codes (sign bits flipped): sv, bv are its columns' scale and bias.
+template <typename T, bool EVEN>
+__device__ __forceinline__ uint32_t norm_word(uint32_t codes, F2 minus_mean, F2 inv_std, const F2 *sv, const F2 *bv, F2 in_scale, F2 rescale, F2 half, F2 one)
+{
+    constexpr int V = Word<T>::V;
+    int q[V];
+#pragma unroll
+    for (int k = 0; k < V; k += 2) {
+        // products with a power of two are exact, so a fused multiply-add there rounds as the separate operations do
+        const F2 d = fma2(codes_to_floats<T>(codes, k), in_scale, minus_mean);
+        const F2 y = add_product2(mul2(mul2(d, inv_std), sv[k / 2]), bv[k / 2], one);
+        float a, b;
+        split(EVEN ? mul2(y, rescale) : fma2(y, rescale, half), a, b);
+        q[k] = EVEN ? __float2int_rn(a) : __float2int_rd(a), q[k + 1] = EVEN ? __float2int_rn(b) : __float2int_rd(b);
+    }
+    uint32_t w;
+    if (V == 4) {
+        uint32_t hi;
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(q[V - 1]), "r"(q[V - 2]));
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q[1]), "r"(q[0]), "r"(hi));
+    } else {
+        asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(w) : "r"(q[1]), "r"(q[0]));
+    }
+    return w;
+}
+
 // LayerNormalization with the rows of a block side by side in shared memory.  The variance is an ordered fp32 sum, so a row
 // costs `len` dependent additions whoever does them; a warp per row made all 32 lanes do the same ones.  Here a thread walks one
 // row (row pitch an odd number of words: thread r reading word i of row r meets no bank conflict), 32 rows of a warp side by
@@ -297,12 +368,15 @@ __device__ __forceinline__ F2 codes_to_floats(uint32_t flipped, int k)
 // down the rows.  Bound by instruction issue (100352 rows of 768: 101 -> 80 us with asynchronous copies in, codes to floats without conversions, all
 // threads in the normalising pass and as many blocks as there are groups of rows; 80 -> 69 with two elements an instruction).
 // Rows of whole aligned 16-byte units have a pitch of an odd number of those: copies and a row's reads are of 16 bytes then, a quarter warp's
-// without bank conflicts as well (69 -> 63 us, issue slots 68 % busy).
+// without bank conflicts as well (69 -> 63 us).  A thread copies down its columns and normalises two (int16: four) words of a row at a time, scale and bias are
+// converted as words of codes: what is done for a word besides its arithmetic was a third of all instructions (63.6 -> 57.3 us; int16 114 -> 92, 200000 rows of
+// 64 21.3 -> 12.8).  Copying, summing and normalising take 9, 17 and 31 us of these 57, hardly beside each other although blocks are independent; a warp that
+// copies and sums the next rows while eight normalise these was slower (80: the one warp's chain of additions is in the way).
 // WORDS: rows are whole aligned words in global memory; otherwise the block's rows, one contiguous run of bytes, are dealt out to
 // and collected from the padded rows byte by byte.  UNITS: rows of whole 16-byte units; forms of their own, because what a block fetches of a kernel's code
 // counts in the shortest launches (6250 rows of 16: 3.77 us, 3.99 with both forms in one kernel).
 template <typename T, bool WORDS, bool EVEN, bool UNITS>
-__global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, int pitch, int early)
+__global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, int pitch, int across, int across16, int early)
 {
     if (early)
         grid_dep_launch();
@@ -323,11 +397,16 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
         if (WORDS) {
             // asynchronous copies: all of the block's rows in flight at once (with loads through registers a block spent half its time here)
             const uint32_t to = (uint32_t)__cvta_generic_to_shared(rows_s);
-            if (UNITS)
-                for (int rr = warp; rr < nr; rr += 8)
-                    for (int i = 4 * lane; i < words; i += 128)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 4u * (uint32_t)(rr * pitch + i)), "l"(src + (long long)rr * words + i) : "memory");
-            else
+            if (UNITS) { // a thread copies down its columns
+                const int columns = words / 4, wide = min(across16, columns), down = 256 / wide, first = threadIdx.x / wide;
+                if (first < down)
+                    for (int c = threadIdx.x % wide; c < columns; c += wide) {
+                        uint32_t at = to + 4u * (uint32_t)(first * pitch + 4 * c);
+                        const uint32_t *from = src + (long long)first * words + 4 * c;
+                        for (int rr = first; rr < nr; rr += down, at += 4u * (uint32_t)(down * pitch), from += (long long)down * words)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(from) : "memory");
+                    }
+            } else
                 for (int rr = warp; rr < nr; rr += 8)
                     for (int i = lane; i < words; i += 32)
                         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + 4u * (uint32_t)(rr * pitch + i)), "l"(src + (long long)rr * words + i) : "memory");
@@ -336,8 +415,9 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
             deal_rows<T>(src, total, row_bytes, rows_s, pitch);
         }
         __syncthreads();
-        if ((int)threadIdx.x < nr) {
-            const uint32_t *row = rows_s + threadIdx.x * pitch;
+        const int own = threadIdx.x;
+        if (own < nr) {
+            const uint32_t *row = rows_s + own * pitch;
             const int full = p.len / V;
             int sum = 0;
             auto add_word = [&](uint32_t w) {
@@ -379,10 +459,7 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
                 }
             };
             if (UNITS)
-                for (int i = 0; i < full; i += 4) {
-                    const uint4 w = *(const uint4 *)(row + i);
-                    add_squares(w.x), add_squares(w.y), add_squares(w.z), add_squares(w.w);
-                }
+                var = ordered_squares<T>((const uint4 *)row, full / 4, mean);
             else
 #pragma unroll 4
                 for (int i = 0; i < full; i++) add_squares(row[i]);
@@ -390,7 +467,7 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
             for (int k = 0; k < V; k++)
                 if (full * V + k < p.len)
                     add(code_to_float<T>(last.w ^ FLIP, k));
-            const long long out_row = r0 + threadIdx.x;
+            const long long out_row = r0 + own;
             if (p.mean)
                 store_q((T *)p.mean, out_row, fround(__fmul_rn(__fmul_rn(mean, p.mean_rescale), p.in_scale), p.half_even));
             mean = __fmul_rn(mean, p.in_scale);
@@ -399,54 +476,74 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
             const float inv_std = __fdiv_rn(1.0f, sqrt_newton_dev(__fadd_rn(var, p.epsilon)));
             if (p.inv_std)
                 store_q((T *)p.inv_std, out_row, fround(__fmul_rn(inv_std, p.inv_std_rescale), p.half_even));
-            stats[threadIdx.x] = make_float2(mean, inv_std);
+            stats[own] = make_float2(mean, inv_std);
         }
         __syncthreads();
         const T *sc = (const T *)p.scale, *bi = (const T *)p.bias;
-        const int across = words >= 64 ? 64 : words, down = 256 / across; // threads along a row, rows at a time
-        const int first_row = threadIdx.x / across;
         uint32_t *dst = (uint32_t *)((T *)p.out + r0 * p.len);
-        for (int cw = threadIdx.x % across; cw < words && first_row < down; cw += across) {
-            F2 sv[V / 2], bv[V / 2];
+        const F2 in_scale = pair(p.in_scale, p.in_scale), rescale = pair(p.out_rescale, p.out_rescale), half = pair(0.5f, 0.5f), one = pair(p.one, p.one);
+        // scale and bias of a thread's columns, from element e on
+        auto constants = [&](int e, F2 &s, F2 &b) {
+            float s2[2], b2[2];
 #pragma unroll
-            for (int k = 0; k < V; k += 2) {
-                float s2[2], b2[2];
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int e = min(cw * V + k + h, p.len - 1);
-                    s2[h] = sc ? __fmul_rn(__int2float_rn((int)sc[e]), p.scale_scale) : 1.0f;
-                    b2[h] = bi ? __fmul_rn(__int2float_rn((int)bi[e]), p.bias_scale) : 0.0f;
-                }
-                sv[k / 2] = pair(s2[0], s2[1]), bv[k / 2] = pair(b2[0], b2[1]);
+            for (int h = 0; h < 2; h++) {
+                const int at = min(e + h, p.len - 1);
+                s2[h] = sc ? __fmul_rn(__int2float_rn((int)sc[at]), p.scale_scale) : 1.0f;
+                b2[h] = bi ? __fmul_rn(__int2float_rn((int)bi[at]), p.bias_scale) : 0.0f;
             }
-            const F2 in_scale = pair(p.in_scale, p.in_scale), rescale = pair(p.out_rescale, p.out_rescale), half = pair(0.5f, 0.5f), one = pair(p.one, p.one);
-#pragma unroll 2
-            for (int rr = first_row; rr < nr; rr += down) {
-                const float2 st = stats[rr];
-                const uint32_t codes = rows_s[rr * pitch + cw] ^ FLIP;
-                const F2 minus_mean = pair(-st.x, -st.x), inv_std = pair(st.y, st.y);
-                int q[V];
+            s = pair(s2[0], s2[1]), b = pair(b2[0], b2[1]);
+        };
+        auto word = [&](uint32_t codes, F2 minus_mean, F2 inv_std, const F2 *sv, const F2 *bv) {
+            return norm_word<T, EVEN>(codes, minus_mean, inv_std, sv, bv, in_scale, rescale, half, one);
+        };
+        // W words of a row a thread: a whole 16-byte unit where rows are made of these, so that addresses, bounds and the row's figures cost a quarter as much
+        constexpr int W = UNITS ? (sizeof(T) == 1 ? 2 : 4) : 1;
+        const int columns = words / W, down = 256 / across; // threads along a row, rows at a time
+        const int first_row = threadIdx.x / across;
+        for (int c = threadIdx.x % across; c < columns && first_row < down; c += across) {
+            F2 sv[W * V / 2], bv[W * V / 2];
+            if (W * sizeof(uint32_t) % 8 == 0 && sc && bi && (((uintptr_t)sc | (uintptr_t)bi) & 15) == 0) { // whole words of codes, as the rows' own
+                const F2 s_scale = pair(p.scale_scale, p.scale_scale), b_scale = pair(p.bias_scale, p.bias_scale);
 #pragma unroll
-                for (int k = 0; k < V; k += 2) {
-                    // products with a power of two are exact, so a fused multiply-add there rounds as the separate operations do
-                    const F2 d = fma2(codes_to_floats<T>(codes, k), in_scale, minus_mean);
-                    const F2 y = add_product2(mul2(mul2(d, inv_std), sv[k / 2]), bv[k / 2], one);
-                    float a, b;
-                    split(EVEN ? mul2(y, rescale) : fma2(y, rescale, half), a, b);
-                    q[k] = EVEN ? __float2int_rn(a) : __float2int_rd(a), q[k + 1] = EVEN ? __float2int_rn(b) : __float2int_rd(b);
+                for (int i = 0; i < W; i++) {
+                    const uint32_t sw = ((const uint32_t *)sc)[c * W + i] ^ FLIP, bw = ((const uint32_t *)bi)[c * W + i] ^ FLIP;
+#pragma unroll
+                    for (int k = 0; k < V; k += 2) {
+                        sv[(i * V + k) / 2] = mul2(codes_to_floats<T>(sw, k), s_scale);
+                        bv[(i * V + k) / 2] = mul2(codes_to_floats<T>(bw, k), b_scale);
+                    }
                 }
-                uint32_t w;
-                if (V == 4) {
-                    uint32_t hi;
-                    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(q[V - 1]), "r"(q[V - 2]));
-                    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q[1]), "r"(q[0]), "r"(hi));
+            } else {
+#pragma unroll
+                for (int k = 0; k < W * V; k += 2) constants(c * W * V + k, sv[k / 2], bv[k / 2]);
+            }
+            const uint32_t *from = rows_s + first_row * pitch + c * W;
+            uint32_t *to = dst + (long long)first_row * words + c * W;
+#pragma unroll(W == 1 ? 2 : 1)
+            for (int rr = first_row; rr < nr; rr += down, from += down * pitch, to += (long long)down * words) {
+                const float2 st = stats[rr];
+                const F2 minus_mean = pair(-st.x, -st.x), inv_std = pair(st.y, st.y);
+                if (W == 2) {
+                    const uint2 x = *(const uint2 *)from;
+                    uint2 y;
+                    y.x = word(x.x ^ FLIP, minus_mean, inv_std, sv, bv);
+                    y.y = word(x.y ^ FLIP, minus_mean, inv_std, sv + V / 2, bv + V / 2);
+                    *(uint2 *)to = y;
+                } else if (W == 4) {
+                    const uint4 x = *(const uint4 *)from;
+                    uint4 y;
+                    y.x = word(x.x ^ FLIP, minus_mean, inv_std, sv, bv);
+                    y.y = word(x.y ^ FLIP, minus_mean, inv_std, sv + V / 2, bv + V / 2);
+                    y.z = word(x.z ^ FLIP, minus_mean, inv_std, sv + V, bv + V);
+                    y.w = word(x.w ^ FLIP, minus_mean, inv_std, sv + 3 * V / 2, bv + 3 * V / 2);
+                    *(uint4 *)to = y;
                 } else {
-                    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(w) : "r"(q[1]), "r"(q[0]));
+                    const uint32_t y = word(*from ^ FLIP, minus_mean, inv_std, sv, bv);
+                    if (WORDS)
+                        *to = y;
+                    else
+                        rows_s[rr * pitch + c] = y;
                 }
-                if (WORDS)
-                    dst[(long long)rr * words + cw] = w;
-                else
-                    rows_s[rr * pitch + cw] = w;
             }
         }
         if (!WORDS) {
@@ -475,7 +572,19 @@ int launch_layer_rows(const NormParams &p, int R, int pitch, cudaStream_t s)
     const auto kernel = pitch % 4 == 0 ? (p.half_even ? layer_rows_kernel<T, true, true, true> : layer_rows_kernel<T, true, false, true>)
         : words                        ? (p.half_even ? layer_rows_kernel<T, true, true, false> : layer_rows_kernel<T, true, false, false>)
                                        : (p.half_even ? layer_rows_kernel<T, false, true, false> : layer_rows_kernel<T, false, false, false>);
-    launch_mover(kernel, dim3((unsigned)min(groups, (long long)num_sms() * 64)), dim3(256), smem, s, p, R, pitch);
+    // threads along a row: all of its columns, or such a part of them that most of a block has work
+    const int columns = (p.len + Word<T>::V - 1) / Word<T>::V / (pitch % 4 != 0 ? 1 : sizeof(T) == 1 ? 2 : 4);
+    const auto spread = [](int columns) {
+        int across = 1;
+        for (int passes = (columns + 255) / 256, best = 0; passes <= 8; passes++) {
+            const int a = (columns + passes - 1) / passes, busy = 256 / a * columns / passes; // threads at work in an average pass
+            if (busy > best + 8)
+                best = busy, across = a;
+        }
+        return across;
+    };
+    const int across = spread(columns), across16 = spread(max(1, (p.len + Word<T>::V - 1) / Word<T>::V / 4)); // (the units that are copied)
+    launch_mover(kernel, dim3((unsigned)min(groups, (long long)num_sms() * 64)), dim3(256), smem, s, p, R, pitch, across, across16);
     count_launch();
     return check_launch("layer norm");
 }
@@ -513,7 +622,7 @@ extern "C" int espdl_b200_norm(const espdl_norm_desc *d, void *stream)
     if (d->op == ESPDL_NORM_LAYER && ((uintptr_t)d->input % 4) == 0 && ((uintptr_t)d->output % 4) == 0) {
         // rows a block: 48 KB of them (four blocks an SM keep eight warps at their rows), fewer where that leaves SMs without a block
         const int V = d->dtype == ESPDL_DTYPE_INT8 ? 4 : 2, words = (d->len + V - 1) / V;
-        const bool units = d->len % (4 * V) == 0 && ((uintptr_t)d->input % 16) == 0;
+        const bool units = d->len % (4 * V) == 0 && (((uintptr_t)d->input | (uintptr_t)d->output) % 16) == 0;
         const int pitch = units ? 4 * (words / 4 | 1) : words | 1;
         const long long fit = (50 * 1024) / ((long long)pitch * 4 + 8), share = (d->rows + num_sms() - 1) / num_sms();
         const int R = (int)min(min(256ll, max(fit, (96 * 1024) / ((long long)pitch * 4 + 8) >= 32 ? 32ll : 0ll)), max(32ll, share)) / 32 * 32;

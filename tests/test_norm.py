@@ -138,6 +138,28 @@ def test_gpu_rows_of_whole_units(rows, n, skip, in_place, kw, dt, round_mode):
     assert want["y"].std() > 0
 
 
+# two and three units a row (int8), more columns than a block has threads at once, ragged rows in several passes; scale and bias off a word's boundary, and an
+# output off a unit's, take the general conversions and the kernel form of whole words
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("off", ["", "scale", "y"])
+@pytest.mark.parametrize("rows,n", [(259, 32), (300, 48), (5003, 1040), (5003, 2064), (5003, 300), (600, 29)])
+def test_gpu_columns_and_alignments(rows, n, off, dt):
+    import gpu_util
+    a = make(abi.NORM_LAYER, dt, rows, n, seed=rows + n)
+    want = fresh(a)
+    assert checkers.oracle().oracle_norm(C.byref(desc(want))) == 0
+    with gpu_util.DeviceBuffers() as dev:
+        ptrs = {}
+        for k in ("scale", "bias", "mean", "inv", "x", "y"):
+            skip = {"scale": (1 if k in ("scale", "bias") else 0), "y": (4 if k == "y" else 0)}.get(off, 0)
+            pad = np.zeros(skip, dtype=a[k].dtype)
+            ptrs[k] = dev.upload(np.concatenate([pad, a[k].reshape(-1)])) + pad.nbytes
+        abi.check(dev.lib.espdl_b200_norm(C.byref(desc(a, ptrs)), None), "norm")
+        for k in ("y", "mean", "inv"):
+            np.testing.assert_array_equal(dev.download(ptrs[k], want[k]), want[k], err_msg=k)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("op", [abi.NORM_RMS, abi.NORM_LAYER])
 @pytest.mark.parametrize("shape,axis", [((2, 9, 64), -1), ((3, 4, 5, 16), 2)])
