@@ -33,7 +33,7 @@
 // and one multiplies lo by both (into 1, 2): half the instructions of four separate products, and each wide enough to be bound
 // by its math (max(N/2, 32 + N/4) cycles at M = 128).  The epilogue recombines in two 32-bit halves (requant_wide; 64 bits for
 // shifts outside 1 .. 31) and takes off 32768 * (sum of the input row).  Exact as long as K <= 16384 (a partial sum stays below
-// 97,665 * K < 2^31).  4096x1024x1024 with the packing: 85 us with four products and 64-bit sums, 25 now.
+// 97,665 * K < 2^31).  4096x1024x1024 with the packing: 85 us with four products and 64-bit sums, 25 with one set of accumulators, 23 now.
 //
 // Every mbarrier wait is bounded (about two seconds); on expiry the kernel records ESPDL_ERR_TIMEOUT in the mapped host word
 // (common.cuh) that espdl_b200_stream_sync reports, and all roles leave.
@@ -87,7 +87,7 @@ struct TcParams {
     int swz;        // bytes of K per stage row: 32, 64 or 128
     int k_blocks;   // ceil(K / swz)
     int stages;
-    int acc_stages; // TMEM accumulator buffers: 4 or 2 (int8), 1 (int16)
+    int acc_stages; // TMEM accumulator buffers: 8, 4, 2 or 1 (int8), 2 or 1 sets of three (int16)
     int tmem_cols;  // power of two >= 32
     int out_pw;     // staged epilogue: bytes per row of a group's output piece (0 = rows are stored directly); int16: a quarter
                     // of the bytes per row of the one tile that all groups share
@@ -583,7 +583,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     TC_STAMP(0);
     const int total_tiles = p.batch * p.m_tiles * p.n_tiles;
     const int sets = RES && p.in_turn ? p.acc_stages / 2 : p.acc_stages;
-    const int parts = 4 / sets; // epilogue groups that share one tile (they split its columns)
+    const int parts = I16 ? 4 : 4 / sets; // epilogue groups that share one tile (they split its columns)
     // Tiles are numbered n-fastest: tile = row_tile * n_tiles + n_tile with row_tile running over batch x m_tiles.  A CTA
     // starts with tile blockIdx.x; every further tile comes from a global counter (p.sched), so that an SM that runs
     // slower than the others (measured: one in ten takes 15-25 % longer per tile) gets fewer tiles instead of setting
@@ -830,8 +830,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // ------------------------------------------------------------ epilogue (warps 2..17)
         const int ew = warp - 2;
         const int group = ew >> 2;               // 0..3
-        const int own_acc = group % sets;        // accumulator buffer this group reads (in turn: with the one `sets` further)
-        const int part = group / sets;           // which share of the tile's columns
+        const int own_acc = I16 ? 0 : group % sets; // accumulator buffer this group reads (in turn: with the one `sets` further; int16: all in turn)
+        const int part = I16 ? group : group / sets; // which share of the tile's columns
         int turn = 0;
         const int lane_group = warp & 3;         // TMEM lanes this warp may read: 32*lane_group .. +31
         const int row_in_tile = lane_group * 32 + lane;
@@ -874,7 +874,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 ok = epilogue_resident<EVEN, 0>(p, map_out, tmem_base, fp_base, stage, tfull_bar, tempty_bar, epi_row, epi_col, tbl, group, lane_group, lane);
         }
         while (ok && !own_loop) {
-            const int acc = RES ? own_acc + turn : own_acc;
+            const int acc = RES || I16 ? own_acc + turn : own_acc;
             TC_LAP(w_work);
             if (!mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase)) {
                 ok = false;
@@ -893,6 +893,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const long long m = (long long)bi * p.M + m0 + row_in_tile; // row of the output tensor
             const uint32_t t0 = tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)(acc * NACC * p.block_n);
             acc_phase ^= 1;
+            if (I16 && p.acc_stages == 2) {
+                acc_phase ^= 1 ^ turn;
+                turn ^= 1;
+            }
             if (RES && p.in_turn) { // (general epilogue: a channel outside the fast form)
                 if (!turn)
                     acc_phase ^= 1;
@@ -990,8 +994,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const bool slow = *(volatile int *)slow_flag;
                 const long long base = -(long long)sum * 32768;
                 const int row_h = (int)(base >> 16), row_l = (int)(base & 0xffff);
-                // staged rows: pieces of 64 columns for a TMA store each, or whole rows
-                const uint32_t buf = smem_u32(out_stage), pitch = p.out_rows ? 2u * (uint32_t)p.block_n : 128u, mask = 7u;
+                // staged rows: pieces of 64 columns for a TMA store each, or whole rows for one (without its swizzle) or for the warps
+                const bool pieces = !p.out_rows && p.block_n % 64 == 0;
+                const uint32_t buf = smem_u32(out_stage), pitch = pieces ? 128u : 2u * (uint32_t)p.block_n, mask = p.out_rows || pieces ? 7u : 0u;
                 int chunk = 0;
                 for (int c0 = 0; c0 < p.block_n; c0 += 16, chunk++) {
                     if (chunk % parts != part)
@@ -1024,7 +1029,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                             pk[j >> 1] = j & 1 ? pk[j >> 1] | ((uint32_t)q << 16) : (uint32_t)q & 0xffffu;
                         }
                     }
-                    const uint32_t off = (p.out_rows ? 2u * (uint32_t)c0 : (uint32_t)(c0 >> 6) * (BLOCK_M * 128u) + 2u * (uint32_t)(c0 & 63)) + (uint32_t)row_in_tile * pitch;
+                    const uint32_t off = (!pieces ? 2u * (uint32_t)c0 : (uint32_t)(c0 >> 6) * (BLOCK_M * 128u) + 2u * (uint32_t)(c0 & 63)) + (uint32_t)row_in_tile * pitch;
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (off ^ (((off >> 7) & mask) << 4))), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
                     const uint32_t off2 = off + 16u;
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (off2 ^ (((off2 >> 7) & mask) << 4))), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
@@ -1038,7 +1043,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 named_bar(EPI_BAR, EPI_WARPS * 32);
                 if (!p.out_rows) {
                     if (et == 0) { // rows >= M and columns >= N are clipped
-                        for (int c0 = 0; c0 < p.block_n; c0 += 64) tma_store_3d(&map_out, buf + (uint32_t)(c0 >> 6) * (BLOCK_M * 128u), 2 * (n0 + c0), m0, bi);
+                        for (int c0 = 0; c0 < p.block_n; c0 += pieces ? 64 : p.block_n) tma_store_3d(&map_out, buf + (uint32_t)(c0 >> 6) * (BLOCK_M * 128u), 2 * (n0 + c0), m0, bi);
                         bulk_commit();
                     }
                     continue;
@@ -1434,6 +1439,15 @@ void plan_resident(TcParams &p)
     p = q;
 }
 
+// int16 products in tiles of bn columns: rounds of tiles over the SMs; a tile's instructions (two of twice the width every 32 bytes of K), its loads of two planes at
+// 64 bytes a cycle, and its results at 47 cycles a column, beside the next tile's products where there are two sets of accumulators.
+double int16_tile_cycles(const TcParams &p, int bn)
+{
+    const double rounds = ceil((double)p.m_tiles * ((p.N + bn - 1) / bn) / num_sms()), results = 47.0 * bn;
+    const double products = max((p.K + 31) / 32 * 2.0 * max(bn, 32 + bn / 2), 2.0 * (BLOCK_M + bn) * p.K / 64);
+    return 6 * bn <= 512 ? rounds * max(products, results) + results : rounds * (products + results);
+}
+
 bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
 {
     const bool i16 = d.dtype == ESPDL_DTYPE_INT16;
@@ -1453,8 +1467,20 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     // Few rows: narrower tiles put more SMs to work while they still make one wave - a tile's time is the stream of its filter rows
     // through one SM plus its columns' epilogue.
     while (max_bn > 32 && 2ll * p.batch * p.m_tiles * ((p.N + max_bn - 1) / max_bn) <= num_sms()) max_bn /= 2;
+    const auto width = [&](int cap) {
+        const int tiles = (p.N + cap - 1) / cap;
+        return (((p.N + tiles - 1) / tiles) + 15) / 16 * 16;
+    };
+    if (i16 && max_bn > 64) {
+        // Tiles of up to 80 columns leave room for a second set of accumulators, so that a tile is multiplied while the one before it is requantised; wider ones
+        // load less for a result.  Cycles by what either takes (int16_tile_cycles); narrower where that is a tenth less.  us at most 128 / 80 / 64 columns:
+        // 4096x1024x1024 24.7 / 23.1 / 25.9, 2887x1072x3768 72 / 62 / 68, 65536x512x128 57.2 / - / 52.9, 4096x2048x512 22.7 / 26.1 / 24.9, 25916x48x952 48 / 51 / 54.
+        const double wide = int16_tile_cycles(p, width(max_bn)), mid = int16_tile_cycles(p, width(80)), narrow = int16_tile_cycles(p, width(64));
+        if (min(mid, narrow) < 0.9 * wide)
+            max_bn = mid < narrow ? 80 : 64;
+    }
     p.n_tiles = (p.N + max_bn - 1) / max_bn;
-    p.block_n = (((p.N + p.n_tiles - 1) / p.n_tiles) + 15) / 16 * 16;
+    p.block_n = width(max_bn);
     if (!i16 && p.block_n > 128)
         p.block_n = (p.block_n + 31) / 32 * 32; // two epilogue groups split a wide tile into whole 16-byte pieces
     p.n_tiles = (p.N + p.block_n - 1) / p.block_n;
@@ -1462,7 +1488,7 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     if (i16 && p.swz == 128 && p.block_n > 80)
         p.swz = 64; // a stage holds two planes of each operand: 64-byte rows leave room for five stages beside a wide output tile
     p.k_blocks = (p.K + p.swz - 1) / p.swz;
-    p.acc_stages = i16 ? 1 : (4 * p.block_n <= 512 ? 4 : 2);
+    p.acc_stages = i16 ? (6 * p.block_n <= 512 ? 2 : 1) : (4 * p.block_n <= 512 ? 4 : 2);
     const long long rps = d.residual_pixel_stride ? d.residual_pixel_stride : d.out_c;
     const bool res_ok = !d.residual || (rps % 16 == 0 && ((uintptr_t)d.residual % 16) == 0);
     const bool stageable = res_ok && !force_direct && !getenv("ESPDL_B200_DIRECT_STORES");
@@ -1483,7 +1509,7 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     p.out_rows = 0;
     if (i16) {
         p.out_pw = p.block_n / 2; // four times [128][out_pw] = the tile
-        p.out_rows = p.block_n % 64 != 0 || ops % 8 != 0 || p.N % 8 != 0 || ((uintptr_t)d.output % 16) != 0; // (see below)
+        p.out_rows = ops % 8 != 0 || p.N % 8 != 0 || ((uintptr_t)d.output % 16) != 0; // (see below)
     } else if (stageable) {
         // A TMA store clips rows in units of 16 bytes: behind a row that ends in the middle of one it would write the neighbour's columns.
         p.out_rows = ops % 16 != 0 || p.N % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
@@ -1700,7 +1726,8 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
                            (uint64_t)p.M * (uint64_t)p.ops)))
             return st;
     }
-    if (i16 && !p.out_rows && (st = make_map(&mo, d.output, (uint64_t)p.M, 2 * (uint64_t)p.N, 2 * (uint64_t)p.ops, BLOCK_M, 128, 128)))
+    if (i16 && !p.out_rows && (st = p.block_n % 64 == 0 ? make_map(&mo, d.output, (uint64_t)p.M, 2 * (uint64_t)p.N, 2 * (uint64_t)p.ops, BLOCK_M, 128, 128)
+                                                        : make_map(&mo, d.output, (uint64_t)p.M, 2 * (uint64_t)p.N, 2 * (uint64_t)p.ops, BLOCK_M, 2 * (uint32_t)p.block_n, 0)))
         return st;
     if (smem < 120 * 1024) // more than half an SM's shared memory: one CTA per SM, so TMEM allocation never waits on a neighbour
         smem = 120 * 1024;

@@ -78,6 +78,16 @@ def test_pointwise_conv_tc_nhwc_and_strides():
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), gpu_util.run_conv_oracle(case))
 
 
+# Tiles of 80 and 64 columns with two sets of accumulators, several a CTA; one set (128 columns); rows that no TMA store can address; the wide shifts' form
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("m,k,n,opts", [(3000, 1024, 1200, {}), (30000, 64, 64, {}), (20000, 96, 80, {}), (40000, 32, 48, {}), (20000, 64, 200, {}), (4000, 512, 1024, {}),
+                                        (30000, 48, 75, {}), (20000, 32, 72, dict(out_stride=80)), (20000, 32, 64, dict(out_stride=65)), (20000, 32, 64, dict(e_out=20))])
+def test_gemm_s16_accumulators_in_turn(m, k, n, opts, round_mode):
+    opts = dict(dict(e_in=-14, e_w=(-15, -15), e_out=-12), **opts)
+    case = cases.gemm_case(seed=m + n, dtype=abi.DTYPE_INT16, m=m, k=k, n_out=n, wide=True, bias_mag=1 << 20, round_mode=round_mode, **opts)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), gpu_util.run_conv_oracle(case))
+
+
 @pytest.mark.parametrize("kind", ["rows", "resident", "rows-int16", "window"])
 def test_rows_that_end_inside_a_16_byte_unit_leave_the_neighbours_columns(kind):
     """100 channels into rows of 112 (int16: 60 of 64): the columns behind them belong to another tensor of a Concat."""
