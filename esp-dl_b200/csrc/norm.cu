@@ -11,6 +11,7 @@
 // rounded on its own (no fused multiply-add), as in the reference built without contraction.
 #include "rows.cuh"
 
+#include <climits>
 #include <mutex>
 
 namespace espdl {
@@ -572,18 +573,19 @@ int launch_layer_rows(const NormParams &p, int R, int pitch, cudaStream_t s)
     const auto kernel = pitch % 4 == 0 ? (p.half_even ? layer_rows_kernel<T, true, true, true> : layer_rows_kernel<T, true, false, true>)
         : words                        ? (p.half_even ? layer_rows_kernel<T, true, true, false> : layer_rows_kernel<T, true, false, false>)
                                        : (p.half_even ? layer_rows_kernel<T, false, true, false> : layer_rows_kernel<T, false, false, false>);
-    // threads along a row: all of its columns, or such a part of them that most of a block has work
+    // Threads along a row: all of its columns, or a part of them at a time where that leaves fewer threads without work; a pass converts the constants of its
+    // columns first, about two rows' work (8370 rows of 264, whose 66 words are three rows at once or seven in two passes: 6.8 us in one, 7.9 in two).
     const int columns = (p.len + Word<T>::V - 1) / Word<T>::V / (pitch % 4 != 0 ? 1 : sizeof(T) == 1 ? 2 : 4);
-    const auto spread = [](int columns) {
-        int across = 1;
-        for (int passes = (columns + 255) / 256, best = 0; passes <= 8; passes++) {
-            const int a = (columns + passes - 1) / passes, busy = 256 / a * columns / passes; // threads at work in an average pass
-            if (busy > best + 8)
-                best = busy, across = a;
+    const auto spread = [R](int columns, int first) {
+        int across = 1, least = INT_MAX;
+        for (int passes = (columns + 255) / 256; passes <= 8; passes++) {
+            const int a = (columns + passes - 1) / passes, down = 256 / a, cost = passes * (first + (R + down - 1) / down);
+            if (cost < least)
+                least = cost, across = a;
         }
         return across;
     };
-    const int across = spread(columns), across16 = spread(max(1, (p.len + Word<T>::V - 1) / Word<T>::V / 4)); // (the units that are copied)
+    const int across = spread(columns, 2), across16 = spread(max(1, (p.len + Word<T>::V - 1) / Word<T>::V / 4), 0); // (the units that are copied)
     launch_mover(kernel, dim3((unsigned)min(groups, (long long)num_sms() * 64)), dim3(256), smem, s, p, R, pitch, across, across16);
     count_launch();
     return check_launch("layer norm");
