@@ -246,31 +246,40 @@ __device__ __forceinline__ uint32_t staged_word(uint32_t buf, uint32_t off, uint
     return v;
 }
 
-__device__ __forceinline__ void store_staged_row(int8_t *dst, uint32_t buf, uint32_t at, int len, uint32_t mask, int lane)
+// `rows` of them, `step` bytes apart in the tile and `pitch` in global memory.  Four at a time: one row's loads, shifts and stores after the other's took a tile
+// 3.3 us whatever its width (49314 rows of 16 -> 1634: 114 us, now 72; 20000 of 256 -> 333 25.4 / 15.6; 60000 of 48 -> 99 19.1 / 11.6).
+__device__ __forceinline__ void store_staged_rows(int8_t *dst, long long pitch, uint32_t buf, uint32_t at, uint32_t step, int rows, int len, uint32_t mask, int lane)
 {
-    if ((((uintptr_t)dst | (uintptr_t)len) & 15) == 0) {
-        for (int c = lane * 16; c < len; c += 512) {
-            const uint32_t off = at + (uint32_t)c;
-            uint4 v;
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(buf + (off ^ (((off >> 7) & mask) << 4))));
-            *(uint4 *)(dst + c) = v;
+    constexpr int U = 4;
+    const int eu = lane >> 3, ei = lane & 7; // head and tail bytes, at most six a row: eight lanes a row
+    for (int i = 0; i < rows; i += U, dst += U * pitch, at += U * step) {
+        for (int w = lane; 4 * (w - lane) < len; w += 32) {
+            uint32_t a[U], b[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int head = (int)((0u - (uint32_t)(uintptr_t)(dst + u * pitch)) & 3u);
+                const uint32_t off = at + (uint32_t)u * step + 4u * (uint32_t)w; // the aligned word that holds the first byte (head < 4)
+                a[u] = b[u] = 0u;
+                if (i + u < rows && head + 4 * w + 4 <= len) {
+                    a[u] = staged_word(buf, off, mask);
+                    if (head)
+                        b[u] = staged_word(buf, off + 4, mask);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int head = (int)((0u - (uint32_t)(uintptr_t)(dst + u * pitch)) & 3u);
+                if (i + u < rows && head + 4 * w + 4 <= len)
+                    *(uint32_t *)(dst + u * pitch + head + 4 * w) = __funnelshift_r(a[u], b[u], 8u * (uint32_t)head);
+            }
         }
-        return;
-    }
-    const int head = min((int)((0u - (uint32_t)(uintptr_t)dst) & 3u), len), words = (len - head) >> 2;
-    const uint32_t sh = (uint32_t)(head & 3) * 8u;
-    for (int w = lane; w < words; w += 32) {
-        const uint32_t off = at + (uint32_t)(4 * w); // the aligned word that holds the first byte (head < 4)
-        uint32_t v = staged_word(buf, off, mask);
-        if (sh)
-            v = __funnelshift_r(v, staged_word(buf, off + 4, mask), sh);
-        *(uint32_t *)(dst + head + 4 * w) = v;
-    }
-    const int edge = len - 4 * words; // head and tail bytes
-    if (lane < edge) {
-        const int b = lane < head ? lane : lane + 4 * words;
-        const uint32_t off = at + (uint32_t)b;
-        dst[b] = (int8_t)(staged_word(buf, off & ~3u, mask) >> (8 * (off & 3u)));
+        int8_t *edge = dst + eu * pitch;
+        const int head = min((int)((0u - (uint32_t)(uintptr_t)edge) & 3u), len), words = (len - head) >> 2;
+        if (i + eu < rows && ei < len - 4 * words) {
+            const int byte = ei < head ? ei : ei + 4 * words;
+            const uint32_t off = at + (uint32_t)eu * step + (uint32_t)byte;
+            edge[byte] = (int8_t)(staged_word(buf, off & ~3u, mask) >> (8 * (off & 3u)));
+        }
     }
 }
 
@@ -949,8 +958,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         const int len = min(p.out_pw, p.N - (n0 + col0)), rows_left = min(32, p.M - m0 - lane_group * 32);
                         int8_t *dst = (int8_t *)p.out + ((long long)bi * p.M + m0 + lane_group * 32) * p.ops + n0 + col0;
                         if (len > 0)
-                            for (int i = 0; i < rows_left; i++, dst += p.ops)
-                                store_staged_row(dst, buf, (uint32_t)((lane_group * 32 + i) * p.out_pw), len, (uint32_t)p.out_mask, lane);
+                            store_staged_rows(dst, p.ops, buf, (uint32_t)(lane_group * 32 * p.out_pw), (uint32_t)p.out_pw, rows_left, len, (uint32_t)p.out_mask, lane);
                         continue;
                     }
                     fence_async_smem();
@@ -1049,8 +1057,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     continue;
                 }
                 const int len = 2 * min(p.block_n, p.N - n0);
-                for (int row = ew; row < BLOCK_M && m0 + row < p.M; row += EPI_WARPS)
-                    store_staged_row((int8_t *)p.out + 2 * (((long long)bi * p.M + m0 + row) * p.ops + n0), buf, (uint32_t)row * pitch, len, mask, lane);
+                const int row0 = ew * (BLOCK_M / EPI_WARPS);
+                store_staged_rows((int8_t *)p.out + 2 * (((long long)bi * p.M + m0 + row0) * p.ops + n0), 2 * p.ops, buf, (uint32_t)row0 * pitch, pitch,
+                                  min(BLOCK_M / EPI_WARPS, p.M - m0 - row0), len, mask, lane);
                 continue;
             }
             fence_before();
@@ -1514,12 +1523,12 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
         // A TMA store clips rows in units of 16 bytes: behind a row that ends in the middle of one it would write the neighbour's columns.
         p.out_rows = ops % 16 != 0 || p.N % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
         const int parts = 4 / p.acc_stages;
-        // Rows that no TMA store can address: a warp per staged row takes a tile 3.3 us whatever its width, a thread storing its own row about 1.2 and
-        // 0.12 for every store its alignment makes of it (131072 rows of 64: 14 columns 11.1 against 24.6 staged, 40 13.3 / 22.5, 100 28.7 / 24.9, 150
-        // 202 / 48); a lone tile waits for either.
+        // Rows that no TMA store can address: staged, a tile of any width takes its warps as long as a thread of theirs some stores of its own row (131072 rows of 64,
+        // us from registers / staged: 13 stores of four bytes 12.4 / 14.8, 15 14.4 / 14.9, 17 16.8 / 15.4, 25 21.8 / 16.1; of two 9 11.3 / 15.2, 11 15.5 / 15.2,
+        // 13 21.8 / 15.2; of one 13 9.4 / 14.9, 21 14.7 / 15.2).
         const uintptr_t mixed = (uintptr_t)ops | (uintptr_t)d.output | (p.n_tiles > 1 ? (uintptr_t)p.block_n : 16u) | 16u;
-        const int stores = min(p.N, p.block_n) / (int)(mixed & (~mixed + 1));
-        const bool few_stores = p.out_rows && stores < ((long long)p.batch * p.m_tiles * p.n_tiles > 4ll * num_sms() ? 20 : 30);
+        const int bytes = (int)(mixed & (~mixed + 1)), stores = min(p.N, p.block_n) / bytes;
+        const bool few_stores = p.out_rows && stores < (bytes >= 4 ? 16 : bytes == 2 ? 11 : 21);
         if (few_stores)
             p.out_rows = 0;
         else if (p.block_n % (16 * parts) == 0 && p.block_n / parts <= 128) {

@@ -88,6 +88,17 @@ def test_gemm_s16_accumulators_in_turn(m, k, n, opts, round_mode):
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), gpu_util.run_conv_oracle(case))
 
 
+# Rows that leave by warps, four at a time: rows that begin at every byte of a word, the last ones of a tile and of a group of four, pieces of one word and less,
+# of more words than lanes (int16); columns on both sides of the lines to stores from registers
+@pytest.mark.parametrize("m,k,n,opts", [(130, 32, 333, {}), (257, 64, 99, {}), (131, 64, 22, {}), (130, 64, 26, {}), (129, 32, 68, {}), (133, 48, 60, {}), (20000, 32, 101, {}),
+                                        (129, 32, 257, dict(out_stride=259)), (40000, 16, 130, {}), (127, 64, 513, {})])
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+def test_rows_that_leave_by_warps(m, k, n, opts, dtype):
+    exps = dict(e_in=-7, e_out=-5, e_w=(-9, -6), per_channel=True) if dtype == abi.DTYPE_INT8 else dict(e_in=-14, e_w=(-15, -15), e_out=-12)
+    case = cases.gemm_case(seed=m + n, dtype=dtype, m=m, k=k, n_out=n, **exps, **opts)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05), gpu_util.run_conv_oracle(case))
+
+
 @pytest.mark.parametrize("kind", ["rows", "resident", "rows-int16", "window"])
 def test_rows_that_end_inside_a_16_byte_unit_leave_the_neighbours_columns(kind):
     """100 channels into rows of 112 (int16: 60 of 64): the columns behind them belong to another tensor of a Concat."""
