@@ -575,8 +575,8 @@ static bool overlaps(const espdl_conv_desc &d)
 
 // int16 on the warp-level instructions, where the other kernels take longer.  Packing and the tile kernel: two launches, the reduction's length, the
 // unrolled rows (windows about twice), the results and the products, from 37 layers, 20 % (standard deviation) off 380 others.  The
-// products' rate is a third of theirs: 4096x1024x1024 25 us there, 66 here; 45 of 11x11x256 -> 80, 3x3 22 / 37.  Results of fewer than 16 channels leave the tile kernel a row at a time
-// (58800x96x8 22.4 / 11.0).  Eight-element reductions are padded to 64 here, and the CUDA cores read many of them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
+// products' rate is a third of theirs: 4096x1024x1024 23 us there, 64 here; 45 of 11x11x256 -> 80, 3x3 22 / 37.  Results of fewer than 16 channels leave the tile kernel by
+// warps (58800x96x8 15.6 / 9.2).  Eight-element reductions are padded to 64 here, and the CUDA cores read many of them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
 // 6.0; 5977x8x5 3.6 / 3.3, 1088x8x192 8.9 / 3.8).  A product whose results overwrite its inputs stays with the tile kernel, which has copied those before it writes.
 static bool runs_mma16(const espdl_conv_desc &d)
 {

@@ -3,16 +3,18 @@
 // Replaces dl::base::conv2d<int16_t,...> (esp-dl/dl/base/dl_base_conv2d.cpp) where the tensor-core tile kernel's two launches - its operands
 // unrolled and split into byte planes in memory first - are most of the time: 4 x 40x40x64 -> 64, 3x3 took 12.3 us, 8 of them
 // the packing and its launch.  Here the planes never reach memory: a block copies 64-element runs of its input
-// pixels' windows and filter rows to shared memory as they are (asynchronous copies, four stages, zero fill outside the image), a warp splits
+// pixels' windows and filter rows to shared memory as they are (asynchronous copies, three runs at a time, zero fill outside the image), a warp splits
 // the words of a fragment into high and low bytes by byte permutes, and multiplies: x = 256 xh + xl with xh signed and xl unsigned, so a
 // product is 65536 hh + 256 (hl + lh) + ll, four instructions of the matching signedness into three 32-bit accumulators, exact for
 // reductions up to 16384 terms, put together in 64 bits.
 // The order of the reduction is free as long as both operands agree: lane (g, t) takes the 16 consecutive elements 16t .. 16t + 15 of a run.  A run's 16-byte
 // units lie XORed with the row, so a quarter warp's 16-byte reads meet no bank conflict.
-// Bound by the latency of a run - its copies, fragments and 32 products a warp, one after the other - while there is a block an SM (4 of 40x40: matrix pipe
-// 21 %, issue slots 44 % busy), by the matrix instruction (39 %), permutes and addresses (issue slots 53 %) together beyond that (256 of 28x28).  The 64 x 64
-// form spills 64 bytes at 128 registers, 64 x 32 8 bytes at 80.  us before and now: 4 of 40x40x64 -> 64 12.3 / 9.7, one of them 12.4 / 5.4,
-// 112x112x8 -> 16 at stride 2 12.3 / 3.7, 128x512x512 10.1 / 4.6, 51200x288x32 37 / 18, 200704x576x64 173 / 136.
+// Bound by the latency of copies, fragments and products, one after the other, while there is a block an SM (4 of 40x40: matrix pipe 21 %, issue slots 44 %
+// busy), by the matrix instruction (39 %), permutes and addresses (issue slots 53 %) together beyond that (256 of 28x28).  A barrier for three runs of
+// the reduction instead of each, the next three on their way: 4 of 40x40x64 -> 64, 3x3 10.0 -> 8.7 us, 34 of 70x71x64 -> 24 70.8 -> 59.6, 8 of 40x40x64 14.1 -> 12.1,
+// 10x10x256 -> 256 13.2 -> 11.7 (two at a time in two / three groups 9.2 / 9.3, 62.5 / 63.2, 12.7 / 13.0, 13.3 / 12.8).  Up to five runs are all asked for at the
+// start (80x80x32 6.4 -> 6.0).  The form of 64 x 64 spills 32 bytes, 64 x 32 4.
+// us before this kernel and now: 4 of 40x40x64 -> 64 12.3 / 8.7, one of them 12.4 / 5.8, 112x112x8 -> 16 at stride 2 12.3 / 3.2, 128x512x512 10.1 / 4.5.
 #include "common.cuh"
 
 #include <climits>
@@ -22,7 +24,7 @@ namespace espdl {
 
 namespace {
 
-constexpr int M16_STAGES = 4, M16_RUN = 64; // elements of the reduction a stage
+constexpr int M16_RUN = 64; // elements of the reduction a stage
 
 struct Mma16Params {
     const int16_t *in, *w;
@@ -69,11 +71,13 @@ __device__ __forceinline__ Planes split_planes(uint32_t run, int row, int t)
     return p;
 }
 
-// BM pixels x BN channels a block of eight warps, WM of them along the pixels (16 each), NT instructions' columns a warp.
-template <int WM, int NT>
+// BM pixels x BN channels a block of eight warps, WM of them along the pixels (16 each), NT instructions' columns a warp.  PAR runs are waited for, met and
+// multiplied together; GROUPS = 2: the next ones are on their way meanwhile, 1: they are all there are, all asked for at the start.
+template <int WM, int NT, int PAR, int GROUPS>
 __global__ void __launch_bounds__(256) conv_mma16_kernel(const __grid_constant__ Mma16Params p)
 {
     constexpr int WN = 8 / WM, BM = 16 * WM, BN = 8 * NT * WN, ROWS = BM + BN, PER = (ROWS + 31) / 32; // rows of a stage, copied 32 at a time
+    constexpr int STAGES = PAR * GROUPS, AHEAD = GROUPS == 1 ? PAR : STAGES - PAR;
     extern __shared__ __align__(128) uint8_t stage_mem[];
     grid_dep_launch(); // nothing is set up that the next kernel's blocks could disturb
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(stage_mem);
@@ -113,7 +117,7 @@ __global__ void __launch_bounds__(256) conv_mma16_kernel(const __grid_constant__
         const int r = row0 + 32 * j;
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + (uint32_t)r * 2u * M16_RUN + 16u * (uint32_t)(unit ^ (r & 7))), "l"(ok ? at : p.w), "r"(ok ? 16 : 0) : "memory");
     };
-    auto stage_of = [&](int run) { return base + (uint32_t)(run % M16_STAGES) * (ROWS * 2 * M16_RUN); };
+    auto stage_of = [&](int run) { return base + (uint32_t)(run % STAGES) * (ROWS * 2 * M16_RUN); };
     auto copy_filter = [&](int run) {
         const int at = run * M16_RUN + 8 * unit;
 #pragma unroll
@@ -132,13 +136,16 @@ __global__ void __launch_bounds__(256) conv_mma16_kernel(const __grid_constant__
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
     if (p.early)
-        for (int s = 0; s < M16_STAGES - 1; s++) copy_filter(s);
+        for (int s = 0; s < min(AHEAD, p.runs); s++) copy_filter(s);
     grid_dep_wait();
-    for (int s = 0; s < M16_STAGES - 1; s++) { // runs beyond the reduction are zeros
-        copy_pixels(s);
-        if (!p.early)
-            copy_filter(s);
-        commit();
+    for (int s = 0; s < AHEAD; s++) { // runs beyond the reduction are zeros
+        if (s < p.runs) {
+            copy_pixels(s);
+            if (!p.early)
+                copy_filter(s);
+        }
+        if ((s + 1) % PAR == 0)
+            commit();
     }
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, wm = warp % WM, wn = warp / WM;
@@ -147,26 +154,37 @@ __global__ void __launch_bounds__(256) conv_mma16_kernel(const __grid_constant__
     for (int j = 0; j < NT; j++)
 #pragma unroll
         for (int i = 0; i < 4; i++) hh[j][i] = mid[j][i] = ll[j][i] = 0;
-    for (int run = 0; run < p.runs; run++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(M16_STAGES - 2) : "memory");
-        __syncthreads(); // this run is there for all, and the stage of the run before is read by all
-        const uint32_t at = stage_of(run);
-        const Planes a0 = split_planes(at, 16 * wm + g, t), a1 = split_planes(at, 16 * wm + 8 + g, t);
+    for (int run0 = 0; run0 < p.runs; run0 += PAR) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GROUPS == 1 ? 0 : GROUPS - 2) : "memory");
+        __syncthreads(); // these runs are there for all, and the stages of the runs before are read by all
+        if (GROUPS > 1) { // on their way behind the products
 #pragma unroll
-        for (int j = 0; j < NT; j++) {
-            const Planes b = split_planes(at, BM + 8 * (NT * wn + j) + g, t);
-            mma_bytes<true, true>(hh[j], a0.hi.x, a1.hi.x, a0.hi.y, a1.hi.y, b.hi.x, b.hi.y);
-            mma_bytes<true, false>(mid[j], a0.hi.x, a1.hi.x, a0.hi.y, a1.hi.y, b.lo.x, b.lo.y);
-            mma_bytes<false, false>(ll[j], a0.lo.x, a1.lo.x, a0.lo.y, a1.lo.y, b.lo.x, b.lo.y);
-            mma_bytes<false, true>(mid[j], a0.lo.x, a1.lo.x, a0.lo.y, a1.lo.y, b.hi.x, b.hi.y);
-            mma_bytes<true, true>(hh[j], a0.hi.z, a1.hi.z, a0.hi.w, a1.hi.w, b.hi.z, b.hi.w);
-            mma_bytes<true, false>(mid[j], a0.hi.z, a1.hi.z, a0.hi.w, a1.hi.w, b.lo.z, b.lo.w);
-            mma_bytes<false, false>(ll[j], a0.lo.z, a1.lo.z, a0.lo.w, a1.lo.w, b.lo.z, b.lo.w);
-            mma_bytes<false, true>(mid[j], a0.lo.z, a1.lo.z, a0.lo.w, a1.lo.w, b.hi.z, b.hi.w);
+            for (int u = 0; u < PAR; u++)
+                if (run0 + AHEAD + u < p.runs) {
+                    copy_pixels(run0 + AHEAD + u);
+                    copy_filter(run0 + AHEAD + u);
+                }
+            commit();
         }
-        copy_pixels(run + M16_STAGES - 1); // behind the products, which run meanwhile
-        copy_filter(run + M16_STAGES - 1);
-        commit();
+#pragma unroll
+        for (int u = 0; u < PAR; u++) {
+            if (run0 + u >= p.runs)
+                break;
+            const uint32_t at = stage_of(run0 + u);
+            const Planes a0 = split_planes(at, 16 * wm + g, t), a1 = split_planes(at, 16 * wm + 8 + g, t);
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                const Planes b = split_planes(at, BM + 8 * (NT * wn + j) + g, t);
+                mma_bytes<true, true>(hh[j], a0.hi.x, a1.hi.x, a0.hi.y, a1.hi.y, b.hi.x, b.hi.y);
+                mma_bytes<true, false>(mid[j], a0.hi.x, a1.hi.x, a0.hi.y, a1.hi.y, b.lo.x, b.lo.y);
+                mma_bytes<false, false>(ll[j], a0.lo.x, a1.lo.x, a0.lo.y, a1.lo.y, b.lo.x, b.lo.y);
+                mma_bytes<false, true>(mid[j], a0.lo.x, a1.lo.x, a0.lo.y, a1.lo.y, b.hi.x, b.hi.y);
+                mma_bytes<true, true>(hh[j], a0.hi.z, a1.hi.z, a0.hi.w, a1.hi.w, b.hi.z, b.hi.w);
+                mma_bytes<true, false>(mid[j], a0.hi.z, a1.hi.z, a0.hi.w, a1.hi.w, b.lo.z, b.lo.w);
+                mma_bytes<false, false>(ll[j], a0.lo.z, a1.lo.z, a0.lo.w, a1.lo.w, b.lo.z, b.lo.w);
+                mma_bytes<false, true>(mid[j], a0.lo.z, a1.lo.z, a0.lo.w, a1.lo.w, b.hi.z, b.hi.w);
+            }
+        }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
 
@@ -239,19 +257,25 @@ Mma16Plan mma16_plan(const espdl_conv_desc &d)
     return best;
 }
 
-template <int WM, int NT>
-int launch_mma16(Mma16Params &p, cudaStream_t s)
+template <int WM, int NT, int PAR, int GROUPS>
+int launch_mma16_as(Mma16Params &p, cudaStream_t s)
 {
-    constexpr int BM = 16 * WM, BN = 8 * NT * (8 / WM), smem = M16_STAGES * (BM + BN) * 2 * M16_RUN;
+    constexpr int BM = 16 * WM, BN = 8 * NT * (8 / WM), stage = (BM + BN) * 2 * M16_RUN;
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] { attr_err = cudaFuncSetAttribute(conv_mma16_kernel<WM, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+    std::call_once(once, [] { attr_err = cudaFuncSetAttribute(conv_mma16_kernel<WM, NT, PAR, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAR * GROUPS * stage); });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(conv_mma16_kernel)");
     p.tiles_n = (p.N + BN - 1) / BN;
-    launch_overlapped(conv_mma16_kernel<WM, NT>, dim3((unsigned)(p.tiles_n * ((p.M + BM - 1) / BM))), dim3(256), smem, s, p);
+    launch_overlapped(conv_mma16_kernel<WM, NT, PAR, GROUPS>, dim3((unsigned)(p.tiles_n * ((p.M + BM - 1) / BM))), dim3(256), min(p.runs, PAR * GROUPS) * stage, s, p);
     count_launch();
     return check_launch("conv_mma16");
+}
+
+template <int WM, int NT>
+int launch_mma16(Mma16Params &p, cudaStream_t s)
+{
+    return p.runs <= 5 ? launch_mma16_as<WM, NT, 5, 1>(p, s) : launch_mma16_as<WM, NT, 3, 2>(p, s);
 }
 
 } // namespace

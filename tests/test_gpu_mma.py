@@ -122,6 +122,15 @@ def test_conv_int16(i, act, round_mode, monkeypatch):
     assert want.size < 8 or want.std() > 0
 
 
+# Runs of 64 elements of the reduction: all asked for at the start (up to five), whole and partial groups of three, the tiles of 64 x 64, 64 x 32 and 32 x 32
+@pytest.mark.parametrize("k", [8, 64, 72, 320, 328, 384, 392, 512, 576, 640, 832])
+@pytest.mark.parametrize("m,n", [(65, 40), (6400, 64), (40000, 72)])
+def test_int16_runs_of_the_reduction(m, n, k, monkeypatch):
+    monkeypatch.setenv("ESPDL_B200_MMA16", "always")
+    case = cases.gemm_case(seed=m + k, dtype=abi.DTYPE_INT16, m=m, k=k, n_out=n, per_channel=True, e_in=-13, e_out=-6, e_w=(-14, -11))
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+
+
 @pytest.mark.parametrize("e_w", [(-60, -30), (-1, 3), (20, 40)])
 def test_conv_int16_ends_of_the_range_and_any_shift(e_w, monkeypatch):
     """Every element at an end of the type, so that each plane's sum is as large as it gets; shifts from far left to beyond the sum."""
