@@ -5,7 +5,7 @@
 // The op is bandwidth bound by design (9 MACs per byte read).  3x3 filters with stride 1 or 2 - the shapes of
 // MobileNet-style networks - run on dw3x3_dp4a_kernel (a thread walks along a band of rows, dp4a over byte-transposed
 // columns), other windows of 3x3, 5x5 and 7x7 on dwk_dp4a_kernel; other int8 shapes with C % 16 == 0 on dw_s8_vec16_kernel (16 channels per thread, 128-bit loads and
-// stores, a warp reads and writes contiguous runs of the NHWC tensor); everything else on dw_generic_kernel.
+// stores, a warp reads and writes contiguous runs of the NHWC tensor), small ones and int16 on dw_taps_kernel; everything else on dw_generic_kernel.
 #include "common.cuh"
 
 namespace espdl {
@@ -450,6 +450,137 @@ __global__ void __launch_bounds__(256) dw_generic_kernel(DwParams p)
     }
 }
 
+// Any window, stride and dilation, int8 and int16, four channels of an output pixel a thread.  Eight taps' words are asked for before the first is used (one
+// after the other, each waited for, three taps over 24 pixels took as long as a launch more), and meet in dot products: groups of four taps of a channel in
+// dp4a, pairs in dp2a with the filter's high (signed) and low (unsigned) bytes - |sum| < 2^31 for 255 taps - where 64-bit multiply-adds a channel at a time
+// took twice as long.  us before / after: int8 24x32, 1x3 4.6 / 2.4, 20x20x128 3x3 at dilation 2 7.0 / 3.2; int16 154 of 12x11x192 5x5 146 / 65,
+// 64 of 56x56x96 3x3 421 / 178, 4 of 47x44x64 at stride 2 7.8 / 5.1.
+template <typename T>
+struct TapWord; // four channels
+template <>
+struct TapWord<int8_t> {
+    uint32_t v;
+};
+template <>
+struct TapWord<int16_t> {
+    uint2 v;
+};
+__device__ __forceinline__ void clear(TapWord<int8_t> &w) { w.v = 0u; }
+__device__ __forceinline__ void clear(TapWord<int16_t> &w) { w.v = make_uint2(0u, 0u); }
+__device__ __forceinline__ void load(TapWord<int8_t> &w, const int8_t *p) { w.v = __ldg((const uint32_t *)p); }
+__device__ __forceinline__ void load(TapWord<int16_t> &w, const int16_t *p) { w.v = __ldg((const uint2 *)p); }
+
+struct TapSums {
+    int hi[4], lo[4]; // int8: hi only
+};
+// Bytes of four words as one word per channel.
+__device__ __forceinline__ void transpose4(const TapWord<int8_t> *t, uint32_t (&c)[4])
+{
+    const uint32_t lo0 = __byte_perm(t[0].v, t[1].v, 0x5140), lo1 = __byte_perm(t[2].v, t[3].v, 0x5140), hi0 = __byte_perm(t[0].v, t[1].v, 0x7362),
+                   hi1 = __byte_perm(t[2].v, t[3].v, 0x7362);
+    c[0] = __byte_perm(lo0, lo1, 0x5410), c[1] = __byte_perm(lo0, lo1, 0x7632), c[2] = __byte_perm(hi0, hi1, 0x5410), c[3] = __byte_perm(hi0, hi1, 0x7632);
+}
+__device__ __forceinline__ void add_taps(TapSums &s, const TapWord<int8_t> (&x)[8], const TapWord<int8_t> (&w)[8])
+{
+#pragma unroll
+    for (int g = 0; g < 8; g += 4) {
+        uint32_t a[4], b[4];
+        transpose4(x + g, a), transpose4(w + g, b);
+#pragma unroll
+        for (int c = 0; c < 4; c++) s.hi[c] = __dp4a((int)a[c], (int)b[c], s.hi[c]);
+    }
+}
+__device__ __forceinline__ void add_taps(TapSums &s, const TapWord<int16_t> (&x)[8], const TapWord<int16_t> (&w)[8])
+{
+#pragma unroll
+    for (int g = 0; g < 8; g += 2)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const uint32_t x0 = c < 2 ? x[g].v.x : x[g].v.y, x1 = c < 2 ? x[g + 1].v.x : x[g + 1].v.y, w0 = c < 2 ? w[g].v.x : w[g].v.y, w1 = c < 2 ? w[g + 1].v.x : w[g + 1].v.y;
+            const uint32_t a = __byte_perm(x0, x1, c & 1 ? 0x7632 : 0x5410), b = __byte_perm(w0, w1, c & 1 ? 0x6273 : 0x4051); // b: high bytes, low bytes
+            asm("dp2a.lo.s32.s32 %0, %1, %2, %0;" : "+r"(s.hi[c]) : "r"(a), "r"(b));
+            asm("dp2a.hi.s32.u32 %0, %1, %2, %0;" : "+r"(s.lo[c]) : "r"(a), "r"(b));
+        }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128) dw_taps_kernel(DwParams p)
+{
+    grid_dep_launch();
+    if (!p.early)
+        grid_dep_wait();
+    const T *__restrict__ in = (const T *)p.in;
+    const T *__restrict__ w = (const T *)p.w;
+    T *__restrict__ out = (T *)p.out;
+    const unsigned words = (unsigned)p.c / 4, total = (unsigned)p.total;
+    const int taps = p.kh * p.kw;
+    bool first = true;
+    for (unsigned item = blockIdx.x * blockDim.x + threadIdx.x; item < total; item += gridDim.x * blockDim.x, first = false) {
+        const unsigned pix = item / words, ch = 4 * (item - pix * words), line = pix / (unsigned)p.ow, image = line / (unsigned)p.oh;
+        const int iy0 = (int)(line - image * p.oh) * p.sh - p.pt, ix0 = (int)(pix - line * p.ow) * p.sw - p.pl;
+        TapWord<T> wv[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            clear(wv[t]);
+            if (t < taps)
+                load(wv[t], w + (long long)t * p.c + ch);
+        }
+        int shift[4];
+        long long bias[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            shift[i] = p.e_shift_base - (p.per_channel ? __ldg(p.ew + ch + i) : p.ew_scalar);
+            bias[i] = !p.bias ? 0ll : sizeof(T) == 1 ? (long long)__ldg((const int32_t *)p.bias + ch + i) : __ldg((const long long *)p.bias + ch + i);
+        }
+        if (p.early && first)
+            grid_dep_wait();
+        const T *from = in + (long long)image * p.ih * p.iw * p.ips + ch;
+        TapSums s;
+#pragma unroll
+        for (int c = 0; c < 4; c++) s.hi[c] = s.lo[c] = 0;
+        int ky = 0, kx = 0;
+        for (int t0 = 0; t0 < taps; t0 += 8) {
+            TapWord<T> xv[8];
+#pragma unroll
+            for (int t = 0; t < 8; t++) {
+                const int iy = iy0 + ky * p.dh, ix = ix0 + kx * p.dw;
+                clear(xv[t]);
+                if (t0 + t < taps && (unsigned)iy < (unsigned)p.ih && (unsigned)ix < (unsigned)p.iw)
+                    load(xv[t], from + ((long long)iy * p.iw + ix) * p.ips);
+                if (++kx == p.kw)
+                    kx = 0, ky++;
+            }
+            if (t0) {
+#pragma unroll
+                for (int t = 0; t < 8; t++) {
+                    clear(wv[t]);
+                    if (t0 + t < taps)
+                        load(wv[t], w + (long long)(t0 + t) * p.c + ch);
+                }
+            }
+            add_taps(s, xv, wv);
+        }
+        int q[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (sizeof(T) == 1) {
+                q[i] = requant8(s.hi[i], (int)bias[i], max(-31, min(32, shift[i])), p.relu, p.half_even);
+                if (p.lut)
+                    q[i] = p.lut[(long long)(ch + i) * p.lut_stride + ((uint8_t)q[i] ^ 0x80u)];
+            } else {
+                q[i] = requant16((long long)s.hi[i] * 256 + s.lo[i], bias[i], max(-62, min(62, shift[i])), p.relu, p.half_even);
+            }
+        }
+        T *to = out + (long long)pix * p.ops + ch;
+        if (sizeof(T) == 1)
+            *(uint32_t *)to = ((uint32_t)q[0] & 0xffu) | (((uint32_t)q[1] & 0xffu) << 8) | (((uint32_t)q[2] & 0xffu) << 16) | ((uint32_t)q[3] << 24);
+        else
+            *(uint2 *)to = make_uint2(((uint32_t)q[0] & 0xffffu) | ((uint32_t)q[1] << 16), ((uint32_t)q[2] & 0xffffu) | ((uint32_t)q[3] << 16));
+    }
+    if (first && p.early)
+        grid_dep_wait();
+}
+
 int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
 {
     DwParams p;
@@ -470,6 +601,9 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
         ((uintptr_t)d.input % 16) == 0 && ((uintptr_t)d.output % 16) == 0 && ((uintptr_t)d.filter % 16) == 0;
     const bool words4 = d.dtype == ESPDL_DTYPE_INT8 && d.in_c % 4 == 0 && p.ips % 4 == 0 && p.ops % 4 == 0 && ((uintptr_t)d.input % 4) == 0 &&
         ((uintptr_t)d.output % 4) == 0 && ((uintptr_t)d.filter % 4) == 0;
+    const size_t word = d.dtype == ESPDL_DTYPE_INT8 ? 4 : 8; // four channels
+    const bool taps = d.in_c % 4 == 0 && p.ips % 4 == 0 && p.ops % 4 == 0 && (((uintptr_t)d.input | (uintptr_t)d.output | (uintptr_t)d.filter) % word) == 0 &&
+        d.kh * d.kw <= 255 && pixels * (d.in_c / 4) < 1ll << 31;
     const bool k3 = words4 && d.kh == 3 && d.kw == 3 && d.dilation_h == 1 && d.dilation_w == 1 && d.stride_h == d.stride_w &&
         (d.stride_h == 1 || d.stride_h == 2);
     const long long filter_bytes = (d.kh * d.kw + 3ll) / 4 * 4 * d.in_c; // of dwk_dp4a_kernel
@@ -499,6 +633,12 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
         p.total = pixels * (d.in_c / 4);
         const long long blocks = min((p.total + 255) / 256, max_blocks);
         launch_overlapped(d.kh == 3 ? dwk_dp4a_kernel<3> : (d.kh == 5 ? dwk_dp4a_kernel<5> : dwk_dp4a_kernel<7>), dim3((unsigned)blocks), dim3(256), (size_t)filter_bytes, s, p);
+    } else if (taps && (d.dtype == ESPDL_DTYPE_INT16 || !vec || pixels * (d.in_c / 4) <= 1024ll * num_sms())) {
+        // int8 beyond: sixteen channels a thread, whose address and epilogue cost a quarter (64x56x56x96 at dilation 2 67 us, 154 here; 4x40x40x64 7.1 / 6.7)
+        p.chunks = 0;
+        p.total = pixels * (d.in_c / 4);
+        const long long blocks = min((p.total + 127) / 128, max_blocks * 2);
+        launch_overlapped(d.dtype == ESPDL_DTYPE_INT8 ? dw_taps_kernel<int8_t> : dw_taps_kernel<int16_t>, dim3((unsigned)blocks), dim3(128), 0, s, p);
     } else if (vec) {
         p.chunks = d.in_c / 16;
         p.total = pixels * p.chunks;

@@ -85,6 +85,27 @@ DW_SHAPES = [
 ]
 
 
+# Any window in groups of eight taps (one group, whole ones, a remainder), windows that leave the image, strides of rows, the largest window that its sums allow at the
+# ends of the type, fused tables, and both sides of the line to sixteen channels a thread
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("dtype", [abi.DTYPE_INT8, abi.DTYPE_INT16])
+@pytest.mark.parametrize("kw", [dict(n=1, h=1, w=24, cin=32, kh=1, kw=3, pad=(0, 0, 2, 0)), dict(n=3, h=9, w=7, cin=20, kh=3, kw=3, dil=2, pad=(2, 2, 2, 2)),
+                                dict(n=2, h=11, w=13, cin=48, kh=4, kw=4, pad=(1, 2, 2, 1)), dict(n=1, h=6, w=40, cin=8, kh=2, kw=9, stride=2, pad=(0, 0, 4, 4)),
+                                dict(n=2, h=20, w=19, cin=4, kh=15, kw=17, pad=(7, 7, 8, 8)), dict(n=1, h=5, w=5, cin=36, kh=1, kw=1, pad=(0, 0, 0, 0)),
+                                dict(n=2, h=8, w=9, cin=24, kh=5, kw=5, in_stride=40, out_stride=56), dict(n=2, h=9, w=9, cin=16, kh=1, kw=5, pad=(0, 0, 2, 2), lut="channels"),
+                                dict(n=40, h=40, w=41, cin=16, kh=1, kw=5, pad=(0, 0, 2, 2))])
+def test_depthwise_taps(kw, dtype, round_mode):
+    exps = dict(e_in=-7, e_out=-4, e_w=(-9, -6)) if dtype == abi.DTYPE_INT8 else dict(e_in=-13, e_out=-9, e_w=(-14, -11), wide=True)
+    if dtype == abi.DTYPE_INT16:
+        kw = {k: v for k, v in kw.items() if k != "lut"}
+    case = cases.conv_case(seed=77, dtype=dtype, depthwise=True, per_channel=True, round_mode=round_mode, **exps, **kw)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+    if dtype == abi.DTYPE_INT16 and kw["kh"] * kw["kw"] == 255:
+        case["x"][...], case["w"][...] = -32768, -1
+        case["w"][..., 1::2] = -32768
+        np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+
+
 @pytest.mark.parametrize("tma", [False, True], ids=["auto", "tma"])
 @pytest.mark.parametrize("kw", DW_SHAPES, ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "pad"))
 def test_depthwise_3x3_shapes(kw, tma, monkeypatch):
