@@ -205,14 +205,30 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
 {
     if (early)
         grid_dep_launch();
-    grid_dep_wait();
     constexpr int V = 4 * W / (int)sizeof(T), PER_WORD = 4 / (int)sizeof(T), BITS = 8 * (int)sizeof(T);
     __shared__ int8_t table[256];
     // One-operand int8 -> int8 operators are functions of the input byte: every block tabulates the operator once with
     // the scalar code (so the rounding is the reference's) and then runs as a table lookup like LUT itself.
     constexpr bool TABULATED = sizeof(T) == 1 && (OP == ESPDL_ELT_REQUANTIZE || OP == ESPDL_ELT_CLIP || OP == ESPDL_ELT_RELU);
     constexpr bool LOOKUP = sizeof(T) == 1 && (OP == ESPDL_ELT_LUT || TABULATED);
+    // In a small network a launch is one trip through memory: where the first unit lies and, inside a model's plan, whose tables no launch
+    // writes, the table are found out before the wait for the previous kernel, and the unit is on its way while the block meets over the table.
+    auto offsets = [&](long long v, long long &io, long long &ia, long long &ib) {
+        if (BCAST) {
+            const long long row = v < 0x7fffffffll ? (long long)((unsigned)v / (unsigned)p.vpr) : v / p.vpr, col = v - row * p.vpr;
+            const long long image = v < 0x7fffffffll ? (long long)((unsigned)row / (unsigned)p.rows_per_image) : row / p.rows_per_image;
+            io = row * p.ro + col, ia = row * p.ra + col, ib = image * p.b_image + col;
+        } else {
+            vec_offsets(p, v, io, ia, ib);
+        }
+    };
+    const long long threads = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    long long io = 0, ia = 0, ib = 0;
+    if (first < nvec)
+        offsets(first, io, ia, ib);
     if (LOOKUP) {
+        if (!early && OP == ESPDL_ELT_LUT)
+            grid_dep_wait();
         for (int i = threadIdx.x; i < 256; i += blockDim.x) {
             if (OP == ESPDL_ELT_LUT) {
                 table[i] = ((const int8_t *)p.b)[i];
@@ -222,8 +238,9 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
                 table[i] = (int8_t)sat8((int)max(-1000000ll, min(1000000ll, elt_int(q2, (int)(int8_t)(uint8_t)(i ^ 0x80), 0))));
             }
         }
-        __syncthreads();
     }
+    if (!LOOKUP || early || OP != ESPDL_ELT_LUT)
+        grid_dep_wait();
     auto one = [&](int a, int b) -> int {
         if (LOOKUP)
             return table[(uint8_t)a ^ 0x80u];
@@ -238,23 +255,17 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
         const int lo = -(1 << (BITS - 1));
         return (int)max((long long)lo, min((long long)(-lo - 1), v));
     };
-    const long long threads = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    for (long long v = first; v < nvec; v += threads) {
-        long long io, ia, ib;
-        if (BCAST) {
-            const long long row = v < 0x7fffffffll ? (long long)((unsigned)v / (unsigned)p.vpr) : v / p.vpr, col = v - row * p.vpr;
-            const long long image = v < 0x7fffffffll ? (long long)((unsigned)row / (unsigned)p.rows_per_image) : row / p.rows_per_image;
-            io = row * p.ro + col, ia = row * p.ra + col, ib = image * p.b_image + col;
-        } else {
-            vec_offsets(p, v, io, ia, ib);
-        }
-        struct alignas(4 * W) Unit {
-            uint32_t w[W];
-        };
-        const Unit a = ((const Unit *)p.a)[ia];
-        Unit b = {}, o;
+    struct alignas(4 * W) Unit {
+        uint32_t w[W];
+    };
+    Unit a = {}, b = {};
+    auto fetch = [&] {
+        a = ((const Unit *)p.a)[ia];
         if (elt_two_operands(OP))
             b = ((const Unit *)p.b)[ib];
+    };
+    auto finish = [&] {
+        Unit o;
 #pragma unroll
         for (int q = 0; q < W; q++) {
             uint32_t wd = 0;
@@ -266,6 +277,22 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
             o.w[q] = wd;
         }
         ((Unit *)p.out)[io] = o;
+    };
+    if (nvec <= threads) { // one unit a thread
+        if (first < nvec)
+            fetch();
+        if (LOOKUP)
+            __syncthreads();
+        if (first < nvec)
+            finish();
+    } else {
+        if (LOOKUP)
+            __syncthreads();
+        for (long long v = first; v < nvec; v += threads) {
+            offsets(v, io, ia, ib);
+            fetch();
+            finish();
+        }
     }
     if (!BCAST && !p.vpr)
         for (long long i = nvec * V + first; i < p.total; i += threads)

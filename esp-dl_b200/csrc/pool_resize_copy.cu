@@ -837,16 +837,18 @@ __global__ void __launch_bounds__(256) concat_split_kernel(PartsParams p, int ea
 {
     if (early)
         grid_dep_launch();
-    grid_dep_wait();
     const int upr = p.start[p.n_parts];
+    bool waited = false;
     for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < p.total; u += (long long)gridDim.x * blockDim.x) {
-        const long long row = u / upr;
+        const long long row = u < 0x7fffffffll ? (long long)((unsigned)u / (unsigned)upr) : u / upr;
         const int col = (int)(u - row * upr);
         int i = 0;
 #pragma unroll
         for (int k = 1; k < 8; k++)
             if (k < p.n_parts && col >= p.start[k])
                 i = k;
+        if (!waited) // the first unit's place is found out before
+            grid_dep_wait(), waited = true;
         if (!p.parts[i])
             continue;
         uint4 *part = p.parts[i] + row * p.pitch[i] + (col - p.start[i]);
@@ -855,6 +857,8 @@ __global__ void __launch_bounds__(256) concat_split_kernel(PartsParams p, int ea
         else
             p.wide[u] = *part;
     }
+    if (!waited)
+        grid_dep_wait();
 }
 } // namespace
 } // namespace espdl
