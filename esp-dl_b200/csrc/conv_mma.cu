@@ -170,9 +170,11 @@ __global__ void __launch_bounds__(32 * MMA_WARPS) conv_mma_kernel(const __grid_c
             row_ok[i][h] = active && m < p.M;
             const long long pix = image0 + (row_ok[i][h] ? m : 0);
             if (WINDOW) {
-                const int ox = (int)(pix % p.ow), oy = (int)(pix / p.ow % p.oh);
+                // at most 2^24 pixels: divisions of 32 bits (of 64 they were a tenth of a first layer's instructions)
+                const unsigned line = (unsigned)pix / (unsigned)p.ow, image = line / (unsigned)p.oh;
+                const int ox = (int)((unsigned)pix - line * (unsigned)p.ow), oy = (int)(line - image * (unsigned)p.oh);
                 iy0[i][h] = oy * p.sh - p.pt, ix0[i][h] = ox * p.sw - p.pl;
-                row[i][h] = p.in + (pix / ((long long)p.ow * p.oh)) * p.ih * p.iw * p.ips;
+                row[i][h] = p.in + (long long)image * p.ih * p.iw * p.ips;
             } else {
                 row[i][h] = p.in + pix * p.ips;
             }
