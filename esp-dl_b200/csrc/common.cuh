@@ -235,6 +235,28 @@ __device__ __forceinline__ int fround_half_up(float v) { return (int)floorf(__fa
 __device__ __forceinline__ int fround_half_even(float v) { return __float2int_rn(v); }
 __device__ __forceinline__ int fround(float v, int half_even) { return half_even ? fround_half_even(v) : fround_half_up(v); }
 
+// a / b and what is left, a >= 0, b > 0.  A 64-bit division is some hundred instructions; a few of them were a third of the time of a small launch, most tensors'
+// indices fit 32 bits.
+__device__ __forceinline__ long long div_rem(long long a, long long b, long long &rem)
+{
+    if (((a | b) >> 32) == 0) {
+        const unsigned q = (unsigned)a / (unsigned)b;
+        rem = (unsigned)a - q * (unsigned)b;
+        return q;
+    }
+    const long long q = a / b;
+    rem = a - q * b;
+    return q;
+}
+
+// Column, row and image of an output pixel.
+__device__ __forceinline__ void split_pixel(long long pix, int ow, int oh, int &x, int &y, int &n)
+{
+    long long rem_x, rem_y;
+    n = (int)div_rem(div_rem(pix, ow, rem_x), oh, rem_y);
+    x = (int)rem_x, y = (int)rem_y;
+}
+
 // DL_SCALE / DL_RESCALE: exact powers of two as floats.
 __host__ __device__ __forceinline__ float dl_scale(int e) { return e > 0 ? (float)(1 << e) : 1.0f / (float)(1 << -e); }
 __host__ __device__ __forceinline__ float dl_rescale(int e) { return e > 0 ? 1.0f / (float)(1 << e) : (float)(1 << -e); }

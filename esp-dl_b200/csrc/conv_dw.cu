@@ -35,11 +35,11 @@ __global__ void __launch_bounds__(256) dw_s8_vec16_kernel(DwParams p)
     int8_t *__restrict__ out = (int8_t *)p.out;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < p.total;
          item += (long long)gridDim.x * blockDim.x) {
-        const int ch = (int)(item % p.chunks) * 16;
-        const long long pix = item / p.chunks;
-        const int ox = (int)(pix % p.ow);
-        const int oy = (int)((pix / p.ow) % p.oh);
-        const int n = (int)(pix / ((long long)p.ow * p.oh));
+        long long ch_rem;
+        const long long pix = div_rem(item, p.chunks, ch_rem);
+        const int ch = (int)ch_rem * 16;
+        int ox, oy, n;
+        split_pixel(pix, p.ow, p.oh, ox, oy, n);
         int32_t acc[16];
 #pragma unroll
         for (int j = 0; j < 16; j++) acc[j] = 0;
@@ -240,12 +240,11 @@ __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xseg
     const long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (item >= p.total)
         return;
-    const int cq = (int)(item % quads);
-    long long r = item / quads;
-    const int yt = (int)(r % ytiles);
-    r /= ytiles;
-    const int xs = (int)(r % xsegs);
-    const int n = (int)(r / xsegs);
+    long long cq_rem;
+    long long r = div_rem(item, quads, cq_rem);
+    const int cq = (int)cq_rem;
+    int yt, xs, n;
+    split_pixel(r, ytiles, xsegs, yt, xs, n);
     const int c0 = cq * 4;
 
     // filter columns as dp4a operands: wv[kx][i] = (w[0][kx][i], w[1][kx][i], w[2][kx][i], 0)
@@ -418,11 +417,11 @@ __global__ void __launch_bounds__(256) dw_generic_kernel(DwParams p)
     T *__restrict__ out = (T *)p.out;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < p.total;
          item += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(item % p.c);
-        const long long pix = item / p.c;
-        const int ox = (int)(pix % p.ow);
-        const int oy = (int)((pix / p.ow) % p.oh);
-        const int n = (int)(pix / ((long long)p.ow * p.oh));
+        long long c_rem;
+        const long long pix = div_rem(item, p.c, c_rem);
+        const int c = (int)c_rem;
+        int ox, oy, n;
+        split_pixel(pix, p.ow, p.oh, ox, oy, n);
         ACC acc = 0;
         for (int ky = 0; ky < p.kh; ky++) {
             const int iy = oy * p.sh + ky * p.dh - p.pt;

@@ -32,7 +32,8 @@ __global__ void __launch_bounds__(256) detect_candidates_kernel(espdl_detect_des
                 if (slot >= (uint32_t)d.capacity)
                     continue; // counted, not stored: the caller sees count > capacity
                 espdl_detect_record *r = d.records + slot;
-                const int x = (int)(pix % d.w), y = (int)((pix / d.w) % d.h), img = (int)(pix / ((long long)d.w * d.h));
+                int x, y, img;
+                split_pixel(pix, d.w, d.h, x, y, img);
                 r->image = (uint16_t)img, r->stage = (uint16_t)d.stage, r->y = (uint16_t)y, r->x = (uint16_t)x;
                 r->category = (uint16_t)(c0 + j), r->score = v[j], r->pad = 0, r->reserved = 0;
                 const int8_t *bp = d.box + pix * d.box_channels;

@@ -35,9 +35,8 @@ __global__ void __launch_bounds__(256) image_pre_kernel(ImgParams p, int early)
     const int inner_w = p.dw - p.bl - p.br, inner_h = p.dh - p.bt - p.bb;
     T *out = (T *)p.out;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < p.total; item += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(item % p.dw);
-        const int y = (int)((item / p.dw) % p.dh);
-        const int img = (int)(item / ((long long)p.dw * p.dh));
+        int x, y, img;
+        split_pixel(item, p.dw, p.dh, x, y, img);
         const int xi = x - p.bl, yi = y - p.bt;
         uint8_t v[3];
         if (xi < 0 || xi >= inner_w || yi < 0 || yi >= inner_h) {

@@ -22,11 +22,11 @@ __global__ void __launch_bounds__(256) pool_kernel(PoolParams p, int early)
         grid_dep_launch();
     grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % p.c);
-        const long long pix = i / p.c;
-        const int ox = (int)(pix % p.ow);
-        const int oy = (int)((pix / p.ow) % p.oh);
-        const int n = (int)(pix / ((long long)p.ow * p.oh));
+        long long c_rem;
+        const long long pix = div_rem(i, p.c, c_rem);
+        const int c = (int)c_rem;
+        int ox, oy, n;
+        split_pixel(pix, p.ow, p.oh, ox, oy, n);
         long long sum = 0;
         int mx = INT32_MIN;
         for (int ky = 0; ky < p.kh; ky++) {
@@ -68,11 +68,11 @@ __global__ void __launch_bounds__(256) maxpool_s8_vec16_kernel(PoolParams p, int
     const int chunks = p.c >> 4;
     const long long total = (long long)p.n * p.oh * p.ow * chunks;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int ch = (int)(i % chunks) * 16;
-        const long long pix = i / chunks;
-        const int ox = (int)(pix % p.ow);
-        const int oy = (int)((pix / p.ow) % p.oh);
-        const int n = (int)(pix / ((long long)p.ow * p.oh));
+        long long ch_rem;
+        const long long pix = div_rem(i, chunks, ch_rem);
+        const int ch = (int)ch_rem * 16;
+        int ox, oy, n;
+        split_pixel(pix, p.ow, p.oh, ox, oy, n);
         uint4 m = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u); // -128 in every byte
         for (int ky = 0; ky < p.kh; ky++) {
             const int iy = oy * p.sh + ky - p.pt;
@@ -131,10 +131,12 @@ __global__ void __launch_bounds__(256) maxpool_s8_walk_kernel(PoolParams p, int 
     const int seg_rows = (p.oh + segments - 1) / segments; // a column is cut into `segments` runs of output rows when there are few columns
     const long long total = (long long)p.n * segments * p.ow * chunks;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < total; item += (long long)gridDim.x * blockDim.x) {
-        const int ch = (int)(item % chunks) * 16;
-        const int ox = (int)((item / chunks) % p.ow);
-        const int seg = (int)((item / ((long long)chunks * p.ow)) % segments);
-        const long long n = item / ((long long)chunks * p.ow * segments);
+        long long ch_rem;
+        const long long column = div_rem(item, chunks, ch_rem);
+        const int ch = (int)ch_rem * 16;
+        int ox, seg, image;
+        split_pixel(column, p.ow, segments, ox, seg, image);
+        const long long n = image;
         const int oy0 = seg * seg_rows, oy1 = min(p.oh, oy0 + seg_rows);
         const int8_t *in = (const int8_t *)p.in + n * p.ih * (long long)p.iw * p.c + ch;
         int8_t *out = (int8_t *)p.out + (n * p.oh * (long long)p.ow + ox) * p.c + ch;
@@ -202,10 +204,12 @@ __global__ void __launch_bounds__(256) maxpool_walk_kernel(PoolParams p, int seg
     const int seg_rows = (p.oh + segments - 1) / segments;
     const long long total = (long long)p.n * segments * p.ow * chunks;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < total; item += (long long)gridDim.x * blockDim.x) {
-        const int ch = (int)(item % chunks) * V;
-        const int ox = (int)((item / chunks) % p.ow);
-        const int seg = (int)((item / ((long long)chunks * p.ow)) % segments);
-        const long long n = item / ((long long)chunks * p.ow * segments);
+        long long ch_rem;
+        const long long column = div_rem(item, chunks, ch_rem);
+        const int ch = (int)ch_rem * V;
+        int ox, seg, image;
+        split_pixel(column, p.ow, segments, ox, seg, image);
+        const long long n = image;
         const int oy0 = seg * seg_rows, oy1 = min(p.oh, oy0 + seg_rows);
         const T *in = (const T *)p.in + n * p.ih * (long long)p.iw * p.c + ch;
         T *out = (T *)p.out + (n * p.oh * (long long)p.ow + ox) * p.c + ch;
@@ -322,11 +326,11 @@ __global__ void __launch_bounds__(256) resize_nearest_kernel(ResizeParams p, int
         grid_dep_launch();
     grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % p.c);
-        const long long pix = i / p.c;
-        const int x = (int)(pix % p.ow);
-        const int y = (int)((pix / p.ow) % p.oh);
-        const int n = (int)(pix / ((long long)p.ow * p.oh));
+        long long c_rem;
+        const long long pix = div_rem(i, p.c, c_rem);
+        const int c = (int)c_rem;
+        int x, y, n;
+        split_pixel(pix, p.ow, p.oh, x, y, n);
         int iy = p.two ? y / 2 : (int)__fmul_rn((float)y, p.sh_inv);
         int ix = p.two ? x / 2 : (int)__fmul_rn((float)x, p.sw_inv);
         iy = min(iy, p.ih - 1);
@@ -348,11 +352,11 @@ __global__ void __launch_bounds__(256) resize_nearest_vec16_kernel(ResizeParams 
     const int chunks = p.c >> 4;
     const long long total = (long long)p.n * p.oh * p.ow * chunks;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int ch = (int)(i % chunks) * 16;
-        const long long pix = i / chunks;
-        const int x = (int)(pix % p.ow);
-        const int y = (int)((pix / p.ow) % p.oh);
-        const int n = (int)(pix / ((long long)p.ow * p.oh));
+        long long ch_rem;
+        const long long pix = div_rem(i, chunks, ch_rem);
+        const int ch = (int)ch_rem * 16;
+        int x, y, n;
+        split_pixel(pix, p.ow, p.oh, x, y, n);
         int iy = p.two ? y / 2 : (int)__fmul_rn((float)y, p.sh_inv);
         int ix = p.two ? x / 2 : (int)__fmul_rn((float)x, p.sw_inv);
         iy = min(iy, p.ih - 1);
@@ -381,8 +385,8 @@ __global__ void __launch_bounds__(256) copy_kernel(CopyParams p, int early)
         long long r = i, si = 0, di = 0;
 #pragma unroll
         for (int k = 5; k >= 0; k--) {
-            const int idx = (int)(r % p.shape[k]);
-            r /= p.shape[k];
+            long long idx;
+            r = div_rem(r, p.shape[k], idx);
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
@@ -406,17 +410,16 @@ __global__ void __launch_bounds__(256) copy_transpose_kernel(CopyParams p, int y
     const int tx_count = (nx + TILE - 1) / TILE, ty_count = (ny + TILE - 1) / TILE;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         long long r = t;
-        const int x0 = (int)(r % tx_count) * TILE;
-        r /= tx_count;
-        const int y0 = (int)(r % ty_count) * TILE;
-        r /= ty_count;
+        long long tx, ty;
+        r = div_rem(div_rem(r, tx_count, tx), ty_count, ty);
+        const int x0 = (int)tx * TILE, y0 = (int)ty * TILE;
         long long si = 0, di = 0;
 #pragma unroll
         for (int k = 4; k >= 0; k--) {
             if (k == ya)
                 continue;
-            const int idx = (int)(r % p.shape[k]);
-            r /= p.shape[k];
+            long long idx;
+            r = div_rem(r, p.shape[k], idx);
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
@@ -457,17 +460,16 @@ __global__ void __launch_bounds__(256) copy_transpose_words_kernel(CopyParams p,
     const int tx_count = (nx + TILE - 1) / TILE, ty_count = (ny + TILE - 1) / TILE;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         long long r = t;
-        const int x0 = (int)(r % tx_count) * TILE;
-        r /= tx_count;
-        const int y0 = (int)(r % ty_count) * TILE;
-        r /= ty_count;
+        long long tx, ty;
+        r = div_rem(div_rem(r, tx_count, tx), ty_count, ty);
+        const int x0 = (int)tx * TILE, y0 = (int)ty * TILE;
         long long si = 0, di = 0;
 #pragma unroll
         for (int k = 4; k >= 0; k--) {
             if (k == ya)
                 continue;
-            const int idx = (int)(r % p.shape[k]);
-            r /= p.shape[k];
+            long long idx;
+            r = div_rem(r, p.shape[k], idx);
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
@@ -515,17 +517,16 @@ __global__ void __launch_bounds__(256) copy_transpose_bytes4_kernel(CopyParams p
     const int tx_count = (nx + TILE - 1) / TILE, ty_count = (ny + TILE - 1) / TILE;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         long long r = t;
-        const int x0 = (int)(r % tx_count) * TILE;
-        r /= tx_count;
-        const int y0 = (int)(r % ty_count) * TILE;
-        r /= ty_count;
+        long long tx, ty;
+        r = div_rem(div_rem(r, tx_count, tx), ty_count, ty);
+        const int x0 = (int)tx * TILE, y0 = (int)ty * TILE;
         long long si = 0, di = 0;
 #pragma unroll
         for (int k = 4; k >= 0; k--) {
             if (k == ya)
                 continue;
-            const int idx = (int)(r % p.shape[k]);
-            r /= p.shape[k];
+            long long idx;
+            r = div_rem(r, p.shape[k], idx);
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
@@ -694,11 +695,11 @@ __global__ void __launch_bounds__(256) resize_linear_kernel(ResizeLinearParams p
         grid_dep_launch();
     grid_dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % p.c);
-        const long long pix = i / p.c;
-        const int x = (int)(pix % p.ow);
-        const int y = (int)((pix / p.ow) % p.oh);
-        const int n = (int)(pix / ((long long)p.ow * p.oh));
+        long long c_rem;
+        const long long pix = div_rem(i, p.c, c_rem);
+        const int c = (int)c_rem;
+        int x, y, n;
+        split_pixel(pix, p.ow, p.oh, x, y, n);
         int ix, iy = 0;
         float xr0, xr1, yr0 = 1.f, yr1 = 0.f;
         linear_coeffs_dev(x, ix, xr0, xr1, p.iw, p.sw_inv, p.align);
