@@ -240,11 +240,12 @@ __global__ void __launch_bounds__(128, 4) dw3x3_dp4a_kernel(DwParams p, int xseg
     const long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (item >= p.total)
         return;
-    long long cq_rem;
-    long long r = div_rem(item, quads, cq_rem);
-    const int cq = (int)cq_rem;
-    int yt, xs, n;
-    split_pixel(r, ytiles, xsegs, yt, xs, n);
+    const int cq = (int)(item % quads);
+    long long r = item / quads;
+    const int yt = (int)(r % ytiles);
+    r /= ytiles;
+    const int xs = (int)(r % xsegs);
+    const int n = (int)(r / xsegs);
     const int c0 = cq * 4;
 
     // filter columns as dp4a operands: wv[kx][i] = (w[0][kx][i], w[1][kx][i], w[2][kx][i], 0)

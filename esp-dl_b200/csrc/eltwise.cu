@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
     };
     const long long threads = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     long long io = 0, ia = 0, ib = 0;
-    if (first < nvec)
+    if (sizeof(T) == 1 && first < nvec)
         offsets(first, io, ia, ib);
     if (LOOKUP) {
         if (!early && OP == ESPDL_ELT_LUT)
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
         }
         ((Unit *)p.out)[io] = o;
     };
-    if (nvec <= threads) { // one unit a thread
+    if (sizeof(T) == 1 && nvec <= threads) { // one unit a thread (int16: its results' code twice costs the large launches more than the small ones gain)
         if (first < nvec)
             fetch();
         if (LOOKUP)

@@ -68,11 +68,11 @@ __global__ void __launch_bounds__(256) maxpool_s8_vec16_kernel(PoolParams p, int
     const int chunks = p.c >> 4;
     const long long total = (long long)p.n * p.oh * p.ow * chunks;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        long long ch_rem;
-        const long long pix = div_rem(i, chunks, ch_rem);
-        const int ch = (int)ch_rem * 16;
-        int ox, oy, n;
-        split_pixel(pix, p.ow, p.oh, ox, oy, n);
+        const int ch = (int)(i % chunks) * 16;
+        const long long pix = i / chunks;
+        const int ox = (int)(pix % p.ow);
+        const int oy = (int)((pix / p.ow) % p.oh);
+        const int n = (int)(pix / ((long long)p.ow * p.oh));
         uint4 m = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u); // -128 in every byte
         for (int ky = 0; ky < p.kh; ky++) {
             const int iy = oy * p.sh + ky - p.pt;
@@ -131,12 +131,10 @@ __global__ void __launch_bounds__(256) maxpool_s8_walk_kernel(PoolParams p, int 
     const int seg_rows = (p.oh + segments - 1) / segments; // a column is cut into `segments` runs of output rows when there are few columns
     const long long total = (long long)p.n * segments * p.ow * chunks;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < total; item += (long long)gridDim.x * blockDim.x) {
-        long long ch_rem;
-        const long long column = div_rem(item, chunks, ch_rem);
-        const int ch = (int)ch_rem * 16;
-        int ox, seg, image;
-        split_pixel(column, p.ow, segments, ox, seg, image);
-        const long long n = image;
+        const int ch = (int)(item % chunks) * 16;
+        const int ox = (int)((item / chunks) % p.ow);
+        const int seg = (int)((item / ((long long)chunks * p.ow)) % segments);
+        const long long n = item / ((long long)chunks * p.ow * segments);
         const int oy0 = seg * seg_rows, oy1 = min(p.oh, oy0 + seg_rows);
         const int8_t *in = (const int8_t *)p.in + n * p.ih * (long long)p.iw * p.c + ch;
         int8_t *out = (int8_t *)p.out + (n * p.oh * (long long)p.ow + ox) * p.c + ch;
@@ -204,12 +202,10 @@ __global__ void __launch_bounds__(256) maxpool_walk_kernel(PoolParams p, int seg
     const int seg_rows = (p.oh + segments - 1) / segments;
     const long long total = (long long)p.n * segments * p.ow * chunks;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < total; item += (long long)gridDim.x * blockDim.x) {
-        long long ch_rem;
-        const long long column = div_rem(item, chunks, ch_rem);
-        const int ch = (int)ch_rem * V;
-        int ox, seg, image;
-        split_pixel(column, p.ow, segments, ox, seg, image);
-        const long long n = image;
+        const int ch = (int)(item % chunks) * V;
+        const int ox = (int)((item / chunks) % p.ow);
+        const int seg = (int)((item / ((long long)chunks * p.ow)) % segments);
+        const long long n = item / ((long long)chunks * p.ow * segments);
         const int oy0 = seg * seg_rows, oy1 = min(p.oh, oy0 + seg_rows);
         const T *in = (const T *)p.in + n * p.ih * (long long)p.iw * p.c + ch;
         T *out = (T *)p.out + (n * p.oh * (long long)p.ow + ox) * p.c + ch;
@@ -410,16 +406,17 @@ __global__ void __launch_bounds__(256) copy_transpose_kernel(CopyParams p, int y
     const int tx_count = (nx + TILE - 1) / TILE, ty_count = (ny + TILE - 1) / TILE;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         long long r = t;
-        long long tx, ty;
-        r = div_rem(div_rem(r, tx_count, tx), ty_count, ty);
-        const int x0 = (int)tx * TILE, y0 = (int)ty * TILE;
+        const int x0 = (int)(r % tx_count) * TILE;
+        r /= tx_count;
+        const int y0 = (int)(r % ty_count) * TILE;
+        r /= ty_count;
         long long si = 0, di = 0;
 #pragma unroll
         for (int k = 4; k >= 0; k--) {
             if (k == ya)
                 continue;
-            long long idx;
-            r = div_rem(r, p.shape[k], idx);
+            const int idx = (int)(r % p.shape[k]);
+            r /= p.shape[k];
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
@@ -460,16 +457,17 @@ __global__ void __launch_bounds__(256) copy_transpose_words_kernel(CopyParams p,
     const int tx_count = (nx + TILE - 1) / TILE, ty_count = (ny + TILE - 1) / TILE;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         long long r = t;
-        long long tx, ty;
-        r = div_rem(div_rem(r, tx_count, tx), ty_count, ty);
-        const int x0 = (int)tx * TILE, y0 = (int)ty * TILE;
+        const int x0 = (int)(r % tx_count) * TILE;
+        r /= tx_count;
+        const int y0 = (int)(r % ty_count) * TILE;
+        r /= ty_count;
         long long si = 0, di = 0;
 #pragma unroll
         for (int k = 4; k >= 0; k--) {
             if (k == ya)
                 continue;
-            long long idx;
-            r = div_rem(r, p.shape[k], idx);
+            const int idx = (int)(r % p.shape[k]);
+            r /= p.shape[k];
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
@@ -517,16 +515,17 @@ __global__ void __launch_bounds__(256) copy_transpose_bytes4_kernel(CopyParams p
     const int tx_count = (nx + TILE - 1) / TILE, ty_count = (ny + TILE - 1) / TILE;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         long long r = t;
-        long long tx, ty;
-        r = div_rem(div_rem(r, tx_count, tx), ty_count, ty);
-        const int x0 = (int)tx * TILE, y0 = (int)ty * TILE;
+        const int x0 = (int)(r % tx_count) * TILE;
+        r /= tx_count;
+        const int y0 = (int)(r % ty_count) * TILE;
+        r /= ty_count;
         long long si = 0, di = 0;
 #pragma unroll
         for (int k = 4; k >= 0; k--) {
             if (k == ya)
                 continue;
-            long long idx;
-            r = div_rem(r, p.shape[k], idx);
+            const int idx = (int)(r % p.shape[k]);
+            r /= p.shape[k];
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
