@@ -9,7 +9,7 @@
 // reductions up to 16384 terms, put together in 64 bits.
 // The order of the reduction is free as long as both operands agree: lane (g, t) takes the 16 consecutive elements 16t .. 16t + 15 of a run.  A run's 16-byte
 // units lie XORed with the row, so a quarter warp's 16-byte reads meet no bank conflict.
-// Bound by the latency of copies, fragments and products, one after the other, while there is a block an SM (4 of 40x40: matrix pipe 21 %, issue slots 44 %
+// Bound by the latency of copies, fragments and products, one after the other, while there is a block an SM (4 of 40x40: matrix pipe 24 %, issue slots 43 %
 // busy), by the matrix instruction (39 %), permutes and addresses (issue slots 53 %) together beyond that (256 of 28x28).  A barrier for three runs of
 // the reduction instead of each, the next three on their way: 4 of 40x40x64 -> 64, 3x3 10.0 -> 8.7 us, 34 of 70x71x64 -> 24 70.8 -> 59.6, 8 of 40x40x64 14.1 -> 12.1,
 // 10x10x256 -> 256 13.2 -> 11.7 (two at a time in two / three groups 9.2 / 9.3, 62.5 / 63.2, 12.7 / 13.0, 13.3 / 12.8).  Up to five runs are all asked for at the
