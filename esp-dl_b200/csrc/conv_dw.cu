@@ -5,7 +5,8 @@
 // The op is bandwidth bound by design (9 MACs per byte read).  3x3 filters with stride 1 or 2 - the shapes of
 // MobileNet-style networks - run on dw3x3_dp4a_kernel (a thread walks along a band of rows, dp4a over byte-transposed
 // columns), other windows of 3x3, 5x5 and 7x7 on dwk_dp4a_kernel; other int8 shapes with C % 16 == 0 on dw_s8_vec16_kernel (16 channels per thread, 128-bit loads and
-// stores, a warp reads and writes contiguous runs of the NHWC tensor), small ones and int16 on dw_taps_kernel; everything else on dw_generic_kernel.
+// stores, a warp reads and writes contiguous runs of the NHWC tensor), int16 3x3 and 5x5 on dw_run_s16_kernel, small ones
+// and other int16 on dw_taps_kernel; everything else on dw_generic_kernel.
 #include "common.cuh"
 
 namespace espdl {
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(256) dw_generic_kernel(DwParams p)
 // after the other, each waited for, three taps over 24 pixels took as long as a launch more), and meet in dot products: groups of four taps of a channel in
 // dp4a, pairs in dp2a with the filter's high (signed) and low (unsigned) bytes - |sum| < 2^31 for 255 taps - where 64-bit multiply-adds a channel at a time
 // took twice as long.  us before / after: int8 24x32, 1x3 4.6 / 2.4, 20x20x128 3x3 at dilation 2 7.0 / 3.2; int16 154 of 12x11x192 5x5 146 / 65,
-// 64 of 56x56x96 3x3 421 / 178, 4 of 47x44x64 at stride 2 7.8 / 5.1.
+// 64 of 56x56x96 3x3 421 / 178, 4 of 47x44x64 at stride 2 7.8 / 5.1 (large int16 maps of these windows have since a kernel of their own below).
 template <typename T>
 struct TapWord; // four channels
 template <>
@@ -581,6 +582,131 @@ __global__ void __launch_bounds__(128) dw_taps_kernel(DwParams p)
         grid_dep_wait();
 }
 
+// int16's epilogue after the sums in 32-bit instructions, as the products' (gemm_tc.cu): 256 hi + lo + bias + 2^(s-1) as H * 65536 + L, H bounded so that the shift
+// leaves what saturates.  1 <= s <= 31, |bias| < 2^45.
+struct HalvesParam {
+    int h, l, limit, shift;
+};
+template <bool EVEN>
+__device__ __forceinline__ int requant_halves(int hi, int lo, const HalvesParam &c)
+{
+    int l = ((hi & 0xff) << 8) + (lo & 0xffff) + c.l;
+    int h = (hi >> 8) + (lo >> 16) + c.h + (l >> 16);
+    if (EVEN) { // a tie is rounded up only where that gives an even number
+        const uint32_t q = __funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+        l = (l & 0xffff) + (int)(q & 1u);
+        h += l >> 16;
+    }
+    h = max(min(h, c.limit), ~c.limit);
+    return (int)__funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+}
+__device__ __noinline__ int requant16_any(int hi, int lo, long long bias, int shift, int relu, int half_even)
+{
+    return requant16((long long)hi * 256 + lo, bias, max(-62, min(62, shift)), relu, half_even);
+}
+
+// int16, 3x3 and 5x5 at stride 1 and 2: four channels of four (two at stride 2) neighbouring outputs of a row a thread, so that a row's words, their pairs and the
+// filter's bytes serve all of them and the results leave through 32-bit instructions; dw_taps_kernel spends most of its instructions on addresses, pads nine taps
+// to sixteen and requantises in 64 bits.  Bound by the integer pipe (62 % busy, issue slots 59 %) with 4 to 6 warps a scheduler to cover its chains: constants
+// worked out behind the sums leave registers for them (116 of 75x75x192 3x3 403 -> 336 us), as six blocks an SM do for 5x5 (361 -> 343); a row's loads after
+// the row before's products cost 3x3 a tenth, two outputs a thread instead of four a sixth.
+// us dw_taps_kernel / here: 116 of 75x75x192 3x3 1141 / 334, 965 of 40x40x48 5x5 1170 / 343, 64 of 56x56x96 3x3 177 / 53, 313 of 30x33x96 at stride 2 73 / 32.
+template <int K, int S, bool EVEN>
+__global__ void __launch_bounds__(128, 6) dw_run_s16_kernel(DwParams p, int segs)
+{
+    constexpr int R = S == 1 ? 4 : 2, IN = (R - 1) * S + K;
+    grid_dep_launch();
+    grid_dep_wait();
+    const unsigned words = (unsigned)p.c / 4, item = blockIdx.x * blockDim.x + threadIdx.x;
+    if (item >= (unsigned)p.total)
+        return;
+    const unsigned run = item / words, line = run / (unsigned)segs, image = line / (unsigned)p.oh;
+    const int ch = 4 * (int)(item - run * words), ox = (int)(run - line * segs) * R, iy0 = (int)(line - image * p.oh) * S - p.pt, ix0 = ox * S - p.pl;
+    const int16_t *from = (const int16_t *)p.in + (long long)image * p.ih * p.iw * p.ips + (long long)ix0 * p.ips + ch;
+    const int16_t *w = (const int16_t *)p.w + ch;
+    int hi[R][4], lo[R][4];
+#pragma unroll
+    for (int j = 0; j < R; j++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) hi[j][c] = lo[j][c] = 0;
+#pragma unroll(K == 3 ? 3 : 1)
+    for (int ky = 0; ky < K; ky++, w += K * p.c) {
+        const int iy = iy0 + ky;
+        if ((unsigned)iy >= (unsigned)p.ih)
+            continue;
+        const int16_t *row = from + (long long)iy * p.iw * p.ips;
+        uint2 x[IN], f[K];
+#pragma unroll
+        for (int i = 0; i < IN; i++) {
+            x[i] = make_uint2(0u, 0u);
+            if ((unsigned)(ix0 + i) < (unsigned)p.iw)
+                x[i] = __ldg((const uint2 *)(row + (long long)i * p.ips));
+        }
+#pragma unroll
+        for (int i = 0; i < K; i++) f[i] = __ldg((const uint2 *)(w + i * p.c));
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+#pragma unroll
+            for (int g = 0; g < K; g += 2) {
+                const uint32_t f0 = c < 2 ? f[g].x : f[g].y, f1 = g + 1 < K ? (c < 2 ? f[g + 1 < K ? g + 1 : g].x : f[g + 1 < K ? g + 1 : g].y) : 0u;
+                // high bytes, low bytes; the last tap of a row meets the two channels of its word as they lie
+                const uint32_t b = g + 1 < K ? __byte_perm(f0, f1, c & 1 ? 0x6273 : 0x4051) : __byte_perm(f0, 0u, c & 1 ? 0x2434 : 0x4041);
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    const int i = j * S + g;
+                    const uint32_t x0 = c < 2 ? x[i].x : x[i].y;
+                    uint32_t a = x0;
+                    if (g + 1 < K)
+                        a = __byte_perm(x0, c < 2 ? x[i + 1 < IN ? i + 1 : i].x : x[i + 1 < IN ? i + 1 : i].y, c & 1 ? 0x7632 : 0x5410);
+                    asm("dp2a.lo.s32.s32 %0, %1, %2, %0;" : "+r"(hi[j][c]) : "r"(a), "r"(b));
+                    asm("dp2a.hi.s32.u32 %0, %1, %2, %0;" : "+r"(lo[j][c]) : "r"(a), "r"(b));
+                }
+            }
+        }
+    }
+    HalvesParam k[4];
+    bool fast = true;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const int sh = p.e_shift_base - (p.per_channel ? __ldg(p.ew + ch + c) : p.ew_scalar);
+        const long long b = p.bias ? __ldg((const long long *)p.bias + ch + c) : 0ll;
+        fast = fast && sh >= 1 && sh <= 31 && b < (1ll << 45) && b > -(1ll << 45);
+        const int fs = max(1, min(31, sh));
+        const long long add = b + (1ll << (fs - 1)) - (EVEN ? 1 : 0);
+        k[c] = {(int)(add >> 16), (int)(add & 0xffff), (int)((32768ll << max(0, fs - 16)) - 1), fs};
+    }
+    int16_t *to = (int16_t *)p.out + ((long long)line * p.ow + ox) * p.ops + ch;
+#pragma unroll
+    for (int j = 0; j < R; j++, to += p.ops) {
+        if (ox + j >= p.ow)
+            break;
+        int q[4];
+        if (fast) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) q[c] = requant_halves<EVEN>(hi[j][c], lo[j][c], k[c]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                q[c] = requant16_any(hi[j][c], lo[j][c], p.bias ? __ldg((const long long *)p.bias + ch + c) : 0ll,
+                                     p.e_shift_base - (p.per_channel ? __ldg(p.ew + ch + c) : p.ew_scalar), p.relu, EVEN);
+        }
+        uint2 o;
+        asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(o.x) : "r"(q[1]), "r"(q[0]));
+        asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(o.y) : "r"(q[3]), "r"(q[2]));
+        if (p.relu) {
+            asm("max.s16x2 %0, %0, %1;" : "+r"(o.x) : "r"(0));
+            asm("max.s16x2 %0, %0, %1;" : "+r"(o.y) : "r"(0));
+        }
+        *(uint2 *)to = o;
+    }
+}
+
+template <int K, int S>
+void launch_dw_run(const DwParams &p, int segs, unsigned blocks, cudaStream_t s)
+{
+    launch_overlapped(p.half_even ? dw_run_s16_kernel<K, S, true> : dw_run_s16_kernel<K, S, false>, dim3(blocks), dim3(128), 0, s, p, segs);
+}
+
 int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
 {
     DwParams p;
@@ -606,6 +732,12 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
         d.kh * d.kw <= 255 && pixels * (d.in_c / 4) < 1ll << 31;
     const bool k3 = words4 && d.kh == 3 && d.kw == 3 && d.dilation_h == 1 && d.dilation_w == 1 && d.stride_h == d.stride_w &&
         (d.stride_h == 1 || d.stride_h == 2);
+    // Threads of a few pixels' work each: fewer of them than this leave the chip idle.  us by runs / dw_taps_kernel: 20x20x96 5x5 5.2 / 4.6, 28x28x96 5.2 / 4.9,
+    // 40x40x96 5.2 / 7.6; 3x3 20x20x128 3.3 / 3.2, 28x28x96 3.2 / 3.4, 64 of 7x7x32 3.2 / 4.5; 28x28x128 at stride 2 2.9 / 3.1 (5x5 4.4 / 4.6).
+    const int run = d.stride_h == 1 ? 4 : 2, segs = (d.out_w + run - 1) / run; // of dw_run_s16_kernel
+    const long long run_items = (long long)d.n * d.out_h * segs * (d.in_c / 4);
+    const bool runs = taps && d.dtype == ESPDL_DTYPE_INT16 && (d.kh == 3 || d.kh == 5) && d.kh == d.kw && d.dilation_h == 1 && d.dilation_w == 1 &&
+        d.stride_h == d.stride_w && (d.stride_h == 1 || d.stride_h == 2) && run_items >= (d.kh == 5 && d.stride_h == 1 ? 40ll : 16ll) * num_sms();
     const long long filter_bytes = (d.kh * d.kw + 3ll) / 4 * 4 * d.in_c; // of dwk_dp4a_kernel
     if (k3 && ((long long)d.in_w + 10) * p.ips <= DW_ZERO_ROW_BYTES) {
         // a thread walks along a whole band of rows when the batch gives enough threads without cutting the band
@@ -633,6 +765,14 @@ int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s)
         p.total = pixels * (d.in_c / 4);
         const long long blocks = min((p.total + 255) / 256, max_blocks);
         launch_overlapped(d.kh == 3 ? dwk_dp4a_kernel<3> : (d.kh == 5 ? dwk_dp4a_kernel<5> : dwk_dp4a_kernel<7>), dim3((unsigned)blocks), dim3(256), (size_t)filter_bytes, s, p);
+    } else if (runs) {
+        p.chunks = 0;
+        p.total = run_items;
+        const unsigned blocks = (unsigned)((run_items + 127) / 128);
+        if (d.kh == 3)
+            d.stride_h == 1 ? launch_dw_run<3, 1>(p, segs, blocks, s) : launch_dw_run<3, 2>(p, segs, blocks, s);
+        else
+            d.stride_h == 1 ? launch_dw_run<5, 1>(p, segs, blocks, s) : launch_dw_run<5, 2>(p, segs, blocks, s);
     } else if (taps && (d.dtype == ESPDL_DTYPE_INT16 || !vec || pixels * (d.in_c / 4) <= 1024ll * num_sms())) {
         // int8 beyond: sixteen channels a thread, whose address and epilogue cost a quarter (64x56x56x96 at dilation 2 67 us, 154 here; 4x40x40x64 7.1 / 6.7)
         p.chunks = 0;

@@ -106,6 +106,22 @@ def test_depthwise_taps(kw, dtype, round_mode):
         np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
 
 
+# int16 by runs of a row: ragged runs, windows that leave the image, strides of rows, shifts and biases that need the general form, sums at the ends of the type
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("exps", [dict(e_out=-9, e_w=(-14, -11)), dict(e_out=-20, e_w=(-14, -6)), dict(e_out=-3, e_w=(-24, -11))], ids=["usual", "left", "beyond-31"])
+@pytest.mark.parametrize("kw", [dict(n=3, h=30, w=29, cin=20, k=3, pad=(1, 1, 1, 1)), dict(n=40, h=7, w=6, cin=64, k=3, pad=(3, 0, 2, 4), in_stride=72, out_stride=68),
+                                dict(n=7, h=21, w=22, cin=64, k=3, stride=2, pad=(0, 1, 1, 0)), dict(n=4, h=30, w=33, cin=28, k=5, pad=(2, 2, 2, 2)),
+                                dict(n=90, h=6, w=5, cin=64, k=5, pad=(5, 2, 0, 3)), dict(n=6, h=23, w=27, cin=32, k=5, stride=2, pad=(2, 1, 1, 2), out_stride=40)])
+def test_depthwise_runs_s16(kw, exps, round_mode):
+    kw = dict(kw, kh=kw["k"], kw=kw["k"])
+    del kw["k"]
+    case = cases.conv_case(seed=79, dtype=abi.DTYPE_INT16, depthwise=True, per_channel=True, round_mode=round_mode, e_in=-13, wide=True, **exps, **kw)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+    case["x"][...], case["w"][...] = -32768, -1
+    case["w"][..., 1::2] = -32768
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case), gpu_util.run_conv_oracle(case))
+
+
 @pytest.mark.parametrize("tma", [False, True], ids=["auto", "tma"])
 @pytest.mark.parametrize("kw", DW_SHAPES, ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "pad"))
 def test_depthwise_3x3_shapes(kw, tma, monkeypatch):
