@@ -608,9 +608,9 @@ __device__ __noinline__ int requant16_any(int hi, int lo, long long bias, int sh
 // int16, 3x3 and 5x5 at stride 1 and 2: four channels of four (two at stride 2) neighbouring outputs of a row a thread, so that a row's words, their pairs and the
 // filter's bytes serve all of them and the results leave through 32-bit instructions; dw_taps_kernel spends most of its instructions on addresses, pads nine taps
 // to sixteen and requantises in 64 bits.  Bound by the integer pipe (62 % busy, issue slots 59 %) with 4 to 6 warps a scheduler to cover its chains: constants
-// worked out behind the sums leave registers for them (116 of 75x75x192 3x3 403 -> 336 us), as six blocks an SM do for 5x5 (361 -> 343); a row's loads after
+// worked out behind the sums leave registers for them (116 of 75x75x192 3x3 403 -> 336 us), as six blocks an SM do for 5x5 (361 -> 343), one wait for the launch before without the form that waits later (334 -> 306); a row's loads after
 // the row before's products cost 3x3 a tenth, two outputs a thread instead of four a sixth.
-// us dw_taps_kernel / here: 116 of 75x75x192 3x3 1141 / 334, 965 of 40x40x48 5x5 1170 / 343, 64 of 56x56x96 3x3 177 / 53, 313 of 30x33x96 at stride 2 73 / 32.
+// us dw_taps_kernel / here: 116 of 75x75x192 3x3 1141 / 306, 965 of 40x40x48 5x5 1170 / 323, 64 of 56x56x96 3x3 177 / 49, 313 of 30x33x96 at stride 2 73 / 29.
 template <int K, int S, bool EVEN>
 __global__ void __launch_bounds__(128, 6) dw_run_s16_kernel(DwParams p, int segs)
 {
