@@ -6,6 +6,8 @@
 //   Concat             esp-dl/dl/module/include/dl_module_concat.hpp:87-107
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace espdl {
 
 struct PoolParams {
@@ -182,17 +184,18 @@ __global__ void __launch_bounds__(256) maxpool_s8_walk_kernel(PoolParams p, int 
     }
 }
 
-// The same walk for what the kernel above does not take: int16 with whole 16-byte units (V = 8, packed maxima as they are), and single
-// elements of either type (V = 1) where channels do not fill units - a warp's lanes are then consecutive elements.
+// The same walk for what the kernel above does not take: int16 with whole 16-byte units (V = 8, packed maxima as they are), words of four or
+// two elements (int8: four, taken apart into 16-bit lanes) and single elements of either type (V = 1) - a warp's lanes are then consecutive
+// elements.  Bound by the issue of loads and maxima, so fewer and wider ones pay: 60000 pixels of 100 channels 5x5 38 -> 16 us.
 template <int K, typename T, int V>
 __global__ void __launch_bounds__(256) maxpool_walk_kernel(PoolParams p, int segments, int early)
 {
     if (early)
         grid_dep_launch();
     grid_dep_wait();
-    constexpr int WORDS = V > 1 ? 4 : 1;
+    constexpr int WORDS = V > 1 ? V / 2 : 1;
     struct Unit {
-        uint32_t w[WORDS]; // V > 1: two int16 a word; V = 1: the element, sign extended
+        uint32_t w[WORDS]; // V > 1: two int16 a word, or the bytes as their high halves; V = 1: the element, sign extended
     };
     auto max_unit = [](Unit &a, const Unit &b) {
 #pragma unroll
@@ -228,11 +231,21 @@ __global__ void __launch_bounds__(256) maxpool_walk_kernel(PoolParams p, int seg
                     const int x = ox - p.pl + kx;
                     v[kx] = lowest;
                     if (row_in && x >= 0 && x < p.iw) {
-                        if constexpr (V > 1) {
-                            const uint4 t = __ldg((const uint4 *)(row + (long long)x * p.c));
+                        const T *at = row + (long long)x * p.c;
+                        if constexpr (sizeof(T) == 1 && V > 1) {
+                            static_assert(V == 4);
+                            const uint32_t t = __ldg((const uint32_t *)at);
+                            v[kx].w[0] = __byte_perm(t, 0u, 0x1404), v[kx].w[1] = __byte_perm(t, 0u, 0x3424);
+                        } else if constexpr (V == 2) {
+                            v[kx].w[0] = __ldg((const uint32_t *)at);
+                        } else if constexpr (V == 4) {
+                            const uint2 t = __ldg((const uint2 *)at);
+                            v[kx].w[0] = t.x, v[kx].w[1] = t.y;
+                        } else if constexpr (V > 1) {
+                            const uint4 t = __ldg((const uint4 *)at);
                             v[kx].w[0] = t.x, v[kx].w[1] = t.y, v[kx].w[2] = t.z, v[kx].w[3] = t.w;
                         } else {
-                            v[kx].w[0] = (uint32_t)(int)__ldg(row + (long long)x * p.c);
+                            v[kx].w[0] = (uint32_t)(int)__ldg(at);
                         }
                     }
                 }
@@ -244,10 +257,17 @@ __global__ void __launch_bounds__(256) maxpool_walk_kernel(PoolParams p, int seg
                     Unit m = ring[0];
 #pragma unroll
                     for (int d = 1; d < K; d++) max_unit(m, ring[d]);
-                    if constexpr (V > 1)
-                        *(uint4 *)(out + (long long)oy * p.ow * p.c) = make_uint4(m.w[0], m.w[1], m.w[2], m.w[3]);
+                    T *to = out + (long long)oy * p.ow * p.c;
+                    if constexpr (sizeof(T) == 1 && V == 4)
+                        *(uint32_t *)to = __byte_perm(m.w[0], m.w[1], 0x7531);
+                    else if constexpr (V == 2)
+                        *(uint32_t *)to = m.w[0];
+                    else if constexpr (V == 4)
+                        *(uint2 *)to = make_uint2(m.w[0], m.w[1]);
+                    else if constexpr (V > 1)
+                        *(uint4 *)to = make_uint4(m.w[0], m.w[1], m.w[2], m.w[3]);
                     else
-                        out[(long long)oy * p.ow * p.c] = (T)(int)m.w[0];
+                        *to = (T)(int)m.w[0];
                 }
             }
         }
@@ -642,15 +662,24 @@ extern "C" int espdl_b200_pool(const espdl_pool_desc *d, void *stream)
         return check_launch("max pool");
     }
     if (d->op == ESPDL_POOL_MAX && p.sh == 1 && p.sw == 1 && p.kh == p.kw && (p.kh == 3 || p.kh == 5) && !getenv("ESPDL_B200_NO_POOL_WALK")) {
-        // int16 units of 16 bytes, else single elements (5x5 over 591164 pixels of 127 channels: 2138 us with a thread per output)
-        const bool units = p.is16 && whole_units;
-        const long long columns = (long long)p.n * p.ow * (units ? p.c / 8 : p.c);
+        // int16 units of 16 bytes, else four or two elements where they divide the channels and the addresses, else one (5x5 over 591164 pixels of 127 channels:
+        // 2138 us with a thread per output).  int8 takes four where that leaves enough threads (6400 pixels of 4 channels 8.4 us by one, 8.6 by four; 60000 of
+        // 100 37 / 16) and never two, whose bytes cost more to take apart than they save (24000 of 22 10 / 16); int16 60000 of 100 38 / 16, 100000 of 370 by two 170 / 96.
+        const uintptr_t low = (uintptr_t)d->input | (uintptr_t)d->output;
+        const int v = !p.is16 ? (p.c % 4 == 0 && low % 4 == 0 && p.total >= 8192ll * num_sms() ? 4 : 1)
+                              : (whole_units ? 8 : (p.c % 4 == 0 && low % 8 == 0 ? 4 : (p.c % 2 == 0 && low % 4 == 0 ? 2 : 1)));
+        const long long columns = (long long)p.n * p.ow * (p.c / v);
         int segments = 1;
         while (columns * segments < (long long)num_sms() * 2048 && p.oh / (segments * 2) >= 2 * p.kh) segments *= 2;
         const unsigned grid = (unsigned)min((columns * segments + 255) / 256, (long long)num_sms() * 32);
-        const auto k3 = units ? maxpool_walk_kernel<3, int16_t, 8> : (p.is16 ? maxpool_walk_kernel<3, int16_t, 1> : maxpool_walk_kernel<3, int8_t, 1>);
-        const auto k5 = units ? maxpool_walk_kernel<5, int16_t, 8> : (p.is16 ? maxpool_walk_kernel<5, int16_t, 1> : maxpool_walk_kernel<5, int8_t, 1>);
-        launch_mover(p.kh == 3 ? k3 : k5, dim3(grid), dim3(256), 0, (cudaStream_t)stream, p, segments);
+        const auto pick = [&](auto k) {
+            constexpr int K = decltype(k)::value;
+            if (p.is16)
+                return v == 8 ? maxpool_walk_kernel<K, int16_t, 8> : v == 4 ? maxpool_walk_kernel<K, int16_t, 4> : v == 2 ? maxpool_walk_kernel<K, int16_t, 2> : maxpool_walk_kernel<K, int16_t, 1>;
+            return v == 4 ? maxpool_walk_kernel<K, int8_t, 4> : maxpool_walk_kernel<K, int8_t, 1>;
+        };
+        const auto kernel = p.kh == 3 ? pick(std::integral_constant<int, 3>{}) : pick(std::integral_constant<int, 5>{});
+        launch_mover(kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, p, segments);
         count_launch();
         return check_launch("max pool walk");
     }

@@ -69,6 +69,16 @@ def test_max_pool_walk(kw, dtype):
     pool_matches(cases.pool_case(abi.POOL_MAX, seed=kw["c"], dtype=dtype, stride=1, **kw))
 
 
+# two and four elements a thread, segments of a column, pads wider than the window needs on one side
+@pytest.mark.parametrize("dtype", BOTH)
+@pytest.mark.parametrize("kw", [dict(n=2, h=23, w=9, c=18, kh=5, kw=5, pad=(2, 2, 2, 2)), dict(n=1, h=64, w=7, c=20, kh=3, kw=3, pad=(1, 1, 1, 1)),
+                                dict(n=3, h=6, w=5, c=2, kh=5, kw=5, pad=(4, 0, 1, 3)), dict(n=2, h=41, w=6, c=44, kh=5, kw=5, pad=(0, 0, 0, 0)),
+                                dict(n=1, h=3, w=2, c=4, kh=3, kw=3, pad=(1, 1, 1, 1)), dict(n=60, h=40, w=40, c=6, kh=3, kw=3, pad=(2, 1, 0, 2)),
+                                dict(n=31, h=41, w=40, c=28, kh=5, kw=5, pad=(2, 2, 2, 2)), dict(n=24, h=33, w=41, c=44, kh=3, kw=3, pad=(0, 2, 2, 0))])
+def test_max_pool_walk_words(kw, dtype):
+    pool_matches(cases.pool_case(abi.POOL_MAX, seed=kw["c"], dtype=dtype, stride=1, **kw))
+
+
 def pool_matches(case):
     want = case["out"].copy()
     assert checkers.oracle().oracle_pool(cases.pool_desc(dict(case, out=want))) == 0
