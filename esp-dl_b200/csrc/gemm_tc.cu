@@ -81,6 +81,7 @@ constexpr int MAX_ACC = 8;
 
 struct TcParams {
     int early; // bias, exponents and table are constants of the model: read ahead of the previous kernel's end
+    int filter_early; // so is the filter: not one that was packed, which the launch directly before writes
     int M, N, K;    // rows per matrix, output channels, reduction length
     int batch;      // independent matrices (1 unless every image has its own filter)
     int block_n, n_tiles, m_tiles;
@@ -335,8 +336,8 @@ __device__ __forceinline__ bool produce_resident(const TcParams &p, const CUtens
     const int a_bytes = BLOCK_M * p.swz, b_bytes = p.block_n * p.swz;
     const ResidentShare share = resident_share(p);
     const int first = share.first, across = share.across, member = share.member, members = share.members;
-    if (!p.early)
-        grid_dep_wait(); // outside a model's plan a caller may just have written the filter
+    if (!p.filter_early)
+        grid_dep_wait(); // outside a model's plan a caller may just have written the filter, and a packed one is what the launch before writes
     const uint32_t fbar = smem_u32(filter_bar), filter = smem + (uint32_t)(p.stages * a_bytes);
     mbar_arrive_expect_tx(fbar, (uint32_t)(across * p.k_blocks * b_bytes));
     for (int j = 0; j < across; j++)
@@ -1691,6 +1692,7 @@ int launch_tc(const espdl_conv_desc &d, TcParams &p, const PackedOperands *o, cu
     const bool i16 = d.dtype == ESPDL_DTYPE_INT16;
     const int ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
     p.early = in_model_scope();
+    p.filter_early = p.early && !o;
     p.out = d.output;
     p.ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     p.row_sum = o ? o->row_sum : nullptr;

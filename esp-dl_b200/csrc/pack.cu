@@ -59,7 +59,7 @@ __device__ __forceinline__ int split16(const uint4 a, const uint4 b, uint4 &hi, 
 template <typename T, bool WINDOW>
 __global__ void __launch_bounds__(256) pack_kernel(PackParams p)
 {
-    grid_dep_launch(); // what this writes is read by the tile kernel's loads only, which wait for it
+    grid_dep_launch(); // what this writes is read by the tile kernel's loads only, all of which wait for it (TcParams::filter_early)
     grid_dep_wait();
     const int lane = threadIdx.x & 31, sub = lane % p.lanes, per_warp = 32 / p.lanes;
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);

@@ -41,6 +41,33 @@ def test_packed_conv(i, dtype, round_mode):
     assert want.std() > 0
 
 
+def test_packed_convs_of_a_plan_that_share_scratch():
+    """A tile kernel with a resident filter (two row tiles an SM and more) starts beside the packing that writes this filter: inside a model's scope, where other
+    filters are read ahead, and with another layer's filter still in the scratch."""
+    import ctypes as C
+    layers = [cases.conv_case(seed=i, n=1, h=200, w=200, per_channel=True, **kw) for i, kw in enumerate((dict(cin=24, cout=64), dict(cin=40, cout=48), dict(cin=3, cout=64, kh=7, kw=7)))]
+    want = [gpu_util.run_conv_oracle(case) for case in layers]
+    with gpu_util.DeviceBuffers() as dev:
+        descs, scratch_bytes = [], 0
+        for case in layers:
+            names = dict(input="x", filter="w", bias="b", filter_exponents="ew", output="out")
+            descs.append(cases.conv_desc(case, {k: dev.upload(case[v]) for k, v in names.items()}))
+            need = C.c_size_t(0)
+            abi.check(dev.lib.espdl_b200_conv2d_workspace_bytes(C.byref(descs[-1]), C.byref(need)), "workspace_bytes")
+            assert need.value >= 40000 * case["kh"] * case["kw"] * case["in_c"]  # the packed path
+            scratch_bytes = max(scratch_bytes, need.value)
+        scratch = dev.alloc(scratch_bytes)
+        for _ in range(10):
+            dev.lib.espdl_b200_model_scope(1)
+            try:
+                for d in descs:
+                    abi.check(dev.lib.espdl_b200_conv2d_ws(C.byref(d), scratch, scratch_bytes, None), "conv2d_ws")
+            finally:
+                dev.lib.espdl_b200_model_scope(0)
+            for d, w in zip(descs, want):
+                np.testing.assert_array_equal(dev.download(d.output, w), w)
+
+
 @pytest.mark.parametrize("m,k,n", [(129, 16, 16), (300, 16384, 8), (128, 4096, 129), (1000, 272, 260)])
 @pytest.mark.parametrize("sign", [-1, 1, 0])
 def test_int16_products_at_the_ends_of_the_type(m, k, n, sign):
