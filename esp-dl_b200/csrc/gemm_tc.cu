@@ -1557,8 +1557,8 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
     p.resident = p.in_turn = 0;
     if (!i16)
         plan_resident(p);
-    if (p.resident) {
-        p.frag = p.N % 16 == 0;
+    if (p.resident) { // (rows that leave by warps have no fragment form with a table)
+        p.frag = p.N % 16 == 0 && (p.in_turn || !d.lut);
         return true;
     }
     if (!i16 && !p.one_tile && p.out_pw && !p.out_rows && p.k_blocks > 2 && stages < 4) {

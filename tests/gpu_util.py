@@ -55,18 +55,22 @@ class DeviceBuffers:
         return out
 
 
-def run_conv_gpu(case, kernel=abi.KERNEL_AUTO, expect=abi.OK):
+def run_conv_gpu(case, kernel=abi.KERNEL_AUTO, expect=abi.OK, out_offset=0):
+    """out_offset: bytes from a 16-byte boundary to the output, what lies before it is checked to be left alone."""
     import cases
     with DeviceBuffers() as dev:
         ptrs = dict(input=dev.upload(case["x"]), filter=dev.upload(case["w"]), bias=dev.upload(case["b"]),
                     filter_exponents=dev.upload(case["ew"]), lut=dev.upload(case["lut"]), residual=dev.upload(case.get("res")),
-                    output=dev.upload(np.full_like(case["out"], 0x55)))
+                    output=dev.upload(np.full(out_offset + case["out"].nbytes, 0x55, dtype=np.uint8) if out_offset else np.full_like(case["out"], 0x55)))
+        ptrs["output"] += out_offset
         d = cases.conv_desc(dict(case, kernel=kernel), ptrs)
         st = dev.lib.espdl_b200_conv2d(C.byref(d), None)
         if expect != abi.OK:
             assert st == expect
             return None
         abi.check(st, "espdl_b200_conv2d")
+        if out_offset:
+            assert (dev.download(ptrs["output"] - out_offset, np.empty(out_offset, dtype=np.uint8)) == 0x55).all()
         return dev.download(ptrs["output"], case["out"])
 
 

@@ -63,6 +63,15 @@ def test_gemm_s8_resident_filter(shape, round_mode):
     assert want.std() > 0
 
 
+# Whole groups of 16 columns in rows that no TMA store can address: with a resident filter, with tiles that bring theirs along, in one tile a CTA
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("out_stride,out_offset", [(100, 0), (97, 0), (96, 4), (112, 5)])
+@pytest.mark.parametrize("m", [37900, 20000, 129])
+def test_whole_columns_in_unaligned_rows_with_a_table(m, out_stride, out_offset, round_mode):
+    case = cases.gemm_case(seed=m + out_stride, m=m, k=64, n_out=96, per_channel=True, lut=True, round_mode=round_mode, out_stride=out_stride, e_in=-7, e_out=-5, e_w=(-9, -6))
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05, out_offset=out_offset), gpu_util.run_conv_oracle(case))
+
+
 @pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
 @pytest.mark.parametrize("act", [abi.ACT_LINEAR, abi.ACT_RELU])
 def test_gemm_s8_tc_epilogue_variants(act, round_mode):
