@@ -205,12 +205,14 @@ __device__ __noinline__ void epilogue_direct_tile(const TcParams &p, const FastP
 }
 
 // The general epilogue of a tile whose columns are channels in the order frag_channel (a channel outside the fast form, or tables of channels): 16 columns
-// at a time, put back into order.  Rows are 16-byte aligned, columns whole groups of 16.
+// at a time, put back into order, columns whole groups of 16.  Residual rows are 16-byte aligned, rows of results begin anywhere (those that leave by warps).
 __device__ __noinline__ void epilogue_frag_general(const TcParams &p, uint32_t t0, long long m, int n0, bool row_ok, int parts, int part)
 {
     const int ncols = min(p.block_n, p.N - n0);
     int8_t *orow = (int8_t *)p.out + m * p.ops + n0;
     const int8_t *rrow = p.res + m * p.rps + n0;
+    const uintptr_t amix = (uintptr_t)p.ops | (uintptr_t)p.out | (uintptr_t)n0 | 16u; // see epilogue_direct
+    const int out_align = (int)(amix & (~amix + 1));
 #pragma unroll 1
     for (int c0 = 16 * part; c0 < ncols; c0 += 16 * parts) {
         int32_t u[16], v[16];
@@ -233,7 +235,7 @@ __device__ __noinline__ void epilogue_frag_general(const TcParams &p, uint32_t t
                 pk[q] = w;
             }
         }
-        *(uint4 *)(orow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        store_bytes(orow + c0, pk, 16, out_align);
     }
 }
 

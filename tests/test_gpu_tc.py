@@ -72,6 +72,20 @@ def test_whole_columns_in_unaligned_rows_with_a_table(m, out_stride, out_offset,
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05, out_offset=out_offset), gpu_util.run_conv_oracle(case))
 
 
+# The same rows from fragments: all channels in the fast form, shifts outside it, a table of each channel
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("opts", [{}, dict(e_out=-14), dict(lut="channels"), dict(res=True), dict(e_out=-14, res=True)], ids=lambda o: "_".join(o) or "fast")
+@pytest.mark.parametrize("n,out_stride,out_offset", [(96, 100, 0), (96, 97, 0), (272, 280, 0), (96, 96, 4)])
+@pytest.mark.parametrize("m", [37900, 20000, 129])
+def test_whole_columns_in_unaligned_rows(m, n, out_stride, out_offset, opts, round_mode):
+    opts = dict(dict(e_out=-5), **opts)
+    res = opts.pop("res", False)
+    case = cases.gemm_case(seed=m + out_stride, m=m, k=64, n_out=n, per_channel=True, round_mode=round_mode, out_stride=out_stride, e_in=-7, e_w=(-9, -6), **opts)
+    if res:  # rows of its own, whose columns are whole units
+        case["res"] = np.random.default_rng(n).integers(-128, 128, size=(1, 1, m, n), dtype=np.int8)
+    np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05, out_offset=out_offset), gpu_util.run_conv_oracle(case))
+
+
 @pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
 @pytest.mark.parametrize("act", [abi.ACT_LINEAR, abi.ACT_RELU])
 def test_gemm_s8_tc_epilogue_variants(act, round_mode):
