@@ -509,7 +509,7 @@ __device__ __forceinline__ bool epilogue_resident(const TcParams &p, const CUten
         const int n = epi_col[acc] * block_n + part * PIECE, cols = min(PIECE, N - n);
         fence_after();
         if (elect_one())
-            bulk_wait_read_but_one(); // the store out of this buffer has read it, the other buffer's may be under way
+            bulk_wait_read_but_one(); // the store out of this buffer has read it, the other buffer's (the last piece's) may be under way
         __syncwarp();
         TC_LAP(w_store);
         const uint32_t t0 = tmem + (uint32_t)(acc * block_n + part * PIECE), fp = fp_base + (uint32_t)n * 8u;
@@ -534,9 +534,10 @@ __device__ __forceinline__ bool epilogue_resident(const TcParams &p, const CUten
         }
         fence_async_smem();
         __syncwarp();
-        if (cols > 0 && row * BLOCK_M < M && elect_one()) { // rows >= M and columns >= N are clipped
-            tma_store_3d(&map_out, buf + (uint32_t)(lane_group * 32 * PIECE), n, row * BLOCK_M + lane_group * 32, 0);
-            bulk_commit();
+        if (elect_one()) {
+            if (cols > 0 && row * BLOCK_M < M) // rows >= M and columns >= N are clipped
+                tma_store_3d(&map_out, buf + (uint32_t)(lane_group * 32 * PIECE), n, row * BLOCK_M + lane_group * 32, 0);
+            bulk_commit(); // an empty group for a piece without columns, too: the wait above counts pieces
         }
         __syncwarp();
         // The other accumulator and buffer.  Pieces of a tile of 65 to 127 columns change hands, they are not two of 64.

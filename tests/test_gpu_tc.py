@@ -38,6 +38,7 @@ def test_gemm_s8_tc(shape):
 RESIDENT_SHAPES = [
     (38000, 64, 128, {}), (38000, 64, 80, {}), (37900, 96, 48, {}), (37900, 32, 16, {}),  # whole pieces, ragged ones, eight accumulators, one piece a tile
     (37900, 128, 272, {}), (38000, 48, 192, {}),                                          # several column tiles, the last of 16 / 64 columns
+    (120000, 16, 192, {}), (90000, 32, 320, {}), (60000, 48, 576, {}),                    # every second piece of a column tile without columns, many tiles a CTA
     (37900, 1040, 32, {}),                                                               # more blocks of K than stages
     (13000, 320, 272, {}),                                                               # groups of CTAs, a column tile each
     (76000, 16, 32, {}), (80000, 32, 144, {}),                                           # tiles handed out by the counter
