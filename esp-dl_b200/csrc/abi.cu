@@ -561,8 +561,7 @@ static bool runs_mma(const espdl_conv_desc &d)
     return conv2d_mma_estimate_us(d) < min(other, 8.f);
 }
 
-// Do results lie where inputs do?  Channels side by side in the same rows don't.
-static bool overlaps(const espdl_conv_desc &d)
+bool espdl::overlaps(const espdl_conv_desc &d)
 {
     const long long es = d.dtype == ESPDL_DTYPE_INT16 ? 2 : 1, ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c, ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     const long long in_bytes = (((long long)d.n * d.in_h * d.in_w - 1) * ips + d.in_c) * es, out_bytes = (((long long)d.n * d.out_h * d.out_w - 1) * ops + d.out_c) * es;

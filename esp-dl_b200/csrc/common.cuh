@@ -84,6 +84,7 @@ float conv2d_narrow_estimate_us(const espdl_conv_desc &d);
 float conv2d_simt_estimate_us(const espdl_conv_desc &d); // about what it takes, for the choice against packed operands
 int conv2d_depthwise(const espdl_conv_desc &d, cudaStream_t s);
 bool conv2d_tc_supported(const espdl_conv_desc &d);
+bool overlaps(const espdl_conv_desc &d); // do results lie where inputs do?  Channels side by side in the same rows don't
 size_t conv2d_tc_workspace_bytes(const espdl_conv_desc &d);
 int conv2d_tc(const espdl_conv_desc &d, void *workspace, size_t workspace_bytes, cudaStream_t s, const long long *peer_delta = nullptr,
               int n_peer = 0, int *row_sums = nullptr); // peer_delta: byte distances to copies of the output on other GPUs that receive every row as well

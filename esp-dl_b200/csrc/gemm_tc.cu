@@ -1421,8 +1421,9 @@ size_t aux_bytes(const TcParams &p, bool i16 = false)
 // tiles out where they do not all fit - and every row tile serves all of them.  Tiles are 128 columns wide: two accumulators for each of two sets of
 // epilogue warps, so that a warp finds the next tile's sums ready (64 columns and fewer: for each of four).  us before / after (floor: bytes): 401408 x 128 ->
 // 768 93 / 73 (55), 802816 x 96 -> 96 56 / 28 (24), 200704 x 64 -> 384 27.4 / 23.5 (14), 50176 x 320 -> 1280 46 / 30 (12), 65536 x 384 -> 384 24 / 15 (8).
-// From two row tiles a CTA on: below, the filter is not used often enough (8192 x 256 -> 1024: 7.1 us, 8.5 resident).
-void plan_resident(TcParams &p)
+// From two row tiles a CTA on: below, the filter is not used often enough (8192 x 256 -> 1024: 7.1 us, 8.5 resident).  Results that overwrite the inputs
+// stay with one column tile (up to 256 columns without a resident filter), which has all of a row before any of it is written: here a row tile's columns may be two CTAs'.
+void plan_resident(const espdl_conv_desc &d, TcParams &p)
 {
     p.resident = p.in_turn = 0, p.n_groups = 1;
     if (p.one_tile || !p.out_pw || p.batch != 1)
@@ -1433,6 +1434,8 @@ void plan_resident(TcParams &p)
         q.in_turn = 1, q.acc_stages = q.block_n > 64 ? 4 : 8, q.tmem_cols = 512;
         q.out_pw = 64, q.out_mask = 3;
     }
+    if (q.n_tiles > p.n_tiles && p.n_tiles == 1 && overlaps(d))
+        return;
     const size_t a_stage = (size_t)BLOCK_M * q.swz, b_tile = (size_t)q.block_n * q.k_blocks * q.swz;
     const size_t room = SMEM_BUDGET_DEEP - aux_bytes(q) - 4 * ((size_t)((BLOCK_M * q.out_pw + 1023) & ~1023) << q.in_turn) - 2048;
     // one column tile: a row tile's stages are free as soon as they are multiplied; several: two row tiles
@@ -1559,7 +1562,7 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
         stages = (int)((SMEM_BUDGET_DEEP - aux_bytes(p) - out_bytes - 1024) / stage_bytes);
     p.resident = p.in_turn = 0;
     if (!i16)
-        plan_resident(p);
+        plan_resident(d, p);
     if (p.resident) { // (rows that leave by warps have no fragment form with a table)
         p.frag = p.N % 16 == 0 && (p.in_turn || !d.lut);
         return true;

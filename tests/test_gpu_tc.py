@@ -87,6 +87,20 @@ def test_whole_columns_in_unaligned_rows(m, n, out_stride, out_offset, opts, rou
     np.testing.assert_array_equal(gpu_util.run_conv_gpu(case, kernel=abi.KERNEL_TCGEN05, out_offset=out_offset), gpu_util.run_conv_oracle(case))
 
 
+@pytest.mark.parametrize("m,n", [(80000, 256), (80000, 144), (38000, 192), (38000, 128)])
+def test_products_that_overwrite_their_inputs(m, n):
+    """Up to 256 columns a tile has a whole row before any of it is written."""
+    case = cases.gemm_case(seed=n, m=m, k=n, n_out=n, per_channel=True, e_in=-7, e_out=-5, e_w=(-9, -6))
+    want = gpu_util.run_conv_oracle(case)
+    with gpu_util.DeviceBuffers() as dev:
+        ptrs = {k: dev.upload(case[v]) for k, v in dict(input="x", filter="w", bias="b", filter_exponents="ew").items()}
+        for _ in range(5):
+            abi.check(dev.lib.espdl_b200_upload(ptrs["input"], case["x"].ctypes.data, case["x"].nbytes, None), "upload")
+            d = cases.conv_desc(dict(case, kernel=abi.KERNEL_TCGEN05), dict(ptrs, output=ptrs["input"]))
+            abi.check(dev.lib.espdl_b200_conv2d(C.byref(d), None), "conv2d")
+            np.testing.assert_array_equal(dev.download(ptrs["input"], case["out"]), want)
+
+
 @pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
 @pytest.mark.parametrize("act", [abi.ACT_LINEAR, abi.ACT_RELU])
 def test_gemm_s8_tc_epilogue_variants(act, round_mode):
