@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
     // the scalar code (so the rounding is the reference's) and then runs as a table lookup like LUT itself.
     constexpr bool TABULATED = sizeof(T) == 1 && (OP == ESPDL_ELT_REQUANTIZE || OP == ESPDL_ELT_CLIP || OP == ESPDL_ELT_RELU);
     constexpr bool LOOKUP = sizeof(T) == 1 && (OP == ESPDL_ELT_LUT || TABULATED);
-    // In a small network a launch is one trip through memory: where the first unit lies and, inside a model's plan, whose tables no launch
-    // writes, the table are found out before the wait for the previous kernel, and the unit is on its way while the block meets over the table.
+    // In a small network a launch is one trip through memory: where the first unit lies and what the operator makes of a byte are found out before the wait for
+    // the previous kernel, and the unit is on its way while the block meets over the table (LUT's own, an operand like any other, is read behind the wait).
     auto offsets = [&](long long v, long long &io, long long &ia, long long &ib) {
         if (BCAST) {
             const long long row = v < 0x7fffffffll ? (long long)((unsigned)v / (unsigned)p.vpr) : v / p.vpr, col = v - row * p.vpr;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
     if (sizeof(T) == 1 && first < nvec)
         offsets(first, io, ia, ib);
     if (LOOKUP) {
-        if (!early && OP == ESPDL_ELT_LUT)
+        if (OP == ESPDL_ELT_LUT)
             grid_dep_wait();
         for (int i = threadIdx.x; i < 256; i += blockDim.x) {
             if (OP == ESPDL_ELT_LUT) {
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
             }
         }
     }
-    if (!LOOKUP || early || OP != ESPDL_ELT_LUT)
+    if (!LOOKUP || OP != ESPDL_ELT_LUT)
         grid_dep_wait();
     auto one = [&](int a, int b) -> int {
         if (LOOKUP)

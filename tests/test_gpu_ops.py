@@ -260,6 +260,32 @@ def test_binary(op, dtype, shapes, round_mode):
     np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("shape", [(1, 4, 5, 16), (64, 40, 40, 96)])
+def test_lut_whose_table_the_launch_before_writes(shape):
+    """Inside a model's scope filters, biases and exponents are constants, the second operand of a lookup is none of these."""
+    x = np.random.default_rng(5).integers(-128, 128, size=shape, dtype=np.int8)
+    tables = [np.random.default_rng(i).integers(-128, 128, size=256, dtype=np.int8) for i in range(4)]
+    with gpu_util.DeviceBuffers() as dev:
+        sources = [dev.upload(t) for t in tables]
+        table, xd, outs = dev.alloc(256), dev.upload(x), [dev.alloc(x.nbytes) for _ in range(8)]
+        dev.lib.espdl_b200_model_scope(1)
+        try:
+            for i, out in enumerate(outs):
+                copy = cases.copy_desc(sources[i % 4], table, 1, (256,), (1,), (1,))
+                abi.check(dev.lib.espdl_b200_copy(C.byref(copy), None), "copy")
+                d = abi.EltwiseDesc()
+                d.op, d.in_dtype, d.out_dtype, d.ndim = abi.ELT_LUT, abi.DTYPE_INT8, abi.DTYPE_INT8, 4
+                for k, v in enumerate(shape):
+                    d.out_shape[k] = d.in0_shape[k] = v
+                    d.in1_shape[k] = 1
+                d.input0, d.input1, d.output = xd, table, out
+                abi.check(dev.lib.espdl_b200_eltwise(C.byref(d), None), "eltwise")
+        finally:
+            dev.lib.espdl_b200_model_scope(0)
+        for i, out in enumerate(outs):
+            np.testing.assert_array_equal(dev.download(out, x), tables[i % 4][x.view(np.uint8) ^ 0x80])
+
+
 @pytest.mark.parametrize("inplace", ["input0", "input1"])
 def test_add_in_place(inplace):
     """The planner runs Add in place: the output may alias either input."""
