@@ -196,6 +196,45 @@ __global__ void __launch_bounds__(256) elt_generic_kernel(EltParams p, int early
     }
 }
 
+// One-operand int8 -> int8 operators are functions of the input byte: every block tabulates the operator once with
+// the scalar code (so the rounding is the reference's) and then runs as a table lookup like LUT itself.
+template <typename T>
+__device__ constexpr bool elt_lookup(int op)
+{
+    return sizeof(T) == 1 && (op == ESPDL_ELT_LUT || op == ESPDL_ELT_REQUANTIZE || op == ESPDL_ELT_CLIP || op == ESPDL_ELT_RELU);
+}
+
+template <int OP>
+__device__ __forceinline__ void fill_table(const EltParams &p, int8_t *table)
+{
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+        if (OP == ESPDL_ELT_LUT) {
+            table[i] = ((const int8_t *)p.b)[i];
+        } else {
+            EltParams q2 = p;
+            q2.op = OP;
+            table[i] = (int8_t)sat8((int)max(-1000000ll, min(1000000ll, elt_int(q2, (int)(int8_t)(uint8_t)(i ^ 0x80), 0))));
+        }
+    }
+}
+
+template <int OP, typename T>
+__device__ __forceinline__ int elt_one(const EltParams &p, const int8_t *table, int a, int b)
+{
+    if (elt_lookup<T>(OP))
+        return table[(uint8_t)a ^ 0x80u];
+    if (OP == ESPDL_ELT_LUT) // int16
+        return ((const int16_t *)p.b)[lut16_index(p, a)];
+    long long v = OP == ESPDL_ELT_ADD ? a + b : (OP == ESPDL_ELT_SUB ? a - b : 0);
+    if (OP != ESPDL_ELT_ADD && OP != ESPDL_ELT_SUB) {
+        EltParams q2 = p;
+        q2.op = OP;
+        v = elt_int(q2, a, b);
+    }
+    const int lo = -(1 << (8 * (int)sizeof(T) - 1));
+    return (int)max((long long)lo, min((long long)(-lo - 1), v));
+}
+
 // 16 bytes per thread: int8 or int16 in and out, operands of one shape or (BCAST) the second one repeated over the rows of an image - a
 // gate [n][1][1][c] over a map [n][h][w][c].  Flat tensors of any length: what does not fill a unit is done by single threads.
 // (int16 and lengths that are no multiple of 16 ran a strided scalar kernel: 0.75 TB/s and 0.37 TB/s against 5.8 here.)
@@ -205,15 +244,18 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
 {
     if (early)
         grid_dep_launch();
+    grid_dep_wait();
     constexpr int V = 4 * W / (int)sizeof(T), PER_WORD = 4 / (int)sizeof(T), BITS = 8 * (int)sizeof(T);
     __shared__ int8_t table[256];
-    // One-operand int8 -> int8 operators are functions of the input byte: every block tabulates the operator once with
-    // the scalar code (so the rounding is the reference's) and then runs as a table lookup like LUT itself.
-    constexpr bool TABULATED = sizeof(T) == 1 && (OP == ESPDL_ELT_REQUANTIZE || OP == ESPDL_ELT_CLIP || OP == ESPDL_ELT_RELU);
-    constexpr bool LOOKUP = sizeof(T) == 1 && (OP == ESPDL_ELT_LUT || TABULATED);
-    // In a small network a launch is one trip through memory: where the first unit lies and what the operator makes of a byte are found out before the wait for
-    // the previous kernel, and the unit is on its way while the block meets over the table (LUT's own, an operand like any other, is read behind the wait).
-    auto offsets = [&](long long v, long long &io, long long &ia, long long &ib) {
+    constexpr bool LOOKUP = elt_lookup<T>(OP);
+    if (LOOKUP) {
+        fill_table<OP>(p, table);
+        __syncthreads();
+    }
+    auto one = [&](int a, int b) { return elt_one<OP, T>(p, table, a, b); };
+    const long long threads = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long v = first; v < nvec; v += threads) {
+        long long io, ia, ib;
         if (BCAST) {
             const long long row = v < 0x7fffffffll ? (long long)((unsigned)v / (unsigned)p.vpr) : v / p.vpr, col = v - row * p.vpr;
             const long long image = v < 0x7fffffffll ? (long long)((unsigned)row / (unsigned)p.rows_per_image) : row / p.rows_per_image;
@@ -221,51 +263,13 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
         } else {
             vec_offsets(p, v, io, ia, ib);
         }
-    };
-    const long long threads = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    long long io = 0, ia = 0, ib = 0;
-    if (sizeof(T) == 1 && first < nvec)
-        offsets(first, io, ia, ib);
-    if (LOOKUP) {
-        if (OP == ESPDL_ELT_LUT)
-            grid_dep_wait();
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-            if (OP == ESPDL_ELT_LUT) {
-                table[i] = ((const int8_t *)p.b)[i];
-            } else {
-                EltParams q2 = p;
-                q2.op = OP;
-                table[i] = (int8_t)sat8((int)max(-1000000ll, min(1000000ll, elt_int(q2, (int)(int8_t)(uint8_t)(i ^ 0x80), 0))));
-            }
-        }
-    }
-    if (!LOOKUP || OP != ESPDL_ELT_LUT)
-        grid_dep_wait();
-    auto one = [&](int a, int b) -> int {
-        if (LOOKUP)
-            return table[(uint8_t)a ^ 0x80u];
-        if (OP == ESPDL_ELT_LUT) // int16
-            return ((const int16_t *)p.b)[lut16_index(p, a)];
-        long long v = OP == ESPDL_ELT_ADD ? a + b : (OP == ESPDL_ELT_SUB ? a - b : 0);
-        if (OP != ESPDL_ELT_ADD && OP != ESPDL_ELT_SUB) {
-            EltParams q2 = p;
-            q2.op = OP;
-            v = elt_int(q2, a, b);
-        }
-        const int lo = -(1 << (BITS - 1));
-        return (int)max((long long)lo, min((long long)(-lo - 1), v));
-    };
-    struct alignas(4 * W) Unit {
-        uint32_t w[W];
-    };
-    Unit a = {}, b = {};
-    auto fetch = [&] {
-        a = ((const Unit *)p.a)[ia];
+        struct alignas(4 * W) Unit {
+            uint32_t w[W];
+        };
+        const Unit a = ((const Unit *)p.a)[ia];
+        Unit b = {}, o;
         if (elt_two_operands(OP))
             b = ((const Unit *)p.b)[ib];
-    };
-    auto finish = [&] {
-        Unit o;
 #pragma unroll
         for (int q = 0; q < W; q++) {
             uint32_t wd = 0;
@@ -277,26 +281,68 @@ __global__ void __launch_bounds__(256) elt_vec_kernel(EltParams p, long long nve
             o.w[q] = wd;
         }
         ((Unit *)p.out)[io] = o;
-    };
-    if (sizeof(T) == 1 && nvec <= threads) { // one unit a thread (int16: its results' code twice costs the large launches more than the small ones gain)
-        if (first < nvec)
-            fetch();
-        if (LOOKUP)
-            __syncthreads();
-        if (first < nvec)
-            finish();
-    } else {
-        if (LOOKUP)
-            __syncthreads();
-        for (long long v = first; v < nvec; v += threads) {
-            offsets(v, io, ia, ib);
-            fetch();
-            finish();
-        }
     }
     if (!BCAST && !p.vpr)
         for (long long i = nvec * V + first; i < p.total; i += threads)
             ((T *)p.out)[i] = (T)one((int)((const T *)p.a)[i], elt_two_operands(OP) ? (int)((const T *)p.b)[i] : 0);
+}
+
+// The same for int8 tensors of no more units than a launch has threads (int16 gains nothing by it).  In a small network a launch is one trip through memory: where the
+// unit lies and what the operator makes of a byte are found out before the wait for the previous kernel, and the unit is on its way while the block
+// meets over the table; LUT's own table, an operand like any other, is read behind the wait.  A kernel of its own: with both forms in one, launches of several units
+// a thread lost 2 to 5 % (requantize of 170194 x 95 6.73 / 7.04 us).
+template <int OP, bool BCAST, int W = 4>
+__global__ void __launch_bounds__(256) elt_unit_kernel(EltParams p, long long nvec, int early)
+{
+    if (early)
+        grid_dep_launch();
+    constexpr int V = 4 * W;
+    __shared__ int8_t table[256];
+    constexpr bool LOOKUP = elt_lookup<int8_t>(OP);
+    const long long threads = (long long)gridDim.x * blockDim.x, v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    long long io = 0, ia = 0, ib = 0;
+    if (v < nvec) {
+        if (BCAST) {
+            const unsigned row = (unsigned)v / (unsigned)p.vpr, image = row / (unsigned)p.rows_per_image; // (a launch's threads are far fewer than 2^31)
+            const long long col = (unsigned)v - row * (unsigned)p.vpr;
+            io = row * p.ro + col, ia = row * p.ra + col, ib = image * p.b_image + col;
+        } else {
+            vec_offsets(p, v, io, ia, ib);
+        }
+    }
+    const bool ahead = OP != ESPDL_ELT_LUT && early; // (outside a model's plan this starts at the other kernel's end)
+    if (LOOKUP && ahead)
+        fill_table<OP>(p, table);
+    grid_dep_wait();
+    struct alignas(4 * W) Unit {
+        uint32_t w[W];
+    };
+    Unit a = {}, b = {};
+    if (v < nvec) {
+        a = ((const Unit *)p.a)[ia];
+        if (elt_two_operands(OP))
+            b = ((const Unit *)p.b)[ib];
+    }
+    if (LOOKUP) {
+        if (!ahead)
+            fill_table<OP>(p, table);
+        __syncthreads();
+    }
+    if (v < nvec) {
+        Unit o;
+#pragma unroll
+        for (int q = 0; q < W; q++) {
+            uint32_t wd = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                wd |= ((uint32_t)elt_one<OP, int8_t>(p, table, (int)(int8_t)(a.w[q] >> (8 * j)), (int)(int8_t)(b.w[q] >> (8 * j))) & 0xffu) << (8 * j);
+            o.w[q] = wd;
+        }
+        ((Unit *)p.out)[io] = o;
+    }
+    if (!BCAST && !p.vpr)
+        for (long long i = nvec * V + v; i < p.total; i += threads)
+            ((int8_t *)p.out)[i] = (int8_t)elt_one<OP, int8_t>(p, table, (int)((const int8_t *)p.a)[i], elt_two_operands(OP) ? (int)((const int8_t *)p.b)[i] : 0);
 }
 
 // int8 (op) one-element int8 -> int8 (Mul by a scalar factor, Add of a constant, ...): with the second operand fixed the
@@ -340,18 +386,20 @@ static void launch_vec(const EltParams &p, long long nvec, bool bcast, int unit,
     const dim3 grid((unsigned)max(min((nvec + 255) / 256, (long long)num_sms() * 16), 1ll)), block(256);
     constexpr bool two = OP == ESPDL_ELT_ADD || OP == ESPDL_ELT_SUB || OP == ESPDL_ELT_MUL || OP == ESPDL_ELT_MAX || OP == ESPDL_ELT_MIN;
     constexpr bool compares = OP >= ESPDL_ELT_GREATER && OP <= ESPDL_ELT_LESS_EQUAL; // int16 in, a byte out: the scalar kernel
+    const bool one = nvec <= 256ll * grid.x, s8 = p.idt == ESPDL_DTYPE_INT8; // a unit a thread
     if constexpr (two) {
-        const auto units = p.idt == ESPDL_DTYPE_INT8 ? elt_vec_kernel<OP, int8_t, true> : elt_vec_kernel<OP, int16_t, true>;
-        const auto words = p.idt == ESPDL_DTYPE_INT8 ? elt_vec_kernel<OP, int8_t, true, 1> : elt_vec_kernel<OP, int16_t, true, 1>;
+        const auto units = !s8 ? elt_vec_kernel<OP, int16_t, true> : one ? elt_unit_kernel<OP, true> : elt_vec_kernel<OP, int8_t, true>;
+        const auto words = !s8 ? elt_vec_kernel<OP, int16_t, true, 1> : one ? elt_unit_kernel<OP, true, 1> : elt_vec_kernel<OP, int8_t, true, 1>;
         if (bcast)
             launch_mover(unit == 16 ? units : words, grid, block, 0, s, p, nvec);
     }
     if (bcast)
         return;
+    const auto bytes = one ? elt_unit_kernel<OP, false> : elt_vec_kernel<OP, int8_t, false>;
     if constexpr (compares)
-        launch_mover(elt_vec_kernel<OP, int8_t, false>, grid, block, 0, s, p, nvec);
+        launch_mover(bytes, grid, block, 0, s, p, nvec);
     else
-        launch_mover(p.idt == ESPDL_DTYPE_INT8 ? elt_vec_kernel<OP, int8_t, false> : elt_vec_kernel<OP, int16_t, false>, grid, block, 0, s, p, nvec);
+        launch_mover(s8 ? bytes : elt_vec_kernel<OP, int16_t, false>, grid, block, 0, s, p, nvec);
 }
 
 } // namespace espdl
