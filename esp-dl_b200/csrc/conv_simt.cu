@@ -86,11 +86,11 @@ __global__ void __launch_bounds__(256) conv_s8_kernel(ConvParams p)
     for (long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / lanes; __any_sync(0xffffffffu, first < p.total); first += step) {
         const bool live = first < p.total;
         const long long item = live ? first : p.total - 1;
-        long long g_rem;
-        const long long pix = div_rem(item, p.groups, g_rem);
-        const int g = (int)g_rem;
-        int ox, oy, n;
-        split_pixel(pix, p.ow, p.oh, ox, oy, n);
+        const int g = (int)(item % p.groups);
+        const long long pix = item / p.groups;
+        const int ox = (int)(pix % p.ow);
+        const int oy = (int)((pix / p.ow) % p.oh);
+        const int n = (int)(pix / ((long long)p.ow * p.oh));
         const int oc0 = g * OCT;
         int32_t acc[OCT];
 #pragma unroll
@@ -139,11 +139,11 @@ __global__ void __launch_bounds__(256) conv_s16_kernel(ConvParams p)
     for (long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / lanes; __any_sync(0xffffffffu, first < p.total); first += step) {
         const bool live = first < p.total;
         const long long item = live ? first : p.total - 1;
-        long long g_rem;
-        const long long pix = div_rem(item, p.groups, g_rem);
-        const int g = (int)g_rem;
-        int ox, oy, n;
-        split_pixel(pix, p.ow, p.oh, ox, oy, n);
+        const int g = (int)(item % p.groups);
+        const long long pix = item / p.groups;
+        const int ox = (int)(pix % p.ow);
+        const int oy = (int)((pix / p.ow) % p.oh);
+        const int n = (int)(pix / ((long long)p.ow * p.oh));
         const int oc0 = g * OCT;
         long long acc[OCT];
 #pragma unroll
@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(256) conv_s8_small_k_kernel(ConvParams p)
     const long long pixels = (long long)p.n * p.oh * p.ow;
     const bool vec_store = (p.oc % 16 == 0) && (p.ops % 16 == 0) && (((uintptr_t)p.out) % 16 == 0);
     for (long long pix = blockIdx.x * (long long)blockDim.x + threadIdx.x; pix < pixels; pix += (long long)gridDim.x * blockDim.x) {
-        int ox, oy, n;
-        split_pixel(pix, p.ow, p.oh, ox, oy, n);
+        const int ox = (int)(pix % p.ow);
+        const int oy = (int)((pix / p.ow) % p.oh);
+        const int n = (int)(pix / ((long long)p.ow * p.oh));
         int a[words];
 #pragma unroll
         for (int i = 0; i < words; i++) a[i] = 0;
