@@ -108,6 +108,7 @@ struct TcParams {
     int resident;     // the filter stays in shared memory, see plan_resident: column tiles of a CTA (0: tiles bring their part of it with them)
     int in_turn;      // resident: epilogue groups take two accumulators in turn and stage pieces of 64 columns in two buffers, see plan_resident
     int n_groups;     // resident: groups of CTAs, each with its own column tiles (resident_share)
+    int share, shares; // what a row tile costs a group, and all groups (the last one's columns may be fewer)
     EpiConfig epi;
 };
 
@@ -311,17 +312,17 @@ __device__ __forceinline__ int requant_wide(int vh, int vm, int vl, int row_h, i
     return (int)__funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
 }
 
-// Whose column tiles a CTA has: group g has tiles g * resident .. + resident - 1 of the filter and a share of the CTAs in proportion to its columns.
+// Whose column tiles a CTA has: group g has tiles g * resident .. + resident - 1 of the filter and a share of the CTAs in proportion to what a row tile costs it.
 struct ResidentShare {
     int first, across;   // column tiles
     int member, members; // this CTA's place in its group
 };
 __device__ __forceinline__ ResidentShare resident_share(const TcParams &p)
 {
-    const int width = p.resident * p.block_n, grid = (int)gridDim.x;
+    const int grid = (int)gridDim.x;
     int g = 0, begin = 0, end = grid;
     for (; g < p.n_groups; g++, begin = end) {
-        end = g + 1 == p.n_groups ? grid : (int)((long long)grid * ((g + 1) * width) / p.N);
+        end = g + 1 == p.n_groups ? grid : (int)((long long)grid * ((g + 1) * p.share) / p.shares);
         if ((int)blockIdx.x < end)
             break;
     }
@@ -1450,6 +1451,19 @@ void plan_resident(const espdl_conv_desc &d, TcParams &p)
         return;
     // more memory than the other plans take only for what has to fit: what it leaves of an SM's serves kernels of parallel branches
     q.stages = (int)min((size_t)MAX_STAGES, max(ring, room - q.resident * b_tile - min(room - q.resident * b_tile, SMEM_BUDGET_DEEP - SMEM_BUDGET)) / a_stage);
+    // A row tile costs a group its columns' results (4.5 ns each; the two sets of epilogue warps take the tiles in turn, so that with an even number of them one set has
+    // the wide ones), and no less than the way of its 128 x K bytes into shared memory (26 bytes a cycle when all SMs load) or the latency of that, shared by the row
+    // tiles that the ring holds (1.6 us).  By columns alone a last group of 16 had two of 148 CTAs for as many rows as the others.
+    const int across = q.n_tiles - (q.n_groups - 1) * q.resident, load = max(5 * q.K / 8, 360 * q.k_blocks / q.stages);
+    q.share = max(q.resident * q.block_n, load);
+    q.shares = (q.n_groups - 1) * q.share + max(across % 2 ? q.N - (q.n_tiles - across) * q.block_n : across * q.block_n, load);
+    // Several groups load the rows several times: not where that outweighs the columns (65536 x 384 -> 144 8.6 us, 10.8 resident), where rows leave by warps (31646 x 160 -> 2648
+    // 62 / 115), and where parts of a 32-byte sector are written by different groups and rows and results are more than L2 holds, unless
+    // the rows' own sectors are cut as well and tiles of 256 columns read them oftener (90000 x 64 -> 3088 81 / 105, 60000 x 192 -> 2032 45 / 50; 84843 x 144 -> 1616 72 / 59).
+    const long long ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c, ips = d.in_pixel_stride ? d.in_pixel_stride : d.in_c;
+    const bool cut = ops % 32 && q.M * (ops + ips) > 126000000ll && (q.k_blocks == 1 || q.K % 32 == 0);
+    if (q.n_groups > 1 && (!q.in_turn || 5 * q.shares > 12 * q.N || cut))
+        return;
     if (q.resident > 1 && q.stages < 2 * q.k_blocks) // (more stages than there are barriers)
         return;
     p = q;

@@ -41,6 +41,7 @@ RESIDENT_SHAPES = [
     (120000, 16, 192, {}), (90000, 32, 320, {}), (60000, 48, 576, {}),                    # every second piece of a column tile without columns, many tiles a CTA
     (37900, 1040, 32, {}),                                                               # more blocks of K than stages
     (13000, 320, 272, {}),                                                               # groups of CTAs, a column tile each
+    (20000, 256, 528, {}), (20000, 256, 912, {}), (38000, 160, 1984, {}),                 # the last group's share: one column tile of 16, an even number, one of 64
     (76000, 16, 32, {}), (80000, 32, 144, {}),                                           # tiles handed out by the counter
     (38000, 32, 50, {}), (37900, 48, 100, {}), (40000, 16, 410, {}),                         # columns that are no multiple of 16
     (37900, 64, 96, dict(e_out=-14)), (37900, 32, 176, dict(e_out=-14, res=True)),                                                    # shifts outside the fast form
