@@ -1470,10 +1470,11 @@ void plan_resident(const espdl_conv_desc &d, TcParams &p)
 }
 
 // int16 products in tiles of bn columns: rounds of tiles over the SMs; a tile's instructions (two of twice the width every 32 bytes of K), its loads of two planes at
-// 64 bytes a cycle, and its results at 47 cycles a column, beside the next tile's products where there are two sets of accumulators.
-double int16_tile_cycles(const TcParams &p, int bn)
+// 64 bytes a cycle, and its results at 35 cycles a column and 2400 a tile (rows that leave by warps: a column of whole groups of 64), beside the next tile's products
+// where there are two sets of accumulators.
+double int16_tile_cycles(const TcParams &p, int bn, bool by_warps)
 {
-    const double rounds = ceil((double)p.m_tiles * ((p.N + bn - 1) / bn) / num_sms()), results = 47.0 * bn;
+    const double rounds = ceil((double)p.m_tiles * ((p.N + bn - 1) / bn) / num_sms()), results = 2400 + 35.0 * (by_warps ? (bn + 63) / 64 * 64 : bn);
     const double products = max((p.K + 31) / 32 * 2.0 * max(bn, 32 + bn / 2), 2.0 * (BLOCK_M + bn) * p.K / 64);
     return 6 * bn <= 512 ? rounds * max(products, results) + results : rounds * (products + results);
 }
@@ -1501,12 +1502,15 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
         const int tiles = (p.N + cap - 1) / cap;
         return (((p.N + tiles - 1) / tiles) + 15) / 16 * 16;
     };
+    const long long ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
+    const bool rows16 = ops % 8 != 0 || p.N % 8 != 0 || ((uintptr_t)d.output % 16) != 0; // int16 rows that leave by warps (see below)
     if (i16 && max_bn > 64) {
         // Tiles of up to 80 columns leave room for a second set of accumulators, so that a tile is multiplied while the one before it is requantised; wider ones
-        // load less for a result.  Cycles by what either takes (int16_tile_cycles); narrower where that is a tenth less.  us at most 128 / 80 / 64 columns:
-        // 4096x1024x1024 24.7 / 23.1 / 25.9, 2887x1072x3768 72 / 62 / 68, 65536x512x128 57.2 / - / 52.9, 4096x2048x512 22.7 / 26.1 / 24.9, 25916x48x952 48 / 51 / 54.
-        const double wide = int16_tile_cycles(p, width(max_bn)), mid = int16_tile_cycles(p, width(80)), narrow = int16_tile_cycles(p, width(64));
-        if (min(mid, narrow) < 0.9 * wide)
+        // load less for a result.  Cycles by what either takes (int16_tile_cycles), within 0.8 % of the best of the three over 190 products; without a tile's
+        // own cost the choice lost up to 13 % of the widest.  us at most 128 / 80 / 64 columns: 4096x1024x1024 24.7 / 23.1 / 25.9, 2887x1072x3768 72 / 62 / 68,
+        // 65536x512x128 57.2 / - / 52.9, 4096x2048x512 22.7 / 26.1 / 24.9, 65536x96x2048 215 / 240 / 245; by warps 65536x256x1006 164 / 214 / 198.
+        const double wide = int16_tile_cycles(p, width(max_bn), rows16), mid = int16_tile_cycles(p, width(80), rows16), narrow = int16_tile_cycles(p, width(64), rows16);
+        if (min(mid, narrow) < 0.95 * wide)
             max_bn = mid < narrow ? 80 : 64;
     }
     p.n_tiles = (p.N + max_bn - 1) / max_bn;
@@ -1534,12 +1538,11 @@ bool plan(const espdl_conv_desc &d, TcParams &p, bool force_direct = false)
         return false;
     p.tmem_cols = pow2;
     // staged epilogue (int8): each group of four epilogue warps owns a piece of block_n / parts columns
-    const long long ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     p.out_pw = 0, p.out_mask = 0;
     p.out_rows = 0;
     if (i16) {
         p.out_pw = p.block_n / 2; // four times [128][out_pw] = the tile
-        p.out_rows = ops % 8 != 0 || p.N % 8 != 0 || ((uintptr_t)d.output % 16) != 0; // (see below)
+        p.out_rows = rows16;
     } else if (stageable) {
         // A TMA store clips rows in units of 16 bytes: behind a row that ends in the middle of one it would write the neighbour's columns.
         p.out_rows = ops % 16 != 0 || p.N % 16 != 0 || ((uintptr_t)d.output % 16) != 0;
