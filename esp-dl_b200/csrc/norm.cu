@@ -308,7 +308,7 @@ __device__ __forceinline__ void unit_squares(uint4 w, F2 minus_mean, float (&d2)
 }
 
 // The ordered sum of a row's squared differences, `units` 16-byte units: the next unit's squares are made beside the chain of this one's additions, which
-// alone is four cycles an element (100352 rows of 768: 57.3 us pair by pair, 54.9; 40000 of 1024, where its registers cost a block an SM, 31.1 / 33.8).
+// alone is four cycles an element (100352 rows of 768: 57.3 us pair by pair, 54.9).  Its registers leave four blocks an SM, see launch_layer_rows.
 template <typename T>
 __device__ __forceinline__ float ordered_squares(const uint4 *row, int units, float mean)
 {
@@ -374,9 +374,9 @@ __device__ __forceinline__ uint32_t norm_word(uint32_t codes, F2 minus_mean, F2 
 // 64 21.3 -> 12.8).  Copying, summing and normalising take 9, 17 and 31 us of these 57, hardly beside each other although blocks are independent; a warp that
 // copies and sums the next rows while eight normalise these was slower (80: the one warp's chain of additions is in the way).
 // WORDS: rows are whole aligned words in global memory; otherwise the block's rows, one contiguous run of bytes, are dealt out to
-// and collected from the padded rows byte by byte.  UNITS: rows of whole 16-byte units; forms of their own, because what a block fetches of a kernel's code
+// and collected from the padded rows byte by byte.  UNITS: rows of whole 16-byte units, 2: their squares made ahead; forms of their own, because what a block fetches of a kernel's code
 // counts in the shortest launches (6250 rows of 16: 3.77 us, 3.99 with both forms in one kernel).
-template <typename T, bool WORDS, bool EVEN, bool UNITS>
+template <typename T, bool WORDS, bool EVEN, int UNITS>
 __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, int pitch, int across, int across16, int early)
 {
     if (early)
@@ -459,8 +459,13 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
                     var = __fadd_rn(__fadd_rn(var, a), b);
                 }
             };
-            if (UNITS)
+            if (UNITS == 2)
                 var = ordered_squares<T>((const uint4 *)row, full / 4, mean);
+            else if (UNITS)
+                for (int i = 0; i < full; i += 4) {
+                    const uint4 w = *(const uint4 *)(row + i);
+                    add_squares(w.x), add_squares(w.y), add_squares(w.z), add_squares(w.w);
+                }
             else
 #pragma unroll 4
                 for (int i = 0; i < full; i++) add_squares(row[i]);
@@ -562,17 +567,23 @@ int launch_layer_rows(const NormParams &p, int R, int pitch, cudaStream_t s)
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        for (auto k : {layer_rows_kernel<T, true, false, false>, layer_rows_kernel<T, true, true, false>, layer_rows_kernel<T, false, false, false>,
-                       layer_rows_kernel<T, false, true, false>, layer_rows_kernel<T, true, false, true>, layer_rows_kernel<T, true, true, true>})
+        for (auto k : {layer_rows_kernel<T, true, false, 0>, layer_rows_kernel<T, true, true, 0>, layer_rows_kernel<T, false, false, 0>, layer_rows_kernel<T, false, true, 0>,
+                       layer_rows_kernel<T, true, false, 1>, layer_rows_kernel<T, true, true, 1>, layer_rows_kernel<T, true, false, 2>, layer_rows_kernel<T, true, true, 2>})
             if (attr_err == cudaSuccess)
                 attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     });
     if (attr_err != cudaSuccess)
         return set_cuda_error(attr_err, "cudaFuncSetAttribute(layer_rows_kernel)");
     const long long groups = (p.rows + R - 1) / R;
-    const auto kernel = pitch % 4 == 0 ? (p.half_even ? layer_rows_kernel<T, true, true, true> : layer_rows_kernel<T, true, false, true>)
-        : words                        ? (p.half_even ? layer_rows_kernel<T, true, true, false> : layer_rows_kernel<T, true, false, false>)
-                                       : (p.half_even ? layer_rows_kernel<T, false, true, false> : layer_rows_kernel<T, false, false, false>);
+    // Squares ahead of their sum where the rows leave four blocks an SM or the launch has no more (7812 rows of 1024 11.3 us, 10.8 so); beyond that the blocks that
+    // its registers cost are worth more: us ahead / not, 58593 rows of 1024 48.9 / 45.6, 104166 of 576 44.4 / 42.7, int16 58593 of 512 38.9 / 34.7, 234375 of
+    // 128 29.0 / 27.9.  int8 at five blocks is even (156250 of 384 40.2 / 40.4, 187500 of 320 39.4 / 40.6).
+    const int blocks = (int)(227 * 1024 / (smem + 1024));
+    const bool ahead = groups <= 4ll * num_sms() || blocks < (sizeof(T) == 1 ? 6 : 5);
+    const auto kernel = pitch % 4 == 0 ? (ahead ? (p.half_even ? layer_rows_kernel<T, true, true, 2> : layer_rows_kernel<T, true, false, 2>)
+                                                : (p.half_even ? layer_rows_kernel<T, true, true, 1> : layer_rows_kernel<T, true, false, 1>))
+        : words                        ? (p.half_even ? layer_rows_kernel<T, true, true, 0> : layer_rows_kernel<T, true, false, 0>)
+                                       : (p.half_even ? layer_rows_kernel<T, false, true, 0> : layer_rows_kernel<T, false, false, 0>);
     // Threads along a row: all of its columns, or a part of them at a time where that leaves fewer threads without work; a pass converts the constants of its
     // columns first, about two rows' work (8370 rows of 264, whose 66 words are three rows at once or seven in two passes: 6.8 us in one, 7.9 in two).
     const int columns = (p.len + Word<T>::V - 1) / Word<T>::V / (pitch % 4 != 0 ? 1 : sizeof(T) == 1 ? 2 : 4);

@@ -160,6 +160,22 @@ def test_gpu_columns_and_alignments(rows, n, off, dt):
             np.testing.assert_array_equal(dev.download(ptrs[k], want[k]), want[k], err_msg=k)
 
 
+# more blocks than four an SM, of which five and more fit: squares are not made ahead
+@pytest.mark.gpu
+@pytest.mark.parametrize("round_mode", [abi.ROUND_HALF_UP, abi.ROUND_HALF_EVEN])
+@pytest.mark.parametrize("rows,n,dt", [(19100, 1024, abi.DTYPE_INT8), (19100, 512, abi.DTYPE_INT16), (95200, 128, abi.DTYPE_INT16)])
+def test_gpu_many_blocks_of_few_rows(rows, n, dt, round_mode):
+    import gpu_util
+    a = make(abi.NORM_LAYER, dt, rows, n, seed=rows + n, round_mode=round_mode)
+    want = fresh(a)
+    assert checkers.oracle().oracle_norm(C.byref(desc(want))) == 0
+    with gpu_util.DeviceBuffers() as dev:
+        ptrs = {k: dev.upload(a[k]) for k in ("scale", "bias", "mean", "inv", "x", "y")}
+        abi.check(dev.lib.espdl_b200_norm(C.byref(desc(a, ptrs)), None), "norm")
+        for k in ("y", "mean", "inv"):
+            np.testing.assert_array_equal(dev.download(ptrs[k], want[k]), want[k], err_msg=k)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("op", [abi.NORM_RMS, abi.NORM_LAYER])
 @pytest.mark.parametrize("shape,axis", [((2, 9, 64), -1), ((3, 4, 5, 16), 2)])
