@@ -374,7 +374,7 @@ __device__ __forceinline__ uint32_t norm_word(uint32_t codes, F2 minus_mean, F2 
 // 64 21.3 -> 12.8).  Copying, summing and normalising take 9, 17 and 31 us of these 57, hardly beside each other although blocks are independent; a warp that
 // copies and sums the next rows while eight normalise these was slower (80: the one warp's chain of additions is in the way).
 // WORDS: rows are whole aligned words in global memory; otherwise the block's rows, one contiguous run of bytes, are dealt out to
-// and collected from the padded rows byte by byte.  UNITS: rows of whole 16-byte units, 2: their squares made ahead; forms of their own, because what a block fetches of a kernel's code
+// and collected from the padded rows byte by byte.  UNITS: rows of whole 16-byte units, 2: their squares made ahead, 3: results that begin at any word; forms of their own, because what a block fetches of a kernel's code
 // counts in the shortest launches (6250 rows of 16: 3.77 us, 3.99 with both forms in one kernel).
 template <typename T, bool WORDS, bool EVEN, int UNITS>
 __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, int pitch, int across, int across16, int early)
@@ -534,7 +534,10 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
                     uint2 y;
                     y.x = word(x.x ^ FLIP, minus_mean, inv_std, sv, bv);
                     y.y = word(x.y ^ FLIP, minus_mean, inv_std, sv + V / 2, bv + V / 2);
-                    *(uint2 *)to = y;
+                    if (UNITS == 3)
+                        to[0] = y.x, to[1] = y.y;
+                    else
+                        *(uint2 *)to = y;
                 } else if (W == 4) {
                     const uint4 x = *(const uint4 *)from;
                     uint4 y;
@@ -542,7 +545,10 @@ __global__ void __launch_bounds__(256) layer_rows_kernel(NormParams p, int R, in
                     y.y = word(x.y ^ FLIP, minus_mean, inv_std, sv + V / 2, bv + V / 2);
                     y.z = word(x.z ^ FLIP, minus_mean, inv_std, sv + V, bv + V);
                     y.w = word(x.w ^ FLIP, minus_mean, inv_std, sv + 3 * V / 2, bv + 3 * V / 2);
-                    *(uint4 *)to = y;
+                    if (UNITS == 3)
+                        to[0] = y.x, to[1] = y.y, to[2] = y.z, to[3] = y.w;
+                    else
+                        *(uint4 *)to = y;
                 } else {
                     const uint32_t y = word(*from ^ FLIP, minus_mean, inv_std, sv, bv);
                     if (WORDS)
@@ -568,7 +574,8 @@ int launch_layer_rows(const NormParams &p, int R, int pitch, cudaStream_t s)
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
         for (auto k : {layer_rows_kernel<T, true, false, 0>, layer_rows_kernel<T, true, true, 0>, layer_rows_kernel<T, false, false, 0>, layer_rows_kernel<T, false, true, 0>,
-                       layer_rows_kernel<T, true, false, 1>, layer_rows_kernel<T, true, true, 1>, layer_rows_kernel<T, true, false, 2>, layer_rows_kernel<T, true, true, 2>})
+                       layer_rows_kernel<T, true, false, 1>, layer_rows_kernel<T, true, true, 1>, layer_rows_kernel<T, true, false, 2>, layer_rows_kernel<T, true, true, 2>,
+                       layer_rows_kernel<T, true, false, 3>, layer_rows_kernel<T, true, true, 3>})
             if (attr_err == cudaSuccess)
                 attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     });
@@ -580,8 +587,9 @@ int launch_layer_rows(const NormParams &p, int R, int pitch, cudaStream_t s)
     // 128 29.0 / 27.9.  int8 at five blocks is even (156250 of 384 40.2 / 40.4, 187500 of 320 39.4 / 40.6).
     const int blocks = (int)(227 * 1024 / (smem + 1024));
     const bool ahead = groups <= 4ll * num_sms() || blocks < (sizeof(T) == 1 ? 6 : 5);
-    const auto kernel = pitch % 4 == 0 ? (ahead ? (p.half_even ? layer_rows_kernel<T, true, true, 2> : layer_rows_kernel<T, true, false, 2>)
-                                                : (p.half_even ? layer_rows_kernel<T, true, true, 1> : layer_rows_kernel<T, true, false, 1>))
+    const auto kernel = pitch % 4 == 0 ? ((uintptr_t)p.out % 16 != 0 ? (p.half_even ? layer_rows_kernel<T, true, true, 3> : layer_rows_kernel<T, true, false, 3>)
+                                              : ahead ? (p.half_even ? layer_rows_kernel<T, true, true, 2> : layer_rows_kernel<T, true, false, 2>)
+                                                      : (p.half_even ? layer_rows_kernel<T, true, true, 1> : layer_rows_kernel<T, true, false, 1>))
         : words                        ? (p.half_even ? layer_rows_kernel<T, true, true, 0> : layer_rows_kernel<T, true, false, 0>)
                                        : (p.half_even ? layer_rows_kernel<T, false, true, 0> : layer_rows_kernel<T, false, false, 0>);
     // Threads along a row: all of its columns, or a part of them at a time where that leaves fewer threads without work; a pass converts the constants of its
@@ -635,7 +643,7 @@ extern "C" int espdl_b200_norm(const espdl_norm_desc *d, void *stream)
     if (d->op == ESPDL_NORM_LAYER && ((uintptr_t)d->input % 4) == 0 && ((uintptr_t)d->output % 4) == 0) {
         // rows a block: 48 KB of them (four blocks an SM keep eight warps at their rows), fewer where that leaves SMs without a block
         const int V = d->dtype == ESPDL_DTYPE_INT8 ? 4 : 2, words = (d->len + V - 1) / V;
-        const bool units = d->len % (4 * V) == 0 && (((uintptr_t)d->input | (uintptr_t)d->output) % 16) == 0;
+        const bool units = d->len % (4 * V) == 0 && ((uintptr_t)d->input % 16) == 0;
         const int pitch = units ? 4 * (words / 4 | 1) : words | 1;
         const long long fit = (50 * 1024) / ((long long)pitch * 4 + 8), share = (d->rows + num_sms() - 1) / num_sms();
         const int R = (int)min(min(256ll, max(fit, (96 * 1024) / ((long long)pitch * 4 + 8) >= 32 ? 32ll : 0ll)), max(32ll, share)) / 32 * 32;

@@ -139,7 +139,7 @@ def test_gpu_rows_of_whole_units(rows, n, skip, in_place, kw, dt, round_mode):
 
 
 # two and three units a row (int8), more columns than a block has threads at once, ragged rows in several passes; scale and bias off a word's boundary, and an
-# output off a unit's, take the general conversions and the kernel form of whole words
+# output off a unit's, take the general conversions and the form whose results begin at any word
 @pytest.mark.gpu
 @pytest.mark.parametrize("dt", [abi.DTYPE_INT8, abi.DTYPE_INT16])
 @pytest.mark.parametrize("off", ["", "scale", "y"])
