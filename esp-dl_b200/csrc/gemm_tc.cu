@@ -1432,7 +1432,8 @@ void plan_resident(const espdl_conv_desc &d, TcParams &p)
     TcParams q = p;
     if (q.N % 16 == 0 && !q.out_rows) {
         q.block_n = min(128, q.N), q.n_tiles = (q.N + q.block_n - 1) / q.block_n;
-        q.in_turn = 1, q.acc_stages = q.block_n > 64 ? 4 : 8, q.tmem_cols = 512;
+        q.in_turn = 1, q.acc_stages = q.block_n > 64 ? 4 : 8;
+        for (q.tmem_cols = 32; q.tmem_cols < q.acc_stages * q.block_n;) q.tmem_cols *= 2; // (what they leave serves kernels of parallel branches)
         q.out_pw = 64, q.out_mask = 3;
     }
     if (q.n_tiles > p.n_tiles && p.n_tiles == 1 && overlaps(d))
