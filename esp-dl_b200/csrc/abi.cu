@@ -553,7 +553,8 @@ static bool runs_mma(const espdl_conv_desc &d)
     else if (d.filter_image_stride == 0 && conv2d_conv_tc_supported(d))
         other = d.stride_h == 1 && d.dilation_h == 1 && cin_blocks == 1 && d.in_c % 32 == 0 && d.in_c != 96 && d.out_c <= 256 ? 3.9f : 2.5f + 0.33f * d.kh * d.kw * cin_blocks;
     else if (conv2d_tc_supported(d))
-        other = 3.4f + 0.33f * (cin_blocks - 1) + ((d.out_pixel_stride ? d.out_pixel_stride : d.out_c) % 16 ? 9e-6f * d.n * d.out_h * d.out_w * d.out_c : 0.f);
+        // (rows that no TMA store can address: 150 products, the one chosen within 0.1 % of the faster on average; 1930x640x176 5.2 us there, 8.2 here, 3501x544x101 7.8 / 6.8)
+        other = 3.4f + 0.33f * (cin_blocks - 1) + ((d.out_pixel_stride ? d.out_pixel_stride : d.out_c) % 16 ? 2e-6f * d.n * d.out_h * d.out_w * d.out_c : 0.f);
     else
         // packed operands: two launches, one pass over the unrolled rows; no kernel's start-up is worth waiting for beyond that
         return conv2d_mma_estimate_us(d) < (conv2d_packed_supported(d) ? min(9.f + (d.in_c % 16 == 0 ? 2.5e-7f : 3.5e-6f) * (float)d.n * d.out_h * d.out_w * d.kh * d.kw * d.in_c, conv2d_simt_estimate_us(d))
