@@ -236,6 +236,35 @@ __device__ __forceinline__ int fround_half_up(float v) { return (int)floorf(__fa
 __device__ __forceinline__ int fround_half_even(float v) { return __float2int_rn(v); }
 __device__ __forceinline__ int fround(float v, int half_even) { return half_even ? fround_half_even(v) : fround_half_up(v); }
 
+// int16's epilogue after the sums in 32-bit instructions (64-bit sums, shifts and comparisons took more than twice as many): sum + bias + 2^(s-1) as H * 65536 + L,
+// L in 16 bits, H bounded so that the shift leaves what saturates.  1 <= s <= 31, |bias| < 2^45, H below 2^30.
+struct alignas(16) HalvesParam { // of a channel
+    int h, l;  // bias + 2^(s-1)
+    int limit; // |H| beyond it is outside int16 after the shift
+    int shift;
+};
+__device__ __forceinline__ bool halves_fit(long long bias, int shift) { return shift >= 1 && shift <= 31 && bias < (1ll << 45) && bias > -(1ll << 45); }
+template <bool EVEN>
+__device__ __forceinline__ HalvesParam halves_param(long long bias, int shift)
+{
+    const int s = max(1, min(31, shift));
+    const long long add = bias + (1ll << (s - 1)) - (EVEN ? 1 : 0);
+    return {(int)(add >> 16), (int)(add & 0xffff), (int)((32768ll << max(0, s - 16)) - 1), s};
+}
+// (sum + bias + 2^(s-1)) >> s, the constants added: l with what it carries.
+template <bool EVEN>
+__device__ __forceinline__ int shift_halves(int h, int l, const HalvesParam &c)
+{
+    h += l >> 16;
+    if (EVEN) { // a tie is rounded up only where that gives an even number
+        const uint32_t q = __funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+        l = (l & 0xffff) + (int)(q & 1u);
+        h += l >> 16;
+    }
+    h = max(min(h, c.limit), ~c.limit);
+    return (int)__funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+}
+
 // a / b and what is left, a >= 0, b > 0.  A 64-bit division is some hundred instructions; a few of them were a third of the time of a small launch, most tensors'
 // indices fit 32 bits.
 __device__ __forceinline__ long long div_rem(long long a, long long b, long long &rem)

@@ -582,23 +582,11 @@ __global__ void __launch_bounds__(128) dw_taps_kernel(DwParams p)
         grid_dep_wait();
 }
 
-// int16's epilogue after the sums in 32-bit instructions, as the products' (gemm_tc.cu): 256 hi + lo + bias + 2^(s-1) as H * 65536 + L, H bounded so that the shift
-// leaves what saturates.  1 <= s <= 31, |bias| < 2^45.
-struct HalvesParam {
-    int h, l, limit, shift;
-};
+// The sums' bytes in halves (HalvesParam): 256 hi + lo.
 template <bool EVEN>
 __device__ __forceinline__ int requant_halves(int hi, int lo, const HalvesParam &c)
 {
-    int l = ((hi & 0xff) << 8) + (lo & 0xffff) + c.l;
-    int h = (hi >> 8) + (lo >> 16) + c.h + (l >> 16);
-    if (EVEN) { // a tie is rounded up only where that gives an even number
-        const uint32_t q = __funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
-        l = (l & 0xffff) + (int)(q & 1u);
-        h += l >> 16;
-    }
-    h = max(min(h, c.limit), ~c.limit);
-    return (int)__funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+    return shift_halves<EVEN>((hi >> 8) + (lo >> 16) + c.h, ((hi & 0xff) << 8) + (lo & 0xffff) + c.l, c);
 }
 __device__ __noinline__ int requant16_any(int hi, int lo, long long bias, int shift, int relu, int half_even)
 {
@@ -670,10 +658,8 @@ __global__ void __launch_bounds__(128, 6) dw_run_s16_kernel(DwParams p, int segs
     for (int c = 0; c < 4; c++) {
         const int sh = p.e_shift_base - (p.per_channel ? __ldg(p.ew + ch + c) : p.ew_scalar);
         const long long b = p.bias ? __ldg((const long long *)p.bias + ch + c) : 0ll;
-        fast = fast && sh >= 1 && sh <= 31 && b < (1ll << 45) && b > -(1ll << 45);
-        const int fs = max(1, min(31, sh));
-        const long long add = b + (1ll << (fs - 1)) - (EVEN ? 1 : 0);
-        k[c] = {(int)(add >> 16), (int)(add & 0xffff), (int)((32768ll << max(0, fs - 16)) - 1), fs};
+        fast = fast && halves_fit(b, sh);
+        k[c] = halves_param<EVEN>(b, sh);
     }
     int16_t *to = (int16_t *)p.out + ((long long)line * p.ow + ox) * p.ops + ch;
 #pragma unroll

@@ -287,29 +287,12 @@ __device__ __forceinline__ void store_staged_rows(int8_t *dst, long long pitch, 
     }
 }
 
-// Per-column constants of an int16 tile: q = (sum + bias_half) >> shift in 64 bits, as the int8 form (fast_constants).
-// w = H * 65536 + L as two 32-bit numbers, L in 16 bits: the constant bias + 2^(s-1), the bound that saturates H before the shift, the shift.
-struct alignas(16) WideParam {
-    int h, l;
-    int limit; // |H| beyond it is outside int16 after the shift
-    int shift;
-};
-
-// The whole of int16's epilogue after the sums, in 32-bit instructions (64-bit sums, shifts and comparisons took more than twice as many: 4100
-// cycles per 16 columns of a tile, and 31 us for 4096x1024x1024, now 26).  1 <= shift <= 31.
+// The three sums of an int16 result in halves (HalvesParam; K <= 16384 keeps H below 2^30).  64-bit sums took 4100 cycles for 16 columns of a tile, and
+// 31 us for 4096x1024x1024, 26 so.
 template <bool EVEN>
-__device__ __forceinline__ int requant_wide(int vh, int vm, int vl, int row_h, int row_l, const WideParam c)
+__device__ __forceinline__ int requant_wide(int vh, int vm, int vl, int row_h, int row_l, const HalvesParam c)
 {
-    int h = vh + (vm >> 8) + (c.h + row_h);
-    int l = (int)__byte_perm((uint32_t)vm, 0u, 0x4404) + vl + c.l + row_l; // the low byte of vm in the second
-    h += l >> 16;
-    if (EVEN) { // a tie is rounded up only where that gives an even number
-        const uint32_t q = __funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
-        l = (l & 0xffff) + (int)(q & 1u);
-        h += l >> 16;
-    }
-    h = max(min(h, c.limit), ~c.limit);
-    return (int)__funnelshift_r(__byte_perm((uint32_t)l, (uint32_t)h, 0x5410), (uint32_t)(h >> 16), c.shift);
+    return shift_halves<EVEN>(vh + (vm >> 8) + (c.h + row_h), (int)__byte_perm((uint32_t)vm, 0u, 0x4404) + vl + c.l + row_l, c); // (the low byte of vm in the second)
 }
 
 // Whose column tiles a CTA has: group g has tiles g * resident .. + resident - 1 of the filter and a share of the CTAs in proportion to what a row tile costs it.
@@ -581,8 +564,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int out_tile_bytes = ((BLOCK_M * p.out_pw + 1023) & ~1023) << (RES ? p.in_turn : 0); // (in turn: of two buffers)
     uint8_t *aux = smem + load_bytes + (p.one_tile ? 0 : 4 * (size_t)out_tile_bytes);
     FastParam *fast_s = (FastParam *)aux; // n_pad entries, 16-byte aligned (block_n % 16 == 0)
-    WideParam *wide_s = (WideParam *)aux; // int16: the current tile's columns
-    uint64_t *bars = (uint64_t *)(aux + (I16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)n_pad));
+    HalvesParam *wide_s = (HalvesParam *)aux; // int16: the current tile's columns
+    uint64_t *bars = (uint64_t *)(aux + (I16 ? sizeof(HalvesParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)n_pad));
     uint64_t *full_bar = bars, *empty_bar = bars + MAX_STAGES, *tfull_bar = bars + 2 * MAX_STAGES, *tempty_bar = tfull_bar + MAX_ACC;
     uint64_t *filter_bar = tempty_bar + MAX_ACC;
     uint32_t *tmem_slot = (uint32_t *)(filter_bar + 2); // (16-byte aligned)
@@ -997,11 +980,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const int n = min(n0 + j, p.N - 1);
                     const int e = p.epi.per_channel ? __ldg(p.epi.ew + n) : p.epi.ew_scalar, sh = p.epi.e_shift_base - e;
                     const long long b = p.epi.bias ? __ldg((const long long *)p.epi.bias + n) : 0ll;
-                    if (sh < 1 || sh > 31 || b >= (1ll << 45) || b <= -(1ll << 45)) // H stays below 2^30: K <= 16384
+                    if (!halves_fit(b, sh))
                         *slow_flag = 1;
-                    const int fs = max(1, min(31, sh));
-                    const long long c = b + (1ll << (fs - 1)) - (EVEN ? 1 : 0);
-                    wide_s[j] = {(int)(c >> 16), (int)(c & 0xffff), (int)((32768ll << max(0, fs - 16)) - 1), fs};
+                    wide_s[j] = halves_param<EVEN>(b, sh);
                 }
                 named_bar(EPI_BAR, EPI_WARPS * 32);
                 const bool slow = *(volatile int *)slow_flag;
@@ -1413,7 +1394,7 @@ constexpr size_t SMEM_BUDGET_DEEP = 225 * 1024; // long reductions with direct r
 
 size_t aux_bytes(const TcParams &p, bool i16 = false)
 {
-    return (i16 ? sizeof(WideParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)p.n_tiles * p.block_n) + (2 * MAX_STAGES + 2 * MAX_ACC + 2) * 8 + 32 + 256 + 2 * (TILE_RING + MAX_ACC) * 4;
+    return (i16 ? sizeof(HalvesParam) * (size_t)p.block_n : sizeof(FastParam) * (size_t)p.n_tiles * p.block_n) + (2 * MAX_STAGES + 2 * MAX_ACC + 2) * 8 + 32 + 256 + 2 * (TILE_RING + MAX_ACC) * 4;
 }
 
 // A filter that stays in shared memory.  With tiles that bring their part of the filter along, a tile of a short reduction loads more of the filter than
