@@ -419,11 +419,11 @@ __global__ void __launch_bounds__(256) dw_generic_kernel(DwParams p)
     T *__restrict__ out = (T *)p.out;
     for (long long item = blockIdx.x * (long long)blockDim.x + threadIdx.x; item < p.total;
          item += (long long)gridDim.x * blockDim.x) {
-        long long c_rem;
-        const long long pix = div_rem(item, p.c, c_rem);
-        const int c = (int)c_rem;
-        int ox, oy, n;
-        split_pixel(pix, p.ow, p.oh, ox, oy, n);
+        const int c = (int)(item % p.c);
+        const long long pix = item / p.c;
+        const int ox = (int)(pix % p.ow);
+        const int oy = (int)((pix / p.ow) % p.oh);
+        const int n = (int)(pix / ((long long)p.ow * p.oh));
         ACC acc = 0;
         for (int ky = 0; ky < p.kh; ky++) {
             const int iy = oy * p.sh + ky * p.dh - p.pt;
