@@ -401,8 +401,8 @@ __global__ void __launch_bounds__(256) copy_kernel(CopyParams p, int early)
         long long r = i, si = 0, di = 0;
 #pragma unroll
         for (int k = 5; k >= 0; k--) {
-            long long idx;
-            r = div_rem(r, p.shape[k], idx);
+            const int idx = (int)(r % p.shape[k]);
+            r /= p.shape[k];
             si += idx * p.ss[k];
             di += idx * p.ds[k];
         }
