@@ -574,9 +574,11 @@ bool espdl::overlaps(const espdl_conv_desc &d)
 }
 
 // int16 on the warp-level instructions, where the other kernels take longer.  Packing and the tile kernel: two launches, the reduction's length, the
-// unrolled rows (windows about twice), the results and the products, from 37 layers, 20 % (standard deviation) off 380 others.  The
-// products' rate is a third of theirs: 4096x1024x1024 23 us there, 64 here; 45 of 11x11x256 -> 80, 3x3 22 / 37.  Results of fewer than 16 channels leave the tile kernel by
-// warps (58800x96x8 15.6 / 9.2).  Eight-element reductions are padded to 64 here, and the CUDA cores read many of them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
+// rows packed (more where they and their planes are beyond L2), the results, rows that leave by warps and tiles of 16 columns, the products, and of windows the taps
+// and units that groups of eight channels cut; from 4300 layers, 10 % (standard deviation) off them.  2000 others take 0.6 % longer than with the faster kernel of
+// the two each time; 3.8 % with the line as it was before either kernel's last changes (us here / there: 49 of 101x104x24 -> 24, 3x3 112 / 305, 120067x48x8 13 / 24; 2028x6400x48 51 / 30).
+// The products' rate is a third of theirs: 4096x1024x1024 23 us there, 64 here; 45 of 11x11x256 -> 80, 3x3 20 / 33.
+// Eight-element reductions are padded to 64 here, and the CUDA cores read many of them at once (29585x8x1 3.2 / 7.0, 12164x8x17 5.0 /
 // 6.0; 5977x8x5 3.6 / 3.3, 1088x8x192 8.9 / 3.8).  A product whose results overwrite its inputs stays with the tile kernel, which has copied those before it writes.
 static bool runs_mma16(const espdl_conv_desc &d)
 {
@@ -591,9 +593,12 @@ static bool runs_mma16(const espdl_conv_desc &d)
     const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c, us = conv2d_mma16_estimate_us(d);
     if (!product && !conv2d_packed_supported(d))
         return us < conv2d_simt_estimate_us(d) && !(K <= 8 && d.out_c <= 64 && M >= 7000);
-    const float tile = 8.0f + 2.5e-3f * K + M * K * (product ? 0.6e-6f : 1.07e-6f) + M * d.out_c * 2.0e-6f + M * K * d.out_c * 1.6e-9f +
-        (d.out_c < 16 ? M * 1.6e-4f : 0.0f);
-    return us < 0.85f * tile;
+    const int ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
+    const float N = (float)d.out_c, beyond = fmaxf(0.0f, M * K - 2.5e7f), by_warps = ops % 8 || d.out_c % 8 ? 1.0f : 0.0f, narrow = d.out_c <= 16 ? 1.0f : 0.0f;
+    const float tile = product ? 6.4f + 3.11e-3f * K + 5.4e-7f * M * K + 4.09e-7f * beyond + 1.91e-6f * M * N + 1.95e-9f * M * K * N + by_warps * M * (8.4e-5f + 4.6e-7f * N) + narrow * M * 4.2e-5f
+                               : 6.9f + 2.67e-3f * K + 4.33e-7f * M * K + 5.41e-7f * beyond + 2.12e-6f * M * N + 1.65e-9f * M * K * N + by_warps * M * 1.1e-4f + narrow * M * 2.5e-5f +
+            1.28e-5f * M * d.kh * d.kw + (d.in_c % 16 ? 6.81e-7f * M * K : 0.0f);
+    return us < 0.95f * tile; // 5040x800x96, 5x5: 13.3 us there, 15.5 here; 6400x576x64, 3x3 10.4 / 8.2
 }
 
 // Shapes no kernel reads in place, large enough for packed operands to pay (a caller without the scratch gets the CUDA-core kernel).

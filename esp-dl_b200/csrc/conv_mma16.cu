@@ -231,27 +231,34 @@ struct Mma16Plan {
 
 // The tile by waves of as many blocks as an SM holds, each its start, its results, and its runs, which take their share of the matrix instructions or the
 // latency of copies and fragments (4 of 40x40x64 -> 64, 3x3: 13.2 us with 64 x 64, 10.2 with 64 x 32, 12.0 with 32 x 32; 400x1152x128 14.5, 10.6, 7.9;
-// 102400x576x64 70, 88, 112).  That estimate is low for long reductions in few blocks, so the choice against the other kernels also looks at what 500 layers
-// took in the tile that they get, inputs in L2 and not: launch, a wave's start, what a block and a run cost beside others and alone; within 12 % (standard
-// deviation).  It counts 0.88 of that, as runs_mma16 asks for 0.85 of the other kernels' time where the first estimate decides and 0.97 where this one does.
+// 102400x576x64 70, 88, 112).  The choice against the other kernels looks at what 4500 layers took in the tile that they get, inputs in L2: a launch, a window's
+// addresses, and the blocks of the SM that has most of them, as many at a time as fit, each its results and its runs beside others or their latency alone; of many
+// blocks an SM's share and a part of the last wave.  Blocks of 32 x 32 that are one for nearly every SM take longer than fewer or more (the next launch's begin beside
+// them: 136 of 100 runs 50 us, 186 of 112 48), and inputs beyond L2 cost them.  Within 7 to 13 % (standard deviation) of 2700 other layers.
 Mma16Plan mma16_plan(const espdl_conv_desc &d)
 {
     static const struct {
         int bm, bn, resident;
         float start, block, run, latency; // us, of the choice
-        float launch, wave, side, beside, alone, first;
-    } shapes[3] = {{64, 64, 2, 1.3f, 1.8f, 0.42f, 0.85f, 2.9f, 0.85f, 2.25f, 0.35f, 0.98f, -0.6f},
-                   {64, 32, 3, 1.3f, 1.2f, 0.263f, 0.5f, 1.2f, 1.3f, 1.1f, 0.285f, 0.96f, -1.45f},
-                   {32, 32, 4, 1.0f, 1.0f, 0.2f, 0.22f, 0.1f, 0.1f, 1.95f, 0.3f, 0.205f, -1.05f}};
+        float launch, window, results, beside, alone, every, rest, beyond;
+    } shapes[3] = {{64, 64, 2, 1.3f, 1.8f, 0.42f, 0.85f, 2.4f, 0.57f, 1.83f, 0.427f, 0.5f, 0.5f, 0.25f, 0.0f},
+                   {64, 32, 3, 1.3f, 1.2f, 0.263f, 0.5f, 1.35f, 0.83f, 0.84f, 0.256f, 0.74f, 0.74f, 0.28f, 0.0f},
+                   {32, 32, 4, 1.0f, 1.0f, 0.2f, 0.22f, 0.0f, 0.31f, 1.77f, 0.267f, 0.267f, 0.49f, 0.13f, 2.4e-7f}};
     const float M = (float)d.n * d.out_h * d.out_w, runs = ceilf((float)d.kh * d.kw * d.in_c / M16_RUN);
+    const float beyond = fmaxf(0.0f, M * d.kh * d.kw * d.in_c - 2.5e7f);
+    const bool window = d.kh * d.kw > 1 || d.in_c % 16;
     Mma16Plan best = {0, 0, 1e30f};
     float least = 1e30f;
     for (const auto &s : shapes) {
-        const float blocks = ceilf(M / s.bm) * ceilf((float)d.out_c / s.bn), side = fminf((float)s.resident, ceilf(blocks / num_sms()));
-        const float waves = fmaxf(1.0f, blocks / (num_sms() * s.resident)), us = 2.0f + waves * (s.start + s.block * side + runs * fmaxf(s.latency, side * s.run));
+        const float share = ceilf(M / s.bm) * ceilf((float)d.out_c / s.bn) / num_sms(), most = ceilf(share), side = fminf((float)s.resident, most);
+        const float us = 2.0f + fmaxf(1.0f, share / s.resident) * (s.start + s.block * side + runs * fmaxf(s.latency, side * s.run));
         if (us < least) {
+            const float alone = share > 0.8f && share <= 1.0f ? s.every : s.alone;
+            const auto wave = [&](float blocks) { return s.results * blocks + runs * fmaxf(alone, blocks * s.beside); };
+            const float full = floorf(most / s.resident), last = most - full * s.resident;
             least = us;
-            best = {s.bm, s.bn, fmaxf(us, 0.876f * (s.launch + waves * (s.wave + s.side * side + fmaxf(runs * s.alone + s.first, side * runs * s.beside))))};
+            best = {s.bm, s.bn, s.launch + (window ? s.window : 0.0f) + beyond * s.beyond + (share > 2 * s.resident ? (share / s.resident + s.rest) * wave((float)s.resident)
+                                                                                              : full * wave((float)s.resident) + (last > 0 ? wave(last) : 0.0f))};
         }
     }
     return best;

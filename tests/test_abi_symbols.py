@@ -73,3 +73,11 @@ def test_int16_windows_take_the_faster_kernel(library, image, k, cin, cout, here
     need = C.c_size_t(0)
     assert library.espdl_b200_conv2d_workspace_bytes(C.byref(d), C.byref(need)) == abi.OK
     assert (need.value == 0) == (here < packed)
+
+
+# the same since rows of the reduction meet in threes here and results leave the tile kernel faster; a CUDA-core kernel asks for no scratch either
+@pytest.mark.parametrize("image,k,cin,cout,here,packed", [((49, 101, 104), 3, 24, 24, 111.7, 304.8), ((4, 41, 43), 3, 8, 80, 6.1, 10.7), ((27, 98, 95), 1, 24, 12, 30.4, 49.2),
+                                                          ((3, 46, 47), 7, 24, 48, 15.7, 25.2), ((63, 67, 66), 1, 24, 12, 33.5, 53.6), ((20, 91, 92), 3, 16, 32, 36.0, 57.6),
+                                                          ((105, 8, 8), 5, 192, 12, 54.7, 33.6), ((19, 17, 20), 5, 96, 12, 29.4, 20.7)])
+def test_int16_windows_since_both_kernels_changed(library, image, k, cin, cout, here, packed):
+    test_int16_windows_take_the_faster_kernel(library, image, k, cin, cout, here, packed)
