@@ -544,7 +544,7 @@ static bool runs_mma(const espdl_conv_desc &d)
     // What the kernel that would run otherwise takes for a small layer, from the same chains of launches (us): a start-up of 2.5
     // to 4, and 0.33 for every 128 bytes of the reduction that its matrix instructions walk one after the other.  Large layers
     // are decided by this estimate's growth: tile kernels stay below 6 us up to 200 M multiply-adds.
-    const int cin_blocks = (d.in_c + 127) / 128;
+    const int cin_blocks = (d.in_c + 127) / 128, ops = d.out_pixel_stride ? d.out_pixel_stride : d.out_c;
     float other;
     if (conv2d_stem_tc_supported(d))
         other = 4.f;
@@ -553,8 +553,10 @@ static bool runs_mma(const espdl_conv_desc &d)
     else if (d.filter_image_stride == 0 && conv2d_conv_tc_supported(d))
         other = d.stride_h == 1 && d.dilation_h == 1 && cin_blocks == 1 && d.in_c % 32 == 0 && d.in_c != 96 && d.out_c <= 256 ? 3.9f : 2.5f + 0.33f * d.kh * d.kw * cin_blocks;
     else if (conv2d_tc_supported(d))
-        // (rows that no TMA store can address: 150 products, the one chosen within 0.1 % of the faster on average; 1930x640x176 5.2 us there, 8.2 here, 3501x544x101 7.8 / 6.8)
-        other = 3.4f + 0.33f * (cin_blocks - 1) + ((d.out_pixel_stride ? d.out_pixel_stride : d.out_c) % 16 ? 2e-6f * d.n * d.out_h * d.out_w * d.out_c : 0.f);
+        // (rows that no TMA store can address leave a tile by warps: 560 products with rows of whole words within 0.6 % of the faster of the two on average, 1.1 % with 9e-6 as for others,
+        // 1930x640x176 into rows of 184 5.2 us there, 8.2 here; 2050 with other rows 0.7 %, and lower costs made dozens of them slower: by 2e-6 10352x240x100 took 7.7 there,
+        // 5.9 here, 4557x976x53 8.5 / 5.6)
+        other = 3.4f + 0.33f * (cin_blocks - 1) + (ops % 16 ? (ops % 4 ? 9e-6f : 4e-6f) * d.n * d.out_h * d.out_w * d.out_c : 0.f);
     else
         // packed operands: two launches, one pass over the unrolled rows; no kernel's start-up is worth waiting for beyond that
         return conv2d_mma_estimate_us(d) < (conv2d_packed_supported(d) ? min(9.f + (d.in_c % 16 == 0 ? 2.5e-7f : 3.5e-6f) * (float)d.n * d.out_h * d.out_w * d.kh * d.kw * d.in_c, conv2d_simt_estimate_us(d))
