@@ -11,10 +11,11 @@
 // units lie XORed with the row, so a quarter warp's 16-byte reads meet no bank conflict.
 // Bound by the latency of copies, fragments and products, one after the other, while there is a block an SM (4 of 40x40: matrix pipe 24 %, issue slots 43 %
 // busy), by the matrix instruction (39 %), permutes and addresses (issue slots 53 %) together beyond that (256 of 28x28).  A barrier for three runs of
-// the reduction instead of each, the next three on their way: 4 of 40x40x64 -> 64, 3x3 10.0 -> 8.7 us, 34 of 70x71x64 -> 24 70.8 -> 59.6, 8 of 40x40x64 14.1 -> 12.1,
-// 10x10x256 -> 256 13.2 -> 11.7 (two at a time in two / three groups 9.2 / 9.3, 62.5 / 63.2, 12.7 / 13.0, 13.3 / 12.8).  Up to five runs are all asked for at the
-// start (80x80x32 6.4 -> 6.0).  The form of 64 x 64 spills 32 bytes, 64 x 32 4.
-// us before this kernel and now: 4 of 40x40x64 -> 64 12.3 / 8.7, one of them 12.4 / 5.8, 112x112x8 -> 16 at stride 2 12.3 / 3.2, 128x512x512 10.1 / 4.5.
+// the reduction instead of each, the next three on their way (both sides in turn, launches in a chain): 4 of 40x40x64 -> 64, 3x3 9.5 -> 8.1 us, 34 of 70x71x64 -> 24
+// 69.9 -> 58.5, 8 of 40x40x64 13.4 -> 11.4, 8 of 10x10x256 -> 256 16.1 -> 14.5, 256 of 28x28x64 136 -> 124; one of 40x40x64 stays at 5.0.  (Two at a time in two / three
+// groups took 1.06 / 1.07 times as long.)  Up to five runs are all asked for at the start (112x112x8 -> 16 at stride 2 3.0 -> 2.8; 80x80x32 stays at 4.8).
+// The form of 64 x 64 spills 32 bytes, 64 x 32 4.
+// us packed and here: 4 of 40x40x64 -> 64 12.3 / 8.1, one of them 12.4 / 5.0, 112x112x8 -> 16 at stride 2 12.3 / 2.8, 128x512x512 10.1 / 4.4.
 #include "common.cuh"
 
 #include <climits>
@@ -233,8 +234,9 @@ struct Mma16Plan {
 // latency of copies and fragments (4 of 40x40x64 -> 64, 3x3: 13.2 us with 64 x 64, 10.2 with 64 x 32, 12.0 with 32 x 32; 400x1152x128 14.5, 10.6, 7.9;
 // 102400x576x64 70, 88, 112).  The choice against the other kernels looks at what 4500 layers took in the tile that they get, inputs in L2: a launch, a window's
 // addresses, and the blocks of the SM that has most of them, as many at a time as fit, each its results and its runs beside others or their latency alone; of many
-// blocks an SM's share and a part of the last wave.  Blocks of 32 x 32 that are one for nearly every SM take longer than fewer or more (the next launch's begin beside
-// them: 136 of 100 runs 50 us, 186 of 112 48), and inputs beyond L2 cost them.  Within 7 to 13 % (standard deviation) of 2700 other layers.
+// blocks an SM's share and a part of the last wave.  Blocks of 32 x 32 that are one for nearly every SM take longer in a chain than fewer or more, as the next launch's begin
+// beside them, several on each SM that has none (25 of 13x13x256 -> 16, 3x3 31 us in a chain, about 12 alone); inputs beyond L2 cost them.  Within 7 to 13 %
+// (standard deviation) of 2700 other layers.
 Mma16Plan mma16_plan(const espdl_conv_desc &d)
 {
     static const struct {
