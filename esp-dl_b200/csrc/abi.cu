@@ -575,6 +575,13 @@ bool espdl::overlaps(const espdl_conv_desc &d)
     return !(ips == ops && into >= d.in_c * es && into + d.out_c * es <= row);
 }
 
+// Can int16 layers run on the warp-level instructions?  Without scratch for packed operands (a caller's choice, or a stream under capture) they do wherever they can.
+static bool may_mma16(const espdl_conv_desc &d, bool product)
+{
+    const char *knob = getenv("ESPDL_B200_MMA16"); // 0: never, always: wherever it can run
+    return d.dtype == ESPDL_DTYPE_INT16 && d.kernel == ESPDL_KERNEL_AUTO && d.n > 0 && conv2d_mma16_supported(d) && !(knob && *knob == '0') && !(product && overlaps(d));
+}
+
 // int16 on the warp-level instructions, where the other kernels take longer.  Packing and the tile kernel: two launches, the reduction's length, the
 // rows packed (more where they and their planes are beyond L2), the results, rows that leave by warps and tiles of 16 columns, the products, and of windows the taps
 // and units that groups of eight channels cut; from 4300 layers, 10 % (standard deviation) off them.  2000 others take 0.6 % longer than with the faster kernel of
@@ -584,12 +591,10 @@ bool espdl::overlaps(const espdl_conv_desc &d)
 // 6.0; 5977x8x5 3.6 / 3.3, 1088x8x192 8.9 / 3.8).  A product whose results overwrite its inputs stays with the tile kernel, which has copied those before it writes.
 static bool runs_mma16(const espdl_conv_desc &d)
 {
-    if (d.dtype != ESPDL_DTYPE_INT16 || d.kernel != ESPDL_KERNEL_AUTO || d.n <= 0 || !conv2d_mma16_supported(d))
-        return false;
-    const char *knob = getenv("ESPDL_B200_MMA16"); // 0: never, always: wherever it can run
     const bool product = conv2d_tc_supported(d);
-    if ((knob && *knob == '0') || (product && overlaps(d)))
+    if (!may_mma16(d, product))
         return false;
+    const char *knob = getenv("ESPDL_B200_MMA16");
     if (knob && *knob == 'a')
         return true;
     const float M = (float)d.n * d.out_h * d.out_w, K = (float)d.kh * d.kw * d.in_c, us = conv2d_mma16_estimate_us(d);
@@ -774,6 +779,8 @@ int espdl_b200_conv2d_ws(const espdl_conv_desc *desc, void *workspace, size_t wo
     }
     if (runs_packed(*desc) && workspace && workspace_bytes >= conv2d_packed_workspace_bytes(*desc))
         return conv2d_packed(*desc, workspace, workspace_bytes, s);
+    if (runs_packed(*desc) && may_mma16(*desc, false) && conv2d_mma16_estimate_us(*desc) < conv2d_simt_estimate_us(*desc))
+        return conv2d_mma16(*desc, s);
     return conv2d_simt(*desc, s);
 }
 
@@ -795,6 +802,9 @@ int espdl_b200_conv2d(const espdl_conv_desc *desc, void *stream)
     // int16 Gemms and pointwise convs: the cached scratch is shared by all of them, which are serialised on the host here and must be
     // ordered on the device by the caller's streams.
     if (need > g_ws_bytes) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (may_mma16(*desc, true) && cudaStreamIsCapturing((cudaStream_t)stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+            return conv2d_mma16(*desc, (cudaStream_t)stream); // nothing can be allocated now
         if (g_ws) {
             ESPDL_CUDA_TRY(cudaDeviceSynchronize());
             ESPDL_CUDA_TRY(cudaFree(g_ws));

@@ -1,6 +1,10 @@
 """Convs whose operands are packed for the tile kernel (int16 windows, reductions and channel counts that are no multiple of 16),
 the int16 product's combined planes, and batches of products on the CUDA cores: bit-exact against the plain-C oracle at the
 extremes of the types, around tile and chunk ends."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -286,3 +290,58 @@ def test_packed_convs_on_streams_of_their_own(dtype):
             np.testing.assert_array_equal(dev.download(out, want[i]), want[i])
     for s in streams:
         lib.espdl_b200_stream_destroy(s)
+
+
+@pytest.mark.parametrize("layer", [dict(n=19, h=17, w=20, cin=96, cout=12, kh=5, kw=5, pad=(2, 2, 2, 2)), dict(n=2, h=45, w=47, cin=256, cout=48, kh=5, kw=5, pad=(2, 2, 2, 2))])
+def test_int16_windows_without_scratch(layer, monkeypatch):
+    """Layers that pack their operands where they get scratch; without it the warp-level instructions run them (the CUDA cores take a hundred times as long)."""
+    import ctypes as C
+    monkeypatch.delenv("ESPDL_B200_MMA16")
+    case = cases.conv_case(seed=7, per_channel=True, **dict(S16, wide=True), **layer)
+    want = gpu_util.run_conv_oracle(case)
+    with gpu_util.DeviceBuffers() as dev:
+        out = dev.upload(np.full_like(case["out"], 0x55))
+        d = cases.conv_desc(case, dict(input=dev.upload(case["x"]), filter=dev.upload(case["w"]), bias=dev.upload(case["b"]), filter_exponents=dev.upload(case["ew"]), output=out))
+        need = C.c_size_t(0)
+        abi.check(dev.lib.espdl_b200_conv2d_workspace_bytes(C.byref(d), C.byref(need)), "workspace")
+        assert need.value > 0
+        for size in (0, need.value - 1, need.value):
+            scratch = dev.upload(np.zeros(max(size, 1), dtype=np.uint8))
+            abi.check(dev.lib.espdl_b200_conv2d_ws(C.byref(d), scratch if size else None, size, None), "conv2d_ws")
+            np.testing.assert_array_equal(dev.download(out, want), want)
+
+
+CAPTURED_PRODUCT = r"""
+import ctypes as C, sys
+sys.path.insert(0, sys.argv[1])
+import conftest
+import numpy as np
+import cases, gpu_util
+from espdl_b200 import abi
+lib = gpu_util.lib()
+case = cases.gemm_case(seed=9, m=871, k=1920, n_out=139, per_channel=True, dtype=abi.DTYPE_INT16, **eval(sys.argv[2]))
+want = gpu_util.run_conv_oracle(case)
+stream, graph = C.c_void_p(), C.c_void_p()
+abi.check(lib.espdl_b200_stream_create(C.byref(stream)), "stream")
+with gpu_util.DeviceBuffers() as dev:
+    out = dev.upload(np.full_like(case["out"], 0x55))
+    d = cases.conv_desc(case, dict(input=dev.upload(case["x"]), filter=dev.upload(case["w"]), bias=dev.upload(case["b"]), filter_exponents=dev.upload(case["ew"]), output=out))
+    abi.check(lib.espdl_b200_graph_begin(stream), "begin")
+    st = lib.espdl_b200_conv2d(C.byref(d), stream)
+    end = lib.espdl_b200_graph_end(stream, C.byref(graph))
+    assert (st, end) == (abi.OK, abi.OK), (st, end)
+    abi.check(lib.espdl_b200_graph_launch(graph, stream), "launch")
+    abi.check(lib.espdl_b200_stream_sync(stream), "sync")
+    np.testing.assert_array_equal(dev.download(out, want), want)
+    lib.espdl_b200_graph_destroy(graph)
+lib.espdl_b200_stream_destroy(stream)
+"""
+
+
+def test_an_int16_product_is_captured_before_any_scratch_is_there():
+    """In a process of its own: a product beside the line between the kernels, whose scratch nothing could allocate any more."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    opts = {k: v for k, v in S16.items() if k != "dtype"}
+    env = {k: v for k, v in os.environ.items() if k != "ESPDL_B200_MMA16"}
+    r = subprocess.run([sys.executable, "-c", CAPTURED_PRODUCT, here, repr(opts)], capture_output=True, text=True, timeout=300, env=env)
+    assert r.returncode == 0, r.stderr[-2000:]
